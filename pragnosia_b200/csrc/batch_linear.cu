@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(BL_NT, 1) batch_linear_kernel(const __grid_con
     auto bar_empty = [&](int s) { return mb + 128 + 8 * s; };
     const uint32_t bar_acc = mb + 256;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5);
     const int n0 = blockIdx.x * BN;
     const int KB = (K + BL_BK - 1) / BL_BK;
 
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(BL_NT, 1) batch_linear_kernel(const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = warp_uniform(*tmem_slot);
     pdl_launch_dependents();
 
     if (warp == 0) {

@@ -137,7 +137,7 @@ __global__ void __launch_bounds__((2 + EPI) * 32, 1) linear_gelu_kernel(const __
     auto bar_acc_full = [&](int a) { return mb + 64 + 8 * a; };
     auto bar_acc_empty = [&](int a) { return mb + 80 + 8 * a; };
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5);
     const int tiles_n = (N + LG_BN - 1) / LG_BN;
     const long long tiles = ((M + LG_BM - 1) / LG_BM) * tiles_n;
     const int KB = (K + LG_BK - 1) / LG_BK;
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__((2 + EPI) * 32, 1) linear_gelu_kernel(const __
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = warp_uniform(*tmem_slot);
     // Launched as a programmatic dependent: the set-up above overlaps the tail of the kernel that produces x.
     pdl_wait();
     pdl_launch_dependents();
@@ -269,15 +269,12 @@ __device__ __forceinline__ void lp_arrive_cluster(uint32_t cluster_bar) {
 }
 // bounded wait on a barrier of this CTA whose arrivals come from both CTAs of the pair
 __device__ __forceinline__ bool lp_wait_cluster(uint32_t bar, uint32_t parity, int code) {
-    const long long t0 = clock64();
-    do {
-        for (int i = 0; i < 32; ++i) {
-            uint32_t ok;
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-            if (ok) return true;
-        }
-    } while (clock64() - t0 < TC_WAIT_CYCLES);
+    for (uint32_t n = WAIT_TRIES; n != 0; --n) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(bar), "r"(parity), "r"(WAIT_HINT) : "memory");
+        if (ok) return true;
+    }
     atomicExch(&g_tc_error, code);
     return false;
 }
@@ -313,7 +310,7 @@ linear_gelu_pair_kernel(const __grid_constant__ CUtensorMap mx, const __grid_con
     auto bar_acc_full = [&](int a) { return mb + 128 + 8 * a; };
     auto bar_acc_empty = [&](int a) { return mb + 144 + 8 * a; };      // used in the first CTA only
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5);
     const uint32_t rank = cluster_rank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int tiles_n = (N + LP_BN - 1) / LP_BN;
@@ -333,7 +330,7 @@ linear_gelu_pair_kernel(const __grid_constant__ CUtensorMap mx, const __grid_con
     __syncthreads();
     cluster_sync_all();                                                // the partner's barriers and tensor memory exist from here on
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = warp_uniform(*tmem_slot);
     pdl_wait();
     pdl_launch_dependents();
 

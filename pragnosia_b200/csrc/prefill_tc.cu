@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
     constexpr uint32_t ROT_BYTES = TC_C * (D / 2) * 8;
     const float2 *rot_sm = reinterpret_cast<const float2 *>(sm + SM::off_ah);
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wg = warp >> 2, sub = warp & 3;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5), wg = warp >> 2, sub = warp & 3;
     const int bh = blockIdx.x, h = bh % p.H, b = bh / p.H;
     const int T = p.T, NC = (T + TC_C - 1) / TC_C;
     const float *la = p.la != nullptr ? p.la + (size_t)bh * T : nullptr;
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = warp_uniform(*tmem_slot);
 
     // ---- fragment geometry (16x256b loads): rows l/4 and l/4+8 of the warp's 16-row group, column pairs 2(l%4)
     const int fr = lane >> 2, fq = lane & 3;

@@ -47,28 +47,6 @@ struct WsSmem {
                          stats = 512, red = 4608, rmsw = 5632;
 };
 
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void named_sync(int id, int nthreads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory"); }
-// bounded wait whose verdict is the same for every lane of the warp (the lanes leave the chunk loop together)
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int code) {
-    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;     // the common case: already complete, no suspension
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, code)) != 0;
-}
-// one arrival per warp, after every lane's shared-memory writes are visible to the async proxy
-__device__ __forceinline__ void warp_arrive(uint32_t bar, int lane) {
-    fence_proxy_async();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(bar);
-}
-
 
 template <bool RAW>
 __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
@@ -104,7 +82,7 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
     auto bar_done = [&](int s) { return mb + SM::bar_done + 8 * s; };     // tail through with chunk c        c&3
     auto bar_q = [&](int s) { return mb + SM::bar_q + 8 * s; };           // P, U issued: tiles of c final    c&3
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5);
     const int bh = blockIdx.x, h = bh % p.H, b = bh / p.H;
     const int T = p.T, NC = (T + TC_C - 1) / TC_C;
     const int tma_c0 = RAW ? h * D : 0, tma_c2 = RAW ? b : bh;
@@ -127,7 +105,7 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = warp_uniform(*tmem_slot);
     pdl_launch_dependents();
 
     if (warp < WS_FRONT) {

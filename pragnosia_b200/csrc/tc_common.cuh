@@ -9,7 +9,6 @@ namespace pgb {
 
 constexpr int TC_C = 64;
 constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;                        // polls of a sleeping poll loop
-constexpr long long TC_WAIT_CYCLES = 1ll << 27;                      // SM cycles a blocking mbarrier wait may take
 
 // Set (to the code of the wait) when a bounded mbarrier wait inside a tensor-core kernel runs out. One copy per
 // translation unit (no relocatable device code in this build); each unit exports a reader, the C ABI takes the maximum.
@@ -56,6 +55,22 @@ static inline bool tc_make_map(CUtensorMap *m, const void *ptr, long long n2, lo
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// [n2][n1][cols] dense, bf16 or fp32; box = box_cols x box_rows x 1, rows packed in shared memory (no swizzle): what a warp
+// stores through when a lane owns a column
+static inline bool tc_make_store_map(CUtensorMap *m, const void *ptr, bool f32, long long n2, long long n1, long long cols, int box_cols,
+                                     int box_rows) {
+    EncodeTiledFn fn = tc_encode_fn();
+    if (fn == nullptr) return false;
+    const int e = f32 ? 4 : 2;
+    cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)n1, (cuuint64_t)n2};
+    cuuint64_t strides[2] = {(cuuint64_t)cols * e, (cuuint64_t)(cols * n1) * e};
+    cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    return fn(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(ptr), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // ---------------------------------------------------------------------------------------------- PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -71,21 +86,37 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// bounded wait: false (and the error flag set) if the barrier has not flipped after TC_WAIT_CYCLES of the SM clock
-// (about 70 ms; a healthy kernel waits microseconds), so a broken pipeline winds down in a fraction of a second
+// Bounded wait, a handful of instructions a site: the waits of a kernel with many roles are a good part of its code, and the
+// roles share the instruction caches (a poll loop with a clock in it, unrolled at every site, made the delta walk 28 % slower).
+// Each try suspends the thread for up to WAIT_HINT ns; at most WAIT_TRIES of them: 0.13 s if every one sleeps its full time,
+// and still milliseconds, a thousand times a healthy wait, if none does. False (and the error flag set) when used up, so a
+// broken pipeline winds down in a fraction of a second.
+constexpr uint32_t WAIT_HINT = 1000, WAIT_TRIES = 1u << 17;
+__device__ __forceinline__ bool mbar_wait_tries(uint32_t bar, uint32_t parity) {
+    uint32_t left;
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .u32 n;\n\tmov.u32 n, %4;\n\t"
+                 "AGAIN:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t@p bra DONE;\n\t"
+                 "sub.u32 n, n, 1;\n\tsetp.ne.u32 p, n, 0;\n\t@p bra AGAIN;\n\tDONE:\n\tmov.u32 %0, n;\n\t}"
+                 : "=r"(left) : "r"(bar), "r"(parity), "r"(WAIT_HINT), "n"(WAIT_TRIES) : "memory");
+    return left != 0;
+}
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code) {
-    const long long t0 = clock64();
-    do {
-        for (int i = 0; i < 32; ++i)
-            if (mbar_try(bar, parity)) return true;
-    } while (clock64() - t0 < TC_WAIT_CYCLES);
-    atomicExch(&g_tc_error, code);
-    return false;
+    const bool good = mbar_wait_tries(bar, parity);
+    if (!good) atomicExch(&g_tc_error, code);
+    return good;
 }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
+// shared -> global; rows outside the tensor are not written. One thread: commit, and wait before the source is reused.
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, uint32_t src, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+                 ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void tma_store_source_free() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // plain (untiled) bulk copy global -> shared, completion counted on an mbarrier; addresses and size multiples of 16 B
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -106,6 +137,7 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
                  ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
 }
+template <typename T_> __device__ __forceinline__ T_ warp_uniform(T_ x) { return __shfl_sync(0xffffffffu, x, 0); }
 // The same issued by ONE elected lane of a converged warp: every lane executes the call with identical operands, so the
 // descriptors stay warp-uniform values (the instruction takes them from the uniform datapath) instead of being moved
 // there lane by lane under a divergent branch.
@@ -180,11 +212,62 @@ __device__ __forceinline__ void tmem_ld_frag8(uint32_t taddr, float (&v)[32]) {
                    "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                  : "r"(taddr) : "memory");
 }
+__device__ __forceinline__ void tmem_ld_frag2(uint32_t taddr, float (&v)[8]) {
+    uint32_t *r = reinterpret_cast<uint32_t *>(v);
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr) : "memory");
+}
 template <int NB>
 __device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, float (&v)[4 * NB]) {
     if constexpr (NB == 4) tmem_ld_frag4(taddr, v); else tmem_ld_frag8(taddr, v);
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void named_sync(int id, int nthreads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory"); }
+// the wait of a converged warp: the verdict is the same for every lane (they leave the chunk loop together)
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int code) {
+    const bool good = __all_sync(0xffffffffu, mbar_wait_tries(bar, parity));
+    if (!good) atomicExch(&g_tc_error, code);
+    return good;
+}
+// one arrival per warp, after every lane's shared-memory writes are visible to the async proxy
+__device__ __forceinline__ void warp_arrive(uint32_t bar, int lane) {
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
+
+// ---------------------------------------------------------------------------------------------- operand A in tensor memory
+// D[M x N] (+)= A B with A read from tensor memory: lane = row of A, each 32-bit column two consecutive bf16 along K (the
+// even one in the low half), so one K = 16 step is 8 columns. Always K-major. Called by a converged warp; one elected lane
+// issues (see mma_bf16_elect).
+__device__ __forceinline__ void mma_bf16_ts_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, e;\n\telect.sync _|e, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+                 ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+// thread i of the warp writes lane (base lane + i), 16 consecutive 32-bit columns; tmem_st_wait() before anyone reads them
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+                 "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------------------------- descriptors
 // Shared-memory matrix descriptor, 128-byte swizzle. lbo / sbo in bytes.
