@@ -222,6 +222,24 @@ int pgb_aspin_delta_prefill_noscratch_fwd(const void *q, const void *k, const vo
                                           void *o, int o_dtype, float *S_out, void *sent, int B, int H, int T, int D,
                                           void *stream);
 
+/* -------------------------------------------------------------------------------------------------------
+ * Training through the chunked scan, bf16 operands, tensor cores.
+ * pgb_aspin_delta_prefill_train_fwd: pgb_aspin_delta_prefill_fwd with bf16 output that also keeps what the backward
+ *   reads: sent bf16 [B*H][ceil(T/64)][D][D], the residuals written W bf16 [B*H][T][D], and x_scratch itself (the caller
+ *   keeps the buffer until the backward). The plain rule's forward is pgb_aspin_prefill_fwd with sent.
+ * pgb_aspin_train_bwd: every gradient of (o, S, sent) in one call. beta == NULL: plain rule (W, X, dbeta NULL).
+ *   dout bf16 [B*H][T][D]; dsent fp32 or NULL (gradient on sent); dS fp32 [B*H][D][D] or NULL (on the final state).
+ *   dq, dk, dv bf16 [B*H][T][D]; dla, dbeta fp32 [B*H][T]; dS0 fp32 or NULL. scratch: pgb_aspin_train_scratch_bytes
+ *   bytes. Limits: B*H <= 65535. All tensor pointers 16-byte aligned.
+ * ------------------------------------------------------------------------------------------------------- */
+int pgb_aspin_delta_prefill_train_fwd(const void *q, const void *k, const void *v, const float *la, const float *beta, const float *S0,
+                                      void *o, float *S_out, void *sent, void *W, void *x_scratch, long long x_scratch_bytes, int B, int H,
+                                      int T, int D, void *stream);
+long long pgb_aspin_train_scratch_bytes(int B, int H, int T, int D, int delta);
+int pgb_aspin_train_bwd(const void *q, const void *k, const void *v, const float *la, const float *beta, const void *sent, const void *W,
+                        const void *X, const void *dout, const float *dsent, const float *dS, void *dq, void *dk, void *dv, float *dla,
+                        float *dbeta, float *dS0, void *scratch, long long scratch_bytes, int B, int H, int T, int D, void *stream);
+
 /* ---------------------------------------------------------------------------------------------------------
  * The same chunked prefill (plain rule, bf16 operands, tensor cores) with the layer's neighbouring elementwise steps
  * fused in, so a layer's prefill is: projection GEMM -> prep -> THIS -> output GEMM.

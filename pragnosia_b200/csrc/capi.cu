@@ -53,6 +53,9 @@ size_t prefill_tc_delta_scratch_bytes(int B, int H, int T);
 int prefill_tc_delta_launch(const PrefillArgs &, int, int, void *, cudaStream_t);
 int prefill_tc_delta_static_launch(const PrefillArgs &, int, int, cudaStream_t);
 long long prefill_tc_delta_static_capacity();
+size_t train_bwd_scratch_bytes(int B, int H, int T, int D, bool delta);
+int train_bwd_launch(const TrainBwdArgs &, int, cudaStream_t);
+int tc_train_error_flag(int *);
 int rot_table_launch(const float *, float *, int, int, int, cudaStream_t);
 int decode_embed_launch(const long long *, const long long *, const void *, const void *, void *, int, int, int, int, float *, cudaStream_t);
 int decode_sample_launch(const void *, int, float, float, unsigned long long, long long *, long long *, int, long long *, long long *, float *,
@@ -531,6 +534,9 @@ int pgb_tc_error_flag(int *out_host) {
     int e = 0, f = 0;
     if (rc == PGB_OK) rc = decode_token_error_flag(&e);
     if (rc == PGB_OK) rc = batch_linear_error_flag(&f);
+    int g = 0;
+    if (rc == PGB_OK) rc = tc_train_error_flag(&g);
+    f = f > g ? f : g;
     e = e > f ? e : f;
     b = b > c ? b : c;
     b = b > d ? b : d;
@@ -559,6 +565,43 @@ int pgb_aspin_delta_prefill_fwd(const void *q, const void *k, const void *v, con
         return PGB_ERR_MISALIGNED;
     PrefillArgs a{q, k, v, la, beta, S0, o, S_out, (__nv_bfloat16 *)sent, theta, shift_dev, shift_host, B, H, T};
     return prefill_tc_delta_launch(a, o_dtype, D, x_scratch, (cudaStream_t)stream);
+}
+
+int pgb_aspin_delta_prefill_train_fwd(const void *q, const void *k, const void *v, const float *la, const float *beta, const float *S0,
+                                      void *o, float *S_out, void *sent, void *W, void *x_scratch, long long x_scratch_bytes, int B, int H,
+                                      int T, int D, void *stream) {
+    if (!q || !k || !v || !la || !beta || !o || !S_out || !sent || !W || !x_scratch) return PGB_ERR_NULL_POINTER;
+    if (B <= 0 || H <= 0 || T <= 0) return PGB_ERR_BAD_SHAPE;
+    if ((long long)B * H > 65535 || (T + 63) / 64 > 65535) return PGB_ERR_TOO_LARGE;
+    if (D != 64 && D != 128) return PGB_ERR_UNSUPPORTED_DIM;
+    if (x_scratch_bytes < pgb_aspin_delta_scratch_bytes(B, H, T)) return PGB_ERR_BAD_SHAPE;
+    if (!aligned(q, 16) || !aligned(k, 16) || !aligned(v, 16) || !aligned(o, 16) || !aligned(S_out, 16) || (S0 && !aligned(S0, 16)) ||
+        !aligned(sent, 16) || !aligned(W, 16) || !aligned(x_scratch, 16))
+        return PGB_ERR_MISALIGNED;
+    PrefillArgs a{q, k, v, la, beta, S0, o, S_out, (__nv_bfloat16 *)sent, nullptr, nullptr, 0.f, B, H, T};
+    a.W_out = W;
+    return prefill_tc_delta_launch(a, PGB_BF16, D, x_scratch, (cudaStream_t)stream);
+}
+
+long long pgb_aspin_train_scratch_bytes(int B, int H, int T, int D, int delta) {
+    if (B <= 0 || H <= 0 || T <= 0 || (D != 64 && D != 128)) return 0;
+    return (long long)train_bwd_scratch_bytes(B, H, T, D, delta != 0);
+}
+
+int pgb_aspin_train_bwd(const void *q, const void *k, const void *v, const float *la, const float *beta, const void *sent, const void *W,
+                        const void *X, const void *dout, const float *dsent, const float *dS, void *dq, void *dk, void *dv, float *dla,
+                        float *dbeta, float *dS0, void *scratch, long long scratch_bytes, int B, int H, int T, int D, void *stream) {
+    if (!q || !k || !v || !la || !sent || !dout || !dq || !dk || !dv || !dla || !scratch) return PGB_ERR_NULL_POINTER;
+    if (beta && (!W || !X || !dbeta)) return PGB_ERR_NULL_POINTER;
+    if (B <= 0 || H <= 0 || T <= 0) return PGB_ERR_BAD_SHAPE;
+    if ((long long)B * H > 65535 || (T + 63) / 64 > 65535) return PGB_ERR_TOO_LARGE;
+    if (D != 64 && D != 128) return PGB_ERR_UNSUPPORTED_DIM;
+    if (scratch_bytes < pgb_aspin_train_scratch_bytes(B, H, T, D, beta != nullptr)) return PGB_ERR_BAD_SHAPE;
+    const void *ptrs[] = {q, k, v, sent, W, X, dout, dsent, dS, dq, dk, dv, dS0, scratch};
+    for (const void *x : ptrs)
+        if (x && !aligned(x, 16)) return PGB_ERR_MISALIGNED;
+    TrainBwdArgs a{q, k, v, la, beta, sent, W, X, dout, dsent, dS, dq, dk, dv, dla, dbeta, dS0, scratch, B, H, T};
+    return train_bwd_launch(a, D, (cudaStream_t)stream);
 }
 
 int pgb_rotate_pairs(const void *x, int dtype, const float *theta, const float *pos, void *out, int B, int H, int T, int D,

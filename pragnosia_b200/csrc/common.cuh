@@ -75,7 +75,14 @@ struct PrefillArgs {
     const float *rms_w = nullptr; float rms_eps = 0.f; int o_token_major = 0;
     // raw mode: q, k, v are (B,T,H*D) views of the projection output with strides (raw_sb, raw_st); the kernel does the
     // normalise / gate / rotate itself (gate_raw: write-gate logits with la_raw's strides; rot: table [H][rot_T][D/2])
+    void *W_out = nullptr;                                            // delta rule: the residuals written, bf16 [BH][T][D]
     int raw = 0; long long raw_sb = 0, raw_st = 0; const void *gate_raw = nullptr; const float *rot = nullptr; int rot_T = 0;
+};
+// the backward of the scan as one call (train_chunk.cu); beta, W and X only under the delta rule
+struct TrainBwdArgs {
+    const void *q, *k, *v; const float *la, *beta; const void *sent, *W, *X, *dout; const float *dsent, *dS;
+    void *dq, *dk, *dv; float *dla, *dbeta, *dS0; void *scratch;
+    int B, H, T;
 };
 struct DecodeArgs {
     const void *qp, *kp, *vp; long long in_sb; int normalize;

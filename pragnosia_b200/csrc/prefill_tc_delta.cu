@@ -158,6 +158,7 @@ static int delta_go(const PrefillArgs &a, int o_dtype, void *x_scratch, cudaStre
         !tc_make_map(&m.v, a.v, BH, a.T, D, D, (long long)a.T * D) ||
         !tc_make_map(&m.x, x_scratch, (long long)BH * NC * 2, TC_C, TC_C, TC_C, TC_C * TC_C) ||
         !tc_make_store_map(&m.o, a.o, f32, BH, a.T, D, 32, 32) ||
+        (a.W_out != nullptr && !tc_make_store_map(&m.w, a.W_out, false, BH, a.T, D, 32, 32)) ||
         (a.sent != nullptr && !tc_make_store_map(&m.sent, a.sent, false, (long long)BH * NC, D, D, 32, D / 2))) {
         set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled");
         return PGB_ERR_CUDA;
@@ -172,7 +173,7 @@ static int delta_go(const PrefillArgs &a, int o_dtype, void *x_scratch, cudaStre
     if (rc != PGB_OK) return rc;
     DwParams p{};
     p.la = a.la; p.beta = a.beta; p.S0 = a.S0; p.theta = a.theta; p.shift_dev = a.shift_dev; p.shift_host = a.shift_host;
-    p.S_out = a.S_out; p.want_sent = a.sent != nullptr; p.H = a.H; p.T = a.T; p.o_is_f32 = f32;
+    p.S_out = a.S_out; p.want_sent = a.sent != nullptr; p.want_w = a.W_out != nullptr; p.H = a.H; p.T = a.T; p.o_is_f32 = f32;
     walk<<<(unsigned)BH, DW_NT, DwSmem<D, false>::bytes, stream>>>(m, p);
     return check_launch("delta_walk_kernel");
 }

@@ -180,9 +180,9 @@ def prep(qp, kp, vp, gate_logits, theta, pos, out_dtype=torch.bfloat16):
 
 
 @on_device_of
-def prep_bwd(qp, kp, vp, gate_logits, theta, pos, dq, dk, dv):
+def prep_bwd(qp, kp, vp, gate_logits, theta, pos, dq, dk, dv, want_theta: bool = True):
     """Gradient of prep: returns (dqp, dkp, dvp in the projections' dtype, contiguous (B,T,H,D); dgate (B,T,H) fp32 or
-    None; dtheta (H,D/2) fp32)."""
+    None; dtheta (H,D/2) fp32, None unless want_theta)."""
     need_cuda(qp, kp, vp, theta, pos, dq, dk, dv)
     B, T, H, D = qp.shape
     qp, kp, vp, gate_logits = _prep_views(qp, kp, vp, gate_logits)
@@ -204,7 +204,7 @@ def prep_bwd(qp, kp, vp, gate_logits, theta, pos, dq, dk, dv):
                                    ptr(gate_logits), gsb, gst, ptr(theta), ptr(pos), ptr(dq), ptr(dk), ptr(dv), dtype_code(dq),
                                    ptr(dqp), ptr(dkp), ptr(dvp), ptr(dgl), ptr(part), B, T, H, D, stream_of(qp)),
           "pgb_aspin_prep_bwd")
-    return dqp, dkp, dvp, dgl, part.sum(0)
+    return dqp, dkp, dvp, dgl, (part.sum(0) if want_theta else None)
 
 
 # ----------------------------------------------------------------------------------------------------------
@@ -747,6 +747,48 @@ def delta_loop_bwd(k, v, la, be, X, sent, dW, dsent, dsfin, want_ds0: bool = Tru
                                    ptr(dkp), ptr(dv), ptr(dlap), ptr(dbep), ptr(dXp), ptr(ds0), B, H, T, D, stream_of(k)),
           "pgb_delta_loop_bwd")
     return dkp.sum(0), dv, dlap.sum(0), dbep.sum(0), dXp.sum(0), ds0
+
+
+# ---------------------------------------------------------------------------------------------------------- training
+def scan_trains(q, k, v) -> bool:
+    """Whether scan_train_fwd / scan_train_bwd take these operands (bf16, the tensor-core kernels' head dims)."""
+    return q.is_cuda and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.shape[-1] in (64, 128) and q.shape[0] * q.shape[1] <= 65535
+
+
+@on_device_of
+def scan_train_fwd(q, k, v, la, beta=None, S0=None):
+    """The scan with what its backward reads: (o, S, sent, W or None, X scratch or None); bf16 q, k, v (B,H,T,D) contiguous,
+    la / beta fp32 contiguous."""
+    if beta is None:
+        o, S, sent = prefill(q, k, v, la, None, S0, want_sent=True, precision=_lib.PREFILL_TENSOR)
+        return o, S, sent, None, None
+    B, H, T, D = q.shape
+    o, W = torch.empty_like(q), torch.empty_like(q)
+    S = torch.empty(B, H, D, D, device=q.device, dtype=torch.float32)
+    sent = torch.empty(B, H, (T + CHUNK - 1) // CHUNK, D, D, device=q.device, dtype=torch.bfloat16)
+    nbytes = lib().pgb_aspin_delta_scratch_bytes(B, H, T)
+    X = torch.empty(nbytes, device=q.device, dtype=torch.uint8)
+    check(lib().pgb_aspin_delta_prefill_train_fwd(ptr(q), ptr(k), ptr(v), ptr(la), ptr(beta), ptr(S0), ptr(o), ptr(S), ptr(sent), ptr(W),
+                                                  ptr(X), nbytes, B, H, T, D, stream_of(q)), "pgb_aspin_delta_prefill_train_fwd")
+    return o, S, sent, W, X
+
+
+@on_device_of
+def scan_train_bwd(q, k, v, la, beta, sent, W, X, dout, dsent=None, dS=None, want_dS0: bool = False):
+    """Gradients of scan_train_fwd: (dq, dk, dv bf16, dla, dbeta or None, dS0 or None fp32)."""
+    B, H, T, D = q.shape
+    dout = dout.to(torch.bfloat16).contiguous()
+    dsent, dS = _f32c(dsent), _f32c(dS)
+    dq, dk, dv = torch.empty_like(q), torch.empty_like(q), torch.empty_like(q)
+    dla = torch.empty(B, H, T, device=q.device, dtype=torch.float32)
+    dbe = None if beta is None else torch.empty_like(dla)
+    dS0 = torch.empty(B, H, D, D, device=q.device, dtype=torch.float32) if want_dS0 else None
+    nbytes = lib().pgb_aspin_train_scratch_bytes(B, H, T, D, int(beta is not None))
+    scratch = torch.empty(nbytes, device=q.device, dtype=torch.uint8)
+    check(lib().pgb_aspin_train_bwd(ptr(q), ptr(k), ptr(v), ptr(la), ptr(beta), ptr(sent), ptr(W), ptr(X), ptr(dout), ptr(dsent), ptr(dS),
+                                    ptr(dq), ptr(dk), ptr(dv), ptr(dla), ptr(dbe), ptr(dS0), ptr(scratch), nbytes, B, H, T, D,
+                                    stream_of(q)), "pgb_aspin_train_bwd")
+    return dq, dk, dv, dla, dbe, dS0
 
 
 # ---------------------------------------------------------------------------------------------------------- layer options

@@ -1,0 +1,44 @@
+"""The fused backward of the chunked scan (train_chunk.cu) through the drop-in names, against autograd through the CPU oracle
+in fp64: one token, one whole chunk, a ragged last chunk, several chunks; both rules and head dims; a gradient on each of
+the three results (outputs, final state, the states entering the chunks)."""
+import pytest
+import torch
+
+import oracle
+from pragnosia_b200 import assoc_kernel, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm())
+
+
+@pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T", [1, 64, 130, 333])
+def test_fused_backward_matches_autograd_through_the_oracle(delta, D, T):
+    B, H = 2, 3
+    x = synth.assoc_op_inputs(B, H, T, D, seed=T + D, delta=True, with_state=True)
+    g = torch.Generator().manual_seed(1)
+    w_o = torch.randn(B, H, T, D, generator=g).to(torch.bfloat16)
+    w_s, w_e = torch.randn(B, H, D, D, generator=g) * 0.1, torch.randn(B, H, (T + 63) // 64, D, D, generator=g) * 0.1
+    names = ["q", "k", "v", "la", "S0"] + (["beta"] if delta else [])
+    with torch.enable_grad():
+        ref = {n: (x[n].to(torch.bfloat16) if n in "qkv" else x[n]).double().requires_grad_(True) for n in names}
+        be = ref.get("beta")
+        o_r, S_r = oracle.assoc_scan(ref["q"], ref["k"], ref["v"], ref["la"], ref["S0"], beta=be)
+        loss = (o_r * w_o.double()).sum() + (S_r * w_s).sum()
+        for c in range((T + 63) // 64):                               # the state entering chunk c: the scan of what is before it
+            n = 64 * c
+            S_c = ref["S0"] if c == 0 else oracle.assoc_scan(*(ref[m][:, :, :n] for m in ("q", "k", "v", "la")), ref["S0"],
+                                                             beta=None if be is None else be[:, :, :n])[1]
+            loss = loss + (S_c * w_e[:, :, c]).sum()
+        loss.backward()
+        dev = {n: (x[n].to(torch.bfloat16) if n in "qkv" else x[n]).cuda().requires_grad_(True) for n in names}
+        args = [dev[n] for n in ("q", "k", "v", "la")] + ([dev["beta"]] if delta else []) + [dev["S0"]]
+        o, S, sent = (assoc_kernel.delta_scan_kernel if delta else assoc_kernel.assoc_scan_kernel)(*args)
+        ((o.float() * w_o.cuda().float()).sum() + (S * w_s.cuda()).sum() + (sent.float() * w_e.cuda()).sum()).backward()
+    assert rel(o.detach().cpu(), o_r.detach()) <= 3e-3 and rel(S.detach().cpu(), S_r.detach()) <= 1e-5
+    for n in names:                                                   # bf16 gradients; the saved states are bf16 as the operators keep them
+        assert rel(dev[n].grad.cpu(), ref[n].grad) <= 4e-3, (n, rel(dev[n].grad.cpu(), ref[n].grad))
