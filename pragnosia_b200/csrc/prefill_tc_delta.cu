@@ -6,25 +6,23 @@
 // (reference src/assoc.py:207-251). N does not depend on the state, so
 //
 //   delta_inv_kernel   (chunk-parallel, one CTA per (sequence-head, chunk)): K K^T on the tensor core, N in fp32, then
-//                      X = (I + N)^-1 by forward substitution in true fp32 FFMA -- one thread per column of X, every
-//                      intermediate bounded (the reduced-precision Neumann doubling the reference warns about at
-//                      src/assoc_kernel.py:577-582 is never formed). X goes to a scratch buffer as bf16 head + tail.
+//                      X = (I + N)^-1 by blocked forward substitution in true fp32 FFMA, every intermediate bounded (the
+//                      reduced-precision Neumann doubling the reference warns about at src/assoc_kernel.py:577-582 is
+//                      never formed). X goes to a scratch buffer as bf16 head + tail.
 //   delta_walk_kernel  (delta_walk.cuh; one CTA per (sequence, head), walking the chunks): W = X rhs, the state update and o.
 //
 // Everything fp32 that re-enters the tensor core (S, rhs, X, A, W) is split into bf16 head + tail and multiplied as
 // head*head + head*tail + tail*head. Every mbarrier wait is bounded.
 //
-// Measured, B8 H16 T8192 D128 (1.1 GB of operands): walk 1311 -> 407 us, the whole call 1640 -> 750 us.
+// Measured, B8 H16 T8192 D128 (1.1 GB of operands): walk 1311 -> 407 us, inverse 336 -> 205 us, the whole call 1640 -> 620 us.
 #include "delta_walk.cuh"
 
 namespace pgb {
 
 constexpr float TD_LOG2E = 1.4426950408889634f;
 
-// decay statistics of one 64-token chunk by warps 0 and 1 (tid < 64): L (inclusive cumulative log-decay), e^L,
-// w = e^{L_C - L} (0 past T) and beta (0 past T)
-__device__ __forceinline__ void chunk_stats(const float *la, const float *beta, int t0, int T, int tid, int lane, int warp,
-                                            float *Ls, float *eLs, float *wts, float *bes) {
+// decay statistics of one 64-token chunk by warps 0 and 1 (tid < 64): L (inclusive cumulative log-decay) and beta (0 past T)
+__device__ __forceinline__ void chunk_stats(const float *la, const float *beta, int t0, int T, int tid, int lane, int warp, float *Ls, float *bes) {
     const int t = t0 + tid, tx = t0 + (tid ^ 32);
     const float own = t < T ? la[t] : 0.f, other = tx < T ? la[tx] : 0.f;
     float sc = own;
@@ -33,34 +31,57 @@ __device__ __forceinline__ void chunk_stats(const float *la, const float *beta, 
         const float n = __shfl_up_sync(0xffffffffu, sc, o);
         if (lane >= o) sc += n;
     }
-    const float sum_other = warp_sum(other), sum_own = __shfl_sync(0xffffffffu, sc, 31);
-    const float L = sc + (warp == 1 ? sum_other : 0.f), Ltot = sum_own + sum_other;
-    Ls[tid] = L;
-    if (eLs != nullptr) eLs[tid] = expf(L);
-    if (wts != nullptr) wts[tid] = t < T ? expf(fminf(Ltot - L, 0.f)) : 0.f;
+    const float sum_other = warp_sum(other);
+    Ls[tid] = sc + (warp == 1 ? sum_other : 0.f);
     bes[tid] = t < T ? beta[t] : 0.f;
 }
 
 // ------------------------------------------------------------------------------------------------ X = (I + N)^-1
+// One column of X per thread is a chain of 2016 dependent multiply-adds on half the threads. The blocked form keeps the chain to 16 steps: the four 16 x 16 diagonal blocks are inverted side by side (a warp each, a lane per
+// column), then twice X21 = -X22 (N21 X11) joins neighbouring blocks, 16 and 32 wide, as register-tiled fp32 products of
+// 128 threads reading 16 bytes at a time. Bound by shared-memory bandwidth and latency; five CTAs share an SM.
 template <int D>
 struct InvSmem {
-    static constexpr int off_k = 0;                                   // K tile, TC_C x D bf16
-    static constexpr int NP = 68;                                     // row pitch of N in floats (16-byte aligned, spreads banks)
-    static constexpr int off_n = TC_C * D * 2;                        // N fp32 [64][NP]
-    static constexpr int off_x = off_n + TC_C * NP * 4;               // X head, X tail: [64][64] bf16 each
-    static constexpr int off_misc = off_x + 2 * TC_C * TC_C * 2;
+    static constexpr int NP = 68, TP = 36;                            // row pitches of N / X and of the product T, in floats (16-byte aligned)
+    static constexpr int XB = TC_C * NP * 4;
+    static constexpr int off_k = 0;                                   // K tile, TC_C x D bf16; then X fp32 [64][NP] in its place
+    static constexpr int off_n = XB > TC_C * D * 2 ? (XB + 1023) / 1024 * 1024 : TC_C * D * 2;
+    static constexpr int off_t = off_n + XB;                          // T fp32 [32][TP]
+    static constexpr int off_misc = off_t + 32 * TP * 4;
     static constexpr int bytes = off_misc + 1024 + 1024;
 };
+
+// rows r0, r0 + 1 and columns c0..c0+3 of P = A B for K-long rows of A (pitch pa) and rows of B (pitch pb); K a multiple of 4
+template <int K>
+__device__ __forceinline__ void inv_product(float (&acc)[2][4], const float *A, int pa, const float *B, int pb, int r0, int c0) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
+#pragma unroll
+    for (int k = 0; k < K; k += 4) {
+        const float4 a0 = *reinterpret_cast<const float4 *>(A + r0 * pa + k), a1 = *reinterpret_cast<const float4 *>(A + (r0 + 1) * pa + k);
+        const float f0[4] = {a0.x, a0.y, a0.z, a0.w}, f1[4] = {a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 b = *reinterpret_cast<const float4 *>(B + (k + i) * pb + c0);
+            const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) { acc[0][c] = fmaf(f0[i], bv[c], acc[0][c]); acc[1][c] = fmaf(f1[i], bv[c], acc[1][c]); }
+        }
+    }
+}
 
 template <int D>
 __global__ void __launch_bounds__(128) delta_inv_kernel(const __grid_constant__ CUtensorMap mk, const float *__restrict__ la_all,
                                                         const float *__restrict__ beta_all, __nv_bfloat16 *__restrict__ X, int T,
                                                         int with_tail) {
     using SM = InvSmem<D>;
+    constexpr int NP = SM::NP, TP = SM::TP;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *sm = smem_raw + (base - smem_u32(smem_raw));
-    float *Nf = reinterpret_cast<float *>(sm + SM::off_n);
+    float *Nf = reinterpret_cast<float *>(sm + SM::off_n), *Xf = reinterpret_cast<float *>(sm + SM::off_k), *Tf = reinterpret_cast<float *>(sm + SM::off_t);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + SM::off_misc + 32);
     float *Ls = reinterpret_cast<float *>(sm + SM::off_misc + 64), *bes = Ls + 64;
     const uint32_t bar_k = base + SM::off_misc, bar_m = bar_k + 8;
@@ -75,76 +96,119 @@ __global__ void __launch_bounds__(128) delta_inv_kernel(const __grid_constant__ 
 #pragma unroll
         for (int s = 0; s < D / 64; ++s) tma_load_3d(base + SM::off_k + s * 8192, &mk, bar_k, 64 * s, t0, bh);
     }
-    if (warp == 0) tmem_alloc(smem_u32(tmem_slot), 64);
-    if (warp < 2) chunk_stats(la_all + (size_t)bh * T, beta_all + (size_t)bh * T, t0, T, tid, lane, warp, Ls, nullptr, nullptr, bes);
+    if (warp == 3) tmem_alloc(smem_u32(tmem_slot), 64);
+    if (warp < 2) chunk_stats(la_all + (size_t)bh * T, beta_all + (size_t)bh * T, t0, T, tid, lane, warp, Ls, bes);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = warp_uniform(*tmem_slot);
-    bool ok = mbar_wait(bar_k, 0, 11);
-    if (tid == 0 && ok) {
+    bool ok = mbar_wait_warp(bar_k, 0, 11);
+    if (warp == 2 && ok) {
         constexpr uint32_t I_KK = idesc_bf16(64, 64, 0, 0);
         const uint64_t dk = smem_desc(base + SM::off_k, 16, 1024);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
             const uint32_t ko = ((uint32_t)(k >> 2) * 8192u + (uint32_t)(k & 3) * 32u) >> 4;
-            mma_bf16(tmem, dk + ko, dk + ko, I_KK, k > 0);
+            mma_bf16_elect(tmem, dk + ko, dk + ko, I_KK, k > 0);
         }
-        mma_commit(bar_m);
+        mma_commit_elect(bar_m);
     }
-    if (ok && !mbar_wait(bar_m, 0, 12)) ok = false;
+    if (ok) ok = mbar_wait_warp(bar_m, 0, 12);
     tc_fence_after();
     // ---- N = beta_t (k_t . k_s) exp(min(L_t - L_s, 0)) for s < t, else 0.   Each warp: its 16 rows, all 64 columns.
     {
         const int fr = lane >> 2, fq = lane & 3, r0 = 16 * warp + fr, r1 = r0 + 8;
         float kk[32];
         tmem_ld_frag8(tmem + ((uint32_t)(32 * warp) << 16), kk);
-        tmem_ld_wait();
         const float L0 = Ls[r0] * TD_LOG2E, L1 = Ls[r1] * TD_LOG2E, b0 = bes[r0], b1 = bes[r1];
+        tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int s = 8 * j + 2 * fq + e;
-                const float Lsv = Ls[s] * TD_LOG2E;
-                Nf[r0 * SM::NP + s] = (s < r0) ? b0 * kk[4 * j + e] * exp2f(fminf(L0 - Lsv, 0.f)) : 0.f;
-                Nf[r1 * SM::NP + s] = (s < r1) ? b1 * kk[4 * j + 2 + e] * exp2f(fminf(L1 - Lsv, 0.f)) : 0.f;
-            }
+        for (int j = 0; j < 8; ++j) {
+            const int s = 8 * j + 2 * fq;
+            const float2 Lp = *reinterpret_cast<const float2 *>(Ls + s);
+            const float La = Lp.x * TD_LOG2E, Lb = Lp.y * TD_LOG2E;
+            float2 n0, n1;
+            n0.x = (s < r0) ? b0 * kk[4 * j] * fast_exp2(fminf(L0 - La, 0.f)) : 0.f;
+            n0.y = (s + 1 < r0) ? b0 * kk[4 * j + 1] * fast_exp2(fminf(L0 - Lb, 0.f)) : 0.f;
+            n1.x = (s < r1) ? b1 * kk[4 * j + 2] * fast_exp2(fminf(L1 - La, 0.f)) : 0.f;
+            n1.y = (s + 1 < r1) ? b1 * kk[4 * j + 3] * fast_exp2(fminf(L1 - Lb, 0.f)) : 0.f;
+            *reinterpret_cast<float2 *>(Nf + r0 * NP + s) = n0;
+            *reinterpret_cast<float2 *>(Nf + r1 * NP + s) = n1;
+        }
     }
     tc_fence_before();
-    __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, 64);
-    // ---- column j of X: x_t = [t == j] - sum_{s<t} N[t][s] x_s   (x_s = 0 above the diagonal, so one code path for all j)
-    __nv_bfloat16 *Xh = reinterpret_cast<__nv_bfloat16 *>(sm + SM::off_x), *Xl = Xh + TC_C * TC_C;
-    if (tid < TC_C) {
-        float x[TC_C];
+    __syncthreads();                                                  // K is consumed (the product is complete): X takes its place
+    if (warp == 3) tmem_dealloc(tmem, 64);
+    // ---- diagonal blocks: lane j < 16 of warp b owns column j of block b;  x_t = [t == j] - sum_{s<t} N[t][s] x_s
+    if (lane < 16) {
+        const float *Nb = Nf + 16 * warp * (NP + 1);
+        float *Xb = Xf + 16 * warp * (NP + 1);
+        float x[16];
 #pragma unroll
-        for (int t = 0; t < TC_C; ++t) {
-            float acc0 = (t == tid) ? 1.f : 0.f, acc1 = 0.f;
-            const float4 *row = reinterpret_cast<const float4 *>(Nf + t * SM::NP);
+        for (int t = 0; t < 16; ++t) {
+            float a0 = t == lane ? 1.f : 0.f, a1 = 0.f;
 #pragma unroll
             for (int s4 = 0; s4 < (t + 3) / 4; ++s4) {
-                const float4 n = row[s4];                             // the same address for every thread: a broadcast
-                if (4 * s4 + 0 < t) acc0 = fmaf(-n.x, x[4 * s4 + 0], acc0);
-                if (4 * s4 + 1 < t) acc1 = fmaf(-n.y, x[4 * s4 + 1], acc1);
-                if (4 * s4 + 2 < t) acc0 = fmaf(-n.z, x[4 * s4 + 2], acc0);
-                if (4 * s4 + 3 < t) acc1 = fmaf(-n.w, x[4 * s4 + 3], acc1);
+                const float4 n = *reinterpret_cast<const float4 *>(Nb + t * NP + 4 * s4);   // the same address for every lane: a broadcast
+                if (4 * s4 + 0 < t) a0 = fmaf(-n.x, x[4 * s4 + 0], a0);
+                if (4 * s4 + 1 < t) a1 = fmaf(-n.y, x[4 * s4 + 1], a1);
+                if (4 * s4 + 2 < t) a0 = fmaf(-n.z, x[4 * s4 + 2], a0);
+                if (4 * s4 + 3 < t) a1 = fmaf(-n.w, x[4 * s4 + 3], a1);
             }
-            x[t] = acc0 + acc1;
-            __nv_bfloat16 hi, lo;
-            split_bf16(x[t], hi, lo);
-            Xh[t * 64 + tid] = hi;
-            Xl[t * 64 + tid] = lo;
+            x[t] = a0 + a1;
+            Xb[t * NP + lane] = x[t];
         }
+    }
+    __syncthreads();
+    // ---- join 16 x 16 blocks, a pair of blocks per pair of warps: the first warp's lanes cover the new block as two rows by four
+    //      columns each
+    float acc[2][4];
+    {
+        const int g = 32 * (warp >> 1), r = 2 * (lane >> 2), cc = 4 * (lane & 3);   // the pair's first row; only its first warp works
+        const bool mine = (warp & 1) == 0;
+        float *Tb = Tf + (warp >> 1) * 16 * TP;
+        if (mine) {
+            inv_product<16>(acc, Nf + (g + 16) * NP + g, NP, Xf + g * NP + g, NP, r, cc);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Tb + (r + i) * TP + cc) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+            __syncwarp();
+            inv_product<16>(acc, Xf + (g + 16) * NP + g + 16, NP, Tb, TP, r, cc);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                *reinterpret_cast<float4 *>(Xf + (g + 16 + r + i) * NP + g + cc) = make_float4(-acc[i][0], -acc[i][1], -acc[i][2], -acc[i][3]);
+        } else {                                                      // its second warp zeroes the block above the diagonal
+#pragma unroll
+            for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Xf + (g + r + i) * NP + g + 16 + cc) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    __syncthreads();
+    // ---- join the 32 x 32 blocks: 128 threads, two rows by four columns each
+    {
+        const int r = 2 * (tid >> 3), cc = 4 * (tid & 7);
+        inv_product<32>(acc, Nf + 32 * NP, NP, Xf, NP, r, cc);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Tf + (r + i) * TP + cc) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        __syncthreads();
+        inv_product<32>(acc, Xf + 32 * NP + 32, NP, Tf, TP, r, cc);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Xf + (32 + r + i) * NP + cc) = make_float4(-acc[i][0], -acc[i][1], -acc[i][2], -acc[i][3]);
     }
     __syncthreads();
     // ---- head then tail, 8 KB each, to the scratch buffer; or the head alone, densely packed (the stand-alone operator)
     {
         uint4 *dst = reinterpret_cast<uint4 *>(X + ((size_t)bh * NC + c) * ((with_tail ? 2 : 1) * TC_C * TC_C));
-        const uint4 *src = reinterpret_cast<const uint4 *>(Xh);
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (with_tail || i < 4) dst[tid + 128 * i] = src[tid + 128 * i];
+        for (int i = 0; i < 4; ++i) {
+            const int idx = tid + 128 * i, row = idx >> 3, col = 8 * (idx & 7);
+            uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
+            if (col < (row < 32 ? 32 : 64)) {                         // the block above the diagonal is never written: zero
+                const float4 a = *reinterpret_cast<const float4 *>(Xf + row * NP + col), b = *reinterpret_cast<const float4 *>(Xf + row * NP + col + 4);
+                const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                split8(x, hi, lo);
+            }
+            dst[idx] = hi;
+            if (with_tail) dst[512 + idx] = lo;
+        }
     }
 }
 
