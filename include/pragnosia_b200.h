@@ -277,6 +277,28 @@ int pgb_aspin_layer_prefill_fwd(const void *qp, const void *kp, const void *vp, 
                                 void *o, int o_dtype, float *S_out, void *sent, int B, int H, int T, int D,
                                 void *stream);
 
+/* -------------------------------------------------------------------------------------------------------
+ * A whole sequence through the layer between its two GEMMs, window by window with the state carried (positions restart at
+ * every window, the entering state is rotated back by the previous window's length), in one call: what a loop of
+ * pgb_aspin_layer_prefill_fwd (plain rule) or of prep / delta prefill / norm (delta rule) over the windows computes.
+ * bf16 (B,T,H*D) projection views (strides multiples of 8); o bf16 (B,T,H*D); S_out fp32 [B][H][D][D], the final state.
+ * window: a multiple of 64; plain rule: head dim 64, window <= 1024, rot_T >= the longest window in whole chunks.
+ * pos (delta rule): int64 [T], the position of every token inside its window. Scratch from the _scratch_bytes calls (plain
+ * rule: none needed when T <= window).
+ * ------------------------------------------------------------------------------------------------------- */
+long long pgb_aspin_layer_windows_scratch_bytes(int B, int H, int T, int window);
+int pgb_aspin_layer_prefill_windows_fwd(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
+                                        const void *gate_logits, const void *decay_logits, long long aux_stride_b, long long aux_stride_t,
+                                        const float *decay_A, const float *rot_table, int rot_T, const float *theta, const float *rms_weight,
+                                        float rms_eps, void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H,
+                                        int T, int D, void *stream);
+long long pgb_aspin_delta_layer_scratch_bytes(int B, int H, int T, int D);
+int pgb_aspin_delta_layer_windows_fwd(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
+                                      const void *decay_logits, const void *beta_logits, long long aux_stride_b, long long aux_stride_t,
+                                      const float *decay_A, const float *theta, const long long *pos, const float *rms_weight, float rms_eps,
+                                      void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H, int T, int D,
+                                      void *stream);
+
 /* table[h][t][i] = (cos, sin)(t * theta[h][i]), t in [0,T): the rotation phases of one layer (src/assoc.py:34-39 with
  * positions 0..T-1), built once per layer and reused by every pgb_aspin_layer_prefill_fwd call.
  *   theta [H][D/2] fp32;  table [H][T][D/2][2] fp32. */

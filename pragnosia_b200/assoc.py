@@ -183,6 +183,28 @@ class AssocCarrier(nn.Module):
             p_new = T
         return delta, ((S, p_new, cc) if sconv is not None else (S, p_new))
 
+    def windows_fit(self, window: int) -> bool:
+        """Whether mix_windows takes this layer: bf16 weights, no option that changes the step, whole chunks a window."""
+        return (self.plain_step and self.pos_wrap is None and not self.need_sent and self.q.weight.dtype == torch.bfloat16 and window % 64 == 0
+                and (self.delta or (self.dk == 64 and window <= 1024)))
+
+    def mix_windows(self, z, window: int, pos, tail: int, S_out=None):
+        """mix over a sequence of windows with the state carried, as one call per layer: z (B,T,d), pos (T,) the tokens'
+        positions inside their windows. Returns (what is added to the last `tail` tokens of x, final state): the GEMM
+        behind the scan runs for those tokens only."""
+        B, T, d = z.shape
+        H, dk = self.h, self.dk
+        c = self._consts()
+        y = F.linear(z, c["W"], c["b"])
+        qp, kp, vp = (y[..., i * d:(i + 1) * d].unflatten(-1, (H, dk)) for i in range(3))
+        a_logit, g_logit = y[..., 3 * d:3 * d + H], y[..., 3 * d + H:3 * d + 2 * H]
+        if self.delta:
+            o, S = ops.delta_layer_windows(qp, kp, vp, a_logit, g_logit, c["A"], c["theta"], pos, window, c["onw"], self._rms_eps(), S_out)
+        else:
+            o, S = ops.layer_prefill_windows(qp, kp, vp, g_logit, a_logit, c["A"], self._rot_table(min(T, window), c), c["theta"], window,
+                                             c["onw"], self._rms_eps(), S_out)
+        return F.linear(o if tail == T else o[:, T - tail:], c["ow"]), S
+
     def _mix_train(self, z, h0):
         """The layer with a gradient wanted (the reference's training path, src/assoc.py:384-512 with its kernels on):
         separate projections of the live parameters, the differentiable prep / scan operators (their backward kernels are

@@ -56,6 +56,12 @@ long long prefill_tc_delta_static_capacity();
 size_t train_bwd_scratch_bytes(int B, int H, int T, int D, bool delta);
 int train_bwd_launch(const TrainBwdArgs &, int, cudaStream_t);
 int tc_train_error_flag(int *);
+int prep_gates_launch(const void *, const void *, const void *, long long, long long, long long, const void *, const void *, long long, long long,
+                      const float *, const float *, const long long *, void *, void *, void *, float *, float *, int, int, int, int, cudaStream_t);
+int head_norm_launch(const void *, const float *, float, void *, int, int, int, int, cudaStream_t);
+size_t segment_scratch_bytes(int B, int H, int T, int seg_len);
+int segment_states_launch(const PrefillArgs &, float *, cudaStream_t);
+int tc_segment_error_flag(int *);
 int rot_table_launch(const float *, float *, int, int, int, cudaStream_t);
 int decode_embed_launch(const long long *, const long long *, const void *, const void *, void *, int, int, int, int, float *, cudaStream_t);
 int decode_sample_launch(const void *, int, float, float, unsigned long long, long long *, long long *, int, long long *, long long *, float *,
@@ -90,6 +96,17 @@ static int tc_dispatch(const PrefillArgs &a, int o_dtype, int D, cudaStream_t st
     if (D == 64 && g_tc_variant == 0) return prefill_tc_ws_launch(a, o_dtype, stream);
     return prefill_tc_launch(a, o_dtype, D, stream);
 }
+
+// one buffer for what lies between the delta layer's two GEMMs: the scan's operands and output, gates, inverses
+struct DeltaLayerScratch {
+    size_t q, k, v, o, la, beta, x, bytes;
+    DeltaLayerScratch(long long B, long long H, long long T, int D) {
+        auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
+        const size_t rows = (size_t)(B * H * T), tile = up(rows * D * 2);
+        q = 0; k = tile; v = 2 * tile; o = 3 * tile; la = 4 * tile; beta = la + up(rows * 4); x = beta + up(rows * 4);
+        bytes = x + prefill_tc_delta_scratch_bytes((int)B, (int)H, (int)T);
+    }
+};
 
 static inline size_t esize(int dt) { return dt == PGB_BF16 ? 2 : 4; }
 static inline bool dtype_ok(int dt) { return dt == PGB_F32 || dt == PGB_BF16; }
@@ -353,6 +370,73 @@ int pgb_aspin_layer_prefill_fwd(const void *qp, const void *kp, const void *vp, 
     return tc_dispatch(a, o_dtype, D, (cudaStream_t)stream);
 }
 
+long long pgb_aspin_layer_windows_scratch_bytes(int B, int H, int T, int window) {
+    if (B <= 0 || H <= 0 || T <= 0 || window <= 0) return 0;
+    return T <= window ? 0 : (long long)segment_scratch_bytes(B, H, T, window);
+}
+
+int pgb_aspin_layer_prefill_windows_fwd(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
+                                        const void *gate_logits, const void *decay_logits, long long aux_stride_b, long long aux_stride_t,
+                                        const float *decay_A, const float *rot_table, int rot_T, const float *theta, const float *rms_weight,
+                                        float rms_eps, void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H,
+                                        int T, int D, void *stream) {
+    if (!qp || !kp || !vp || !decay_logits || !decay_A || !rot_table || !theta || !o || !S_out) return PGB_ERR_NULL_POINTER;
+    if (D != 64) return PGB_ERR_UNSUPPORTED_DIM;
+    if (window < 64 || window % 64 != 0 || window > 1024) return PGB_ERR_BAD_SHAPE;
+    const int longest = T < window ? T : window;
+    if (B <= 0 || H <= 0 || T <= 0 || (long long)B * H > 65535 || aux_stride_b < 0 || aux_stride_t < H || in_stride_t < (long long)H * D ||
+        in_stride_b < 0 || rot_T < (longest + 63) / 64 * 64 || (long long)B * H * ((T + window - 1) / window) > 0x7fffffffLL)
+        return PGB_ERR_BAD_SHAPE;
+    if (T > window && (!scratch || scratch_bytes < pgb_aspin_layer_windows_scratch_bytes(B, H, T, window))) return PGB_ERR_BAD_SHAPE;
+    if (!aligned(qp, 16) || !aligned(kp, 16) || !aligned(vp, 16) || in_stride_b % 8 || in_stride_t % 8 || !aligned(o, 16) || !aligned(S_out, 16) ||
+        !aligned(rot_table, 16) || (scratch && !aligned(scratch, 16)))
+        return PGB_ERR_MISALIGNED;
+    PrefillArgs a{qp, kp, vp, nullptr, nullptr, T > window ? (const float *)scratch : nullptr, o, S_out, nullptr, theta, nullptr, (float)window, B, H, T};
+    a.la_raw = decay_logits; a.la_sb = aux_stride_b; a.la_st = aux_stride_t; a.decay_A = decay_A;
+    a.rms_w = rms_weight; a.rms_eps = rms_eps; a.o_token_major = 1;
+    a.raw = 1; a.raw_sb = in_stride_b; a.raw_st = in_stride_t; a.gate_raw = gate_logits; a.rot = rot_table; a.rot_T = rot_T;
+    a.seg_len = window;
+    if (T > window) {
+        const int rc = segment_states_launch(a, (float *)scratch, (cudaStream_t)stream);
+        if (rc != PGB_OK) return rc;
+    }
+    return prefill_tc_ws_launch(a, PGB_BF16, (cudaStream_t)stream);
+}
+
+int pgb_aspin_delta_layer_windows_fwd(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
+                                      const void *decay_logits, const void *beta_logits, long long aux_stride_b, long long aux_stride_t,
+                                      const float *decay_A, const float *theta, const long long *pos, const float *rms_weight, float rms_eps,
+                                      void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H, int T, int D,
+                                      void *stream) {
+    if (!qp || !kp || !vp || !decay_logits || !beta_logits || !decay_A || !theta || !pos || !rms_weight || !o || !S_out || !scratch)
+        return PGB_ERR_NULL_POINTER;
+    if (D != 64 && D != 128) return PGB_ERR_UNSUPPORTED_DIM;
+    if (B <= 0 || H <= 0 || T <= 0 || aux_stride_b < 0 || aux_stride_t < H || in_stride_t < (long long)H * D || in_stride_b < 0 || window < 64 ||
+        window % 64 != 0)
+        return PGB_ERR_BAD_SHAPE;
+    if ((long long)B * H > 65535 || (T + 63) / 64 > 65535) return PGB_ERR_TOO_LARGE;
+    if (scratch_bytes < pgb_aspin_delta_layer_scratch_bytes(B, H, T, D)) return PGB_ERR_BAD_SHAPE;
+    if (!aligned(qp, 16) || !aligned(kp, 16) || !aligned(vp, 16) || in_stride_b % 8 || in_stride_t % 8 || !aligned(o, 16) || !aligned(S_out, 16) ||
+        !aligned(scratch, 256) || !aligned(theta, 16) || !aligned(rms_weight, 16))
+        return PGB_ERR_MISALIGNED;
+    const DeltaLayerScratch sc(B, H, T, D);
+    uint8_t *buf = (uint8_t *)scratch;
+    void *q = buf + sc.q, *k = buf + sc.k, *v = buf + sc.v, *os = buf + sc.o;
+    float *la = (float *)(buf + sc.la), *beta = (float *)(buf + sc.beta);
+    int rc = prep_gates_launch(qp, kp, vp, in_stride_b, in_stride_t, D, decay_logits, beta_logits, aux_stride_b, aux_stride_t, decay_A, theta, pos, q,
+                               k, v, la, beta, B, T, H, D, (cudaStream_t)stream);
+    if (rc != PGB_OK) return rc;
+    PrefillArgs a{q, k, v, la, beta, nullptr, os, S_out, nullptr, theta, nullptr, 0.f, B, H, T};
+    a.rebase_chunks = window / 64;
+    rc = prefill_tc_delta_launch(a, PGB_BF16, D, buf + sc.x, (cudaStream_t)stream);
+    return rc != PGB_OK ? rc : head_norm_launch(os, rms_weight, rms_eps, o, B, T, H, D, (cudaStream_t)stream);
+}
+
+long long pgb_aspin_delta_layer_scratch_bytes(int B, int H, int T, int D) {
+    if (B <= 0 || H <= 0 || T <= 0 || (D != 64 && D != 128)) return 0;
+    return (long long)DeltaLayerScratch(B, H, T, D).bytes;
+}
+
 int pgb_rot_table_build(const float *theta, float *table, int H, int T, int D, void *stream) {
     if (!theta || !table) return PGB_ERR_NULL_POINTER;
     if (H <= 0 || T <= 0 || D <= 0 || (D & 1)) return PGB_ERR_BAD_SHAPE;
@@ -536,6 +620,8 @@ int pgb_tc_error_flag(int *out_host) {
     if (rc == PGB_OK) rc = batch_linear_error_flag(&f);
     int g = 0;
     if (rc == PGB_OK) rc = tc_train_error_flag(&g);
+    f = f > g ? f : g;
+    if (rc == PGB_OK) rc = tc_segment_error_flag(&g);
     f = f > g ? f : g;
     e = e > f ? e : f;
     b = b > c ? b : c;

@@ -493,7 +493,7 @@ int tc_go(const PrefillArgs &a, int o_dtype, cudaStream_t stream) {
     if (e != cudaSuccess) { set_cuda_error(e, "prefill_tc smem attribute"); return PGB_ERR_CUDA; }
     TcParams p{a.la, a.S0, a.theta, a.shift_dev, a.shift_host, a.o, a.S_out, a.sent, a.H, a.T, o_dtype == PGB_F32,
                (const __nv_bfloat16 *)a.la_raw, a.la_sb, a.la_st, a.decay_A, a.rms_w, a.rms_eps, a.o_token_major,
-               (const __nv_bfloat16 *)a.gate_raw, (const float2 *)a.rot, a.rot_T};
+               (const __nv_bfloat16 *)a.gate_raw, (const float2 *)a.rot, a.rot_T, BH, a.T};
     kern<<<(unsigned)BH, TC_NT, SM::bytes, stream>>>(mq, mk, mv, p);
     return check_launch("prefill_tc_kernel");
 }

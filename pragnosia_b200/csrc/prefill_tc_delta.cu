@@ -37,8 +37,8 @@ __device__ __forceinline__ void chunk_stats(const float *la, const float *beta, 
 }
 
 // ------------------------------------------------------------------------------------------------ X = (I + N)^-1
-// One column of X per thread is a chain of 2016 dependent multiply-adds on half the threads. The blocked form keeps the chain to 16 steps: the four 16 x 16 diagonal blocks are inverted side by side (a warp each, a lane per
-// column), then twice X21 = -X22 (N21 X11) joins neighbouring blocks, 16 and 32 wide, as register-tiled fp32 products of
+// One column of X per thread is a chain of 2016 dependent multiply-adds on half the threads. The blocked form keeps the
+// chain to 16 steps: the four 16 x 16 diagonal blocks are inverted side by side (a warp each, a lane per column), then twice X21 = -X22 (N21 X11) joins neighbouring blocks, 16 and 32 wide, as register-tiled fp32 products of
 // 128 threads reading 16 bytes at a time. Bound by shared-memory bandwidth and latency; five CTAs share an SM.
 template <int D>
 struct InvSmem {
@@ -238,6 +238,7 @@ static int delta_go(const PrefillArgs &a, int o_dtype, void *x_scratch, cudaStre
     DwParams p{};
     p.la = a.la; p.beta = a.beta; p.S0 = a.S0; p.theta = a.theta; p.shift_dev = a.shift_dev; p.shift_host = a.shift_host;
     p.S_out = a.S_out; p.want_sent = a.sent != nullptr; p.want_w = a.W_out != nullptr; p.H = a.H; p.T = a.T; p.o_is_f32 = f32;
+    p.rebase_chunks = a.rebase_chunks; p.rebase_shift = (float)(a.rebase_chunks * TC_C);
     walk<<<(unsigned)BH, DW_NT, DwSmem<D, false>::bytes, stream>>>(m, p);
     return check_launch("delta_walk_kernel");
 }

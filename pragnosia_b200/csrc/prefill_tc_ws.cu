@@ -83,8 +83,11 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
     auto bar_q = [&](int s) { return mb + SM::bar_q + 8 * s; };           // P, U issued: tiles of c final    c&3
 
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5);
-    const int bh = blockIdx.x, h = bh % p.H, b = bh / p.H;
-    const int T = p.T, NC = (T + TC_C - 1) / TC_C;
+    // A chain may be cut into segments of seg_len tokens (whole chunks), each with its own entering state: one CTA a segment.
+    // T, positions and chunks below are the segment's own; tb is its first token.
+    const int seg = blockIdx.x / p.BH, bh = blockIdx.x - seg * p.BH, h = bh % p.H, b = bh / p.H;
+    const int tb = seg * p.seg_len, T = min(p.T - tb, p.seg_len), NC = (T + TC_C - 1) / TC_C;
+    const float *S0 = p.S0 == nullptr || p.seg_len >= p.T ? p.S0 : (seg == 0 ? nullptr : p.S0 + (size_t)(seg - 1) * p.BH * WS_D * WS_D);
     const int tma_c0 = RAW ? h * D : 0, tma_c2 = RAW ? b : bh;
 
     if (tid == 0) {
@@ -210,12 +213,12 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
         float S[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) S[j] = 0.f;
-        if (p.S0 != nullptr) {
+        if (S0 != nullptr) {
             const float shift = p.theta == nullptr ? 0.f : (p.shift_dev != nullptr ? *p.shift_dev : p.shift_host);
 #pragma unroll
             for (int hi8 = 0; hi8 < 2; ++hi8) {
                 const int row = hi8 ? row1 : row0;
-                const float *src = p.S0 + ((size_t)bh * D + row) * D + col0 + 2 * fq;
+                const float *src = S0 + ((size_t)bh * D + row) * D + col0 + 2 * fq;
                 float sn = 0.f, cs = 1.f;
                 if (shift != 0.f) sincosf(-shift * p.theta[(size_t)h * (D / 2) + (row >> 1)], &sn, &cs);
 #pragma unroll
@@ -305,7 +308,7 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
                 publish_state(c + 1);
             }
         }
-        if (ok) {
+        if (ok && tb + T == p.T) {                                    // the chain's last segment
 #pragma unroll
             for (int hi8 = 0; hi8 < 2; ++hi8) {
                 float *dst = p.S_out + ((size_t)bh * D + (hi8 ? row1 : row0)) * D + col0 + 2 * fq;
@@ -362,7 +365,7 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
                 const int trow = hi8 ? row1 : row0;
                 if (t0 + trow < T) {
                     const float sc = hi8 ? sc1 : sc0;
-                    const size_t row = p.o_token_major ? ((size_t)b * T + t0 + trow) * p.H + h : (size_t)bh * T + t0 + trow;
+                    const size_t row = p.o_token_major ? ((size_t)b * p.T + tb + t0 + trow) * p.H + h : (size_t)bh * p.T + tb + t0 + trow;
                     const size_t off = row * D + col0 + 2 * fq;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
@@ -379,16 +382,16 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
     } else if (warp == WS_STATS || warp == WS_STATS + 1) {
         // =========================================================================================== statistics
         // two warps take alternate chunks; lane l owns tokens l and l + 32 of the chunk: two interleaved warp scans
-        const float *la = p.la != nullptr ? p.la + (size_t)bh * T : nullptr;
+        const float *la = p.la != nullptr ? p.la + (size_t)bh * p.T + tb : nullptr;
         const float expA = p.decay_A != nullptr ? expf(p.decay_A[h]) : 1.f;
         auto fetch_decay = [&](int t) -> float {
             if (t >= T) return 0.f;
-            if (p.la_raw != nullptr) return __bfloat162float(p.la_raw[(size_t)b * p.aux_sb + (size_t)t * p.aux_st + h]);
+            if (p.la_raw != nullptr) return __bfloat162float(p.la_raw[(size_t)b * p.aux_sb + (size_t)(tb + t) * p.aux_st + h]);
             return la[t];
         };
         auto fetch_gate = [&](int t) -> float {
             if (!RAW || p.gate_raw == nullptr || t >= T) return 0.f;
-            return __bfloat162float(p.gate_raw[(size_t)b * p.aux_sb + (size_t)t * p.aux_st + h]);
+            return __bfloat162float(p.gate_raw[(size_t)b * p.aux_sb + (size_t)(tb + t) * p.aux_st + h]);
         };
         const int first = warp - WS_STATS;
         float nx_lo = fetch_decay(first * TC_C + lane), nx_hi = fetch_decay(first * TC_C + lane + 32);
@@ -431,9 +434,9 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
             const int s3 = c % 3;
             const uint32_t sb = base + SM::off_stage + s3 * STAGE_BYTES;
             mbar_expect_tx(bar_full(s3), STAGE_BYTES);
-            tma_load_3d(sb, &mq, bar_full(s3), tma_c0, c * TC_C, tma_c2);
-            tma_load_3d(sb + SM::TILE, &mk, bar_full(s3), tma_c0, c * TC_C, tma_c2);
-            tma_load_3d(sb + 2 * SM::TILE, &mv, bar_full(s3), tma_c0, c * TC_C, tma_c2);
+            tma_load_3d(sb, &mq, bar_full(s3), tma_c0, tb + c * TC_C, tma_c2);
+            tma_load_3d(sb + SM::TILE, &mk, bar_full(s3), tma_c0, tb + c * TC_C, tma_c2);
+            tma_load_3d(sb + 2 * SM::TILE, &mv, bar_full(s3), tma_c0, tb + c * TC_C, tma_c2);
         };
         auto load_rot = [&](int c) {
             if (!RAW) return;
@@ -534,18 +537,19 @@ int prefill_tc_ws_launch(const PrefillArgs &a, int o_dtype, cudaStream_t stream)
         made = tc_make_map(&mq, a.q, BH, a.T, D, D, (long long)a.T * D) && tc_make_map(&mk, a.k, BH, a.T, D, D, (long long)a.T * D) &&
                tc_make_map(&mv, a.v, BH, a.T, D, D, (long long)a.T * D);
     if (!made) { set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled"); return PGB_ERR_CUDA; }
+    const int seg_len = a.seg_len > 0 ? a.seg_len : (a.T + TC_C - 1) / TC_C * TC_C, nseg = (a.T + seg_len - 1) / seg_len;
     TcParams p{a.la, a.S0, a.theta, a.shift_dev, a.shift_host, a.o, a.S_out, a.sent, a.H, a.T, o_dtype == PGB_F32,
                (const __nv_bfloat16 *)a.la_raw, a.la_sb, a.la_st, a.decay_A, a.rms_w, a.rms_eps, a.o_token_major,
-               (const __nv_bfloat16 *)a.gate_raw, (const float2 *)a.rot, a.rot_T};
+               (const __nv_bfloat16 *)a.gate_raw, (const float2 *)a.rot, a.rot_T, BH, seg_len};
     cudaError_t e;
     if (a.raw) {
         e = cudaFuncSetAttribute(prefill_tc_ws_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, WsSmem::bytes);
         if (e != cudaSuccess) { set_cuda_error(e, "prefill_tc_ws smem attribute"); return PGB_ERR_CUDA; }
-        e = pdl_launch(prefill_tc_ws_kernel<true>, dim3((unsigned)BH), dim3(WS_NT), (size_t)WsSmem::bytes, stream, mq, mk, mv, p);
+        e = pdl_launch(prefill_tc_ws_kernel<true>, dim3((unsigned)(BH * nseg)), dim3(WS_NT), (size_t)WsSmem::bytes, stream, mq, mk, mv, p);
     } else {
         e = cudaFuncSetAttribute(prefill_tc_ws_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, WsSmem::bytes);
         if (e != cudaSuccess) { set_cuda_error(e, "prefill_tc_ws smem attribute"); return PGB_ERR_CUDA; }
-        e = pdl_launch(prefill_tc_ws_kernel<false>, dim3((unsigned)BH), dim3(WS_NT), (size_t)WsSmem::bytes, stream, mq, mk, mv, p);
+        e = pdl_launch(prefill_tc_ws_kernel<false>, dim3((unsigned)(BH * nseg)), dim3(WS_NT), (size_t)WsSmem::bytes, stream, mq, mk, mv, p);
     }
     if (e != cudaSuccess) { set_cuda_error(e, "prefill_tc_ws launch"); return PGB_ERR_CUDA; }
     return check_launch("prefill_tc_ws_kernel");

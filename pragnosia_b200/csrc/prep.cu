@@ -83,6 +83,116 @@ prep_kernel(const TIN *__restrict__ qp, const TIN *__restrict__ kp, const TIN *_
     st_row<TOUT, PER>(v + out_off, ov);
 }
 
+// The same for bf16 in and out with 16-byte aligned rows: D/8 lanes share a row (a lane owns 8 channels, whole pairs), so a
+// warp takes four rows (D = 64) or two at once -- three shuffles a norm instead of five, 16-byte accesses, and a quarter of
+// the instructions per row. With the gates' logits it also writes the scan's log-decay and write strength,
+// la = -softplus(decay logit) e^{A_h}, beta = sigmoid(beta logit), as fp32 [B][H][T].
+// Bound by instruction issue (sincosf per pair) before HBM. 90112 rows of 64: 35 -> 14 us.
+struct PrepGates { const __nv_bfloat16 *decay, *beta; const float *A; float *la_out, *beta_out; };
+
+template <int D>
+__global__ void __launch_bounds__(PREP_WARPS * 32)
+prep8_kernel(const __nv_bfloat16 *__restrict__ qp, const __nv_bfloat16 *__restrict__ kp, const __nv_bfloat16 *__restrict__ vp, long long sb, long long st,
+             long long sh, const __nv_bfloat16 *__restrict__ gate, long long gsb, long long gst, const float *__restrict__ theta,
+             const long long *__restrict__ pos, __nv_bfloat16 *__restrict__ q, __nv_bfloat16 *__restrict__ k, __nv_bfloat16 *__restrict__ v,
+             PrepGates ga, int B, int T, int H) {
+    constexpr int LPR = D / 8, RPC = PREP_WARPS * 32 / LPR;           // lanes a row, rows a CTA
+    const int li = threadIdx.x % LPR, t = blockIdx.x * RPC + threadIdx.x / LPR, bh = blockIdx.y, b = bh / H, h = bh % H;
+    if (t >= T) return;                                               // the shuffles below stay inside a row's lanes
+    const unsigned mask = (LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1u)) << ((threadIdx.x & 31) / LPR * LPR);
+    const size_t in = (size_t)b * sb + (size_t)t * st + (size_t)h * sh + 8 * li, out = ((size_t)bh * T + t) * D + 8 * li;
+    const uint4 raw[3] = {*reinterpret_cast<const uint4 *>(qp + in), *reinterpret_cast<const uint4 *>(kp + in), *reinterpret_cast<const uint4 *>(vp + in)};
+    const float p = (float)pos[t];
+    const float4 th = *reinterpret_cast<const float4 *>(theta + (size_t)h * (D / 2) + 4 * li);
+    const float ang[4] = {th.x, th.y, th.z, th.w};
+    const size_t gi = (size_t)b * gsb + (size_t)t * gst + h;
+    float cs[4], sn[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sincosf(p * ang[i], &sn[i], &cs[i]);
+    uint4 o[3];
+#pragma unroll
+    for (int w = 0; w < 3; ++w) {
+        const __nv_bfloat162 *x2 = reinterpret_cast<const __nv_bfloat162 *>(&raw[w]);
+        __nv_bfloat162 *o2 = reinterpret_cast<__nv_bfloat162 *>(&o[w]);
+        float2 x[4];
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { x[i] = __bfloat1622float2(x2[i]); ss += x[i].x * x[i].x + x[i].y * x[i].y; }
+#pragma unroll
+        for (int m = 1; m < LPR; m <<= 1) ss += __shfl_xor_sync(mask, ss, m);
+        float inv = 1.0f / fmaxf(sqrtf(ss), 1e-12f);
+        if (w == 1 && gate != nullptr) inv *= sigmoidf_(__bfloat162float(gate[gi]));
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            o2[i] = w < 2 ? __floats2bfloat162_rn((x[i].x * cs[i] - x[i].y * sn[i]) * inv, (x[i].x * sn[i] + x[i].y * cs[i]) * inv)
+                          : __floats2bfloat162_rn(x[i].x * inv, x[i].y * inv);
+    }
+    *reinterpret_cast<uint4 *>(q + out) = o[0];
+    *reinterpret_cast<uint4 *>(k + out) = o[1];
+    *reinterpret_cast<uint4 *>(v + out) = o[2];
+    if (li == 0 && ga.la_out != nullptr) ga.la_out[(size_t)bh * T + t] = -softplusf_(__bfloat162float(ga.decay[gi])) * expf(ga.A[h]);
+    if (li == 1 && ga.beta_out != nullptr) ga.beta_out[(size_t)bh * T + t] = sigmoidf_(__bfloat162float(ga.beta[gi]));
+}
+
+static bool prep8_fits(const void *qp, const void *kp, const void *vp, long long sb, long long st, long long sh, const void *q, const void *k,
+                       const void *v, const float *theta, long long BH) {
+    return aligned(qp, 16) && aligned(kp, 16) && aligned(vp, 16) && aligned(q, 16) && aligned(k, 16) && aligned(v, 16) && aligned(theta, 16) &&
+           sb % 8 == 0 && st % 8 == 0 && sh % 8 == 0 && BH <= 65535;
+}
+static int prep8_go(const void *qp, const void *kp, const void *vp, long long sb, long long st, long long sh, const void *gate, long long gsb,
+                    long long gst, const float *theta, const long long *pos, void *q, void *k, void *v, const PrepGates &ga, int B, int T, int H,
+                    int D, cudaStream_t stream) {
+    typedef const __nv_bfloat16 *In;
+    typedef __nv_bfloat16 *Out;
+    const int rpc = PREP_WARPS * 32 / (D / 8);
+    const dim3 grid((unsigned)((T + rpc - 1) / rpc), (unsigned)(B * H));
+    auto go = [&](auto kern) {
+        kern<<<grid, PREP_WARPS * 32, 0, stream>>>((In)qp, (In)kp, (In)vp, sb, st, sh, (In)gate, gsb, gst, theta, pos, (Out)q, (Out)k, (Out)v, ga, B, T, H);
+    };
+    if (D == 64) go(prep8_kernel<64>); else go(prep8_kernel<128>);
+    return check_launch("prep8_kernel");
+}
+
+// plumbing and gates of the delta layer in one pass (bf16, 16-byte aligned rows; the caller has checked)
+int prep_gates_launch(const void *qp, const void *kp, const void *vp, long long sb, long long st, long long sh, const void *decay, const void *beta,
+                      long long gsb, long long gst, const float *A, const float *theta, const long long *pos, void *q, void *k, void *v, float *la_out,
+                      float *beta_out, int B, int T, int H, int D, cudaStream_t stream) {
+    const PrepGates ga{(const __nv_bfloat16 *)decay, (const __nv_bfloat16 *)beta, A, la_out, beta_out};
+    return prep8_go(qp, kp, vp, sb, st, sh, nullptr, gsb, gst, theta, pos, q, k, v, ga, B, T, H, D, stream);
+}
+
+// ---- per-head RMS norm of the scan's output and its transposition: o (B,H,T,D) bf16 -> (B,T,H*D) bf16, D/8 lanes a row
+template <int D>
+__global__ void __launch_bounds__(256) head_norm_kernel(const __nv_bfloat16 *__restrict__ o, const float *__restrict__ w, float eps,
+                                                        __nv_bfloat16 *__restrict__ out, int T, int H) {
+    constexpr int LPR = D / 8, RPC = 256 / LPR;
+    const int li = threadIdx.x % LPR, t = blockIdx.x * RPC + threadIdx.x / LPR, bh = blockIdx.y, b = bh / H, h = bh % H;
+    if (t >= T) return;
+    const unsigned mask = ((1u << LPR) - 1u) << ((threadIdx.x & 31) / LPR * LPR);
+    const uint4 raw = *reinterpret_cast<const uint4 *>(o + ((size_t)bh * T + t) * D + 8 * li);
+    const __nv_bfloat162 *x2 = reinterpret_cast<const __nv_bfloat162 *>(&raw);
+    float2 x[4];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { x[i] = __bfloat1622float2(x2[i]); ss += x[i].x * x[i].x + x[i].y * x[i].y; }
+#pragma unroll
+    for (int m = 1; m < LPR; m <<= 1) ss += __shfl_xor_sync(mask, ss, m);
+    const float r = rsqrtf(ss * (1.0f / D) + eps);
+    const float4 w0 = *reinterpret_cast<const float4 *>(w + 8 * li), w1 = *reinterpret_cast<const float4 *>(w + 8 * li + 4);
+    uint4 res;
+    __nv_bfloat162 *o2 = reinterpret_cast<__nv_bfloat162 *>(&res);
+    o2[0] = __floats2bfloat162_rn(x[0].x * r * w0.x, x[0].y * r * w0.y); o2[1] = __floats2bfloat162_rn(x[1].x * r * w0.z, x[1].y * r * w0.w);
+    o2[2] = __floats2bfloat162_rn(x[2].x * r * w1.x, x[2].y * r * w1.y); o2[3] = __floats2bfloat162_rn(x[3].x * r * w1.z, x[3].y * r * w1.w);
+    *reinterpret_cast<uint4 *>(out + (((size_t)b * T + t) * H + h) * D + 8 * li) = res;
+}
+int head_norm_launch(const void *o, const float *w, float eps, void *out, int B, int T, int H, int D, cudaStream_t stream) {
+    const int rpc = 256 / (D / 8);
+    const dim3 grid((unsigned)((T + rpc - 1) / rpc), (unsigned)(B * H));
+    if (D == 64) head_norm_kernel<64><<<grid, 256, 0, stream>>>((const __nv_bfloat16 *)o, w, eps, (__nv_bfloat16 *)out, T, H);
+    else head_norm_kernel<128><<<grid, 256, 0, stream>>>((const __nv_bfloat16 *)o, w, eps, (__nv_bfloat16 *)out, T, H);
+    return check_launch("head_norm_kernel");
+}
+
 template <typename TIN, typename TOUT>
 static int prep_dispatch(const void *qp, const void *kp, const void *vp, long long sb, long long st, long long sh,
                          const void *gate, long long gsb, long long gst, const float *theta, const long long *pos,
@@ -108,6 +218,8 @@ int prep_launch(const void *qp, const void *kp, const void *vp, int in_dtype, lo
         return prep_dispatch<float, __nv_bfloat16>(qp, kp, vp, sb, st, sh, gate, gsb, gst, theta, pos, q, k, v, B, T, H, D, stream);
     if (in_dtype == PGB_BF16 && out_dtype == PGB_F32)
         return prep_dispatch<__nv_bfloat16, float>(qp, kp, vp, sb, st, sh, gate, gsb, gst, theta, pos, q, k, v, B, T, H, D, stream);
+    if (prep8_fits(qp, kp, vp, sb, st, sh, q, k, v, theta, (long long)B * H))
+        return prep8_go(qp, kp, vp, sb, st, sh, gate, gsb, gst, theta, pos, q, k, v, PrepGates{}, B, T, H, D, stream);
     return prep_dispatch<__nv_bfloat16, __nv_bfloat16>(qp, kp, vp, sb, st, sh, gate, gsb, gst, theta, pos, q, k, v, B, T, H, D, stream);
 }
 

@@ -1,0 +1,246 @@
+// The states entering the windows of a long sequence, for the plain rule on the layer's raw projections (head dim 64), so that
+// the windows of one sequence can run side by side instead of one behind the other (the reference walks them in order,
+// src/model.py:857-863).
+//
+//   segment_state_kernel    a CTA per (window but the last, sequence, head): what the window adds to the state by its end,
+//                               U = sum_s e^{L_end - L_s} k_s v_s^T,
+//                           one long product over the window's tokens. With the decay taken to the window's END (every
+//                           exponent <= 0) nothing in it is sequential: the chunks stream through the plumbing (normalise,
+//                           gate, rotate; the same arithmetic and roundings as the prefill kernel's) and accumulate in
+//                           tensor memory.
+//   segment_combine_kernel  E_{w+1} = e^{L_w} R(-len theta) E_w + U_w over the windows, elementwise, in place of U.
+//
+// prefill_tc_ws_kernel then takes every window as a segment with its own entering state. Bound by the tiles' latency (K and V
+// are read a second time: 16 KB a chunk, three stages ahead of the product); with 12 chains of 8192 tokens the walk of a layer is
+// 12 CTAs of 128 chunks without it and 192 CTAs of 8 with it.
+#include "tc_common.cuh"
+
+namespace pgb {
+
+constexpr int SG_NT = 256, SG_D = 64, SG_ST = 3, SG_MAX = 1024;       // threads; head dim; stages; tokens of a segment at most
+
+struct SgSmem {
+    static constexpr int TILE = 8192, STAGE = 3 * TILE;               // K (then heads of K w), V, tails of K w
+    static constexpr int off_w = SG_ST * STAGE, off_g = off_w + SG_MAX * 4, off_misc = off_g + SG_MAX * 4, bytes = off_misc + 256 + 1024;
+};
+struct SgParams {
+    const __nv_bfloat16 *decay, *gate; long long sb, st;              // logits (gate NULL: write everything), token and batch strides
+    const float *decay_A; const float2 *rot; int rot_T;
+    float *U, *Lend;                                                  // [nseg - 1][BH][D][D], [nseg - 1][BH]
+    int BH, H, seg_len;
+};
+
+__global__ void __launch_bounds__(SG_NT, 2) segment_state_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv,
+                                                                 SgParams p) {
+    using SM = SgSmem;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t *sm = smem_raw + (base - smem_u32(smem_raw));
+    float *ws = reinterpret_cast<float *>(sm + SM::off_w), *gs = reinterpret_cast<float *>(sm + SM::off_g);
+    uint8_t *misc = sm + SM::off_misc;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(misc + 64);
+    float *part = reinterpret_cast<float *>(misc + 96);
+    auto full = [&](int s) { return base + SM::off_misc + 8 * s; };
+    auto done = [&](int s) { return base + SM::off_misc + 24 + 8 * s; };
+    const uint32_t bar_end = base + SM::off_misc + 48;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5), wg = warp >> 2, sub = warp & 3;
+    const int seg = blockIdx.x / p.BH, bh = blockIdx.x - seg * p.BH, h = bh % p.H, b = bh / p.H, tb = seg * p.seg_len, NC = p.seg_len / TC_C;
+    auto load = [&](int c) {
+        const uint32_t sb = base + (c % SG_ST) * SM::STAGE, bar = full(c % SG_ST);
+        mbar_expect_tx(bar, 2 * SM::TILE);
+        tma_load_3d(sb, &mk, bar, h * SG_D, tb + c * TC_C, b);
+        tma_load_3d(sb + SM::TILE, &mv, bar, h * SG_D, tb + c * TC_C, b);
+    };
+    if (tid == 0) {
+        for (int s = 0; s < SG_ST; ++s) { mbar_init(full(s), 1); mbar_init(done(s), 1); }
+        mbar_init(bar_end, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 64);
+    pdl_wait();
+    if (tid == 0)
+        for (int c = 0; c < 2 && c < NC; ++c) load(c);
+    // ---- decay to the end of the segment and key gate of its tokens: a thread owns four consecutive ones
+    {
+        const float expA = expf(p.decay_A[h]);
+        float la[4], g[4], s = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = 4 * tid + i;
+            la[i] = 0.f; g[i] = 1.f;
+            if (t < p.seg_len) {
+                const size_t off = (size_t)b * p.sb + (size_t)(tb + t) * p.st + h;
+                la[i] = -fast_softplus(__bfloat162float(p.decay[off])) * expA;
+                if (p.gate != nullptr) g[i] = fast_sigmoid(__bfloat162float(p.gate[off]));
+            }
+            s += la[i]; la[i] = s;                                    // running sum inside the thread
+        }
+        float sc = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float n = __shfl_up_sync(0xffffffffu, sc, o);
+            if (lane >= o) sc += n;
+        }
+        if (lane == 31) part[warp] = sc;
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        float before = sc - s, total = 0.f;
+#pragma unroll
+        for (int w = 0; w < SG_NT / 32; ++w) { total += part[w]; if (w < warp) before += part[w]; }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (4 * tid + i < p.seg_len) { ws[4 * tid + i] = expf(fminf(total - (before + la[i]), 0.f)); gs[4 * tid + i] = g[i]; }
+        if (tid == 0) p.Lend[(size_t)seg * p.BH + bh] = total;
+        __syncthreads();
+    }
+    const uint32_t tmem = warp_uniform(*tmem_slot);
+    pdl_launch_dependents();
+    bool ok = true;
+    for (int c = 0; c < NC; ++c) {
+        const int st = c % SG_ST;
+        uint8_t *kt = sm + st * SM::STAGE, *vt = kt + SM::TILE, *lt = vt + SM::TILE;
+        ok = mbar_wait_warp(full(st), (c / SG_ST) & 1, 11);
+        if (ok) {
+            const int cp = lane & 7;
+#pragma unroll
+            for (int pass = 0; pass < 2; ++pass) {
+                const int row = 32 * pass + 4 * warp + (lane >> 3), t = c * TC_C + row;
+                const uint32_t off = swz(row, cp);
+                uint4 raw[2] = {*reinterpret_cast<const uint4 *>(kt + off), *reinterpret_cast<const uint4 *>(vt + off)};
+                const float4 *rt = reinterpret_cast<const float4 *>(p.rot + ((size_t)h * p.rot_T + t) * (SG_D / 2) + cp * 4);
+                const float4 r01 = rt[0], r23 = rt[1];
+                const float cs[4] = {r01.x, r01.z, r23.x, r23.z}, sn[4] = {r01.y, r01.w, r23.y, r23.w};
+                const float w = ws[t], g = gs[t];
+                uint4 hi, lo, vo;
+#pragma unroll
+                for (int which = 0; which < 2; ++which) {
+                    const __nv_bfloat162 *b2 = reinterpret_cast<const __nv_bfloat162 *>(&raw[which]);
+                    float x[8], ss = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 f = __bfloat1622float2(b2[i]);
+                        x[2 * i] = f.x; x[2 * i + 1] = f.y;
+                        ss = fmaf(f.x, f.x, fmaf(f.y, f.y, ss));
+                    }
+                    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+                    ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+                    ss += __shfl_xor_sync(0xffffffffu, ss, 4);
+                    const float inv = rsqrtf(fmaxf(ss, 1e-24f)) * (which == 0 ? g : 1.f);
+                    __nv_bfloat162 o2[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        o2[i] = which == 0 ? __floats2bfloat162_rn((x[2 * i] * cs[i] - x[2 * i + 1] * sn[i]) * inv, (x[2 * i] * sn[i] + x[2 * i + 1] * cs[i]) * inv)
+                                           : __floats2bfloat162_rn(x[2 * i] * inv, x[2 * i + 1] * inv);
+                    if (which == 0) {                                 // K w from the ROUNDED k, as the prefill kernel forms it
+                        float kw[8];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(o2[i]); kw[2 * i] = f.x * w; kw[2 * i + 1] = f.y * w; }
+                        split8(kw, hi, lo);
+                    } else vo = *reinterpret_cast<const uint4 *>(o2);
+                }
+                *reinterpret_cast<uint4 *>(kt + off) = hi;
+                *reinterpret_cast<uint4 *>(lt + off) = lo;
+                *reinterpret_cast<uint4 *>(vt + off) = vo;
+            }
+        }
+        fence_proxy_async();
+        ok = __syncthreads_and(ok);
+        if (!ok) break;
+        if (warp == 0) {
+            constexpr uint32_t I_U = idesc_bf16(64, 64, 1, 1);
+            const uint32_t sb = base + st * SM::STAGE;
+            const uint64_t dh = smem_desc(sb, 8192, 1024), dv = smem_desc(sb + SM::TILE, 8192, 1024), dl = smem_desc(sb + 2 * SM::TILE, 8192, 1024);
+            tc_fence_after();
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem, dh + k * 128, dv + k * 128, I_U, (c > 0) | (k > 0));
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem, dl + k * 128, dv + k * 128, I_U, 1);
+            mma_commit_elect(done(st));
+            if (c + 1 == NC) mma_commit_elect(bar_end);
+            if (c + 2 < NC) {                                         // into the stage of chunk c - 1, whose product is an iteration old
+                if (c > 0 && !mbar_wait_warp(done((c - 1) % SG_ST), ((c - 1) / SG_ST) & 1, 12)) ok = false;
+                if (ok && lane == 0) load(c + 2);
+            }
+        }
+    }
+    if (ok) ok = mbar_wait_warp(bar_end, 0, 13);
+    tc_fence_after();
+    if (ok) {
+        const int fr = lane >> 2, fq = lane & 3;
+        float x[16];
+        tmem_ld_frag4(tmem + ((uint32_t)(32 * sub) << 16) + 32 * wg, x);
+        tmem_ld_wait();
+#pragma unroll
+        for (int hi8 = 0; hi8 < 2; ++hi8) {
+            float *dst = p.U + ((size_t)blockIdx.x * SG_D + 16 * sub + fr + 8 * hi8) * SG_D + 32 * wg + 2 * fq;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) *reinterpret_cast<float2 *>(dst + 8 * j) = make_float2(x[4 * j + 2 * hi8], x[4 * j + 2 * hi8 + 1]);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem, 64);
+}
+
+// a thread owns two value columns of one pair of key rows; four windows' additions are requested ahead of the recurrence
+__global__ void __launch_bounds__(256) segment_combine_kernel(float *__restrict__ E, const float *__restrict__ Lend, const float *__restrict__ theta,
+                                                              int n, int BH, int H, float shift) {
+    pdl_wait();
+    const int e = blockIdx.x * 256 + threadIdx.x, bh = blockIdx.y, i = e / (SG_D / 2), j = 2 * (e % (SG_D / 2));
+    float sn, cs;
+    sincosf(-shift * theta[(size_t)(bh % H) * (SG_D / 2) + i], &sn, &cs);
+    const size_t step = (size_t)BH * SG_D * SG_D;
+    float *at = E + ((size_t)bh * SG_D + 2 * i) * SG_D + j;
+    float2 a = make_float2(0.f, 0.f), b = a;                          // rows 2i, 2i + 1
+    for (int w0 = 0; w0 < n; w0 += 4) {
+        float2 ua[4], ub[4];
+        float d[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (w0 + k < n) {
+                ua[k] = *reinterpret_cast<const float2 *>(at + (w0 + k) * step);
+                ub[k] = *reinterpret_cast<const float2 *>(at + (w0 + k) * step + SG_D);
+                d[k] = expf(Lend[(size_t)(w0 + k) * BH + bh]);
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (w0 + k < n) {
+                // the state enters the window rotated back by the previous one's length; the first window enters with zero
+                const float2 ra = make_float2(a.x * cs - b.x * sn, a.y * cs - b.y * sn), rb = make_float2(a.x * sn + b.x * cs, a.y * sn + b.y * cs);
+                a = make_float2(fmaf(d[k], ra.x, ua[k].x), fmaf(d[k], ra.y, ua[k].y));
+                b = make_float2(fmaf(d[k], rb.x, ub[k].x), fmaf(d[k], rb.y, ub[k].y));
+                *reinterpret_cast<float2 *>(at + (w0 + k) * step) = a;
+                *reinterpret_cast<float2 *>(at + (w0 + k) * step + SG_D) = b;
+            }
+    }
+}
+
+size_t segment_scratch_bytes(int B, int H, int T, int seg_len) {
+    const size_t n = (size_t)(T + seg_len - 1) / seg_len - 1;
+    return n * B * H * (SG_D * SG_D + 1) * sizeof(float);
+}
+
+// the states entering segments 1, 2, ... of the raw layer prefill `a` (head dim 64) into scratch
+int segment_states_launch(const PrefillArgs &a, float *scratch, cudaStream_t stream) {
+    const int BH = a.B * a.H, nseg = (a.T + a.seg_len - 1) / a.seg_len;
+    CUtensorMap mk, mv;
+    if (!tc_make_map(&mk, a.k, a.B, a.T, (long long)a.H * SG_D, a.raw_st, a.raw_sb) || !tc_make_map(&mv, a.v, a.B, a.T, (long long)a.H * SG_D, a.raw_st, a.raw_sb)) {
+        set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled");
+        return PGB_ERR_CUDA;
+    }
+    float *Lend = scratch + (size_t)(nseg - 1) * BH * SG_D * SG_D;
+    SgParams p{(const __nv_bfloat16 *)a.la_raw, (const __nv_bfloat16 *)a.gate_raw, a.la_sb, a.la_st, a.decay_A, (const float2 *)a.rot, a.rot_T,
+               scratch, Lend, BH, a.H, a.seg_len};
+    cudaError_t e = cudaFuncSetAttribute(segment_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SgSmem::bytes);
+    if (e == cudaSuccess) e = pdl_launch(segment_state_kernel, dim3((unsigned)(BH * (nseg - 1))), dim3(SG_NT), (size_t)SgSmem::bytes, stream, mk, mv, p);
+    if (e == cudaSuccess)
+        e = pdl_launch(segment_combine_kernel, dim3(SG_D * SG_D / 4 / 256, (unsigned)BH), dim3(256), (size_t)0, stream, scratch, (const float *)Lend, a.theta,
+                       nseg - 1, BH, a.H, (float)a.seg_len);
+    if (e != cudaSuccess) { set_cuda_error(e, "segment_state launch"); return PGB_ERR_CUDA; }
+    return check_launch("segment_state_kernel");
+}
+
+int tc_segment_error_flag(int *out) { return tc_read_error_flag(out); }
+
+}  // namespace pgb

@@ -58,6 +58,8 @@ class LM(nn.Module):
         self.use_graphs = True          # CUDA: replay one captured graph per window in forward_carried
         self._graphs = {}
         self._graphs_stamp = None
+        self._shapes = {}               # _windows_pass: shapes seen, and their captured graphs, in order of use
+        self._wpos = None
         if norm == "rms":                      # every residual-stream LayerNorm becomes an RMSNorm of the same width
             for mod in list(self.modules()):
                 for nm, child in list(mod.named_children()):
@@ -103,6 +105,62 @@ class LM(nn.Module):
             delta = mp.ff(z)
         return x, delta
 
+    def windows_fit(self, window: int) -> bool:
+        return (self.e.weight.is_cuda and self.e.weight.dtype == torch.bfloat16 and
+                all(isinstance(mx, AssocCarrier) and mx.windows_fit(window) for mx in self.mix))
+
+    def _window_positions(self, T, window, device):
+        """(position inside its window of every token, the same modulo the position table)."""
+        key = (T, window, device)
+        if self._wpos is None or self._wpos[0] != key:
+            pos = torch.arange(T, device=device) % window
+            self._wpos = (key, pos, pos % self.p.num_embeddings)
+        return self._wpos[1], self._wpos[2]
+
+    def _layers_windows(self, ids, window, tail, states=None):
+        """Every layer over ALL windows of the sequence at once: layer l of a window needs the layer below on that window
+        and, of the window before, only this layer's state, so nothing but the carried state inside a layer is sequential --
+        one set of GEMMs per layer over the whole sequence instead of one per window. Returns (x, delta) of the last `tail`
+        tokens (the last layer is computed for those only behind its scan) and the layers' final states, written into
+        `states` (tensors) when given."""
+        B, T = ids.shape
+        wpos, epos = self._window_positions(T, window, ids.device)
+        x, delta, new, last = self.e(ids) + self.p(epos), None, [], self.layers - 1
+        for i, (mx, mp) in enumerate(zip(self.mix, self.mlp)):
+            x, z = self._add_norm(x, delta, mx.ln)
+            n = tail if i == last else T
+            delta, S = mx.mix_windows(z, window, wpos, n, None if states is None else states[i])
+            new.append(S)
+            x, z = self._add_norm(x if n == T else x[:, T - n:], delta, mp.n)
+            delta = mp.ff(z)
+        return (x, delta), new
+
+    def _windows_pass(self, ids, window, tail):
+        """_layers_windows, from the second call with a shape on as one CUDA-graph replay (the first call of a shape runs
+        eagerly: a shape that never comes back is not worth a capture). Returns ((x, delta), states); the states are the
+        caller's own."""
+        if not self.use_graphs:
+            return self._layers_windows(ids, window, tail)
+        stamp = self.weights_stamp()
+        if stamp != self._graphs_stamp:
+            self._graphs.clear()
+            self._shapes.clear()
+            self._graphs_stamp = stamp
+        key = (tuple(ids.shape), window, tail, ids.device)
+        run = self._shapes.pop(key, None)
+        if run is None:
+            self._shapes[key] = False
+            if len(self._shapes) > 64:
+                self._shapes.pop(next(iter(self._shapes)))
+            return self._layers_windows(ids, window, tail)
+        if run is False:
+            held = [k for k, v in self._shapes.items() if v is not False]
+            if len(held) >= 8:                                        # eight captured shapes at most, the longest unused one goes
+                self._shapes.pop(held[0])
+            run = _ShapeGraph(self, ids, window, tail)
+        self._shapes[key] = run                                       # last in the order: most recently used
+        return run(ids)
+
     def trunk(self, x, states=None, carry=False):
         """Everything but the output head; with carry=True also takes / returns the per-layer states."""
         new = list(states) if states is not None else [None] * self.layers
@@ -121,7 +179,12 @@ class LM(nn.Module):
         window). On CUDA, with use_graphs set and whole windows, each window pass is one CUDA-graph replay."""
         window = window or self.ctx
         B, T = x.shape
-        if self.use_graphs and x.is_cuda and T % window == 0 and T >= window:
+        if self.windows_fit(window) and x.is_cuda and (B * self.mix[0].h < 148 or T % window):
+            # fewer chains than SMs, or a ragged last window: layer by layer over the whole sequence. With more chains and whole
+            # windows the window-by-window graph below keeps the GPU as full and its activations in the L2.
+            last, states = self._windows_pass(x, window, (T - 1) % window + 1)
+            states = [(S, (T - 1) % window + 1) for S in states]
+        elif self.use_graphs and x.is_cuda and T % window == 0 and T >= window:
             # A captured graph holds the addresses of the parameters and of the constants the mixers derive from them
             # (the concatenated projection weight, the gated output weight): any change of either retires every graph.
             stamp = self.weights_stamp()
@@ -152,6 +215,30 @@ class LM(nn.Module):
                 last = self._layers(self._embed(x[:, s:s + window]), states)
         logits = F.linear(self._add_norm(*last, self.n)[1], self.e.weight)
         return (logits, states) if return_states else logits
+
+
+class _ShapeGraph:
+    """One captured _layers_windows: static ids in, (x, delta) of the last tokens and one tensor of every layer's final state
+    out (cloned per call, so that what a caller keeps is not overwritten by the next one)."""
+
+    def __init__(self, model, ids, window, tail):
+        mx = model.mix[0]
+        self.ids = torch.zeros_like(ids)
+        self.states = torch.empty(model.layers, ids.shape[0], mx.h, mx.dk, mx.dk, device=ids.device, dtype=torch.float32)
+        run = lambda: model._layers_windows(self.ids, window, tail, self.states)[0]
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):                                  # warm-up: library workspaces, cached constants
+            run()
+        torch.cuda.current_stream().wait_stream(side)
+        self.graph = torch.cuda.CUDAGraph()
+        with graph_capture(self.graph):
+            self.out = run()
+
+    def __call__(self, ids):
+        self.ids.copy_(ids)
+        self.graph.replay()
+        return self.out, list(self.states.clone().unbind(0))
 
 
 class _StepGraph:

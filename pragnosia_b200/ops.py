@@ -332,6 +332,46 @@ def layer_prefill(qp, kp, vp, gate_logits, decay_logits, decay_A, table, S0=None
     return o, S, sent
 
 
+@on_device_of
+def layer_prefill_windows(qp, kp, vp, gate_logits, decay_logits, decay_A, table, theta, window: int, rms_weight, rms_eps: float, S_out=None):
+    """layer_prefill over a sequence of `window`-token windows with the state carried, in one call (head dim 64): the windows run
+    side by side, each from its own entering state. Returns (o (B,T,H*D), S)."""
+    need_cuda(qp, kp, vp, decay_logits, table)
+    B, T, H, D = qp.shape
+    o = torch.empty(B, T, H * D, device=qp.device, dtype=qp.dtype)
+    S = _state_out(S_out, B, H, D, qp.device)
+    L = lib()
+    nbytes = L.pgb_aspin_layer_windows_scratch_bytes(B, H, T, window)
+    scratch = torch.empty(nbytes, device=qp.device, dtype=torch.uint8) if nbytes else None
+    sbq = qp.stride(0) if B > 1 else T * qp.stride(1)
+    sba = decay_logits.stride(0) if B > 1 else T * decay_logits.stride(1)
+    check(L.pgb_aspin_layer_prefill_windows_fwd(
+        ptr(qp), ptr(kp), ptr(vp), sbq, qp.stride(1), ptr(gate_logits), ptr(decay_logits), sba, decay_logits.stride(1), ptr(decay_A),
+        ptr(table), table.shape[1], ptr(theta), ptr(rms_weight), float(rms_eps), ptr(o), ptr(S), ptr(scratch), nbytes, int(window), B, H, T, D,
+        stream_of(qp)), "pgb_aspin_layer_prefill_windows_fwd")
+    return o, S
+
+
+@on_device_of
+def delta_layer_windows(qp, kp, vp, decay_logits, beta_logits, decay_A, theta, pos, window: int, rms_weight, rms_eps: float, S_out=None):
+    """The delta layer between its two GEMMs over a sequence of windows with the state carried: plumbing and gates, inverses, one
+    walk, per-head norm. pos (T,) int64: every token's position inside its window. Returns (o (B,T,H*D), S)."""
+    need_cuda(qp, kp, vp, decay_logits, beta_logits)
+    B, T, H, D = qp.shape
+    o = torch.empty(B, T, H * D, device=qp.device, dtype=qp.dtype)
+    S = _state_out(S_out, B, H, D, qp.device)
+    L = lib()
+    nbytes = L.pgb_aspin_delta_layer_scratch_bytes(B, H, T, D)
+    scratch = torch.empty(nbytes, device=qp.device, dtype=torch.uint8)
+    sbq = qp.stride(0) if B > 1 else T * qp.stride(1)
+    sba = decay_logits.stride(0) if B > 1 else T * decay_logits.stride(1)
+    check(L.pgb_aspin_delta_layer_windows_fwd(
+        ptr(qp), ptr(kp), ptr(vp), sbq, qp.stride(1), ptr(decay_logits), ptr(beta_logits), sba, decay_logits.stride(1), ptr(decay_A), ptr(theta),
+        ptr(pos), ptr(rms_weight), float(rms_eps), ptr(o), ptr(S), ptr(scratch), nbytes, int(window), B, H, T, D, stream_of(qp)),
+        "pgb_aspin_delta_layer_windows_fwd")
+    return o, S
+
+
 # ----------------------------------------------------------------------------------------------------------
 @on_device_of
 def rotate(x, theta, pos):

@@ -1,0 +1,82 @@
+"""A layer over a whole sequence of carried windows in one call (mix_windows: the windows side by side for the plain rule, one
+rebasing walk for the delta rule) against the same layer called window by window with the state handed on."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from pragnosia_b200 import ops, synth
+from pragnosia_b200.assoc import AssocCarrier
+from pragnosia_b200.model import LM
+
+pytestmark = pytest.mark.gpu
+torch.set_grad_enabled(False)
+DEV = "cuda"
+
+
+def rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm())
+
+
+@pytest.mark.parametrize("delta,head_dim", [(False, 64), (True, 64), (True, 128)])
+@pytest.mark.parametrize("window,T", [(64, 64), (64, 200), (128, 1), (128, 128), (128, 129), (192, 700), (512, 1333), (1024, 2500)])
+@pytest.mark.parametrize("B", [1, 3])
+def test_all_windows_at_once_match_window_by_window(delta, head_dim, window, T, B):
+    torch.manual_seed(T + window)
+    m = AssocCarrier(256, head_dim=head_dim, delta=delta).to(DEV).to(torch.bfloat16)
+    m.theta.add_(0.01 * torch.randn_like(m.theta))
+    z = torch.randn(B, T, 256, device=DEV).to(torch.bfloat16)
+    assert m.windows_fit(window)
+    c, H, dk, d = m._consts(), m.h, m.dk, 256
+    y = F.linear(z, c["W"], c["b"])                                   # one projection for both: another M may round elsewhere
+    outs, S = [], None
+    for s in range(0, T, window):
+        yw = y[:, s:s + window]
+        n = yw.shape[1]
+        qkv = [yw[..., i * d:(i + 1) * d].unflatten(-1, (H, dk)) for i in range(3)]
+        a, g = yw[..., 3 * d:3 * d + H], yw[..., 3 * d + H:3 * d + 2 * H]
+        kw = dict(theta=c["theta"], shift=0.0 if S is None else float(window))
+        if delta:
+            q, k, v = ops.prep(*qkv, None, c["theta"], torch.arange(n, device=DEV))
+            o, S, _ = ops.prefill(q, k, v, m._la(a, c).transpose(1, 2).contiguous(), m._beta(g).transpose(1, 2).contiguous(), S, **kw)
+            o = m.on(o).transpose(1, 2).reshape(B, n, d)
+        else:
+            o, S, _ = ops.layer_prefill(*qkv, g, a, c["A"], m._rot_table(window, c), S, rms_weight=c["onw"], rms_eps=m._rms_eps(), **kw)
+        outs.append(o)
+    want = F.linear(torch.cat(outs, 1), c["ow"])
+    pos = torch.arange(T, device=DEV) % window
+    got, S2 = m.mix_windows(z, window, pos, T)
+    assert rel(got, want) <= 2e-3 and rel(S2, S) <= 1e-5, (rel(got, want), rel(S2, S))
+    tail = (T - 1) % window + 1
+    assert rel(m.mix_windows(z, window, pos, tail)[0], got[:, T - tail:]) <= 5e-3
+
+
+@pytest.mark.parametrize("mixer", ["aspin", "dspin"])
+def test_shape_graphs_and_what_the_caller_keeps(mixer):
+    """First call eager, second captured, later ones replayed: the same logits and states every time, and a state kept from one
+    call is not overwritten by the next."""
+    torch.manual_seed(0)
+    m = LM(vocab=256, d=128, layers=2, mlp_mult=2, ctx=64, mixer=mixer, norm="rms").to(DEV).to(torch.bfloat16).eval()
+    a, b = (synth.token_ids(2, 150, 256, seed=s).to(DEV) for s in (1, 2))
+    la, sa = m.forward_carried(a, return_states=True)
+    keep = [s[0].clone() for s in sa]
+    m.forward_carried(b)
+    for _ in range(2):
+        l2, s2 = m.forward_carried(a, return_states=True)
+        assert torch.equal(l2, la) and all(torch.equal(x[0], y) for x, y in zip(s2, keep))
+        m.forward_carried(b)
+        assert all(torch.equal(x[0], y) for x, y in zip(s2, keep))
+    assert all(s[1] == 150 % 64 for s in s2)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T", [1, 31, 33, 100])
+def test_prep_with_aligned_rows_matches_the_strided_form(D, T):
+    """prep8_kernel (16-byte aligned rows) against prep_kernel (rows offset by four bytes)."""
+    B, H = 2, 3
+    g = torch.Generator(device=DEV).manual_seed(T)
+    buf = torch.randn(3, B, T, H * D + D // 32, device=DEV, generator=g).to(torch.bfloat16)
+    views = [b[..., :H * D].unflatten(-1, (H, D)) for b in buf]
+    gate = torch.randn(B, T, H, device=DEV, generator=g).to(torch.bfloat16)
+    th, pos = synth.rope_theta(H, D).to(DEV), torch.arange(T, device=DEV)
+    for x, y in zip(ops.prep(*views, gate, th, pos), ops.prep(*[v.contiguous() for v in views], gate, th, pos)):
+        assert (x.float() - y.float()).abs().max() <= 2 ** -7 * x.float().abs().max()
