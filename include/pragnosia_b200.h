@@ -185,6 +185,13 @@ int pgb_aspin_prefill_fwd(const void *q, const void *k, const void *v, int io_dt
                           float shift_host, void *o, int o_dtype, float *S_out, void *sent, int B, int H, int T,
                           int D, int precision, void *stream);
 
+/* The plain rule in full fp32 with scratch (pgb_aspin_prefill_fp32_scratch_bytes bytes): pgb_aspin_prefill_fwd's fp32 arithmetic
+ * with the chunks of a sequence side by side instead of one behind the other. Limit B*H <= 65535. */
+long long pgb_aspin_prefill_fp32_scratch_bytes(int B, int H, int T, int D);
+int pgb_aspin_prefill_fp32_fwd(const float *q, const float *k, const float *v, const float *la, const float *S0, const float *theta,
+                               const float *shift_dev, float shift_host, void *o, int o_dtype, float *S_out, void *sent, void *scratch,
+                               long long scratch_bytes, int B, int H, int T, int D, void *stream);
+
 /* ---------------------------------------------------------------------------------------------------------
  * Delta-rule chunked prefill on the tensor cores (bf16 operands): X = (I + beta strictly_lower(K K^T dec))^-1 for every
  * chunk by a chunk-parallel kernel (exact fp32 substitution), then the walk over chunks with W = X rhs.

@@ -62,6 +62,8 @@ int head_norm_launch(const void *, const float *, float, void *, int, int, int, 
 size_t segment_scratch_bytes(int B, int H, int T, int seg_len);
 int segment_states_launch(const PrefillArgs &, float *, cudaStream_t);
 int tc_segment_error_flag(int *);
+size_t prefill_fp32_chunk_scratch_bytes(int B, int H, int T, int D);
+int prefill_fp32_chunk_launch(const PrefillArgs &, int, int, void *, cudaStream_t);
 int rot_table_launch(const float *, float *, int, int, int, cudaStream_t);
 int decode_embed_launch(const long long *, const long long *, const void *, const void *, void *, int, int, int, int, float *, cudaStream_t);
 int decode_sample_launch(const void *, int, float, float, unsigned long long, long long *, long long *, int, long long *, long long *, float *,
@@ -327,6 +329,27 @@ int pgb_aspin_prefill_fwd(const void *q, const void *k, const void *v, int io_dt
     if (precision == PGB_PREFILL_TENSOR || (precision == PGB_PREFILL_AUTO && tc_ok && kAutoUsesTensor))
         return tc_dispatch(a, o_dtype, D, (cudaStream_t)stream);
     return prefill_fp32_launch(a, io_dtype, o_dtype, D, (cudaStream_t)stream);
+}
+
+long long pgb_aspin_prefill_fp32_scratch_bytes(int B, int H, int T, int D) {
+    if (B <= 0 || H <= 0 || T <= 0 || (D != 64 && D != 128)) return 0;
+    return (long long)prefill_fp32_chunk_scratch_bytes(B, H, T, D);
+}
+
+int pgb_aspin_prefill_fp32_fwd(const float *q, const float *k, const float *v, const float *la, const float *S0, const float *theta,
+                               const float *shift_dev, float shift_host, void *o, int o_dtype, float *S_out, void *sent, void *scratch,
+                               long long scratch_bytes, int B, int H, int T, int D, void *stream) {
+    if (!q || !k || !v || !la || !o || !S_out || !scratch) return PGB_ERR_NULL_POINTER;
+    if (!dtype_ok(o_dtype)) return PGB_ERR_BAD_DTYPE;
+    if (B <= 0 || H <= 0 || T <= 0) return PGB_ERR_BAD_SHAPE;
+    if ((long long)B * H > 65535) return PGB_ERR_TOO_LARGE;
+    if (D != 64 && D != 128) return PGB_ERR_UNSUPPORTED_DIM;
+    if (scratch_bytes < pgb_aspin_prefill_fp32_scratch_bytes(B, H, T, D)) return PGB_ERR_BAD_SHAPE;
+    if (!aligned(q, 16) || !aligned(k, 16) || !aligned(v, 16) || !aligned(o, 16) || !aligned(S_out, 16) || (S0 && !aligned(S0, 16)) ||
+        (sent && !aligned(sent, 16)) || !aligned(scratch, 16))
+        return PGB_ERR_MISALIGNED;
+    PrefillArgs a{q, k, v, la, nullptr, S0, o, S_out, (__nv_bfloat16 *)sent, theta, shift_dev, shift_host, B, H, T};
+    return prefill_fp32_chunk_launch(a, o_dtype, D, scratch, (cudaStream_t)stream);
 }
 
 int pgb_aspin_prefill_fused_fwd(const void *q, const void *k, const void *v, const void *decay_logits,

@@ -80,6 +80,7 @@ class _LambdaScan(torch.autograd.Function):
         h0 = None if h0r is None else (h0r, h0i)
         y, (hr, hi), hia = ops.lambda_scan(u, logmag, ang, h0, keep_imag=True)
         ctx.save_for_backward(u, logmag, ang, y, hia)
+        ctx.set_materialize_grads(False)                              # no gradient arrived: None, not a tensor of zeros to add
         ctx.has = h0r is not None
         return y, hr, hi
 
@@ -90,6 +91,8 @@ class _LambdaScan(torch.autograd.Function):
         if g_last_r is not None:
             g = g.clone()
             g[:, -1] += g_last_r.to(torch.float32)
+        if g_last_i is not None:
+            g_last_i = g_last_i.to(torch.float32)
         du, dlm, dan, d0r, d0i = ops.lambda_scan_bwd(g.contiguous(), u, logmag, ang, y, hia, g_last_i, want_dh0=ctx.has)
         return du, dlm, dan, d0r, d0i
 

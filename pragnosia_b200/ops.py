@@ -17,10 +17,18 @@ from . import _lib
 from ._lib import check, dtype_code, lib, need_cuda, on_device_of, ptr, stream_of
 
 CHUNK = 64
+FP32_CHUNK_SCRATCH = 8 << 30      # bytes of per-chunk states the fp32 plain prefill may take; beyond (B*H*T > 33 M at D = 64) it walks the chains
 
 
 def _f32c(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-    return None if t is None else t.to(torch.float32).contiguous()
+    if t is None or (t.dtype is torch.float32 and t.is_contiguous()):
+        return t
+    return t.to(torch.float32).contiguous()
+
+
+def _like(t: torch.Tensor, ref: torch.Tensor) -> torch.Tensor:
+    """t, contiguous and of ref's dtype (t itself where it is)."""
+    return t if t.dtype is ref.dtype and t.is_contiguous() else t.to(ref.dtype).contiguous()
 
 
 def _compiling() -> bool:
@@ -218,7 +226,7 @@ def prefill(q, k, v, la, beta=None, S0=None, theta=None, shift=0.0, want_sent: b
     B, H, T, D = q.shape
     if q.dtype not in (torch.float32, torch.bfloat16):
         q = q.float()
-    q, k, v = q.contiguous(), k.to(q.dtype).contiguous(), v.to(q.dtype).contiguous()
+    q, k, v = _like(q, q), _like(k, q), _like(v, q)
     la, beta, S0 = _f32c(la), _f32c(beta), _f32c(S0)
     theta, shift_dev, shift_host = _shift_args(theta, S0, shift)
     if shift_dev is not None:
@@ -240,6 +248,14 @@ def prefill(q, k, v, la, beta=None, S0=None, theta=None, shift=0.0, want_sent: b
                                                 shift_host, ptr(o), dtype_code(o), ptr(S), ptr(sent), ptr(scratch), nbytes,
                                                 B, H, T, D, stream_of(q)), "pgb_aspin_delta_prefill_fwd")
         return o, S, sent
+    if beta is None and q.dtype == torch.float32 and precision != _lib.PREFILL_TENSOR and B * H <= 65535:
+        nbytes = lib().pgb_aspin_prefill_fp32_scratch_bytes(B, H, T, D)      # fp32 plain rule: the chunks side by side
+        if nbytes <= FP32_CHUNK_SCRATCH:
+            scratch = torch.empty(nbytes, device=q.device, dtype=torch.uint8)
+            check(lib().pgb_aspin_prefill_fp32_fwd(ptr(q), ptr(k), ptr(v), ptr(la), ptr(S0), ptr(theta), ptr(shift_dev), shift_host, ptr(o),
+                                                   dtype_code(o), ptr(S), ptr(sent), ptr(scratch), nbytes, B, H, T, D, stream_of(q)),
+                  "pgb_aspin_prefill_fp32_fwd")
+            return o, S, sent
     check(lib().pgb_aspin_prefill_fwd(ptr(q), ptr(k), ptr(v), dtype_code(q), ptr(la), ptr(beta), ptr(S0), ptr(theta),
                                       ptr(shift_dev), shift_host, ptr(o), dtype_code(o), ptr(S), ptr(sent), B, H, T, D, precision,
                                       stream_of(q)), "pgb_aspin_prefill_fwd")
