@@ -99,8 +99,8 @@ int pgb_aspin_prep_fwd(const void *qp, const void *kp, const void *vp, int in_dt
 /* Gradient of pgb_aspin_prep_fwd. Replaces src/assoc_kernel.py:774-826 _prep_bwd (op membrae::assoc_prep_bwd :850).
  *   qp, kp, vp, gate, theta, pos: the forward inputs, same strides.  dq, dk, dv: grad_dtype, contiguous (B,H,T,D).
  *   dqp, dkp, dvp: in_dtype, contiguous (B,T,H,D).  dgate [B][T][H] fp32 (required when gate is given).
- *   dtheta_partial [B * pgb_aspin_prep_bwd_tiles(T)][H][D/2] fp32: one partial per CTA; theta's gradient is their sum
- *   over the first axis (a fixed summation order, so results repeat bit for bit). */
+ *   dtheta_partial [B * pgb_aspin_prep_bwd_tiles(T)][H][D/2] fp32, or NULL where theta's gradient is not wanted; that gradient
+ *   is the sum over the first axis (a fixed summation order, so results repeat bit for bit). */
 int pgb_aspin_prep_bwd(const void *qp, const void *kp, const void *vp, int in_dtype, long long in_stride_b, long long in_stride_t,
                        long long in_stride_h, const void *gate, long long gate_stride_b, long long gate_stride_t, const float *theta,
                        const long long *pos, const void *dq, const void *dk, const void *dv, int grad_dtype, void *dqp, void *dkp,

@@ -1,127 +1,14 @@
-// Backward kernels of the two simplest operators on the path, for callers that train through them:
-//
-//   lambda_scan_bwd   the adjoint of h_t = lambda_t h_{t-1} + u_t (reference: src/scan_kernel.py:54-101 _bwd, wired by
-//                     _Scan.backward :121-140). The adjoint state obeys the same kind of recurrence run backwards in time,
-//                     a_{t-1} = conj(lambda_t) a_t + g_{t-1}, so it is the forward kernel's chunked shuffle scan on the
-//                     reversed sequence; with R_t h_{t-1} = h_t - (u_t, 0) the three per-token gradients are
-//                         du_t = Re a_t,   dlogmag_t = a_t . (h_t - u_t),   dang_t = a_t . i (h_t - u_t).
-//   prep_bwd          the gradient of the normalise / gate / rotate plumbing (reference: src/assoc_kernel.py:774-826
-//                     _prep_bwd): with u = x / |x|, r = R(ang) u and g the gradient on r: du = R^T g,
-//                     dx = (du - u (u . du)) / |x|, d ang = g2 r1 - g1 r2 per pair; theta's gradient is the sum of
-//                     pos * d ang over batch and time, written as one partial per CTA and summed by the caller.
+// prep_bwd: the gradient of the normalise / gate / rotate plumbing (reference: src/assoc_kernel.py:774-826 _prep_bwd), for
+// callers that train through it: with u = x / |x|, r = R(ang) u and g the gradient on r: du = R^T g,
+// dx = (du - u (u . du)) / |x|, d ang = g2 r1 - g1 r2 per pair; theta's gradient is the sum of pos * d ang over batch and time,
+// written as one partial per CTA and summed by the caller.
 #include "common.cuh"
 
 namespace pgb {
 
-// ---------------------------------------------------------------------------------------------------- lambda scan adjoint
-constexpr int LB_SEG = 4, LB_WARPS = 4;
-
-template <int TS>
-__global__ void __launch_bounds__(LB_WARPS * 32)
-lambda_scan_bwd_kernel(const float *__restrict__ g, const float *__restrict__ u, const float *__restrict__ lm, const float *__restrict__ an,
-                       long long an_sb, long long an_st, const float *__restrict__ hr_all, const float *__restrict__ hi_all,
-                       const float *__restrict__ gli, float *__restrict__ du, float *__restrict__ dlm, float *__restrict__ dan,
-                       float *__restrict__ dh0r, float *__restrict__ dh0i, int B, int T, int D) {
-    constexpr int CQ = 32 / TS;
-    constexpr unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int wpb = (D + CQ - 1) / CQ;                                // warps per batch row
-    const long long wg = (long long)blockIdx.x * LB_WARPS + (threadIdx.x >> 5);
-    if (wg >= (long long)B * wpb) return;                             // a whole warp leaves together
-    const int b = (int)(wg / wpb), cq = lane % CQ, seg = lane / CQ;
-    const int d = (int)(wg % wpb) * CQ + cq;
-    const bool live = d < D;
-    const size_t row0 = (size_t)b * T;
-    float ar = 0.f, ai = (live && gli != nullptr) ? gli[(size_t)b * D + d] : 0.f;   // adjoint state entering the tile (from later times)
-
-    for (int r0 = 0; r0 < T; r0 += TS * LB_SEG) {
-        const int rb = r0 + seg * LB_SEG;                             // reversed step index; time t = T - 1 - r
-        float c[LB_SEG], s[LB_SEG], x[LB_SEG];
-#pragma unroll
-        for (int i = 0; i < LB_SEG; ++i) {
-            const int t = T - 1 - (rb + i);
-            c[i] = 1.f; s[i] = 0.f; x[i] = 0.f;                       // steps before time 0, and the first (latest) step: the identity
-            if (live && t >= 0) {
-                x[i] = g[(row0 + t) * D + d];
-                if (t + 1 < T) {
-                    const float mag = expf(lm[(row0 + t + 1) * D + d]);
-                    float sn, cs;
-                    sincosf(an[(size_t)b * an_sb + (size_t)(t + 1) * an_st + d], &sn, &cs);
-                    c[i] = mag * cs; s[i] = -mag * sn;                 // conj(lambda_{t+1})
-                }
-            }
-        }
-        float hsr = ar, hsi = ai;
-        if constexpr (TS > 1) {
-            float Ar = 1.f, Ai = 0.f, Br = 0.f, Bi = 0.f;             // this segment's affine map a -> A a + B
-#pragma unroll
-            for (int i = 0; i < LB_SEG; ++i) {
-                const float nbr = c[i] * Br - s[i] * Bi + x[i], nbi = s[i] * Br + c[i] * Bi;
-                const float nar = c[i] * Ar - s[i] * Ai, nai = s[i] * Ar + c[i] * Ai;
-                Br = nbr; Bi = nbi; Ar = nar; Ai = nai;
-            }
-#pragma unroll
-            for (int off = 1; off < TS; off <<= 1) {
-                const float par = __shfl_up_sync(FULL, Ar, off * CQ), pai = __shfl_up_sync(FULL, Ai, off * CQ);
-                const float pbr = __shfl_up_sync(FULL, Br, off * CQ), pbi = __shfl_up_sync(FULL, Bi, off * CQ);
-                if (seg >= off) {
-                    const float nbr = Ar * pbr - Ai * pbi + Br, nbi = Ai * pbr + Ar * pbi + Bi;
-                    const float nar = Ar * par - Ai * pai, nai = Ai * par + Ar * pai;
-                    Br = nbr; Bi = nbi; Ar = nar; Ai = nai;
-                }
-            }
-            float ear = __shfl_up_sync(FULL, Ar, CQ), eai = __shfl_up_sync(FULL, Ai, CQ);
-            float ebr = __shfl_up_sync(FULL, Br, CQ), ebi = __shfl_up_sync(FULL, Bi, CQ);
-            if (seg == 0) { ear = 1.f; eai = 0.f; ebr = 0.f; ebi = 0.f; }
-            hsr = ear * ar - eai * ai + ebr;
-            hsi = eai * ar + ear * ai + ebi;
-        }
-#pragma unroll
-        for (int i = 0; i < LB_SEG; ++i) {
-            const int t = T - 1 - (rb + i);
-            const float nr = c[i] * hsr - s[i] * hsi + x[i], ni = s[i] * hsr + c[i] * hsi;
-            hsr = nr; hsi = ni;
-            if (live && t >= 0) {
-                const size_t off = (row0 + t) * D + d;
-                const float rr = hr_all[off] - u[off], ri = hi_all[off];      // lambda_t h_{t-1}
-                du[off] = nr;
-                dlm[off] = nr * rr + ni * ri;
-                dan[off] = ni * rr - nr * ri;
-            }
-        }
-        if constexpr (TS > 1) {
-            ar = __shfl_sync(FULL, hsr, (TS - 1) * CQ + cq);
-            ai = __shfl_sync(FULL, hsi, (TS - 1) * CQ + cq);
-        } else {
-            ar = hsr; ai = hsi;
-        }
-    }
-    if (live && seg == 0 && dh0r != nullptr) {                        // a_{-1} = conj(lambda_0) a_0
-        const float mag = expf(lm[row0 * D + d]);
-        float sn, cs;
-        sincosf(an[(size_t)b * an_sb + d], &sn, &cs);
-        dh0r[(size_t)b * D + d] = mag * (cs * ar + sn * ai);
-        dh0i[(size_t)b * D + d] = mag * (cs * ai - sn * ar);
-    }
-}
-
-int lambda_scan_bwd_launch(const float *g, const float *u, const float *lm, const float *an, long long sb, long long st,
-                           const float *hr_all, const float *hi_all, const float *gli, float *du, float *dlm, float *dan,
-                           float *dh0r, float *dh0i, int B, int T, int D, cudaStream_t stream) {
-    // many channels: one lane per channel walks its sequence; few: 8 time segments per warp share the walk
-    const bool wide = (long long)B * D >= 148LL * 8 * 32 || T <= 2 * LB_SEG;
-    const int cq = wide ? 32 : 4;
-    const long long warps = (long long)B * ((D + cq - 1) / cq), ctas = (warps + LB_WARPS - 1) / LB_WARPS;
-    if (ctas > 0x7fffffffLL) return PGB_ERR_TOO_LARGE;
-    if (wide)
-        lambda_scan_bwd_kernel<1><<<(unsigned)ctas, LB_WARPS * 32, 0, stream>>>(g, u, lm, an, sb, st, hr_all, hi_all, gli, du, dlm, dan, dh0r, dh0i, B, T, D);
-    else
-        lambda_scan_bwd_kernel<8><<<(unsigned)ctas, LB_WARPS * 32, 0, stream>>>(g, u, lm, an, sb, st, hr_all, hi_all, gli, du, dlm, dan, dh0r, dh0i, B, T, D);
-    return check_launch("lambda_scan_bwd_kernel");
-}
-
 // ---------------------------------------------------------------------------------------------------- prep backward
-constexpr int PB_WARPS = 8;                                           // consecutive tokens of one (sequence, head) per CTA
+constexpr int PB_WARPS = 8;                                           // consecutive tokens of one (sequence, head) per partial of theta's gradient
+constexpr int PB_TOK = 32;                                            // ... and per CTA of the 16-byte form, which fills four partials' places
 
 template <typename T_, int PER>
 __device__ __forceinline__ void pb_ld(float (&d)[PER], const T_ *p) {
@@ -135,7 +22,7 @@ __device__ __forceinline__ void pb_st(T_ *p, const float (&d)[PER]) {
 }
 
 // qp, kp, vp: TIN views (B,T,H,D) with element strides (sb, st, sh);  dq, dk, dv: TG, contiguous (B,H,T,D)
-// dqp, dkp, dvp: TIN, contiguous (B,T,H,D);  dgl fp32 (B,T,H);  dth_part fp32 [B * NT][H][D/2], NT = ceil(T / PB_WARPS)
+// dqp, dkp, dvp: TIN, contiguous (B,T,H,D);  dgl fp32 (B,T,H);  dth_part fp32 [B * NT][H][D/2], NT = ceil(T / PB_WARPS); dth_part NULL: theta's gradient is not wanted
 template <typename TIN, typename TG, int D>
 __global__ void __launch_bounds__(PB_WARPS * 32)
 prep_bwd_kernel(const TIN *__restrict__ qp, const TIN *__restrict__ kp, const TIN *__restrict__ vp, long long sb, long long st, long long sh,
@@ -213,6 +100,7 @@ prep_bwd_kernel(const TIN *__restrict__ qp, const TIN *__restrict__ kp, const TI
         for (int i = 0; i < PER; ++i) out[i] = (gr[i] - x[i] * inv * dot) * inv;
         pb_st<TIN, PER>(dvp + o_off, out);
     }
+    if (dth_part == nullptr) return;
     // ---- theta: this CTA's share of the sum over batch and time, tokens added in a fixed order
 #pragma unroll
     for (int i = 0; i < NP; ++i) part[warp][lane * NP + i] = dang[i] * p;
@@ -222,6 +110,90 @@ prep_bwd_kernel(const TIN *__restrict__ qp, const TIN *__restrict__ kp, const TI
 #pragma unroll
         for (int w = 0; w < PB_WARPS; ++w) s += part[w][threadIdx.x];
         dth_part[(((size_t)b * NT + pt) * H + h) * (D / 2) + threadIdx.x] = s;
+    }
+}
+
+// The same for bf16 operands and gradients with 16-byte aligned rows: D/8 lanes share a row, 8 channels (four pairs) each, so a
+// warp takes four rows (D = 64) or two: 16-byte accesses, a shuffle tree of three or four steps per sum instead of five, and a
+// quarter of the instructions a row. Bound by instruction issue before HBM (four sincosf a lane). 90112 rows of 64: 54 -> 30-34 us.
+template <int D>
+__global__ void __launch_bounds__(PB_WARPS * 32)
+prep8_bwd_kernel(const __nv_bfloat16 *__restrict__ qp, const __nv_bfloat16 *__restrict__ kp, const __nv_bfloat16 *__restrict__ vp, long long sb, long long st,
+                 long long sh, const __nv_bfloat16 *__restrict__ gate, long long gsb, long long gst, const float *__restrict__ theta,
+                 const long long *__restrict__ pos, const __nv_bfloat16 *__restrict__ dq, const __nv_bfloat16 *__restrict__ dk,
+                 const __nv_bfloat16 *__restrict__ dv, __nv_bfloat16 *__restrict__ dqp, __nv_bfloat16 *__restrict__ dkp, __nv_bfloat16 *__restrict__ dvp,
+                 float *__restrict__ dgl, float *__restrict__ dth_part, int T, int H, int NT) {
+    constexpr int LPR = D / 8, RPC = PB_WARPS * 32 / LPR;
+    __shared__ float part[PB_WARPS][D / 2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, li = threadIdx.x % LPR;
+    const int pt = blockIdx.x, bh = blockIdx.y, b = bh / H, h = bh % H;
+    const unsigned mask = (LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1u)) << (lane / LPR * LPR);
+    auto row_sum = [&](float x) {
+#pragma unroll
+        for (int m = 1; m < LPR; m <<= 1) x += __shfl_xor_sync(mask, x, m);
+        return x;
+    };
+    const float4 th = *reinterpret_cast<const float4 *>(theta + (size_t)h * (D / 2) + 4 * li);
+    const float ang[4] = {th.x, th.y, th.z, th.w};
+    float dsum[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int t = pt * PB_TOK + threadIdx.x / LPR; t < min(T, (pt + 1) * PB_TOK); t += RPC) {
+        const size_t in = (size_t)b * sb + (size_t)t * st + (size_t)h * sh + 8 * li, gr = ((size_t)bh * T + t) * D + 8 * li,
+                     out = (((size_t)b * T + t) * H + h) * D + 8 * li;
+        const uint4 xr[3] = {*reinterpret_cast<const uint4 *>(qp + in), *reinterpret_cast<const uint4 *>(kp + in), *reinterpret_cast<const uint4 *>(vp + in)};
+        const uint4 gv[3] = {*reinterpret_cast<const uint4 *>(dq + gr), *reinterpret_cast<const uint4 *>(dk + gr), *reinterpret_cast<const uint4 *>(dv + gr)};
+        const float p = (float)pos[t];
+        const float sg = gate != nullptr ? sigmoidf_(__bfloat162float(gate[(size_t)b * gsb + (size_t)t * gst + h])) : 1.f;
+        float cs[4], sn[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sincosf(p * ang[i], &sn[i], &cs[i]);
+#pragma unroll
+        for (int w = 0; w < 3; ++w) {
+            const __nv_bfloat162 *x2 = reinterpret_cast<const __nv_bfloat162 *>(&xr[w]), *g2 = reinterpret_cast<const __nv_bfloat162 *>(&gv[w]);
+            float2 x[4], g[4];
+            float ss = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { x[i] = __bfloat1622float2(x2[i]); g[i] = __bfloat1622float2(g2[i]); ss = fmaf(x[i].x, x[i].x, fmaf(x[i].y, x[i].y, ss)); }
+            const float inv = 1.0f / fmaxf(sqrtf(row_sum(ss)), 1e-12f);
+            float2 du[4];
+            float dot = 0.f, dsg = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float u1 = x[i].x * inv, u2 = x[i].y * inv;
+                if (w < 2) {
+                    const float r1 = u1 * cs[i] - u2 * sn[i], r2 = u1 * sn[i] + u2 * cs[i];
+                    if (w == 1) { dsg += g[i].x * r1 + g[i].y * r2; g[i].x *= sg; g[i].y *= sg; }
+                    dsum[i] = fmaf(p, g[i].y * r1 - g[i].x * r2, dsum[i]);
+                    du[i] = make_float2(g[i].x * cs[i] + g[i].y * sn[i], g[i].y * cs[i] - g[i].x * sn[i]);
+                } else du[i] = g[i];
+                dot += u1 * du[i].x + u2 * du[i].y;
+            }
+            dot = row_sum(dot);
+            if (w == 1 && gate != nullptr) {
+                dsg = row_sum(dsg);
+                if (li == 0) dgl[((size_t)b * T + t) * H + h] = dsg * sg * (1.0f - sg);
+            }
+            uint4 res;
+            __nv_bfloat162 *o2 = reinterpret_cast<__nv_bfloat162 *>(&res);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o2[i] = __floats2bfloat162_rn((du[i].x - x[i].x * inv * dot) * inv, (du[i].y - x[i].y * inv * dot) * inv);
+            *reinterpret_cast<uint4 *>((w == 0 ? dqp : w == 1 ? dkp : dvp) + out) = res;
+        }
+    }
+    if (dth_part == nullptr) return;
+    // theta: the warp's rows, then the warps, in a fixed order
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int m = LPR; m < 32; m <<= 1) dsum[i] += __shfl_xor_sync(0xffffffffu, dsum[i], m);
+        if (lane < LPR) part[warp][4 * li + i] = dsum[i];
+    }
+    __syncthreads();
+    if (threadIdx.x < D / 2) {
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < PB_WARPS; ++w) s += part[w][threadIdx.x];
+        for (int k = 0; k < PB_TOK / PB_WARPS && 4 * pt + k < NT; ++k)
+            dth_part[(((size_t)b * NT + 4 * pt + k) * H + h) * (D / 2) + threadIdx.x] = k == 0 ? s : 0.f;
     }
 }
 
@@ -246,6 +218,20 @@ int prep_bwd_launch(const void *qp, const void *kp, const void *vp, int in_dtype
                     long long gsb, long long gst, const float *theta, const long long *pos, const void *dq, const void *dk, const void *dv,
                     int g_dtype, void *dqp, void *dkp, void *dvp, float *dgl, float *dth_part, int B, int T, int H, int D,
                     cudaStream_t stream) {
+    const void *rows[] = {qp, kp, vp, dq, dk, dv, dqp, dkp, dvp, theta};
+    bool wide = in_dtype == PGB_BF16 && g_dtype == PGB_BF16 && sb % 8 == 0 && st % 8 == 0 && sh % 8 == 0;
+    for (const void *r : rows) wide = wide && aligned(r, 16);
+    if (wide) {
+        typedef const __nv_bfloat16 *In;
+        typedef __nv_bfloat16 *Out;
+        const int NT = prep_bwd_tiles(T);
+        auto go = [&](auto kern) {
+            kern<<<dim3((T + PB_TOK - 1) / PB_TOK, B * H), PB_WARPS * 32, 0, stream>>>((In)qp, (In)kp, (In)vp, sb, st, sh, (In)gate, gsb, gst, theta, pos, (In)dq, (In)dk, (In)dv,
+                                                               (Out)dqp, (Out)dkp, (Out)dvp, dgl, dth_part, T, H, NT);
+        };
+        if (D == 64) go(prep8_bwd_kernel<64>); else go(prep8_bwd_kernel<128>);
+        return check_launch("prep8_bwd_kernel");
+    }
 #define PB_ARGS qp, kp, vp, sb, st, sh, gate, gsb, gst, theta, pos, dq, dk, dv, dqp, dkp, dvp, dgl, dth_part, B, T, H, D, stream
     if (in_dtype == PGB_F32) return g_dtype == PGB_F32 ? prep_bwd_go<float, float>(PB_ARGS) : prep_bwd_go<float, __nv_bfloat16>(PB_ARGS);
     return g_dtype == PGB_F32 ? prep_bwd_go<__nv_bfloat16, float>(PB_ARGS) : prep_bwd_go<__nv_bfloat16, __nv_bfloat16>(PB_ARGS);

@@ -187,7 +187,7 @@ int pgb_aspin_prep_bwd(const void *qp, const void *kp, const void *vp, int in_dt
                        long long in_stride_h, const void *gate, long long gate_stride_b, long long gate_stride_t, const float *theta,
                        const long long *pos, const void *dq, const void *dk, const void *dv, int grad_dtype, void *dqp, void *dkp,
                        void *dvp, float *dgate, float *dtheta_partial, int B, int T, int H, int D, void *stream) {
-    if (!qp || !kp || !vp || !theta || !pos || !dq || !dk || !dv || !dqp || !dkp || !dvp || !dtheta_partial) return PGB_ERR_NULL_POINTER;
+    if (!qp || !kp || !vp || !theta || !pos || !dq || !dk || !dv || !dqp || !dkp || !dvp) return PGB_ERR_NULL_POINTER;
     if (gate && !dgate) return PGB_ERR_NULL_POINTER;
     if (!dtype_ok(in_dtype) || !dtype_ok(grad_dtype)) return PGB_ERR_BAD_DTYPE;
     if (B <= 0 || T <= 0 || H <= 0 || (long long)B * H > 65535) return PGB_ERR_BAD_SHAPE;

@@ -7,7 +7,8 @@
 //   3. fp32_out_kernel     a CTA per (chain, chunk, 64 value columns):           o = ((Q K^T) dec) V + e^L (Q S_c)
 // Every product is 64 x 64 outputs by 256 threads, a 4 x 4 tile each, with both operands contraction-major in shared memory
 // (two 16-byte loads per 16 multiply-adds), which puts the FFMA pipe ahead of shared memory. Same masking as the walk: rows
-// past T are zero tokens with log-decay 0. B2 H12 T512 D64: 131 us (walk) -> see the launcher.
+// past T are zero tokens with log-decay 0. B2 H12 T512 D64: 131 us as a walk -> 27 us (states 6.5,
+// prefix 3.2, outputs 17.4).
 #include "common.cuh"
 
 namespace pgb {

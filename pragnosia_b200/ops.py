@@ -206,8 +206,7 @@ def prep_bwd(qp, kp, vp, gate_logits, theta, pos, dq, dk, dv, want_theta: bool =
     dqp = torch.empty(B, T, H, D, device=qp.device, dtype=qp.dtype)
     dkp, dvp = torch.empty_like(dqp), torch.empty_like(dqp)
     dgl = None if gate_logits is None else torch.empty(B, T, H, device=qp.device, dtype=torch.float32)
-    nt = lib().pgb_aspin_prep_bwd_tiles(T)
-    part = torch.empty(B * nt, H, D // 2, device=qp.device, dtype=torch.float32)
+    part = torch.empty(B * lib().pgb_aspin_prep_bwd_tiles(T), H, D // 2, device=qp.device, dtype=torch.float32) if want_theta else None
     check(lib().pgb_aspin_prep_bwd(ptr(qp), ptr(kp), ptr(vp), dtype_code(qp), qp.stride(0), qp.stride(1), qp.stride(2),
                                    ptr(gate_logits), gsb, gst, ptr(theta), ptr(pos), ptr(dq), ptr(dk), ptr(dv), dtype_code(dq),
                                    ptr(dqp), ptr(dkp), ptr(dvp), ptr(dgl), ptr(part), B, T, H, D, stream_of(qp)),

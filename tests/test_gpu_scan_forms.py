@@ -1,0 +1,71 @@
+"""The forms the lambda scan, the prep backward and the fp32 chunked prefill choose between, at the edges of their ranges, against
+the fp64 definitions: lanes of 4, 2 or 1 channels, the form with many warps and the one that loads ahead, angles past the range
+of the fast sin/cos; rows read 16 bytes at a time or not."""
+import pytest
+import torch
+
+import oracle.carrier_oracle as oracle
+from pragnosia_b200 import ops, synth
+from pragnosia_b200._lib import PREFILL_FP32
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
+
+
+@pytest.mark.parametrize("B,T,D", [(1, 1, 4), (2, 7, 6), (3, 65, 5), (1, 129, 8), (700, 9, 512), (5, 257, 64), (2, 33, 301)])
+@pytest.mark.parametrize("per_channel", [False, True])
+def test_lambda_scan_and_adjoint_forms(B, T, D, per_channel):
+    g = torch.Generator(device=DEV).manual_seed(B + T + D)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    u, lm, h0, w = r(B, T, D), -r(B, T, D).abs() * 3, (r(B, D), r(B, D)), r(B, T, D)
+    an = r(1, 1, D).expand(B, T, D) if per_channel else r(B, T, D)
+    if not per_channel:
+        an[:, ::5] *= 1e5                                             # past the range of the reduction: the library's own sin and cos
+    y, (hr, hi), him = ops.lambda_scan(u, lm, an, h0, keep_imag=True)
+    y0, (hr0, hi0) = ops.lambda_scan(u, lm, an, h0)
+    assert torch.equal(y, y0) and torch.equal(hr, hr0) and torch.equal(hi, hi0)
+    ry, (rr, ri) = oracle.lambda_literal(u.double(), lm.double(), an.double(), (h0[0].double(), h0[1].double()))
+    for a, b in ((y, ry), (hr, rr), (hi, ri), (him[:, -1], ri)):
+        assert rel(a, b) < 5e-6
+    d = ops.lambda_scan_bwd(w, u, lm, an, y, him, g_last_i=r(B, D) * 0, want_dh0=True)
+    if B < 100:
+        ref = oracle.lambda_scan_grads(u, lm, an, h0, w, torch.zeros(B, D, device=DEV), torch.zeros(B, D, device=DEV))
+        for a, b in zip(d, ref):
+            assert rel(a, b) < 2e-5
+
+
+@pytest.mark.parametrize("T", [1, 31, 32, 33, 100])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("strided", [False, True])
+def test_prep_backward_row_forms(T, D, strided):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    B, H = 2, 3
+    wide = torch.randn(B, T, 3 * H * D + 8, device=DEV, generator=g).bfloat16()
+    off = 4 if strided else 0                                        # 8 bytes off: the rows are not 16-byte aligned
+    qp, kp, vp = (wide[..., off + i * H * D:off + (i + 1) * H * D].unflatten(-1, (H, D)) for i in range(3))
+    gl = torch.randn(B, T, H, device=DEV, generator=g).bfloat16()
+    th, pos = synth.rope_theta(H, D).to(DEV), 50 + torch.arange(T, device=DEV)
+    dy = [torch.randn(B, H, T, D, device=DEV, generator=g).bfloat16() for _ in range(3)]
+    got = ops.prep_bwd(qp, kp, vp, gl, th, pos, *dy)
+    with torch.enable_grad():
+        a = [t.detach().float().requires_grad_(True) for t in (qp, kp, vp, gl, th)]
+        ref = torch.autograd.grad(sum((o * d.float()).sum() for o, d in zip(oracle.prep_ref(*a, pos), dy)), a)
+    for x, y_, tol in zip(got, ref, (4e-3, 4e-3, 4e-3, 1e-4, 1e-3)):
+        assert rel(x.float(), y_) < tol
+    assert ops.prep_bwd(qp, kp, vp, gl, th, pos, *dy, want_theta=False)[4] is None
+
+
+@pytest.mark.parametrize("T", [1, 63, 64, 65, 200])
+@pytest.mark.parametrize("D", [64, 128])
+def test_fp32_prefill_chunks(T, D):
+    g = torch.Generator().manual_seed(T)
+    q, k, v = (torch.nn.functional.normalize(torch.randn(2, 3, T, D, generator=g), dim=-1) for _ in range(3))
+    la, S0 = -torch.rand(2, 3, T, generator=g), torch.randn(2, 3, D, D, generator=g)
+    a = [t.to(DEV) for t in (q, k, v, la, S0)]
+    o, S = ops.prefill(*a[:4], S0=a[4], precision=PREFILL_FP32)[:2]
+    ro, rS = oracle.plain_literal(*(t.double() for t in (q, k, v, la, S0)))
+    assert rel(o.cpu(), ro) < 2e-6 and rel(S.cpu(), rS) < 2e-6
