@@ -6,12 +6,14 @@ from __future__ import annotations
 
 import contextlib
 import ctypes as C
+import importlib.util
 from pathlib import Path
 
 import torch
 
 PKG = Path(__file__).resolve().parent
 LIB_PATH = PKG / "lib" / "libpragnosia_b200.so"
+HOST_PATH = PKG / "lib" / "pgb_torch.so"
 
 F32, BF16 = 0, 1
 PREFILL_AUTO, PREFILL_FP32, PREFILL_TENSOR = 0, 1, 2
@@ -106,6 +108,22 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The C++ half of the tensor-level wrappers (csrc/torch_host.cpp): an extension module beside the library it calls."""
+    global _host
+    if _host is None:
+        lib()
+        if not HOST_PATH.exists():
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m pragnosia_b200.build`.")
+        spec = importlib.util.spec_from_file_location(HOST_PATH.stem, HOST_PATH)
+        _host = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_host)
+    return _host
+
+
 def check(status: int, what: str) -> None:
     if status != 0:
         L = lib()
@@ -114,12 +132,16 @@ def check(status: int, what: str) -> None:
         raise RuntimeError(f"{what}: {msg}" + (f" [{extra}]" if extra else ""))
 
 
-def dtype_code(t: torch.Tensor) -> int:
-    if t.dtype == torch.float32:
+def type_code(dt: torch.dtype) -> int:
+    if dt is torch.float32:
         return F32
-    if t.dtype == torch.bfloat16:
+    if dt is torch.bfloat16:
         return BF16
-    raise TypeError(f"pragnosia_b200 kernels take float32 or bfloat16 tensors, got {t.dtype}")
+    raise TypeError(f"pragnosia_b200 kernels take float32 or bfloat16 tensors, got {dt}")
+
+
+def dtype_code(t: torch.Tensor) -> int:
+    return type_code(t.dtype)
 
 
 def ptr(t) -> int | None:

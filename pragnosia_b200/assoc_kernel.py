@@ -11,50 +11,11 @@ from __future__ import annotations
 import torch
 
 from . import ops
+from ._lib import host
 
 
 def _wants_grad(*ts) -> bool:
     return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in ts)
-
-
-class _Prep(torch.autograd.Function):
-    """prep_kernel with its backward kernel, without the operator dispatch a compiled caller needs."""
-
-    @staticmethod
-    def forward(ctx, qp, kp, vp, gl, theta, pos):
-        ctx.save_for_backward(qp, kp, vp, gl, theta, pos)
-        return ops.prep(qp, kp, vp, gl, theta, pos)
-
-    @staticmethod
-    def backward(ctx, dq, dk, dv):
-        qp, kp, vp, gl, theta, pos = ctx.saved_tensors
-        dqp, dkp, dvp, dgl, dth = ops.prep_bwd(qp, kp, vp, gl, theta, pos, dq, dk, dv, want_theta=ctx.needs_input_grad[4])
-        return (dqp.to(qp.dtype), dkp.to(kp.dtype), dvp.to(vp.dtype), None if gl is None else dgl.to(gl.dtype),
-                None if dth is None else dth.to(theta.dtype), None)
-
-
-class _Scan(torch.autograd.Function):
-    """The scan of bf16 operands with all its gradients as one library call each way (train_chunk.cu): (o, final state,
-    state entering each chunk), each of them differentiable. beta None: the plain rule."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, la, beta, S0):
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        la32, be32 = ops._f32c(la), ops._f32c(beta)
-        o, S, sent, W, X = ops.scan_train_fwd(q, k, v, la32, be32, ops._f32c(S0))
-        ctx.save_for_backward(q, k, v, la32, be32, sent, W, X)
-        ctx.set_materialize_grads(False)
-        ctx.types = (la.dtype, None if beta is None else beta.dtype, None if S0 is None else S0.dtype)
-        return o, S, sent
-
-    @staticmethod
-    def backward(ctx, do, dS, dsent):
-        q, k, v, la, beta, sent, W, X = ctx.saved_tensors
-        lt, bt, st = ctx.types
-        do = torch.zeros_like(q) if do is None else do
-        dq, dk, dv, dla, dbe, dS0 = ops.scan_train_bwd(q, k, v, la, beta, sent, W, X, do, dsent, dS,
-                                                       want_dS0=st is not None and ctx.needs_input_grad[5])
-        return dq, dk, dv, dla.to(lt), None if dbe is None else dbe.to(bt), None if dS0 is None else dS0.to(st)
 
 
 def prep_kernel(qp, kp, vp, gate_logits, theta, pos):
@@ -62,7 +23,7 @@ def prep_kernel(qp, kp, vp, gate_logits, theta, pos):
     positions. Returns bf16 q, k, v as (B,H,T,D). Differentiable (the backward kernel of src/assoc_kernel.py:774-826)."""
     if _wants_grad(qp, kp, vp, gate_logits, theta):
         if not torch.compiler.is_compiling():
-            return _Prep.apply(qp, kp, vp, gate_logits, theta, pos)
+            return host().prep_diff(qp, kp, vp, gate_logits, theta, pos)
         from . import custom_ops  # noqa: F401
         return tuple(torch.ops.pragnosia_b200.assoc_prep(qp, kp, vp, gate_logits, theta, pos))
     return ops.prep(qp, kp, vp, gate_logits, theta, pos)
@@ -79,12 +40,12 @@ def _chunk_decay(logalpha, T):
 
 def assoc_scan_kernel(q, k, v, logalpha, S0=None, bv: int = 16):
     """Plain rule: (o in q's dtype, final state fp32, state entering each 64-token chunk bf16 (B,H,NC,D,D)).
-    With a gradient wanted, bf16 operands take the fused forward and backward (_Scan); fp32 operands, and a caller being
+    With a gradient wanted, bf16 operands take the fused forward and backward (csrc/torch_host.cpp Scan); fp32 operands, and a caller being
     compiled, the composition of the differentiable operators, as the reference composes it (prefix_scan, then assoc_out:
     src/assoc_kernel.py:302-323). Without: the one fused walk."""
     if _wants_grad(q, k, v, logalpha, S0):
         if not torch.compiler.is_compiling() and ops.scan_trains(q, k, v):
-            return _Scan.apply(q, k, v, logalpha, None, S0)
+            return host().scan_diff(q, k, v, logalpha, None, S0)
         T = q.shape[2]
         pad = (-T) % ops.CHUNK
         a_log, w = _chunk_decay(logalpha, T)
@@ -101,7 +62,7 @@ def delta_scan_kernel(q, k, v, logalpha, beta, S0=None, chunk: int = 64, bv: int
     residuals (src/assoc_kernel.py:512-546)."""
     if _wants_grad(q, k, v, logalpha, beta, S0):
         if not torch.compiler.is_compiling() and ops.scan_trains(q, k, v):
-            return _Scan.apply(q, k, v, logalpha, beta, S0)
+            return host().scan_diff(q, k, v, logalpha, beta, S0)
         NC = (q.shape[2] + ops.CHUNK - 1) // ops.CHUNK
         X = ops.delta_inv(k, logalpha, beta, NC)
         W, sent, S = ops.delta_loop_fwd(k, v, logalpha, beta, X, S0)

@@ -1,6 +1,7 @@
 """Build the CUDA library in-tree: python -m pragnosia_b200.build
 
-One nvcc invocation per source, sm_100a only, then one link into pragnosia_b200/lib/libpragnosia_b200.so.
+One nvcc invocation per source, sm_100a only, then one link into pragnosia_b200/lib/libpragnosia_b200.so; then the torch side of
+the host code (csrc/torch_host.cpp) by the C++ compiler into pragnosia_b200/lib/pgb_torch.so, linked to it.
 Sources are rebuilt only when they (or a header) are newer than their object file.
 """
 from __future__ import annotations
@@ -8,6 +9,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -15,6 +17,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIBDIR = PKG / "lib"
 LIB = LIBDIR / "libpragnosia_b200.so"
+HOST_SRC, HOST = CSRC / "torch_host.cpp", LIBDIR / "pgb_torch.so"
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 
@@ -30,7 +33,29 @@ def _stale(src: Path, obj: Path, headers) -> bool:
     return src.stat().st_mtime > t or any(h.stat().st_mtime > t for h in headers)
 
 
+def build_host(force: bool = False) -> None:
+    """The extension module over torch's C++ API. Its only dependencies beside torch are the library and its header."""
+    deps = [HOST_SRC, PKG.parent / "include" / "pragnosia_b200.h"]
+    if not force and HOST.exists() and all(f.stat().st_mtime <= HOST.stat().st_mtime for f in deps):
+        return
+    from torch.utils import cpp_extension as ext
+    inc = [*ext.include_paths(), str(Path(NVCC).parents[1] / "include"), sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-DTORCH_EXTENSION_NAME={HOST.stem}",
+           "-DTORCH_API_INCLUDE_EXTENSION_H", *(f"-I{d}" for d in inc), str(HOST_SRC), "-o", str(HOST), *(f"-L{d}" for d in ext.library_paths()),
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", f"-L{LIBDIR}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed for {HOST_SRC.name}:\n{r.stdout}\n{r.stderr}")
+    print(f"  linked {HOST.relative_to(PKG.parent)}")
+
+
 def build(verbose: bool = False, force: bool = False) -> Path:
+    build_lib(verbose, force)
+    build_host(force)
+    return LIB
+
+
+def build_lib(verbose: bool = False, force: bool = False) -> Path:
     LIBDIR.mkdir(exist_ok=True)
     headers = list(CSRC.glob("*.cuh")) + list((PKG.parent / "include").glob("*.h"))
     if not force and LIB.exists() and all(f.stat().st_mtime <= LIB.stat().st_mtime for f in sources() + headers):

@@ -73,7 +73,8 @@ def _(g, u, logmag, ang, hr_all, hi_all, g_last_i, want_dh0):
 
 
 class _LambdaScan(torch.autograd.Function):
-    """Differentiable scan (the reference's _Scan, src/scan_kernel.py:105-140): the forward keeps Im h for the adjoint."""
+    """Differentiable scan (the reference's _Scan, src/scan_kernel.py:105-140): the forward keeps Im h for the adjoint.
+    For callers being compiled; an eager one takes the same node in C++ (csrc/torch_host.cpp)."""
 
     @staticmethod
     def forward(ctx, u, logmag, ang, h0r, h0i):

@@ -1,4 +1,6 @@
-"""Tensor-level wrappers of the C ABI: shape checks, output allocation (by torch), one library call each.
+"""Tensor-level wrappers of the C ABI: shape checks, output allocation (by torch), one library call each. Those of the scans
+and the plumbing before them, whose kernels can be shorter than a Python call, have their checks, allocation and library call in
+C++ (csrc/torch_host.cpp, `host()`).
 
 All functions take CUDA tensors, launch on torch's current stream and never synchronise, so they can be captured in a
 CUDA graph. They raise on CPU tensors: there is no fallback path.
@@ -14,10 +16,9 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._lib import check, dtype_code, lib, need_cuda, on_device_of, ptr, stream_of
+from ._lib import check, dtype_code, host, lib, need_cuda, on_device_of, ptr, stream_of, type_code
 
 CHUNK = 64
-FP32_CHUNK_SCRATCH = 8 << 30      # bytes of per-chunk states the fp32 plain prefill may take; beyond (B*H*T > 33 M at D = 64) it walks the chains
 
 
 def _f32c(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -74,75 +75,33 @@ def _norm_args(norm: torch.nn.Module):
 
 
 # ----------------------------------------------------------------------------------------------------------
-def _angle_view(ang, B, T, D):
-    """The angle as fp32 with unit stride over D and either zero (batch, time) strides -- one angle per channel, read as
-    such -- or the dense strides."""
-    a32 = ang if ang.dtype == torch.float32 else ang.to(torch.float32)
-    if a32.dim() == 1:
-        a32 = a32.expand(B, T, D)
-    if tuple(a32.shape) != (B, T, D):
-        raise ValueError("lambda_scan: u, logmag, ang must share the shape (B,T,D)")
-    if D > 1 and a32.stride(2) != 1:
-        a32 = a32.contiguous()
-    sb, st = (a32.stride(0) if B > 1 else 0), (a32.stride(1) if T > 1 else 0)
-    if not (sb == 0 and st == 0) and not (st == D and sb == T * D):
-        a32 = a32.contiguous(); sb, st = T * D, D
-    return a32, sb, st
-
-
-@on_device_of
 def lambda_scan(u: torch.Tensor, logmag: torch.Tensor, ang: torch.Tensor, h0=None, time_segments: int = 0,
                 keep_imag: bool = False):
     """h_t = lambda_t h_{t-1} + u_t with lambda_t = exp(logmag_t + i ang_t); returns (Re h (B,T,D) fp32,
     (Re h_T, Im h_T)).  `ang` may be an expanded view with zero batch/time strides (one angle per channel): it is
     read as such, not materialised.  keep_imag: also return Im h for every token as a third value (what the
     backward pass needs)."""
-    need_cuda(u, logmag, ang)
-    B, T, D = u.shape
-    u32, lm32 = _f32c(u), _f32c(logmag)
-    if tuple(lm32.shape) != (B, T, D):
-        raise ValueError("lambda_scan: u, logmag, ang must share the shape (B,T,D)")
-    h0r = h0i = None
-    if h0 is not None:
-        h0r, h0i = _f32c(h0[0]), _f32c(h0[1])
-        need_cuda(h0r, h0i)
+    h0r, h0i = (None, None) if h0 is None else h0
     if _compiling():
-        y, hr, hi, hia = _cops().lambda_scan(u32, lm32, ang, h0r, h0i, int(time_segments), bool(keep_imag))
-        return (y, (hr, hi), hia) if keep_imag else (y, (hr, hi))
-    a32, sb, st = _angle_view(ang, B, T, D)
-    y = torch.empty(B, T, D, device=u.device, dtype=torch.float32)
-    hr = torch.empty(B, D, device=u.device, dtype=torch.float32)
-    hi = torch.empty_like(hr)
-    if keep_imag:
-        hia = torch.empty_like(y)
-        check(lib().pgb_lambda_scan_fwd_train(ptr(u32), ptr(lm32), ptr(a32), sb, st, ptr(h0r), ptr(h0i), ptr(y), ptr(hia), ptr(hr),
-                                              ptr(hi), B, T, D, stream_of(u)), "pgb_lambda_scan_fwd_train")
-        return y, (hr, hi), hia
-    check(lib().pgb_lambda_scan_fwd_ex(ptr(u32), ptr(lm32), ptr(a32), sb, st, ptr(h0r), ptr(h0i), ptr(y), ptr(hr), ptr(hi),
-                                       B, T, D, time_segments, stream_of(u)), "pgb_lambda_scan_fwd")
-    return y, (hr, hi)
+        need_cuda(u, logmag, ang, h0r, h0i)
+        if tuple(logmag.shape) != tuple(u.shape):
+            raise ValueError("lambda_scan: u, logmag, ang must share the shape (B,T,D)")
+        y, hr, hi, hia = _cops().lambda_scan(_f32c(u), _f32c(logmag), ang, _f32c(h0r), _f32c(h0i), int(time_segments), bool(keep_imag))
+    else:
+        y, hr, hi, hia = host().lambda_scan(u, logmag, ang, h0r, h0i, time_segments, keep_imag)
+    return (y, (hr, hi), hia) if keep_imag else (y, (hr, hi))
 
 
-@on_device_of
 def lambda_scan_bwd(g, u, logmag, ang, hr_all, hi_all, g_last_i=None, want_dh0: bool = False):
     """Adjoint of lambda_scan: g (B,T,D) is the gradient on Re h (the gradient on the final Re state already added to its
     last row), g_last_i (B,D) the gradient on the final Im state. Returns (du, dlogmag, dang, dh0r, dh0i); the last two
     are None unless want_dh0."""
-    need_cuda(g, u, logmag, ang, hr_all, hi_all)
-    B, T, D = u.shape
-    g, u, logmag, hr_all, hi_all = (_f32c(t) for t in (g, u, logmag, hr_all, hi_all))
-    gli = _f32c(g_last_i)
     if _compiling():
-        du, dlm, dan, d0r, d0i = _cops().lambda_scan_bwd(g, u, logmag, ang, hr_all, hi_all, gli, bool(want_dh0))
+        need_cuda(g, u, logmag, ang, hr_all, hi_all)
+        g, u, logmag, hr_all, hi_all = (_f32c(t) for t in (g, u, logmag, hr_all, hi_all))
+        du, dlm, dan, d0r, d0i = _cops().lambda_scan_bwd(g, u, logmag, ang, hr_all, hi_all, _f32c(g_last_i), bool(want_dh0))
         return du, dlm, dan, _opt(d0r), _opt(d0i)
-    a32, sb, st = _angle_view(ang, B, T, D)
-    du = torch.empty(B, T, D, device=u.device, dtype=torch.float32)
-    dlm, dan = torch.empty_like(du), torch.empty_like(du)
-    d0r = torch.empty(B, D, device=u.device, dtype=torch.float32) if want_dh0 else None
-    d0i = torch.empty_like(d0r) if want_dh0 else None
-    check(lib().pgb_lambda_scan_bwd(ptr(g), ptr(u), ptr(logmag), ptr(a32), sb, st, ptr(hr_all), ptr(hi_all), ptr(gli), ptr(du),
-                                    ptr(dlm), ptr(dan), ptr(d0r), ptr(d0i), B, T, D, stream_of(u)), "pgb_lambda_scan_bwd")
-    return du, dlm, dan, d0r, d0i
+    return host().lambda_scan_bwd(g, u, logmag, ang, hr_all, hi_all, g_last_i, want_dh0)
 
 
 # ----------------------------------------------------------------------------------------------------------
@@ -168,100 +127,47 @@ def _prep_views(qp, kp, vp, gate_logits):
     return qp, kp, vp, gate_logits
 
 
-@on_device_of
 def prep(qp, kp, vp, gate_logits, theta, pos, out_dtype=torch.bfloat16):
     """Normalise / gate / rotate / cast / transpose: (B,T,H,D) projections -> (B,H,T,D) scan operands."""
+    if not _compiling():
+        return host().prep(qp, kp, vp, gate_logits, theta, pos, type_code(out_dtype) == _lib.BF16)
     need_cuda(qp, kp, vp, theta, pos)
-    B, T, H, D = qp.shape
     qp, kp, vp, gate_logits = _prep_views(qp, kp, vp, gate_logits)
-    theta = _f32c(theta)
-    pos = pos.to(torch.int64).contiguous()
-    if _compiling():
-        return tuple(_cops().assoc_prep_ex(qp, kp, vp, gate_logits, theta, pos, out_dtype == torch.bfloat16))
-    gsb, gst = (0, 0) if gate_logits is None else (gate_logits.stride(0), gate_logits.stride(1))
-    q = torch.empty(B, H, T, D, device=qp.device, dtype=out_dtype)
-    k, v = torch.empty_like(q), torch.empty_like(q)
-    check(lib().pgb_aspin_prep_fwd(ptr(qp), ptr(kp), ptr(vp), dtype_code(qp), qp.stride(0), qp.stride(1), qp.stride(2),
-                                   ptr(gate_logits), gsb, gst, ptr(theta), ptr(pos), ptr(q), ptr(k), ptr(v), dtype_code(q),
-                                   B, T, H, D, stream_of(qp)), "pgb_aspin_prep_fwd")
-    return q, k, v
+    return tuple(_cops().assoc_prep_ex(qp, kp, vp, gate_logits, _f32c(theta), pos.to(torch.int64).contiguous(), out_dtype == torch.bfloat16))
 
 
-@on_device_of
 def prep_bwd(qp, kp, vp, gate_logits, theta, pos, dq, dk, dv, want_theta: bool = True):
     """Gradient of prep: returns (dqp, dkp, dvp in the projections' dtype, contiguous (B,T,H,D); dgate (B,T,H) fp32 or
     None; dtheta (H,D/2) fp32, None unless want_theta)."""
+    if not _compiling():
+        return host().prep_bwd(qp, kp, vp, gate_logits, theta, pos, dq, dk, dv, want_theta)
     need_cuda(qp, kp, vp, theta, pos, dq, dk, dv)
-    B, T, H, D = qp.shape
     qp, kp, vp, gate_logits = _prep_views(qp, kp, vp, gate_logits)
-    theta = _f32c(theta)
-    pos = pos.to(torch.int64).contiguous()
     if dq.dtype not in (torch.float32, torch.bfloat16):
         dq = dq.float()
     dq, dk, dv = dq.contiguous(), dk.to(dq.dtype).contiguous(), dv.to(dq.dtype).contiguous()
-    if _compiling():
-        dqp, dkp, dvp, dgl, dth = _cops().assoc_prep_bwd(qp, kp, vp, gate_logits, theta, pos, dq, dk, dv)
-        return dqp, dkp, dvp, _opt(dgl), dth
-    gsb, gst = (0, 0) if gate_logits is None else (gate_logits.stride(0), gate_logits.stride(1))
-    dqp = torch.empty(B, T, H, D, device=qp.device, dtype=qp.dtype)
-    dkp, dvp = torch.empty_like(dqp), torch.empty_like(dqp)
-    dgl = None if gate_logits is None else torch.empty(B, T, H, device=qp.device, dtype=torch.float32)
-    part = torch.empty(B * lib().pgb_aspin_prep_bwd_tiles(T), H, D // 2, device=qp.device, dtype=torch.float32) if want_theta else None
-    check(lib().pgb_aspin_prep_bwd(ptr(qp), ptr(kp), ptr(vp), dtype_code(qp), qp.stride(0), qp.stride(1), qp.stride(2),
-                                   ptr(gate_logits), gsb, gst, ptr(theta), ptr(pos), ptr(dq), ptr(dk), ptr(dv), dtype_code(dq),
-                                   ptr(dqp), ptr(dkp), ptr(dvp), ptr(dgl), ptr(part), B, T, H, D, stream_of(qp)),
-          "pgb_aspin_prep_bwd")
-    return dqp, dkp, dvp, dgl, (part.sum(0) if want_theta else None)
+    dqp, dkp, dvp, dgl, dth = _cops().assoc_prep_bwd(qp, kp, vp, gate_logits, _f32c(theta), pos.to(torch.int64).contiguous(), dq, dk, dv)
+    return dqp, dkp, dvp, _opt(dgl), dth
 
 
-# ----------------------------------------------------------------------------------------------------------
-@on_device_of
 def prefill(q, k, v, la, beta=None, S0=None, theta=None, shift=0.0, want_sent: bool = False,
             precision: int = _lib.PREFILL_AUTO, out_dtype=None, S_out=None):
     """Chunked prefill. q,k,v (B,H,T,D) fp32 or bf16 (same dtype); la (B,H,T); beta (B,H,T) or None (plain rule);
     S0 (B,H,D,D) or None.  theta/shift: rebase S0's key axis by -shift*theta first (shift: number or 0-d CUDA tensor).
     Returns (o in out_dtype (default q's dtype), S fp32, sent bf16 (B,H,NC,D,D) or None)."""
+    theta, shift_dev, shift_host = _shift_args(theta, S0, shift)
+    if not _compiling():
+        return host().prefill(q, k, v, la, beta, S0, theta, shift_dev, shift_host, want_sent, precision,
+                              -1 if out_dtype is None else type_code(out_dtype), S_out)
     need_cuda(q, k, v, la)
-    B, H, T, D = q.shape
     if q.dtype not in (torch.float32, torch.bfloat16):
         q = q.float()
     q, k, v = _like(q, q), _like(k, q), _like(v, q)
-    la, beta, S0 = _f32c(la), _f32c(beta), _f32c(S0)
-    theta, shift_dev, shift_host = _shift_args(theta, S0, shift)
-    if shift_dev is not None:
-        need_cuda(shift_dev)
-    odt = out_dtype or q.dtype
-    if _compiling():
-        o, S, sent = _cops().aspin_prefill(q, k, v, la, beta, S0, theta, shift_dev, shift_host, bool(want_sent), int(precision),
-                                           odt == torch.float32)
-        return o, S, _opt(sent)
-    o = torch.empty(B, H, T, D, device=q.device, dtype=odt)
-    S = _state_out(S_out, B, H, D, q.device)
-    NC = (T + CHUNK - 1) // CHUNK
-    sent = torch.empty(B, H, NC, D, D, device=q.device, dtype=torch.bfloat16) if want_sent else None
-    if beta is not None and q.dtype == torch.bfloat16 and precision != _lib.PREFILL_FP32 and B * H <= 65535:
-        # delta rule on the tensor cores: the chunk inverses go through a scratch buffer (allocated here, by torch)
-        nbytes = lib().pgb_aspin_delta_scratch_bytes(B, H, T)
-        scratch = torch.empty(nbytes, device=q.device, dtype=torch.uint8)
-        check(lib().pgb_aspin_delta_prefill_fwd(ptr(q), ptr(k), ptr(v), ptr(la), ptr(beta), ptr(S0), ptr(theta), ptr(shift_dev),
-                                                shift_host, ptr(o), dtype_code(o), ptr(S), ptr(sent), ptr(scratch), nbytes,
-                                                B, H, T, D, stream_of(q)), "pgb_aspin_delta_prefill_fwd")
-        return o, S, sent
-    if beta is None and q.dtype == torch.float32 and precision != _lib.PREFILL_TENSOR and B * H <= 65535:
-        nbytes = lib().pgb_aspin_prefill_fp32_scratch_bytes(B, H, T, D)      # fp32 plain rule: the chunks side by side
-        if nbytes <= FP32_CHUNK_SCRATCH:
-            scratch = torch.empty(nbytes, device=q.device, dtype=torch.uint8)
-            check(lib().pgb_aspin_prefill_fp32_fwd(ptr(q), ptr(k), ptr(v), ptr(la), ptr(S0), ptr(theta), ptr(shift_dev), shift_host, ptr(o),
-                                                   dtype_code(o), ptr(S), ptr(sent), ptr(scratch), nbytes, B, H, T, D, stream_of(q)),
-                  "pgb_aspin_prefill_fp32_fwd")
-            return o, S, sent
-    check(lib().pgb_aspin_prefill_fwd(ptr(q), ptr(k), ptr(v), dtype_code(q), ptr(la), ptr(beta), ptr(S0), ptr(theta),
-                                      ptr(shift_dev), shift_host, ptr(o), dtype_code(o), ptr(S), ptr(sent), B, H, T, D, precision,
-                                      stream_of(q)), "pgb_aspin_prefill_fwd")
-    return o, S, sent
+    o, S, sent = _cops().aspin_prefill(q, k, v, _f32c(la), _f32c(beta), _f32c(S0), theta, shift_dev, shift_host, bool(want_sent), int(precision),
+                                       (out_dtype or q.dtype) == torch.float32)
+    return o, S, _opt(sent)
 
 
-# ----------------------------------------------------------------------------------------------------------
 @on_device_of
 def prefill_fused(q, k, v, decay_logits, decay_A, S0=None, theta=None, shift=0.0, rms_weight=None, rms_eps=0.0,
                   want_sent: bool = False, out_dtype=None, S_out=None):
@@ -810,40 +716,15 @@ def scan_trains(q, k, v) -> bool:
     return q.is_cuda and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.shape[-1] in (64, 128) and q.shape[0] * q.shape[1] <= 65535
 
 
-@on_device_of
 def scan_train_fwd(q, k, v, la, beta=None, S0=None):
     """The scan with what its backward reads: (o, S, sent, W or None, X scratch or None); bf16 q, k, v (B,H,T,D) contiguous,
     la / beta fp32 contiguous."""
-    if beta is None:
-        o, S, sent = prefill(q, k, v, la, None, S0, want_sent=True, precision=_lib.PREFILL_TENSOR)
-        return o, S, sent, None, None
-    B, H, T, D = q.shape
-    o, W = torch.empty_like(q), torch.empty_like(q)
-    S = torch.empty(B, H, D, D, device=q.device, dtype=torch.float32)
-    sent = torch.empty(B, H, (T + CHUNK - 1) // CHUNK, D, D, device=q.device, dtype=torch.bfloat16)
-    nbytes = lib().pgb_aspin_delta_scratch_bytes(B, H, T)
-    X = torch.empty(nbytes, device=q.device, dtype=torch.uint8)
-    check(lib().pgb_aspin_delta_prefill_train_fwd(ptr(q), ptr(k), ptr(v), ptr(la), ptr(beta), ptr(S0), ptr(o), ptr(S), ptr(sent), ptr(W),
-                                                  ptr(X), nbytes, B, H, T, D, stream_of(q)), "pgb_aspin_delta_prefill_train_fwd")
-    return o, S, sent, W, X
+    return host().scan_train_fwd(q, k, v, la, beta, S0)
 
 
-@on_device_of
 def scan_train_bwd(q, k, v, la, beta, sent, W, X, dout, dsent=None, dS=None, want_dS0: bool = False):
     """Gradients of scan_train_fwd: (dq, dk, dv bf16, dla, dbeta or None, dS0 or None fp32)."""
-    B, H, T, D = q.shape
-    dout = dout.to(torch.bfloat16).contiguous()
-    dsent, dS = _f32c(dsent), _f32c(dS)
-    dq, dk, dv = torch.empty_like(q), torch.empty_like(q), torch.empty_like(q)
-    dla = torch.empty(B, H, T, device=q.device, dtype=torch.float32)
-    dbe = None if beta is None else torch.empty_like(dla)
-    dS0 = torch.empty(B, H, D, D, device=q.device, dtype=torch.float32) if want_dS0 else None
-    nbytes = lib().pgb_aspin_train_scratch_bytes(B, H, T, D, int(beta is not None))
-    scratch = torch.empty(nbytes, device=q.device, dtype=torch.uint8)
-    check(lib().pgb_aspin_train_bwd(ptr(q), ptr(k), ptr(v), ptr(la), ptr(beta), ptr(sent), ptr(W), ptr(X), ptr(dout), ptr(dsent), ptr(dS),
-                                    ptr(dq), ptr(dk), ptr(dv), ptr(dla), ptr(dbe), ptr(dS0), ptr(scratch), nbytes, B, H, T, D,
-                                    stream_of(q)), "pgb_aspin_train_bwd")
-    return dq, dk, dv, dla, dbe, dS0
+    return host().scan_train_bwd(q, k, v, la, beta, sent, W, X, dout, dsent, dS, want_dS0)
 
 
 # ---------------------------------------------------------------------------------------------------------- layer options
