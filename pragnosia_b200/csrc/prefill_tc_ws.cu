@@ -5,9 +5,9 @@
 //                        chain of shuffles and exponentials that nothing has to wait for when it runs ahead.
 //   front  (warps 0-7)   chunk c+1: the plumbing on the TMA tiles (RAW mode: normalise, gate, rotate) and K*w head/tail --
 //                        all shared memory to shared memory, no tensor-memory access.
-//   issuer (warp 24)     one thread: TMA loads three chunks ahead, and the tcgen05.mma stream
+//   issuer (warp 24)     TMA loads three chunks ahead, and the tcgen05.mma stream
 //                        P(c+1) = Q K^T, U(c+1) = (K w)^T V   as soon as the front is done with chunk c+1.
-//   issuer (warp 27)     one thread (a single thread issues an MMA only every few tens of cycles):
+//   issuer (warp 27)     (both issuers stay converged and elect a lane per instruction: see mma_bf16_elect)
 //                        O2(c) = Q S_c                         as soon as S_c is in shared memory,
 //                        O1(c) = A V                           as soon as A(c) is.
 //   back   (warps 8-15)  chunk c: scores -> A (decay mask, head/tail), S_{c+1} = e^{L_C} S_c + U in registers and to shared
@@ -363,16 +363,30 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
 #pragma unroll
             for (int hi8 = 0; hi8 < 2; ++hi8) {
                 const int trow = hi8 ? row1 : row0;
-                if (t0 + trow < T) {
-                    const float sc = hi8 ? sc1 : sc0;
-                    const size_t row = p.o_token_major ? ((size_t)b * p.T + tb + t0 + trow) * p.H + h : (size_t)bh * p.T + tb + t0 + trow;
-                    const size_t off = row * D + col0 + 2 * fq;
+                const float sc = hi8 ? sc1 : sc0;
+                const size_t row = p.o_token_major ? ((size_t)b * p.T + tb + t0 + trow) * p.H + h : (size_t)bh * p.T + tb + t0 + trow;
+                const size_t off = row * D + col0;
+                float x[8];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        float x0 = ov[4 * j + 2 * hi8] * sc, x1 = ov[4 * j + 2 * hi8 + 1] * sc;
-                        if (p.rms_w != nullptr) { x0 *= rmsw[col0 + 8 * j + 2 * fq]; x1 *= rmsw[col0 + 8 * j + 2 * fq + 1]; }
-                        if (p.o_is_f32) *reinterpret_cast<float2 *>((float *)p.o + off + 8 * j) = make_float2(x0, x1);
-                        else *reinterpret_cast<__nv_bfloat162 *>((__nv_bfloat16 *)p.o + off + 8 * j) = __floats2bfloat162_rn(x0, x1);
+                for (int j = 0; j < 4; ++j) {
+                    x[2 * j] = ov[4 * j + 2 * hi8] * sc; x[2 * j + 1] = ov[4 * j + 2 * hi8 + 1] * sc;
+                    if (p.rms_w != nullptr) { x[2 * j] *= rmsw[col0 + 8 * j + 2 * fq]; x[2 * j + 1] *= rmsw[col0 + 8 * j + 2 * fq + 1]; }
+                }
+                if (p.o_is_f32) {
+                    if (t0 + trow < T)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) *reinterpret_cast<float2 *>((float *)p.o + off + 8 * j + 2 * fq) = make_float2(x[2 * j], x[2 * j + 1]);
+                } else {
+                    // neighbouring lanes trade column pairs, so that a lane stores four columns and a row's quad 32 bytes: a whole
+                    // memory sector per store instead of half of one
+#pragma unroll
+                    for (int j = 0; j < 4; j += 2) {
+                        const __nv_bfloat162 e = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]), o = __floats2bfloat162_rn(x[2 * j + 2], x[2 * j + 3]);
+                        const uint32_t ev = *reinterpret_cast<const uint32_t *>(&e), od = *reinterpret_cast<const uint32_t *>(&o);
+                        const uint32_t got = __shfl_xor_sync(0xffffffffu, (fq & 1) ? ev : od, 1);
+                        const uint2 pair = (fq & 1) ? make_uint2(got, od) : make_uint2(ev, got);
+                        if (t0 + trow < T)
+                            *reinterpret_cast<uint2 *>((__nv_bfloat16 *)p.o + off + 8 * (j + (fq & 1)) + 4 * (fq >> 1)) = pair;
                     }
                 }
             }
@@ -427,96 +441,81 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_stats(c & 3));
         }
-    } else if (warp == WS_ISSUER && lane == 0) {
+    } else if (warp == WS_ISSUER) {
         // =========================================================================================== issuer: loads, P, U
         constexpr uint32_t I_P = idesc_bf16(64, 64, 0, 0), I_U = idesc_bf16(64, 64, 1, 1);
         auto load_chunk = [&](int c) {
             const int s3 = c % 3;
             const uint32_t sb = base + SM::off_stage + s3 * STAGE_BYTES;
-            mbar_expect_tx(bar_full(s3), STAGE_BYTES);
-            tma_load_3d(sb, &mq, bar_full(s3), tma_c0, tb + c * TC_C, tma_c2);
-            tma_load_3d(sb + SM::TILE, &mk, bar_full(s3), tma_c0, tb + c * TC_C, tma_c2);
-            tma_load_3d(sb + 2 * SM::TILE, &mv, bar_full(s3), tma_c0, tb + c * TC_C, tma_c2);
+            if (lane == 0) {
+                mbar_expect_tx(bar_full(s3), STAGE_BYTES);
+                tma_load_3d(sb, &mq, bar_full(s3), tma_c0, tb + c * TC_C, tma_c2);
+                tma_load_3d(sb + SM::TILE, &mk, bar_full(s3), tma_c0, tb + c * TC_C, tma_c2);
+                tma_load_3d(sb + 2 * SM::TILE, &mv, bar_full(s3), tma_c0, tb + c * TC_C, tma_c2);
+            }
+            __syncwarp();
         };
         auto load_rot = [&](int c) {
-            if (!RAW) return;
-            mbar_expect_tx(bar_rot(c & 1), ROT_BYTES);
-            bulk_load_1d(base + SM::off_rot + (c & 1) * ROT_BYTES, p.rot + ((size_t)h * p.rot_T + (size_t)c * TC_C) * (D / 2), ROT_BYTES,
-                         bar_rot(c & 1));
-        };
-        int tma_c = 0, pu_c = 0;
-        for (; tma_c < 3 && tma_c < NC; ++tma_c) load_chunk(tma_c);
-        for (int c = 0; c < 2 && c < NC; ++c) load_rot(c);
-        uint32_t idle = 0;
-        while (pu_c < NC) {
-            bool progress = false;
-            if (tma_c < NC && mbar_test(bar_empty(tma_c % 3), ((tma_c / 3) + 1) & 1)) { load_chunk(tma_c); ++tma_c; progress = true; }
-            if (mbar_test(bar_ready(pu_c & 1), (pu_c >> 1) & 1)) {
-                const int c = pu_c, s2 = c & 1;
-                const uint32_t sb = base + SM::off_stage + (c % 3) * STAGE_BYTES;
-                const uint64_t dq = smem_desc(sb, 16, 1024), dk = smem_desc(sb + SM::TILE, 16, 1024), dv = smem_desc(sb + 2 * SM::TILE, 8192, 1024);
-                const uint64_t dkwh = smem_desc(base + SM::off_kw + s2 * 2 * SM::TILE, 8192, 1024), dkwl = dkwh + (SM::TILE >> 4);
-                tc_fence_after();
-#pragma unroll
-                for (int k = 0; k < 4; ++k) mma_bf16(tmem + TM_P + 64 * s2, dq + k * 2, dk + k * 2, I_P, k > 0);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) mma_bf16(tmem + TM_U + 64 * s2, dkwh + k * 128, dv + k * 128, I_U, k > 0);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) mma_bf16(tmem + TM_U + 64 * s2, dkwl + k * 128, dv + k * 128, I_U, 1);
-                mma_commit(bar_pu(s2));
-                mma_commit(bar_empty(c % 3));                         // this issuer's half: P and U have read the chunk's tiles
-                mbar_arrive(bar_q(c & 3));                            // the other issuer may use the chunk's Q and V tiles
-                if (c + 2 < NC) load_rot(c + 2);                      // the front is done with this slot's rotation rows
-                ++pu_c; progress = true;
+            if (RAW && lane == 0) {
+                mbar_expect_tx(bar_rot(c & 1), ROT_BYTES);
+                bulk_load_1d(base + SM::off_rot + (c & 1) * ROT_BYTES, p.rot + ((size_t)h * p.rot_T + (size_t)c * TC_C) * (D / 2), ROT_BYTES,
+                             bar_rot(c & 1));
             }
-            if (progress) idle = 0;
-            else {
-                if (++idle > (TC_WAIT_LIMIT >> 2)) { atomicExch(&g_tc_error, 51); break; }
-                __nanosleep(20);                                      // leave the issue slots to the working warps
+            __syncwarp();
+        };
+        for (int c = 0; c < 3 && c < NC; ++c) load_chunk(c);
+        for (int c = 0; c < 2 && c < NC; ++c) load_rot(c);
+        for (int c = 0; c < NC; ++c) {
+            const int s2 = c & 1;
+            if (!mbar_wait_warp(bar_ready(s2), (c >> 1) & 1, 51)) break;
+            const uint32_t sb = base + SM::off_stage + (c % 3) * STAGE_BYTES;
+            const uint64_t dq = smem_desc(sb, 16, 1024), dk = smem_desc(sb + SM::TILE, 16, 1024), dv = smem_desc(sb + 2 * SM::TILE, 8192, 1024);
+            const uint64_t dkwh = smem_desc(base + SM::off_kw + s2 * 2 * SM::TILE, 8192, 1024), dkwl = dkwh + (SM::TILE >> 4);
+            tc_fence_after();
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem + TM_P + 64 * s2, dq + k * 2, dk + k * 2, I_P, k > 0);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem + TM_U + 64 * s2, dkwh + k * 128, dv + k * 128, I_U, k > 0);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem + TM_U + 64 * s2, dkwl + k * 128, dv + k * 128, I_U, 1);
+            mma_commit_elect(bar_pu(s2));
+            mma_commit_elect(bar_empty(c % 3));                       // this issuer's half: P and U have read the chunk's tiles
+            if (lane == 0) mbar_arrive(bar_q(c & 3));                 // the other issuer may use the chunk's Q and V tiles
+            if (c + 2 < NC) load_rot(c + 2);                          // the front is done with this slot's rotation rows
+            // chunk c+2's tiles go where chunk c-1's were. Its products finish about when the front is done with chunk c+1 (both
+            // follow the back's reading of chunk c-1), so this wait holds up nothing the next one would not
+            if (c >= 1 && c + 2 < NC) {
+                if (!mbar_wait_warp(bar_empty((c + 2) % 3), ((c + 2) / 3 + 1) & 1, 53)) break;
+                load_chunk(c + 2);
             }
         }
-        // the last loads were issued inside the loop: tma_c == NC by the time pu_c == NC (a chunk's P, U need its tiles)
-    } else if (warp == WS_ISSUER_O && lane == 0) {
+    } else if (warp == WS_ISSUER_O) {
         // =========================================================================================== issuer: O2, O1
         constexpr uint32_t I_O = idesc_bf16(64, 64, 0, 1);
-        int q_c = 0, o2_c = 0, o1_c = 0;
-        uint32_t idle = 0;
-        while (o1_c < NC) {
-            bool progress = false;
-            // bar_q has four slots: its completion c+4 needs the back at chunk c+2, which needs O1(c) from this loop,
-            // so this thread is never two phases behind it
-            if (q_c < NC && mbar_test(bar_q(q_c & 3), (q_c >> 2) & 1)) { ++q_c; progress = true; }
-            // O2(c) and O1(c) go to tensor-memory slot c&1, which the tail has drained once chunk c-2 is finished
-            if (o2_c < q_c && mbar_test(bar_s(o2_c & 1), (o2_c >> 1) & 1) &&
-                (o2_c < 2 || mbar_test(bar_done((o2_c - 2) & 3), ((o2_c - 2) >> 2) & 1))) {
-                const int c = o2_c;
-                const uint64_t dq = smem_desc(base + SM::off_stage + (c % 3) * STAGE_BYTES, 16, 1024);
-                const uint64_t dsh = smem_desc(base + SM::off_s + (c & 1) * 2 * SM::TILE, 16, 1024), dsl = dsh + (SM::TILE >> 4);
-                tc_fence_after();
+        for (int c = 0; c < NC; ++c) {
+            const uint32_t sb = base + SM::off_stage + (c % 3) * STAGE_BYTES;
+            // bar_q has four slots: its completion c+4 needs the back at chunk c+2, which needs O1(c) from this loop, so this
+            // warp is never two phases behind it. O2(c) and O1(c) go to tensor-memory slot c&1, which the tail has drained
+            // once chunk c-2 is finished. S_{c+1} is published behind A(c), so O1(c) before O2(c+1) holds up nothing.
+            if (!(mbar_wait_warp(bar_q(c & 3), (c >> 2) & 1, 52) && (c < 2 || mbar_wait_warp(bar_done((c - 2) & 3), ((c - 2) >> 2) & 1, 54)) &&
+                  mbar_wait_warp(bar_s(c & 1), (c >> 1) & 1, 55))) break;
+            const uint64_t dq = smem_desc(sb, 16, 1024);
+            const uint64_t dsh = smem_desc(base + SM::off_s + (c & 1) * 2 * SM::TILE, 16, 1024), dsl = dsh + (SM::TILE >> 4);
+            tc_fence_after();
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma_bf16(tmem + TM_O2 + 64 * (c & 1), dq + k * 2, dsh + k * 128, I_O, k > 0);
+            for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem + TM_O2 + 64 * (c & 1), dq + k * 2, dsh + k * 128, I_O, k > 0);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma_bf16(tmem + TM_O2 + 64 * (c & 1), dq + k * 2, dsl + k * 128, I_O, 1);
-                ++o2_c; progress = true;
-            }
-            if (o1_c < o2_c && mbar_test(bar_a(o1_c & 1), (o1_c >> 1) & 1)) {
-                const int c = o1_c;
-                const uint64_t dv = smem_desc(base + SM::off_stage + (c % 3) * STAGE_BYTES + 2 * SM::TILE, 8192, 1024);
-                const uint64_t dah = smem_desc(base + SM::off_a + (c & 1) * 2 * SM::TILE, 16, 1024), dal = dah + (SM::TILE >> 4);
-                tc_fence_after();
+            for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem + TM_O2 + 64 * (c & 1), dq + k * 2, dsl + k * 128, I_O, 1);
+            if (!mbar_wait_warp(bar_a(c & 1), (c >> 1) & 1, 56)) break;
+            const uint64_t dv = smem_desc(sb + 2 * SM::TILE, 8192, 1024);
+            const uint64_t dah = smem_desc(base + SM::off_a + (c & 1) * 2 * SM::TILE, 16, 1024), dal = dah + (SM::TILE >> 4);
+            tc_fence_after();
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma_bf16(tmem + TM_O1 + 64 * (c & 1), dah + k * 2, dv + k * 128, I_O, k > 0);
+            for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem + TM_O1 + 64 * (c & 1), dah + k * 2, dv + k * 128, I_O, k > 0);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma_bf16(tmem + TM_O1 + 64 * (c & 1), dal + k * 2, dv + k * 128, I_O, 1);
-                mma_commit(bar_o(c & 1));
-                mma_commit(bar_empty(c % 3));                         // this issuer's half: O2 and O1 have read the chunk's tiles
-                ++o1_c; progress = true;
-            }
-            if (progress) idle = 0;
-            else {
-                if (++idle > (TC_WAIT_LIMIT >> 2)) { atomicExch(&g_tc_error, 52); break; }
-                __nanosleep(20);
-            }
+            for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem + TM_O1 + 64 * (c & 1), dal + k * 2, dv + k * 128, I_O, 1);
+            mma_commit_elect(bar_o(c & 1));
+            mma_commit_elect(bar_empty(c % 3));                       // this issuer's half: O2 and O1 have read the chunk's tiles
         }
     }
     tc_fence_before();
