@@ -48,6 +48,11 @@ __device__ __forceinline__ void decode_step_body(const DecodeArgs &a, int b, int
         if (shift != 0.f) sincosf(-shift * a.theta[(size_t)h * (D / 2) + rg + p * NRG], &rsn[p], &rcs[p]);
     }
 
+    // the constants of the head as well: a load behind the wait costs a round trip of its own on the path of the step
+    const float onw = a.rms_w != nullptr && tid < D ? a.rms_w[tid] : 1.f;
+    const bool raw_decay = a.decay_A != nullptr;
+    const float expA = warp == 3 && raw_decay ? expf(a.decay_A[h]) : 1.f;
+
     if (!between()) return;
 
     // ---- vectors: load, normalise (warps 0,1,2 take q,k,v), scalars (warp 3)
@@ -62,14 +67,14 @@ __device__ __forceinline__ void decode_step_body(const DecodeArgs &a, int b, int
 #pragma unroll
         for (int i = 0; i < D / 32; ++i) dst[lane + 32 * i] = x[i] * inv;
     } else if (warp == 3 && lane == 0) {
-        float d = to_f32(((const TIN *)a.decay)[(size_t)b * a.decay_sb + h]);
-        if (a.decay_A != nullptr) d = -softplusf_(d) * expf(a.decay_A[h]);
+        // both loads before either is used
+        const TIN *dp = (const TIN *)a.decay + (size_t)b * a.decay_sb + h, *gp = a.gate != nullptr ? (const TIN *)a.gate + (size_t)b * a.gate_sb + h : dp;
+        const TIN draw = *dp, graw = *gp;
+        float d = to_f32(draw), g = to_f32(graw);
+        if (raw_decay) d = -softplusf_(d) * expA;
         sc[0] = expf(d);
-        float g = 1.f;
-        if (a.gate != nullptr) {
-            g = to_f32(((const TIN *)a.gate)[(size_t)b * a.gate_sb + h]);
-            if (a.gate_is_logit) g = sigmoidf_(g);
-        }
+        if (a.gate == nullptr) g = 1.f;
+        else if (a.gate_is_logit) g = sigmoidf_(g);
         sc[1] = g;
     }
     __syncthreads();
@@ -152,7 +157,7 @@ __device__ __forceinline__ void decode_step_body(const DecodeArgs &a, int b, int
             sc[2] = rsqrtf(tot / (float)D + a.rms_eps);
         }
         __syncthreads();
-        if (tid < D) oj = oj * sc[2] * a.rms_w[tid];
+        if (tid < D) oj = oj * sc[2] * onw;
     }
     if (tid < D) {
         TOUT *o = (TOUT *)a.o + (size_t)b * a.out_sb + (size_t)h * D;

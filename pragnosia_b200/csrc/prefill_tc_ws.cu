@@ -234,21 +234,28 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
                 }
             }
         }
+        // A fragment is four 8 x 8 matrices per two column blocks (rows row0.., row1.., of each block): stmatrix stores them in one
+        // instruction, 16 bytes a row, where a store per register takes four. Lane l names row l & 7 of matrix l >> 3.
+        uint32_t frag_off[2];
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) frag_off[jj] = swz(16 * sub + 8 * ((lane >> 3) & 1) + (lane & 7), 4 * wg + 2 * jj + (lane >> 4));
+        auto store_frag = [&](uint32_t tile, const uint32_t (&v)[8]) {     // v[2 j], v[2 j + 1]: block j, row0 and row1
+#pragma unroll
+            for (int jj = 0; jj < 2; ++jj) stmatrix4(tile + frag_off[jj], v[4 * jj], v[4 * jj + 1], v[4 * jj + 2], v[4 * jj + 3]);
+        };
         auto publish_state = [&](int c) {                             // S_c as the MN-major B operand of O2(c), head and tail
-            uint8_t *sh = sm + SM::off_s + (c & 1) * 2 * SM::TILE, *sl = sh + SM::TILE;
+            const uint32_t sh = base + SM::off_s + (c & 1) * 2 * SM::TILE;
+            uint32_t hi[8], lo[8];
 #pragma unroll
-            for (int hi8 = 0; hi8 < 2; ++hi8) {
-                const int row = hi8 ? row1 : row0;
+            for (int i = 0; i < 8; ++i) split2(S[2 * i], S[2 * i + 1], hi[i], lo[i]);
+            store_frag(sh, hi);
+            store_frag(sh + SM::TILE, lo);
+            if (p.sent != nullptr) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    uint32_t hi, lo;
-                    split2(S[4 * j + 2 * hi8], S[4 * j + 2 * hi8 + 1], hi, lo);
-                    const uint32_t off = swz(row, 4 * wg + j) + 4 * fq;
-                    *reinterpret_cast<uint32_t *>(sh + off) = hi;
-                    *reinterpret_cast<uint32_t *>(sl + off) = lo;
-                    if (p.sent != nullptr)
-                        *reinterpret_cast<uint32_t *>(p.sent + (((size_t)bh * NC + c) * D + row) * D + col0 + 8 * j + 2 * fq) = hi;
-                }
+                for (int hi8 = 0; hi8 < 2; ++hi8)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        *reinterpret_cast<uint32_t *>(p.sent + (((size_t)bh * NC + c) * D + (hi8 ? row1 : row0)) * D + col0 + 8 * j + 2 * fq) = hi[2 * j + hi8];
             }
             warp_arrive(bar_s(c & 1), lane);
         };
@@ -274,7 +281,7 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
             const float aC = expf(Ls[TC_C - 1]);
             tmem_ld_wait();
             {
-                uint8_t *ah = sm + SM::off_a + s2 * 2 * SM::TILE, *al = ah + SM::TILE;
+                const uint32_t ah = base + SM::off_a + s2 * 2 * SM::TILE;
                 uint32_t hi[8], lo[8];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -286,12 +293,8 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
                     split2(a00, a01, hi[2 * j], lo[2 * j]);
                     split2(a10, a11, hi[2 * j + 1], lo[2 * j + 1]);
                 }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t o0 = swz(row0, 4 * wg + j) + 4 * fq, o1 = swz(row1, 4 * wg + j) + 4 * fq;
-                    *reinterpret_cast<uint32_t *>(ah + o0) = hi[2 * j];     *reinterpret_cast<uint32_t *>(al + o0) = lo[2 * j];
-                    *reinterpret_cast<uint32_t *>(ah + o1) = hi[2 * j + 1]; *reinterpret_cast<uint32_t *>(al + o1) = lo[2 * j + 1];
-                }
+                store_frag(ah, hi);
+                store_frag(ah + SM::TILE, lo);
             }
             warp_arrive(bar_a(s2), lane);                             // A(c) is there: O1(c) may go
             float uv[16];
