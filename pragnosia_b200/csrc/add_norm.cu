@@ -17,8 +17,7 @@ template <> struct Piece<__nv_bfloat16> { static constexpr int N = 8; };
 template <> struct Piece<float> { static constexpr int N = 4; };
 
 template <typename T_>
-__device__ __forceinline__ void ld_piece(float (&d)[Piece<T_>::N], const T_ *p) {
-    const uint4 raw = *reinterpret_cast<const uint4 *>(p);
+__device__ __forceinline__ void unpack_piece(float (&d)[Piece<T_>::N], const uint4 &raw) {
     if constexpr (sizeof(T_) == 2) {
         const __nv_bfloat162 *b = reinterpret_cast<const __nv_bfloat162 *>(&raw);
 #pragma unroll
@@ -59,16 +58,32 @@ add_norm_kernel(const T_ *__restrict__ x, const T_ *__restrict__ delta, const T_
     if (row >= rows) return;
     const int npieces = d / N;
     const size_t base = (size_t)row * d;
+    auto ld = [&](const T_ *p, int pc) { return *reinterpret_cast<const uint4 *>(p + (size_t)pc * N); };
+    // Every load of the row first, the norm's vectors with it (up to four pieces a lane: beyond, the registers are short and the
+    // rows long enough): a small batch's call is one round trip to the L2 and little else. 64 rows of 768: 4.0 -> 2.9 us;
+    // 8192 rows: 9.5 -> 7.8.
+    constexpr bool EARLY = NCH <= 4;
+    uint4 xr[NCH], dr[NCH], wr[EARLY ? NCH : 1], br[EARLY && KIND == 1 ? NCH : 1];
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) {
+        const int pc = lane + 32 * c;
+        if (pc < npieces) {
+            xr[c] = ld(x + base, pc);
+            if (delta != nullptr) dr[c] = ld(delta + base, pc);
+            if constexpr (EARLY) wr[c] = ld(w, pc);
+            if constexpr (EARLY && KIND == 1) br[c] = ld(b, pc);
+        }
+    }
     float v[NCH][N];
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
         const int pc = lane + 32 * c;
         if (pc < npieces) {
-            ld_piece<T_>(v[c], x + base + (size_t)pc * N);
+            unpack_piece<T_>(v[c], xr[c]);
             if (delta != nullptr) {
                 float dl[N];
-                ld_piece<T_>(dl, delta + base + (size_t)pc * N);
+                unpack_piece<T_>(dl, dr[c]);
 #pragma unroll
                 for (int i = 0; i < N; ++i) v[c][i] = round_io<T_>(v[c][i] + dl[i]);
                 if (y != nullptr) st_piece<T_>(y + base + (size_t)pc * N, v[c]);
@@ -97,8 +112,8 @@ add_norm_kernel(const T_ *__restrict__ x, const T_ *__restrict__ delta, const T_
         const int pc = lane + 32 * c;
         if (pc < npieces) {
             float ww[N], bb[N], out[N];
-            ld_piece<T_>(ww, w + (size_t)pc * N);
-            if constexpr (KIND == 1) ld_piece<T_>(bb, b + (size_t)pc * N);
+            unpack_piece<T_>(ww, EARLY ? wr[EARLY ? c : 0] : ld(w, pc));
+            if constexpr (KIND == 1) unpack_piece<T_>(bb, EARLY ? br[EARLY ? c : 0] : ld(b, pc));
 #pragma unroll
             for (int i = 0; i < N; ++i) out[i] = KIND == 1 ? (v[c][i] - mean) * rstd * ww[i] + bb[i] : v[c][i] * rstd * ww[i];
             st_piece<T_>(z + base + (size_t)pc * N, out);
