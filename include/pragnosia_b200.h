@@ -345,6 +345,10 @@ int pgb_skinny_linear_ex(const void *x, const void *delta, const void *norm_weig
                          const void *W, const void *bias, int act, void *y, void *x_out, int B, int K, int N, int flags,
                          void *stream);
 
+/* pos = (pos + 1) mod window, shift = 1: the bookkeeping between two recurrent decode steps, one launch (the reference's loop
+ * does it with tensor ops, src/bench.py:242-317). */
+int pgb_decode_advance(long long *pos, float *shift, int window, void *stream);
+
 /* ---------------------------------------------------------------------------------------------------------
  * The two ends of a decode step as single launches, so that a token is a fixed kernel sequence with no work on the host
  * (the reference samples on the host and syncs per token: src/bench.py:79-86, 193-239; embedding: src/model.py:859).
@@ -430,6 +434,12 @@ int pgb_decode_token_fwd(const void *layer_table, int L, const void *E, const vo
                          const long long *pos, const float *shift, void *work, long long work_bytes, float *logits,
                          unsigned long long *sync, int B, int d, int H, int D, int NP, int dff, int V, int ctx, int delta,
                          void *stream);
+/* The same, and with window > 0 the bookkeeping of the next token by the same launch: pos = (pos + 1) mod window, shift = 1. */
+int pgb_decode_token_step_fwd(const void *layer_table, int L, const void *E, const void *P, const void *final_norm_weight,
+                              const void *final_norm_bias, int final_norm_kind, float final_norm_eps, const long long *tok,
+                              long long *pos, float *shift, int window, void *work, long long work_bytes, float *logits,
+                              unsigned long long *sync, int B, int d, int H, int D, int NP, int dff, int V, int ctx, int delta,
+                              void *stream);
 
 /* ---------------------------------------------------------------------------------------------------------
  * y = act(x W^T + bias) as one tcgen05 GEMM with the bias and the activation applied on the accumulator in the epilogue.

@@ -54,10 +54,13 @@ SIGNATURES = {
     "pgb_batch_linear_ex": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _i, _vp, _vp, _i, _f, _vp, _vp, _i, _vp],
     "pgb_batch_linear_parts": [_i],
     "pgb_decode_embed_ex": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
+    "pgb_decode_advance": [_vp, _vp, _i, _vp],
     "pgb_decode_token_work_bytes": [_i, _i, _i, _i],
     "pgb_decode_token_wait_selftest": [_vp, _ll, _vp],
     "pgb_decode_token_fwd": [_vp, _i, _vp, _vp, _vp, _vp, _i, _f, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i,
                              _i, _vp],
+    "pgb_decode_token_step_fwd": [_vp, _i, _vp, _vp, _vp, _vp, _i, _f, _vp, _vp, _vp, _i, _vp, _ll, _vp, _vp, _i, _i, _i, _i, _i, _i, _i,
+                                  _i, _i, _vp],
     "pgb_tc_wait_selftest": [_ll, _vp],
     "pgb_linear_act": [_vp, _vp, _vp, _vp, _ll, _i, _i, _i, _vp],
     "pgb_skinny_linear": [_vp, _vp, _vp, _vp, _i, _f, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _vp],

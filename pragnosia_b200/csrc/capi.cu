@@ -65,6 +65,7 @@ int tc_segment_error_flag(int *);
 size_t prefill_fp32_chunk_scratch_bytes(int B, int H, int T, int D);
 int prefill_fp32_chunk_launch(const PrefillArgs &, int, int, void *, cudaStream_t);
 int rot_table_launch(const float *, float *, int, int, int, cudaStream_t);
+int decode_advance_launch(long long *, float *, int, cudaStream_t);
 int decode_embed_launch(const long long *, const long long *, const void *, const void *, void *, int, int, int, int, float *, cudaStream_t);
 int decode_sample_launch(const void *, int, float, float, unsigned long long, long long *, long long *, int, long long *, long long *, float *,
                          unsigned int *, int, int, int, cudaStream_t);
@@ -79,7 +80,7 @@ int add_norm_launch(const void *, const void *, const void *, const void *, floa
 int rotate_launch(const void *, int, const float *, const float *, void *, int, int, int, int, cudaStream_t);
 int decode_token_launch(const void *, int, const void *, const void *, const void *, const void *, int, float, const long long *,
                         const long long *, const float *, void *, float *, unsigned long long *, int, int, int, int, int, int, int, int,
-                        int, cudaStream_t);
+                        int, int, cudaStream_t);
 size_t decode_token_work_bytes(int B, int d, int NP, int dff);
 int decode_token_error_flag(int *);
 int batch_linear_launch(const void *, const void *, const void *, void *, int, int, int, int, const float *, int, const float *, const float *,
@@ -484,6 +485,13 @@ int pgb_aspin_delta_prefill_noscratch_fwd(const void *q, const void *k, const vo
     return prefill_tc_delta_static_launch(a, o_dtype, D, (cudaStream_t)stream);
 }
 
+int pgb_decode_advance(long long *pos, float *shift, int window, void *stream) {
+    if (!pos || !shift) return PGB_ERR_NULL_POINTER;
+    if (window < 1) return PGB_ERR_BAD_SHAPE;
+    if (!aligned(pos, 8) || !aligned(shift, 4)) return PGB_ERR_MISALIGNED;
+    return decode_advance_launch(pos, shift, window, (cudaStream_t)stream);
+}
+
 int pgb_decode_embed_ex(const long long *tok, const long long *pos, const void *E, const void *P, void *x, float *row_sums, int B, int d,
                         int vocab, int ctx, void *stream) {
     if (!tok || !pos || !E || !P || !x) return PGB_ERR_NULL_POINTER;
@@ -510,16 +518,16 @@ long long pgb_decode_token_work_bytes(int B, int d, int NP, int dff) {
     return (long long)decode_token_work_bytes(B, d, NP, dff);
 }
 
-int pgb_decode_token_fwd(const void *layer_table, int L, const void *E, const void *P, const void *final_norm_weight,
+int pgb_decode_token_step_fwd(const void *layer_table, int L, const void *E, const void *P, const void *final_norm_weight,
                          const void *final_norm_bias, int final_norm_kind, float final_norm_eps, const long long *tok,
-                         const long long *pos, const float *shift, void *work, long long work_bytes, float *logits,
+                         long long *pos, float *shift, int window, void *work, long long work_bytes, float *logits,
                          unsigned long long *sync, int B, int d, int H, int D, int NP, int dff, int V, int ctx, int delta,
                          void *stream) {
     if (!layer_table || !E || !P || !final_norm_weight || !tok || !pos || !shift || !work || !logits || !sync) return PGB_ERR_NULL_POINTER;
     if (final_norm_kind != 1 && final_norm_kind != 2) return PGB_ERR_BAD_SHAPE;
     if (final_norm_kind == 2 && !final_norm_bias) return PGB_ERR_NULL_POINTER;
     if (D != 64 && D != 128) return PGB_ERR_UNSUPPORTED_DIM;
-    if (L < 1 || B < 1 || H < 1 || d != H * D || (dff % 8) != 0 || dff < 8 || (NP % 8) != 0 || NP < 3 * d + 2 * H || V < 1 || ctx < 1)
+    if (L < 1 || B < 1 || H < 1 || d != H * D || (dff % 8) != 0 || dff < 8 || (NP % 8) != 0 || NP < 3 * d + 2 * H || V < 1 || ctx < 1 || window < 0)
         return PGB_ERR_BAD_SHAPE;
     if (B > 4 || (long long)4 * (dff > d ? dff : d) * 2 + (long long)L * 144 > 72 * 1024) return PGB_ERR_TOO_LARGE;   // shared memory
     if (work_bytes < pgb_decode_token_work_bytes(B, d, NP, dff)) return PGB_ERR_BAD_SHAPE;
@@ -528,8 +536,18 @@ int pgb_decode_token_fwd(const void *layer_table, int L, const void *E, const vo
         !aligned(logits, 4) || !aligned(sync, 16))
         return PGB_ERR_MISALIGNED;
     return decode_token_launch(layer_table, L, E, P, final_norm_weight, final_norm_bias, final_norm_kind, final_norm_eps, tok, pos,
-                               shift, work, logits, sync, B, d, H, D, NP, dff, V, ctx, delta ? 1 : 0,
+                               shift, work, logits, sync, B, d, H, D, NP, dff, V, ctx, delta ? 1 : 0, window,
                                (cudaStream_t)stream);
+}
+
+int pgb_decode_token_fwd(const void *layer_table, int L, const void *E, const void *P, const void *final_norm_weight,
+                         const void *final_norm_bias, int final_norm_kind, float final_norm_eps, const long long *tok,
+                         const long long *pos, const float *shift, void *work, long long work_bytes, float *logits,
+                         unsigned long long *sync, int B, int d, int H, int D, int NP, int dff, int V, int ctx, int delta,
+                         void *stream) {
+    return pgb_decode_token_step_fwd(layer_table, L, E, P, final_norm_weight, final_norm_bias, final_norm_kind, final_norm_eps, tok,
+                                     const_cast<long long *>(pos), const_cast<float *>(shift), 0, work, work_bytes, logits, sync, B, d, H, D,
+                                     NP, dff, V, ctx, delta, stream);
 }
 
 int pgb_decode_sample(const void *logits, int dtype, float temp, unsigned long long seed, long long *tok, long long *hist,

@@ -57,6 +57,7 @@ struct DtArgs {
     float *logits;
     unsigned long long *sync;                                         // [0] arrivals, [1] reserved
     int L, B, d, H, NP, dff, V, ctx, fn_kind;
+    int window;                                                       // > 0: leave pos and shift as the next token needs them
     float fn_eps;
 };
 
@@ -454,7 +455,12 @@ __global__ void __launch_bounds__(DT_THREADS, 1) decode_token_kernel(DtArgs a) {
     }
     // ---- final norm and the tied head
     const DtRows rw{1, xcur, a.dl, nullptr, a.fn_kind, a.fn_eps, a.fn_w, a.fn_b, d};
-    dt_phase<float, NB>(a, rw, true, gen, a.E, nullptr, a.V, false, a.logits, zs, wstage);
+    const bool alive = dt_phase<float, NB>(a, rw, true, gen, a.E, nullptr, a.V, false, a.logits, zs, wstage);
+    // every CTA has passed the last layer's barriers, behind its last reading of the position and the shift
+    if (alive && a.window > 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+        const_cast<long long *>(a.pos)[0] = (a.pos[0] + 1) % a.window;
+        const_cast<float *>(a.shift)[0] = 1.f;
+    }
 }
 
 // The barrier's failure path on its own: one CTA arrives at a barrier of a "grid" that it alone will never complete
@@ -516,14 +522,14 @@ static int decode_token_nb(const DtArgs &a, cudaStream_t stream) {
 int decode_token_launch(const void *layers, int L, const void *E, const void *P, const void *fn_w, const void *fn_b, int fn_kind,
                         float fn_eps, const long long *tok, const long long *pos, const float *shift, void *work, float *logits,
                         unsigned long long *sync, int B, int d, int H, int D, int NP, int dff, int V, int ctx, int delta,
-                        cudaStream_t stream) {
+                        int window, cudaStream_t stream) {
     __nv_bfloat16 *w = (__nv_bfloat16 *)work;
     DtArgs a{};
     a.layers = (const DtLayer *)layers; a.E = (const __nv_bfloat16 *)E; a.P = (const __nv_bfloat16 *)P;
     a.fn_w = (const __nv_bfloat16 *)fn_w; a.fn_b = (const __nv_bfloat16 *)fn_b; a.tok = tok; a.pos = pos; a.shift = shift;
     a.xa = w; a.xb = a.xa + (size_t)B * d; a.o = a.xb + (size_t)B * d; a.dl = a.o + (size_t)B * d; a.y = a.dl + (size_t)B * d;
     a.hmid = a.y + (size_t)B * NP;
-    a.logits = logits; a.sync = sync; a.L = L; a.B = B; a.d = d; a.H = H; a.NP = NP; a.dff = dff; a.V = V; a.ctx = ctx;
+    a.logits = logits; a.sync = sync; a.L = L; a.B = B; a.d = d; a.H = H; a.NP = NP; a.dff = dff; a.V = V; a.ctx = ctx; a.window = window;
     a.fn_kind = fn_kind; a.fn_eps = fn_eps;
     if (D == 64) return delta ? decode_token_nb<64, true>(a, stream) : decode_token_nb<64, false>(a, stream);
     return delta ? decode_token_nb<128, true>(a, stream) : decode_token_nb<128, false>(a, stream);

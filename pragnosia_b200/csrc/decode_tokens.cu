@@ -188,6 +188,20 @@ static cudaError_t sample_go(const T_ *logits, float temp, float min_p, unsigned
     return cudaLaunchKernelEx(&cfg, decode_sample_kernel<T_>, logits, temp, min_p, seed, tok, hist, hist_cols, count, pos, shift, ticket, V, ctx);
 }
 
+// The step's bookkeeping after the model has run: the next token's position inside its window, and the one position the carried
+// states are then rotated back by. One launch where torch took four.
+__global__ void decode_advance_kernel(long long *pos, float *shift, int window) {
+    pdl_wait();
+    pdl_launch_dependents();
+    pos[0] = (pos[0] + 1) % window;
+    shift[0] = 1.f;
+}
+int decode_advance_launch(long long *pos, float *shift, int window, cudaStream_t stream) {
+    cudaError_t e = pdl_launch(decode_advance_kernel, dim3(1), dim3(1), 0, stream, pos, shift, window);
+    if (e != cudaSuccess) { set_cuda_error(e, "decode_advance launch"); return PGB_ERR_CUDA; }
+    return check_launch("decode_advance_kernel");
+}
+
 int decode_embed_launch(const long long *tok, const long long *pos, const void *E, const void *P, void *x, int B, int d, int vocab,
                         int ctx, float *stats, cudaStream_t stream) {
     cudaError_t e = pdl_launch(decode_embed_kernel, dim3((unsigned)B), dim3(128), 0, stream, tok, pos, (const __nv_bfloat16 *)E,

@@ -134,13 +134,18 @@ class Decoder:
                           logits=torch.empty(self.B, m.e.weight.shape[0], dtype=torch.float32, device=self.dev))
         return self._plan
 
+    def _advance(self):
+        if self.dev.type == "cuda":
+            ops.decode_advance(self.pos, self.shift, self.w)
+        else:
+            self.shift.fill_(1.0)
+            self.pos.copy_((self.pos + 1) % self.w)
+
     def _step_token(self, advance: bool = True, out: Optional[torch.Tensor] = None):
         m, p = self.m, self._token_plan()
         lg = ops.decode_token(p["table"], m.e.weight, m.p.weight, m.n, self.tok, self.pos, self.shift, p["work"],
-                              p["logits"] if out is None else out, p["sync"], p["H"], p["D"], p["NP"], p["dff"], p["delta"])
-        if advance:
-            self.shift.fill_(1.0)
-            self.pos.copy_((self.pos + 1) % self.w)
+                              p["logits"] if out is None else out, p["sync"], p["H"], p["D"], p["NP"], p["dff"], p["delta"],
+                              window=self.w if advance else 0)
         return lg
 
     @property
@@ -172,8 +177,7 @@ class Decoder:
             hmid, x = ops.skinny_linear(x, mp.a.weight, mp.a.bias, delta=d1, norm=mp.n, act="gelu", want_sum=True)
             delta = ops.skinny_linear(hmid, mp.b.weight, mp.b.bias)
         if advance:
-            self.shift.fill_(1.0)
-            self.pos.copy_((self.pos + 1) % self.w)
+            self._advance()
         return ops.skinny_linear(x, m.e.weight, delta=delta, norm=m.n).float()
 
     def _wide_ok(self):
@@ -215,8 +219,7 @@ class Decoder:
             hmid = ops.batch_linear(x, Wa, act="gelu", folded=(sums, c1a, c2a, ka, ea))
             x, sums = ops.batch_linear(hmid, mp.b.weight, mp.b.bias, resid=x, want_sums=True)
         if advance:
-            self.shift.fill_(1.0)
-            self.pos.copy_((self.pos + 1) % self.w)
+            self._advance()
         We, c1e, c2e, ke, ee = head
         return ops.batch_linear(x, We, folded=(sums, c1e, c2e, ke, ee)).float()
 
@@ -228,7 +231,11 @@ class Decoder:
         if self._wide_ok():
             return self._step_wide(advance)
         m = self.m
-        x, delta = m.e(self.tok) + m.p(self.pos), None
+        if m.e.weight.is_cuda and m.e.weight.dtype == torch.bfloat16 and m.d % 8 == 0:
+            x = ops.decode_embed(self.tok, self.pos, m.e.weight, m.p.weight).view(self.B, 1, m.d)
+        else:
+            x = m.e(self.tok) + m.p(self.pos)
+        delta = None
         for i, (mx, mp) in enumerate(zip(m.mix, m.mlp)):
             st = self.states[i]
             x, z = m._add_norm(x, delta, mx.ln)
@@ -244,8 +251,7 @@ class Decoder:
             x, z = m._add_norm(x, delta, mp.n)
             delta = mp.ff(z)
         if advance:
-            self.shift.fill_(1.0)
-            self.pos.copy_((self.pos + 1) % self.w)
+            self._advance()
         z = m._add_norm(x, delta, m.n)[1]
         if self.B <= 128 and z.dtype == torch.bfloat16 and m.e.weight.dtype == torch.bfloat16 and m.d % 8 == 0 and m.e.weight.shape[0] % 8 == 0:
             # the tied head for up to 128 rows on this library's tensor-core kernel: for 64 rows by 8192 columns the

@@ -483,11 +483,21 @@ def decode_embed(tok, pos, E, P, want_sums: bool = False):
 
 
 @on_device_of
-def decode_token(table, E, P, final_norm, tok, pos, shift, work, logits, sync, H, D, NP, dff, delta: bool):
+def decode_advance(pos, shift, window: int):
+    """pos = (pos + 1) mod window, shift = 1 on the device: the bookkeeping of a decode step as one launch."""
+    need_cuda(pos, shift)
+    if pos.dtype != torch.long or shift.dtype != torch.float32:
+        raise ValueError("decode_advance: int64 position, fp32 shift")
+    check(lib().pgb_decode_advance(ptr(pos), ptr(shift), int(window), stream_of(pos)), "pgb_decode_advance")
+
+
+@on_device_of
+def decode_token(table, E, P, final_norm, tok, pos, shift, work, logits, sync, H, D, NP, dff, delta: bool, window: int = 0):
     """One decode step of the whole model in ONE cooperative launch (decode_token.cu): embedding, every layer, final norm
     and tied head for 1..4 sequences. table (L,18) int64 on the device: the per-layer pointers and norm settings the C
     header documents (generate.Decoder builds it); work / sync: scratch from decode_token_work_bytes and two zeroed
-    64-bit words; logits (B,V) fp32 out. The states the table points at are updated in place."""
+    64-bit words; logits (B,V) fp32 out. The states the table points at are updated in place; window > 0: pos
+    and shift as well, as the next token needs them ((pos + 1) mod window, 1)."""
     need_cuda(table, E, P, tok, pos, shift, work, logits, sync)
     if E.dtype != torch.bfloat16 or P.dtype != torch.bfloat16 or tok.dtype != torch.long or pos.dtype != torch.long:
         raise ValueError("decode_token: bf16 tables, int64 ids")
@@ -499,9 +509,10 @@ def decode_token(table, E, P, final_norm, tok, pos, shift, work, logits, sync, H
     if nw.dtype != torch.bfloat16 or (nb is not None and nb.dtype != torch.bfloat16):
         raise ValueError("decode_token: bf16 norm parameters")
     B, V, d = logits.shape[0], E.shape[0], E.shape[1]
-    check(lib().pgb_decode_token_fwd(ptr(table), table.shape[0], ptr(E), ptr(P), ptr(nw), ptr(nb), kind, float(eps), ptr(tok), ptr(pos),
-                                     ptr(shift), ptr(work), work.numel() * work.element_size(), ptr(logits), ptr(sync), B, d, H, D, NP,
-                                     dff, V, P.shape[0], 1 if delta else 0, stream_of(E)), "pgb_decode_token_fwd")
+    check(lib().pgb_decode_token_step_fwd(ptr(table), table.shape[0], ptr(E), ptr(P), ptr(nw), ptr(nb), kind, float(eps), ptr(tok),
+                                          ptr(pos), ptr(shift), window, ptr(work), work.numel() * work.element_size(), ptr(logits),
+                                          ptr(sync), B, d, H, D, NP, dff, V, P.shape[0], 1 if delta else 0, stream_of(E)),
+          "pgb_decode_token_step_fwd")
     return logits
 
 
