@@ -12,6 +12,8 @@
 //   * one elected thread issues the MMAs stage by stage; four warps take the accumulator out of tensor memory (a row per
 //     thread), add the bias, round to bf16 where the separate Linear would, apply the erf-GELU if asked, and store 16-byte
 //     pieces of their row.
+//   * where that leaves more than half the SMs without a CTA and K is long (the MLP's down-projection), K is cut over a cluster of
+//     up to four CTAs, whose sums meet in the first one's shared memory, added in rank order.
 //
 // x [B][K] bf16 (K contiguous) is the K-major A operand, W [N][K] (torch.nn.Linear layout) the K-major B operand.
 // Replaces, for T = 1 and 8 < batch <= 128, the F.linear (+ GELU) calls of src/assoc.py:384-512 and src/model.py:552-560.
@@ -58,7 +60,18 @@ __device__ __forceinline__ bool bl_elect_one() {
     return e != 0;
 }
 
-template <int BM, int BN>
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// 16 bytes into the same place of the shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ void st_cluster(uint32_t addr, int rank, float a, float b, float c, float d) {
+    uint32_t at;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+// SPLIT: CTAs of a cluster over which K is cut (slabs of at most 32 columns). Every thread of the cluster passes the cluster barrier twice
+// whatever became of its waits, so a wait that ran out strands nobody there.
+template <int BM, int BN, int SPLIT>
 __global__ void __launch_bounds__(BL_NT, 1) batch_linear_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw,
                                                                const __nv_bfloat16 *__restrict__ bias, __nv_bfloat16 *__restrict__ y,
                                                                int B, int N, int K, int act, BlFused f) {
@@ -75,8 +88,10 @@ __global__ void __launch_bounds__(BL_NT, 1) batch_linear_kernel(const __grid_con
     const uint32_t bar_acc = mb + 256;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5);
-    const int n0 = blockIdx.x * BN;
-    const int KB = (K + BL_BK - 1) / BL_BK;
+    const int rank = SPLIT > 1 ? (int)(blockIdx.x % SPLIT) : 0, nb = blockIdx.x / SPLIT, n0 = nb * BN;
+    const int KB_all = (K + BL_BK - 1) / BL_BK, kb0 = KB_all * rank / SPLIT, KB = KB_all * (rank + 1) / SPLIT - kb0;
+    const uint32_t parts = base + STAGES * STAGE + 1024;              // [SPLIT - 1][BM][BN] fp32, the other ranks' sums
+    if constexpr (SPLIT > 1) cluster_arrive();                        // waited for before the first remote store: every CTA has started
 
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), 1); }
@@ -99,14 +114,14 @@ __global__ void __launch_bounds__(BL_NT, 1) batch_linear_kernel(const __grid_con
         auto request_w = [&]() {
             for (int kb = 0; kb < pre; ++kb) {
                 mbar_expect_tx(bar_full(kb), STAGE);
-                bl_tma_2d(base + kb * STAGE + A_BYTES, &mw, bar_full(kb), kb * BL_BK, n0);
+                bl_tma_2d(base + kb * STAGE + A_BYTES, &mw, bar_full(kb), (kb0 + kb) * BL_BK, n0);
             }
         };
         if (leader && !f.late_consts) request_w();
         pdl_wait();                                                   // x is the kernel ahead's output
         if (leader) {
             if (f.late_consts) request_w();
-            for (int kb = 0; kb < pre; ++kb) bl_tma_2d(base + kb * STAGE, &mx, bar_full(kb), kb * BL_BK, 0);
+            for (int kb = 0; kb < pre; ++kb) bl_tma_2d(base + kb * STAGE, &mx, bar_full(kb), (kb0 + kb) * BL_BK, 0);
         }
         __syncwarp();
         bool ok = true;
@@ -115,11 +130,12 @@ __global__ void __launch_bounds__(BL_NT, 1) batch_linear_kernel(const __grid_con
             ok = __all_sync(0xffffffffu, mbar_wait(bar_empty(s), ((kb / STAGES) + 1) & 1, 75));
             if (ok && leader) {
                 mbar_expect_tx(bar_full(s), STAGE);
-                bl_tma_2d(base + s * STAGE + A_BYTES, &mw, bar_full(s), kb * BL_BK, n0);
-                bl_tma_2d(base + s * STAGE, &mx, bar_full(s), kb * BL_BK, 0);
+                bl_tma_2d(base + s * STAGE + A_BYTES, &mw, bar_full(s), (kb0 + kb) * BL_BK, n0);
+                bl_tma_2d(base + s * STAGE, &mx, bar_full(s), (kb0 + kb) * BL_BK, 0);
             }
             __syncwarp();
         }
+        if constexpr (SPLIT > 1) { cluster_wait(); cluster_arrive(); cluster_wait(); }
     } else if (warp == 1) {
         // ------------------------------------------------------------------------------------------ MMA issuer
         constexpr uint32_t IDESC = idesc_bf16(BM, BN, 0, 0);
@@ -139,6 +155,7 @@ __global__ void __launch_bounds__(BL_NT, 1) batch_linear_kernel(const __grid_con
             mma_commit_elect(bar_empty(s));                           // the stage is free once these MMAs have read it
         }
         if (ok) mma_commit_elect(bar_acc);
+        if constexpr (SPLIT > 1) { cluster_wait(); cluster_arrive(); cluster_wait(); }
     } else {
         // ------------------------------------------------------------------------------------------ epilogue: a row per thread
         // 128 rows: tensor-memory lane = row. 64 rows: each quarter of the lanes holds 16 rows in its first 16 lanes.
@@ -181,6 +198,10 @@ __global__ void __launch_bounds__(BL_NT, 1) batch_linear_kernel(const __grid_con
         }
         float q1 = 0.f, q2 = 0.f;                                     // this row's partial sums of the new residual stream
         const bool ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, 0, 77));
+        if constexpr (SPLIT > 1) {
+            cluster_wait();
+            if (!ok) { cluster_arrive(); cluster_wait(); }
+        }
         if (ok) {
             tc_fence_after();
 #pragma unroll
@@ -190,6 +211,23 @@ __global__ void __launch_bounds__(BL_NT, 1) batch_linear_kernel(const __grid_con
                 tmem_ld32(tmem + lane_base + ACC + c0, v1);
 #pragma unroll
                 for (int i = 0; i < 32; ++i) v[i] += v1[i];
+                if constexpr (SPLIT > 1) {
+                    if (rank != 0 && row < BM)
+#pragma unroll
+                        for (int q = 0; q < BN; q += 4)
+                            st_cluster(parts + (((rank - 1) * BM + row) * BN + q) * 4, 0, v[q], v[q + 1], v[q + 2], v[q + 3]);
+                    cluster_arrive();
+                    cluster_wait();
+                    if (rank != 0) break;
+                    const float *pp = reinterpret_cast<const float *>(sm + STAGES * STAGE + 1024) + (row < BM ? row : 0) * BN;
+#pragma unroll
+                    for (int r = 0; r < SPLIT - 1; ++r)
+#pragma unroll
+                        for (int q = 0; q < BN; q += 4) {
+                            const float4 t = *reinterpret_cast<const float4 *>(pp + r * BM * BN + q);
+                            v[q] += t.x; v[q + 1] += t.y; v[q + 2] += t.z; v[q + 3] += t.w;
+                        }
+                }
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
                     const int col = n0 + c0 + 8 * g;
@@ -237,7 +275,7 @@ __global__ void __launch_bounds__(BL_NT, 1) batch_linear_kernel(const __grid_con
                     }
                 }
             }
-            if (f.stats_out != nullptr && row < B) *reinterpret_cast<float2 *>(f.stats_out + ((size_t)blockIdx.x * B + row) * 2) = make_float2(q1, q2);
+            if (f.stats_out != nullptr && rank == 0 && row < B) *reinterpret_cast<float2 *>(f.stats_out + ((size_t)nb * B + row) * 2) = make_float2(q1, q2);
         }
     }
     tc_fence_before();
@@ -245,7 +283,7 @@ __global__ void __launch_bounds__(BL_NT, 1) batch_linear_kernel(const __grid_con
     if (warp == 1) tmem_dealloc(tmem, TCOLS);
 }
 
-template <int BM, int BN>
+template <int BM, int BN, int SPLIT = 1>
 static int batch_linear_go(const void *x, const void *W, const void *bias, void *y, int B, int N, int K, int act, const BlFused &f,
                            cudaStream_t stream) {
     CUtensorMap mx, mw;
@@ -253,11 +291,16 @@ static int batch_linear_go(const void *x, const void *W, const void *bias, void 
         set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled");
         return PGB_ERR_CUDA;
     }
-    constexpr int SMEM = BlSizes<BM, BN>::SMEM;
-    cudaError_t e = cudaFuncSetAttribute(batch_linear_kernel<BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    constexpr int SMEM = BlSizes<BM, BN>::SMEM + (SPLIT - 1) * BM * BN * 4;
+    cudaError_t e = cudaFuncSetAttribute(batch_linear_kernel<BM, BN, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) { set_cuda_error(e, "batch_linear smem attribute"); return PGB_ERR_CUDA; }
-    e = pdl_launch(batch_linear_kernel<BM, BN>, dim3((unsigned)((N + BN - 1) / BN)), dim3(BL_NT), (size_t)SMEM, stream, mx, mw,
-                   (const __nv_bfloat16 *)bias, (__nv_bfloat16 *)y, B, N, K, act, f);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((N + BN - 1) / BN * SPLIT)); cfg.blockDim = dim3(BL_NT); cfg.dynamicSmemBytes = SMEM; cfg.stream = stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = SPLIT; at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = SPLIT > 1 ? 2 : 1;
+    e = cudaLaunchKernelEx(&cfg, batch_linear_kernel<BM, BN, SPLIT>, mx, mw, (const __nv_bfloat16 *)bias, (__nv_bfloat16 *)y, B, N, K, act, f);
     if (e != cudaSuccess) { set_cuda_error(e, "batch_linear launch"); return PGB_ERR_CUDA; }
     return check_launch("batch_linear_kernel");
 }
@@ -274,6 +317,16 @@ int batch_linear_launch(const void *x, const void *W, const void *bias, void *y,
     // the narrowest slab that still gives about one CTA per SM: every CTA re-reads x from the L2, so fewer, wider CTAs
     // once the grid would pass the SM count. A residual (and the row sums that go with it) is taken by the narrowest only.
     const int bn = (resid != nullptr || stats_out != nullptr || (N + 15) / 16 <= sms) ? 16 : ((N + 31) / 32 <= sms ? 32 : 64);
+    // K over a cluster where 16-column slabs leave half the SMs idle and K is long enough that every CTA keeps half a ring of
+    // stages: two CTAs a slab, or four on slabs twice as wide, which read x half as often (not with a residual, which the
+    // narrowest slabs take, nor past 64 rows, where the sums do not fit beside the ring). Clusters of three did not pack onto the
+    // chip (10.0 us). 64 rows, K 3072, N 768: 8.9 -> 6.4 us
+    const int kb = (K + BL_BK - 1) / BL_BK;
+    if (bn == 16 && kb >= 16 && (N + 15) / 16 * 2 <= sms) {
+        if (B <= 64 && kb >= 32 && resid == nullptr && stats_out == nullptr) return batch_linear_go<64, 32, 4>(x, W, bias, y, B, N, K, act, f, stream);
+        if (B <= 64) return batch_linear_go<64, 16, 2>(x, W, bias, y, B, N, K, act, f, stream);
+        return batch_linear_go<128, 16, 2>(x, W, bias, y, B, N, K, act, f, stream);
+    }
     if (B <= 64) {
         if (bn == 16) return batch_linear_go<64, 16>(x, W, bias, y, B, N, K, act, f, stream);
         if (bn == 32) return batch_linear_go<64, 32>(x, W, bias, y, B, N, K, act, f, stream);

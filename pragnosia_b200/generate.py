@@ -141,6 +141,15 @@ class Decoder:
             self.shift.fill_(1.0)
             self.pos.copy_((self.pos + 1) % self.w)
 
+    def _ff_rows(self, mp, z):
+        """The MLP block for up to 128 decode rows on the decode linear kernel: the GELU goes into the first layer's epilogue, the
+        second layer's long contraction over a cluster."""
+        if not (32 < self.B <= 128 and z.dtype == torch.bfloat16 and mp.a.weight.dtype == torch.bfloat16 and z.is_cuda and
+                mp.a.weight.shape[0] % 8 == 0 and z.shape[-1] % 8 == 0):
+            return mp.ff(z)
+        h = ops.batch_linear(z.reshape(self.B, z.shape[-1]), mp.a.weight, mp.a.bias, act="gelu")
+        return ops.batch_linear(h, mp.b.weight, mp.b.bias).view(z.shape)
+
     def _step_token(self, advance: bool = True, out: Optional[torch.Tensor] = None):
         m, p = self.m, self._token_plan()
         lg = ops.decode_token(p["table"], m.e.weight, m.p.weight, m.n, self.tok, self.pos, self.shift, p["work"],
@@ -249,7 +258,7 @@ class Decoder:
                 delta, new = mx.mix(z, st)
                 for a, b in zip(st, new): a.copy_(b)
             x, z = m._add_norm(x, delta, mp.n)
-            delta = mp.ff(z)
+            delta = self._ff_rows(mp, z)
         if advance:
             self._advance()
         z = m._add_norm(x, delta, m.n)[1]
