@@ -161,7 +161,8 @@ class Decoder:
     @property
     def launches_per_token(self):
         """Kernels in one token's graph: this library's on the one-launch path (draw, step) and on the fused path (draw,
-        embedding, five per layer, head); on the library-GEMM path the count includes the GEMMs and the copies around them."""
+        embedding, five per layer, head); on the library-GEMM path the count includes the GEMMs and the copies around them
+        (an upper bound: batches up to 128 take the embedding as one launch and the GELU inside the first MLP layer)."""
         L = self.m.layers
         if self._token_ok():
             return 2
