@@ -40,35 +40,42 @@ static inline EncodeTiledFn tc_encode_fn() {
     return fn;
 }
 
+// A thread that has done no CUDA work yet (an autograd worker on its first backward, a server's new thread) has no context
+// current, which the encoding wants although the runtime's calls do without: bind the current device's and try once more.
+static inline bool tc_encode_map(CUtensorMap *m, CUtensorMapDataType type, const void *ptr, const cuuint64_t *dims, const cuuint64_t *strides,
+                                 const cuuint32_t *box, CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promotion) {
+    EncodeTiledFn fn = tc_encode_fn();
+    if (fn == nullptr) return false;
+    const cuuint32_t estr[3] = {1, 1, 1};
+    auto encode = [&]() {
+        return fn(m, type, 3, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promotion,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    if (encode()) return true;
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && encode();
+}
+
 // bf16 [n2][n1][cols] with the given row / slab strides (elements); box = 64 columns x box_rows x 1, 128-byte swizzle,
 // zero fill outside the tensor
 static inline bool tc_make_map(CUtensorMap *m, const void *ptr, long long n2, long long n1, long long cols, long long stride_1,
                                long long stride_2, int box_rows = 64) {
-    EncodeTiledFn fn = tc_encode_fn();
-    if (fn == nullptr) return false;
     cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)n1, (cuuint64_t)n2};
     cuuint64_t strides[2] = {(cuuint64_t)stride_1 * 2, (cuuint64_t)stride_2 * 2};
     cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(ptr), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return tc_encode_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
 }
 
 // [n2][n1][cols] dense, bf16 or fp32; box = box_cols x box_rows x 1, rows packed in shared memory (no swizzle): what a warp
 // stores through when a lane owns a column
 static inline bool tc_make_store_map(CUtensorMap *m, const void *ptr, bool f32, long long n2, long long n1, long long cols, int box_cols,
                                      int box_rows) {
-    EncodeTiledFn fn = tc_encode_fn();
-    if (fn == nullptr) return false;
     const int e = f32 ? 4 : 2;
     cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)n1, (cuuint64_t)n2};
     cuuint64_t strides[2] = {(cuuint64_t)cols * e, (cuuint64_t)(cols * n1) * e};
     cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    return fn(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(ptr), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return tc_encode_map(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_L2_PROMOTION_NONE);
 }
 
 // ---------------------------------------------------------------------------------------------- PTX wrappers
