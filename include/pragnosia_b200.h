@@ -185,6 +185,14 @@ int pgb_aspin_prefill_fwd(const void *q, const void *k, const void *v, int io_dt
                           float shift_host, void *o, int o_dtype, float *S_out, void *sent, int B, int H, int T,
                           int D, int precision, void *stream);
 
+/* The plain rule on bf16 operands at D = 64 with scratch (pgb_aspin_prefill_segments_scratch_bytes bytes; 0: the sequences are too
+ * short, or the chains fill the GPU, and pgb_aspin_prefill_fwd is the call): the same arithmetic with each chain cut into segments
+ * that run side by side. S_out must not be S0. */
+long long pgb_aspin_prefill_segments_scratch_bytes(int B, int H, int T, int D);
+int pgb_aspin_prefill_segments_fwd(const void *q, const void *k, const void *v, const float *la, const float *S0, const float *theta,
+                                   const float *shift_dev, float shift_host, void *o, int o_dtype, float *S_out, void *sent, void *scratch,
+                                   long long scratch_bytes, int B, int H, int T, int D, void *stream);
+
 /* The plain rule in full fp32 with scratch (pgb_aspin_prefill_fp32_scratch_bytes bytes): pgb_aspin_prefill_fwd's fp32 arithmetic
  * with the chunks of a sequence side by side instead of one behind the other. Limit B*H <= 65535. */
 long long pgb_aspin_prefill_fp32_scratch_bytes(int B, int H, int T, int D);

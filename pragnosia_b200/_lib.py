@@ -27,6 +27,8 @@ SIGNATURES = {
     "pgb_lambda_scan_fwd_ex": [_vp, _vp, _vp, _ll, _ll, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "pgb_aspin_prep_fwd": [_vp, _vp, _vp, _i, _ll, _ll, _ll, _vp, _ll, _ll, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "pgb_aspin_prefill_fwd": [_vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp],
+    "pgb_aspin_prefill_segments_scratch_bytes": [_i, _i, _i, _i],
+    "pgb_aspin_prefill_segments_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _vp],
     "pgb_aspin_prefill_fp32_scratch_bytes": [_i, _i, _i, _i],
     "pgb_aspin_prefill_fp32_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _vp],
     "pgb_aspin_delta_prefill_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _vp],

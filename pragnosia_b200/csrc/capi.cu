@@ -61,6 +61,7 @@ int prep_gates_launch(const void *, const void *, const void *, long long, long 
 int head_norm_launch(const void *, const float *, float, void *, int, int, int, int, cudaStream_t);
 size_t segment_scratch_bytes(int B, int H, int T, int seg_len);
 int segment_states_launch(const PrefillArgs &, float *, cudaStream_t);
+int segment_len_prepared(long long BH, int T);
 int tc_segment_error_flag(int *);
 size_t prefill_fp32_chunk_scratch_bytes(int B, int H, int T, int D);
 int prefill_fp32_chunk_launch(const PrefillArgs &, int, int, void *, cudaStream_t);
@@ -332,6 +333,31 @@ int pgb_aspin_prefill_fwd(const void *q, const void *k, const void *v, int io_dt
     return prefill_fp32_launch(a, io_dtype, o_dtype, D, (cudaStream_t)stream);
 }
 
+long long pgb_aspin_prefill_segments_scratch_bytes(int B, int H, int T, int D) {
+    if (B <= 0 || H <= 0 || T <= 0 || D != 64 || g_tc_variant != 0) return 0;
+    const int len = segment_len_prepared((long long)B * H, T);
+    return len == 0 ? 0 : (long long)segment_scratch_bytes(B, H, T, len);
+}
+
+int pgb_aspin_prefill_segments_fwd(const void *q, const void *k, const void *v, const float *la, const float *S0, const float *theta,
+                                   const float *shift_dev, float shift_host, void *o, int o_dtype, float *S_out, void *sent, void *scratch,
+                                   long long scratch_bytes, int B, int H, int T, int D, void *stream) {
+    if (!q || !k || !v || !la || !o || !S_out || !scratch) return PGB_ERR_NULL_POINTER;
+    if (!dtype_ok(o_dtype)) return PGB_ERR_BAD_DTYPE;
+    if (B <= 0 || H <= 0 || T <= 0) return PGB_ERR_BAD_SHAPE;
+    if (D != 64) return PGB_ERR_UNSUPPORTED_DIM;
+    const long long need = pgb_aspin_prefill_segments_scratch_bytes(B, H, T, D);
+    if (need == 0 || scratch_bytes < need) return PGB_ERR_BAD_SHAPE;
+    if (!aligned(q, 16) || !aligned(k, 16) || !aligned(v, 16) || !aligned(o, 16) || !aligned(S_out, 16) || (S0 && !aligned(S0, 16)) ||
+        (sent && !aligned(sent, 16)) || !aligned(scratch, 16))
+        return PGB_ERR_MISALIGNED;
+    PrefillArgs a{q, k, v, la, nullptr, S0, o, S_out, (__nv_bfloat16 *)sent, theta, shift_dev, shift_host, B, H, T};
+    a.seg_len = segment_len_prepared((long long)B * H, T);
+    a.seg_states = (const float *)scratch;
+    const int rc = segment_states_launch(a, (float *)scratch, (cudaStream_t)stream);
+    return rc != PGB_OK ? rc : prefill_tc_ws_launch(a, o_dtype, (cudaStream_t)stream);
+}
+
 long long pgb_aspin_prefill_fp32_scratch_bytes(int B, int H, int T, int D) {
     if (B <= 0 || H <= 0 || T <= 0 || (D != 64 && D != 128)) return 0;
     return (long long)prefill_fp32_chunk_scratch_bytes(B, H, T, D);
@@ -415,11 +441,11 @@ int pgb_aspin_layer_prefill_windows_fwd(const void *qp, const void *kp, const vo
     if (!aligned(qp, 16) || !aligned(kp, 16) || !aligned(vp, 16) || in_stride_b % 8 || in_stride_t % 8 || !aligned(o, 16) || !aligned(S_out, 16) ||
         !aligned(rot_table, 16) || (scratch && !aligned(scratch, 16)))
         return PGB_ERR_MISALIGNED;
-    PrefillArgs a{qp, kp, vp, nullptr, nullptr, T > window ? (const float *)scratch : nullptr, o, S_out, nullptr, theta, nullptr, (float)window, B, H, T};
+    PrefillArgs a{qp, kp, vp, nullptr, nullptr, nullptr, o, S_out, nullptr, theta, nullptr, (float)window, B, H, T};
     a.la_raw = decay_logits; a.la_sb = aux_stride_b; a.la_st = aux_stride_t; a.decay_A = decay_A;
     a.rms_w = rms_weight; a.rms_eps = rms_eps; a.o_token_major = 1;
     a.raw = 1; a.raw_sb = in_stride_b; a.raw_st = in_stride_t; a.gate_raw = gate_logits; a.rot = rot_table; a.rot_T = rot_T;
-    a.seg_len = window;
+    a.seg_len = window; a.seg_rotates = 1; a.seg_states = T > window ? (const float *)scratch : nullptr;
     if (T > window) {
         const int rc = segment_states_launch(a, (float *)scratch, (cudaStream_t)stream);
         if (rc != PGB_OK) return rc;

@@ -77,7 +77,8 @@ struct PrefillArgs {
     // normalise / gate / rotate itself (gate_raw: write-gate logits with la_raw's strides; rot: table [H][rot_T][D/2])
     void *W_out = nullptr;                                            // delta rule: the residuals written, bf16 [BH][T][D]
     int raw = 0; long long raw_sb = 0, raw_st = 0; const void *gate_raw = nullptr; const float *rot = nullptr; int rot_T = 0;
-    int seg_len = 0;                                                  // > 0: chains cut into segments (head dim 64; see TcParams)
+    // > 0: chains cut into segments (head dim 64; see TcParams), entered with seg_states from the second on
+    int seg_len = 0; const float *seg_states = nullptr; int seg_rotates = 0;
     int rebase_chunks = 0;                                            // delta rule: rebase the state every so many chunks (by that many tokens)
 };
 // the backward of the scan as one call (train_chunk.cu); beta, W and X only under the delta rule

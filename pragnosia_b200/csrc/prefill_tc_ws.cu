@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
     // T, positions and chunks below are the segment's own; tb is its first token.
     const int seg = blockIdx.x / p.BH, bh = blockIdx.x - seg * p.BH, h = bh % p.H, b = bh / p.H;
     const int tb = seg * p.seg_len, T = min(p.T - tb, p.seg_len), NC = (T + TC_C - 1) / TC_C;
-    const float *S0 = p.S0 == nullptr || p.seg_len >= p.T ? p.S0 : (seg == 0 ? nullptr : p.S0 + (size_t)(seg - 1) * p.BH * WS_D * WS_D);
+    const float *S0 = seg == 0 ? p.S0 : p.seg_states + (size_t)(seg - 1) * p.BH * WS_D * WS_D;
     const int tma_c0 = RAW ? h * D : 0, tma_c2 = RAW ? b : bh;
 
     if (tid == 0) {
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
 #pragma unroll
         for (int j = 0; j < 16; ++j) S[j] = 0.f;
         if (S0 != nullptr) {
-            const float shift = p.theta == nullptr ? 0.f : (p.shift_dev != nullptr ? *p.shift_dev : p.shift_host);
+            const float shift = p.theta == nullptr || (seg > 0 && !p.seg_rotates) ? 0.f : (p.shift_dev != nullptr ? *p.shift_dev : p.shift_host);
 #pragma unroll
             for (int hi8 = 0; hi8 < 2; ++hi8) {
                 const int row = hi8 ? row1 : row0;
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
                 for (int hi8 = 0; hi8 < 2; ++hi8)
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        *reinterpret_cast<uint32_t *>(p.sent + (((size_t)bh * NC + c) * D + (hi8 ? row1 : row0)) * D + col0 + 8 * j + 2 * fq) = hi[2 * j + hi8];
+                        *reinterpret_cast<uint32_t *>(p.sent + (((size_t)bh * ((p.T + TC_C - 1) / TC_C) + tb / TC_C + c) * D + (hi8 ? row1 : row0)) * D + col0 + 8 * j + 2 * fq) = hi[2 * j + hi8];
             }
             warp_arrive(bar_s(c & 1), lane);
         };
@@ -542,7 +542,7 @@ int prefill_tc_ws_launch(const PrefillArgs &a, int o_dtype, cudaStream_t stream)
     const int seg_len = a.seg_len > 0 ? a.seg_len : (a.T + TC_C - 1) / TC_C * TC_C, nseg = (a.T + seg_len - 1) / seg_len;
     TcParams p{a.la, a.S0, a.theta, a.shift_dev, a.shift_host, a.o, a.S_out, a.sent, a.H, a.T, o_dtype == PGB_F32,
                (const __nv_bfloat16 *)a.la_raw, a.la_sb, a.la_st, a.decay_A, a.rms_w, a.rms_eps, a.o_token_major,
-               (const __nv_bfloat16 *)a.gate_raw, (const float2 *)a.rot, a.rot_T, BH, seg_len};
+               (const __nv_bfloat16 *)a.gate_raw, (const float2 *)a.rot, a.rot_T, BH, seg_len, a.seg_states, a.seg_rotates};
     cudaError_t e;
     if (a.raw) {
         e = cudaFuncSetAttribute(prefill_tc_ws_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, WsSmem::bytes);

@@ -1,38 +1,44 @@
-// The states entering the windows of a long sequence, for the plain rule on the layer's raw projections (head dim 64), so that
-// the windows of one sequence can run side by side instead of one behind the other (the reference walks them in order,
-// src/model.py:857-863).
+// The states entering the segments of a sequence, for the plain rule at head dim 64, so that the segments of one sequence can run
+// side by side instead of one behind the other (the reference walks them in order, src/model.py:857-863). RAW: the windows of a
+// long sequence, on the layer's raw projections. Else: a long prepared sequence cut so that its chains fill the chip.
 //
-//   segment_state_kernel    a CTA per (window but the last, sequence, head): what the window adds to the state by its end,
+//   segment_state_kernel    a CTA per (segment but the last, sequence, head): what the segment adds to the state by its end,
 //                               U = sum_s e^{L_end - L_s} k_s v_s^T,
-//                           one long product over the window's tokens. With the decay taken to the window's END (every
-//                           exponent <= 0) nothing in it is sequential: the chunks stream through the plumbing (normalise,
+//                           one long product over the segment's tokens. With the decay taken to the segment's END (every
+//                           exponent <= 0) nothing in it is sequential: the chunks stream through the plumbing (RAW: normalise,
 //                           gate, rotate; the same arithmetic and roundings as the prefill kernel's) and accumulate in
 //                           tensor memory.
-//   segment_combine_kernel  E_{w+1} = e^{L_w} R(-len theta) E_w + U_w over the windows, elementwise, in place of U.
+//   segment_combine_kernel  E_{w+1} = e^{L_w} R E_w + U_w over the segments, elementwise, in place of U; R rotates by -len theta
+//                           where the segments are windows, else only the sequence's own entering state is rebased.
 //
-// prefill_tc_ws_kernel then takes every window as a segment with its own entering state. Bound by the tiles' latency (K and V
-// are read a second time: 16 KB a chunk, three stages ahead of the product); with 12 chains of 8192 tokens the walk of a layer is
-// 12 CTAs of 128 chunks without it and 192 CTAs of 8 with it.
+// prefill_tc_ws_kernel then takes every segment with its own entering state. Bound by the tiles' latency (K and V are read a
+// second time: 16 KB a chunk, three stages ahead of the product); with 12 chains of 8192 tokens the walk of a layer is 12 CTAs of
+// 128 chunks without it and 192 CTAs of 8 with it. Prepared
+// operands, whole call: B1 H12 T8192 174 -> 36 us, B1 H12 T2048 47 -> 19, B4 H16 T4096 93 -> 77.
 #include "tc_common.cuh"
 
 namespace pgb {
 
-constexpr int SG_NT = 256, SG_D = 64, SG_ST = 3, SG_MAX = 1024;       // threads; head dim; stages; tokens of a segment at most
+constexpr int SG_NT = 256, SG_D = 64, SG_ST = 3;                      // threads; head dim; stages
+constexpr int SG_MAX = 1024, SG_MAX_PREPARED = 4096;                  // tokens of a segment at most
 
-struct SgSmem {
+template <bool RAW> struct SgSmem {
     static constexpr int TILE = 8192, STAGE = 3 * TILE;               // K (then heads of K w), V, tails of K w
-    static constexpr int off_w = SG_ST * STAGE, off_g = off_w + SG_MAX * 4, off_misc = off_g + SG_MAX * 4, bytes = off_misc + 256 + 1024;
+    static constexpr int MAX = RAW ? SG_MAX : SG_MAX_PREPARED;
+    static constexpr int off_w = SG_ST * STAGE, off_g = off_w + MAX * 4, off_misc = off_g + (RAW ? MAX * 4 : 0), bytes = off_misc + 256 + 1024;
 };
 struct SgParams {
     const __nv_bfloat16 *decay, *gate; long long sb, st;              // logits (gate NULL: write everything), token and batch strides
     const float *decay_A; const float2 *rot; int rot_T;
+    const float *la; int T;                                           // prepared operands: log-decays [BH][T]
     float *U, *Lend;                                                  // [nseg - 1][BH][D][D], [nseg - 1][BH]
     int BH, H, seg_len;
 };
 
+template <bool RAW>
 __global__ void __launch_bounds__(SG_NT, 2) segment_state_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv,
                                                                  SgParams p) {
-    using SM = SgSmem;
+    using SM = SgSmem<RAW>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *sm = smem_raw + (base - smem_u32(smem_raw));
@@ -48,8 +54,8 @@ __global__ void __launch_bounds__(SG_NT, 2) segment_state_kernel(const __grid_co
     auto load = [&](int c) {
         const uint32_t sb = base + (c % SG_ST) * SM::STAGE, bar = full(c % SG_ST);
         mbar_expect_tx(bar, 2 * SM::TILE);
-        tma_load_3d(sb, &mk, bar, h * SG_D, tb + c * TC_C, b);
-        tma_load_3d(sb + SM::TILE, &mv, bar, h * SG_D, tb + c * TC_C, b);
+        tma_load_3d(sb, &mk, bar, RAW ? h * SG_D : 0, tb + c * TC_C, RAW ? b : bh);
+        tma_load_3d(sb + SM::TILE, &mv, bar, RAW ? h * SG_D : 0, tb + c * TC_C, RAW ? b : bh);
     };
     if (tid == 0) {
         for (int s = 0; s < SG_ST; ++s) { mbar_init(full(s), 1); mbar_init(done(s), 1); }
@@ -60,19 +66,23 @@ __global__ void __launch_bounds__(SG_NT, 2) segment_state_kernel(const __grid_co
     pdl_wait();
     if (tid == 0)
         for (int c = 0; c < 2 && c < NC; ++c) load(c);
-    // ---- decay to the end of the segment and key gate of its tokens: a thread owns four consecutive ones
+    // ---- decay to the end of the segment and key gate of its tokens: a thread owns a few consecutive ones
     {
-        const float expA = expf(p.decay_A[h]);
-        float la[4], g[4], s = 0.f;
+        constexpr int PER = SM::MAX / SG_NT;
+        const float expA = RAW ? expf(p.decay_A[h]) : 1.f;
+        float la[PER], g[RAW ? PER : 1], s = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int t = 4 * tid + i;
-            la[i] = 0.f; g[i] = 1.f;
-            if (t < p.seg_len) {
-                const size_t off = (size_t)b * p.sb + (size_t)(tb + t) * p.st + h;
-                la[i] = -fast_softplus(__bfloat162float(p.decay[off])) * expA;
-                if (p.gate != nullptr) g[i] = fast_sigmoid(__bfloat162float(p.gate[off]));
-            }
+        for (int i = 0; i < PER; ++i) {
+            const int t = PER * tid + i;
+            la[i] = 0.f;
+            if constexpr (RAW) {
+                g[i] = 1.f;
+                if (t < p.seg_len) {
+                    const size_t off = (size_t)b * p.sb + (size_t)(tb + t) * p.st + h;
+                    la[i] = -fast_softplus(__bfloat162float(p.decay[off])) * expA;
+                    if (p.gate != nullptr) g[i] = fast_sigmoid(__bfloat162float(p.gate[off]));
+                }
+            } else if (t < p.seg_len) la[i] = p.la[(size_t)bh * p.T + tb + t];
             s += la[i]; la[i] = s;                                    // running sum inside the thread
         }
         float sc = s;
@@ -89,8 +99,11 @@ __global__ void __launch_bounds__(SG_NT, 2) segment_state_kernel(const __grid_co
 #pragma unroll
         for (int w = 0; w < SG_NT / 32; ++w) { total += part[w]; if (w < warp) before += part[w]; }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (4 * tid + i < p.seg_len) { ws[4 * tid + i] = expf(fminf(total - (before + la[i]), 0.f)); gs[4 * tid + i] = g[i]; }
+        for (int i = 0; i < PER; ++i)
+            if (PER * tid + i < p.seg_len) {
+                ws[PER * tid + i] = expf(fminf(total - (before + la[i]), 0.f));
+                if constexpr (RAW) gs[PER * tid + i] = g[i];
+            }
         if (tid == 0) p.Lend[(size_t)seg * p.BH + bh] = total;
         __syncthreads();
     }
@@ -101,7 +114,24 @@ __global__ void __launch_bounds__(SG_NT, 2) segment_state_kernel(const __grid_co
         const int st = c % SG_ST;
         uint8_t *kt = sm + st * SM::STAGE, *vt = kt + SM::TILE, *lt = vt + SM::TILE;
         ok = mbar_wait_warp(full(st), (c / SG_ST) & 1, 11);
-        if (ok) {
+        if (!RAW && ok) {                                             // K w, head and tail; V as it came
+#pragma unroll
+            for (int pass = 0; pass < 2; ++pass) {
+                const int row = 32 * pass + 4 * warp + (lane >> 3);
+                const uint32_t off = swz(row, lane & 7);
+                const uint4 raw = *reinterpret_cast<const uint4 *>(kt + off);
+                const __nv_bfloat162 *b2 = reinterpret_cast<const __nv_bfloat162 *>(&raw);
+                const float w = ws[c * TC_C + row];
+                float kw[8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(b2[i]); kw[2 * i] = f.x * w; kw[2 * i + 1] = f.y * w; }
+                uint4 hi, lo;
+                split8(kw, hi, lo);
+                *reinterpret_cast<uint4 *>(kt + off) = hi;
+                *reinterpret_cast<uint4 *>(lt + off) = lo;
+            }
+        }
+        if (RAW && ok) {
             const int cp = lane & 7;
 #pragma unroll
             for (int pass = 0; pass < 2; ++pass) {
@@ -184,15 +214,26 @@ __global__ void __launch_bounds__(SG_NT, 2) segment_state_kernel(const __grid_co
 }
 
 // a thread owns two value columns of one pair of key rows; four windows' additions are requested ahead of the recurrence
-__global__ void __launch_bounds__(256) segment_combine_kernel(float *__restrict__ E, const float *__restrict__ Lend, const float *__restrict__ theta,
-                                                              int n, int BH, int H, float shift) {
+__global__ void __launch_bounds__(256) segment_combine_kernel(float *__restrict__ E, const float *__restrict__ Lend, const float *__restrict__ S0,
+                                                              const float *__restrict__ theta, const float *__restrict__ shift_dev, int n, int BH, int H,
+                                                              float shift_host, bool windows) {
     pdl_wait();
     const int e = blockIdx.x * 256 + threadIdx.x, bh = blockIdx.y, i = e / (SG_D / 2), j = 2 * (e % (SG_D / 2));
-    float sn, cs;
-    sincosf(-shift * theta[(size_t)(bh % H) * (SG_D / 2) + i], &sn, &cs);
+    float sn = 0.f, cs = 1.f;
+    const float shift = theta == nullptr ? 0.f : (shift_dev != nullptr ? *shift_dev : shift_host);
+    if (shift != 0.f) sincosf(-shift * theta[(size_t)(bh % H) * (SG_D / 2) + i], &sn, &cs);
     const size_t step = (size_t)BH * SG_D * SG_D;
     float *at = E + ((size_t)bh * SG_D + 2 * i) * SG_D + j;
     float2 a = make_float2(0.f, 0.f), b = a;                          // rows 2i, 2i + 1
+    if (S0 != nullptr) {
+        const float *src = S0 + ((size_t)bh * SG_D + 2 * i) * SG_D + j;
+        a = *reinterpret_cast<const float2 *>(src); b = *reinterpret_cast<const float2 *>(src + SG_D);
+    }
+    auto rotate = [&]() {
+        const float2 ra = make_float2(a.x * cs - b.x * sn, a.y * cs - b.y * sn), rb = make_float2(a.x * sn + b.x * cs, a.y * sn + b.y * cs);
+        a = ra; b = rb;
+    };
+    if (!windows) rotate();
     for (int w0 = 0; w0 < n; w0 += 4) {
         float2 ua[4], ub[4];
         float d[4];
@@ -206,10 +247,10 @@ __global__ void __launch_bounds__(256) segment_combine_kernel(float *__restrict_
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (w0 + k < n) {
-                // the state enters the window rotated back by the previous one's length; the first window enters with zero
-                const float2 ra = make_float2(a.x * cs - b.x * sn, a.y * cs - b.y * sn), rb = make_float2(a.x * sn + b.x * cs, a.y * sn + b.y * cs);
-                a = make_float2(fmaf(d[k], ra.x, ua[k].x), fmaf(d[k], ra.y, ua[k].y));
-                b = make_float2(fmaf(d[k], rb.x, ub[k].x), fmaf(d[k], rb.y, ub[k].y));
+                // the state enters a window rotated back by the previous one's length; the first window enters with zero
+                if (windows) rotate();
+                a = make_float2(fmaf(d[k], a.x, ua[k].x), fmaf(d[k], a.y, ua[k].y));
+                b = make_float2(fmaf(d[k], b.x, ub[k].x), fmaf(d[k], b.y, ub[k].y));
                 *reinterpret_cast<float2 *>(at + (w0 + k) * step) = a;
                 *reinterpret_cast<float2 *>(at + (w0 + k) * step + SG_D) = b;
             }
@@ -221,22 +262,39 @@ size_t segment_scratch_bytes(int B, int H, int T, int seg_len) {
     return n * B * H * (SG_D * SG_D + 1) * sizeof(float);
 }
 
-// the states entering segments 1, 2, ... of the raw layer prefill `a` (head dim 64) into scratch
+// Tokens of a segment for prepared chains of T tokens, 0: not worth cutting. Where the chains leave SMs idle, a chunk costs its walk
+// 1.3 us and the state pass 0.9, the two launches before the walk about 7 (train of 44 chains of 32 chunks: 45 us whole).
+int segment_len_prepared(long long BH, int T) {
+    const int NC = (T + TC_C - 1) / TC_C;
+    if (NC < 16 || BH * 2 > 148) return 0;
+    int best = 0;
+    double cost = 1.3 * NC;
+    for (int n = 2; n * BH <= 148; ++n) {
+        const int len = (NC + n - 1) / n;
+        if (len < 2) break;
+        if (len * TC_C <= SG_MAX_PREPARED && len * 2.2 + 7.0 < cost) { cost = len * 2.2 + 7.0; best = len * TC_C; }
+    }
+    return best;
+}
+
+// the states entering segments 1, 2, ... of the prefill `a` (head dim 64, a.seg_len set) into scratch
 int segment_states_launch(const PrefillArgs &a, float *scratch, cudaStream_t stream) {
     const int BH = a.B * a.H, nseg = (a.T + a.seg_len - 1) / a.seg_len;
     CUtensorMap mk, mv;
-    if (!tc_make_map(&mk, a.k, a.B, a.T, (long long)a.H * SG_D, a.raw_st, a.raw_sb) || !tc_make_map(&mv, a.v, a.B, a.T, (long long)a.H * SG_D, a.raw_st, a.raw_sb)) {
-        set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled");
-        return PGB_ERR_CUDA;
-    }
+    const bool made = a.raw ? tc_make_map(&mk, a.k, a.B, a.T, (long long)a.H * SG_D, a.raw_st, a.raw_sb) && tc_make_map(&mv, a.v, a.B, a.T, (long long)a.H * SG_D, a.raw_st, a.raw_sb)
+                            : tc_make_map(&mk, a.k, BH, a.T, SG_D, SG_D, (long long)a.T * SG_D) && tc_make_map(&mv, a.v, BH, a.T, SG_D, SG_D, (long long)a.T * SG_D);
+    if (!made) { set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled"); return PGB_ERR_CUDA; }
     float *Lend = scratch + (size_t)(nseg - 1) * BH * SG_D * SG_D;
-    SgParams p{(const __nv_bfloat16 *)a.la_raw, (const __nv_bfloat16 *)a.gate_raw, a.la_sb, a.la_st, a.decay_A, (const float2 *)a.rot, a.rot_T,
+    SgParams p{(const __nv_bfloat16 *)a.la_raw, (const __nv_bfloat16 *)a.gate_raw, a.la_sb, a.la_st, a.decay_A, (const float2 *)a.rot, a.rot_T, a.la, a.T,
                scratch, Lend, BH, a.H, a.seg_len};
-    cudaError_t e = cudaFuncSetAttribute(segment_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SgSmem::bytes);
-    if (e == cudaSuccess) e = pdl_launch(segment_state_kernel, dim3((unsigned)(BH * (nseg - 1))), dim3(SG_NT), (size_t)SgSmem::bytes, stream, mk, mv, p);
+    auto go = [&](auto kern, int smem) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        return e != cudaSuccess ? e : pdl_launch(kern, dim3((unsigned)(BH * (nseg - 1))), dim3(SG_NT), (size_t)smem, stream, mk, mv, p);
+    };
+    cudaError_t e = a.raw ? go(segment_state_kernel<true>, SgSmem<true>::bytes) : go(segment_state_kernel<false>, SgSmem<false>::bytes);
     if (e == cudaSuccess)
-        e = pdl_launch(segment_combine_kernel, dim3(SG_D * SG_D / 4 / 256, (unsigned)BH), dim3(256), (size_t)0, stream, scratch, (const float *)Lend, a.theta,
-                       nseg - 1, BH, a.H, (float)a.seg_len);
+        e = pdl_launch(segment_combine_kernel, dim3(SG_D * SG_D / 4 / 256, (unsigned)BH), dim3(256), (size_t)0, stream, scratch, (const float *)Lend, a.S0,
+                       a.theta, a.shift_dev, nseg - 1, BH, a.H, a.shift_host, (bool)a.seg_rotates);
     if (e != cudaSuccess) { set_cuda_error(e, "segment_state launch"); return PGB_ERR_CUDA; }
     return check_launch("segment_state_kernel");
 }
