@@ -115,9 +115,11 @@ prep_bwd_kernel(const TIN *__restrict__ qp, const TIN *__restrict__ kp, const TI
 
 // The same for bf16 operands and gradients with 16-byte aligned rows: D/8 lanes share a row, 8 channels (four pairs) each, so a
 // warp takes four rows (D = 64) or two: 16-byte accesses, a shuffle tree of three or four steps per sum instead of five, and a
-// quarter of the instructions a row. Bound by instruction issue before HBM (four sincosf a lane). 90112 rows of 64: 54 -> 30-34 us.
+// quarter of the instructions a row. Bound by instruction issue before HBM (four sincosf a lane). 90112 rows of 64:
+// 54 -> 30-34 us; three CTAs an SM (80 registers, a few of them spilled in sincosf's slow path) instead of two: with a
+// flushed L2 41.5 -> 34.9.
 template <int D>
-__global__ void __launch_bounds__(PB_WARPS * 32)
+__global__ void __launch_bounds__(PB_WARPS * 32, 3)
 prep8_bwd_kernel(const __nv_bfloat16 *__restrict__ qp, const __nv_bfloat16 *__restrict__ kp, const __nv_bfloat16 *__restrict__ vp, long long sb, long long st,
                  long long sh, const __nv_bfloat16 *__restrict__ gate, long long gsb, long long gst, const float *__restrict__ theta,
                  const long long *__restrict__ pos, const __nv_bfloat16 *__restrict__ dq, const __nv_bfloat16 *__restrict__ dk,
