@@ -29,6 +29,10 @@
 // shared memory after the TMA lands: L2-normalise q, k, v, scale k by the write gate, rotate q and k (cos/sin from a
 // per-layer table), so the separate prep pass and its HBM round trip disappear.
 //
+// Bound by the latency of the chunk's steps, one behind the other: two groups of products with the scores between them. The
+// scores are formed while U and O2 run and the state while O1 does; the MMAs are issued by a converged warp, scores and state
+// stored by stmatrix, outputs a sector at a time. D 128: B8 H16 T1024 100 -> 81 us, B2 H6 T2048 184 -> 142.
+//
 // Every mbarrier wait is bounded; a wait that runs out sets g_tc_error, and the CTA still frees its TMEM and returns.
 #include "tc_common.cuh"
 
@@ -75,7 +79,7 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
     float *eLs = Ls + 64, *wts = eLs + 64, *red = wts + 64, *rmsw = red + 128; // red[2][64], rmsw[D]
     float *gts = rmsw + 128;                                                   // sigmoid(write gate) of the chunk's tokens
     const uint32_t bar_full0 = base + SM::off_misc, bar_full1 = bar_full0 + 8, bar_a = bar_full0 + 16, bar_b = bar_full0 + 24,
-                   bar_rot = bar_full0 + 32;
+                   bar_rot = bar_full0 + 32, bar_p = bar_full0 + 40;
     // RAW, D = 64: the chunk's 64 x 32 (cos, sin) pairs are bulk-copied into the A-operand buffers, which are idle
     // between one chunk's O1 product and the next chunk's score pass
     constexpr bool ROT_SMEM = RAW && D == 64;
@@ -89,7 +93,7 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
     const int tma_c0 = RAW ? h * D : 0, tma_c2 = RAW ? b : bh;
 
     if (tid == 0) {
-        mbar_init(bar_full0, 1); mbar_init(bar_full1, 1); mbar_init(bar_a, 1); mbar_init(bar_b, 1); mbar_init(bar_rot, 1);
+        mbar_init(bar_full0, 1); mbar_init(bar_full1, 1); mbar_init(bar_a, 1); mbar_init(bar_b, 1); mbar_init(bar_rot, 1); mbar_init(bar_p, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) tmem_alloc(smem_u32(tmem_slot), TM_COLS);
@@ -105,6 +109,8 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
     const uint32_t lane_base = (uint32_t)(32 * sub) << 16;
     const int pcol0 = 32 * wg;                                        // first score column of this warp
     const int ocol0 = HALF * wg;                                      // first value column of this warp (O1, O2, U, S)
+    // a fragment's four 8 x 8 matrices of two column blocks, stored by one instruction: lane l names row l & 7 of matrix l >> 3
+    const int mrow = 8 * ((lane >> 3) & 1) + (lane & 7), mblk = lane >> 4;
     auto state_row = [&](int g, int hi8) { return (D == 128 ? 32 * sub + 16 * g : 16 * sub) + fr + 8 * hi8; };
 
     // ---- entering state in fragment order, rotated back by shift*theta (key rows 2i, 2i+1 are lanes l, l^4)
@@ -204,22 +210,22 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
         }
         // ---- the entering state as an MN-major B operand, hi and lo (and to HBM if asked for)
         {
-            uint8_t *sh = sm + SM::off_sh + (D == 128 ? wg * (D * 128) : 0), *sl = sm + SM::off_sl + (D == 128 ? wg * (D * 128) : 0);
+            const uint32_t sh = base + SM::off_sh + (D == 128 ? wg * (D * 128) : 0), sl = sh + (SM::off_sl - SM::off_sh);
 #pragma unroll
             for (int g = 0; g < NSG; ++g)
 #pragma unroll
-                for (int hi8 = 0; hi8 < 2; ++hi8) {
-                    const int row = state_row(g, hi8);
+                for (int jj = 0; jj < NBO; jj += 2) {
+                    uint32_t hi[4], lo[4];
 #pragma unroll
-                    for (int j = 0; j < NBO; ++j) {
-                        uint32_t hi, lo;
-                        split2(S[g][4 * j + 2 * hi8], S[g][4 * j + 2 * hi8 + 1], hi, lo);
-                        const uint32_t off = swz(row, (D == 128 ? j : 4 * wg + j)) + 4 * fq;
-                        *reinterpret_cast<uint32_t *>(sh + off) = hi;
-                        *reinterpret_cast<uint32_t *>(sl + off) = lo;
+                    for (int m = 0; m < 4; ++m) {
+                        const int j = jj + (m >> 1), hi8 = m & 1;
+                        split2(S[g][4 * j + 2 * hi8], S[g][4 * j + 2 * hi8 + 1], hi[m], lo[m]);
                         if (p.sent != nullptr)
-                            *reinterpret_cast<uint32_t *>(p.sent + (((size_t)bh * NC + c) * D + row) * D + ocol0 + 8 * j + 2 * fq) = hi;
+                            *reinterpret_cast<uint32_t *>(p.sent + (((size_t)bh * NC + c) * D + state_row(g, hi8)) * D + ocol0 + 8 * j + 2 * fq) = hi[m];
                     }
+                    const uint32_t off = swz(state_row(g, 0) - fr + mrow, (D == 128 ? 0 : 4 * wg) + jj + mblk);
+                    stmatrix4(sh + off, hi[0], hi[1], hi[2], hi[3]);
+                    stmatrix4(sl + off, lo[0], lo[1], lo[2], lo[3]);
                 }
         }
         if (!mbar_wait(st ? bar_full1 : bar_full0, (c >> 1) & 1, 1)) { ok = false; }
@@ -313,8 +319,8 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
         fence_proxy_async();
         tc_fence_before();
         __syncthreads();
-        // ---- P, U, O2
-        if (tid == 0 && ok) {
+        // ---- P, then U and O2 behind it, by the converged first warp (see mma_bf16_elect)
+        if (warp == 0 && ok) {
             tc_fence_after();
             constexpr uint32_t I_P = idesc_bf16(64, 64, 0, 0), I_U = idesc_bf16(D, D, 1, 1), I_O = idesc_bf16(64, D, 0, 1);
             // a descriptor's start-address field counts 16-byte units: stepping is an add on the low word
@@ -324,38 +330,35 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
 #pragma unroll
             for (int k = 0; k < D / 16; ++k) {                        // P = Q K^T, K-major steps of 32 B inside a sub-tile
                 const uint32_t ko = ((uint32_t)(k >> 2) * 8192u + (uint32_t)(k & 3) * 32u) >> 4;
-                mma_bf16(tmem + TM_P, dq + ko, dk + ko, I_P, k > 0);
+                mma_bf16_elect(tmem + TM_P, dq + ko, dk + ko, I_P, k > 0);
             }
+            mma_commit_elect(bar_p);
 #pragma unroll
             for (int k = 0; k < TC_C / 16; ++k)                       // U = (K w)^T V over the 64 tokens, 16 rows (2048 B) a step
-                mma_bf16(tmem + TM_U, dkwh + k * 128, dv + k * 128, I_U, k > 0);
+                mma_bf16_elect(tmem + TM_U, dkwh + k * 128, dv + k * 128, I_U, k > 0);
 #pragma unroll
-            for (int k = 0; k < TC_C / 16; ++k) mma_bf16(tmem + TM_U, dkwl + k * 128, dv + k * 128, I_U, 1);
+            for (int k = 0; k < TC_C / 16; ++k) mma_bf16_elect(tmem + TM_U, dkwl + k * 128, dv + k * 128, I_U, 1);
+            mma_commit_elect(bar_a);
 #pragma unroll
             for (int k = 0; k < D / 16; ++k) {                        // O2 = Q S (hi then lo); S rows are the key index
                 const uint32_t qo = ((uint32_t)(k >> 2) * 8192u + (uint32_t)(k & 3) * 32u) >> 4;
-                mma_bf16(tmem + TM_O2, dq + qo, dsh + k * 128, I_O, k > 0);
+                mma_bf16_elect(tmem + TM_O2, dq + qo, dsh + k * 128, I_O, k > 0);
             }
 #pragma unroll
             for (int k = 0; k < D / 16; ++k) {
                 const uint32_t qo = ((uint32_t)(k >> 2) * 8192u + (uint32_t)(k & 3) * 32u) >> 4;
-                mma_bf16(tmem + TM_O2, dq + qo, dsl + k * 128, I_O, 1);
+                mma_bf16_elect(tmem + TM_O2, dq + qo, dsl + k * 128, I_O, 1);
             }
-            mma_commit(bar_a);
         }
-        if (ok && !mbar_wait(bar_a, c & 1, 2)) ok = false;
-        ok = __syncthreads_and(ok);
+        if (ok) ok = mbar_wait_warp(bar_p, c & 1, 2);
         tc_fence_after();
         if (ok) {
             // ---- A = P * decay, causal; hi and lo rows of the K-major A operand
             float pv[16];
             tmem_ld_frag4(tmem + lane_base + TM_P + pcol0, pv);
-            // ---- and the state leaving the chunk: S <- e^{L_C} S + U
-            float uv[NSG][4 * NBO];
-#pragma unroll
-            for (int g = 0; g < NSG; ++g) tmem_ld_frag<NBO>(tmem + lane_base + ((uint32_t)(16 * g) << 16) + TM_U + ocol0, uv[g]);
             tmem_ld_wait();
             const float Lt0 = Ls[trow0] * LOG2E, Lt1 = Ls[trow1] * LOG2E;
+            uint32_t ah[8], al[8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int s0 = pcol0 + 8 * j + 2 * fq;
@@ -364,35 +367,45 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
                 const float a01 = (s0 + 1 <= trow0) ? pv[4 * j + 1] * exp2f(fminf(Lt0 - Ls1, 0.f)) : 0.f;
                 const float a10 = (s0 <= trow1) ? pv[4 * j + 2] * exp2f(fminf(Lt1 - Ls0, 0.f)) : 0.f;
                 const float a11 = (s0 + 1 <= trow1) ? pv[4 * j + 3] * exp2f(fminf(Lt1 - Ls1, 0.f)) : 0.f;
-                uint32_t hi, lo;
-                split2(a00, a01, hi, lo);
-                *reinterpret_cast<uint32_t *>(sm + SM::off_ah + swz(trow0, 4 * wg + j) + 4 * fq) = hi;
-                *reinterpret_cast<uint32_t *>(sm + SM::off_al + swz(trow0, 4 * wg + j) + 4 * fq) = lo;
-                split2(a10, a11, hi, lo);
-                *reinterpret_cast<uint32_t *>(sm + SM::off_ah + swz(trow1, 4 * wg + j) + 4 * fq) = hi;
-                *reinterpret_cast<uint32_t *>(sm + SM::off_al + swz(trow1, 4 * wg + j) + 4 * fq) = lo;
+                split2(a00, a01, ah[2 * j], al[2 * j]);
+                split2(a10, a11, ah[2 * j + 1], al[2 * j + 1]);
             }
 #pragma unroll
-            for (int g = 0; g < NSG; ++g)
-#pragma unroll
-                for (int j = 0; j < 4 * NBO; ++j) S[g][j] = fmaf(aC, S[g][j], uv[g][j]);
+            for (int jj = 0; jj < 2; ++jj) {
+                const uint32_t off = swz(16 * sub + mrow, 4 * wg + 2 * jj + mblk);
+                stmatrix4(base + SM::off_ah + off, ah[4 * jj], ah[4 * jj + 1], ah[4 * jj + 2], ah[4 * jj + 3]);
+                stmatrix4(base + SM::off_al + off, al[4 * jj], al[4 * jj + 1], al[4 * jj + 2], al[4 * jj + 3]);
+            }
         }
         fence_proxy_async();
         tc_fence_before();
-        __syncthreads();
+        ok = __syncthreads_and(ok);                                   // one verdict for the whole CTA
         // ---- O1 = A V
-        if (tid == 0 && ok) {
+        if (warp == 0 && ok) {
             tc_fence_after();
             constexpr uint32_t I_O = idesc_bf16(64, D, 0, 1);
             const uint64_t dah = smem_desc(base + SM::off_ah, 16, 1024), dal = smem_desc(base + SM::off_al, 16, 1024);
             const uint64_t dv = smem_desc(vs, 8192, 1024);
 #pragma unroll
-            for (int k = 0; k < TC_C / 16; ++k) mma_bf16(tmem + TM_O1, dah + k * 2, dv + k * 128, I_O, k > 0);
+            for (int k = 0; k < TC_C / 16; ++k) mma_bf16_elect(tmem + TM_O1, dah + k * 2, dv + k * 128, I_O, k > 0);
 #pragma unroll
-            for (int k = 0; k < TC_C / 16; ++k) mma_bf16(tmem + TM_O1, dal + k * 2, dv + k * 128, I_O, 1);
-            mma_commit(bar_b);
+            for (int k = 0; k < TC_C / 16; ++k) mma_bf16_elect(tmem + TM_O1, dal + k * 2, dv + k * 128, I_O, 1);
+            mma_commit_elect(bar_b);
         }
-        if (ok && !mbar_wait(bar_b, c & 1, 3)) ok = false;
+        // ---- meanwhile the state leaving the chunk: S <- e^{L_C} S + U
+        if (ok) ok = mbar_wait_warp(bar_a, c & 1, 5);
+        tc_fence_after();
+        if (ok) {
+            float uv[NSG][4 * NBO];
+#pragma unroll
+            for (int g = 0; g < NSG; ++g) tmem_ld_frag<NBO>(tmem + lane_base + ((uint32_t)(16 * g) << 16) + TM_U + ocol0, uv[g]);
+            tmem_ld_wait();
+#pragma unroll
+            for (int g = 0; g < NSG; ++g)
+#pragma unroll
+                for (int j = 0; j < 4 * NBO; ++j) S[g][j] = fmaf(aC, S[g][j], uv[g][j]);
+        }
+        if (ok) ok = mbar_wait_warp(bar_b, c & 1, 3);
         ok = __syncthreads_and(ok);
         tc_fence_after();
         if (ROT_SMEM && tid == 0 && ok && c + 1 < NC) {              // A buffers are idle again: next chunk's (cos, sin) rows
@@ -434,16 +447,29 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
 #pragma unroll
             for (int hi8 = 0; hi8 < 2; ++hi8) {
                 const int trow = hi8 ? trow1 : trow0;
-                if (t0 + trow < T) {
-                    const float sc = hi8 ? sc1 : sc0;
-                    const size_t row = p.o_token_major ? ((size_t)b * T + t0 + trow) * p.H + h : (size_t)bh * T + t0 + trow;
-                    const size_t off = row * D + ocol0 + 2 * fq;
+                const float sc = hi8 ? sc1 : sc0;
+                const size_t row = p.o_token_major ? ((size_t)b * T + t0 + trow) * p.H + h : (size_t)bh * T + t0 + trow;
+                const size_t off = row * D + ocol0;
+                // neighbouring lanes trade column pairs, so that a row's quad stores 32 bytes at a time (see prefill_tc_ws.cu)
 #pragma unroll
-                    for (int j = 0; j < NBO; ++j) {
-                        float x0 = ov[4 * j + 2 * hi8] * sc, x1 = ov[4 * j + 2 * hi8 + 1] * sc;
-                        if (p.rms_w != nullptr) { x0 *= rmsw[ocol0 + 8 * j + 2 * fq]; x1 *= rmsw[ocol0 + 8 * j + 2 * fq + 1]; }
-                        if (p.o_is_f32) *reinterpret_cast<float2 *>((float *)p.o + off + 8 * j) = make_float2(x0, x1);
-                        else *reinterpret_cast<__nv_bfloat162 *>((__nv_bfloat16 *)p.o + off + 8 * j) = __floats2bfloat162_rn(x0, x1);
+                for (int j = 0; j < NBO; j += 2) {
+                    float x[4] = {ov[4 * j + 2 * hi8] * sc, ov[4 * j + 2 * hi8 + 1] * sc, ov[4 * j + 4 + 2 * hi8] * sc, ov[4 * j + 5 + 2 * hi8] * sc};
+                    if (p.rms_w != nullptr) {
+                        const float *w = rmsw + ocol0 + 8 * j + 2 * fq;
+                        x[0] *= w[0]; x[1] *= w[1]; x[2] *= w[8]; x[3] *= w[9];
+                    }
+                    if (p.o_is_f32) {
+                        if (t0 + trow < T) {
+                            *reinterpret_cast<float2 *>((float *)p.o + off + 8 * j + 2 * fq) = make_float2(x[0], x[1]);
+                            *reinterpret_cast<float2 *>((float *)p.o + off + 8 * j + 8 + 2 * fq) = make_float2(x[2], x[3]);
+                        }
+                    } else {
+                        const __nv_bfloat162 e = __floats2bfloat162_rn(x[0], x[1]), o = __floats2bfloat162_rn(x[2], x[3]);
+                        const uint32_t ev = *reinterpret_cast<const uint32_t *>(&e), od = *reinterpret_cast<const uint32_t *>(&o);
+                        const uint32_t got = __shfl_xor_sync(0xffffffffu, (fq & 1) ? ev : od, 1);
+                        if (t0 + trow < T)
+                            *reinterpret_cast<uint2 *>((__nv_bfloat16 *)p.o + off + 8 * (j + (fq & 1)) + 4 * (fq >> 1)) =
+                                (fq & 1) ? make_uint2(got, od) : make_uint2(ev, got);
                     }
                 }
             }
