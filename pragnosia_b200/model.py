@@ -135,12 +135,29 @@ class LM(nn.Module):
             delta = mp.ff(z)
         return (x, delta), new
 
+    def _by_window(self, ids, window, tail, states=None):
+        """What _layers_windows returns, window by window (mixers without a call over all of them)."""
+        new = [None] * self.layers
+        for s in range(0, ids.shape[1], window):
+            last = self._layers(self._embed(ids[:, s:s + window]), new)
+        S = [st[0] for st in new]
+        if states is not None:
+            torch._foreach_copy_(list(states), S)
+            S = states
+        return last, S
+
+    def _replays(self, window: int) -> bool:
+        """Whether a pass window by window is the same kernels on the same addresses every time: no option in the way."""
+        return (self.use_graphs and self.e.weight.is_cuda and self.e.weight.dtype == torch.bfloat16 and
+                all(isinstance(mx, AssocCarrier) and mx.plain_step and mx.pos_wrap is None and not mx.need_sent for mx in self.mix))
+
     def _windows_pass(self, ids, window, tail):
-        """_layers_windows, from the second call with a shape on as one CUDA-graph replay (the first call of a shape runs
+        """_layers_windows (or _by_window where that does not fit), from the second call with a shape on as one CUDA-graph replay (the first call of a shape runs
         eagerly: a shape that never comes back is not worth a capture). Returns ((x, delta), states); the states are the
         caller's own."""
+        body = self._layers_windows if self.windows_fit(window) else self._by_window
         if not self.use_graphs:
-            return self._layers_windows(ids, window, tail)
+            return body(ids, window, tail)
         stamp = self.weights_stamp()
         if stamp != self._graphs_stamp:
             self._graphs.clear()
@@ -152,12 +169,12 @@ class LM(nn.Module):
             self._shapes[key] = False
             if len(self._shapes) > 64:
                 self._shapes.pop(next(iter(self._shapes)))
-            return self._layers_windows(ids, window, tail)
+            return body(ids, window, tail)
         if run is False:
             held = [k for k, v in self._shapes.items() if v is not False]
             if len(held) >= 8:                                        # eight captured shapes at most, the longest unused one goes
                 self._shapes.pop(held[0])
-            run = _ShapeGraph(self, ids, window, tail)
+            run = _ShapeGraph(self, ids, body, window, tail)
         self._shapes[key] = run                                       # last in the order: most recently used
         return run(ids)
 
@@ -208,6 +225,11 @@ class LM(nn.Module):
                 for s in range(0, T, window):
                     last = run(x[:, s:s + window], first=(s == 0))
             states = run.states
+        elif x.is_cuda and self._replays(window):
+            # a ragged last window on mixers without a call over all windows: seven launches a layer and window, whose issue from
+            # Python took longer than they did
+            last, states = self._windows_pass(x, window, (T - 1) % window + 1)
+            states = [(S, (T - 1) % window + 1) for S in states]
         else:
             states = [None] * self.layers
             last = None
@@ -218,14 +240,14 @@ class LM(nn.Module):
 
 
 class _ShapeGraph:
-    """One captured _layers_windows: static ids in, (x, delta) of the last tokens and one tensor of every layer's final state
+    """One captured _layers_windows or _by_window: static ids in, (x, delta) of the last tokens and one tensor of every layer's final state
     out (cloned per call, so that what a caller keeps is not overwritten by the next one)."""
 
-    def __init__(self, model, ids, window, tail):
+    def __init__(self, model, ids, body, window, tail):
         mx = model.mix[0]
         self.ids = torch.zeros_like(ids)
         self.states = torch.empty(model.layers, ids.shape[0], mx.h, mx.dk, mx.dk, device=ids.device, dtype=torch.float32)
-        run = lambda: model._layers_windows(self.ids, window, tail, self.states)[0]
+        run = lambda: body(self.ids, window, tail, self.states)[0]
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):                                  # warm-up: library workspaces, cached constants

@@ -80,3 +80,19 @@ def test_prep_with_aligned_rows_matches_the_strided_form(D, T):
     th, pos = synth.rope_theta(H, D).to(DEV), torch.arange(T, device=DEV)
     for x, y in zip(ops.prep(*views, gate, th, pos), ops.prep(*[v.contiguous() for v in views], gate, th, pos)):
         assert (x.float() - y.float()).abs().max() <= 2 ** -7 * x.float().abs().max()
+
+
+@pytest.mark.parametrize("T", [1, 130, 200])
+def test_ragged_windows_by_replay(T):
+    """Head dim 128 under the plain rule has no call over all windows: its ragged passes are replayed from the second on."""
+    torch.manual_seed(T)
+    with torch.device(DEV):
+        m = LM(vocab=128, d=256, layers=2, mlp_mult=2, ctx=64, mixer="hspin", norm="rms")
+    m = m.to(torch.bfloat16).eval()
+    for seed in range(4):
+        ids = torch.randint(0, 128, (2, T), device=DEV)
+        m.use_graphs = True
+        lg, st = m.forward_carried(ids, 64, return_states=True)
+        m.use_graphs = False
+        want, ws = m.forward_carried(ids, 64, return_states=True)
+        assert torch.equal(lg, want) and all(torch.equal(a[0], b[0]) and a[1] == b[1] for a, b in zip(st, ws))
