@@ -286,6 +286,7 @@ class Decoder:
             self._graph = torch.cuda.CUDAGraph()
             with graph_capture(self._graph):
                 self.logits = self._step()
+            self._held = (self.m.held(), getattr(self, "_wide", None), self._plan)     # what the graph reads, for as long as it lives
             for st, sv in zip(self.states, saved):           # warm-up and capture advanced the state: restore it
                 for a, b in zip(st, sv):
                     if torch.is_tensor(a): a.copy_(b)
@@ -345,6 +346,7 @@ class Decoder:
             self._gen_graph = torch.cuda.CUDAGraph()
             with graph_capture(self._gen_graph):
                 self._token_body(temp, seed)
+            self._gen_held = (self.m.held(), getattr(self, "_wide", None), self._plan)
             for st, sv in zip(self.states, saved):           # warm-up and capture advanced the state: restore it
                 for a, b in zip(st, sv):
                     if torch.is_tensor(a): a.copy_(b)

@@ -109,6 +109,11 @@ class LM(nn.Module):
         return (self.e.weight.is_cuda and self.e.weight.dtype == torch.bfloat16 and
                 all(isinstance(mx, AssocCarrier) and mx.windows_fit(window) for mx in self.mix))
 
+    def held(self):
+        """What the kernels of a pass read beside the parameters: constants the mixers and this model derive and cache. Each cache
+        is replaced when it is outgrown (a longer window, another sequence length), so a captured graph keeps these itself."""
+        return [getattr(mx, n, None) for mx in self.mix for n in ("_fused", "_rot", "_pos")] + [self._wpos]
+
     def _window_positions(self, T, window, device):
         """(position inside its window of every token, the same modulo the position table)."""
         key = (T, window, device)
@@ -256,6 +261,7 @@ class _ShapeGraph:
         self.graph = torch.cuda.CUDAGraph()
         with graph_capture(self.graph):
             self.out = run()
+        self.held = model.held()
 
     def __call__(self, ids):
         self.ids.copy_(ids)
@@ -323,6 +329,7 @@ class _StepGraph:
             self.graph = torch.cuda.CUDAGraph()
             with graph_capture(self.graph):
                 self.out, self.states = self._pass()
+            self.held = self.m.held()
         self.ids.copy_(ids)
         self.graph.replay()
         return self.out
@@ -373,6 +380,7 @@ class _WindowGraphs:
         self.later = torch.cuda.CUDAGraph()
         with graph_capture(self.later, pool=self.first.pool()):
             self.out_later, _ = self._pass(self.states, True)
+        self.held = self.m.held()
 
     def __call__(self, ids, first):
         if self.first is None:
