@@ -300,6 +300,8 @@ int pgb_aspin_layer_prefill_fwd(const void *qp, const void *kp, const void *vp, 
  * window: a multiple of 64; plain rule: head dim 64, window <= 1024, rot_T >= the longest window in whole chunks.
  * pos (delta rule): int64 [T], the position of every token inside its window. Scratch from the _scratch_bytes calls (plain
  * rule: none needed when T <= window).
+ * The _ex forms take the state S0 fp32 [B][H][D][D] that the sequence enters with (NULL: zero), rotated back by `window` tokens
+ * first: it left a full window, so a long sequence can be handed over in pieces of whole windows. S_out must not be S0.
  * ------------------------------------------------------------------------------------------------------- */
 long long pgb_aspin_layer_windows_scratch_bytes(int B, int H, int T, int window);
 int pgb_aspin_layer_prefill_windows_fwd(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
@@ -307,10 +309,20 @@ int pgb_aspin_layer_prefill_windows_fwd(const void *qp, const void *kp, const vo
                                         const float *decay_A, const float *rot_table, int rot_T, const float *theta, const float *rms_weight,
                                         float rms_eps, void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H,
                                         int T, int D, void *stream);
+int pgb_aspin_layer_prefill_windows_ex(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
+                                        const void *gate_logits, const void *decay_logits, long long aux_stride_b, long long aux_stride_t,
+                                        const float *decay_A, const float *rot_table, int rot_T, const float *theta, const float *S0, const float *rms_weight,
+                                        float rms_eps, void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H,
+                                        int T, int D, void *stream);
 long long pgb_aspin_delta_layer_scratch_bytes(int B, int H, int T, int D);
 int pgb_aspin_delta_layer_windows_fwd(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
                                       const void *decay_logits, const void *beta_logits, long long aux_stride_b, long long aux_stride_t,
                                       const float *decay_A, const float *theta, const long long *pos, const float *rms_weight, float rms_eps,
+                                      void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H, int T, int D,
+                                      void *stream);
+int pgb_aspin_delta_layer_windows_ex(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
+                                      const void *decay_logits, const void *beta_logits, long long aux_stride_b, long long aux_stride_t,
+                                      const float *decay_A, const float *theta, const long long *pos, const float *S0, const float *rms_weight, float rms_eps,
                                       void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H, int T, int D,
                                       void *stream);
 

@@ -44,9 +44,13 @@ SIGNATURES = {
     "pgb_aspin_layer_windows_scratch_bytes": [_i, _i, _i, _i],
     "pgb_aspin_layer_prefill_windows_fwd": [_vp, _vp, _vp, _ll, _ll, _vp, _vp, _ll, _ll, _vp, _vp, _i, _vp, _vp, _f, _vp, _vp, _vp, _ll,
                                             _i, _i, _i, _i, _i, _vp],
+    "pgb_aspin_layer_prefill_windows_ex": [_vp, _vp, _vp, _ll, _ll, _vp, _vp, _ll, _ll, _vp, _vp, _i, _vp, _vp, _vp, _f, _vp, _vp, _vp, _ll,
+                                           _i, _i, _i, _i, _i, _vp],
     "pgb_aspin_delta_layer_scratch_bytes": [_i, _i, _i, _i],
     "pgb_aspin_delta_layer_windows_fwd": [_vp, _vp, _vp, _ll, _ll, _vp, _vp, _ll, _ll, _vp, _vp, _vp, _vp, _f, _vp, _vp, _vp, _ll,
                                           _i, _i, _i, _i, _i, _vp],
+    "pgb_aspin_delta_layer_windows_ex": [_vp, _vp, _vp, _ll, _ll, _vp, _vp, _ll, _ll, _vp, _vp, _vp, _vp, _vp, _f, _vp, _vp, _vp, _ll,
+                                         _i, _i, _i, _i, _i, _vp],
     "pgb_rot_table_build": [_vp, _vp, _i, _i, _i, _vp],
     "pgb_add_norm": [_vp, _vp, _vp, _vp, _f, _i, _vp, _vp, _ll, _i, _i, _vp],
     "pgb_decode_embed": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],

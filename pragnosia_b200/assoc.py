@@ -188,10 +188,11 @@ class AssocCarrier(nn.Module):
         return (self.plain_step and self.pos_wrap is None and not self.need_sent and self.q.weight.dtype == torch.bfloat16 and window % 64 == 0
                 and (self.delta or (self.dk == 64 and window <= 1024)))
 
-    def mix_windows(self, z, window: int, pos, tail: int, S_out=None):
+    def mix_windows(self, z, window: int, pos, tail: int, S_out=None, S0=None):
         """mix over a sequence of windows with the state carried, as one call per layer: z (B,T,d), pos (T,) the tokens'
-        positions inside their windows. Returns (what is added to the last `tail` tokens of x, final state): the GEMM
-        behind the scan runs for those tokens only."""
+        positions inside their windows, S0 the state that a full window ahead of them left (None: the sequence's start). Returns
+        (what is added to the last `tail` tokens of x, final state): the GEMM behind the scan runs for those tokens only, and
+        for tail 0 not at all (None)."""
         B, T, d = z.shape
         H, dk = self.h, self.dk
         c = self._consts()
@@ -199,11 +200,11 @@ class AssocCarrier(nn.Module):
         qp, kp, vp = (y[..., i * d:(i + 1) * d].unflatten(-1, (H, dk)) for i in range(3))
         a_logit, g_logit = y[..., 3 * d:3 * d + H], y[..., 3 * d + H:3 * d + 2 * H]
         if self.delta:
-            o, S = ops.delta_layer_windows(qp, kp, vp, a_logit, g_logit, c["A"], c["theta"], pos, window, c["onw"], self._rms_eps(), S_out)
+            o, S = ops.delta_layer_windows(qp, kp, vp, a_logit, g_logit, c["A"], c["theta"], pos, window, c["onw"], self._rms_eps(), S_out, S0)
         else:
             o, S = ops.layer_prefill_windows(qp, kp, vp, g_logit, a_logit, c["A"], self._rot_table(min(T, window), c), c["theta"], window,
-                                             c["onw"], self._rms_eps(), S_out)
-        return F.linear(o if tail == T else o[:, T - tail:], c["ow"]), S
+                                             c["onw"], self._rms_eps(), S_out, S0)
+        return (F.linear(o if tail == T else o[:, T - tail:], c["ow"]) if tail else None), S
 
     def _mix_train(self, z, h0):
         """The layer with a gradient wanted (the reference's training path, src/assoc.py:384-512 with its kernels on):

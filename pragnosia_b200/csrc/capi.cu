@@ -425,12 +425,13 @@ long long pgb_aspin_layer_windows_scratch_bytes(int B, int H, int T, int window)
     return T <= window ? 0 : (long long)segment_scratch_bytes(B, H, T, window);
 }
 
-int pgb_aspin_layer_prefill_windows_fwd(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
+int pgb_aspin_layer_prefill_windows_ex(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
                                         const void *gate_logits, const void *decay_logits, long long aux_stride_b, long long aux_stride_t,
-                                        const float *decay_A, const float *rot_table, int rot_T, const float *theta, const float *rms_weight,
+                                        const float *decay_A, const float *rot_table, int rot_T, const float *theta, const float *S0, const float *rms_weight,
                                         float rms_eps, void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H,
                                         int T, int D, void *stream) {
     if (!qp || !kp || !vp || !decay_logits || !decay_A || !rot_table || !theta || !o || !S_out) return PGB_ERR_NULL_POINTER;
+    if (S0 == S_out) return PGB_ERR_BAD_SHAPE;                        // the first window reads S0 while the last writes S_out
     if (D != 64) return PGB_ERR_UNSUPPORTED_DIM;
     if (window < 64 || window % 64 != 0 || window > 1024) return PGB_ERR_BAD_SHAPE;
     const int longest = T < window ? T : window;
@@ -439,9 +440,9 @@ int pgb_aspin_layer_prefill_windows_fwd(const void *qp, const void *kp, const vo
         return PGB_ERR_BAD_SHAPE;
     if (T > window && (!scratch || scratch_bytes < pgb_aspin_layer_windows_scratch_bytes(B, H, T, window))) return PGB_ERR_BAD_SHAPE;
     if (!aligned(qp, 16) || !aligned(kp, 16) || !aligned(vp, 16) || in_stride_b % 8 || in_stride_t % 8 || !aligned(o, 16) || !aligned(S_out, 16) ||
-        !aligned(rot_table, 16) || (scratch && !aligned(scratch, 16)))
+        !aligned(rot_table, 16) || (scratch && !aligned(scratch, 16)) || (S0 && !aligned(S0, 16)))
         return PGB_ERR_MISALIGNED;
-    PrefillArgs a{qp, kp, vp, nullptr, nullptr, nullptr, o, S_out, nullptr, theta, nullptr, (float)window, B, H, T};
+    PrefillArgs a{qp, kp, vp, nullptr, nullptr, S0, o, S_out, nullptr, theta, nullptr, (float)window, B, H, T};
     a.la_raw = decay_logits; a.la_sb = aux_stride_b; a.la_st = aux_stride_t; a.decay_A = decay_A;
     a.rms_w = rms_weight; a.rms_eps = rms_eps; a.o_token_major = 1;
     a.raw = 1; a.raw_sb = in_stride_b; a.raw_st = in_stride_t; a.gate_raw = gate_logits; a.rot = rot_table; a.rot_T = rot_T;
@@ -453,13 +454,24 @@ int pgb_aspin_layer_prefill_windows_fwd(const void *qp, const void *kp, const vo
     return prefill_tc_ws_launch(a, PGB_BF16, (cudaStream_t)stream);
 }
 
-int pgb_aspin_delta_layer_windows_fwd(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
+int pgb_aspin_layer_prefill_windows_fwd(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
+                                        const void *gate_logits, const void *decay_logits, long long aux_stride_b, long long aux_stride_t,
+                                        const float *decay_A, const float *rot_table, int rot_T, const float *theta, const float *rms_weight,
+                                        float rms_eps, void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H,
+                                        int T, int D, void *stream) {
+    return pgb_aspin_layer_prefill_windows_ex(qp, kp, vp, in_stride_b, in_stride_t, gate_logits, decay_logits, aux_stride_b, aux_stride_t, decay_A,
+                                              rot_table, rot_T, theta, nullptr, rms_weight, rms_eps, o, S_out, scratch, scratch_bytes, window, B, H, T,
+                                              D, stream);
+}
+
+int pgb_aspin_delta_layer_windows_ex(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
                                       const void *decay_logits, const void *beta_logits, long long aux_stride_b, long long aux_stride_t,
-                                      const float *decay_A, const float *theta, const long long *pos, const float *rms_weight, float rms_eps,
+                                      const float *decay_A, const float *theta, const long long *pos, const float *S0, const float *rms_weight, float rms_eps,
                                       void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H, int T, int D,
                                       void *stream) {
     if (!qp || !kp || !vp || !decay_logits || !beta_logits || !decay_A || !theta || !pos || !rms_weight || !o || !S_out || !scratch)
         return PGB_ERR_NULL_POINTER;
+    if (S0 == S_out) return PGB_ERR_BAD_SHAPE;
     if (D != 64 && D != 128) return PGB_ERR_UNSUPPORTED_DIM;
     if (B <= 0 || H <= 0 || T <= 0 || aux_stride_b < 0 || aux_stride_t < H || in_stride_t < (long long)H * D || in_stride_b < 0 || window < 64 ||
         window % 64 != 0)
@@ -467,7 +479,7 @@ int pgb_aspin_delta_layer_windows_fwd(const void *qp, const void *kp, const void
     if ((long long)B * H > 65535 || (T + 63) / 64 > 65535) return PGB_ERR_TOO_LARGE;
     if (scratch_bytes < pgb_aspin_delta_layer_scratch_bytes(B, H, T, D)) return PGB_ERR_BAD_SHAPE;
     if (!aligned(qp, 16) || !aligned(kp, 16) || !aligned(vp, 16) || in_stride_b % 8 || in_stride_t % 8 || !aligned(o, 16) || !aligned(S_out, 16) ||
-        !aligned(scratch, 256) || !aligned(theta, 16) || !aligned(rms_weight, 16))
+        !aligned(scratch, 256) || !aligned(theta, 16) || !aligned(rms_weight, 16) || (S0 && !aligned(S0, 16)))
         return PGB_ERR_MISALIGNED;
     const DeltaLayerScratch sc(B, H, T, D);
     uint8_t *buf = (uint8_t *)scratch;
@@ -476,10 +488,19 @@ int pgb_aspin_delta_layer_windows_fwd(const void *qp, const void *kp, const void
     int rc = prep_gates_launch(qp, kp, vp, in_stride_b, in_stride_t, D, decay_logits, beta_logits, aux_stride_b, aux_stride_t, decay_A, theta, pos, q,
                                k, v, la, beta, B, T, H, D, (cudaStream_t)stream);
     if (rc != PGB_OK) return rc;
-    PrefillArgs a{q, k, v, la, beta, nullptr, os, S_out, nullptr, theta, nullptr, 0.f, B, H, T};
+    PrefillArgs a{q, k, v, la, beta, S0, os, S_out, nullptr, theta, nullptr, (float)window, B, H, T};
     a.rebase_chunks = window / 64;
     rc = prefill_tc_delta_launch(a, PGB_BF16, D, buf + sc.x, (cudaStream_t)stream);
     return rc != PGB_OK ? rc : head_norm_launch(os, rms_weight, rms_eps, o, B, T, H, D, (cudaStream_t)stream);
+}
+
+int pgb_aspin_delta_layer_windows_fwd(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
+                                      const void *decay_logits, const void *beta_logits, long long aux_stride_b, long long aux_stride_t,
+                                      const float *decay_A, const float *theta, const long long *pos, const float *rms_weight, float rms_eps,
+                                      void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H, int T, int D,
+                                      void *stream) {
+    return pgb_aspin_delta_layer_windows_ex(qp, kp, vp, in_stride_b, in_stride_t, decay_logits, beta_logits, aux_stride_b, aux_stride_t, decay_A, theta,
+                                            pos, nullptr, rms_weight, rms_eps, o, S_out, scratch, scratch_bytes, window, B, H, T, D, stream);
 }
 
 long long pgb_aspin_delta_layer_scratch_bytes(int B, int H, int T, int D) {

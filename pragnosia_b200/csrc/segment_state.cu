@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(256) segment_combine_kernel(float *__restrict_
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (w0 + k < n) {
-                // the state enters a window rotated back by the previous one's length; the first window enters with zero
+                // the state enters a window rotated back by the previous one's length, the sequence's own (S0) too
                 if (windows) rotate();
                 a = make_float2(fmaf(d[k], a.x, ua[k].x), fmaf(d[k], a.y, ua[k].y));
                 b = make_float2(fmaf(d[k], b.x, ub[k].x), fmaf(d[k], b.y, ub[k].y));

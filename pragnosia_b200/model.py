@@ -42,6 +42,11 @@ _MIXERS = {
 }
 
 
+# Tokens of a batch that one pass over many windows takes at most: activations of about 20 KB a token at width 768 (0.65 GB), and
+# GEMMs that long gain nothing from more rows.
+WINDOWS_TOKENS = 32768
+
+
 class LM(nn.Module):
     def __init__(self, vocab=8192, d=768, layers=12, mlp_mult=4, ctx=512, mixer="aspin", norm="ln"):
         super().__init__()
@@ -115,30 +120,41 @@ class LM(nn.Module):
         return [getattr(mx, n, None) for mx in self.mix for n in ("_fused", "_rot", "_pos")] + [self._wpos]
 
     def _window_positions(self, T, window, device):
-        """(position inside its window of every token, the same modulo the position table)."""
-        key = (T, window, device)
-        if self._wpos is None or self._wpos[0] != key:
+        """(position inside its window of every token, the same modulo the position table) for the first T tokens."""
+        if self._wpos is None or self._wpos[0] != (window, device) or self._wpos[1].numel() < T:
             pos = torch.arange(T, device=device) % window
-            self._wpos = (key, pos, pos % self.p.num_embeddings)
-        return self._wpos[1], self._wpos[2]
+            self._wpos = ((window, device), pos, pos % self.p.num_embeddings)
+        return self._wpos[1][:T], self._wpos[2][:T]
+
+    def _piece(self, B, window):
+        """Tokens of a sequence that go through the layers together: whole windows, WINDOWS_TOKENS tokens over the batch at most (or
+        one window)."""
+        return window * max(1, WINDOWS_TOKENS // (B * window))
 
     def _layers_windows(self, ids, window, tail, states=None):
-        """Every layer over ALL windows of the sequence at once: layer l of a window needs the layer below on that window
+        """Every layer over many windows of the sequence at once: layer l of a window needs the layer below on that window
         and, of the window before, only this layer's state, so nothing but the carried state inside a layer is sequential --
-        one set of GEMMs per layer over the whole sequence instead of one per window. Returns (x, delta) of the last `tail`
+        one set of GEMMs per layer over all of them instead of one per window. A sequence longer than a piece goes through piece by
+        piece with the states handed on, so the activations' memory does not grow with it. Returns (x, delta) of the last `tail`
         tokens (the last layer is computed for those only behind its scan) and the layers' final states, written into
         `states` (tensors) when given."""
         B, T = ids.shape
-        wpos, epos = self._window_positions(T, window, ids.device)
-        x, delta, new, last = self.e(ids) + self.p(epos), None, [], self.layers - 1
-        for i, (mx, mp) in enumerate(zip(self.mix, self.mlp)):
-            x, z = self._add_norm(x, delta, mx.ln)
-            n = tail if i == last else T
-            delta, S = mx.mix_windows(z, window, wpos, n, None if states is None else states[i])
-            new.append(S)
-            x, z = self._add_norm(x if n == T else x[:, T - n:], delta, mp.n)
-            delta = mp.ff(z)
-        return (x, delta), new
+        piece, last, S = self._piece(B, window), self.layers - 1, [None] * self.layers
+        for s in range(0, T, piece):
+            n, end = min(piece, T - s), s + piece >= T
+            wpos, epos = self._window_positions(n, window, ids.device)
+            x, delta, new = self.e(ids[:, s:s + n]) + self.p(epos), None, []
+            for i, (mx, mp) in enumerate(zip(self.mix, self.mlp)):
+                x, z = self._add_norm(x, delta, mx.ln)
+                keep = n if i != last else tail if end else 0
+                delta, Si = mx.mix_windows(z, window, wpos, keep, states[i] if end and states is not None else None, S[i])
+                new.append(Si)
+                if keep == 0:
+                    break
+                x, z = self._add_norm(x if keep == n else x[:, n - keep:], delta, mp.n)
+                delta = mp.ff(z)
+            S = new
+        return (x, delta), S
 
     def _by_window(self, ids, window, tail, states=None):
         """What _layers_windows returns, window by window (mixers without a call over all of them)."""
@@ -157,11 +173,11 @@ class LM(nn.Module):
                 all(isinstance(mx, AssocCarrier) and mx.plain_step and mx.pos_wrap is None and not mx.need_sent for mx in self.mix))
 
     def _windows_pass(self, ids, window, tail):
-        """_layers_windows (or _by_window where that does not fit), from the second call with a shape on as one CUDA-graph replay (the first call of a shape runs
-        eagerly: a shape that never comes back is not worth a capture). Returns ((x, delta), states); the states are the
-        caller's own."""
+        """_layers_windows (or _by_window where that does not fit), from the second call with a shape on as one CUDA-graph replay (the
+        first call of a shape runs eagerly: a shape that never comes back is not worth a capture; nor is a pass of several pieces,
+        whose kernels take longer than their launches). Returns ((x, delta), states); the states are the caller's own."""
         body = self._layers_windows if self.windows_fit(window) else self._by_window
-        if not self.use_graphs:
+        if not self.use_graphs or ids.shape[1] > self._piece(ids.shape[0], window):
             return body(ids, window, tail)
         stamp = self.weights_stamp()
         if stamp != self._graphs_stamp:

@@ -254,9 +254,11 @@ def layer_prefill(qp, kp, vp, gate_logits, decay_logits, decay_A, table, S0=None
 
 
 @on_device_of
-def layer_prefill_windows(qp, kp, vp, gate_logits, decay_logits, decay_A, table, theta, window: int, rms_weight, rms_eps: float, S_out=None):
+def layer_prefill_windows(qp, kp, vp, gate_logits, decay_logits, decay_A, table, theta, window: int, rms_weight, rms_eps: float, S_out=None,
+                          S0=None):
     """layer_prefill over a sequence of `window`-token windows with the state carried, in one call (head dim 64): the windows run
-    side by side, each from its own entering state. Returns (o (B,T,H*D), S)."""
+    side by side, each from its own entering state. S0: the state a full window ahead of these left, None: zero (never S_out
+    itself). Returns (o (B,T,H*D), S)."""
     need_cuda(qp, kp, vp, decay_logits, table)
     B, T, H, D = qp.shape
     o = torch.empty(B, T, H * D, device=qp.device, dtype=qp.dtype)
@@ -264,19 +266,22 @@ def layer_prefill_windows(qp, kp, vp, gate_logits, decay_logits, decay_A, table,
     L = lib()
     nbytes = L.pgb_aspin_layer_windows_scratch_bytes(B, H, T, window)
     scratch = torch.empty(nbytes, device=qp.device, dtype=torch.uint8) if nbytes else None
+    S0 = _f32c(S0)
     sbq = qp.stride(0) if B > 1 else T * qp.stride(1)
     sba = decay_logits.stride(0) if B > 1 else T * decay_logits.stride(1)
-    check(L.pgb_aspin_layer_prefill_windows_fwd(
+    check(L.pgb_aspin_layer_prefill_windows_ex(
         ptr(qp), ptr(kp), ptr(vp), sbq, qp.stride(1), ptr(gate_logits), ptr(decay_logits), sba, decay_logits.stride(1), ptr(decay_A),
-        ptr(table), table.shape[1], ptr(theta), ptr(rms_weight), float(rms_eps), ptr(o), ptr(S), ptr(scratch), nbytes, int(window), B, H, T, D,
-        stream_of(qp)), "pgb_aspin_layer_prefill_windows_fwd")
+        ptr(table), table.shape[1], ptr(theta), ptr(S0), ptr(rms_weight), float(rms_eps), ptr(o), ptr(S), ptr(scratch), nbytes, int(window), B, H, T,
+        D, stream_of(qp)), "pgb_aspin_layer_prefill_windows_ex")
     return o, S
 
 
 @on_device_of
-def delta_layer_windows(qp, kp, vp, decay_logits, beta_logits, decay_A, theta, pos, window: int, rms_weight, rms_eps: float, S_out=None):
+def delta_layer_windows(qp, kp, vp, decay_logits, beta_logits, decay_A, theta, pos, window: int, rms_weight, rms_eps: float, S_out=None,
+                        S0=None):
     """The delta layer between its two GEMMs over a sequence of windows with the state carried: plumbing and gates, inverses, one
-    walk, per-head norm. pos (T,) int64: every token's position inside its window. Returns (o (B,T,H*D), S)."""
+    walk, per-head norm. pos (T,) int64: every token's position inside its window; S0 as for layer_prefill_windows. Returns
+    (o (B,T,H*D), S)."""
     need_cuda(qp, kp, vp, decay_logits, beta_logits)
     B, T, H, D = qp.shape
     o = torch.empty(B, T, H * D, device=qp.device, dtype=qp.dtype)
@@ -284,12 +289,13 @@ def delta_layer_windows(qp, kp, vp, decay_logits, beta_logits, decay_A, theta, p
     L = lib()
     nbytes = L.pgb_aspin_delta_layer_scratch_bytes(B, H, T, D)
     scratch = torch.empty(nbytes, device=qp.device, dtype=torch.uint8)
+    S0 = _f32c(S0)
     sbq = qp.stride(0) if B > 1 else T * qp.stride(1)
     sba = decay_logits.stride(0) if B > 1 else T * decay_logits.stride(1)
-    check(L.pgb_aspin_delta_layer_windows_fwd(
+    check(L.pgb_aspin_delta_layer_windows_ex(
         ptr(qp), ptr(kp), ptr(vp), sbq, qp.stride(1), ptr(decay_logits), ptr(beta_logits), sba, decay_logits.stride(1), ptr(decay_A), ptr(theta),
-        ptr(pos), ptr(rms_weight), float(rms_eps), ptr(o), ptr(S), ptr(scratch), nbytes, int(window), B, H, T, D, stream_of(qp)),
-        "pgb_aspin_delta_layer_windows_fwd")
+        ptr(pos), ptr(S0), ptr(rms_weight), float(rms_eps), ptr(o), ptr(S), ptr(scratch), nbytes, int(window), B, H, T, D, stream_of(qp)),
+        "pgb_aspin_delta_layer_windows_ex")
     return o, S
 
 

@@ -96,3 +96,47 @@ def test_ragged_windows_by_replay(T):
         m.use_graphs = False
         want, ws = m.forward_carried(ids, 64, return_states=True)
         assert torch.equal(lg, want) and all(torch.equal(a[0], b[0]) and a[1] == b[1] for a, b in zip(st, ws))
+
+
+@pytest.mark.parametrize("mixer,d,window", [("aspin", 128, 64), ("dspin", 128, 64), ("hdspin", 256, 128)])
+@pytest.mark.parametrize("B,pieces,rest", [(1, 2, 0), (1, 3, 37), (3, 2, 64), (3, 2, 1)])
+def test_pieces_of_a_long_sequence(mixer, d, window, B, pieces, rest, monkeypatch):
+    """A sequence cut into pieces of whole windows with the states handed on, against the same windows in one piece."""
+    from pragnosia_b200 import model as M
+    torch.manual_seed(rest)
+    m = LM(vocab=256, d=d, layers=2, mlp_mult=2, ctx=window, mixer=mixer, norm="rms").to(DEV).to(torch.bfloat16).eval()
+    for mx in m.mix:
+        mx.theta.add_(0.01 * torch.randn_like(mx.theta))
+    tokens = 2 * window * B
+    ids = torch.randint(0, 256, (B, pieces * 2 * window + rest), device=DEV)
+    tail = (ids.shape[1] - 1) % window + 1
+    (x, y), S = m._layers_windows(ids, window, tail)
+    monkeypatch.setattr(M, "WINDOWS_TOKENS", tokens)
+    assert m._piece(B, window) == 2 * window
+    out = torch.empty_like(torch.stack(S))
+    (x1, y1), S1 = m._layers_windows(ids, window, tail, out)
+    assert x1.shape == x.shape and all(a.data_ptr() == b.data_ptr() for a, b in zip(S1, out.unbind(0)))
+    # bf16 activations of GEMMs with another M: one rounding apart
+    assert rel((x1 + y1).float(), (x + y).float()) <= 1e-2 and all(rel(a, b) <= 1e-2 for a, b in zip(S1, S))
+
+
+def test_a_long_sequence_takes_no_more_memory():
+    m = LM(vocab=256, d=768, layers=3, mlp_mult=4, ctx=512, mixer="dspin", norm="rms").to(DEV).to(torch.bfloat16).eval()
+    peak = []
+    for T in (32768 + 5, 4 * 32768 + 5):
+        ids = torch.randint(0, 256, (1, T), device=DEV)
+        torch.cuda.synchronize(); torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        m.forward_carried(ids)
+        peak.append(torch.cuda.max_memory_allocated() - before)
+    assert peak[1] <= 1.05 * peak[0] and peak[1] < 1.5e9, peak
+
+
+def test_windows_beyond_65535_chunks():
+    """The delta rule over a sequence of more chunks than one call of its kernels takes."""
+    m = LM(vocab=64, d=64, layers=1, mlp_mult=1, ctx=4096, mixer="dspin", norm="rms").to(DEV).to(torch.bfloat16).eval()
+    ids = torch.randint(0, 64, (1, 65536 * 64 + 100), device=DEV)
+    lg, S = m.forward_carried(ids, return_states=True)
+    # what far-away tokens left has decayed: the end of the sequence alone gives the same
+    lg1, S1 = m.forward_carried(ids[:, -(40 * 4096 + 100):], return_states=True)
+    assert rel(lg.float(), lg1.float()) < 2e-2 and rel(S[0][0], S1[0][0]) < 2e-2
