@@ -6,7 +6,9 @@ from __future__ import annotations
 
 import contextlib
 import ctypes as C
+import gc
 import importlib.util
+import threading
 from pathlib import Path
 
 import torch
@@ -203,18 +205,45 @@ def need_cuda(*ts) -> None:
             raise RuntimeError("pragnosia_b200 ops run on CUDA tensors only (there is no CPU path)")
 
 
+_capture_lock = threading.RLock()
+
+
 @contextlib.contextmanager
-def graph_capture(graph, **kw):
-    """torch.cuda.graph(graph, **kw) with the cyclic garbage collector out of the way. A CUDAGraph of an earlier model
-    that the collector frees in the middle of a capture destroys its executable graph; CUDA refuses that call while the
-    thread is capturing and the capture is invalidated. So: collect first, then no collections until the capture ends."""
-    import gc
-    gc.collect()
-    was_enabled = gc.isenabled()
-    gc.disable()
-    try:
-        with torch.cuda.graph(graph, **kw):
+def warm_up(stream: torch.cuda.Stream):
+    """A pass ahead of a capture, on the stream that will capture: library workspaces, cached constants. One thread at a time (the
+    lock graph_capture takes as well), so hold it over both."""
+    with _capture_lock:
+        here = torch.cuda.current_stream()
+        stream.wait_stream(here)
+        with torch.cuda.stream(stream):
             yield
-    finally:
-        if was_enabled:
-            gc.enable()
+        here.wait_stream(stream)
+
+
+@contextlib.contextmanager
+def graph_capture(graph, stream: torch.cuda.Stream | None = None, pool=None):
+    """What the block launches goes into `graph`. One capture at a time in the process, in CUDA's thread-local mode: another
+    thread may launch, allocate and synchronise its stream meanwhile (in torch's default mode its first cudaMalloc invalidates the
+    capture), and no device-wide synchronisation or emptying of the allocator's cache on the way in, which stalls every other stream.
+
+    The cyclic garbage collector stays off until the capture ends: a CUDAGraph of an earlier model that it frees in the middle
+    destroys its executable graph, which CUDA refuses while the thread is capturing, and the capture is invalidated."""
+    with _capture_lock:
+        was_enabled = gc.isenabled()
+        gc.disable()
+        here, stream = torch.cuda.current_stream(), stream or torch.cuda.Stream()
+        stream.wait_stream(here)
+        try:
+            with torch.cuda.stream(stream):
+                graph.capture_begin(**({} if pool is None else dict(pool=pool)), capture_error_mode="thread_local")
+                try:
+                    yield
+                except BaseException:
+                    with contextlib.suppress(RuntimeError):           # the block's own error is the one to see
+                        graph.capture_end()
+                    raise
+                graph.capture_end()
+            here.wait_stream(stream)
+        finally:
+            if was_enabled:
+                gc.enable()

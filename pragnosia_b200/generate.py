@@ -14,7 +14,7 @@ import torch
 import torch.nn.functional as F
 
 from . import ops
-from ._lib import graph_capture
+from ._lib import graph_capture, warm_up
 from .assoc import AssocCarrier
 
 
@@ -279,13 +279,12 @@ class Decoder:
         if self._graph is None:
             saved = [tuple(t.clone() if torch.is_tensor(t) else t for t in st) for st in self.states]
             pos, shift = self.pos.clone(), self.shift.clone()
-            s = torch.cuda.Stream(); s.wait_stream(torch.cuda.current_stream())
-            with torch.cuda.stream(s):
+            s, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+            with warm_up(s):
                 for _ in range(2): self._step()
-            torch.cuda.current_stream().wait_stream(s)
-            self._graph = torch.cuda.CUDAGraph()
-            with graph_capture(self._graph):
-                self.logits = self._step()
+                with graph_capture(graph, s):
+                    self.logits = self._step()
+            self._graph = graph
             self._held = (self.m.held(), getattr(self, "_wide", None), self._plan)     # what the graph reads, for as long as it lives
             for st, sv in zip(self.states, saved):           # warm-up and capture advanced the state: restore it
                 for a, b in zip(st, sv):
@@ -339,13 +338,12 @@ class Decoder:
             self._lg_in.copy_(lg)
             saved = [tuple(t.clone() if torch.is_tensor(t) else t for t in st) for st in self.states]
             pos, shift = self.pos.clone(), self.shift.clone()
-            s = torch.cuda.Stream(); s.wait_stream(torch.cuda.current_stream())
-            with torch.cuda.stream(s):
+            s, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+            with warm_up(s):
                 for _ in range(2): self._token_body(temp, seed)
-            torch.cuda.current_stream().wait_stream(s)
-            self._gen_graph = torch.cuda.CUDAGraph()
-            with graph_capture(self._gen_graph):
-                self._token_body(temp, seed)
+                with graph_capture(graph, s):
+                    self._token_body(temp, seed)
+            self._gen_graph = graph
             self._gen_held = (self.m.held(), getattr(self, "_wide", None), self._plan)
             for st, sv in zip(self.states, saved):           # warm-up and capture advanced the state: restore it
                 for a, b in zip(st, sv):

@@ -8,7 +8,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
-from ._lib import graph_capture
+from ._lib import graph_capture, warm_up
 from .assoc import AssocCarrier
 from .spin import SpinCarrier
 
@@ -270,13 +270,11 @@ class _ShapeGraph:
         self.states = torch.empty(model.layers, ids.shape[0], mx.h, mx.dk, mx.dk, device=ids.device, dtype=torch.float32)
         run = lambda: body(self.ids, window, tail, self.states)[0]
         side = torch.cuda.Stream()
-        side.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(side):                                  # warm-up: library workspaces, cached constants
+        with warm_up(side):
             run()
-        torch.cuda.current_stream().wait_stream(side)
-        self.graph = torch.cuda.CUDAGraph()
-        with graph_capture(self.graph):
-            self.out = run()
+            self.graph = torch.cuda.CUDAGraph()
+            with graph_capture(self.graph, side):
+                self.out = run()
         self.held = model.held()
 
     def __call__(self, ids):
@@ -336,15 +334,13 @@ class _StepGraph:
 
     def __call__(self, ids):
         if self.graph is None:
-            warm = torch.cuda.Stream()
-            warm.wait_stream(torch.cuda.current_stream())
-            with torch.cuda.stream(warm):                              # warm-up: library workspaces, cached constants
+            main = torch.cuda.Stream()
+            with warm_up(main):
                 self._pass()
-            torch.cuda.current_stream().wait_stream(warm)
-            torch.cuda.synchronize()
-            self.graph = torch.cuda.CUDAGraph()
-            with graph_capture(self.graph):
-                self.out, self.states = self._pass()
+                main.synchronize()                                     # the pass's tensors crossed streams; they are free from here on
+                self.graph = torch.cuda.CUDAGraph()
+                with graph_capture(self.graph, main):
+                    self.out, self.states = self._pass()
             self.held = self.m.held()
         self.ids.copy_(ids)
         self.graph.replay()
@@ -385,17 +381,15 @@ class _WindowGraphs:
     def _capture(self):
         none = [None] * self.m.layers
         side = torch.cuda.Stream()
-        side.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(side):                                  # warm-up: library workspaces, cached constants
+        with warm_up(side):
             _, st = self._pass(none, False)
             self._pass(st, True)
-        torch.cuda.current_stream().wait_stream(side)
-        self.first = torch.cuda.CUDAGraph()
-        with graph_capture(self.first):
-            self.out_first, self.states = self._pass(none, False)
-        self.later = torch.cuda.CUDAGraph()
-        with graph_capture(self.later, pool=self.first.pool()):
-            self.out_later, _ = self._pass(self.states, True)
+            self.first = torch.cuda.CUDAGraph()
+            with graph_capture(self.first, side):
+                self.out_first, self.states = self._pass(none, False)
+            self.later = torch.cuda.CUDAGraph()
+            with graph_capture(self.later, side, pool=self.first.pool()):
+                self.out_later, _ = self._pass(self.states, True)
         self.held = self.m.held()
 
     def __call__(self, ids, first):

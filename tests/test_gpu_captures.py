@@ -1,9 +1,11 @@
 """Captured passes against what changes around them: caches that are outgrown, switches."""
+import threading
 import weakref
 
 import pytest
 import torch
 
+from pragnosia_b200.generate import Decoder
 from pragnosia_b200.model import LM
 
 pytestmark = pytest.mark.gpu
@@ -37,3 +39,35 @@ def test_a_graph_outlives_the_caches_it_read(mixer, d, T):
     fill = [torch.full((1 << n,), 1 << 40, device=DEV) for n in range(4, 20) for _ in range(4)]   # whatever was freed is written over
     assert torch.equal(m.forward_carried(a, 64), want)
     del fill
+
+
+def test_captures_while_another_thread_works():
+    """Captures on one thread while another allocates, copies to the host and synchronises its stream: in CUDA's global capture mode
+    its first cudaMalloc ends the capture."""
+    stop, seen = threading.Event(), []
+
+    def busy():
+        n, keep = 0, []
+        with torch.cuda.stream(torch.cuda.Stream()):
+            while not stop.is_set():
+                t = torch.full(((n % 11 + 1) << 20,), 1.0, device=DEV)
+                assert float(t[:4].sum()) == 4.0
+                torch.cuda.current_stream().synchronize()
+                keep = (keep + [t])[-40:]                             # a growing pool: cudaMalloc again and again
+                n += 1
+        seen.append(n)
+
+    m = lm("aspin")
+    want = {T: m.forward_carried(ids(2, T, T), 64).clone() for T in (70, 100, 130, 200)}
+    t = threading.Thread(target=busy)
+    t.start()
+    try:
+        for T, w in want.items():
+            for _ in range(3):                                        # captured, then replayed
+                assert torch.equal(m.forward_carried(ids(2, T, T), 64), w)
+        dec = Decoder(m, batch=2)
+        dec.prefill(ids(2, 70, 1))
+        a = dec.step(ids(2, 1, 2)[:, 0]).clone()
+    finally:
+        stop.set(); t.join()
+    assert seen and seen[0] > 0 and torch.isfinite(a).all()
