@@ -14,7 +14,7 @@ import torch
 import torch.nn.functional as F
 
 from . import ops
-from ._lib import graph_capture, warm_up
+from ._lib import warm_up
 from .assoc import AssocCarrier
 
 
@@ -50,7 +50,7 @@ class Decoder:
         if stamp != self._stamp:
             self._graph, self._gen_key, self._stamp = None, None, stamp
         if m.windows_fit(w) and ids.is_cuda:
-            (x, delta), new = m._windows_pass(ids, w, 1)         # only the last token leaves the last layer
+            z, new = m._windows_pass(ids, w, 1)                  # only the last token leaves the last layer
             n = (ids.shape[1] - 1) % w + 1
             if self.states is None:
                 self.states = [(S, n) for S in new]
@@ -60,7 +60,7 @@ class Decoder:
                 self._plan["sync"].zero_()
             self.pos.fill_(n % w)
             self.shift.fill_(float(n))
-            return F.linear(m._add_norm(x, delta, m.n)[1], m.e.weight)[:, -1].float()
+            return F.linear(z, m.e.weight)[:, -1].float()
         states = [None] * m.layers
         h = None; n = 0
         for s in range(0, ids.shape[1], w):
@@ -279,13 +279,11 @@ class Decoder:
         if self._graph is None:
             saved = [tuple(t.clone() if torch.is_tensor(t) else t for t in st) for st in self.states]
             pos, shift = self.pos.clone(), self.shift.clone()
-            s, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+            s = torch.cuda.Stream()
             with warm_up(s):
                 for _ in range(2): self._step()
-                with graph_capture(graph, s):
-                    self.logits = self._step()
-            self._graph = graph
-            self._held = (self.m.held(), getattr(self, "_wide", None), self._plan)     # what the graph reads, for as long as it lives
+                self._graph, self.logits, held = self.m.capture(s, self._step)
+            self._held = (held, getattr(self, "_wide", None), self._plan)     # what the graph reads, for as long as it lives
             for st, sv in zip(self.states, saved):           # warm-up and capture advanced the state: restore it
                 for a, b in zip(st, sv):
                     if torch.is_tensor(a): a.copy_(b)
@@ -338,13 +336,11 @@ class Decoder:
             self._lg_in.copy_(lg)
             saved = [tuple(t.clone() if torch.is_tensor(t) else t for t in st) for st in self.states]
             pos, shift = self.pos.clone(), self.shift.clone()
-            s, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+            s = torch.cuda.Stream()
             with warm_up(s):
                 for _ in range(2): self._token_body(temp, seed)
-                with graph_capture(graph, s):
-                    self._token_body(temp, seed)
-            self._gen_graph = graph
-            self._gen_held = (self.m.held(), getattr(self, "_wide", None), self._plan)
+                self._gen_graph, _, held = self.m.capture(s, lambda: self._token_body(temp, seed))
+            self._gen_held = (held, getattr(self, "_wide", None), self._plan)
             for st, sv in zip(self.states, saved):           # warm-up and capture advanced the state: restore it
                 for a, b in zip(st, sv):
                     if torch.is_tensor(a): a.copy_(b)

@@ -3,6 +3,9 @@ interface as the reference's src/model.py LM (:621-864), restricted to the pure-
 hdspin, fspin). Attention controls, hybrids, growth and the training loss are other subsystems and are not here."""
 from __future__ import annotations
 
+import contextlib
+import threading
+
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
@@ -61,9 +64,7 @@ class LM(nn.Module):
         self.mlp = nn.ModuleList([MLP(d, mlp_mult) for _ in range(layers)])
         self.n = nn.LayerNorm(d)
         self.use_graphs = True          # CUDA: replay one captured graph per window in forward_carried
-        self._graphs = {}
-        self._graphs_stamp = None
-        self._shapes = {}               # _windows_pass: shapes seen, and their captured graphs, in order of use
+        self._captured = _Captured()
         self._wpos = None
         if norm == "rms":                      # every residual-stream LayerNorm becomes an RMSNorm of the same width
             for mod in list(self.modules()):
@@ -119,6 +120,15 @@ class LM(nn.Module):
         is replaced when it is outgrown (a longer window, another sequence length), so a captured graph keeps these itself."""
         return [getattr(mx, n, None) for mx in self.mix for n in ("_fused", "_rot", "_pos")] + [self._wpos]
 
+    def capture(self, stream, run, pool=None):
+        """(graph of run(), what run returned, what the graph reads and must keep). Behind a warm_up() on the same stream."""
+        while True:
+            held, graph = self.held(), torch.cuda.CUDAGraph()
+            with graph_capture(graph, stream, pool):
+                out = run()
+            if all(a is b for a, b in zip(held, self.held())):        # else another thread replaced a cache meanwhile: once more
+                return graph, out, held
+
     def _window_positions(self, T, window, device):
         """(position inside its window of every token, the same modulo the position table) for the first T tokens."""
         if self._wpos is None or self._wpos[0] != (window, device) or self._wpos[1].numel() < T:
@@ -172,32 +182,23 @@ class LM(nn.Module):
         return (self.use_graphs and self.e.weight.is_cuda and self.e.weight.dtype == torch.bfloat16 and
                 all(isinstance(mx, AssocCarrier) and mx.plain_step and mx.pos_wrap is None and not mx.need_sent for mx in self.mix))
 
-    def _windows_pass(self, ids, window, tail):
-        """_layers_windows (or _by_window where that does not fit), from the second call with a shape on as one CUDA-graph replay (the
-        first call of a shape runs eagerly: a shape that never comes back is not worth a capture; nor is a pass of several pieces,
-        whose kernels take longer than their launches). Returns ((x, delta), states); the states are the caller's own."""
+    def _windows_pass(self, ids, window, tail, graphs=True):
+        """_layers_windows (or _by_window where that does not fit) and the final norm, from the second call with a shape on as one
+        CUDA-graph replay (the first call of a shape runs eagerly: a shape that never comes back is not worth a capture; nor is a pass
+        of several pieces, whose kernels take longer than their launches). Returns (z (B,tail,d), states), both the caller's own.
+        graphs=False, or a caller that is capturing: eagerly."""
         body = self._layers_windows if self.windows_fit(window) else self._by_window
-        if not self.use_graphs or ids.shape[1] > self._piece(ids.shape[0], window):
-            return body(ids, window, tail)
-        stamp = self.weights_stamp()
-        if stamp != self._graphs_stamp:
-            self._graphs.clear()
-            self._shapes.clear()
-            self._graphs_stamp = stamp
-        key = (tuple(ids.shape), window, tail, ids.device)
-        run = self._shapes.pop(key, None)
-        if run is None:
-            self._shapes[key] = False
-            if len(self._shapes) > 64:
-                self._shapes.pop(next(iter(self._shapes)))
-            return body(ids, window, tail)
-        if run is False:
-            held = [k for k, v in self._shapes.items() if v is not False]
-            if len(held) >= 8:                                        # eight captured shapes at most, the longest unused one goes
-                self._shapes.pop(held[0])
-            run = _ShapeGraph(self, ids, body, window, tail)
-        self._shapes[key] = run                                       # last in the order: most recently used
-        return run(ids)
+        if graphs and self._may_replay(ids) and ids.shape[1] <= self._piece(ids.shape[0], window):
+            with self._captured.turn(self) as c:
+                run = c.shape_graph(self, ids, body, window, tail)
+                if run is not None:
+                    last, states = run(ids)
+                    return self._add_norm(*last, self.n)[1], states
+        last, states = body(ids, window, tail)
+        return self._add_norm(*last, self.n)[1], states
+
+    def _may_replay(self, ids) -> bool:
+        return self.use_graphs and ids.is_cuda and not torch.cuda.is_current_stream_capturing()
 
     def trunk(self, x, states=None, carry=False):
         """Everything but the output head; with carry=True also takes / returns the per-layer states."""
@@ -217,65 +218,124 @@ class LM(nn.Module):
         window). On CUDA, with use_graphs set and whole windows, each window pass is one CUDA-graph replay."""
         window = window or self.ctx
         B, T = x.shape
-        if self.windows_fit(window) and x.is_cuda and (B * self.mix[0].h < 148 or T % window):
-            # fewer chains than SMs, or a ragged last window: layer by layer over the whole sequence. With more chains and whole
-            # windows the window-by-window graph below keeps the GPU as full and its activations in the L2.
-            last, states = self._windows_pass(x, window, (T - 1) % window + 1)
-            states = [(S, (T - 1) % window + 1) for S in states]
-        elif self.use_graphs and x.is_cuda and T % window == 0 and T >= window:
-            # A captured graph holds the addresses of the parameters and of the constants the mixers derive from them
-            # (the concatenated projection weight, the gated output weight): any change of either retires every graph.
-            stamp = self.weights_stamp()
-            if stamp != self._graphs_stamp:
-                self._graphs.clear()
-                self._graphs_stamp = stamp
-            nw = T // window
-            if self.wavefront and nw >= 2 and all(isinstance(mx, AssocCarrier) for mx in self.mix):
-                # every window of the call in ONE graph, consecutive windows on two streams a layer apart
-                key = (B, window, nw, x.device, self.e.weight.dtype)
-                run = self._graphs.get(key)
-                if run is None:
-                    run = self._graphs[key] = _StepGraph(self, B, window, nw, x.device)
-                last = run(x)
-            else:
-                key = (B, window, x.device, self.e.weight.dtype)
-                run = self._graphs.get(key)
-                if run is None:
-                    run = self._graphs[key] = _WindowGraphs(self, B, window, x.device)
-                last = None
-                for s in range(0, T, window):
-                    last = run(x[:, s:s + window], first=(s == 0))
-            states = run.states
-        elif x.is_cuda and self._replays(window):
-            # a ragged last window on mixers without a call over all windows: seven launches a layer and window, whose issue from
-            # Python took longer than they did
-            last, states = self._windows_pass(x, window, (T - 1) % window + 1)
-            states = [(S, (T - 1) % window + 1) for S in states]
+        tail = (T - 1) % window + 1
+        # Fewer chains than SMs, or a ragged last window: layer by layer over the whole sequence (or, on mixers without a call over all
+        # windows, window by window: seven launches a layer and window, whose issue from Python took longer than they did). With more
+        # chains and whole windows the window-by-window graph below keeps the GPU as full and its activations in the L2.
+        all_windows = self.windows_fit(window) and x.is_cuda and (B * self.mix[0].h < 148 or T % window)
+        whole = T % window == 0 and T >= window
+        if all_windows or (x.is_cuda and self._replays(window) and not whole):
+            z, states = self._windows_pass(x, window, tail)
+            states = [(S, tail) for S in states]
+        elif whole and self._may_replay(x):
+            with self._captured.turn(self) as c:
+                last, states = c.window_graphs(self, x, window)
+                z = self._add_norm(*last, self.n)[1]
+                if return_states:                                     # the graph's own are overwritten by the next call
+                    states = [tuple(t.clone() if torch.is_tensor(t) else t for t in st) for st in states]
         else:
             states = [None] * self.layers
             last = None
             for s in range(0, T, window):
                 last = self._layers(self._embed(x[:, s:s + window]), states)
-        logits = F.linear(self._add_norm(*last, self.n)[1], self.e.weight)
+            z = self._add_norm(*last, self.n)[1]
+        logits = F.linear(z, self.e.weight)
         return (logits, states) if return_states else logits
+
+
+class _Captured:
+    """A model's captured passes. They write static tensors of their own and share one memory pool, so they run one at a time:
+    turn() holds the host lock, makes the current stream wait for the turn before (whichever thread and stream it came from) and
+    drops every graph once the weights' stamp has changed. Results are copied out before a turn ends. A copy or a pickle of the
+    model starts with none."""
+
+    def __init__(self):
+        self.lock, self.done = threading.RLock(), None
+        self.stamp = self.pool = self.stream = None
+        self.windows = {}               # whole windows: (batch, window, windows) -> _StepGraph, (batch, window) -> _WindowGraphs
+        self.shapes = {}                # passes over many windows: shapes seen (False) and captured, in order of use
+
+    def __deepcopy__(self, memo):
+        return type(self)()
+
+    def __reduce__(self):
+        return type(self), ()
+
+    @contextlib.contextmanager
+    def turn(self, model):
+        with self.lock:
+            here = torch.cuda.current_stream()
+            if self.done is None:
+                self.done = torch.cuda.Event()
+            else:
+                here.wait_event(self.done)
+            # A captured graph holds the addresses of the parameters and of the constants the mixers derive from them
+            # (the concatenated projection weight, the gated output weight): any change of either retires every graph.
+            stamp = model.weights_stamp()
+            if stamp != self.stamp:
+                self.windows.clear()
+                self.shapes.clear()
+                self.stamp, self.pool = stamp, None
+            try:
+                yield self
+            finally:
+                self.done.record(here)
+
+    def shape_graph(self, model, ids, body, window, tail):
+        """The captured pass of this shape; None the first time it comes."""
+        key = (tuple(ids.shape), ids.dtype, window, tail, ids.device)
+        run = self.shapes.pop(key, None)
+        if run is None:
+            self.shapes[key] = False
+            if len(self.shapes) > 64:
+                self.shapes.pop(next(iter(self.shapes)))
+            return None
+        if run is False:
+            held = [k for k, v in self.shapes.items() if v is not False]
+            if len(held) >= 8:                                        # eight captured shapes at most, the longest unused one goes
+                self.shapes.pop(held[0])
+            if self.pool is None:
+                self.pool, self.stream = torch.cuda.graph_pool_handle(), torch.cuda.Stream()
+            run = _ShapeGraph(model, ids, body, window, tail, self.stream, self.pool)
+        self.shapes[key] = run                                        # last in the order: most recently used
+        return run
+
+    def window_graphs(self, model, x, window):
+        """((x, delta) of the last window, states) of a pass over whole windows."""
+        B, T = x.shape
+        nw = T // window
+        if model.wavefront and nw >= 2 and all(isinstance(mx, AssocCarrier) for mx in model.mix):
+            # every window of the call in ONE graph, consecutive windows on two streams a layer apart
+            key = (B, window, nw, x.device, model.e.weight.dtype)
+            run = self.windows.get(key)
+            if run is None:
+                run = self.windows[key] = _StepGraph(model, B, window, nw, x.device)
+            last = run(x)
+        else:
+            key = (B, window, x.device, model.e.weight.dtype)
+            run = self.windows.get(key)
+            if run is None:
+                run = self.windows[key] = _WindowGraphs(model, B, window, x.device)
+            for s in range(0, T, window):
+                last = run(x[:, s:s + window], first=(s == 0))
+        return last, run.states
 
 
 class _ShapeGraph:
     """One captured _layers_windows or _by_window: static ids in, (x, delta) of the last tokens and one tensor of every layer's final state
-    out (cloned per call, so that what a caller keeps is not overwritten by the next one)."""
+    out (cloned per call, so that what a caller keeps is not overwritten by the next one). All of them lie in the graph's pool."""
 
-    def __init__(self, model, ids, body, window, tail):
+    def __init__(self, model, ids, body, window, tail, stream, pool):
         mx = model.mix[0]
-        self.ids = torch.zeros_like(ids)
-        self.states = torch.empty(model.layers, ids.shape[0], mx.h, mx.dk, mx.dk, device=ids.device, dtype=torch.float32)
-        run = lambda: body(self.ids, window, tail, self.states)[0]
-        side = torch.cuda.Stream()
-        with warm_up(side):
-            run()
-            self.graph = torch.cuda.CUDAGraph()
-            with graph_capture(self.graph, side):
-                self.out = run()
-        self.held = model.held()
+
+        def run():
+            self.ids = torch.empty_like(ids)
+            self.states = torch.empty(model.layers, ids.shape[0], mx.h, mx.dk, mx.dk, device=ids.device, dtype=torch.float32)
+            return body(self.ids, window, tail, self.states)[0]
+
+        with warm_up(stream):
+            body(ids, window, tail)
+            self.graph, self.out, self.held = model.capture(stream, run, pool)
 
     def __call__(self, ids):
         self.ids.copy_(ids)
@@ -338,10 +398,8 @@ class _StepGraph:
             with warm_up(main):
                 self._pass()
                 main.synchronize()                                     # the pass's tensors crossed streams; they are free from here on
-                self.graph = torch.cuda.CUDAGraph()
-                with graph_capture(self.graph, main):
-                    self.out, self.states = self._pass()
-            self.held = self.m.held()
+                self.graph, (self.out, self.states), self.held = self.m.capture(main, self._pass)
+        self.ids.record_stream(torch.cuda.current_stream())            # made on the first caller's stream
         self.ids.copy_(ids)
         self.graph.replay()
         return self.out
@@ -384,17 +442,14 @@ class _WindowGraphs:
         with warm_up(side):
             _, st = self._pass(none, False)
             self._pass(st, True)
-            self.first = torch.cuda.CUDAGraph()
-            with graph_capture(self.first, side):
-                self.out_first, self.states = self._pass(none, False)
-            self.later = torch.cuda.CUDAGraph()
-            with graph_capture(self.later, side, pool=self.first.pool()):
-                self.out_later, _ = self._pass(self.states, True)
-        self.held = self.m.held()
+            self.first, (self.out_first, self.states), held = self.m.capture(side, lambda: self._pass(none, False))
+            self.later, (self.out_later, _), held2 = self.m.capture(side, lambda: self._pass(self.states, True), self.first.pool())
+            self.held = held + held2
 
     def __call__(self, ids, first):
         if self.first is None:
             self._capture()
+        self.ids.record_stream(torch.cuda.current_stream())            # made on the first caller's stream
         self.ids.copy_(ids)
         if first:
             self.first.replay()

@@ -1,4 +1,5 @@
 """Captured passes against what changes around them: caches that are outgrown, switches."""
+import copy
 import threading
 import weakref
 
@@ -71,3 +72,74 @@ def test_captures_while_another_thread_works():
     finally:
         stop.set(); t.join()
     assert seen and seen[0] > 0 and torch.isfinite(a).all()
+
+
+@pytest.mark.parametrize("mixer,T", [("aspin", 100), ("dspin", 100), ("aspin", 192), ("hspin", 100)])
+@pytest.mark.parametrize("what", ["decoder", "carried"])
+def test_two_callers_on_two_streams(mixer, T, what):
+    """Two threads, each on a stream of its own, send prompts of one shape through one model, whose captured pass of that shape has
+    one set of static tensors: every result is the one its prompt gets alone."""
+    m = lm(mixer, d=256, layers=3)
+    prompts = [[ids(2, T, 10 * w + i) for i in range(6)] for w in range(2)]
+
+    def run(dec, p):
+        if what == "decoder":
+            return dec.prefill(p), [st[0] for st in dec.states]
+        lg, st = m.forward_carried(p, 64, return_states=True)
+        return lg, [s[0] for s in st]
+
+    decs = [Decoder(m, batch=2) for _ in range(2)]
+    m.use_graphs = False
+    want = [[[t.clone() for t in (r[0], *r[1])] for r in (run(decs[w], p) for p in prompts[w])] for w in range(2)]
+    m.use_graphs = True
+    for p in (prompts[0][0], prompts[1][0]):
+        run(decs[0], p)                                               # seen, then captured
+    torch.cuda.synchronize()
+    got, start = [[], []], threading.Barrier(2)
+
+    def work(w):
+        with torch.no_grad(), torch.cuda.stream(torch.cuda.Stream()):
+            torch.cuda._sleep(1000 * (1 + w))
+            start.wait()
+            for _ in range(10):
+                for p in prompts[w]:
+                    lg, S = run(decs[w], p)
+                    got[w].append([t.clone() for t in (lg, *S)])
+            torch.cuda.current_stream().synchronize()
+
+    ts = [threading.Thread(target=work, args=(w,)) for w in range(2)]
+    [t.start() for t in ts]; [t.join() for t in ts]
+    for w in range(2):
+        assert len(got[w]) == 60
+        for i, g in enumerate(got[w]):
+            assert all(torch.equal(a, b) for a, b in zip(g, want[w][i % 6])), (w, i)
+
+
+@pytest.mark.parametrize("T", [64, 100])
+def test_inside_a_capture_of_the_caller(T):
+    m = lm("aspin")
+    a = ids(2, T, 1)
+    want = m.forward_carried(a, 64).clone()
+    m.forward_carried(a, 64)
+    g, x = torch.cuda.CUDAGraph(), a.clone()
+    with torch.cuda.graph(g):
+        out = m.forward_carried(x, 64)
+    g.replay()
+    assert torch.equal(out, want)
+
+
+def test_states_of_whole_windows_are_the_callers_own():
+    m = lm("aspin", d=1024, layers=2)                                 # 16 heads x 10 sequences: the window graphs
+    a, b = ids(10, 128, 1), ids(10, 128, 2)
+    _, sa = m.forward_carried(a, 64, return_states=True)
+    keep = [s[0].clone() for s in sa]
+    m.forward_carried(b, 64)
+    assert all(torch.equal(s[0], k) for s, k in zip(sa, keep))
+
+
+def test_a_copied_model_starts_without_graphs():
+    m = lm("aspin")
+    a = ids(2, 100, 1)
+    want = [m.forward_carried(a, 64) for _ in range(3)][-1]
+    c = copy.deepcopy(m)
+    assert not c._captured.shapes and torch.equal(c.forward_carried(a, 64), want)
