@@ -205,6 +205,46 @@ def need_cuda(*ts) -> None:
             raise RuntimeError("pragnosia_b200 ops run on CUDA tensors only (there is no CPU path)")
 
 
+class Cached:
+    """Tensors that one call made for all the later ones. Another stream than the one they were made on waits for the kernels that
+    made them, and the allocator is told, so that a cache replaced meanwhile is not handed out under that stream's kernels. A
+    copy of the module that holds one starts without it. What is made while the caller's stream is captured has no contents until
+    that graph is replayed: keep() leaves it uncached."""
+    __slots__ = ("key", "value", "tensors", "made_on", "done", "told", "kept")
+
+    def __init__(self, key, value, tensors):
+        self.key, self.value, self.tensors = key, value, [t for t in tensors if t.is_cuda]
+        self.made_on = self.done = None
+        self.told = set()
+        self.kept = True
+        if self.tensors and torch.cuda.is_current_stream_capturing():
+            self.kept = False
+        elif self.tensors:
+            here = torch.cuda.current_stream(self.tensors[0].device)
+            self.made_on, self.done = here.cuda_stream, here.record_event()
+
+    def get(self):
+        if self.made_on is not None:
+            raw = stream_of(self.tensors[0])
+            if raw != self.made_on and raw not in self.told and not torch.cuda.is_current_stream_capturing():
+                here = torch.cuda.current_stream(self.tensors[0].device)
+                here.wait_event(self.done)
+                for t in self.tensors:
+                    t.record_stream(here)
+                self.told.add(raw)
+        return self.value
+
+    def keep(self, old):
+        """What to store: this, or the cache as it was."""
+        return self if self.kept else old
+
+    def __deepcopy__(self, memo):
+        return None
+
+    def __reduce__(self):
+        return type(None), ()
+
+
 _capture_lock = threading.RLock()
 
 

@@ -14,6 +14,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
+from ._lib import Cached
 
 
 def rotate(x, theta, pos):
@@ -115,12 +116,13 @@ class AssocCarrier(nn.Module):
     def _consts(self):
         if torch.compiler.is_compiling():
             return self._build_consts()                 # traced into the caller's graph: nothing cached, nothing stale
-        key = self.consts_key()
-        if self._fused is None or self._fused[0] != key:
+        key, got = self.consts_key(), self._fused
+        if got is None or got.key != key:
             with torch.no_grad():
-                self._fused = (key, self._build_consts())
-            self._rot = None                            # the rotation table follows theta
-        return self._fused[1]
+                c = self._build_consts()
+            got = Cached(key, c, c.values())
+            self._fused = got.keep(self._fused)
+        return got.get()
 
     def forward(self, x, h0=None, pos0: int = 0):
         """x (B,T,d) on CUDA; h0 = (S (B,H,dk,dk) fp32, p0[, conv cache]) from the previous window or step, or None.
@@ -286,9 +288,12 @@ class AssocCarrier(nn.Module):
         need = (T + 63) // 64 * 64                                   # whole 64-token chunks
         if torch.compiler.is_compiling():
             return self._wrapped(ops.rot_table(c["theta"], need), need)
-        if self._rot is None or self._rot[0] != self.pos_wrap or self._rot[1].shape[1] < need:
-            self._rot = (self.pos_wrap, self._wrapped(ops.rot_table(c["theta"], need), need))
-        return self._rot[1]
+        got = self._rot
+        if got is None or got.key[0] != self.pos_wrap or got.key[1] is not c or got.value.shape[1] < need:
+            table = self._wrapped(ops.rot_table(c["theta"], need), need)
+            got = Cached((self.pos_wrap, c), table, [table])
+            self._rot = got.keep(self._rot)
+        return got.get()
 
     def _wrapped(self, table, need):
         if not self.pos_wrap:
@@ -299,9 +304,12 @@ class AssocCarrier(nn.Module):
         if torch.compiler.is_compiling():
             pos = torch.arange(T, device=device)
         else:
-            if self._pos is None or self._pos.numel() < T or self._pos.device != device:
-                self._pos = torch.arange(max(T, 512), device=device)
-            pos = self._pos[:T]
+            got = self._pos
+            if got is None or got.value.numel() < T or got.value.device != device:
+                pos = torch.arange(max(T, 512), device=device)
+                got = Cached(None, pos, [pos])
+                self._pos = got.keep(self._pos)
+            pos = got.get()[:T]
         return pos % self.pos_wrap if self.pos_wrap else pos
 
     def _rms_eps(self):

@@ -11,7 +11,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
-from ._lib import graph_capture, warm_up
+from ._lib import Cached, graph_capture, warm_up
 from .assoc import AssocCarrier
 from .spin import SpinCarrier
 
@@ -131,10 +131,13 @@ class LM(nn.Module):
 
     def _window_positions(self, T, window, device):
         """(position inside its window of every token, the same modulo the position table) for the first T tokens."""
-        if self._wpos is None or self._wpos[0] != (window, device) or self._wpos[1].numel() < T:
+        got = self._wpos
+        if got is None or got.key != (window, device) or got.value[0].numel() < T:
             pos = torch.arange(T, device=device) % window
-            self._wpos = ((window, device), pos, pos % self.p.num_embeddings)
-        return self._wpos[1][:T], self._wpos[2][:T]
+            both = (pos, pos % self.p.num_embeddings)
+            got = Cached((window, device), both, both)
+            self._wpos = got.keep(self._wpos)
+        return tuple(t[:T] for t in got.get())
 
     def _piece(self, B, window):
         """Tokens of a sequence that go through the layers together: whole windows, WINDOWS_TOKENS tokens over the batch at most (or

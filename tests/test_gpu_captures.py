@@ -32,7 +32,7 @@ def test_a_graph_outlives_the_caches_it_read(mixer, d, T):
     a = ids(2, T, 1)
     want = m.forward_carried(a, 64).clone()
     m.forward_carried(a, 64)
-    old = [weakref.ref(t) for c in m.held() if c is not None for t in (c if isinstance(c, tuple) else [c]) if torch.is_tensor(t)]
+    old = [weakref.ref(t) for c in m.held() if c is not None for t in c.tensors]
     m.forward_carried(ids(2, 3000, 2), 1024)                          # outgrows every cache
     m.forward_carried(ids(2, 333, 2), 64)
     torch.cuda.synchronize()
@@ -143,3 +143,39 @@ def test_a_copied_model_starts_without_graphs():
     want = [m.forward_carried(a, 64) for _ in range(3)][-1]
     c = copy.deepcopy(m)
     assert not c._captured.shapes and torch.equal(c.forward_carried(a, 64), want)
+
+
+@pytest.mark.parametrize("mixer,d", [("aspin", 256), ("dspin", 256), ("hspin", 256)])
+def test_constants_made_on_one_stream_and_used_on_another(mixer, d):
+    """The first pass of a model makes the constants its layers cache; a pass on another stream waits for them, and a cache replaced
+    meanwhile (another window) is not handed out under that stream's kernels."""
+    want = lm(mixer, d=d).forward_carried(ids(2, 100, 1), 64)
+    for trial in range(3):
+        m = lm(mixer, d=d)
+        torch.cuda.synchronize()
+        one, two = torch.cuda.Stream(), torch.cuda.Stream()
+        with torch.cuda.stream(one):
+            torch.cuda._sleep(20_000_000)                             # the constants' kernels are far from done when the other stream starts
+            a = m.forward_carried(ids(2, 100, 1), 64)
+        with torch.cuda.stream(two):
+            b = m.forward_carried(ids(2, 100, 1), 64)
+        with torch.cuda.stream(one):
+            m.forward_carried(ids(2, 1500, 1), 1024)                  # replaces the tables
+            junk = [torch.full((1 << 18,), 7.0, device=DEV) for _ in range(16)]
+        torch.cuda.synchronize()
+        assert torch.equal(a, want) and torch.equal(b, want)
+        del junk
+
+
+def test_constants_first_made_inside_a_capture_are_not_kept():
+    m = lm("aspin", d=256)
+    x = torch.randn(2, 70, 256, device=DEV).to(torch.bfloat16)
+    layer = m.mix[0]
+    want = copy.deepcopy(layer)(x)[0]
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        out = layer(x)[0]
+    assert torch.equal(layer(x)[0], want)                             # before the graph has ever run
+    g.replay()
+    assert torch.equal(out, want)
