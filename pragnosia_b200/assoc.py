@@ -131,9 +131,11 @@ class AssocCarrier(nn.Module):
         delta, st = self.mix(self.ln(x), h0)
         return x + delta, st
 
-    def mix(self, z, h0=None):
+    def mix(self, z, h0=None, inplace: bool | None = None):
         """The layer without its input norm and residual add: z = ln(x) in, (what is added to x, new state) out. The
-        language model fuses the norm and the add of neighbouring blocks into one kernel and calls this directly."""
+        language model fuses the norm and the add of neighbouring blocks into one kernel and calls this directly. inplace: whether
+        this call overwrites the state it was given (None: as inplace_state says)."""
+        inplace = self.inplace_state if inplace is None else inplace
         B, T, D = z.shape
         H, dk, d = self.h, self.dk, self.d
         sconv = getattr(self, "sconv", None)
@@ -155,12 +157,12 @@ class AssocCarrier(nn.Module):
             ops.key_topk_mask_(kp, self.key_topk)                     # in place, on this call's own projection buffer
         a_logit, g_logit = y[..., 3 * d:3 * d + H], y[..., 3 * d + H:3 * d + 2 * H]
         if T == 1:
-            o, S = self._step(qp, kp, vp, a_logit, g_logit, c, S0, shift)
+            o, S = self._step(qp, kp, vp, a_logit, g_logit, c, S0, shift, inplace)
             o = o.view(B, 1, d)
             self.sent = None
         else:
             bf16 = z.dtype == torch.bfloat16
-            S_out = S0 if (self.inplace_state and S0 is not None) else None
+            S_out = S0 if (inplace and S0 is not None) else None
             if bf16 and not self.delta and not self.hl_floor:
                 # one kernel between the two GEMMs: plumbing (normalise, gate, rotate) on the TMA tiles, decay gate, scan on
                 # the tensor cores, per-head RMS norm, token-major output
@@ -180,7 +182,7 @@ class AssocCarrier(nn.Module):
         delta = F.linear(o, c["ow"])
         if torch.is_tensor(p0):
             # a device-side position (graphed decode): with inplace_state the caller owns and updates it
-            p_new = p0 if self.inplace_state else p0 * 0 + T
+            p_new = p0 if inplace else p0 * 0 + T
         else:
             p_new = T
         return delta, ((S, p_new, cc) if sconv is not None else (S, p_new))
@@ -250,7 +252,7 @@ class AssocCarrier(nn.Module):
             bt = bt.clamp(min=0.75)                                   # beta = 1 makes the chunk inverse singular
         return bt
 
-    def _step(self, qp, kp, vp, a_logit, g_logit, c, S0, shift):
+    def _step(self, qp, kp, vp, a_logit, g_logit, c, S0, shift, inplace):
         """One token per sequence: the fused recurrent step. With an option that changes the gates, the log-decay / write
         strength are formed here and handed over as values instead of logits."""
         B, H, dk, d = qp.shape[0], self.h, self.dk, self.d
@@ -268,10 +270,10 @@ class AssocCarrier(nn.Module):
         o = torch.empty(B, d, device=qp.device, dtype=qp.dtype)
         _, S = ops.decode_step(q3, k3, v3, decay, S0, c["theta"], gate=gate, delta=self.delta, gate_is_logit=is_logit,
                                decay_A=decay_A, normalize=True, shift=shift, rms_weight=c["onw"], rms_eps=self._rms_eps(),
-                               out=o.view(B, H, dk), S_out=S0 if self.inplace_state else None)
+                               out=o.view(B, H, dk), S_out=S0 if inplace else None)
         return o, S
 
-    def step_from_projection(self, y2, S0, shift):
+    def step_from_projection(self, y2, S0, shift, inplace: bool | None = None):
         """The recurrent step of one token per sequence from the fused projection's output y2 (B, 3d+2h[+pad]) =
         [q | k | v | decay logits | gate logits]: one kernel (normalise, gates, rotate the state, write, read, per-head RMS
         norm). Returns (o (B,d), S); with inplace_state the state is updated where it lies. For a layer without options
@@ -280,7 +282,8 @@ class AssocCarrier(nn.Module):
         H, dk, d = self.h, self.dk, self.d
         y3 = y2.unsqueeze(1)
         qp, kp, vp = (y3[..., i * d:(i + 1) * d].unflatten(-1, (H, dk)) for i in range(3))
-        return self._step(qp, kp, vp, y3[..., 3 * d:3 * d + H], y3[..., 3 * d + H:3 * d + 2 * H], c, S0, shift)
+        return self._step(qp, kp, vp, y3[..., 3 * d:3 * d + H], y3[..., 3 * d + H:3 * d + 2 * H], c, S0, shift,
+                          self.inplace_state if inplace is None else inplace)
 
     def _rot_table(self, T, c):
         """(cos, sin) of position * theta for this layer's window positions (wrapped by pos_wrap when set); rebuilt when

@@ -181,9 +181,7 @@ class Decoder:
         for i, (mx, mp) in enumerate(zip(m.mix, m.mlp)):
             c = mx._consts()
             y, x = ops.skinny_linear(x, c["W"], c["b"], delta=delta, norm=mx.ln, want_sum=True)
-            mx.inplace_state = True
-            o, _ = mx.step_from_projection(y, self.states[i][0], self.shift)
-            mx.inplace_state = False
+            o, _ = mx.step_from_projection(y, self.states[i][0], self.shift, inplace=True)
             d1 = ops.skinny_linear(o, c["ow"])
             hmid, x = ops.skinny_linear(x, mp.a.weight, mp.a.bias, delta=d1, norm=mp.n, act="gelu", want_sum=True)
             delta = ops.skinny_linear(hmid, mp.b.weight, mp.b.bias)
@@ -223,9 +221,7 @@ class Decoder:
             c = mx._consts()
             (Wp, c1p, c2p, kp, ep), (Wa, c1a, c2a, ka, ea) = per[i]
             y = ops.batch_linear(x, Wp, folded=(sums, c1p, c2p, kp, ep))
-            mx.inplace_state = True
-            o, _ = mx.step_from_projection(y, self.states[i][0], self.shift)
-            mx.inplace_state = False
+            o, _ = mx.step_from_projection(y, self.states[i][0], self.shift, inplace=True)
             x, sums = ops.batch_linear(o, c["ow"], resid=x, want_sums=True)
             hmid = ops.batch_linear(x, Wa, act="gelu", folded=(sums, c1a, c2a, ka, ea))
             x, sums = ops.batch_linear(hmid, mp.b.weight, mp.b.bias, resid=x, want_sums=True)
@@ -251,9 +247,7 @@ class Decoder:
             st = self.states[i]
             x, z = m._add_norm(x, delta, mx.ln)
             if isinstance(mx, AssocCarrier):
-                mx.inplace_state = True
-                delta, new = mx.mix(z, (st[0], self.shift) + tuple(st[2:]))
-                mx.inplace_state = False
+                delta, new = mx.mix(z, (st[0], self.shift) + tuple(st[2:]), inplace=True)
                 if len(st) == 3:                               # the short convolution's context comes back as a new tensor
                     st[2].copy_(new[2])
             else:

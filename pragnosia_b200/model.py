@@ -99,14 +99,14 @@ class LM(nn.Module):
         y = x if delta is None else x + delta
         return y, norm(y)
 
-    def _layers(self, h, states):
+    def _layers(self, h, states, inplace=None):
         """Every (mixer, MLP) pair over h. Returns (x, delta): the residual stream and the last block's not-yet-added
         output, so the caller's final norm fuses that add as well. Each block's input norm is fused with the previous
-        block's residual add."""
+        block's residual add. inplace: the associative layers update the states where they lie (None: as each layer is set)."""
         x, delta = h, None
         for i, (mx, mp) in enumerate(zip(self.mix, self.mlp)):
             x, z = self._add_norm(x, delta, mx.ln)
-            delta, states[i] = mx.mix(z, states[i])
+            delta, states[i] = mx.mix(z, states[i], inplace) if isinstance(mx, AssocCarrier) else mx.mix(z, states[i])
             x, z = self._add_norm(x, delta, mp.n)
             delta = mp.ff(z)
         return x, delta
@@ -370,29 +370,23 @@ class _StepGraph:
         for sd in self.sides:
             sd.wait_event(fork)
         prev, out = None, None
-        try:
-            for w in range(self.NW):
-                st = streams[w % len(streams)]
-                evs = [torch.cuda.Event() for _ in range(m.layers)]
-                for mx in m.mix:
-                    mx.inplace_state = w > 0                           # later windows update the first window's state tensors
-                with torch.cuda.stream(st):
-                    x, delta = m._embed(self.ids[:, w * self.Tw:(w + 1) * self.Tw]), None
-                    for i, (mx, mp) in enumerate(zip(m.mix, m.mlp)):
-                        x, z = m._add_norm(x, delta, mx.ln)
-                        if prev is not None:
-                            st.wait_event(prev[i])                     # the state this layer enters with
-                        delta, states[i] = mx.mix(z, states[i])
-                        evs[i].record(st)
-                        x, z = m._add_norm(x, delta, mp.n)
-                        delta = mp.ff(z)
-                    out = (x, delta)
-                prev = evs
-            for sd in self.sides:
-                join = torch.cuda.Event(); join.record(sd); main.wait_event(join)
-        finally:
-            for mx in m.mix:
-                mx.inplace_state = False
+        for w in range(self.NW):
+            st = streams[w % len(streams)]
+            evs = [torch.cuda.Event() for _ in range(m.layers)]
+            with torch.cuda.stream(st):
+                x, delta = m._embed(self.ids[:, w * self.Tw:(w + 1) * self.Tw]), None
+                for i, (mx, mp) in enumerate(zip(m.mix, m.mlp)):
+                    x, z = m._add_norm(x, delta, mx.ln)
+                    if prev is not None:
+                        st.wait_event(prev[i])                         # the state this layer enters with
+                    delta, states[i] = mx.mix(z, states[i], inplace=w > 0)     # later windows update the first window's state tensors
+                    evs[i].record(st)
+                    x, z = m._add_norm(x, delta, mp.n)
+                    delta = mp.ff(z)
+                out = (x, delta)
+            prev = evs
+        for sd in self.sides:
+            join = torch.cuda.Event(); join.record(sd); main.wait_event(join)
         return out, states
 
     def __call__(self, ids):
@@ -422,22 +416,14 @@ class _WindowGraphs:
 
     def _pass(self, states, inplace):
         m = self.m
-        for mx in m.mix:
-            if isinstance(mx, AssocCarrier):
-                mx.inplace_state = inplace
-        try:
-            new = list(states)
-            out = m._layers(m._embed(self.ids), new)
-            if inplace:                        # states that came back as new tensors (the diagonal carrier) are copied home
-                for old, cur in zip(states, new):
-                    for a, b in zip(old, cur):
-                        if torch.is_tensor(a) and a.data_ptr() != b.data_ptr():
-                            a.copy_(b)
-            return out, new
-        finally:
-            for mx in m.mix:
-                if isinstance(mx, AssocCarrier):
-                    mx.inplace_state = False
+        new = list(states)
+        out = m._layers(m._embed(self.ids), new, inplace)
+        if inplace:                            # states that came back as new tensors (the diagonal carrier) are copied home
+            for old, cur in zip(states, new):
+                for a, b in zip(old, cur):
+                    if torch.is_tensor(a) and a.data_ptr() != b.data_ptr():
+                        a.copy_(b)
+        return out, new
 
     def _capture(self):
         none = [None] * self.m.layers

@@ -6,6 +6,7 @@ import weakref
 import pytest
 import torch
 
+from pragnosia_b200 import ops
 from pragnosia_b200.generate import Decoder
 from pragnosia_b200.model import LM
 
@@ -179,3 +180,28 @@ def test_constants_first_made_inside_a_capture_are_not_kept():
     assert torch.equal(layer(x)[0], want)                             # before the graph has ever run
     g.replay()
     assert torch.equal(out, want)
+
+
+def test_an_in_place_step_is_not_seen_by_other_callers(monkeypatch):
+    """A decode step updates its states where they lie; a layer call from another thread meanwhile leaves the state it was given alone."""
+    m = lm("aspin")
+    dec = Decoder(m, batch=5, use_graph=False)
+    dec.prefill(ids(5, 70, 1))
+    z, S = torch.randn(5, 1, 128, device=DEV).to(torch.bfloat16), torch.randn(5, 2, 64, 64, device=DEV)
+    keep, step, seen = S.clone(), ops.decode_step, []
+
+    def other():
+        with torch.no_grad():
+            m.mix[0].mix(z, (S, 3))
+
+    def hook(*a, **k):
+        if not seen:
+            seen.append(1)
+            t = threading.Thread(target=other)
+            t.start(); t.join()
+        return step(*a, **k)
+
+    monkeypatch.setattr(ops, "decode_step", hook)
+    before = dec.states[0][0].clone()
+    dec.step(ids(5, 1, 2)[:, 0])
+    assert seen and torch.equal(S, keep) and not torch.equal(dec.states[0][0], before)
