@@ -50,7 +50,7 @@ class Decoder:
         if stamp != self._stamp:
             self._graph, self._gen_key, self._stamp = None, None, stamp
         if m.windows_fit(w) and ids.is_cuda:
-            z, new = m._windows_pass(ids, w, 1)                  # only the last token leaves the last layer
+            z, new = m._windows_pass(ids, w, 1, graphs=self.use_graph)      # only the last token leaves the last layer
             n = (ids.shape[1] - 1) % w + 1
             if self.states is None:
                 self.states = [(S, n) for S in new]

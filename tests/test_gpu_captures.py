@@ -205,3 +205,14 @@ def test_an_in_place_step_is_not_seen_by_other_callers(monkeypatch):
     before = dec.states[0][0].clone()
     dec.step(ids(5, 1, 2)[:, 0])
     assert seen and torch.equal(S, keep) and not torch.equal(dec.states[0][0], before)
+
+
+@pytest.mark.parametrize("mixer", ["aspin", "dspin"])
+def test_a_decoder_without_graphs_captures_nothing(mixer):
+    m = lm(mixer)
+    a = ids(2, 100, 1)
+    dec = Decoder(m, batch=2, use_graph=False)
+    lg = [dec.prefill(a).clone() for _ in range(4)]
+    assert not m._captured.shapes and all(torch.equal(x, lg[0]) for x in lg)
+    with_graphs = Decoder(m, batch=2)
+    assert all(torch.equal(with_graphs.prefill(a), lg[0]) for _ in range(3)) and any(m._captured.shapes.values())
