@@ -216,3 +216,19 @@ def test_a_decoder_without_graphs_captures_nothing(mixer):
     assert not m._captured.shapes and all(torch.equal(x, lg[0]) for x in lg)
     with_graphs = Decoder(m, batch=2)
     assert all(torch.equal(with_graphs.prefill(a), lg[0]) for _ in range(3)) and any(m._captured.shapes.values())
+
+
+def test_the_mlps_switch_reaches_the_decode_step(monkeypatch):
+    m = lm("aspin")
+    calls, linear = [], ops.batch_linear
+    monkeypatch.setattr(ops, "batch_linear", lambda *a, **k: calls.append(k.get("act")) or linear(*a, **k))
+    dec = Decoder(m, batch=6, use_graph=False)
+    out = []
+    for fused in (True, False):
+        for mp in m.mlp:
+            mp.fused_up = fused
+        dec.prefill(ids(6, 70, 1))
+        calls.clear()
+        out.append(dec.step(ids(6, 1, 2)[:, 0]).float())
+        assert calls.count("gelu") == (len(m.mlp) if fused else 0)
+    assert float((out[0] - out[1]).norm() / out[1].norm()) < 2e-2
