@@ -492,6 +492,9 @@ int pgb_tc_wait_selftest(long long limit_cycles, void *stream);
 /* Which plain-rule tensor-core kernel head dim 64 uses: 0 (default) = the warp-specialised pipeline, 1 = the single-role
  * kernel that head dim 128 always uses. Process-wide; for A/B timing and tests. No counterpart in the reference. */
 int pgb_tc_set_variant(int variant);
+/* The three process-wide variants as one number (pgb_tc_set_variant | pgb_linear_act_set_variant << 4 | pgb_decode_set_variant << 12),
+ * 0 when none is set: a caller that keeps captured launches recaptures when it changes. */
+int pgb_variants(void);
 
 /* ---------------------------------------------------------------------------------------------------------
  * Rotation of channel pairs (2i, 2i+1) of x (B,H,T,D) by pos[t] * theta[h][i]; any even D.

@@ -74,6 +74,8 @@ int linear_gelu_launch(const void *, const void *, const void *, void *, long lo
 int linear_gelu_error_flag(int *);
 int linear_gelu_set_variant(int);
 int decode_set_variant(int);
+int linear_gelu_variant();
+int decode_variant();
 int skinny_linear_launch(const void *, const void *, const void *, const void *, int, float, const void *, const void *, int, void *,
                          void *, int, int, int, int, cudaStream_t);
 int add_norm_launch(const void *, const void *, const void *, const void *, float, int, void *, void *, long long, int, int,
@@ -446,6 +448,23 @@ int pgb_aspin_layer_prefill_windows_ex(const void *qp, const void *kp, const voi
     a.la_raw = decay_logits; a.la_sb = aux_stride_b; a.la_st = aux_stride_t; a.decay_A = decay_A;
     a.rms_w = rms_weight; a.rms_eps = rms_eps; a.o_token_major = 1;
     a.raw = 1; a.raw_sb = in_stride_b; a.raw_st = in_stride_t; a.gate_raw = gate_logits; a.rot = rot_table; a.rot_T = rot_T;
+    if (g_tc_variant != 0) {
+        // the single-role kernel asked for: it walks one window of one sequence after the other, the state handed on in S_out
+        for (int b = 0; b < B; ++b)
+            for (int t0 = 0; t0 < T; t0 += window) {
+                PrefillArgs w = a;
+                auto at = [&](const void *base, size_t elements) { return base ? (const void *)((const char *)base + 2 * elements) : nullptr; };
+                const size_t in = (size_t)b * in_stride_b + (size_t)t0 * in_stride_t, aux = (size_t)b * aux_stride_b + (size_t)t0 * aux_stride_t;
+                w.q = at(qp, in); w.k = at(kp, in); w.v = at(vp, in); w.la_raw = at(decay_logits, aux); w.gate_raw = at(gate_logits, aux);
+                w.o = (char *)o + 2 * ((size_t)b * T + t0) * H * D;
+                w.S_out = S_out + (size_t)b * H * D * D;
+                w.S0 = t0 > 0 ? w.S_out : S0 ? S0 + (size_t)b * H * D * D : nullptr;
+                w.B = 1; w.T = T - t0 < window ? T - t0 : window;
+                const int rc = tc_dispatch(w, PGB_BF16, D, (cudaStream_t)stream);
+                if (rc != PGB_OK) return rc;
+            }
+        return PGB_OK;
+    }
     a.seg_len = window; a.seg_rotates = 1; a.seg_states = T > window ? (const float *)scratch : nullptr;
     if (T > window) {
         const int rc = segment_states_launch(a, (float *)scratch, (cudaStream_t)stream);
@@ -688,6 +707,8 @@ int pgb_tc_set_variant(int variant) {
     g_tc_variant = variant;
     return PGB_OK;
 }
+
+int pgb_variants(void) { return g_tc_variant | linear_gelu_variant() << 4 | decode_variant() << 12; }
 
 int pgb_tc_wait_selftest(long long limit_cycles, void *stream) {
     if (limit_cycles < 1 || limit_cycles > (1ll << 31)) return PGB_ERR_BAD_SHAPE;      // at most about a second of SM clock

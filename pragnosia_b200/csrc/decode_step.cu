@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(DW_WARPS * 32) decode_step_warp_kernel(DecodeA
 // served by 256 threads than by one warp's few hundred instructions in a row; batch 1024: the same 70 us (the HBM rate).
 constexpr int DW_MIN_UNITS = 512;
 static int g_decode_variant = 0;
+int decode_variant() { return g_decode_variant; }
 int decode_set_variant(int v) {
     if (v < 0 || v > 2) return PGB_ERR_BAD_SHAPE;
     g_decode_variant = v;

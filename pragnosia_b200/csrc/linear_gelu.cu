@@ -417,6 +417,7 @@ linear_gelu_pair_kernel(const __grid_constant__ CUtensorMap mx, const __grid_con
 // the GELU, so the single-CTA kernel stays the default.
 // Bits 1-2 pick the tile width (0 or 1: 256, 2: 192) for timing and tests.
 static int g_lg_variant = 0;
+int linear_gelu_variant() { return g_lg_variant; }
 int linear_gelu_set_variant(int v) {
     if (v < 0 || v > 5 || (v >> 1) > 2) return PGB_ERR_BAD_SHAPE;
     g_lg_variant = v;

@@ -11,7 +11,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
-from ._lib import Cached, graph_capture, warm_up
+from ._lib import Cached, graph_capture, lib, warm_up
 from .assoc import AssocCarrier
 from .spin import SpinCarrier
 
@@ -82,9 +82,10 @@ class LM(nn.Module):
 
     def weights_stamp(self):
         """Changes whenever a captured graph of this model would compute with something stale: a parameter that moved
-        (another dtype or device) or a mixer whose derived constants must be rebuilt (an in-place update, load_state_dict)."""
+        (another dtype or device), a mixer whose derived constants must be rebuilt (an in-place update, load_state_dict), or
+        another kernel variant chosen (pgb_tc_set_variant and its like)."""
         ptrs = tuple(p.data_ptr() for p in self.parameters())
-        return ptrs, tuple(mx.consts_key() for mx in self.mix if isinstance(mx, AssocCarrier))
+        return ptrs, lib().pgb_variants(), tuple(mx.consts_key() for mx in self.mix if isinstance(mx, AssocCarrier))
 
     def _embed(self, x):
         return self.e(x) + self.p(torch.arange(x.shape[1], device=x.device) % self.p.num_embeddings)

@@ -149,6 +149,14 @@ def test_new_entry_points_reject_bad_calls(L):
     assert tok(nb=None) == 1 and tok(wb=10) == 2 and tok(B=5) == 7 and tok(D=96) == 3
 
 
+def test_variants_as_one_number(L):
+    assert L.pgb_variants() == 0
+    assert L.pgb_tc_set_variant(1) == 0 and L.pgb_linear_act_set_variant(3) == 0 and L.pgb_decode_set_variant(2) == 0
+    assert L.pgb_variants() == 1 + (3 << 4) + (2 << 12)
+    assert L.pgb_tc_set_variant(0) == 0 and L.pgb_linear_act_set_variant(0) == 0 and L.pgb_decode_set_variant(0) == 0
+    assert L.pgb_variants() == 0
+
+
 def test_bench_table_names_are_kernel_bench_cases():
     """bench.py's per-kernel table is built from kernel_bench cases by name: every name it asks for exists."""
     import ast

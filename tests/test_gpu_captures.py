@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from pragnosia_b200 import ops
+from pragnosia_b200._lib import lib
 from pragnosia_b200.generate import Decoder
 from pragnosia_b200.model import LM
 
@@ -232,3 +233,34 @@ def test_the_mlps_switch_reaches_the_decode_step(monkeypatch):
         out.append(dec.step(ids(6, 1, 2)[:, 0]).float())
         assert calls.count("gelu") == (len(m.mlp) if fused else 0)
     assert float((out[0] - out[1]).norm() / out[1].norm()) < 2e-2
+
+
+@pytest.mark.parametrize("B,T,window", [(1, 64, 64), (2, 200, 64), (2, 257, 128)])
+def test_the_single_role_variant_reaches_windows(B, T, window):
+    """pgb_tc_set_variant(1): a pass over windows is that kernel window by window, and a graph captured before is retired."""
+    L = lib()
+    m = lm("aspin", d=256)
+    a = ids(B, T, 1)
+    first = [m.forward_carried(a, window) for _ in range(3)][-1]
+    layer = m.mix[0]
+    z, S0 = torch.randn(B, T, 256, device=DEV).to(torch.bfloat16), torch.randn(B, 4, 64, 64, device=DEV)
+    c = layer._consts()
+    y = torch.nn.functional.linear(z, c["W"], c["b"])
+    try:
+        assert L.pgb_tc_set_variant(1) == 0 and L.pgb_variants() == 1
+        S, outs = S0, []
+        for s in range(0, T, window):
+            yw = y[:, s:s + window]
+            q, k, v = (yw[..., i * 256:(i + 1) * 256].unflatten(-1, (4, 64)) for i in range(3))
+            o, S, _ = ops.layer_prefill(q, k, v, yw[..., 772:776], yw[..., 768:772], c["A"], layer._rot_table(window, c), S, theta=c["theta"],
+                                        shift=float(window), rms_weight=c["onw"], rms_eps=layer._rms_eps())
+            outs.append(o)
+        q, k, v = (y[..., i * 256:(i + 1) * 256].unflatten(-1, (4, 64)) for i in range(3))
+        o, S1 = ops.layer_prefill_windows(q, k, v, y[..., 772:776], y[..., 768:772], c["A"], layer._rot_table(window, c), c["theta"], window, c["onw"],
+                                          layer._rms_eps(), S0=S0)
+        assert torch.equal(o, torch.cat(outs, 1)) and torch.equal(S1, S)
+        second = m.forward_carried(a, window)
+        assert L.pgb_variants() == m._captured.stamp[1] == 1
+    finally:
+        L.pgb_tc_set_variant(0)
+    assert float((first.float() - second.float()).norm() / first.float().norm()) < 2e-2
