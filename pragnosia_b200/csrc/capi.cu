@@ -348,6 +348,7 @@ int pgb_aspin_prefill_segments_fwd(const void *q, const void *k, const void *v, 
     if (!dtype_ok(o_dtype)) return PGB_ERR_BAD_DTYPE;
     if (B <= 0 || H <= 0 || T <= 0) return PGB_ERR_BAD_SHAPE;
     if (D != 64) return PGB_ERR_UNSUPPORTED_DIM;
+    if (S0 == S_out) return PGB_ERR_BAD_SHAPE;                        // the first segment reads S0 while the last writes S_out
     const long long need = pgb_aspin_prefill_segments_scratch_bytes(B, H, T, D);
     if (need == 0 || scratch_bytes < need) return PGB_ERR_BAD_SHAPE;
     if (!aligned(q, 16) || !aligned(k, 16) || !aligned(v, 16) || !aligned(o, 16) || !aligned(S_out, 16) || (S0 && !aligned(S0, 16)) ||

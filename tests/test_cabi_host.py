@@ -149,6 +149,21 @@ def test_new_entry_points_reject_bad_calls(L):
     assert tok(nb=None) == 1 and tok(wb=10) == 2 and tok(B=5) == 7 and tok(D=96) == 3
 
 
+def test_segments_and_windows_refuse_an_in_place_state(L):
+    """Their CTAs run side by side: one would write the state that another has yet to read."""
+    one, st = ctypes.c_void_p(0x1000), ctypes.c_void_p(0x2000)
+    n = L.pgb_aspin_prefill_segments_scratch_bytes(1, 1, 4096, 64)
+    assert n > 0
+    seg = lambda S0, S: L.pgb_aspin_prefill_segments_fwd(one, one, one, one, S0, None, None, 0.0, one, 1, S, None, one, n, 1, 1, 4096, 64, None)
+    assert seg(st, st) == 2
+    win = lambda S0, S: L.pgb_aspin_layer_prefill_windows_ex(one, one, one, 4096, 64, one, one, 4096, 64, one, one, 64, one, S0, one, 1e-5, one, S, one,
+                                                             1 << 30, 64, 1, 1, 128, 64, None)
+    assert win(st, st) == 2
+    delta = lambda S0, S: L.pgb_aspin_delta_layer_windows_ex(one, one, one, 4096, 64, one, one, 4096, 64, one, one, one, S0, one, 1e-5, one, S, one,
+                                                             1 << 30, 64, 1, 1, 128, 64, None)
+    assert delta(st, st) == 2
+
+
 def test_variants_as_one_number(L):
     assert L.pgb_variants() == 0
     assert L.pgb_tc_set_variant(1) == 0 and L.pgb_linear_act_set_variant(3) == 0 and L.pgb_decode_set_variant(2) == 0
