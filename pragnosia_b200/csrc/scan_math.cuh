@@ -21,13 +21,22 @@ __device__ __forceinline__ f2 f2_neg(f2 a) { return a ^ 0x8000000080000000ull; }
 
 constexpr float SM_MAGIC = 12582912.f;                                // 1.5 * 2^23: adding it leaves the nearest integer in the low bits
 
-// e^x of two values; arguments are taken into [-87, 88.7] (a NaN stays one)
-__device__ __forceinline__ f2 f2_exp(float x0, float x1) {
-    asm("max.NaN.f32 %0, %0, 0fC2AE0000;" : "+f"(x0));                // -87
-    asm("max.NaN.f32 %0, %0, 0fC2AE0000;" : "+f"(x1));
-    asm("min.NaN.f32 %0, %0, 0f42B16666;" : "+f"(x0));                // 88.7
-    asm("min.NaN.f32 %0, %0, 0f42B16666;" : "+f"(x1));
-    const f2 x = f2_pack(x0, x1);
+// e^x of two values in [-F2_EXP_MAX, F2_EXP_MAX]. What may lie outside (results that are not normal, infinities, NaN) goes to
+// expf: the caller folds its arguments with f2_exp_fold and looks once for a whole tile of them -- a branch per value held up the
+// independent ones behind it (a training pass of B16 T512 D704: 99 -> 105 us).
+constexpr float F2_EXP_MAX = 87.f;
+__device__ __forceinline__ void f2_exp_fold(float &top, f2 x) {       // the largest magnitude so far; NaN once there was one
+    float a, b;
+    f2_unpack(x, a, b);
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(a)));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(b)));
+}
+__device__ __forceinline__ f2 f2_expf(f2 x) {                         // any argument
+    float a, b;
+    f2_unpack(x, a, b);
+    return f2_pack(expf(a), expf(b));
+}
+__device__ __forceinline__ f2 f2_exp(f2 x) {
     const f2 t = f2_fma(x, f2_both(1.44269504f), f2_both(SM_MAGIC)), n = f2_add(t, f2_both(-SM_MAGIC));
     f2 r = f2_fma(n, f2_both(-0.693145752f), x);                      // ln 2 in two parts, the first with trailing zeros
     r = f2_fma(n, f2_both(-1.42860677e-6f), r);
