@@ -180,6 +180,10 @@ def one_gpu() -> bool:
     return _gpus == 1
 
 
+def sm_count(device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
 def on_device_of(fn):
     """Decorator for the tensor-level wrappers: the library reads CUDA's CURRENT device (SM count, kernel attributes, its
     per-device scratch array and error flags), so a call whose first tensor lives on another GPU runs with that GPU made

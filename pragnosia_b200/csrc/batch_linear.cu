@@ -312,8 +312,7 @@ int batch_linear_launch(const void *x, const void *W, const void *bias, void *y,
                         int parts_in, const float *c1, const float *c2, int norm_kind, float eps, const void *resid, float *stats_out,
                         int late_consts, cudaStream_t stream) {
     const BlFused f{stats_in, parts_in, c1, c2, norm_kind, eps, (const __nv_bfloat16 *)resid, stats_out, late_consts};
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     // the narrowest slab that still gives about one CTA per SM: every CTA re-reads x from the L2, so fewer, wider CTAs
     // once the grid would pass the SM count. A residual (and the row sums that go with it) is taken by the narrowest only.
     const int bn = (resid != nullptr || stats_out != nullptr || (N + 15) / 16 <= sms) ? 16 : ((N + 31) / 32 <= sms ? 32 : 64);

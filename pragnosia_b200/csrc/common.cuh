@@ -20,6 +20,13 @@ inline int check_launch(const char *where) {
     return PGB_OK;
 }
 
+// multiprocessors of the current device (asked per call: cheap, and right when the caller switches devices)
+inline int sm_count() {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 inline bool aligned(const void *p, size_t n) { return (reinterpret_cast<uintptr_t>(p) % n) == 0; }
 
 __device__ __forceinline__ float to_f32(float x) { return x; }

@@ -384,15 +384,6 @@ lambda_scan_bwd_kernel(const float *__restrict__ g, const float *__restrict__ u,
 
 namespace {
 
-struct DevInfo { int sms = 0; bool ok = false; };
-DevInfo dev_info() {
-    // queried per call: cheap, and correct when the caller switches devices
-    DevInfo d; int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return d;
-    if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return d;
-    d.ok = true; return d;
-}
-
 struct LsArgs {
     const float *u, *lm, *an; long long sb, st; const float *h0r, *h0i; float *y, *hro, *hio, *hia;
     int B, T, D;
@@ -494,8 +485,7 @@ int lambda_scan_pick_ts(int B, int T, int D, int vec, int sms, int force_ts) {
 int lambda_scan_launch(const float *u, const float *lm, const float *an, long long sb, long long st, const float *h0r,
                        const float *h0i, float *y, float *hro, float *hio, float *hia, int B, int T, int D, int force_ts,
                        cudaStream_t stream) {
-    DevInfo di = dev_info();
-    const int sms = di.ok ? di.sms : 148;
+    const int sms = sm_count();
     const int vec = ls_vec(D, sb, st, u, lm, an, y, hia, hro, hio, h0r, h0i);
     int ts = lambda_scan_pick_ts(B, T, D, vec, sms, force_ts);
     // the wide form where its warps outnumber what the form that loads ahead can keep resident
@@ -508,9 +498,8 @@ int lambda_scan_launch(const float *u, const float *lm, const float *an, long lo
 int lambda_scan_bwd_launch(const float *g, const float *u, const float *lm, const float *an, long long sb, long long st,
                            const float *hr_all, const float *hi_all, const float *gli, float *du, float *dlm, float *dan,
                            float *dh0r, float *dh0i, int B, int T, int D, cudaStream_t stream) {
-    DevInfo di = dev_info();
     const int vec = ls_vec(D, sb, st, g, u, lm, an, hr_all, hi_all, gli, du, dlm, dan, dh0r, dh0i);
-    const int ts = ls_pick(B, T, D, vec, 4, di.ok ? di.sms : 148, LS_BWD_CTAS_PER_SM);
+    const int ts = ls_pick(B, T, D, vec, 4, sm_count(), LS_BWD_CTAS_PER_SM);
     return launch_any(vec, ts, LsBwdArgs{g, u, lm, an, sb, st, hr_all, hi_all, gli, du, dlm, dan, dh0r, dh0i, B, T, D}, stream);
 }
 

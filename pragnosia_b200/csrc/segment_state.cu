@@ -265,11 +265,11 @@ size_t segment_scratch_bytes(int B, int H, int T, int seg_len) {
 // Tokens of a segment for prepared chains of T tokens, 0: not worth cutting. Where the chains leave SMs idle, a chunk costs its walk
 // 1.3 us and the state pass 0.9, the two launches before the walk about 7 (train of 44 chains of 32 chunks: 45 us whole).
 int segment_len_prepared(long long BH, int T) {
-    const int NC = (T + TC_C - 1) / TC_C;
-    if (NC < 16 || BH * 2 > 148) return 0;
+    const int NC = (T + TC_C - 1) / TC_C, sms = sm_count();
+    if (NC < 16 || BH * 2 > sms) return 0;
     int best = 0;
     double cost = 1.3 * NC;
-    for (int n = 2; n * BH <= 148; ++n) {
+    for (int n = 2; n * BH <= sms; ++n) {
         const int len = (NC + n - 1) / n;
         if (len < 2) break;
         if (len * TC_C <= SG_MAX_PREPARED && len * 2.2 + 7.0 < cost) { cost = len * 2.2 + 7.0; best = len * TC_C; }

@@ -11,7 +11,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
-from ._lib import Cached, graph_capture, lib, warm_up
+from ._lib import Cached, graph_capture, lib, sm_count, warm_up
 from .assoc import AssocCarrier
 from .spin import SpinCarrier
 
@@ -226,7 +226,7 @@ class LM(nn.Module):
         # Fewer chains than SMs, or a ragged last window: layer by layer over the whole sequence (or, on mixers without a call over all
         # windows, window by window: seven launches a layer and window, whose issue from Python took longer than they did). With more
         # chains and whole windows the window-by-window graph below keeps the GPU as full and its activations in the L2.
-        all_windows = self.windows_fit(window) and x.is_cuda and (B * self.mix[0].h < 148 or T % window)
+        all_windows = self.windows_fit(window) and x.is_cuda and (B * self.mix[0].h < sm_count(x.device) or T % window)
         whole = T % window == 0 and T >= window
         if all_windows or (x.is_cuda and self._replays(window) and not whole):
             z, states = self._windows_pass(x, window, tail)

@@ -6,7 +6,7 @@ import weakref
 import pytest
 import torch
 
-from pragnosia_b200 import ops
+from pragnosia_b200 import model as M, ops
 from pragnosia_b200._lib import lib
 from pragnosia_b200.generate import Decoder
 from pragnosia_b200.model import LM
@@ -264,3 +264,16 @@ def test_the_single_role_variant_reaches_windows(B, T, window):
     finally:
         L.pgb_tc_set_variant(0)
     assert float((first.float() - second.float()).norm() / first.float().norm()) < 2e-2
+
+
+@pytest.mark.parametrize("sms,over_all", [(3, False), (4, False), (5, True)])
+def test_the_form_of_a_pass_follows_the_devices_sm_count(sms, over_all, monkeypatch):
+    """Four chains of two sequences: one call over all windows where there are more SMs than that, else the graph window by window."""
+    m = lm("aspin")
+    a = ids(2, 128, 1)
+    want = m.forward_carried(a, 64)
+    monkeypatch.setattr(M, "sm_count", lambda device: sms)
+    m._captured.windows.clear()
+    got = m.forward_carried(a, 64)
+    assert bool(m._captured.windows) != over_all
+    assert float((got.float() - want.float()).norm() / want.float().norm()) < 2e-2
