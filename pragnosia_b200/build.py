@@ -42,7 +42,7 @@ def build_host(force: bool = False) -> None:
     inc = [*ext.include_paths(), str(Path(NVCC).parents[1] / "include"), sysconfig.get_paths()["include"]]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-DTORCH_EXTENSION_NAME={HOST.stem}",
            "-DTORCH_API_INCLUDE_EXTENSION_H", *(f"-I{d}" for d in inc), str(HOST_SRC), "-o", str(HOST), *(f"-L{d}" for d in ext.library_paths()),
-           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", f"-L{LIBDIR}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]
+           "-lc10", "-lc10_cuda", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", f"-L{LIBDIR}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"{cmd[0]} failed for {HOST_SRC.name}:\n{r.stdout}\n{r.stderr}")

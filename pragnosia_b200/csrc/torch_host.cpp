@@ -2,6 +2,7 @@
 // library call and the autograd nodes, in C++. A call of a few microseconds on the GPU spent 15 us in Python, a training pass of
 // the scan (B16 T512 D704: 104 us of kernels) 160, most of it in the autograd functions' Python frames. The C ABI stays what the
 // kernels are reached by; this file only prepares its arguments, and ops.py / scan_kernel.py / assoc_kernel.py call it.
+#include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
@@ -15,8 +16,9 @@ using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
 constexpr int CHUNK = 64;
-// bytes of per-chunk states the fp32 plain prefill may take; beyond (B*H*T > 33 M at D = 64) it walks the chains
-constexpr long long FP32_CHUNK_SCRATCH = 8LL << 30;
+// Bytes of per-chunk states the fp32 plain prefill takes at most: more chains or chunks than that go one group after the other. Without
+// a limit 768 chains of 4096 tokens took 805 MB for 3.41 ms; 3.49 at 256 MiB, 3.66 at 64, 5.2 at 16.
+constexpr long long FP32_SCRATCH = 256LL << 20;
 
 void check(int status, const char *what) {
     if (status == PGB_OK) return;
@@ -215,6 +217,36 @@ Tensor state_out(const OptTensor &S_out, const Tensor &ref, int64_t B, int64_t H
                       "S_out must be a contiguous fp32 (B,H,D,D) tensor");
     return *S_out;
 }
+// The plain rule in fp32 with the chunks of a sequence side by side (prefill_fp32_chunk.cu), in groups whose scratch is bounded: whole
+// batch rows, or some heads of one, or (a chain that is too long by itself) one chain piece by piece with its state handed on. False:
+// the scratch could not be had, nothing was launched.
+bool prefill_fp32_grouped(const Tensor &q, const Tensor &k, const Tensor &v, const Tensor &la, const Tensor &S0, const Tensor &theta, const Tensor &shift,
+                          double shift_host, const Tensor &o, const Tensor &S, const Tensor &sent, void *stream) {
+    const long long B = q.size(0), H = q.size(1), T = q.size(2), D = q.size(3), NC = (T + CHUNK - 1) / CHUNK;
+    const long long chunk = pgb_aspin_prefill_fp32_scratch_bytes(1, 1, CHUNK, D), chain = pgb_aspin_prefill_fp32_scratch_bytes(1, 1, T, D);
+    const long long chains = std::min(B * H, std::max(1LL, FP32_SCRATCH / chain)), piece = chain <= FP32_SCRATCH ? T : FP32_SCRATCH / chunk * CHUNK;
+    const long long nb = std::max(1LL, chains / H), nh = std::min(chains, H);
+    const long long n = pgb_aspin_prefill_fp32_scratch_bytes(nb, nh, std::min(piece, T), D);
+    Tensor scratch;
+    try {
+        scratch = bytes(q, n);
+    } catch (const c10::OutOfMemoryError &) {
+        return false;
+    }
+    char *out = static_cast<char *>(vp(o));
+    for (long long b = 0; b < B; b += nb)
+        for (long long h = 0; h < H; h += nh)
+            for (long long t = 0; t < T; t += piece) {
+                const long long c = b * H + h, Bn = std::min(nb, B - b), Hn = std::min(nh, H - h), Tn = std::min(piece, T - t), row = c * T + t;
+                const float *first = t > 0 ? fp(S) + c * D * D : S0.defined() ? fp(S0) + c * D * D : nullptr;
+                check(pgb_aspin_prefill_fp32_fwd(fp(q) + row * D, fp(k) + row * D, fp(v) + row * D, fp(la) + row, first,
+                                                 t == 0 && theta.defined() ? fp(theta) + h * (D / 2) : nullptr, fp(shift), shift_host,
+                                                 out + row * D * o.element_size(), code(o), fp(S) + c * D * D,
+                                                 sent.defined() ? static_cast<char *>(vp(sent)) + (c * NC + t / CHUNK) * D * D * 2 : nullptr, vp(scratch), n,
+                                                 Bn, Hn, Tn, D, stream), "pgb_aspin_prefill_fp32_fwd");
+            }
+    return true;
+}
 using ScanOut = std::tuple<Tensor, Tensor, OptTensor>;
 // out_type: -1 = q's (fp32 where q is neither fp32 nor bf16), else a dtype code
 ScanOut prefill(const Tensor &q_, const Tensor &k_, const Tensor &v_, const Tensor &la_, const OptTensor &beta_, const OptTensor &S0_, const OptTensor &theta_,
@@ -246,15 +278,12 @@ ScanOut prefill(const Tensor &q_, const Tensor &k_, const Tensor &v_, const Tens
             return {o, S, some(sent)};
         }
     }
-    if (!beta.defined() && dt == at::kFloat && precision != PGB_PREFILL_TENSOR && B * H <= 65535) {
-        const long long n = pgb_aspin_prefill_fp32_scratch_bytes(B, H, T, D);     // fp32 plain rule: the chunks side by side
-        if (n <= FP32_CHUNK_SCRATCH) {
-            const Tensor scratch = bytes(q, n);
-            check(pgb_aspin_prefill_fp32_fwd(fp(q), fp(k), fp(v), fp(la), fp(S0), fp(theta), fp(shift), shift_host, vp(o), oc, fp(S), vp(sent), vp(scratch), n,
-                                             B, H, T, D, dev.stream), "pgb_aspin_prefill_fp32_fwd");
-            return {o, S, some(sent)};
-        }
-    }
+    // fp32 plain rule: the chunks side by side, also where the chains alone fill the GPU (1024 chains of 8 chunks: 616 us against the
+    // walk's 776; 24 of 64: 134 against 1258). A single chunk a chain at D = 64 is the walk's: 96 .. 1024 chains 31 .. 121 us against 32 .. 130.
+    if (!beta.defined() && dt == at::kFloat && precision != PGB_PREFILL_TENSOR && B > 0 && H > 0 && T > 0 && B * H <= 65535 && (D == 64 || D == 128) &&
+        !(D == 64 && T <= CHUNK && 2 * B * H > at::cuda::getCurrentDeviceProperties()->multiProcessorCount) &&
+        prefill_fp32_grouped(q, k, v, la, S0, theta, shift, shift_host, o, S, sent, dev.stream))
+        return {o, S, some(sent)};
     check(pgb_aspin_prefill_fwd(vp(q), vp(k), vp(v), code(q), fp(la), fp(beta), fp(S0), fp(theta), fp(shift), shift_host, vp(o), oc, fp(S), vp(sent), B, H, T,
                                 D, precision, dev.stream), "pgb_aspin_prefill_fwd");
     return {o, S, some(sent)};
