@@ -105,3 +105,15 @@ def test_layer_traces_whole(monkeypatch, delta):
         ep = torch._dynamo.export(layer)(torch.randn(2, 128, 128).to(BF))
         used = [str(n.target) for n in ep.graph_module.graph.nodes if n.op == "call_function"]
         assert used.count("pragnosia_b200.add_norm") == 2
+
+
+def test_training_entry_points_under_fake_tensors():
+    """A torch_dispatch mode (fake tensors, make_fx, selective checkpointing) sees the registered operators, not the C++ node behind
+    an eager call."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from pragnosia_b200.assoc_kernel import prep_kernel
+    with FakeTensorMode():
+        qp, kp, vp = (torch.empty(2, 100, 3, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3))
+        th, pos = torch.empty(3, 32, device="cuda"), torch.empty(100, device="cuda", dtype=torch.long)
+        for t in prep_kernel(qp, kp, vp, None, th, pos):
+            assert tuple(t.shape) == (2, 3, 100, 64) and t.dtype == torch.bfloat16 and t.requires_grad

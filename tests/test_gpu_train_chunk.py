@@ -42,3 +42,32 @@ def test_fused_backward_matches_autograd_through_the_oracle(delta, D, T):
     assert rel(o.detach().cpu(), o_r.detach()) <= 3e-3 and rel(S.detach().cpu(), S_r.detach()) <= 1e-5
     for n in names:                                                   # bf16 gradients; the saved states are bf16 as the operators keep them
         assert rel(dev[n].grad.cpu(), ref[n].grad) <= 4e-3, (n, rel(dev[n].grad.cpu(), ref[n].grad))
+
+
+def _training_calls():
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    q, k, v = (torch.nn.functional.normalize(rn(2, 3, 100, 64), dim=-1).bfloat16().requires_grad_() for _ in range(3))
+    la, be = (-0.1 * torch.rand(2, 3, 100, device="cuda")).requires_grad_(), torch.rand(2, 3, 100, device="cuda").requires_grad_()
+    qp, kp, vp = (rn(2, 100, 3, 64).bfloat16().requires_grad_() for _ in range(3))
+    th, pos = torch.rand(3, 32, device="cuda"), torch.arange(100, device="cuda")
+    return {"plain": (assoc_kernel.assoc_scan_kernel, (q, k, v, la), ("prefix_scan", "assoc_out")),
+            "delta": (assoc_kernel.delta_scan_kernel, (q, k, v, la, be), ("delta_inv", "delta_loop_fwd", "assoc_out")),
+            "prep": (lambda *x: (sum(assoc_kernel.prep_kernel(*x, None, th, pos)),), (qp, kp, vp), ("assoc_prep",))}
+
+
+@pytest.mark.parametrize("what", ["plain", "delta", "prep"])
+@torch.enable_grad()
+def test_a_tracer_sees_operators(what):
+    """make_fx of an eager training call records the registered operators; run without them the graph would hold the traced call's
+    results as constants."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    f, args, ops_seen = _training_calls()[what]
+    w = torch.randn(2, 3, 100, 64, device="cuda")
+    gm = make_fx(lambda *x: torch.autograd.grad((f(*x)[0].float() * w).sum(), x))(*args)
+    code = gm.code
+    assert all(f"pragnosia_b200.{n}" in code for n in ops_seen)
+    other = [(a.detach() * 0.5).requires_grad_() for a in args]
+    want = torch.autograd.grad((f(*other)[0].float() * w).sum(), other)
+    for a, b in zip(gm(*other), want):                                # the composition against the fused form: bf16 states between the operators
+        assert rel(a.detach(), b) < 1e-2
