@@ -5,6 +5,8 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/extension.h>
 
 #include "../../include/pragnosia_b200.h"
@@ -187,6 +189,18 @@ PrepGrads prep_bwd(const Tensor &qp, const Tensor &kp, const Tensor &vp_, const 
     return {dqp, dkp, dvp, some(dgl), want_theta ? OptTensor(part.sum(0)) : OptTensor()};
 }
 
+// The backward kernels have no derivative of their own: with create_graph a second differentiation through `grads` raises instead of
+// leaving its share out.
+variable_list once(const char *what, const variable_list &saved, variable_list grads, const variable_list &incoming) {
+    auto wants = [](const variable_list &l) { return std::any_of(l.begin(), l.end(), wants_grad); };
+    if (!at::GradMode::is_enabled() || !(wants(saved) || wants(incoming))) return grads;
+    const auto node = std::make_shared<torch::autograd::Error>(std::string("Trying to backward through the gradient of ") + what + ": it has no derivative",
+                                                               torch::autograd::collect_next_edges(saved, incoming));
+    for (Tensor &g : grads)
+        if (g.defined()) torch::autograd::set_history(g, node);
+    return grads;
+}
+
 // prep with its backward kernel
 struct Prep : torch::autograd::Function<Prep> {
     static variable_list forward(AutogradContext *ctx, const Tensor &qp, const Tensor &kp, const Tensor &vp_, const OptTensor &gl, const Tensor &theta,
@@ -199,8 +213,8 @@ struct Prep : torch::autograd::Function<Prep> {
     static variable_list backward(AutogradContext *ctx, variable_list g) {
         const variable_list s = ctx->get_saved_variables();
         auto [dq, dk, dv, dgl, dth] = prep_bwd(s[0], s[1], s[2], some(s[3]), s[4], s[5], g[0], g[1], g[2], ctx->saved_data["theta"].toBool());
-        return {as(dq, s[0].scalar_type()), as(dk, s[1].scalar_type()), as(dv, s[2].scalar_type()),
-                dgl ? as(*dgl, s[3].scalar_type()) : Tensor(), dth ? as(*dth, s[4].scalar_type()) : Tensor(), Tensor()};
+        return once("pragnosia_b200 prep", s, {as(dq, s[0].scalar_type()), as(dk, s[1].scalar_type()), as(dv, s[2].scalar_type()),
+                    dgl ? as(*dgl, s[3].scalar_type()) : Tensor(), dth ? as(*dth, s[4].scalar_type()) : Tensor(), Tensor()}, g);
     }
 };
 std::tuple<Tensor, Tensor, Tensor> prep_diff(const Tensor &qp, const Tensor &kp, const Tensor &vp_, const OptTensor &gl, const Tensor &theta, const Tensor &pos) {
@@ -345,8 +359,8 @@ struct Scan : torch::autograd::Function<Scan> {
         auto &d = ctx->saved_data;
         auto type = [&](const char *n) { return static_cast<at::ScalarType>(d[n].toInt()); };
         TrainGrads r = train_bwd(s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], g[0].defined() ? g[0] : at::zeros_like(s[0]), g[2], g[1], d["dS0"].toBool());
-        return {r.dq, r.dk, r.dv, as(r.dla, type("la")), r.dbe.defined() ? as(r.dbe, type("beta")) : Tensor(),
-                r.dS0.defined() ? as(r.dS0, type("S0")) : Tensor()};
+        return once("pragnosia_b200 scan", s, {r.dq, r.dk, r.dv, as(r.dla, type("la")), r.dbe.defined() ? as(r.dbe, type("beta")) : Tensor(),
+                    r.dS0.defined() ? as(r.dS0, type("S0")) : Tensor()}, g);
     }
 };
 std::tuple<Tensor, Tensor, Tensor> scan_diff(const Tensor &q, const Tensor &k, const Tensor &v, const Tensor &la, const OptTensor &beta, const OptTensor &S0) {

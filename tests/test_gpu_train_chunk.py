@@ -71,3 +71,18 @@ def test_a_tracer_sees_operators(what):
     want = torch.autograd.grad((f(*other)[0].float() * w).sum(), other)
     for a, b in zip(gm(*other), want):                                # the composition against the fused form: bf16 states between the operators
         assert rel(a.detach(), b) < 1e-2
+
+
+@pytest.mark.parametrize("what", ["plain", "delta", "prep"])
+@torch.enable_grad()
+def test_a_second_differentiation_raises(what):
+    """A gradient penalty over these operators is an error, not a loss without its gradient; a first derivative under create_graph is
+    what it is without."""
+    f, args, _ = _training_calls()[what]
+    w = torch.randn(2, 3, 100, 64, device="cuda")
+    want = torch.autograd.grad((f(*args)[0].float() * w).sum(), args)
+    got = torch.autograd.grad((f(*args)[0].float() * w).sum(), args, create_graph=True)
+    assert all(torch.equal(a.detach(), b) for a, b in zip(got, want))
+    for g in got:
+        with pytest.raises(RuntimeError, match="Trying to backward through"):
+            torch.autograd.grad(g.float().square().sum() + f(*args)[0].float().sum(), args, retain_graph=True)
