@@ -193,6 +193,13 @@ int pgb_aspin_prefill_segments_fwd(const void *q, const void *k, const void *v, 
                                    const float *shift_dev, float shift_host, void *o, int o_dtype, float *S_out, void *sent, void *scratch,
                                    long long scratch_bytes, int B, int H, int T, int D, void *stream);
 
+/* The plain rule's forward for a caller that will differentiate through it (pgb_aspin_train_bwd): bf16 operands and output, zero shift,
+ * `sent` stored, the final state with fp32's own error (the scaled keys enter its update in three bf16 terms; the inference entries
+ * take two). scratch: pgb_aspin_prefill_segments_scratch_bytes bytes, or NULL: the chains are then walked whole. S_out must not be
+ * S0. Replaces src/assoc_kernel.py:302-323 (prefix_scan, then assoc_out). */
+int pgb_aspin_prefill_train_fwd(const void *q, const void *k, const void *v, const float *la, const float *S0, void *o, float *S_out, void *sent,
+                                void *scratch, long long scratch_bytes, int B, int H, int T, int D, void *stream);
+
 /* The plain rule in full fp32 with scratch (pgb_aspin_prefill_fp32_scratch_bytes bytes): pgb_aspin_prefill_fwd's fp32 arithmetic
  * with the chunks of a sequence side by side instead of one behind the other. Limit B*H <= 65535. */
 long long pgb_aspin_prefill_fp32_scratch_bytes(int B, int H, int T, int D);

@@ -31,6 +31,7 @@ SIGNATURES = {
     "pgb_aspin_prefill_fwd": [_vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "pgb_aspin_prefill_segments_scratch_bytes": [_i, _i, _i, _i],
     "pgb_aspin_prefill_segments_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _vp],
+    "pgb_aspin_prefill_train_fwd": [_vp] * 9 + [_ll, _i, _i, _i, _i, _vp],
     "pgb_aspin_prefill_fp32_scratch_bytes": [_i, _i, _i, _i],
     "pgb_aspin_prefill_fp32_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _vp],
     "pgb_aspin_delta_prefill_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _vp],

@@ -361,6 +361,26 @@ int pgb_aspin_prefill_segments_fwd(const void *q, const void *k, const void *v, 
     return rc != PGB_OK ? rc : prefill_tc_ws_launch(a, o_dtype, (cudaStream_t)stream);
 }
 
+int pgb_aspin_prefill_train_fwd(const void *q, const void *k, const void *v, const float *la, const float *S0, void *o, float *S_out, void *sent,
+                                void *scratch, long long scratch_bytes, int B, int H, int T, int D, void *stream) {
+    if (!q || !k || !v || !la || !o || !S_out || !sent) return PGB_ERR_NULL_POINTER;
+    if (B <= 0 || H <= 0 || T <= 0 || (long long)B * H > 0x7fffffffLL) return PGB_ERR_BAD_SHAPE;
+    if (D != 64 && D != 128) return PGB_ERR_UNSUPPORTED_DIM;
+    if (S0 == S_out) return PGB_ERR_BAD_SHAPE;
+    if (!aligned(q, 16) || !aligned(k, 16) || !aligned(v, 16) || !aligned(o, 16) || !aligned(S_out, 16) || (S0 && !aligned(S0, 16)) ||
+        !aligned(sent, 16) || !aligned(scratch, 16))
+        return PGB_ERR_MISALIGNED;
+    PrefillArgs a{q, k, v, la, nullptr, S0, o, S_out, (__nv_bfloat16 *)sent, nullptr, nullptr, 0.f, B, H, T};
+    a.fine = 1;
+    const long long need = pgb_aspin_prefill_segments_scratch_bytes(B, H, T, D);
+    if (need == 0 || scratch == nullptr) return tc_dispatch(a, PGB_BF16, D, (cudaStream_t)stream);
+    if (scratch_bytes < need) return PGB_ERR_BAD_SHAPE;
+    a.seg_len = segment_len_prepared((long long)B * H, T);
+    a.seg_states = (const float *)scratch;
+    const int rc = segment_states_launch(a, (float *)scratch, (cudaStream_t)stream);
+    return rc != PGB_OK ? rc : prefill_tc_ws_launch(a, PGB_BF16, (cudaStream_t)stream);
+}
+
 long long pgb_aspin_prefill_fp32_scratch_bytes(int B, int H, int T, int D) {
     if (B <= 0 || H <= 0 || T <= 0 || (D != 64 && D != 128)) return 0;
     return (long long)prefill_fp32_chunk_scratch_bytes(B, H, T, D);

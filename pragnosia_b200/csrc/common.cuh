@@ -86,6 +86,9 @@ struct PrefillArgs {
     int raw = 0; long long raw_sb = 0, raw_st = 0; const void *gate_raw = nullptr; const float *rot = nullptr; int rot_T = 0;
     // > 0: chains cut into segments (head dim 64; see TcParams), entered with seg_states from the second on
     int seg_len = 0; const float *seg_states = nullptr; int seg_rotates = 0;
+    // plain rule on prepared operands: the scaled keys K w enter the state update in three bf16 terms instead of two, which is fp32's
+    // own error on the final state (training, whose operators formed it in fp32: 2.1e-6 with two terms, 3.9e-7 in fp32)
+    int fine = 0;
     int rebase_chunks = 0;                                            // delta rule: rebase the state every so many chunks (by that many tokens)
 };
 // the backward of the scan as one call (train_chunk.cu); beta, W and X only under the delta rule

@@ -57,7 +57,9 @@ struct TcSmem {
 
 constexpr int TC_NT = 256;
 
-template <int D, bool RAW>
+// FINE (prepared operands): a third term of K w, in the scores' place; its product goes ahead of P, so that it is through when the
+// scores are formed
+template <int D, bool RAW, bool FINE>
 __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                                                            const __grid_constant__ CUtensorMap mv, TcParams p) {
     using SM = TcSmem<D>;
@@ -310,7 +312,11 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
 #pragma unroll
                     for (int i = 0; i < 4; ++i) { float2 f = __bfloat1622float2(b2[i]); x[2 * i] = f.x * w; x[2 * i + 1] = f.y * w; }
                     uint4 hi, lo;
-                    split8(x, hi, lo);
+                    if constexpr (FINE) {
+                        uint4 rest;
+                        split8(x, hi, lo, rest);
+                        *reinterpret_cast<uint4 *>(sm + SM::off_ah + off) = rest;
+                    } else split8(x, hi, lo);
                     *reinterpret_cast<uint4 *>(sm + SM::off_kwh + off) = hi;
                     *reinterpret_cast<uint4 *>(sm + SM::off_kwl + off) = lo;
                 }
@@ -327,6 +333,11 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
             const uint64_t dq = smem_desc(qs, 16, 1024), dk = smem_desc(ks, 16, 1024), dv = smem_desc(vs, 8192, 1024);
             const uint64_t dkwh = smem_desc(base + SM::off_kwh, 8192, 1024), dkwl = smem_desc(base + SM::off_kwl, 8192, 1024);
             const uint64_t dsh = smem_desc(base + SM::off_sh, D * 128, 1024), dsl = smem_desc(base + SM::off_sl, D * 128, 1024);
+            if constexpr (FINE) {
+                const uint64_t dkwr = smem_desc(base + SM::off_ah, 8192, 1024);
+#pragma unroll
+                for (int k = 0; k < TC_C / 16; ++k) mma_bf16_elect(tmem + TM_U, dkwr + k * 128, dv + k * 128, I_U, k > 0);
+            }
 #pragma unroll
             for (int k = 0; k < D / 16; ++k) {                        // P = Q K^T, K-major steps of 32 B inside a sub-tile
                 const uint32_t ko = ((uint32_t)(k >> 2) * 8192u + (uint32_t)(k & 3) * 32u) >> 4;
@@ -335,7 +346,7 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
             mma_commit_elect(bar_p);
 #pragma unroll
             for (int k = 0; k < TC_C / 16; ++k)                       // U = (K w)^T V over the 64 tokens, 16 rows (2048 B) a step
-                mma_bf16_elect(tmem + TM_U, dkwh + k * 128, dv + k * 128, I_U, k > 0);
+                mma_bf16_elect(tmem + TM_U, dkwh + k * 128, dv + k * 128, I_U, FINE || k > 0);
 #pragma unroll
             for (int k = 0; k < TC_C / 16; ++k) mma_bf16_elect(tmem + TM_U, dkwl + k * 128, dv + k * 128, I_U, 1);
             mma_commit_elect(bar_a);
@@ -497,7 +508,7 @@ __global__ void __launch_bounds__(TC_NT) prefill_tc_kernel(const __grid_constant
 // ---------------------------------------------------------------------------------------------- host side
 namespace {
 
-template <int D, bool RAW>
+template <int D, bool RAW, bool FINE = false>
 int tc_go(const PrefillArgs &a, int o_dtype, cudaStream_t stream) {
     using SM = TcSmem<D>;
     CUtensorMap mq, mk, mv;
@@ -514,7 +525,7 @@ int tc_go(const PrefillArgs &a, int o_dtype, cudaStream_t stream) {
         set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled");
         return PGB_ERR_CUDA;
     }
-    auto kern = prefill_tc_kernel<D, RAW>;
+    auto kern = prefill_tc_kernel<D, RAW, FINE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::bytes);
     if (e != cudaSuccess) { set_cuda_error(e, "prefill_tc smem attribute"); return PGB_ERR_CUDA; }
     TcParams p{a.la, a.S0, a.theta, a.shift_dev, a.shift_host, a.o, a.S_out, a.sent, a.H, a.T, o_dtype == PGB_F32,
@@ -531,6 +542,7 @@ bool prefill_tc_supported(int io_dtype, int D, bool delta) { return io_dtype == 
 
 int prefill_tc_launch(const PrefillArgs &a, int o_dtype, int D, cudaStream_t stream) {
     if (a.raw) return D == 64 ? tc_go<64, true>(a, o_dtype, stream) : tc_go<128, true>(a, o_dtype, stream);
+    if (a.fine) return D == 64 ? tc_go<64, false, true>(a, o_dtype, stream) : tc_go<128, false, true>(a, o_dtype, stream);
     return D == 64 ? tc_go<64, false>(a, o_dtype, stream) : tc_go<128, false>(a, o_dtype, stream);
 }
 

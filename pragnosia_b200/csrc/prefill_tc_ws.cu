@@ -48,7 +48,8 @@ struct WsSmem {
 };
 
 
-template <bool RAW>
+// FINE (prepared operands): a third term of K w, in the rotation rows' place
+template <bool RAW, bool FINE>
 __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                                                                 const __grid_constant__ CUtensorMap mv, TcParams p) {
     using SM = WsSmem;
@@ -196,7 +197,11 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
 #pragma unroll
                     for (int i = 0; i < 4; ++i) { float2 f = __bfloat1622float2(b2[i]); x[2 * i] = f.x * w; x[2 * i + 1] = f.y * w; }
                     uint4 hi, lo;
-                    split8(x, hi, lo);
+                    if constexpr (FINE) {
+                        uint4 rest;
+                        split8(x, hi, lo, rest);
+                        *reinterpret_cast<uint4 *>(sm + SM::off_rot + s2 * SM::TILE + off) = rest;
+                    } else split8(x, hi, lo);
                     *reinterpret_cast<uint4 *>(kwh + off) = hi;
                     *reinterpret_cast<uint4 *>(kwl + off) = lo;
                 }
@@ -481,6 +486,11 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
             for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem + TM_U + 64 * s2, dkwh + k * 128, dv + k * 128, I_U, k > 0);
 #pragma unroll
             for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem + TM_U + 64 * s2, dkwl + k * 128, dv + k * 128, I_U, 1);
+            if constexpr (FINE) {
+                const uint64_t dkwr = smem_desc(base + SM::off_rot + s2 * SM::TILE, 8192, 1024);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem + TM_U + 64 * s2, dkwr + k * 128, dv + k * 128, I_U, 1);
+            }
             mma_commit_elect(bar_pu(s2));
             mma_commit_elect(bar_empty(c % 3));                       // this issuer's half: P and U have read the chunk's tiles
             if (lane == 0) mbar_arrive(bar_q(c & 3));                 // the other issuer may use the chunk's Q and V tiles
@@ -543,16 +553,11 @@ int prefill_tc_ws_launch(const PrefillArgs &a, int o_dtype, cudaStream_t stream)
     TcParams p{a.la, a.S0, a.theta, a.shift_dev, a.shift_host, a.o, a.S_out, a.sent, a.H, a.T, o_dtype == PGB_F32,
                (const __nv_bfloat16 *)a.la_raw, a.la_sb, a.la_st, a.decay_A, a.rms_w, a.rms_eps, a.o_token_major,
                (const __nv_bfloat16 *)a.gate_raw, (const float2 *)a.rot, a.rot_T, BH, seg_len, a.seg_states, a.seg_rotates};
-    cudaError_t e;
-    if (a.raw) {
-        e = cudaFuncSetAttribute(prefill_tc_ws_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, WsSmem::bytes);
-        if (e != cudaSuccess) { set_cuda_error(e, "prefill_tc_ws smem attribute"); return PGB_ERR_CUDA; }
-        e = pdl_launch(prefill_tc_ws_kernel<true>, dim3((unsigned)(BH * nseg)), dim3(WS_NT), (size_t)WsSmem::bytes, stream, mq, mk, mv, p);
-    } else {
-        e = cudaFuncSetAttribute(prefill_tc_ws_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, WsSmem::bytes);
-        if (e != cudaSuccess) { set_cuda_error(e, "prefill_tc_ws smem attribute"); return PGB_ERR_CUDA; }
-        e = pdl_launch(prefill_tc_ws_kernel<false>, dim3((unsigned)(BH * nseg)), dim3(WS_NT), (size_t)WsSmem::bytes, stream, mq, mk, mv, p);
-    }
+    auto go = [&](auto kern) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WsSmem::bytes);
+        return e != cudaSuccess ? e : pdl_launch(kern, dim3((unsigned)(BH * nseg)), dim3(WS_NT), (size_t)WsSmem::bytes, stream, mq, mk, mv, p);
+    };
+    const cudaError_t e = a.raw ? go(prefill_tc_ws_kernel<true, false>) : a.fine ? go(prefill_tc_ws_kernel<false, true>) : go(prefill_tc_ws_kernel<false, false>);
     if (e != cudaSuccess) { set_cuda_error(e, "prefill_tc_ws launch"); return PGB_ERR_CUDA; }
     return check_launch("prefill_tc_ws_kernel");
 }

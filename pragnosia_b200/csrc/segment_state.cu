@@ -22,8 +22,8 @@ namespace pgb {
 constexpr int SG_NT = 256, SG_D = 64, SG_ST = 3;                      // threads; head dim; stages
 constexpr int SG_MAX = 1024, SG_MAX_PREPARED = 4096;                  // tokens of a segment at most
 
-template <bool RAW> struct SgSmem {
-    static constexpr int TILE = 8192, STAGE = 3 * TILE;               // K (then heads of K w), V, tails of K w
+template <bool RAW, bool FINE> struct SgSmem {
+    static constexpr int TILE = 8192, STAGE = (FINE ? 4 : 3) * TILE;  // K (then heads of K w), V, tails of K w, their rest
     static constexpr int MAX = RAW ? SG_MAX : SG_MAX_PREPARED;
     static constexpr int off_w = SG_ST * STAGE, off_g = off_w + MAX * 4, off_misc = off_g + (RAW ? MAX * 4 : 0), bytes = off_misc + 256 + 1024;
 };
@@ -35,10 +35,10 @@ struct SgParams {
     int BH, H, seg_len;
 };
 
-template <bool RAW>
-__global__ void __launch_bounds__(SG_NT, 2) segment_state_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv,
+template <bool RAW, bool FINE>
+__global__ void __launch_bounds__(SG_NT, FINE ? 1 : 2) segment_state_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv,
                                                                  SgParams p) {
-    using SM = SgSmem<RAW>;
+    using SM = SgSmem<RAW, FINE>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *sm = smem_raw + (base - smem_u32(smem_raw));
@@ -126,7 +126,11 @@ __global__ void __launch_bounds__(SG_NT, 2) segment_state_kernel(const __grid_co
 #pragma unroll
                 for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(b2[i]); kw[2 * i] = f.x * w; kw[2 * i + 1] = f.y * w; }
                 uint4 hi, lo;
-                split8(kw, hi, lo);
+                if constexpr (FINE) {
+                    uint4 rest;
+                    split8(kw, hi, lo, rest);
+                    *reinterpret_cast<uint4 *>(lt + SM::TILE + off) = rest;
+                } else split8(kw, hi, lo);
                 *reinterpret_cast<uint4 *>(kt + off) = hi;
                 *reinterpret_cast<uint4 *>(lt + off) = lo;
             }
@@ -186,6 +190,9 @@ __global__ void __launch_bounds__(SG_NT, 2) segment_state_kernel(const __grid_co
             for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem, dh + k * 128, dv + k * 128, I_U, (c > 0) | (k > 0));
 #pragma unroll
             for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem, dl + k * 128, dv + k * 128, I_U, 1);
+            if constexpr (FINE)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mma_bf16_elect(tmem, dl + (SM::TILE >> 4) + k * 128, dv + k * 128, I_U, 1);
             mma_commit_elect(done(st));
             if (c + 1 == NC) mma_commit_elect(bar_end);
             if (c + 2 < NC) {                                         // into the stage of chunk c - 1, whose product is an iteration old
@@ -291,7 +298,9 @@ int segment_states_launch(const PrefillArgs &a, float *scratch, cudaStream_t str
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         return e != cudaSuccess ? e : pdl_launch(kern, dim3((unsigned)(BH * (nseg - 1))), dim3(SG_NT), (size_t)smem, stream, mk, mv, p);
     };
-    cudaError_t e = a.raw ? go(segment_state_kernel<true>, SgSmem<true>::bytes) : go(segment_state_kernel<false>, SgSmem<false>::bytes);
+    cudaError_t e = a.raw    ? go(segment_state_kernel<true, false>, SgSmem<true, false>::bytes)
+                    : a.fine ? go(segment_state_kernel<false, true>, SgSmem<false, true>::bytes)
+                             : go(segment_state_kernel<false, false>, SgSmem<false, false>::bytes);
     if (e == cudaSuccess)
         e = pdl_launch(segment_combine_kernel, dim3(SG_D * SG_D / 4 / 256, (unsigned)BH), dim3(256), (size_t)0, stream, scratch, (const float *)Lend, a.S0,
                        a.theta, a.shift_dev, nseg - 1, BH, a.H, a.shift_host, (bool)a.seg_rotates);

@@ -8,7 +8,6 @@
 namespace pgb {
 
 constexpr int TC_C = 64;
-constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;                        // polls of a sleeping poll loop
 
 // Set (to the code of the wait) when a bounded mbarrier wait inside a tensor-core kernel runs out. One copy per
 // translation unit (no relocatable device code in this build); each unit exports a reader, the C ABI takes the maximum.
@@ -303,6 +302,19 @@ __device__ __forceinline__ void split8(const float (&x)[8], uint4 &hi, uint4 &lo
     }
     hi = *reinterpret_cast<uint4 *>(h);
     lo = *reinterpret_cast<uint4 *>(l);
+}
+
+// the same with what both leave over as a third: 24 bits of x in all
+__device__ __forceinline__ void split8(const float (&x)[8], uint4 &hi, uint4 &lo, uint4 &rest) {
+    split8(x, hi, lo);
+    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&hi), *l = reinterpret_cast<const __nv_bfloat162 *>(&lo);
+    __nv_bfloat162 r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 a = __bfloat1622float2(h[i]), b = __bfloat1622float2(l[i]);
+        r[i] = __floats2bfloat162_rn(x[2 * i] - a.x - b.x, x[2 * i + 1] - a.y - b.y);
+    }
+    rest = *reinterpret_cast<uint4 *>(r);
 }
 
 // two fp32 -> packed bf16 heads and packed bf16 tails

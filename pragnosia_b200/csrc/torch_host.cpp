@@ -306,13 +306,18 @@ ScanOut prefill(const Tensor &q_, const Tensor &k_, const Tensor &v_, const Tens
 // The scan with what its backward reads: (o, S, sent, W, X); bf16 q, k, v, fp32 la, beta, all contiguous; W and X with the delta rule.
 struct TrainOut { Tensor o, S, sent, W, X; };
 TrainOut train_fwd(const Tensor &q, const Tensor &k, const Tensor &v, const Tensor &la, const Tensor &beta, const Tensor &S0) {
-    if (!beta.defined()) {
-        auto [o, S, sent] = prefill(q, k, v, la, {}, some(S0), {}, {}, 0.0, true, PGB_PREFILL_TENSOR, -1, {});
-        return {o, S, *sent, Tensor(), Tensor()};
-    }
     need_cuda(q, k, v, la, beta, S0);
     const int64_t B = q.size(0), H = q.size(1), T = q.size(2), D = q.size(3);
     OnDevice dev(q);
+    if (!beta.defined()) {
+        const long long n = pgb_aspin_prefill_segments_scratch_bytes(B, H, T, D);
+        TrainOut r{alloc(q, {B, H, T, D}, at::kBFloat16), alloc(q, {B, H, D, D}, at::kFloat), alloc(q, {B, H, (T + CHUNK - 1) / CHUNK, D, D}, at::kBFloat16),
+                   Tensor(), Tensor()};
+        const Tensor scratch = n > 0 ? bytes(q, n) : Tensor();
+        check(pgb_aspin_prefill_train_fwd(vp(q), vp(k), vp(v), fp(la), fp(S0), vp(r.o), fp(r.S), vp(r.sent), vp(scratch), n, B, H, T, D, dev.stream),
+              "pgb_aspin_prefill_train_fwd");
+        return r;
+    }
     const long long n = pgb_aspin_delta_scratch_bytes(B, H, T);
     TrainOut r{alloc(q, {B, H, T, D}, at::kBFloat16), alloc(q, {B, H, D, D}, at::kFloat), alloc(q, {B, H, (T + CHUNK - 1) / CHUNK, D, D}, at::kBFloat16),
                alloc(q, {B, H, T, D}, at::kBFloat16), bytes(q, n)};

@@ -86,3 +86,23 @@ def test_a_second_differentiation_raises(what):
     for g in got:
         with pytest.raises(RuntimeError, match="Trying to backward through"):
             torch.autograd.grad(g.float().square().sum() + f(*args)[0].float().sum(), args, retain_graph=True)
+
+
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("B,H,T,D", [(1, 1, 1, 64), (2, 3, 130, 64), (1, 2, 2048, 64), (1, 4, 1025, 64), (2, 3, 200, 128), (1, 2, 1024, 128)])
+def test_the_final_state_of_training_is_fp32s(B, H, T, D, variant):
+    """The plain rule's state against fp64 on the same bf16 operands: fp32 sums (64-token products, then the chunks) stay below 8e-7,
+    scaled keys in two bf16 terms alone are 2e-6 off."""
+    from pragnosia_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    q, k, v = (torch.nn.functional.normalize(rn(B, H, T, D), dim=-1).bfloat16() for _ in range(3))
+    la, S0 = torch.nn.functional.logsigmoid(2.0 + rn(B, H, T)), 0.1 * rn(B, H, D, D)
+    L = la.double().cumsum(-1)
+    want = (k.double() * (L[..., -1:] - L).exp()[..., None]).transpose(-1, -2) @ v.double() + L[..., -1].exp()[..., None, None] * S0.double()
+    try:
+        assert _lib.lib().pgb_tc_set_variant(variant) == 0
+        S = ops.scan_train_fwd(q, k, v, la, None, S0)[1]
+    finally:
+        _lib.lib().pgb_tc_set_variant(0)
+    assert rel(S, want) < 8e-7
