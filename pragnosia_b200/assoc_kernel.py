@@ -14,15 +14,6 @@ from . import ops
 from ._lib import host
 
 
-def _eager(*ts) -> bool:
-    """Plain tensors and nothing between a call and its kernels: no compiler, tracer, torch_dispatch mode (fake tensors, make_fx,
-    selective checkpointing) or functorch transform (vmap). Those see the registered operators; the C++ autograd nodes
-    (csrc/torch_host.cpp) go straight to the library."""
-    return (not torch.compiler.is_compiling() and torch._C._len_torch_dispatch_stack() == 0 and torch._C._get_tracing_state() is None
-            and torch._C._functorch.peek_interpreter_stack() is None
-            and all(t is None or type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in ts))
-
-
 def _wants_grad(*ts) -> bool:
     return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in ts)
 
@@ -31,8 +22,10 @@ def prep_kernel(qp, kp, vp, gate_logits, theta, pos):
     """qp, kp, vp: the projections as (B,T,H,D) views; gate_logits (B,T,H) or None; theta (H,D/2); pos (T,) integer
     positions. Returns bf16 q, k, v as (B,H,T,D). Differentiable (the backward kernel of src/assoc_kernel.py:774-826)."""
     if _wants_grad(qp, kp, vp, gate_logits, theta):
-        if _eager(qp, kp, vp, gate_logits, theta, pos):
-            return host().prep_diff(qp, kp, vp, gate_logits, theta, pos)
+        if not torch.compiler.is_compiling():
+            out = host().prep_diff(qp, kp, vp, gate_logits, theta, pos)
+            if out is not None:                                       # None: something wants to see the operators
+                return out
         from . import custom_ops  # noqa: F401
         return tuple(torch.ops.pragnosia_b200.assoc_prep(qp, kp, vp, gate_logits, theta, pos))
     return ops.prep(qp, kp, vp, gate_logits, theta, pos)
@@ -53,8 +46,10 @@ def assoc_scan_kernel(q, k, v, logalpha, S0=None, bv: int = 16):
     compiled, the composition of the differentiable operators, as the reference composes it (prefix_scan, then assoc_out:
     src/assoc_kernel.py:302-323). Without: the one fused walk."""
     if _wants_grad(q, k, v, logalpha, S0):
-        if _eager(q, k, v, logalpha, S0) and ops.scan_trains(q, k, v):
-            return host().scan_diff(q, k, v, logalpha, None, S0)
+        if not torch.compiler.is_compiling() and ops.scan_trains(q, k, v):
+            out = host().scan_diff(q, k, v, logalpha, None, S0)
+            if out is not None:
+                return out
         T = q.shape[2]
         pad = (-T) % ops.CHUNK
         a_log, w = _chunk_decay(logalpha, T)
@@ -70,8 +65,10 @@ def delta_scan_kernel(q, k, v, logalpha, beta, S0=None, chunk: int = 64, bv: int
     With a gradient wanted: as assoc_scan_kernel; the composition here is delta_inv, delta_loop_fwd, then assoc_out on the
     residuals (src/assoc_kernel.py:512-546)."""
     if _wants_grad(q, k, v, logalpha, beta, S0):
-        if _eager(q, k, v, logalpha, beta, S0) and ops.scan_trains(q, k, v):
-            return host().scan_diff(q, k, v, logalpha, beta, S0)
+        if not torch.compiler.is_compiling() and ops.scan_trains(q, k, v):
+            out = host().scan_diff(q, k, v, logalpha, beta, S0)
+            if out is not None:
+                return out
         NC = (q.shape[2] + ops.CHUNK - 1) // ops.CHUNK
         X = ops.delta_inv(k, logalpha, beta, NC)
         W, sent, S = ops.delta_loop_fwd(k, v, logalpha, beta, X, S0)

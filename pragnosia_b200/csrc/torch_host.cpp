@@ -2,7 +2,10 @@
 // library call and the autograd nodes, in C++. A call of a few microseconds on the GPU spent 15 us in Python, a training pass of
 // the scan (B16 T512 D704: 104 us of kernels) 160, most of it in the autograd functions' Python frames. The C ABI stays what the
 // kernels are reached by; this file only prepares its arguments, and ops.py / scan_kernel.py / assoc_kernel.py call it.
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
@@ -217,9 +220,20 @@ struct Prep : torch::autograd::Function<Prep> {
                     dgl ? as(*dgl, s[3].scalar_type()) : Tensor(), dth ? as(*dth, s[4].scalar_type()) : Tensor(), Tensor()}, g);
     }
 };
-std::tuple<Tensor, Tensor, Tensor> prep_diff(const Tensor &qp, const Tensor &kp, const Tensor &vp_, const OptTensor &gl, const Tensor &theta, const Tensor &pos) {
+using Three = std::optional<std::tuple<Tensor, Tensor, Tensor>>;
+// nullopt: a tracer, a torch_dispatch mode (fake tensors, make_fx, selective checkpointing), a functorch transform or a tensor subclass
+// wants to see the registered operators
+template <typename... P> bool plain(const P &...ts) {
+    using c10::DispatchKey;
+    const c10::DispatchKeySet special{DispatchKey::Python, DispatchKey::FuncTorchBatched, DispatchKey::FuncTorchGradWrapper};
+    return !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::tracer::impl::is_dispatch_enabled() &&
+           !c10::impl::tls_is_dispatch_key_included(DispatchKey::FuncTorchDynamicLayerFrontMode) &&
+           (... && (!ts.defined() || !ts.key_set().has_any(special)));
+}
+Three prep_diff(const Tensor &qp, const Tensor &kp, const Tensor &vp_, const OptTensor &gl, const Tensor &theta, const Tensor &pos) {
+    if (!plain(qp, kp, vp_, opt(gl), theta, pos)) return std::nullopt;
     variable_list r = Prep::apply(qp, kp, vp_, gl, theta, pos);
-    return {r[0], r[1], r[2]};
+    return std::make_tuple(r[0], r[1], r[2]);
 }
 
 // ------------------------------------------------------------------------------------------------ associative scan
@@ -368,9 +382,10 @@ struct Scan : torch::autograd::Function<Scan> {
                     r.dS0.defined() ? as(r.dS0, type("S0")) : Tensor()}, g);
     }
 };
-std::tuple<Tensor, Tensor, Tensor> scan_diff(const Tensor &q, const Tensor &k, const Tensor &v, const Tensor &la, const OptTensor &beta, const OptTensor &S0) {
+Three scan_diff(const Tensor &q, const Tensor &k, const Tensor &v, const Tensor &la, const OptTensor &beta, const OptTensor &S0) {
+    if (!plain(q, k, v, la, opt(beta), opt(S0))) return std::nullopt;
     variable_list r = Scan::apply(q, k, v, la, beta, S0);
-    return {r[0], r[1], r[2]};
+    return std::make_tuple(r[0], r[1], r[2]);
 }
 }  // namespace
 
