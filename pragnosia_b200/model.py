@@ -247,6 +247,9 @@ class LM(nn.Module):
         return (logits, states) if return_states else logits
 
 
+_NO_ROOM = "no room"                    # in place of a captured pass whose memory could not be had: eagerly from then on
+
+
 class _Captured:
     """A model's captured passes. They write static tensors of their own and share one memory pool, so they run one at a time:
     turn() holds the host lock, makes the current stream wait for the turn before (whichever thread and stream it came from) and
@@ -286,21 +289,29 @@ class _Captured:
                 self.done.record(here)
 
     def shape_graph(self, model, ids, body, window, tail):
-        """The captured pass of this shape; None the first time it comes."""
+        """The captured pass of this shape; None the first time it comes, and where there is no room for it."""
         key = (tuple(ids.shape), ids.dtype, window, tail, ids.device)
         run = self.shapes.pop(key, None)
+        if run is _NO_ROOM:
+            self.shapes[key] = run
+            return None
         if run is None:
             self.shapes[key] = False
             if len(self.shapes) > 64:
                 self.shapes.pop(next(iter(self.shapes)))
             return None
         if run is False:
-            held = [k for k, v in self.shapes.items() if v is not False]
+            held = [k for k, v in self.shapes.items() if isinstance(v, _ShapeGraph)]
             if len(held) >= 8:                                        # eight captured shapes at most, the longest unused one goes
                 self.shapes.pop(held[0])
             if self.pool is None:
                 self.pool, self.stream = torch.cuda.graph_pool_handle(), torch.cuda.Stream()
-            run = _ShapeGraph(model, ids, body, window, tail, self.stream, self.pool)
+            try:
+                run = _ShapeGraph(model, ids, body, window, tail, self.stream, self.pool)
+            except torch.cuda.OutOfMemoryError:                       # no room for a second set of activations: give back what is held
+                self.shapes.clear()
+                self.shapes[key], self.pool = _NO_ROOM, None
+                return None
         self.shapes[key] = run                                        # last in the order: most recently used
         return run
 

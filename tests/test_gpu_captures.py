@@ -277,3 +277,28 @@ def test_the_form_of_a_pass_follows_the_devices_sm_count(sms, over_all, monkeypa
     got = m.forward_carried(a, 64)
     assert bool(m._captured.windows) != over_all
     assert float((got.float() - want.float()).norm() / want.float().norm()) < 2e-2
+
+
+@pytest.mark.parametrize("mixer", ["aspin", "dspin"])
+def test_no_room_for_a_captured_pass(mixer):
+    """Memory for an eager pass but not for a graph's own copy of its activations: the pass runs eagerly."""
+    m = lm(mixer, d=512, layers=2)
+    a = ids(4, 4000, 1)
+    want = m.forward_carried(a, 64).clone()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    m._captured.shapes.clear()
+    m.forward_carried(a, 64)                                          # eagerly: what it takes
+    torch.cuda.synchronize()
+    total, peak = torch.cuda.get_device_properties(0).total_memory, torch.cuda.max_memory_reserved()
+    torch.cuda.set_per_process_memory_fraction((peak + (4 << 20)) / total)
+    try:
+        out = [m.forward_carried(a, 64) for _ in range(3)]
+        assert list(m._captured.shapes.values()) == [M._NO_ROOM]
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert all(torch.equal(x, want) for x in out)
+    m._captured.shapes.clear()
+    out = [m.forward_carried(a, 64) for _ in range(3)]
+    assert all(m._captured.shapes.values()) and all(torch.equal(x, want) for x in out)
