@@ -14,7 +14,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
-from ._lib import Cached
+from ._lib import Cached, mark_constants
 
 
 def rotate(x, theta, pos):
@@ -117,12 +117,12 @@ class AssocCarrier(nn.Module):
         if torch.compiler.is_compiling():
             return self._build_consts()                 # traced into the caller's graph: nothing cached, nothing stale
         key, got = self.consts_key(), self._fused
-        if got is None or got.key != key:
+        c = got.get() if got is not None and got.key == key else None
+        if c is None:
             with torch.no_grad():
                 c = self._build_consts()
-            got = Cached(key, c, c.values())
-            self._fused = got.keep(self._fused)
-        return got.get()
+            self._fused = Cached(key, c, c.values()).keep(got)
+        return c
 
     def forward(self, x, h0=None, pos0: int = 0):
         """x (B,T,d) on CUDA; h0 = (S (B,H,dk,dk) fp32, p0[, conv cache]) from the previous window or step, or None.
@@ -180,6 +180,8 @@ class AssocCarrier(nn.Module):
                 o = self.on(o.to(z.dtype)).transpose(1, 2).reshape(B, T, D)
             self.sent = sent
         delta = F.linear(o, c["ow"])
+        if not torch.compiler.is_compiling():
+            mark_constants(z)
         if torch.is_tensor(p0):
             # a device-side position (graphed decode): with inplace_state the caller owns and updates it
             p_new = p0 if inplace else p0 * 0 + T
@@ -292,11 +294,13 @@ class AssocCarrier(nn.Module):
         if torch.compiler.is_compiling():
             return self._wrapped(ops.rot_table(c["theta"], need), need)
         got = self._rot
-        if got is None or got.key[0] != self.pos_wrap or got.key[1] is not c or got.value.shape[1] < need:
+        table = None
+        if got is not None and got.key[0] == self.pos_wrap and got.key[1] is c and got.value.shape[1] >= need:
+            table = got.get()
+        if table is None:
             table = self._wrapped(ops.rot_table(c["theta"], need), need)
-            got = Cached((self.pos_wrap, c), table, [table])
-            self._rot = got.keep(self._rot)
-        return got.get()
+            self._rot = Cached((self.pos_wrap, c), table, [table]).keep(got)
+        return table
 
     def _wrapped(self, table, need):
         if not self.pos_wrap:
@@ -308,11 +312,11 @@ class AssocCarrier(nn.Module):
             pos = torch.arange(T, device=device)
         else:
             got = self._pos
-            if got is None or got.value.numel() < T or got.value.device != device:
+            pos = got.get() if got is not None and got.value.numel() >= T and got.value.device == device else None
+            if pos is None:
                 pos = torch.arange(max(T, 512), device=device)
-                got = Cached(None, pos, [pos])
-                self._pos = got.keep(self._pos)
-            pos = got.get()[:T]
+                self._pos = Cached(None, pos, [pos]).keep(got)
+            pos = pos[:T]
         return pos % self.pos_wrap if self.pos_wrap else pos
 
     def _rms_eps(self):

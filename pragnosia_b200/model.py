@@ -11,7 +11,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
-from ._lib import Cached, graph_capture, lib, sm_count, warm_up
+from ._lib import Cached, graph_capture, lib, mark_constants, sm_count, warm_up
 from .assoc import AssocCarrier
 from .spin import SpinCarrier
 
@@ -133,12 +133,12 @@ class LM(nn.Module):
     def _window_positions(self, T, window, device):
         """(position inside its window of every token, the same modulo the position table) for the first T tokens."""
         got = self._wpos
-        if got is None or got.key != (window, device) or got.value[0].numel() < T:
+        both = got.get() if got is not None and got.key == (window, device) and got.value[0].numel() >= T else None
+        if both is None:
             pos = torch.arange(T, device=device) % window
             both = (pos, pos % self.p.num_embeddings)
-            got = Cached((window, device), both, both)
-            self._wpos = got.keep(self._wpos)
-        return tuple(t[:T] for t in got.get())
+            self._wpos = Cached((window, device), both, both).keep(got)
+        return tuple(t[:T] for t in both)
 
     def _piece(self, B, window):
         """Tokens of a sequence that go through the layers together: whole windows, WINDOWS_TOKENS tokens over the batch at most (or
@@ -199,6 +199,8 @@ class LM(nn.Module):
                     last, states = run(ids)
                     return self._add_norm(*last, self.n)[1], states
         last, states = body(ids, window, tail)
+        if ids.is_cuda:
+            mark_constants(ids)
         return self._add_norm(*last, self.n)[1], states
 
     def _may_replay(self, ids) -> bool:

@@ -302,3 +302,22 @@ def test_no_room_for_a_captured_pass(mixer):
     m._captured.shapes.clear()
     out = [m.forward_carried(a, 64) for _ in range(3)]
     assert all(m._captured.shapes.values()) and all(torch.equal(x, want) for x in out)
+
+
+def test_constants_nobody_has_marked_yet():
+    """Made by a call that has not come to its end (here: the constants alone); the other stream marks their stream itself."""
+    want = lm("aspin", d=256).mix[0]
+    x = torch.randn(2, 70, 256, device=DEV).to(torch.bfloat16)
+    want = want(x)[0]
+    layer = lm("aspin", d=256).mix[0]
+    torch.cuda.synchronize()
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(one):
+        torch.cuda._sleep(20_000_000)
+        layer._consts()
+        assert layer._fused.mark.due
+    with torch.cuda.stream(two):
+        got = layer(x)[0]
+    assert not layer._fused.mark.due
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
