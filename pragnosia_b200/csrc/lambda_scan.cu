@@ -47,13 +47,6 @@ __device__ __forceinline__ void ls_st(float *p, const f2 (&d)[LsVec<VEC>::NP]) {
     else if constexpr (VEC == 2) *reinterpret_cast<f2 *>(p) = d[0];
     else { float a, b; f2_unpack(d[0], a, b); *p = a; }
 }
-// e^x of a row of log-magnitudes, whatever they are
-template <int VEC>
-__device__ __forceinline__ void ls_exp_any(f2 (&d)[LsVec<VEC>::NP], const float *p) {
-    ls_ld<VEC>(d, p);
-#pragma unroll
-    for (int v = 0; v < LsVec<VEC>::NP; ++v) d[v] = f2_expf(d[v]);
-}
 // a complex pair product and sum: (ar + i ai)(br + i bi) + (cr + i ci)
 __device__ __forceinline__ void ls_cfma(f2 &outr, f2 &outi, f2 ar, f2 ai, f2 br, f2 bi, f2 cr, f2 ci) {
     const f2 nai = f2_neg(ai);
@@ -146,22 +139,14 @@ lambda_scan_kernel(const float *__restrict__ u, const float *__restrict__ lm, co
             if (t0 + TS * SEG < T) fetch(tb + TS * SEG, nc, ns, nx);
         } else fetch(tb, c, s, x);
         // lambda of every step; steps past the end keep log-magnitude and angle 0, the identity map
-        float top = 0.f;
-#pragma unroll
-        for (int i = 0; i < SEG; ++i)
-#pragma unroll
-            for (int v = 0; v < NP; ++v) { f2_exp_fold(top, c[i][v]); c[i][v] = f2_exp(c[i][v]); }
-        if (!(top <= F2_EXP_MAX)) {
-#pragma unroll
-            for (int i = 0; i < SEG; ++i)
-                if (live && tb + i < T) ls_exp_any<VEC>(c[i], lm + (row0 + tb + i) * D + d0);
-        }
 #pragma unroll
         for (int i = 0; i < SEG; ++i) {
             const bool ok = live && (tb + i) < T;
 #pragma unroll
             for (int v = 0; v < NP; ++v) {
-                const f2 mag = c[i][v];
+                float l0, l1;
+                f2_unpack(c[i][v], l0, l1);
+                const f2 mag = f2_exp(l0, l1);
                 f2 cs, sn;
                 if constexpr (ANG_BCAST) { cs = ok ? acs[v] : f2_both(1.f); sn = ok ? asn[v] : 0ull; }
                 else { float a0, a1; f2_unpack(s[i][v], a0, a1); f2_sincos(a0, a1, sn, cs); }
@@ -250,7 +235,8 @@ lambda_scan_bwd_kernel(const float *__restrict__ g, const float *__restrict__ u,
 #pragma unroll
         for (int v = 0; v < NP; ++v) {
             float x0, x1;
-            const f2 mag = f2_expf(l[v]);
+            f2_unpack(l[v], x0, x1);
+            const f2 mag = f2_exp(x0, x1);
             f2 cs, sn;
             f2_unpack(a[v], x0, x1);
             f2_sincos(x0, x1, sn, cs);
@@ -297,18 +283,6 @@ lambda_scan_bwd_kernel(const float *__restrict__ g, const float *__restrict__ u,
             }
         }
         // conj(lambda_{t+1}); the latest step and steps before time 0 have log-magnitude and angle 0: the identity
-        float top = 0.f;
-#pragma unroll
-        for (int i = 0; i < SEG; ++i)
-#pragma unroll
-            for (int v = 0; v < NP; ++v) { f2_exp_fold(top, c[i][v]); c[i][v] = f2_exp(c[i][v]); }
-        if (!(top <= F2_EXP_MAX)) {
-#pragma unroll
-            for (int i = 0; i < SEG; ++i) {
-                const int t = T - 1 - (rb + i);
-                if (live && t >= 0 && t + 1 < T) ls_exp_any<VEC>(c[i], lm + (row0 + t + 1) * D + d0);
-            }
-        }
 #pragma unroll
         for (int i = 0; i < SEG; ++i) {
             const int t = T - 1 - (rb + i);
@@ -316,7 +290,8 @@ lambda_scan_bwd_kernel(const float *__restrict__ g, const float *__restrict__ u,
 #pragma unroll
             for (int v = 0; v < NP; ++v) {
                 float x0, x1;
-                const f2 mag = c[i][v];
+                f2_unpack(c[i][v], x0, x1);
+                const f2 mag = f2_exp(x0, x1);
                 f2 cs, sn;
                 if constexpr (ANG_BCAST) { cs = ok ? acs[v] : f2_both(1.f); sn = ok ? asn[v] : 0ull; }
                 else { f2_unpack(s[i][v], x0, x1); f2_sincos(x0, x1, sn, cs); }
