@@ -145,8 +145,8 @@ class Decoder:
         """The MLP block for up to 128 decode rows on the decode linear kernel: the GELU goes into the first layer's epilogue, the
         second layer's long contraction over a cluster. Against the library's two products and the separate
         activation, a token of twelve layers: 397 against 424 us at batch 5, 396 - 415 at 16, 429 - 452 at 64. With the block's
-        fused_up off, the library's."""
-        if not (mp.fused_up and 4 < self.B <= 128 and z.dtype == torch.bfloat16 and mp.a.weight.dtype == torch.bfloat16 and z.is_cuda and
+        fused_up off, or layers that are not plain nn.Linear (a wrapper, a parametrization), the block itself."""
+        if not (mp.fused_up and type(mp.a) is type(mp.b) is torch.nn.Linear and 4 < self.B <= 128 and z.dtype == torch.bfloat16 and mp.a.weight.dtype == torch.bfloat16 and z.is_cuda and
                 mp.a.weight.shape[0] % 8 == 0 and z.shape[-1] % 8 == 0):
             return mp.ff(z)
         h = ops.batch_linear(z.reshape(self.B, z.shape[-1]), mp.a.weight, mp.a.bias, act="gelu")

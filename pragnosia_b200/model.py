@@ -32,7 +32,7 @@ class MLP(nn.Module):
 
     def ff(self, z):
         """The block without its norm and residual add."""
-        if (self.fused_up and z.is_cuda and z.dtype == torch.bfloat16 and self.a.weight.dtype == torch.bfloat16
+        if (self.fused_up and type(self.a) is nn.Linear and z.is_cuda and z.dtype == torch.bfloat16 and self.a.weight.dtype == torch.bfloat16
                 and z.shape[-1] % 8 == 0 and self.a.weight.shape[0] % 8 == 0 and z.numel() // z.shape[-1] >= 128):
             return self.b(ops.linear_act(z, self.a.weight, self.a.bias, act="gelu"))
         return self.b(F.gelu(self.a(z)))

@@ -321,3 +321,30 @@ def test_constants_nobody_has_marked_yet():
     assert not layer._fused.mark.due
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("name", ["a", "b"])
+def test_replaced_mlp_layers_are_called(name):
+    """A layer of the MLP that is more than its weight (an adapter, say) keeps its own forward in the decode step of a batch."""
+    class Adapted(torch.nn.Linear):
+        def forward(self, x):
+            return super().forward(x) * 3
+
+    m = lm("aspin")
+    dec = Decoder(m, batch=6, use_graph=False)
+    dec.prefill(ids(6, 70, 1))
+    plain = dec.step(ids(6, 1, 2)[:, 0]).float()
+    for mp in m.mlp:
+        old = getattr(mp, name)
+        new = Adapted(old.in_features, old.out_features).to(DEV).to(torch.bfloat16)
+        new.load_state_dict(old.state_dict())
+        setattr(mp, name, new)
+    dec.prefill(ids(6, 70, 1))
+    got = dec.step(ids(6, 1, 2)[:, 0]).float()
+    for mp in m.mlp:                                                  # the same as weights
+        lin = getattr(mp, name)
+        setattr(mp, name, torch.nn.Linear(lin.in_features, lin.out_features).to(DEV).to(torch.bfloat16))
+        getattr(mp, name).load_state_dict({k: 3 * v for k, v in lin.state_dict().items()})
+    dec.prefill(ids(6, 70, 1))
+    want = dec.step(ids(6, 1, 2)[:, 0]).float()
+    assert float((got - want).norm() / want.norm()) < 2e-2 < float((plain - want).norm() / want.norm())
