@@ -214,8 +214,8 @@ class AssocCarrier(nn.Module):
 
     def _mix_train(self, z, h0):
         """The layer with a gradient wanted (the reference's training path, src/assoc.py:384-512 with its kernels on):
-        separate projections of the live parameters, the differentiable prep / scan operators (their backward kernels are
-        the reference's six), torch for the rest. Plain rule and delta rule with hl_floor / write_all / beta_scale /
+        separate projections of the live parameters, the differentiable prep / scan operators (bf16: the scan's forward and backward
+        as one library call each; compiled or fp32: the composition of the registered operators), torch for the rest. Plain rule and delta rule with hl_floor / write_all / beta_scale /
         pos_wrap; a carried state must come with position 0."""
         from .assoc_kernel import assoc_scan_kernel, delta_scan_kernel, prep_kernel
         if getattr(self, "sconv", None) is not None or self.key_topk:

@@ -8,7 +8,7 @@ namespace pgb {
 
 // ---------------------------------------------------------------------------------------------------- prep backward
 constexpr int PB_WARPS = 8;                                           // consecutive tokens of one (sequence, head) per partial of theta's gradient
-constexpr int PB_TOK = 32;                                            // ... and per CTA of the 16-byte form, which fills four partials' places
+constexpr int PB_TOK = 32;                                            // ... and per CTA of the 16-byte form: their sum, and zeros in the other three places the callers' buffers have
 
 template <typename T_, int PER>
 __device__ __forceinline__ void pb_ld(float (&d)[PER], const T_ *p) {

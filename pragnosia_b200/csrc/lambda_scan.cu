@@ -1,9 +1,10 @@
 // Per-token complex recurrence h_t = lambda_t h_{t-1} + u_t as a chunked parallel scan, and its adjoint.
 //
 // Layout in HBM: u, logmag, y are [B][T][D] fp32 with D contiguous: 12 B read (8 B when the angle is one value per
-// channel) and 4 B written per (b,t,d) element. With expf and sincosf per element the kernel was bound by instruction issue
-// (about 90 instructions an element); e^x, sin, cos and the recurrence now run on pairs of channels (scan_math.cuh, about 40),
-// which puts HBM first where the launch fills the chip.
+// channel) and 4 B written per (b,t,d) element. What bounds it is the wait for a tile's loads at the warps that the registers
+// allow: 80 a thread leave 24 warps an SM, 19 active; issue slots are 55 % busy and HBM runs at 0.64 of a copy. e^x, sin, cos and
+// the recurrence run on pairs of channels (scan_math.cuh): 90 -> 68 instructions an element, B64 T1024 D768 214 -> 197 us (one angle
+// per channel 56 -> 50, 177 -> 155). Rows of 64 or 128 bytes a warp (four time segments or eight) take the same time.
 //
 // Work split. A lane owns VEC adjacent channels (4 where D, pointers and strides allow: one 128-bit access; else 2 or 1). A warp is TS time-segments x CQ
 // channel groups (TS * CQ = 32): lanes of one segment read 16*CQ contiguous bytes of one time row, so every 128-byte

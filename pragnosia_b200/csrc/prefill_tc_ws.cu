@@ -18,7 +18,7 @@
 // Q/K/V tiles triple-buffered, K*w / A / S operand / rotation rows double-buffered, the statistics four deep. The roles
 // meet only at mbarriers (every wait bounded; a wait that runs out sets g_tc_error and the CTA winds down). A waiter never
 // falls two phases behind a barrier: each barrier's next completion depends on the waiter having passed. Arithmetic,
-// operand layouts, precision (bf16 head + tail for every fp32 operand) and results are those of
+// operand layouts, precision (bf16 head + tail for every fp32 operand; a third term of K*w for training) and results are those of
 // prefill_tc_kernel<64, RAW>; that kernel remains the head-dim-128 path.
 #include "tc_common.cuh"
 

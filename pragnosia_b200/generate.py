@@ -194,8 +194,9 @@ class Decoder:
         """Batches past the few-row kernels and up to one 128-row tensor-core tile: every linear layer as one tcgen05
         launch (ops.batch_linear) with the norm in front and the residual add behind folded in. Opt-in (folded=True): it
         needs none of the library's GEMMs and 5 launches a layer instead of 8, measured 2-5 % faster than the library step
-        (0.49 against 0.50 ms per token at batch 64), but the folded norm rounds at other places than the separate ops --
-        the default keeps the roundings the oracle's bf16 mode models."""
+        (0.49 against 0.50 ms per token at batch 64, before the library step took its MLP onto the same kernel), but the folded norm
+        is never rounded to bf16 where a separate norm is. The default rounds after every linear layer, norm, activation and add,
+        as the oracle's bf16 mode does; only the order of fp32 sums inside a product differs between its kernels."""
         m = self.m
         return (self.fused and self.folded and 4 < self.B <= 128 and m.e.weight.dtype == torch.bfloat16 and m.d % 8 == 0 and
                 m.e.weight.shape[0] % 8 == 0 and all(isinstance(mx, AssocCarrier) and mx.plain_step for mx in m.mix) and

@@ -238,7 +238,11 @@ class LM(nn.Module):
                 last, states = c.window_graphs(self, x, window)
                 z = self._add_norm(*last, self.n)[1]
                 if return_states:                                     # the graph's own are overwritten by the next call
-                    states = [tuple(t.clone() if torch.is_tensor(t) else t for t in st) for st in states]
+                    own = [t for st in states for t in st if torch.is_tensor(t)]
+                    kept = [torch.empty_like(t) for t in own]
+                    torch._foreach_copy_(kept, own)
+                    it = iter(kept)
+                    states = [tuple(next(it) if torch.is_tensor(t) else t for t in st) for st in states]
         else:
             states = [None] * self.layers
             last = None

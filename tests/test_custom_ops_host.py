@@ -107,6 +107,7 @@ def test_layer_traces_whole(monkeypatch, delta):
         assert used.count("pragnosia_b200.add_norm") == 2
 
 
+@torch.enable_grad()
 def test_training_entry_points_under_fake_tensors():
     """A torch_dispatch mode (fake tensors, make_fx, selective checkpointing) sees the registered operators, not the C++ node behind
     an eager call."""

@@ -1,4 +1,4 @@
-"""The decode linear layer with its contraction cut over a cluster (2, 3 and 4 CTAs; whole and ragged K, residual and row sums)
+"""The decode linear layer with its contraction cut over a cluster (2 and 4 CTAs; whole and ragged K, residual and row sums)
 against the product in fp32."""
 import pytest
 import torch
