@@ -49,6 +49,7 @@ int pgb_abi_version(void);
  *   u, logmag [B][T][D] fp32.  ang: fp32 with element strides (ang_stride_b, ang_stride_t) and unit stride
  *   over D; strides (0,0) mean one angle per channel (the fspin layer's broadcast, src/spin.py:244).
  *   h0r, h0i [B][D] fp32 or both NULL (zero state).
+ *   |lambda| = e^logmag is exactly 0 for -inf and below 2^-125.5, inf where it overflows, NaN for NaN.
  *   y [B][T][D] fp32 = Re h_t.  hr_out, hi_out [B][D] fp32 = final state.
  * ------------------------------------------------------------------------------------------------------- */
 int pgb_lambda_scan_fwd(const float *u, const float *logmag, const float *ang, long long ang_stride_b,
