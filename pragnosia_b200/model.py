@@ -45,8 +45,8 @@ _MIXERS = {
 }
 
 
-# Tokens of a batch that one pass over many windows takes at most: activations of about 20 KB a token at width 768 (0.65 GB), and
-# GEMMs that long gain nothing from more rows.
+# Tokens of a batch that one pass over many windows takes at most: activations of 12 KB a token at width 768 (20 under the delta
+# rule: 0.63 GB in all), and GEMMs that long gain nothing from more rows.
 WINDOWS_TOKENS = 32768
 
 
