@@ -1,15 +1,16 @@
 // Per-token complex recurrence h_t = lambda_t h_{t-1} + u_t as a chunked parallel scan, and its adjoint.
 //
 // Layout in HBM: u, logmag, y are [B][T][D] fp32 with D contiguous: 12 B read (8 B when the angle is one value per
-// channel) and 4 B written per (b,t,d) element. What bounds it is the wait for a tile's loads at the warps that the registers
-// allow: 80 a thread leave 24 warps an SM, 19 active; issue slots are 55 % busy and HBM runs at 0.64 of a copy. e^x, sin, cos and
-// the recurrence run on pairs of channels (scan_math.cuh): 90 -> 68 instructions an element, B64 T1024 D768 214 -> 197 us (one angle
-// per channel 56 -> 50, 177 -> 155). Rows of 64 or 128 bytes a warp (four time segments or eight) take the same time.
+// channel) and 4 B written per (b,t,d) element. What bounds it is memory: the bytes move at 4.9 TB/s (0.75 of a copy; the adjoint, nine
+// streams, 5.2) with a tile's loads in flight under the arithmetic of the one before. e^x, sin, cos and
+// the recurrence run on pairs of channels (scan_math.cuh, 68 instructions an element, 50 with one angle per channel). B64 T4096 D768:
+// 760 us with loads ahead of their use but inside the tile, 660 with the slots below (one angle per channel 587 -> 447); B16 T4096 D768
+// 253 -> 200 (199 -> 141).
 //
 // Work split. A lane owns VEC adjacent channels (4 where D, pointers and strides allow: one 128-bit access; else 2 or 1). A warp is TS time-segments x CQ
 // channel groups (TS * CQ = 32): lanes of one segment read 16*CQ contiguous bytes of one time row, so every 128-byte
 // line is used whole. A tile is TS*SEG consecutive time steps; per tile each lane
-//   1. loads its SEG steps (all loads issued before any is used) and forms c_t = |l_t| cos, s_t = |l_t| sin,
+//   1. takes its SEG steps, requested two tiles ahead, and forms c_t = |l_t| cos, s_t = |l_t| sin,
 //   2. folds them into the segment's affine map h -> A h + Bv (complex A, Bv), starting from (1, 0),
 //   3. combines the maps of the segments before it with a shuffle scan over the TS segment lanes
 //      ((A2,B2) o (A1,B1) = (A2 A1, A2 B1 + B2)), which gives the state entering its segment,
@@ -17,20 +18,22 @@
 //      (src/scan_kernel.py:42-48) and stores Re h.
 // The state leaving the tile is broadcast from the last segment lane. With TS = 1 the kernel is the literal sequential
 // recurrence; with TS > 1 only the state at segment boundaries is reassociated (fp32 rounding, no other difference).
+#include <math.h>
+
 #include "scan_math.cuh"
 
 namespace pgb {
 
 constexpr int LS_WARPS = 2;
-// Two forms of the forward kernel. WIDE fills the chip with warps: 24 an SM (80 registers a thread), every load of a tile ahead
-// of its use, four steps a lane and tile (two with one angle per channel, whose cosines take the registers, and with Im h kept). AHEAD is for
-// launches with fewer warps than that, which cannot hide a tile's loads behind one another: two steps a lane and tile (four
-// with narrow vectors) and the next tile requested before this one is worked on, 16 warps an SM (12 with 32 segments).
-// B64 T4096 D768: wide 785-830 us (577 with one angle per channel; with Im h 930 and 719), ahead 1291; B4 T2048 D768, one angle
-// per channel: 63 and 52; B16 T512 D704, one angle per channel, with Im h: 53 and 35.
-template <int VEC, bool AHEAD, bool FEW> struct LsSeg { static constexpr int n = VEC < 4 ? 4 : (AHEAD || FEW ? 2 : 4); };
-constexpr int LS_WIDE_CTAS = 12, LS_AHEAD_CTAS = 8, LS_AHEAD_CTAS_TS32 = 6;
-constexpr int LS_BWD_CTAS_PER_SM = 6;                                 // the adjoint: 168 registers, it holds the states of its steps as well
+// Where a lane owns four channels, its steps of the coming two tiles travel global -> shared memory by asynchronous copies into slots
+// that only this lane reads, so no registers are held while they fly and nobody synchronises: a tile is read out of its slot,
+// the slot is requested again, and the arithmetic of the tile runs under the copy. 16 warps an SM are enough then (a tile of loads ahead of
+// its use needed 24, B64 T4096 D768 760 us against 660, one angle per channel 590 against 480; spills are poison next to this much shared
+// memory, which leaves the L1 no room: 1010 us with 24 warps and 70 bytes spilled). Narrower lanes request the next tile into
+// registers: a copy of 4 or 8 bytes costs an instruction more than it saves (B13 T1111 D510: 44 against 54 us).
+template <int VEC> struct LsForm { static constexpr bool staged = VEC == 4; static constexpr int slots = staged ? 2 : 1; };
+constexpr int LS_SEG = 4;                                             // steps a lane takes of a tile
+constexpr int LS_CTAS_PER_SM = 8;                                     // the same for the adjoint, whose slots make room for two warps more an SM
 
 // VEC adjacent channels of one row as pairs (the last one half empty when VEC is 1)
 template <int VEC> struct LsVec { static constexpr int NP = (VEC + 1) / 2; };
@@ -44,10 +47,22 @@ __device__ __forceinline__ void ls_ld(f2 (&d)[LsVec<VEC>::NP], const float *p) {
 }
 template <int VEC>
 __device__ __forceinline__ void ls_st(float *p, const f2 (&d)[LsVec<VEC>::NP]) {
-    if constexpr (VEC == 4) *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(d[0], d[1]);
+    if constexpr (VEC == 4) __stcs(reinterpret_cast<ulonglong2 *>(p), make_ulonglong2(d[0], d[1]));
     else if constexpr (VEC == 2) *reinterpret_cast<f2 *>(p) = d[0];
     else { float a, b; f2_unpack(d[0], a, b); *p = a; }
 }
+// one step's channels of this lane into its slot; false: zeros (nothing is read)
+template <int VEC>
+__device__ __forceinline__ void ls_cp(float *slot, const float *src, bool live) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(slot);
+    const int n = live ? 4 * VEC : 0;
+    if constexpr (VEC == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+    else if constexpr (VEC == 2) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void ls_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void ls_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 // a complex pair product and sum: (ar + i ai)(br + i bi) + (cr + i ci)
 __device__ __forceinline__ void ls_cfma(f2 &outr, f2 &outi, f2 ar, f2 ai, f2 br, f2 bi, f2 cr, f2 ci) {
     const f2 nai = f2_neg(ai);
@@ -73,14 +88,17 @@ __device__ __forceinline__ void ls_scan_maps(f2 &Ar, f2 &Ai, f2 &Br, f2 &Bi, int
     if (seg == 0) { Ar = f2_both(1.f); Ai = 0ull; Br = 0ull; Bi = 0ull; }
 }
 
-template <int VEC, int TS, bool ANG_BCAST, bool KEEP, bool AHEAD>
-__global__ void __launch_bounds__(LS_WARPS * 32, !AHEAD ? LS_WIDE_CTAS : TS == 32 ? LS_AHEAD_CTAS_TS32 : LS_AHEAD_CTAS)
+template <int VEC, int TS, bool ANG_BCAST, bool KEEP>
+__global__ void __launch_bounds__(LS_WARPS * 32, LS_CTAS_PER_SM)
 lambda_scan_kernel(const float *__restrict__ u, const float *__restrict__ lm, const float *__restrict__ an,
                    long long an_sb, long long an_st, const float *__restrict__ h0r, const float *__restrict__ h0i,
                    float *__restrict__ y, float *__restrict__ hr_out, float *__restrict__ hi_out, float *__restrict__ hi_all,
                    int B, int T, int D) {
-    constexpr int CQ = 32 / TS, SEG = LsSeg<VEC, AHEAD, ANG_BCAST || KEEP>::n, NP = LsVec<VEC>::NP;
+    using Form = LsForm<VEC>;
+    constexpr int CQ = 32 / TS, SEG = LS_SEG, NST = Form::slots, NP = LsVec<VEC>::NP;
+    constexpr int NA = ANG_BCAST ? 2 : 3;                          // u, logmag, angle
     constexpr unsigned FULL = 0xffffffffu;
+    __shared__ __align__(16) float slots[Form::staged ? NST : 1][NA][SEG][Form::staged ? LS_WARPS * 32 * VEC : 1];
     const int lane = threadIdx.x & 31;
     const int ngroups = D / VEC;
     const int wpb = (ngroups + CQ - 1) / CQ;                       // warps per batch row
@@ -111,7 +129,21 @@ lambda_scan_kernel(const float *__restrict__ u, const float *__restrict__ lm, co
     }
 
     const size_t row0 = (size_t)b * T;
-    auto fetch = [&](int tb, f2 (&c)[SEG][NP], f2 (&s)[SEG][NP], f2 (&x)[SEG][NP]) {       // every load of a lane's steps
+    const int my = (int)threadIdx.x * VEC;
+    auto request = [&](int tb, int slot) {                             // one group of copies: a lane's steps of one tile
+        if constexpr (!Form::staged) return;
+#pragma unroll
+        for (int i = 0; i < SEG; ++i) {
+            const int t = tb + i;
+            const bool ok = live && t < T;
+            const size_t off = ok ? (row0 + t) * D + d0 : 0;
+            ls_cp<VEC>(&slots[slot][0][i][my], u + off, ok);
+            ls_cp<VEC>(&slots[slot][1][i][my], lm + off, ok);
+            if constexpr (!ANG_BCAST) ls_cp<VEC>(&slots[slot][NA - 1][i][my], ok ? an + (size_t)b * an_sb + (size_t)t * an_st + d0 : an, ok);
+        }
+        ls_cp_commit();
+    };
+    auto fetch = [&](int tb, f2 (&c)[SEG][NP], f2 (&s)[SEG][NP], f2 (&x)[SEG][NP]) {       // the same into registers
 #pragma unroll
         for (int i = 0; i < SEG; ++i) {
             const int t = tb + i;
@@ -126,19 +158,32 @@ lambda_scan_kernel(const float *__restrict__ u, const float *__restrict__ lm, co
             }
         }
     };
-    f2 nc[AHEAD ? SEG : 1][NP], ns[AHEAD ? SEG : 1][NP], nx[AHEAD ? SEG : 1][NP];
-    if constexpr (AHEAD) fetch(seg * SEG, nc, ns, nx);
-    for (int t0 = 0; t0 < T; t0 += TS * SEG) {
+    constexpr int NREG = Form::staged ? 1 : SEG;
+    f2 nc[NREG][NP], ns[NREG][NP], nx[NREG][NP];
+    if constexpr (Form::staged) {
+#pragma unroll
+        for (int k = 0; k < NST; ++k) request((k * TS + seg) * SEG, k);
+    } else fetch(seg * SEG, nc, ns, nx);
+    for (int t0 = 0, slot = 0; t0 < T; t0 += TS * SEG, slot = slot + 1 == NST ? 0 : slot + 1) {
         const int tb = t0 + seg * SEG;
         f2 c[SEG][NP], s[SEG][NP], x[SEG][NP];
-        // 1. loads first
-        if constexpr (AHEAD) {
+        // 1. the tile out of its slot (or the registers it was requested into), and a later one requested in its place
+        if constexpr (Form::staged) {
+            ls_cp_wait<NST - 1>();
+#pragma unroll
+            for (int i = 0; i < SEG; ++i) {
+                ls_ld<VEC>(x[i], &slots[slot][0][i][my]);
+                ls_ld<VEC>(c[i], &slots[slot][1][i][my]);
+                if constexpr (!ANG_BCAST) ls_ld<VEC>(s[i], &slots[slot][NA - 1][i][my]);
+            }
+            request(tb + NST * TS * SEG, slot);
+        } else {
 #pragma unroll
             for (int i = 0; i < SEG; ++i)
 #pragma unroll
                 for (int v = 0; v < NP; ++v) { c[i][v] = nc[i][v]; s[i][v] = ns[i][v]; x[i][v] = nx[i][v]; }
             if (t0 + TS * SEG < T) fetch(tb + TS * SEG, nc, ns, nx);
-        } else fetch(tb, c, s, x);
+        }
         // lambda of every step; steps past the end keep log-magnitude and angle 0, the identity map
 #pragma unroll
         for (int i = 0; i < SEG; ++i) {
@@ -199,6 +244,7 @@ lambda_scan_kernel(const float *__restrict__ u, const float *__restrict__ lm, co
             }
         }
     }
+    ls_cp_wait<0>();                                                   // nothing may land in the slots behind the block's end
     if (live && seg == 0) {
         ls_st<VEC>(hr_out + (size_t)b * D + d0, hr);
         ls_st<VEC>(hi_out + (size_t)b * D + d0, hi);
@@ -208,16 +254,19 @@ lambda_scan_kernel(const float *__restrict__ u, const float *__restrict__ lm, co
 // The adjoint, a_{t-1} = conj(lambda_t) a_t + g_{t-1}, as the same scan over the reversed sequence (reference:
 // src/scan_kernel.py:54-101, wired at :121-140); with R_t h_{t-1} = h_t - (u_t, 0) the per-token gradients are
 //   du_t = Re a_t,   dlogmag_t = a_t . (h_t - u_t),   dang_t = a_t . i (h_t - u_t).
-// One lane per four channels instead of one, the state's rows requested before the scan over the segments. B64 T4096 D768, one
-// angle per channel: 5716 -> 1430-1670 us (4.3-4.5 TB/s); B16 T512 D704: 123 -> 63 us.
+// One lane per four channels; its loads go through slots as in the forward kernel: maps (g, logmag, angle) a tile ahead, states and u
+// requested when the tile before is done, so that the registers hold the maps only (128, 16 warps an SM; 168 and 12 before).
+// B64 T4096 D768 1563 -> 1310 us, one angle per channel 1347 -> 1090; B16 T512 D704: 58 -> 47.
 template <int VEC, int TS, bool ANG_BCAST>
-__global__ void __launch_bounds__(LS_WARPS * 32, LS_BWD_CTAS_PER_SM)
+__global__ void __launch_bounds__(LS_WARPS * 32, LS_CTAS_PER_SM)
 lambda_scan_bwd_kernel(const float *__restrict__ g, const float *__restrict__ u, const float *__restrict__ lm, const float *__restrict__ an,
                        long long an_sb, long long an_st, const float *__restrict__ hr_all, const float *__restrict__ hi_all,
                        const float *__restrict__ gli, float *__restrict__ du, float *__restrict__ dlm, float *__restrict__ dan,
                        float *__restrict__ dh0r, float *__restrict__ dh0i, int B, int T, int D) {
-    constexpr int CQ = 32 / TS, SEG = 4, NP = LsVec<VEC>::NP;
+    constexpr int CQ = 32 / TS, SEG = LS_SEG, NP = LsVec<VEC>::NP, NA = ANG_BCAST ? 2 : 3;
     constexpr unsigned FULL = 0xffffffffu;
+    // g, logmag, angle: free again before the tile's arithmetic; Re h, Im h, u: read step by step in the replay
+    __shared__ __align__(16) float slots[NA + 3][SEG][LS_WARPS * 32 * VEC];
     const int lane = threadIdx.x & 31;
     const int ngroups = D / VEC;
     const int wpb = (ngroups + CQ - 1) / CQ;
@@ -253,36 +302,43 @@ lambda_scan_bwd_kernel(const float *__restrict__ g, const float *__restrict__ u,
 #pragma unroll
         for (int v = 0; v < NP; ++v) { float a0, a1; f2_unpack(a[v], a0, a1); f2_sincos(a0, a1, asn[v], acs[v]); }
     }
-    for (int r0 = 0; r0 < T; r0 += TS * SEG) {
-        const int rb = r0 + seg * SEG;                             // reversed step index; time t = T - 1 - r
-        f2 c[SEG][NP], s[SEG][NP], x[SEG][NP], rr[SEG][NP], ri[SEG][NP];
+    const int my = (int)threadIdx.x * VEC;
+    auto request_map = [&](int rb) {                                   // steps past either end: zeros, the identity map
 #pragma unroll
         for (int i = 0; i < SEG; ++i) {
             const int t = T - 1 - (rb + i);
-#pragma unroll
-            for (int v = 0; v < NP; ++v) { c[i][v] = 0ull; s[i][v] = 0ull; x[i][v] = 0ull; rr[i][v] = 0ull; ri[i][v] = 0ull; }
-            if (live && t >= 0) {
-                const size_t off = (row0 + t) * D + d0;
-                ls_ld<VEC>(x[i], g + off);
-                if (t + 1 < T) {
-                    ls_ld<VEC>(c[i], lm + off + D);
-                    if constexpr (!ANG_BCAST) ls_ld<VEC>(s[i], an + (size_t)b * an_sb + (size_t)(t + 1) * an_st + d0);
-                }
-            }
+            const bool ok = live && t >= 0, next = ok && t + 1 < T;
+            ls_cp<VEC>(&slots[0][i][my], ok ? g + (row0 + t) * D + d0 : g, ok);
+            ls_cp<VEC>(&slots[1][i][my], next ? lm + (row0 + t + 1) * D + d0 : lm, next);
+            if constexpr (!ANG_BCAST) ls_cp<VEC>(&slots[NA - 1][i][my], next ? an + (size_t)b * an_sb + (size_t)(t + 1) * an_st + d0 : an, next);
         }
+        ls_cp_commit();
+    };
+    auto request_states = [&](int rb) {
 #pragma unroll
-        for (int i = 0; i < SEG; ++i) {                            // lambda_t h_{t-1} = h_t - (u_t, 0)
+        for (int i = 0; i < SEG; ++i) {
             const int t = T - 1 - (rb + i);
-            if (live && t >= 0) {
-                const size_t off = (row0 + t) * D + d0;
-                f2 uu[NP];
-                ls_ld<VEC>(rr[i], hr_all + off);
-                ls_ld<VEC>(uu, u + off);
-                ls_ld<VEC>(ri[i], hi_all + off);
-#pragma unroll
-                for (int v = 0; v < NP; ++v) rr[i][v] = f2_add(rr[i][v], f2_neg(uu[v]));
-            }
+            const bool ok = live && t >= 0;
+            const size_t off = ok ? (row0 + t) * D + d0 : 0;
+            ls_cp<VEC>(&slots[NA][i][my], hr_all + off, ok);
+            ls_cp<VEC>(&slots[NA + 1][i][my], hi_all + off, ok);
+            ls_cp<VEC>(&slots[NA + 2][i][my], u + off, ok);
         }
+        ls_cp_commit();
+    };
+    request_map(seg * SEG);
+    request_states(seg * SEG);
+    for (int r0 = 0; r0 < T; r0 += TS * SEG) {
+        const int rb = r0 + seg * SEG;                             // reversed step index; time t = T - 1 - r
+        f2 c[SEG][NP], s[SEG][NP], x[SEG][NP];
+        ls_cp_wait<1>();                                           // the tile's maps are here, its states may still be on their way
+#pragma unroll
+        for (int i = 0; i < SEG; ++i) {
+            ls_ld<VEC>(x[i], &slots[0][i][my]);
+            ls_ld<VEC>(c[i], &slots[1][i][my]);
+            if constexpr (!ANG_BCAST) ls_ld<VEC>(s[i], &slots[NA - 1][i][my]);
+        }
+        request_map(rb + TS * SEG);
         // conj(lambda_{t+1}); the latest step and steps before time 0 have log-magnitude and angle 0: the identity
 #pragma unroll
         for (int i = 0; i < SEG; ++i) {
@@ -317,17 +373,22 @@ lambda_scan_bwd_kernel(const float *__restrict__ g, const float *__restrict__ u,
                 ls_cfma(hsr[v], hsi[v], Ar, Ai, ar[v], ai[v], Br, Bi);
             }
         }
+        ls_cp_wait<1>();                                           // the tile's states are here, the next one's maps may still be on their way
 #pragma unroll
         for (int i = 0; i < SEG; ++i) {
             const int t = T - 1 - (rb + i);
-            f2 dl[NP], da[NP];
+            f2 dl[NP], da[NP], rr[NP], ri[NP], uu[NP];             // lambda_t h_{t-1} = h_t - (u_t, 0)
+            ls_ld<VEC>(rr, &slots[NA][i][my]);
+            ls_ld<VEC>(ri, &slots[NA + 1][i][my]);
+            ls_ld<VEC>(uu, &slots[NA + 2][i][my]);
 #pragma unroll
             for (int v = 0; v < NP; ++v) {
+                rr[v] = f2_add(rr[v], f2_neg(uu[v]));
                 f2 nr, ni;
                 ls_cfma(nr, ni, c[i][v], s[i][v], hsr[v], hsi[v], x[i][v], 0ull);
                 hsr[v] = nr; hsi[v] = ni;
-                dl[v] = f2_fma(nr, rr[i][v], f2_mul(ni, ri[i][v]));
-                da[v] = f2_fma(ni, rr[i][v], f2_neg(f2_mul(nr, ri[i][v])));
+                dl[v] = f2_fma(nr, rr[v], f2_mul(ni, ri[v]));
+                da[v] = f2_fma(ni, rr[v], f2_neg(f2_mul(nr, ri[v])));
             }
             if (live && t >= 0) {
                 const size_t off = (row0 + t) * D + d0;
@@ -336,6 +397,7 @@ lambda_scan_bwd_kernel(const float *__restrict__ g, const float *__restrict__ u,
                 ls_st<VEC>(dan + off, da);
             }
         }
+        request_states(rb + TS * SEG);
 #pragma unroll
         for (int v = 0; v < NP; ++v) {
             if constexpr (TS > 1) {
@@ -346,6 +408,7 @@ lambda_scan_bwd_kernel(const float *__restrict__ g, const float *__restrict__ u,
             }
         }
     }
+    ls_cp_wait<0>();                                                   // nothing may land in the slots behind the block's end
     if (live && seg == 0 && dh0r != nullptr) {                     // a_{-1} = conj(lambda_0) a_0
         f2 l[NP], a[NP], c[NP], s[NP], outr[NP], outi[NP];
         ls_ld<VEC>(l, lm + row0 * D + d0);
@@ -363,7 +426,6 @@ namespace {
 struct LsArgs {
     const float *u, *lm, *an; long long sb, st; const float *h0r, *h0i; float *y, *hro, *hio, *hia;
     int B, T, D;
-    bool wide;
 };
 struct LsBwdArgs {
     const float *g, *u, *lm, *an; long long sb, st; const float *hr_all, *hi_all, *gli; float *du, *dlm, *dan, *dh0r, *dh0i;
@@ -385,14 +447,8 @@ int launch_ts(const LsArgs &a, cudaStream_t stream) {
         kern<<<(unsigned)ctas, LS_WARPS * 32, 0, stream>>>(a.u, a.lm, a.an, a.sb, a.st, a.h0r, a.h0i, a.y, a.hro, a.hio, a.hia, a.B, a.T, a.D);
     };
     const bool bc = a.sb == 0 && a.st == 0, keep = a.hia != nullptr;
-    if constexpr (VEC == 4 && TS < 32)
-        if (a.wide) {
-            if (keep) { if (bc) go(lambda_scan_kernel<VEC, TS, true, true, false>); else go(lambda_scan_kernel<VEC, TS, false, true, false>); }
-            else { if (bc) go(lambda_scan_kernel<VEC, TS, true, false, false>); else go(lambda_scan_kernel<VEC, TS, false, false, false>); }
-            return check_launch("lambda_scan_kernel");
-        }
-    if (keep) { if (bc) go(lambda_scan_kernel<VEC, TS, true, true, true>); else go(lambda_scan_kernel<VEC, TS, false, true, true>); }
-    else { if (bc) go(lambda_scan_kernel<VEC, TS, true, false, true>); else go(lambda_scan_kernel<VEC, TS, false, false, true>); }
+    if (keep) { if (bc) go(lambda_scan_kernel<VEC, TS, true, true>); else go(lambda_scan_kernel<VEC, TS, false, true>); }
+    else { if (bc) go(lambda_scan_kernel<VEC, TS, true, false>); else go(lambda_scan_kernel<VEC, TS, false, false>); }
     return check_launch("lambda_scan_kernel");
 }
 template <int VEC, int TS>
@@ -432,50 +488,53 @@ int ls_vec(int D, long long sb, long long st, P... ptrs) {
 
 }  // namespace
 
-// Number of time segments per warp. Every warp walks its whole time axis and all warps of a launch take the same time, so the
-// launch lasts rounds x tiles-per-warp x tile cost with rounds = ceil(warps / resident warps). More segments shorten a warp's
-// walk but cost shuffle-scan rounds and, past the resident capacity, a whole extra round; and 32 segments leave each row access
-// 16 bytes wide, half a memory sector, which costs as much again once there are warps enough to load memory (B52 T1579
-// D240: 143 us with 32, 102 with 16). Take the power of two with the smallest estimate. `force_ts` > 0 overrides (tests).
-static int ls_pick(int B, int T, int D, int vec, int seg, int sms, int ctas_per_sm) {
+// Number of time segments per warp, the power of two with the smallest estimate. A launch takes (i) the walk of a warp -- its
+// tiles, 1.2 us each (the adjoint's 1.75) and a little for every round of the scan over the segments, times
+// warps / resident warps where that is more than one -- and (ii) the bytes at 5 (the adjoint 6) TB/s and, for narrow lanes, their
+// instructions; more segments shorten (i), but make the rows a warp reads narrower: the adjoint with rows of 256, 128, 64, 32 and 16 bytes takes
+// 1231, 1315, 1410, 1744 and 3241 us at B64 T4096 D768, the scan forward without a copy of the state 886, 642, 662, 725 and 1300. The two overlap:
+// root of the sum of squares (B16 T4096 D768, 2 to 16 segments: 652, 362, 259, 201 us; the estimate says 645, 370, 258, 209).
+struct LsCost { double tile_us, ps, narrow_ps; bool adjoint; };       // per tile; per element: the bytes' time, the instructions' of lanes with one channel
+static int ls_pick(int B, int T, int D, int vec, const LsCost &k, int sms) {
+    static const double width[7] = {1.0, 1.0, 1.08, 1.4, 2.3, 3.5, 6.0};        // rows of 256, 128, ... 4 bytes
     const int ngroups = D / vec;
-    const long long cap = (long long)sms * ctas_per_sm * LS_WARPS;              // resident warps
+    const double cap = (double)sms * LS_CTAS_PER_SM * LS_WARPS;                 // resident warps
     int best = 1;
     double best_cost = 0.0;
     for (int ts = 1, lg = 0; ts <= 32; ts <<= 1, ++lg) {
-        if (ts > 1 && (ts / 2) * seg >= T) break;                               // the sequence has no more pieces to hand out
+        if (ts > 1 && (ts / 2) * LS_SEG >= T) break;                            // the sequence has no more pieces to hand out
         const int cq = 32 / ts;
-        const long long warps = (long long)B * ((ngroups + cq - 1) / cq);
-        const long long rounds = (warps + cap - 1) / cap;
-        const long long tiles = (T + ts * seg - 1) / (ts * seg);
-        const double tile = seg * 60.0 + lg * 14.0 + 12.0;                      // per lane and channel: steps, scan rounds, hand-over
-        const double cost = (double)rounds * (double)tiles * tile * (ts == 32 && warps > 8LL * sms ? 2.0 : 1.0);
+        const long long warps = (long long)B * ((ngroups + cq - 1) / cq), tiles = (T + ts * LS_SEG - 1) / (ts * LS_SEG);
+        int w = 0;
+        for (int row = 4 * vec * cq; row < 256; row <<= 1) ++w;
+        double f = width[w < 6 ? w : 6];
+        if (!k.adjoint && w <= 4) f = sqrt(f);
+        if (ts == 32 && warps <= 8LL * sms && f > 1.4) f = 1.4;                 // few warps do not load the memory: a narrow row costs no more than another
+        const double walk = (double)tiles * (k.tile_us + 0.1 * lg) * (warps > cap ? (double)warps / cap : 1.0);
+        const double move = (double)B * T * D * 1e-6 * (k.ps * f + (vec == 1 ? k.narrow_ps : 0.0));
+        const double cost = walk * walk + move * move;
         if (ts == 1 || cost < best_cost) { best = ts; best_cost = cost; }
     }
     return best;
 }
+static LsCost ls_cost_fwd(bool bcast, bool keep) { return {1.2, 3.2 - (bcast ? 0.8 : 0.0) + (keep ? 0.8 : 0.0), 3.0, false}; }
 int lambda_scan_pick_ts(int B, int T, int D, int vec, int sms, int force_ts) {
-    return force_ts > 0 ? force_ts : ls_pick(B, T, D, vec, LsSeg<4, false, false>::n, sms, LS_WIDE_CTAS);
+    return force_ts > 0 ? force_ts : ls_pick(B, T, D, vec, ls_cost_fwd(false, false), sms);
 }
 
 int lambda_scan_launch(const float *u, const float *lm, const float *an, long long sb, long long st, const float *h0r,
                        const float *h0i, float *y, float *hro, float *hio, float *hia, int B, int T, int D, int force_ts,
                        cudaStream_t stream) {
-    const int sms = sm_count();
     const int vec = ls_vec(D, sb, st, u, lm, an, y, hia, hro, hio, h0r, h0i);
-    int ts = lambda_scan_pick_ts(B, T, D, vec, sms, force_ts);
-    // the wide form where its warps outnumber what the form that loads ahead can keep resident
-    const int cq = 32 / ts;
-    const bool wide = vec == 4 && ts < 32 && (long long)B * ((D / vec + cq - 1) / cq) > (long long)sms * LS_AHEAD_CTAS * LS_WARPS;
-    if (!wide && force_ts <= 0) ts = ls_pick(B, T, D, vec, LsSeg<4, true, false>::n, sms, LS_AHEAD_CTAS);
-    return launch_any(vec, ts, LsArgs{u, lm, an, sb, st, h0r, h0i, y, hro, hio, hia, B, T, D, wide}, stream);
+    const int ts = force_ts > 0 ? force_ts : ls_pick(B, T, D, vec, ls_cost_fwd(sb == 0 && st == 0, hia != nullptr), sm_count());
+    return launch_any(vec, ts, LsArgs{u, lm, an, sb, st, h0r, h0i, y, hro, hio, hia, B, T, D}, stream);
 }
 
 int lambda_scan_bwd_launch(const float *g, const float *u, const float *lm, const float *an, long long sb, long long st,
                            const float *hr_all, const float *hi_all, const float *gli, float *du, float *dlm, float *dan,
                            float *dh0r, float *dh0i, int B, int T, int D, cudaStream_t stream) {
     const int vec = ls_vec(D, sb, st, g, u, lm, an, hr_all, hi_all, gli, du, dlm, dan, dh0r, dh0i);
-    const int ts = ls_pick(B, T, D, vec, 4, sm_count(), LS_BWD_CTAS_PER_SM);
+    const int ts = ls_pick(B, T, D, vec, LsCost{1.75, sb == 0 && st == 0 ? 5.1 : 6.1, 4.5, true}, sm_count());
     return launch_any(vec, ts, LsBwdArgs{g, u, lm, an, sb, st, hr_all, hi_all, gli, du, dlm, dan, dh0r, dh0i, B, T, D}, stream);
 }
 

@@ -38,6 +38,20 @@ def test_lambda_scan_and_adjoint_forms(B, T, D, per_channel):
             assert rel(a, b) < 2e-5
 
 
+@pytest.mark.parametrize("ts", [1, 4, 32])
+@pytest.mark.parametrize("T", [2, 15, 16, 17, 33, 140, 385])
+@pytest.mark.parametrize("D", [8, 68])
+def test_lambda_scan_slots(ts, T, D):
+    """Tiles of 4 ts steps in two slots a lane: sequences of less than one tile, of exactly one, of a few and a remainder."""
+    g = torch.Generator(device=DEV).manual_seed(T + D)
+    u, lm, an = (torch.randn(2, T, D, device=DEV, generator=g) for _ in range(3))
+    lm = -lm.abs()
+    y, (hr, hi) = ops.lambda_scan(u, lm, an, None, time_segments=ts)
+    ry, (rr, ri) = oracle.lambda_literal(u.double(), lm.double(), an.double(), None)
+    for a, b in ((y, ry), (hr, rr), (hi, ri)):
+        assert rel(a, b) < 5e-6
+
+
 @pytest.mark.parametrize("T", [1, 31, 32, 33, 100])
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("strided", [False, True])
