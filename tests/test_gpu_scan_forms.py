@@ -46,8 +46,9 @@ def test_lambda_scan_slots(ts, T, D):
     g = torch.Generator(device=DEV).manual_seed(T + D)
     u, lm, an = (torch.randn(2, T, D, device=DEV, generator=g) for _ in range(3))
     lm = -lm.abs()
-    y, (hr, hi) = ops.lambda_scan(u, lm, an, None, time_segments=ts)
-    ry, (rr, ri) = oracle.lambda_literal(u.double(), lm.double(), an.double(), None)
+    h0 = (torch.randn(2, D, device=DEV, generator=g), torch.randn(2, D, device=DEV, generator=g))
+    y, (hr, hi) = ops.lambda_scan(u, lm, an, h0, time_segments=ts)
+    ry, (rr, ri) = oracle.lambda_literal(u.double(), lm.double(), an.double(), tuple(h.double() for h in h0))
     for a, b in ((y, ry), (hr, rr), (hi, ri)):
         assert rel(a, b) < 5e-6
 
