@@ -468,6 +468,17 @@ int pgb_decode_token_step_fwd(const void *layer_table, int L, const void *E, con
                               long long *pos, float *shift, int window, void *work, long long work_bytes, float *logits,
                               unsigned long long *sync, int B, int d, int H, int D, int NP, int dff, int V, int ctx, int delta,
                               void *stream);
+/* The same step with no barrier in it: values go from CTA to CTA as 32-bit words that carry the launch's mark.
+ *   work: pgb_decode_flow_work_bytes(L, B, d, NP, dff) bytes, 16-byte aligned, zero before the first launch and then left to the kernel
+ *         (0: the shapes want more shared memory than there is; take the step above).
+ *   sync: as above, and the pair belongs to its work: both are zeroed or replaced together, and another device's launches have their own.
+ * A wait that runs out makes the whole grid return and pgb_tc_error_flag reads 82; nothing needs resetting after it. */
+long long pgb_decode_flow_work_bytes(int L, int B, int d, int NP, int dff);
+int pgb_decode_flow_step_fwd(const void *layer_table, int L, const void *E, const void *P, const void *final_norm_weight,
+                             const void *final_norm_bias, int final_norm_kind, float final_norm_eps, const long long *tok,
+                             long long *pos, float *shift, int window, void *work, long long work_bytes, float *logits,
+                             unsigned long long *sync, int B, int d, int H, int D, int NP, int dff, int V, int ctx, int delta,
+                             void *stream);
 
 /* ---------------------------------------------------------------------------------------------------------
  * y = act(x W^T + bias) as one tcgen05 GEMM with the bias and the activation applied on the accumulator in the epilogue.

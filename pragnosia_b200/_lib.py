@@ -70,6 +70,9 @@ SIGNATURES = {
                              _i, _vp],
     "pgb_decode_token_step_fwd": [_vp, _i, _vp, _vp, _vp, _vp, _i, _f, _vp, _vp, _vp, _i, _vp, _ll, _vp, _vp, _i, _i, _i, _i, _i, _i, _i,
                                   _i, _i, _vp],
+    "pgb_decode_flow_work_bytes": [_i, _i, _i, _i, _i],
+    "pgb_decode_flow_step_fwd": [_vp, _i, _vp, _vp, _vp, _vp, _i, _f, _vp, _vp, _vp, _i, _vp, _ll, _vp, _vp, _i, _i, _i, _i, _i, _i, _i,
+                                 _i, _i, _vp],
     "pgb_tc_wait_selftest": [_ll, _vp],
     "pgb_linear_act": [_vp, _vp, _vp, _vp, _ll, _i, _i, _i, _vp],
     "pgb_skinny_linear": [_vp, _vp, _vp, _vp, _i, _f, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _vp],

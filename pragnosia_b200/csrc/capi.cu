@@ -86,6 +86,10 @@ int decode_token_launch(const void *, int, const void *, const void *, const voi
                         int, int, cudaStream_t);
 size_t decode_token_work_bytes(int B, int d, int NP, int dff);
 int decode_token_error_flag(int *);
+int decode_flow_launch(const void *, int, const void *, const void *, const void *, const void *, int, float, const long long *, long long *, float *,
+                       void *, float *, unsigned long long *, int, int, int, int, int, int, int, int, int, int, cudaStream_t);
+size_t decode_flow_work_bytes(int L, int B, int d, int NP, int dff);
+int decode_flow_error_flag(int *);
 int batch_linear_launch(const void *, const void *, const void *, void *, int, int, int, int, const float *, int, const float *, const float *,
                         int, float, const void *, float *, int, cudaStream_t);
 int batch_linear_parts(int N);
@@ -605,26 +609,60 @@ long long pgb_decode_token_work_bytes(int B, int d, int NP, int dff) {
     return (long long)decode_token_work_bytes(B, d, NP, dff);
 }
 
-int pgb_decode_token_step_fwd(const void *layer_table, int L, const void *E, const void *P, const void *final_norm_weight,
-                         const void *final_norm_bias, int final_norm_kind, float final_norm_eps, const long long *tok,
-                         long long *pos, float *shift, int window, void *work, long long work_bytes, float *logits,
-                         unsigned long long *sync, int B, int d, int H, int D, int NP, int dff, int V, int ctx, int delta,
-                         void *stream) {
+// what both one-launch steps ask of their arguments
+static int decode_token_check(const void *layer_table, int L, const void *E, const void *P, const void *final_norm_weight,
+                              const void *final_norm_bias, int final_norm_kind, const long long *tok, const long long *pos, const float *shift, int window,
+                              const void *work, const float *logits, const unsigned long long *sync, int B, int d, int H, int D, int NP, int dff, int V,
+                              int ctx) {
     if (!layer_table || !E || !P || !final_norm_weight || !tok || !pos || !shift || !work || !logits || !sync) return PGB_ERR_NULL_POINTER;
     if (final_norm_kind != 1 && final_norm_kind != 2) return PGB_ERR_BAD_SHAPE;
     if (final_norm_kind == 2 && !final_norm_bias) return PGB_ERR_NULL_POINTER;
     if (D != 64 && D != 128) return PGB_ERR_UNSUPPORTED_DIM;
     if (L < 1 || B < 1 || H < 1 || d != H * D || (dff % 8) != 0 || dff < 8 || (NP % 8) != 0 || NP < 3 * d + 2 * H || V < 1 || ctx < 1 || window < 0)
         return PGB_ERR_BAD_SHAPE;
-    if (B > 4 || (long long)4 * (dff > d ? dff : d) * 2 + (long long)L * 144 > 72 * 1024) return PGB_ERR_TOO_LARGE;   // shared memory
-    if (work_bytes < pgb_decode_token_work_bytes(B, d, NP, dff)) return PGB_ERR_BAD_SHAPE;
+    if (B > 4) return PGB_ERR_TOO_LARGE;
     if (!aligned(layer_table, 8) || !aligned(E, 16) || !aligned(P, 16) || !aligned(final_norm_weight, 16) ||
         (final_norm_bias && !aligned(final_norm_bias, 16)) || !aligned(tok, 8) || !aligned(pos, 8) || !aligned(work, 16) ||
         !aligned(logits, 4) || !aligned(sync, 16))
         return PGB_ERR_MISALIGNED;
+    return PGB_OK;
+}
+
+int pgb_decode_token_step_fwd(const void *layer_table, int L, const void *E, const void *P, const void *final_norm_weight,
+                         const void *final_norm_bias, int final_norm_kind, float final_norm_eps, const long long *tok,
+                         long long *pos, float *shift, int window, void *work, long long work_bytes, float *logits,
+                         unsigned long long *sync, int B, int d, int H, int D, int NP, int dff, int V, int ctx, int delta,
+                         void *stream) {
+    const int rc = decode_token_check(layer_table, L, E, P, final_norm_weight, final_norm_bias, final_norm_kind, tok, pos, shift, window, work, logits, sync,
+                                      B, d, H, D, NP, dff, V, ctx);
+    if (rc != PGB_OK && rc != PGB_ERR_MISALIGNED) return rc;
+    if ((long long)4 * (dff > d ? dff : d) * 2 + (long long)L * 144 > 72 * 1024) return PGB_ERR_TOO_LARGE;   // shared memory
+    if (work_bytes < pgb_decode_token_work_bytes(B, d, NP, dff)) return PGB_ERR_BAD_SHAPE;
+    if (rc != PGB_OK) return rc;
     return decode_token_launch(layer_table, L, E, P, final_norm_weight, final_norm_bias, final_norm_kind, final_norm_eps, tok, pos,
                                shift, work, logits, sync, B, d, H, D, NP, dff, V, ctx, delta ? 1 : 0, window,
                                (cudaStream_t)stream);
+}
+
+long long pgb_decode_flow_work_bytes(int L, int B, int d, int NP, int dff) {
+    if (L < 1 || B < 1 || B > 4 || d < 1 || NP < 1 || dff < 1) return 0;
+    return (long long)decode_flow_work_bytes(L, B, d, NP, dff);
+}
+
+int pgb_decode_flow_step_fwd(const void *layer_table, int L, const void *E, const void *P, const void *final_norm_weight,
+                             const void *final_norm_bias, int final_norm_kind, float final_norm_eps, const long long *tok,
+                             long long *pos, float *shift, int window, void *work, long long work_bytes, float *logits,
+                             unsigned long long *sync, int B, int d, int H, int D, int NP, int dff, int V, int ctx, int delta,
+                             void *stream) {
+    const int rc = decode_token_check(layer_table, L, E, P, final_norm_weight, final_norm_bias, final_norm_kind, tok, pos, shift, window, work, logits, sync,
+                                      B, d, H, D, NP, dff, V, ctx);
+    if (rc != PGB_OK) return rc;
+    const long long need = pgb_decode_flow_work_bytes(L, B, d, NP, dff);
+    if (need == 0) return PGB_ERR_TOO_LARGE;
+    if (work_bytes < need) return PGB_ERR_BAD_SHAPE;
+    return decode_flow_launch(layer_table, L, E, P, final_norm_weight, final_norm_bias, final_norm_kind, final_norm_eps, tok, pos,
+                              shift, work, logits, sync, B, d, H, D, NP, dff, V, ctx, delta ? 1 : 0, window,
+                              (cudaStream_t)stream);
 }
 
 int pgb_decode_token_fwd(const void *layer_table, int L, const void *E, const void *P, const void *final_norm_weight,
@@ -752,6 +790,8 @@ int pgb_tc_error_flag(int *out_host) {
     if (rc == PGB_OK) rc = tc_train_error_flag(&g);
     f = f > g ? f : g;
     if (rc == PGB_OK) rc = tc_segment_error_flag(&g);
+    f = f > g ? f : g;
+    if (rc == PGB_OK) rc = decode_flow_error_flag(&g);
     f = f > g ? f : g;
     e = e > f ? e : f;
     b = b > c ? b : c;

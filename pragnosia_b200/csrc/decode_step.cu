@@ -19,7 +19,9 @@ __global__ void __launch_bounds__(DEC_THREADS) decode_step_kernel(DecodeArgs a) 
     // kernel behind (the output projection) may start requesting its weights now.
     pdl_wait();
     pdl_launch_dependents();
-    decode_step_body<TIN, TOUT, D, DELTA>(a, blockIdx.x / a.H, blockIdx.x % a.H, [] { return true; });
+    auto ready = [] { return true; };
+    const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
+    decode_step_body<D, DELTA>(a, b, h, DecodeRows<TIN, TOUT, D, decltype(ready)>{a, b, h, ready});
 }
 
 // ---- head dim 64, one WARP per (sequence, head)

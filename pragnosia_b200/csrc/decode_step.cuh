@@ -8,76 +8,108 @@ namespace pgb {
 constexpr int DEC_THREADS = 256;
 
 
-// One (sequence, head) by the calling CTA of DEC_THREADS threads; every thread of the CTA must call it (it synchronises).
-// between(): called by every thread once the loads of the state slice are in flight and before anything of this token's
-// projection is read -- the place for a wait on whoever produces the projection. False from it (the same for the whole
-// CTA) abandons the step with nothing written.
-template <typename TIN, typename TOUT, int D, bool DELTA, typename Between>
-__device__ __forceinline__ void decode_step_body(const DecodeArgs &a, int b, int h, Between &&between) {
-    constexpr int NCG = D / 4;                    // column groups (4 value columns each)
-    constexpr int NRG = DEC_THREADS / NCG;        // row groups
-    constexpr int NPAIR = (D / 2) / NRG;          // row pairs per thread
+// Where a step's projection comes from and its read goes to: rows in memory. between(): called by every thread once the loads of the
+// state slice are in flight and before anything of this token's projection is read -- the place for a wait on whoever produces
+// the projection. False from it, or from the check that follows the reads (the same for the whole CTA), abandons the step with
+// nothing written.
+template <typename TIN, typename TOUT, int D, typename Between>
+struct DecodeRows {
+    const DecodeArgs &a;
+    int b, h;
+    Between between;
+    // elements lane + 32 i of the head's row: 0 q, 1 k, 2 v
+    __device__ __forceinline__ void vec(int which, int lane, float (&x)[D / 32]) const {
+        const TIN *src = (const TIN *)(which == 0 ? a.qp : (which == 1 ? a.kp : a.vp)) + (size_t)b * a.in_sb + (size_t)h * D;
+#pragma unroll
+        for (int i = 0; i < D / 32; ++i) x[i] = to_f32(src[lane + 32 * i]);
+    }
+    __device__ __forceinline__ void scalars(float &d, float &g) const {
+        // both loads before either is used
+        const TIN *dp = (const TIN *)a.decay + (size_t)b * a.decay_sb + h, *gp = a.gate != nullptr ? (const TIN *)a.gate + (size_t)b * a.gate_sb + h : dp;
+        const TIN draw = *dp, graw = *gp;
+        d = to_f32(draw); g = to_f32(graw);
+    }
+    __device__ __forceinline__ bool sync() const { __syncthreads(); return true; }
+    __device__ __forceinline__ void put(int j, float o) const { from_f32(((TOUT *)a.o + (size_t)b * a.out_sb + (size_t)h * D)[j], o); }
+};
+
+// What a thread holds of a step that the projection has no part in: four value columns of its row pairs of the state, and constants
+// of the head. request() loads (the long latency: everything else overlaps with it), constants() evaluates what needs evaluating.
+template <int D>
+struct DecodeHeld {
+    static constexpr int NCG = D / 4;                                // column groups (4 value columns each)
+    static constexpr int NRG = DEC_THREADS / NCG;                    // row groups
+    static constexpr int NPAIR = (D / 2) / NRG;                      // row pairs per thread
+    float4 s0[NPAIR], s1[NPAIR];
+    float rcs[NPAIR], rsn[NPAIR];                                    // rebase rotation of this thread's row pairs (rcs: the frequency, until evaluated)
+    float shift, onw, expA;
+    __device__ __forceinline__ void request(const DecodeArgs &a, int b, int h) {
+        const int tid = threadIdx.x, rg = tid / NCG, col = (tid % NCG) * 4;
+        const float *Sin = a.S_in + (size_t)(b * a.H + h) * D * D;
+#pragma unroll
+        for (int p = 0; p < NPAIR; ++p) {
+            const int pr = rg + p * NRG;                             // pair index: rows 2pr, 2pr+1
+            s0[p] = __ldcs(reinterpret_cast<const float4 *>(Sin + (size_t)(2 * pr) * D + col));
+            s1[p] = __ldcs(reinterpret_cast<const float4 *>(Sin + (size_t)(2 * pr + 1) * D + col));
+        }
+        shift = a.shift_dev != nullptr ? *a.shift_dev : a.shift_host;
+#pragma unroll
+        for (int p = 0; p < NPAIR; ++p) rcs[p] = a.theta != nullptr ? a.theta[(size_t)h * (D / 2) + rg + p * NRG] : 0.f;
+        // the constants of the head as well: a load behind the wait costs a round trip of its own on the path of the step
+        onw = a.rms_w != nullptr && tid < D ? a.rms_w[tid] : 1.f;
+        expA = tid >> 5 == 3 && a.decay_A != nullptr ? a.decay_A[h] : 0.f;
+    }
+    __device__ __forceinline__ void constants() {
+#pragma unroll
+        for (int p = 0; p < NPAIR; ++p) {
+            const float theta = rcs[p];
+            rcs[p] = 1.f; rsn[p] = 0.f;
+            if (shift != 0.f) sincosf(-shift * theta, &rsn[p], &rcs[p]);
+        }
+        if (threadIdx.x >> 5 == 3) expA = expf(expA);
+    }
+};
+
+// One (sequence, head) by the calling CTA of DEC_THREADS threads; every thread of the CTA must call it (it synchronises). held: requested
+// and evaluated for this pair.
+template <int D, bool DELTA, typename IO>
+__device__ __forceinline__ void decode_step_body(const DecodeArgs &a, int b, int h, DecodeHeld<D> &held, const IO &io) {
+    constexpr int NCG = DecodeHeld<D>::NCG, NRG = DecodeHeld<D>::NRG, NPAIR = DecodeHeld<D>::NPAIR;
     __shared__ __align__(16) float sq[D], sk[D], sv[D];             // read and written four floats at a time
     __shared__ __align__(16) float part[NRG][D];
     __shared__ float red[8];
     __shared__ float sc[4];                        // alpha, gate/beta, inv-rms
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int bhx = b * a.H + h;
-    const TIN *qp = (const TIN *)a.qp + (size_t)b * a.in_sb + (size_t)h * D;
-    const TIN *kp = (const TIN *)a.kp + (size_t)b * a.in_sb + (size_t)h * D;
-    const TIN *vp = (const TIN *)a.vp + (size_t)b * a.in_sb + (size_t)h * D;
-
-    // ---- the state slice first: its loads are the long latency, everything below overlaps with them
-    const int cg = tid % NCG, rg = tid / NCG;
-    const int col = cg * 4;
-    const float *Sin = a.S_in + (size_t)bhx * D * D;
-    float *Sout = a.S_out + (size_t)bhx * D * D;
-    float4 s0[NPAIR], s1[NPAIR];
-#pragma unroll
-    for (int p = 0; p < NPAIR; ++p) {
-        const int pr = rg + p * NRG;                                 // pair index: rows 2pr, 2pr+1
-        s0[p] = __ldcs(reinterpret_cast<const float4 *>(Sin + (size_t)(2 * pr) * D + col));
-        s1[p] = __ldcs(reinterpret_cast<const float4 *>(Sin + (size_t)(2 * pr + 1) * D + col));
-    }
-    const float shift = a.shift_dev != nullptr ? *a.shift_dev : a.shift_host;
-    float rcs[NPAIR], rsn[NPAIR];                                    // rebase rotation of this thread's row pairs
-#pragma unroll
-    for (int p = 0; p < NPAIR; ++p) {
-        rcs[p] = 1.f; rsn[p] = 0.f;
-        if (shift != 0.f) sincosf(-shift * a.theta[(size_t)h * (D / 2) + rg + p * NRG], &rsn[p], &rcs[p]);
-    }
-
-    // the constants of the head as well: a load behind the wait costs a round trip of its own on the path of the step
-    const float onw = a.rms_w != nullptr && tid < D ? a.rms_w[tid] : 1.f;
+    const int cg = tid % NCG, rg = tid / NCG, col = cg * 4;
+    float *Sout = a.S_out + (size_t)(b * a.H + h) * D * D;
+    float4 (&s0)[NPAIR] = held.s0, (&s1)[NPAIR] = held.s1;
+    const float (&rcs)[NPAIR] = held.rcs, (&rsn)[NPAIR] = held.rsn;
+    const float onw = held.onw, expA = held.expA;
     const bool raw_decay = a.decay_A != nullptr;
-    const float expA = warp == 3 && raw_decay ? expf(a.decay_A[h]) : 1.f;
-
-    if (!between()) return;
+    if (!io.between()) return;
 
     // ---- vectors: load, normalise (warps 0,1,2 take q,k,v), scalars (warp 3)
     if (warp < 3) {
-        const TIN *src = warp == 0 ? qp : (warp == 1 ? kp : vp);
         float *dst = warp == 0 ? sq : (warp == 1 ? sk : sv);
         float x[D / 32]; float ss = 0.f;
+        io.vec(warp, lane, x);
 #pragma unroll
-        for (int i = 0; i < D / 32; ++i) { x[i] = to_f32(src[lane + 32 * i]); ss += x[i] * x[i]; }
+        for (int i = 0; i < D / 32; ++i) ss += x[i] * x[i];
         float inv = 1.f;
         if (a.normalize) { ss = warp_sum(ss); inv = 1.0f / fmaxf(sqrtf(ss), 1e-12f); }
 #pragma unroll
         for (int i = 0; i < D / 32; ++i) dst[lane + 32 * i] = x[i] * inv;
     } else if (warp == 3 && lane == 0) {
-        // both loads before either is used
-        const TIN *dp = (const TIN *)a.decay + (size_t)b * a.decay_sb + h, *gp = a.gate != nullptr ? (const TIN *)a.gate + (size_t)b * a.gate_sb + h : dp;
-        const TIN draw = *dp, graw = *gp;
-        float d = to_f32(draw), g = to_f32(graw);
+        float d, g;
+        io.scalars(d, g);
         if (raw_decay) d = -softplusf_(d) * expA;
         sc[0] = expf(d);
         if (a.gate == nullptr) g = 1.f;
         else if (a.gate_is_logit) g = sigmoidf_(g);
         sc[1] = g;
     }
-    __syncthreads();
+    if (!io.sync()) return;
     const float alpha = sc[0];
     const float g = sc[1];
     // plain rule: the write gate scales k.  delta rule: g is beta.
@@ -159,11 +191,14 @@ __device__ __forceinline__ void decode_step_body(const DecodeArgs &a, int b, int
         __syncthreads();
         if (tid < D) oj = oj * sc[2] * onw;
     }
-    if (tid < D) {
-        TOUT *o = (TOUT *)a.o + (size_t)b * a.out_sb + (size_t)h * D;
-        from_f32(o[tid], oj);
-    }
+    if (tid < D) io.put(tid, oj);
 }
-
+template <int D, bool DELTA, typename IO>
+__device__ __forceinline__ void decode_step_body(const DecodeArgs &a, int b, int h, const IO &io) {
+    DecodeHeld<D> held;
+    held.request(a, b, h);
+    held.constants();
+    decode_step_body<D, DELTA>(a, b, h, held, io);
+}
 
 }  // namespace pgb

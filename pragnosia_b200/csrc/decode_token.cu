@@ -26,27 +26,11 @@
 // The barrier is one 64-bit arrival counter in global memory that only ever grows (nothing to reset between launches;
 // the second word of the pair is reserved). Its wait is bounded: a CTA that gives up raises a flag every other waiter
 // also watches, so the kernel winds down within about a second instead of hanging, and the host reads the flag.
-#include "decode_step.cuh"
+#include "decode_token.cuh"
 
 namespace pgb {
 
-constexpr int DT_THREADS = DEC_THREADS;                               // 256: what decode_step_body is written for
-constexpr int DT_WARPS = DT_THREADS / 32;
-constexpr unsigned DT_SPIN_LIMIT = 1u << 20;                          // polls of about a microsecond each
-
 static __device__ int g_dt_error = 0;
-
-// One layer's pointers and norm settings; the host lays the table out as 18 64-bit words per layer.
-struct DtLayer {
-    const __nv_bfloat16 *Wc, *bc, *ln_w, *ln_b, *ow, *n_w, *n_b, *a_w, *a_b, *b_w, *b_b;
-    const float *theta, *A, *on_w;
-    float *S;
-    int ln_kind, n_kind;
-    float ln_eps, n_eps;
-    float on_eps;                                                     // of the per-head RMS norm on the read
-    int pad;
-};
-static_assert(sizeof(DtLayer) == 18 * 8, "the host writes 18 words per layer");
 
 struct DtArgs {
     const DtLayer *layers;
@@ -60,20 +44,6 @@ struct DtArgs {
     int window;                                                       // > 0: leave pos and shift as the next token needs them
     float fn_eps;
 };
-
-__device__ __forceinline__ void dt_unpack8(const uint4 &raw, float (&f)[8]) {
-    const __nv_bfloat162 *b = reinterpret_cast<const __nv_bfloat162 *>(&raw);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { const float2 t = __bfloat1622float2(b[i]); f[2 * i] = t.x; f[2 * i + 1] = t.y; }
-}
-__device__ __forceinline__ uint4 dt_pack8(const float (&f)[8]) {
-    uint4 raw;
-    __nv_bfloat162 *b = reinterpret_cast<__nv_bfloat162 *>(&raw);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) b[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-    return raw;
-}
-__device__ __forceinline__ float dt_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // Grid-wide barrier number gen + 1 (every CTA passes the same barriers in the same order), in two halves so that work which
 // does not depend on the other CTAs can sit between them. Arrive: one fire-and-forget add to the arrival counter once the
@@ -247,18 +217,6 @@ __device__ __noinline__ void dt_build_rows(const DtArgs &a, const DtRows &rw, ui
     __syncthreads();
 }
 
-__device__ __forceinline__ void dt_cp_async16(void *smem_dst, const void *gmem_src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void dt_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void dt_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
-
-constexpr int DT_PIECES = 12;                                         // 128-bit pieces of weights a lane has in flight per item
-constexpr int DT_DEPTH = 3;                                           // items a warp has in flight or in use
-constexpr int DT_STAGE_U4 = DT_DEPTH * DT_PIECES * 32;                // a warp's staging buffers, in uint4
-
 // One linear phase: out[b][n] = act(sum_k W[n][k] z[b][k] + bias[n]) with z the rows rw describes.
 //
 // Output rows go in groups of R consecutive rows, groups dealt round-robin to the grid's warps; a warp's work is a list of
@@ -427,10 +385,12 @@ __global__ void __launch_bounds__(DT_THREADS, 1) decode_token_kernel(DtArgs a) {
             bool waited = false, alive = true;
             dt_arrive(a.sync);
             for (int bh = blockIdx.x; bh < a.B * a.H && alive; bh += gridDim.x) {
-                decode_step_body<__nv_bfloat16, __nv_bfloat16, D, DELTA>(da, bh / a.H, bh % a.H, [&]() {
+                auto ready = [&]() {
                     if (!waited) { waited = true; alive = dt_wait(a.sync, gen); }
                     return alive;
-                });
+                };
+                const int b = bh / a.H, h = bh % a.H;
+                decode_step_body<D, DELTA>(da, b, h, DecodeRows<__nv_bfloat16, __nv_bfloat16, D, decltype(ready)>{da, b, h, ready});
                 __syncthreads();
             }
             if (!waited) alive = dt_wait(a.sync, gen);

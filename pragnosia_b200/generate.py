@@ -56,8 +56,7 @@ class Decoder:
                 self.states = [(S, n) for S in new]
             else:
                 torch._foreach_copy_([st[0] for st in self.states], new)
-            if self._plan is not None:
-                self._plan["sync"].zero_()
+            self._reset_barrier()
             self.pos.fill_(n % w)
             self.shift.fill_(float(n))
             return F.linear(z, m.e.weight)[:, -1].float()
@@ -76,11 +75,16 @@ class Decoder:
             for old, cur in zip(self.states, new):
                 for a, b in zip(old, cur):
                     if torch.is_tensor(a): a.copy_(b)
-        if self._plan is not None:
-            self._plan["sync"].zero_()                       # a fresh pair of barrier counters (a step that gave up leaves them uneven)
+        self._reset_barrier()
         self.pos.fill_(pw)
         self.shift.fill_(float(n))                           # the last window's length (src/assoc.py:512 returns p0 + T)
         return F.linear(h[:, -1:], m.e.weight)[:, -1].float()
+
+    def _reset_barrier(self):
+        """A fresh pair of barrier counters: a step that gave up leaves them uneven. (The step without barriers counts its launches
+        there, whatever became of them.)"""
+        if self._plan is not None and not self._plan["flow"]:
+            self._plan["sync"].zero_()
 
     # ---- one token
     def _fused_ok(self):
@@ -128,8 +132,12 @@ class Decoder:
             i32[i, 30], i32[i, 31] = k1, k2
             f32[i, 32], f32[i, 33], f32[i, 34] = e1, e2, mx._rms_eps()
         mx0, NP, dff = m.mix[0], m.mix[0]._consts()["W"].shape[0], m.mlp[0].a.weight.shape[0]
-        work = torch.empty(ops.decode_token_work_bytes(self.B, m.d, NP, dff) // 2, dtype=torch.bfloat16, device=self.dev)
-        self._plan = dict(key=key, keep=keep, table=torch.from_numpy(rows).to(self.dev), work=work, NP=NP, dff=dff,
+        flow = ops.decode_flow_work_bytes(m.layers, self.B, m.d, NP, dff)    # 0: shapes too wide for it, the step with barriers
+        if flow:
+            work = torch.zeros(flow // 4, dtype=torch.int32, device=self.dev)
+        else:
+            work = torch.empty(ops.decode_token_work_bytes(self.B, m.d, NP, dff) // 2, dtype=torch.bfloat16, device=self.dev)
+        self._plan = dict(key=key, keep=keep, table=torch.from_numpy(rows).to(self.dev), work=work, flow=flow > 0, NP=NP, dff=dff,
                           sync=torch.zeros(2, dtype=torch.int64, device=self.dev), H=mx0.h, D=mx0.dk, delta=bool(mx0.delta),
                           logits=torch.empty(self.B, m.e.weight.shape[0], dtype=torch.float32, device=self.dev))
         return self._plan
@@ -156,7 +164,7 @@ class Decoder:
         m, p = self.m, self._token_plan()
         lg = ops.decode_token(p["table"], m.e.weight, m.p.weight, m.n, self.tok, self.pos, self.shift, p["work"],
                               p["logits"] if out is None else out, p["sync"], p["H"], p["D"], p["NP"], p["dff"], p["delta"],
-                              window=self.w if advance else 0)
+                              window=self.w if advance else 0, flow=p["flow"])
         return lg
 
     @property

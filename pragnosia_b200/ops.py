@@ -498,12 +498,13 @@ def decode_advance(pos, shift, window: int):
 
 
 @on_device_of
-def decode_token(table, E, P, final_norm, tok, pos, shift, work, logits, sync, H, D, NP, dff, delta: bool, window: int = 0):
+def decode_token(table, E, P, final_norm, tok, pos, shift, work, logits, sync, H, D, NP, dff, delta: bool, window: int = 0, flow: bool = False):
     """One decode step of the whole model in ONE cooperative launch (decode_token.cu): embedding, every layer, final norm
     and tied head for 1..4 sequences. table (L,18) int64 on the device: the per-layer pointers and norm settings the C
     header documents (generate.Decoder builds it); work / sync: scratch from decode_token_work_bytes and two zeroed
     64-bit words; logits (B,V) fp32 out. The states the table points at are updated in place; window > 0: pos
-    and shift as well, as the next token needs them ((pos + 1) mod window, 1)."""
+    and shift as well, as the next token needs them ((pos + 1) mod window, 1). flow: the step without barriers (decode_flow.cu); work
+    then holds decode_flow_work_bytes, zeroed together with sync before the first call and the call's own from then on."""
     need_cuda(table, E, P, tok, pos, shift, work, logits, sync)
     if E.dtype != torch.bfloat16 or P.dtype != torch.bfloat16 or tok.dtype != torch.long or pos.dtype != torch.long:
         raise ValueError("decode_token: bf16 tables, int64 ids")
@@ -515,15 +516,19 @@ def decode_token(table, E, P, final_norm, tok, pos, shift, work, logits, sync, H
     if nw.dtype != torch.bfloat16 or (nb is not None and nb.dtype != torch.bfloat16):
         raise ValueError("decode_token: bf16 norm parameters")
     B, V, d = logits.shape[0], E.shape[0], E.shape[1]
-    check(lib().pgb_decode_token_step_fwd(ptr(table), table.shape[0], ptr(E), ptr(P), ptr(nw), ptr(nb), kind, float(eps), ptr(tok),
-                                          ptr(pos), ptr(shift), window, ptr(work), work.numel() * work.element_size(), ptr(logits),
-                                          ptr(sync), B, d, H, D, NP, dff, V, P.shape[0], 1 if delta else 0, stream_of(E)),
-          "pgb_decode_token_step_fwd")
+    name = "pgb_decode_flow_step_fwd" if flow else "pgb_decode_token_step_fwd"
+    check(getattr(lib(), name)(ptr(table), table.shape[0], ptr(E), ptr(P), ptr(nw), ptr(nb), kind, float(eps), ptr(tok),
+                               ptr(pos), ptr(shift), window, ptr(work), work.numel() * work.element_size(), ptr(logits),
+                               ptr(sync), B, d, H, D, NP, dff, V, P.shape[0], 1 if delta else 0, stream_of(E)), name)
     return logits
 
 
 def decode_token_work_bytes(B: int, d: int, NP: int, dff: int) -> int:
     return int(lib().pgb_decode_token_work_bytes(B, d, NP, dff))
+
+
+def decode_flow_work_bytes(L: int, B: int, d: int, NP: int, dff: int) -> int:
+    return int(lib().pgb_decode_flow_work_bytes(L, B, d, NP, dff))
 
 
 @on_device_of

@@ -75,6 +75,41 @@ def test_changed_weights_retire_the_table():
     assert not torch.equal(lg0, lg1)
 
 
+@pytest.mark.parametrize("d,mixer,mult,vocab,norm", [
+    (64, "aspin", 1, 40, "rms"),                                       # fewer rows than CTAs
+    (192, "dspin", 12, 300, "ln"),                                     # MLP down with its rows shared across the warps (K 2304)
+    (256, "hspin", 9, 9600, "ln"),                                     # the same on a multiple of eight warps only; a head of several rounds
+    (1280, "hdspin", 4, 5000, "rms"),                                  # phases of several rounds, rows too long for four a warp
+])
+@pytest.mark.parametrize("B", [1, 3])
+def test_step_without_barriers_matches_the_one_with(d, mixer, mult, vocab, norm, B, monkeypatch):
+    """Same roundings, and but for rows shared across warps (fp32 sums in another order: a bf16 rounding may fall the other way, 2^-8) the
+    same order of every sum."""
+    from pragnosia_b200 import ops
+    from pragnosia_b200.model import LM
+    torch.manual_seed(d)
+    m = LM(vocab=vocab, d=d, layers=3, mlp_mult=mult, ctx=16, mixer=mixer, norm=norm).to(DEV).bfloat16().eval()
+    ids = synth.token_ids(B, 40, vocab, seed=d).to(DEV)
+    outs = []
+    for flow in (True, False):
+        if not flow:
+            monkeypatch.setattr(ops, "decode_flow_work_bytes", lambda *a: 0)
+        dec = Decoder(m, batch=B)
+        lg = [dec.prefill(ids[:, :20])]
+        for t in range(20, 30):                                       # crosses the window's edge (ctx 16)
+            lg.append(dec.step(ids[:, t]).clone())
+        lg.append(dec.prefill(ids[:, :17]))                           # a new prompt on the same decoder: the words keep their marks
+        lg.append(dec.step(ids[:, 17]).clone())
+        assert dec._plan["flow"] == flow
+        outs.append((torch.stack(lg, 1), [st[0].clone() for st in dec.states]))
+    close(outs[0][0], outs[1][0], 2e-2, "logits")
+    for a, b in zip(outs[0][1], outs[1][1]):
+        close(a, b, 5e-3, "state")
+    if mult * d < 2048 or d > 1000:
+        assert (outs[0][0] == outs[1][0]).float().mean().item() > 0.9
+    assert healthy() == 0
+
+
 def test_a_barrier_wait_that_runs_out_raises_the_flag_and_returns():
     """The grid barrier's failure path without a fault: one CTA waits, with a short limit, for arrivals that never come."""
     import ctypes
