@@ -153,7 +153,7 @@ def test_new_entry_points_reject_bad_calls(L):
     assert L.pgb_decode_flow_work_bytes(12, 5, 768, 2328, 3072) == 0 and L.pgb_decode_flow_work_bytes(0, 1, 768, 2328, 3072) == 0
     flow = lambda **kw: L.pgb_decode_flow_step_fwd(one, 12, one, one, one, kw.get("nb", one), 2, 1e-5, one, one, one, 512, kw.get("work", one),
                                                    kw.get("wb", 10 ** 6), one, one, kw.get("B", 1), 768, 12, kw.get("D", 64), 2328, 3072, 50257, 512, 0, None)
-    assert flow(nb=None) == 1 and flow(wb=10) == 2 and flow(B=5) == 7 and flow(D=96) == 3 and flow(work=ctypes.c_void_p(0x1008)) == 5
+    assert flow(nb=None) == 1 and flow(wb=10) == 2 and flow(B=5) == 7 and flow(D=96) == 3 and flow(work=ctypes.c_void_p(0x1008)) == 4
 
 
 def test_segments_and_windows_refuse_an_in_place_state(L):
