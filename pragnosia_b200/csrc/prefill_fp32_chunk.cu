@@ -6,9 +6,11 @@
 //   2. fp32_states_kernel  elementwise over the chunks, in place of U:           S_c, and the final state
 //   3. fp32_out_kernel     a CTA per (chain, chunk, 64 value columns):           o = ((Q K^T) dec) V + e^L (Q S_c)
 // Every product is 64 x 64 outputs by 256 threads, a 4 x 4 tile each, with both operands contraction-major in shared memory
-// (two 16-byte loads per 16 multiply-adds), which puts the FFMA pipe ahead of shared memory. Same masking as the walk: rows
-// past T are zero tokens with log-decay 0. B2 H12 T512 D64: 131 us as a walk -> 27 us (states 6.5,
-// prefix 3.2, outputs 17.4).
+// (two 16-byte loads per 16 multiply-adds). Same masking as the walk: rows
+// past T are zero tokens with log-decay 0. The three are programmatic dependents of one another: the output kernel's scores need no state, so its
+// CTAs load and multiply while the two before it run. What bounds the output kernel is instruction issue and the latency of 8 to 24 warps an SM
+// (17 us at B2 H12 T512 D64); 8 x 8 outputs a thread (fewer loads, half the warps) and halves of a chunk per CTA took the same or longer.
+// B2 H12 T512 D64: 131 us as a walk, 26 behind one another, 21 so; a call of one chunk 15 -> 11.
 #include "common.cuh"
 
 namespace pgb {
@@ -28,27 +30,39 @@ __device__ __forceinline__ void pc_product(float (&acc)[4][4], const float *A, c
             for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
     }
 }
+// Operands travel in two steps, all of a thread's loads first and its stores to shared memory behind them (the compiler moves no load across
+// such a store, so written as one step every piece waits for the one before it).
 // rows t0.. of a (T x D) matrix, columns c0..c0+63, as they lie: dst[row][col]
-__device__ __forceinline__ void pc_rows(float *dst, const float *src, int t0, int T, int D, int c0, int tid, const float *scale) {
+__device__ __forceinline__ void pc_load(float4 (&x)[4], const float *src, int t0, int T, int D, int c0, int tid) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int idx = tid + PC_NT * i, r = idx >> 4, c = 4 * (idx & 15);
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (t0 + r < T) x = *reinterpret_cast<const float4 *>(src + (size_t)(t0 + r) * D + c0 + c);
-        if (scale != nullptr) { const float w = scale[r]; x.x *= w; x.y *= w; x.z *= w; x.w *= w; }
-        *reinterpret_cast<float4 *>(dst + r * PC_P + c) = x;
+        x[i] = t0 + r < T ? *reinterpret_cast<const float4 *>(src + (size_t)(t0 + r) * D + c0 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+__device__ __forceinline__ void pc_put(float *dst, const float4 (&x)[4], int tid) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int idx = tid + PC_NT * i;
+        *reinterpret_cast<float4 *>(dst + (idx >> 4) * PC_P + 4 * (idx & 15)) = x[i];
     }
 }
 // the same transposed: dst[col][row], D columns. A thread takes one row's four adjacent columns; lanes run over rows, so the
 // four stores of a warp hit consecutive banks
 template <int D>
-__device__ __forceinline__ void pc_cols(float *dst, const float *src, int t0, int T, int tid) {
+__device__ __forceinline__ void pc_cols_load(float4 (&x)[D / 16], const float *src, int t0, int T, int tid) {
 #pragma unroll
     for (int i = 0; i < D / 16; ++i) {
         const int idx = tid + PC_NT * i, r = idx & 63, c = 4 * (idx >> 6);
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (t0 + r < T) x = *reinterpret_cast<const float4 *>(src + (size_t)(t0 + r) * D + c);
-        dst[c * PC_P + r] = x.x; dst[(c + 1) * PC_P + r] = x.y; dst[(c + 2) * PC_P + r] = x.z; dst[(c + 3) * PC_P + r] = x.w;
+        x[i] = t0 + r < T ? *reinterpret_cast<const float4 *>(src + (size_t)(t0 + r) * D + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+template <int D>
+__device__ __forceinline__ void pc_cols_put(float *dst, const float4 (&x)[D / 16], int tid) {
+#pragma unroll
+    for (int i = 0; i < D / 16; ++i) {
+        const int idx = tid + PC_NT * i, r = idx & 63, c = 4 * (idx >> 6);
+        dst[c * PC_P + r] = x[i].x; dst[(c + 1) * PC_P + r] = x[i].y; dst[(c + 2) * PC_P + r] = x[i].z; dst[(c + 3) * PC_P + r] = x[i].w;
     }
 }
 // L (inclusive cumulative log-decay of the chunk) by warp 0, two tokens a lane; returns nothing, the caller synchronises
@@ -75,13 +89,22 @@ __global__ void __launch_bounds__(PC_NT) fp32_outer_kernel(PcParams p) {
     __shared__ __align__(16) float Ks[PC_C * PC_P], Vs[PC_C * PC_P], L[64], w[64];
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15, c = blockIdx.x, bh = blockIdx.y, t0 = c * PC_C, T = p.T;
     const int i0 = 64 * (blockIdx.z % (D / 64)), j0 = 64 * (blockIdx.z / (D / 64));
-    if (tid < 32) pc_decay(p.la + (size_t)bh * T, t0, T, tid, L);
-    pc_rows(Vs, p.v + (size_t)bh * T * D, t0, T, D, j0, tid, nullptr);
+    float4 kx[4], vx[4];
+    pc_load(kx, p.k + (size_t)bh * T * D, t0, T, D, i0, tid);
+    pc_load(vx, p.v + (size_t)bh * T * D, t0, T, D, j0, tid);
+    pdl_launch_dependents();
+    if (tid < 32) {
+        pc_decay(p.la + (size_t)bh * T, t0, T, tid, L);
+        __syncwarp();
+        const float end = L[63];
+        w[tid] = expf(fminf(end - L[tid], 0.f)); w[tid + 32] = expf(fminf(end - L[tid + 32], 0.f));
+        if (tid == 0 && blockIdx.z == 0) p.Ltot[(size_t)bh * p.NC + c] = end;
+    }
+    pc_put(Vs, vx, tid);
     __syncthreads();
-    if (tid < 64) w[tid] = expf(fminf(L[63] - L[tid], 0.f));
-    if (tid == 0 && blockIdx.z == 0) p.Ltot[(size_t)bh * p.NC + c] = L[63];
-    __syncthreads();
-    pc_rows(Ks, p.k + (size_t)bh * T * D, t0, T, D, i0, tid, w);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const float f = w[(tid + PC_NT * i) >> 4]; kx[i].x *= f; kx[i].y *= f; kx[i].z *= f; kx[i].w *= f; }
+    pc_put(Ks, kx, tid);
     __syncthreads();
     float acc[4][4] = {};
     pc_product<PC_C>(acc, Ks, Vs, ty, tx);
@@ -95,6 +118,7 @@ __global__ void __launch_bounds__(256) fp32_states_kernel(float *__restrict__ U,
                                                           const float *__restrict__ theta, const float *__restrict__ shift_dev, float shift_host,
                                                           __nv_bfloat16 *__restrict__ sent, float *__restrict__ S_out, int NC, int H, int D) {
     const int e = blockIdx.x * 256 + threadIdx.x, bh = blockIdx.y, i = e / (D / 2), j = 2 * (e % (D / 2));
+    pdl_launch_dependents();
     const size_t DD = (size_t)D * D, at = (size_t)(2 * i) * D + j;
     float2 a = make_float2(0.f, 0.f), b = a;
     if (S0 != nullptr) {
@@ -108,6 +132,7 @@ __global__ void __launch_bounds__(256) fp32_states_kernel(float *__restrict__ U,
             a = ra; b = rb;
         }
     }
+    pdl_wait();                                                       // U and the chunks' decays
     for (int c0 = 0; c0 < NC; c0 += 8) {                              // eight chunks' additions requested ahead of the recurrence
         float2 ua[8], ub[8];
         float d[8];
@@ -150,29 +175,36 @@ __global__ void __launch_bounds__(PC_NT) fp32_out_kernel(PcParams p) {
     float *Qt = pc_smem + SM::off_q, *Kt = pc_smem + SM::off_k, *At = pc_smem + SM::off_a, *Vs = pc_smem + SM::off_v, *L = pc_smem + SM::off_l;
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15, c = blockIdx.x, bh = blockIdx.y, j0 = 64 * blockIdx.z, t0 = c * PC_C, T = p.T;
     const size_t base = (size_t)bh * T * D;
-    pc_cols<D>(Qt, p.q + base, t0, T, tid);
-    pc_cols<D>(Kt, p.k + base, t0, T, tid);
-    pc_rows(Vs, p.v + base, t0, T, D, j0, tid, nullptr);
-    if (tid < 32) pc_decay(p.la + (size_t)bh * T, t0, T, tid, L);
+    {
+        float4 qx[D / 16], kx[D / 16], vx[4];
+        pc_cols_load<D>(qx, p.q + base, t0, T, tid);
+        pc_cols_load<D>(kx, p.k + base, t0, T, tid);
+        pc_load(vx, p.v + base, t0, T, D, j0, tid);
+        if (tid < 32) pc_decay(p.la + (size_t)bh * T, t0, T, tid, L);
+        pc_cols_put<D>(Qt, qx, tid);
+        pc_cols_put<D>(Kt, kx, tid);
+        pc_put(Vs, vx, tid);
+    }
     __syncthreads();
     float acc[4][4] = {};
     pc_product<D>(acc, Qt, Kt, ty, tx);
     __syncthreads();                                                  // K is consumed: the state's columns take its place
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {                                     // A = (Q K^T) dec, transposed
+        const int s = 4 * tx + j;
+        float x[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { const int t = 4 * ty + i; x[i] = s <= t ? acc[i][j] * expf(fminf(L[t] - L[s], 0.f)) : 0.f; }
+        *reinterpret_cast<float4 *>(At + s * PC_P + 4 * ty) = make_float4(x[0], x[1], x[2], x[3]);
+    }
+    pdl_wait();                                                       // the entering states
     {
         const float *src = p.U + ((size_t)bh * p.NC + c) * D * D + j0;
+        float4 x[D / 16];
 #pragma unroll
-        for (int i = 0; i < D / 16; ++i) {
-            const int idx = tid + PC_NT * i, r = idx >> 4, cc = 4 * (idx & 15);
-            *reinterpret_cast<float4 *>(Kt + r * PC_P + cc) = *reinterpret_cast<const float4 *>(src + (size_t)r * D + cc);
-        }
+        for (int i = 0; i < D / 16; ++i) { const int idx = tid + PC_NT * i; x[i] = *reinterpret_cast<const float4 *>(src + (size_t)(idx >> 4) * D + 4 * (idx & 15)); }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {                                 // A = (Q K^T) dec, transposed
-            const int s = 4 * tx + j;
-            float x[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { const int t = 4 * ty + i; x[i] = s <= t ? acc[i][j] * expf(fminf(L[t] - L[s], 0.f)) : 0.f; }
-            *reinterpret_cast<float4 *>(At + s * PC_P + 4 * ty) = make_float4(x[0], x[1], x[2], x[3]);
-        }
+        for (int i = 0; i < D / 16; ++i) { const int idx = tid + PC_NT * i; *reinterpret_cast<float4 *>(Kt + (idx >> 4) * PC_P + 4 * (idx & 15)) = x[i]; }
     }
     __syncthreads();
 #pragma unroll
@@ -210,14 +242,19 @@ static int prefill_fp32_chunk_go(const PrefillArgs &a, int o_dtype, float *scrat
     const int BH = a.B * a.H, NC = (a.T + PC_C - 1) / PC_C;
     float *Ltot = scratch + (size_t)BH * NC * D * D;
     const PcParams p{(const float *)a.q, (const float *)a.k, (const float *)a.v, a.la, scratch, Ltot, a.o, o_dtype == PGB_BF16, a.T, NC};
-    const cudaError_t e = cudaFuncSetAttribute(fp32_out_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PcOut<D>::bytes);
+    // Output CTAs that come while the first kernel's are still there go wherever there is room, three to an SM beside SMs with none: where they
+    // all fit one or two to an SM, as many bytes of shared memory as leave room for no more keep them there (192 CTAs on 148 SMs: 30.7 us the call without, 20.7 with).
+    const long long ctas = (long long)BH * NC * (D / 64), sms = sm_count();
+    const size_t least = ctas <= sms ? 116 * 1024 : ctas <= 2 * sms ? 78 * 1024 : 0, out_bytes = PcOut<D>::bytes > least ? PcOut<D>::bytes : least;
+    const cudaError_t e = cudaFuncSetAttribute(fp32_out_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_bytes);
     if (e != cudaSuccess) { set_cuda_error(e, "fp32_out smem attribute"); return PGB_ERR_CUDA; }
     fp32_outer_kernel<D><<<dim3((unsigned)NC, (unsigned)BH, (D / 64) * (D / 64)), PC_NT, 0, st>>>(p);
     int rc = check_launch("fp32_outer_kernel");
     if (rc != PGB_OK) return rc;
-    fp32_states_kernel<<<dim3(D * D / 4 / 256, (unsigned)BH), 256, 0, st>>>(scratch, Ltot, a.S0, a.theta, a.shift_dev, a.shift_host, a.sent, a.S_out, NC, a.H, D);
-    if ((rc = check_launch("fp32_states_kernel")) != PGB_OK) return rc;
-    fp32_out_kernel<D><<<dim3((unsigned)NC, (unsigned)BH, D / 64), PC_NT, PcOut<D>::bytes, st>>>(p);
+    cudaError_t le = pdl_launch(fp32_states_kernel, dim3(D * D / 4 / 256, (unsigned)BH), dim3(256), (size_t)0, st, scratch, (const float *)Ltot, a.S0, a.theta,
+                                a.shift_dev, a.shift_host, a.sent, a.S_out, NC, a.H, D);
+    if (le == cudaSuccess) le = pdl_launch(fp32_out_kernel<D>, dim3((unsigned)NC, (unsigned)BH, D / 64), dim3(PC_NT), out_bytes, st, p);
+    if (le != cudaSuccess) { set_cuda_error(le, "fp32 prefill launch"); return PGB_ERR_CUDA; }
     return check_launch("fp32_out_kernel");
 }
 
