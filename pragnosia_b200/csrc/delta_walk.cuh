@@ -58,8 +58,13 @@ template <int D, bool BWD>
 struct DwSmem {
     static constexpr int QK = TC_C * D * 2, SQ = TC_C * TC_C * 2;
     static constexpr int o_k = 0, o_x = QK, o_q = o_x + 2 * SQ, o_v = o_q + QK;       // K, X head, X tail, then (forward) Q, V
-    static constexpr int STAGE = BWD ? o_q : o_v + QK;
-    static constexpr int NST = D == 128 && !BWD ? 2 : 3;
+    // Backward, dW0 and (at D = 64) D_c of the chunk, fp32, come with its tiles. Loaded by the math warps where they are used, a round trip to
+    // the L2 or two of every chunk were on the chain: B4 H11 T2048 D64 132 -> 93 us, B4 H8 T2048 D128 210 -> 177. At D = 128 D_c does not fit
+    // beside them: its loads run a block of keys ahead.
+    static constexpr bool FETCH_DC = BWD && D == 64;
+    static constexpr int o_dw0 = o_q, o_dc = o_dw0 + TC_C * D * 4;
+    static constexpr int STAGE = FETCH_DC ? o_dc + D * D * 4 : BWD ? o_dc : o_v + QK;
+    static constexpr int NST = D == 128 ? 2 : 3;
     static constexpr int off_a = NST * STAGE;                         // decayed scores, two slots of head and tail (forward)
     static constexpr int off_out = off_a + (BWD ? 0 : 4 * SQ);        // staging of the stores, a slot per warp: math, then output
     static constexpr int MSLOT = (D / 2 > 32 ? D / 2 : 32) * 64, TSLOT = BWD ? 0 : 4096;
@@ -217,12 +222,18 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
                 const uint8_t *vt = sm + st * SM::STAGE + SM::o_v + (v >> 6) * 8192 + (v & 7) * 2;
                 const int vj = (v & 63) >> 3;
                 float d0[32];
+                float d[BWD ? 16 : 1];                                // D_c, a block of keys
+                const float *dc = !BWD ? nullptr : SM::FETCH_DC ? reinterpret_cast<const float *>(sm + st * SM::STAGE + SM::o_dc) + k0 * D + v
+                                                                : p.Dc + (((size_t)bh * NC + c) * D + k0) * D + v;
                 if constexpr (BWD) {
+                    if constexpr (!SM::FETCH_DC) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const int t = t0 + 32 * g + j;
-                        d0[j] = t < T ? p.dW0[((size_t)bh * T + t) * D + v] : 0.f;
+                        for (int k = 0; k < 16; ++k) d[k] = dc[k * D];
                     }
+                    if (!(ok = mbar_wait_warp(full(st), (i / SM::NST) & 1, 12))) break;
+                    const float *dw = reinterpret_cast<const float *>(sm + st * SM::STAGE + SM::o_dw0) + 32 * g * D + v;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) d0[j] = t0 + 32 * g + j < T ? dw[j * D] : 0.f;
                 } else {
                     if (!(ok = mbar_wait_warp(full(st), (i / SM::NST) & 1, 12))) break;
 #pragma unroll
@@ -256,11 +267,14 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
                 if (keep) out.begin();
 #pragma unroll 1
                 for (int b = 0; b < KH; b += 16) {
-                    float x[16], d[BWD ? 16 : 1];
-                    if constexpr (BWD) {
-                        const float *dc = p.Dc + (((size_t)bh * NC + c) * D + k0 + b) * D + v;
+                    float x[16], dn[BWD ? 16 : 1];
+                    if constexpr (SM::FETCH_DC) {
 #pragma unroll
-                        for (int k = 0; k < 16; ++k) d[k] = dc[(size_t)k * D];
+                        for (int k = 0; k < 16; ++k) d[k] = dc[(b + k) * D];
+                    } else if constexpr (BWD) {
+                        const int nb = b + 16 < KH ? b + 16 : b;
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) dn[k] = dc[(nb + k) * D];
                     }
                     tmem_ld16_nowait(lb + TM_S + k0 + b, x);
                     tmem_ld_wait();
@@ -276,6 +290,10 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
 #pragma unroll
                     for (int k = 0; k < 16; ++k) { if constexpr (BWD) x[k] = fmaf(aC, x[k], d[k]); else x[k] *= aC; }
                     tmem_st16(lb + TM_S + k0 + b, reinterpret_cast<const uint32_t (&)[16]>(x));
+                    if constexpr (BWD && !SM::FETCH_DC) {
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) d[k] = dn[k];
+                    }
                 }
                 if (BWD) {
                     out.end(&m.g, 32 * sub, k0, (bh * NC + c) * 2);
@@ -543,7 +561,10 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
             if (i >= SM::NST && !mbar_wait_warp(empty(st), ((i / SM::NST) + 1) & 1, 61)) break;
             if (lane == 0) {
                 const uint32_t sb = base + st * SM::STAGE, bar = full(st);
-                mbar_expect_tx(bar, SM::STAGE);
+                const uint32_t dw0 = BWD ? (uint32_t)(T - t0 < TC_C ? T - t0 : TC_C) * D * 4 : 0, dcb = SM::FETCH_DC ? D * D * 4 : 0;
+                mbar_expect_tx(bar, BWD ? SM::o_dw0 + dw0 + dcb : SM::STAGE);
+                if constexpr (BWD) bulk_load_1d(sb + SM::o_dw0, p.dW0 + ((size_t)bh * T + t0) * D, dw0, bar);
+                if constexpr (SM::FETCH_DC) bulk_load_1d(sb + SM::o_dc, p.Dc + ((size_t)bh * NC + c) * D * D, dcb, bar);
 #pragma unroll
                 for (int s = 0; s < SUB; ++s) tma_load_3d(sb + SM::o_k + s * 8192, &m.k, bar, 64 * s, t0, bh);
                 tma_load_3d(sb + SM::o_x, &m.x, bar, 0, 0, (bh * NC + c) * 2);

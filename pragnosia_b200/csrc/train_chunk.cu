@@ -18,7 +18,7 @@
 //
 // The chunk kernels are bound by latency and by the shared-memory passes between their two groups of products; several CTAs
 // share an SM at D = 64. At B4 H11 T2048 D64 (1408 chunks): plain pre 13 + scan 10 + post 40 us, where the FFMA operators
-// took 698 + 641 us (assoc_out_bwd, prefix_scan_bwd); delta pre 21 + walk 130 + post 57 us against 3134 + 696 + 411 us
+// took 698 + 641 us (assoc_out_bwd, prefix_scan_bwd); delta pre 21 + walk 93 + post 57 us against 3134 + 696 + 411 us
 // (delta_loop_bwd, assoc_out_bwd, delta_inv_bwd).
 #include "delta_walk.cuh"
 
