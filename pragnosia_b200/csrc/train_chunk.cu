@@ -18,7 +18,7 @@
 //
 // The chunk kernels are bound by latency and by the shared-memory passes between their two groups of products; several CTAs
 // share an SM at D = 64. At B4 H11 T2048 D64 (1408 chunks): plain pre 13 + scan 10 + post 40 us, where the FFMA operators
-// took 698 + 641 us (assoc_out_bwd, prefix_scan_bwd); delta pre 21 + walk 93 + post 57 us against 3134 + 696 + 411 us
+// took 698 + 641 us (assoc_out_bwd, prefix_scan_bwd); delta pre 21 + walk 93 + post 47 us against 3134 + 696 + 411 us
 // (delta_loop_bwd, assoc_out_bwd, delta_inv_bwd).
 #include "delta_walk.cuh"
 
@@ -263,22 +263,25 @@ struct PostSmem {
     static constexpr int off_misc = alias ? o_s + ST : o_al + SQ;
     static constexpr int bytes = off_misc + 64 + 4 * 256 + 5 * 512 + 5 * 256 + 64 + 1024;    // statistics, row and column sums, <G, S>
     static constexpr int LOADED = 4 * QK + 3 * ST + (DELTA ? 2 * QK : 0);
-    static constexpr int TM_COLS = D == 64 && !DELTA ? 256 : 512;
+    static constexpr int TM_COLS = D == 64 ? 256 : 512;
 };
 
+// At D = 64 half of the tensor memory has to do, so that two CTAs share an SM (delta, B4 H11 T2048: 57 -> 47 us). The delta rule's first group
+// then leaves out R and R2, which follow into the columns of P and E once those have been read, under the pass over registers.
 template <int D, bool DELTA>
-__global__ void __launch_bounds__(TR_NT, D == 64 && !DELTA ? 2 : 1) train_post_kernel(const __grid_constant__ TrainMaps m, TrainParams p) {
+__global__ void __launch_bounds__(TR_NT, D == 64 ? 2 : 1) train_post_kernel(const __grid_constant__ TrainMaps m, TrainParams p) {
     using SM = PostSmem<D, DELTA>;
     constexpr int SUB = D / 64, HALF = D / 2, NB = D / 64;            // NB: 32-column blocks of this warp's half of a D-wide accumulator
     // first group: P, dA, R = dO S^T (all); plain: VG = V G^T; delta: KK, E = dR W^T, R2 = dR S^T
-    constexpr uint32_t TM_P = 0, TM_DA = 64, TM_KK = 128, TM_E = 192, TM_R = DELTA ? 256 : 128, TM_VG = TM_R + D;   // delta: R2 in VG's place
+    constexpr uint32_t TM_P = 0, TM_DA = 64, TM_KK = 128, TM_E = 192, TM_R = DELTA ? (D == 64 ? 0 : 256) : 128, TM_VG = DELTA && D == 64 ? 192 : TM_R + D;   // delta: R2 in VG's place
+    constexpr bool TIGHT = DELTA && D == 64;
     // second group: dQ = dP K, dK = dP^T Q (+ C K + C^T K); plain: dV = A^T dO, KG = K G; delta: WG = W G^T
-    constexpr uint32_t TM_DK = DELTA ? D : (D == 64 ? 64 : 384), TM_DV = 0, TM_DQ = DELTA ? 0 : TM_R, TM_KG = DELTA ? TM_R : TM_VG;
+    constexpr uint32_t TM_DK = DELTA ? D : (D == 64 ? 64 : 384), TM_DV = 0, TM_DQ = DELTA ? 0 : TM_R, TM_KG = DELTA ? (D == 64 ? 128 : TM_R) : TM_VG;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *sm = smem_raw + (base - smem_u32(smem_raw));
     uint8_t *misc = sm + SM::off_misc;
-    const uint32_t bar_t = base + SM::off_misc, bar_1 = bar_t + 8, bar_2 = bar_t + 16;
+    const uint32_t bar_t = base + SM::off_misc, bar_1 = bar_t + 8, bar_2 = bar_t + 16, bar_r = bar_t + 24;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(misc + 32);
     float *Ls = reinterpret_cast<float *>(misc + 64), *eLs = Ls + 64, *wts = eLs + 64, *bes = wts + 64;
     float *rr = bes + 64;                                             // row sums [quantity][column half][64]: gm, q.R, k.VG, dbeta part, k.R2
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(TR_NT, D == 64 && !DELTA ? 2 : 1) train_post_k
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5), wg = warp >> 2, sub = warp & 3;
     const int c = blockIdx.x, bh = blockIdx.y, NC = gridDim.x, T = p.T, t0 = c * TC_C;
     if (tid == 0) {
-        mbar_init(bar_t, 1); mbar_init(bar_1, 1); mbar_init(bar_2, 1);
+        mbar_init(bar_t, 1); mbar_init(bar_1, 1); mbar_init(bar_2, 1); mbar_init(bar_r, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         mbar_expect_tx(bar_t, SM::LOADED);
         const int ci = bh * NC + c;
@@ -322,6 +325,13 @@ __global__ void __launch_bounds__(TR_NT, D == 64 && !DELTA ? 2 : 1) train_post_k
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) mma_bf16_elect(tmem + acc, a + tr_ko(k, 8192), b + tr_ko(k, sub_b), idesc, onto | (k > 0));
     };
+    auto states = [&]() {                                             // R = dO S^T, R2 = dR S^T
+        if constexpr (DELTA) {
+            rows_rows(TM_VG, drh_k, s_k, D * 128, I_RD, 0);
+            rows_rows(TM_VG, drl_k, s_k, D * 128, I_RD, 1);
+        }
+        rows_rows(TM_R, do_k, s_k, D * 128, I_RD, 0);
+    };
     if (warp == 2 && ok) {
         rows_rows(TM_P, q_k, k_k, 8192, I_SQ, 0);
         rows_rows(TM_DA, do_k, v_k, 8192, I_SQ, 0);
@@ -329,13 +339,11 @@ __global__ void __launch_bounds__(TR_NT, D == 64 && !DELTA ? 2 : 1) train_post_k
             rows_rows(TM_KK, k_k, k_k, 8192, I_SQ, 0);
             rows_rows(TM_E, drh_k, v_k, 8192, I_SQ, 0);
             rows_rows(TM_E, drl_k, v_k, 8192, I_SQ, 1);
-            rows_rows(TM_VG, drh_k, s_k, D * 128, I_RD, 0);
-            rows_rows(TM_VG, drl_k, s_k, D * 128, I_RD, 1);
         } else {
             rows_rows(TM_VG, v_k, gh_k, D * 128, I_RD, 0);
             rows_rows(TM_VG, v_k, gl_k, D * 128, I_RD, 1);
         }
-        rows_rows(TM_R, do_k, s_k, D * 128, I_RD, 0);
+        if constexpr (!TIGHT) states();
         mma_commit_elect(bar_1);
     }
     // <G, S> while they run: the same bytes of two tiles of one layout
@@ -387,7 +395,7 @@ __global__ void __launch_bounds__(TR_NT, D == 64 && !DELTA ? 2 : 1) train_post_k
         if constexpr (DELTA) { tmem_ld_frag4(lb + TM_KK + col0, kk); tmem_ld_frag4(lb + TM_E + col0, ev); }
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
-            tmem_ld_frag4(lb + TM_R + HALF * wg + 32 * b, R[b]);
+            if constexpr (!TIGHT) tmem_ld_frag4(lb + TM_R + HALF * wg + 32 * b, R[b]);
             if constexpr (!DELTA) tmem_ld_frag4(lb + TM_VG + HALF * wg + 32 * b, VG[b]);
         }
         const float L0 = Ls[row0] * TR_LOG2E, L1 = Ls[row1] * TR_LOG2E, be0 = DELTA ? bes[row0] : 0.f, be1 = DELTA ? bes[row1] : 0.f;
@@ -395,6 +403,12 @@ __global__ void __launch_bounds__(TR_NT, D == 64 && !DELTA ? 2 : 1) train_post_k
 #pragma unroll
         for (int j = 0; j < 4; ++j) { Lc[j] = *reinterpret_cast<const float2 *>(Ls + col0 + 8 * j + 2 * fq); Lc[j].x *= TR_LOG2E; Lc[j].y *= TR_LOG2E; }
         tmem_ld_wait();
+        if constexpr (TIGHT) {
+            tc_fence_before();
+            __syncthreads();                                          // every warp has its fragments (ok is the same for the whole CTA)
+            tc_fence_after();
+            if (warp == 2) { states(); mma_commit_elect(bar_r); }
+        }
         float g0 = 0.f, g1 = 0.f, b0 = 0.f, b1 = 0.f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -438,6 +452,12 @@ __global__ void __launch_bounds__(TR_NT, D == 64 && !DELTA ? 2 : 1) train_post_k
         }
         row_out(0, g0, g1);
         if (DELTA) row_out(3, b0, b1);
+        if constexpr (TIGHT) {
+            ok = mbar_wait_warp(bar_r, 0, 34);
+            tc_fence_after();
+            tmem_ld_frag4(lb + TM_R + HALF * wg, R[0]);
+            tmem_ld_wait();
+        }
         float a = 0.f, b = 0.f, x = 0.f, y = 0.f;
 #pragma unroll
         for (int bl = 0; bl < NB; ++bl) {
