@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == DW_ISSUER) tmem_alloc(smem_u32(tmem_slot), TM_COLS);
+    pdl_wait();                                                       // launched as a programmatic dependent: the set-up above overlaps the kernel ahead
     if (!BWD && p.rebase_chunks > 0 && tid < D / 2) {
         float sn, cs;
         sincosf(-p.rebase_shift * p.theta[(size_t)h * (D / 2) + tid], &sn, &cs);
@@ -151,6 +152,7 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = warp_uniform(*tmem_slot);
+    pdl_launch_dependents();                                          // not before the tensor memory is this CTA's: a dependent must not take it first. (The forward walk is launched plainly: under the inverse's tail it cost 8 us of 590.)
 
     if (warp < DW_MATH) {
         // ====================================================================================================== math

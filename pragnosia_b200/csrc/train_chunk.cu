@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(TR_NT) train_pre_kernel(const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = warp_uniform(*tmem_slot);
+    pdl_launch_dependents();                                          // this CTA has its tensor memory
     if (tid == 0) p.Ltot[(size_t)bh * NC + c] = Ls[TC_C - 1];
     bool ok = mbar_wait_warp(bar_t, 0, 21);
     if (DELTA && warp == 2 && ok) {
@@ -222,7 +223,9 @@ __global__ void __launch_bounds__(TR_NT) train_pre_kernel(const __grid_constant_
 __global__ void __launch_bounds__(256) state_grad_scan_kernel(const float *__restrict__ Dc, const float *__restrict__ Ltot, const float *__restrict__ dS,
                                                               __nv_bfloat16 *__restrict__ G, float *__restrict__ dS0, int NC, int DD) {
     const int e = (blockIdx.x * 256 + threadIdx.x) * 4, bh = blockIdx.y;
+    pdl_launch_dependents();
     if (e >= DD) return;
+    pdl_wait();
     float4 g = dS != nullptr ? *reinterpret_cast<const float4 *>(dS + (size_t)bh * DD + e) : make_float4(0.f, 0.f, 0.f, 0.f);
     const float *src = Dc + (size_t)bh * NC * DD + e;
     const float *lt = Ltot + (size_t)bh * NC;
@@ -289,6 +292,7 @@ __global__ void __launch_bounds__(TR_NT, D == 64 ? 2 : 1) train_post_kernel(cons
     float *gs = cs + 320;                                             // (cs[256..]: dR . V per row), <G, S> per warp
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5), wg = warp >> 2, sub = warp & 3;
     const int c = blockIdx.x, bh = blockIdx.y, NC = gridDim.x, T = p.T, t0 = c * TC_C;
+    pdl_wait();
     if (tid == 0) {
         mbar_init(bar_t, 1); mbar_init(bar_1, 1); mbar_init(bar_2, 1); mbar_init(bar_r, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -675,20 +679,21 @@ int train_bwd_go(const TrainBwdArgs &a, cudaStream_t st) {
     const dim3 grid((unsigned)NC, (unsigned)BH);
     pre<<<grid, TR_NT, PreSmem<D, DELTA>::bytes, st>>>(m, p);
     if ((rc = check_launch("train_pre_kernel")) != PGB_OK) return rc;
+    // the rest as programmatic dependents: set-up (barriers, tensor memory) under the tail of the kernel ahead
+    cudaError_t e = cudaSuccess;
     if constexpr (DELTA) {
         auto walk = delta_walk_kernel<D, true>;
         if ((rc = tr_attr(walk, DwSmem<D, true>::bytes, "delta_walk backward smem attribute")) != PGB_OK) return rc;
         w.k = m.k;
         DwParams d{};
         d.la = a.la; d.beta = a.beta; d.S0 = a.dS; d.S_out = a.dS0; d.dW0 = p.dW0; d.Dc = p.Dc; d.H = a.H; d.T = a.T;
-        walk<<<(unsigned)BH, DW_NT, DwSmem<D, true>::bytes, st>>>(w, d);
-        rc = check_launch("delta_walk_kernel backward");
+        e = pdl_launch(walk, dim3((unsigned)BH), dim3(DW_NT), (size_t)DwSmem<D, true>::bytes, st, w, d);
     } else {
-        state_grad_scan_kernel<<<dim3((unsigned)(D * D / 1024), (unsigned)BH), 256, 0, st>>>(p.Dc, p.Ltot, a.dS, G, a.dS0, NC, D * D);
-        rc = check_launch("state_grad_scan_kernel");
+        e = pdl_launch(state_grad_scan_kernel, dim3((unsigned)(D * D / 1024), (unsigned)BH), dim3(256), (size_t)0, st, (const float *)p.Dc, (const float *)p.Ltot,
+                       a.dS, G, a.dS0, NC, D * D);
     }
-    if (rc != PGB_OK) return rc;
-    post<<<grid, TR_NT, PostSmem<D, DELTA>::bytes, st>>>(m, p);
+    if (e == cudaSuccess) e = pdl_launch(post, grid, dim3(TR_NT), (size_t)PostSmem<D, DELTA>::bytes, st, m, p);
+    if (e != cudaSuccess) { set_cuda_error(e, "train backward launch"); return PGB_ERR_CUDA; }
     return check_launch("train_post_kernel");
 }
 
