@@ -187,8 +187,8 @@ int pgb_aspin_prefill_fwd(const void *q, const void *k, const void *v, int io_dt
                           int D, int precision, void *stream);
 
 /* The plain rule on bf16 operands at D = 64 with scratch (pgb_aspin_prefill_segments_scratch_bytes bytes; 0: the sequences are too
- * short, or the chains fill the GPU, and pgb_aspin_prefill_fwd is the call): the same arithmetic with each chain cut into segments
- * that run side by side. S_out must not be S0. */
+ * short, or the chains fill the GPU evenly, and pgb_aspin_prefill_fwd is the call): the same arithmetic with chains cut into segments
+ * that run side by side -- all of them where they leave the GPU half empty, those of the last round where that leaves it so. S_out must not be S0. */
 long long pgb_aspin_prefill_segments_scratch_bytes(int B, int H, int T, int D);
 int pgb_aspin_prefill_segments_fwd(const void *q, const void *k, const void *v, const float *la, const float *S0, const float *theta,
                                    const float *shift_dev, float shift_host, void *o, int o_dtype, float *S_out, void *sent, void *scratch,

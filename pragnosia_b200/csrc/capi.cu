@@ -61,7 +61,7 @@ int prep_gates_launch(const void *, const void *, const void *, long long, long 
 int head_norm_launch(const void *, const float *, float, void *, int, int, int, int, cudaStream_t);
 size_t segment_scratch_bytes(int B, int H, int T, int seg_len);
 int segment_states_launch(const PrefillArgs &, float *, cudaStream_t);
-int segment_len_prepared(long long BH, int T);
+SegPlan segment_plan(int B, int H, int T);
 int tc_segment_error_flag(int *);
 size_t prefill_fp32_chunk_scratch_bytes(int B, int H, int T, int D);
 int prefill_fp32_chunk_launch(const PrefillArgs &, int, int, void *, cudaStream_t);
@@ -341,8 +341,32 @@ int pgb_aspin_prefill_fwd(const void *q, const void *k, const void *v, int io_dt
 
 long long pgb_aspin_prefill_segments_scratch_bytes(int B, int H, int T, int D) {
     if (B <= 0 || H <= 0 || T <= 0 || D != 64 || g_tc_variant != 0) return 0;
-    const int len = segment_len_prepared((long long)B * H, T);
-    return len == 0 ? 0 : (long long)segment_scratch_bytes(B, H, T, len);
+    const SegPlan plan = segment_plan(B, H, T);
+    return plan.len == 0 ? 0 : (long long)segment_scratch_bytes(plan.rows, H, T, plan.len);
+}
+
+// the plain rule on prepared operands at head dim 64: rows of the batch whose chains are walked whole, then those that are cut
+static int plain_with_segments(const PrefillArgs &all, int o_dtype, const SegPlan &plan, void *scratch, cudaStream_t stream) {
+    const int whole = all.B - plan.rows;
+    PrefillArgs a = all;
+    if (whole > 0) {
+        a.B = whole;
+        const int rc = prefill_tc_ws_launch(a, o_dtype, stream);
+        if (rc != PGB_OK) return rc;
+        const size_t chains = (size_t)whole * a.H, rows = chains * a.T, DD = 64 * 64, NC = (a.T + 63) / 64;
+        a = all;
+        a.B = plan.rows;
+        a.q = (const char *)a.q + rows * 64 * 2; a.k = (const char *)a.k + rows * 64 * 2; a.v = (const char *)a.v + rows * 64 * 2;
+        a.la += rows;
+        if (a.S0 != nullptr) a.S0 += chains * DD;
+        a.o = (char *)a.o + rows * 64 * (o_dtype == PGB_F32 ? 4 : 2);
+        a.S_out += chains * DD;
+        if (a.sent != nullptr) a.sent += chains * NC * DD;
+    }
+    a.seg_len = plan.len;
+    a.seg_states = (const float *)scratch;
+    const int rc = segment_states_launch(a, (float *)scratch, stream);
+    return rc != PGB_OK ? rc : prefill_tc_ws_launch(a, o_dtype, stream);
 }
 
 int pgb_aspin_prefill_segments_fwd(const void *q, const void *k, const void *v, const float *la, const float *S0, const float *theta,
@@ -359,10 +383,7 @@ int pgb_aspin_prefill_segments_fwd(const void *q, const void *k, const void *v, 
         (sent && !aligned(sent, 16)) || !aligned(scratch, 16))
         return PGB_ERR_MISALIGNED;
     PrefillArgs a{q, k, v, la, nullptr, S0, o, S_out, (__nv_bfloat16 *)sent, theta, shift_dev, shift_host, B, H, T};
-    a.seg_len = segment_len_prepared((long long)B * H, T);
-    a.seg_states = (const float *)scratch;
-    const int rc = segment_states_launch(a, (float *)scratch, (cudaStream_t)stream);
-    return rc != PGB_OK ? rc : prefill_tc_ws_launch(a, o_dtype, (cudaStream_t)stream);
+    return plain_with_segments(a, o_dtype, segment_plan(B, H, T), scratch, (cudaStream_t)stream);
 }
 
 int pgb_aspin_prefill_train_fwd(const void *q, const void *k, const void *v, const float *la, const float *S0, void *o, float *S_out, void *sent,
@@ -379,10 +400,7 @@ int pgb_aspin_prefill_train_fwd(const void *q, const void *k, const void *v, con
     const long long need = pgb_aspin_prefill_segments_scratch_bytes(B, H, T, D);
     if (need == 0 || scratch == nullptr) return tc_dispatch(a, PGB_BF16, D, (cudaStream_t)stream);
     if (scratch_bytes < need) return PGB_ERR_BAD_SHAPE;
-    a.seg_len = segment_len_prepared((long long)B * H, T);
-    a.seg_states = (const float *)scratch;
-    const int rc = segment_states_launch(a, (float *)scratch, (cudaStream_t)stream);
-    return rc != PGB_OK ? rc : prefill_tc_ws_launch(a, PGB_BF16, (cudaStream_t)stream);
+    return plain_with_segments(a, PGB_BF16, segment_plan(B, H, T), scratch, (cudaStream_t)stream);
 }
 
 long long pgb_aspin_prefill_fp32_scratch_bytes(int B, int H, int T, int D) {

@@ -91,6 +91,8 @@ struct PrefillArgs {
     int fine = 0;
     int rebase_chunks = 0;                                            // delta rule: rebase the state every so many chunks (by that many tokens)
 };
+// prepared chains cut into segments: the last `rows` rows of the batch, `len` tokens a segment (len 0: none)
+struct SegPlan { int rows, len; };
 // the backward of the scan as one call (train_chunk.cu); beta, W and X only under the delta rule
 struct TrainBwdArgs {
     const void *q, *k, *v; const float *la, *beta; const void *sent, *W, *X, *dout; const float *dsent, *dS;

@@ -269,17 +269,30 @@ size_t segment_scratch_bytes(int B, int H, int T, int seg_len) {
     return n * B * H * (SG_D * SG_D + 1) * sizeof(float);
 }
 
-// Tokens of a segment for prepared chains of T tokens, 0: not worth cutting. Where the chains leave SMs idle, a chunk costs its walk
-// 1.3 us and the state pass 0.9, the two launches before the walk about 7 (train of 44 chains of 32 chunks: 45 us whole).
-int segment_len_prepared(long long BH, int T) {
+// Which prepared chains of T tokens are cut, and into how long segments. Where all chains leave SMs idle, all of them: a chunk costs its walk
+// 1.3 us and the state pass 0.9, the two launches before the walk about 7 (train of 44 chains of 32 chunks: 45 us whole). Where they fill the
+// SMs more than once, those of the last round, as whole rows of the batch, so that the round is as short as the SMs can make it instead of a whole
+// chain long (9 us more for the launches and the round's ragged start; at 4 us more 200 chains of 64 chunks and 640 of 24 were taken and lost 0 to 2 %).
+// Whole and cut, us: 64 x 12 chains of 64 chunks 477 and 451, 64 x 7 315 and 268, 25 x 12 of 63 232 and 188, 13 x 12 of 128 303 and 197, 16 x 12 of 32 84 and 79.
+SegPlan segment_plan(int B, int H, int T) {
     const int NC = (T + TC_C - 1) / TC_C, sms = sm_count();
-    if (NC < 16 || BH * 2 > sms) return 0;
-    int best = 0;
-    double cost = 1.3 * NC;
-    for (int n = 2; n * BH <= sms; ++n) {
+    const long long BH = (long long)B * H;
+    if (NC < 16) return {0, 0};
+    SegPlan best{0, 0};
+    int rows = B;
+    double cost = 1.3 * NC, extra = 7.0;                              // of the part that could be cut
+    if (BH > sms) {
+        const long long rounds = (BH + sms - 1) / sms;
+        const long long rest = BH - (rounds - 1) * sms;              // chains of the last round
+        rows = (int)((rest + H - 1) / H);
+        extra = 16.0;
+    }
+    const long long chains = (long long)rows * H;
+    if (rows > B || chains * 2 > sms) return best;
+    for (int n = 2; n * chains <= sms; ++n) {
         const int len = (NC + n - 1) / n;
         if (len < 2) break;
-        if (len * TC_C <= SG_MAX_PREPARED && len * 2.2 + 7.0 < cost) { cost = len * 2.2 + 7.0; best = len * TC_C; }
+        if (len * TC_C <= SG_MAX_PREPARED && len * 2.2 + extra < cost) { cost = len * 2.2 + extra; best = {rows, len * TC_C}; }
     }
     return best;
 }

@@ -298,7 +298,7 @@ ScanOut prefill(const Tensor &q_, const Tensor &k_, const Tensor &v_, const Tens
         return {o, S, some(sent)};
     }
     if (!beta.defined() && dt == at::kBFloat16 && precision != PGB_PREFILL_FP32 && D == 64 && !(S0.defined() && S0.is_same_size(S) && S0.data_ptr() == S.data_ptr())) {
-        const long long n = pgb_aspin_prefill_segments_scratch_bytes(B, H, T, D); // few long chains: their segments side by side
+        const long long n = pgb_aspin_prefill_segments_scratch_bytes(B, H, T, D); // few long chains, or few in the last round: their segments side by side
         if (n > 0) {
             const Tensor scratch = bytes(q, n);
             check(pgb_aspin_prefill_segments_fwd(vp(q), vp(k), vp(v), fp(la), fp(S0), fp(theta), fp(shift), shift_host, vp(o), oc, fp(S), vp(sent),

@@ -13,7 +13,8 @@ def rel(a, b):
     return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
 
 
-@pytest.mark.parametrize("B,H,T", [(1, 1, 1024), (1, 2, 1025), (2, 6, 2048), (4, 11, 2047), (1, 12, 8192), (1, 1, 20000), (1, 74, 2817)])
+@pytest.mark.parametrize("B,H,T", [(1, 1, 1024), (1, 2, 1025), (2, 6, 2048), (4, 11, 2047), (1, 12, 8192), (1, 1, 20000), (1, 74, 2817),
+                                   (13, 12, 1100), (150, 2, 1090), (25, 12, 2050)])   # the last round's only
 @pytest.mark.parametrize("shift", [0.0, 37.0])
 def test_segments_match_the_whole_walk(B, H, T, shift):
     assert _lib.lib().pgb_aspin_prefill_segments_scratch_bytes(B, H, T, 64) > 0
@@ -32,6 +33,6 @@ def test_segments_match_the_whole_walk(B, H, T, shift):
             assert rel(o.cpu(), ro) < 4e-3 and rel(S.cpu(), rS) < 1e-4
 
 
-@pytest.mark.parametrize("B,H,T,D", [(1, 1, 960, 64), (1, 75, 4096, 64), (1, 2, 4096, 128)])
+@pytest.mark.parametrize("B,H,T,D", [(1, 1, 960, 64), (1, 75, 4096, 64), (1, 2, 4096, 128), (3, 100, 4096, 64), (13, 12, 960, 64), (20, 10, 4096, 64)])
 def test_not_worth_cutting(B, H, T, D):
     assert _lib.lib().pgb_aspin_prefill_segments_scratch_bytes(B, H, T, D) == 0
