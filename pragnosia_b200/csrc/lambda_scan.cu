@@ -20,6 +20,8 @@
 // recurrence; with TS > 1 only the state at segment boundaries is reassociated (fp32 rounding, no other difference).
 #include <math.h>
 
+#include <type_traits>
+
 #include "scan_math.cuh"
 
 namespace pgb {
@@ -31,8 +33,13 @@ constexpr int LS_WARPS = 2;
 // its use needed 24, B64 T4096 D768 760 us against 660, one angle per channel 590 against 480; spills are poison next to this much shared
 // memory, which leaves the L1 no room: 1010 us with 24 warps and 70 bytes spilled). Narrower lanes request the next tile into
 // registers: a copy of 4 or 8 bytes costs an instruction more than it saves (B13 T1111 D510: 44 against 54 us).
-template <int VEC> struct LsForm { static constexpr bool staged = VEC == 4; static constexpr int slots = staged ? 2 : 1; };
-constexpr int LS_SEG = 4;                                             // steps a lane takes of a tile
+// So does BRIEF, for walks of a few tiles, with two steps a lane and tile: what counts there is the way of a tile through a lane (1.3 us, of four
+// steps through slots 1.9), and the slots' extra step through shared memory (one sequence of 64 tokens: 3.2 us against 3.8; of 700: 15.9 and 13.3).
+template <int VEC, bool BRIEF = false> struct LsForm {
+    static constexpr bool staged = VEC == 4 && !BRIEF;
+    static constexpr int slots = staged ? 2 : 1, seg = BRIEF ? 2 : 4;
+};
+constexpr int LS_SEG = LsForm<4>::seg;                                // steps a lane takes of a tile
 constexpr int LS_CTAS_PER_SM = 8;                                     // the same for the adjoint, whose slots make room for two warps more an SM
 
 // VEC adjacent channels of one row as pairs (the last one half empty when VEC is 1)
@@ -88,14 +95,14 @@ __device__ __forceinline__ void ls_scan_maps(f2 &Ar, f2 &Ai, f2 &Br, f2 &Bi, int
     if (seg == 0) { Ar = f2_both(1.f); Ai = 0ull; Br = 0ull; Bi = 0ull; }
 }
 
-template <int VEC, int TS, bool ANG_BCAST, bool KEEP>
+template <int VEC, int TS, bool ANG_BCAST, bool KEEP, bool BRIEF>
 __global__ void __launch_bounds__(LS_WARPS * 32, LS_CTAS_PER_SM)
 lambda_scan_kernel(const float *__restrict__ u, const float *__restrict__ lm, const float *__restrict__ an,
                    long long an_sb, long long an_st, const float *__restrict__ h0r, const float *__restrict__ h0i,
                    float *__restrict__ y, float *__restrict__ hr_out, float *__restrict__ hi_out, float *__restrict__ hi_all,
                    int B, int T, int D) {
-    using Form = LsForm<VEC>;
-    constexpr int CQ = 32 / TS, SEG = LS_SEG, NST = Form::slots, NP = LsVec<VEC>::NP;
+    using Form = LsForm<VEC, BRIEF>;
+    constexpr int CQ = 32 / TS, SEG = Form::seg, NST = Form::slots, NP = LsVec<VEC>::NP;
     constexpr int NA = ANG_BCAST ? 2 : 3;                          // u, logmag, angle
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ __align__(16) float slots[Form::staged ? NST : 1][NA][SEG][Form::staged ? LS_WARPS * 32 * VEC : 1];
@@ -426,6 +433,7 @@ namespace {
 struct LsArgs {
     const float *u, *lm, *an; long long sb, st; const float *h0r, *h0i; float *y, *hro, *hio, *hia;
     int B, T, D;
+    bool brief;
 };
 struct LsBwdArgs {
     const float *g, *u, *lm, *an; long long sb, st; const float *hr_all, *hi_all, *gli; float *du, *dlm, *dan, *dh0r, *dh0i;
@@ -447,8 +455,14 @@ int launch_ts(const LsArgs &a, cudaStream_t stream) {
         kern<<<(unsigned)ctas, LS_WARPS * 32, 0, stream>>>(a.u, a.lm, a.an, a.sb, a.st, a.h0r, a.h0i, a.y, a.hro, a.hio, a.hia, a.B, a.T, a.D);
     };
     const bool bc = a.sb == 0 && a.st == 0, keep = a.hia != nullptr;
-    if (keep) { if (bc) go(lambda_scan_kernel<VEC, TS, true, true>); else go(lambda_scan_kernel<VEC, TS, false, true>); }
-    else { if (bc) go(lambda_scan_kernel<VEC, TS, true, false>); else go(lambda_scan_kernel<VEC, TS, false, false>); }
+    auto form = [&](auto brief) {
+        constexpr bool BRIEF = decltype(brief)::value;
+        if (keep) { if (bc) go(lambda_scan_kernel<VEC, TS, true, true, BRIEF>); else go(lambda_scan_kernel<VEC, TS, false, true, BRIEF>); }
+        else { if (bc) go(lambda_scan_kernel<VEC, TS, true, false, BRIEF>); else go(lambda_scan_kernel<VEC, TS, false, false, BRIEF>); }
+    };
+    if constexpr (VEC == 4) {
+        if (a.brief) form(std::true_type{}); else form(std::false_type{});
+    } else form(std::false_type{});
     return check_launch("lambda_scan_kernel");
 }
 template <int VEC, int TS>
@@ -494,47 +508,57 @@ int ls_vec(int D, long long sb, long long st, P... ptrs) {
 // instructions; more segments shorten (i), but make the rows a warp reads narrower: the adjoint with rows of 256, 128, 64, 32 and 16 bytes takes
 // 1231, 1315, 1410, 1744 and 3241 us at B64 T4096 D768, the scan forward without a copy of the state 886, 642, 662, 725 and 1300. The two overlap:
 // root of the sum of squares (B16 T4096 D768, 2 to 16 segments: 652, 362, 259, 201 us; the estimate says 645, 370, 258, 209).
-struct LsCost { double tile_us, ps, narrow_ps; bool adjoint; };       // per tile; per element: the bytes' time, the instructions' of lanes with one channel
-static int ls_pick(int B, int T, int D, int vec, const LsCost &k, int sms) {
+struct LsCost { double tile_us, ps, narrow_ps; bool adjoint; int seg; };   // per tile; per element: the bytes' time, the instructions' of lanes with one channel
+struct LsPick { int ts; double cost; };
+static LsPick ls_pick(int B, int T, int D, int vec, const LsCost &k, int sms) {
     static const double width[7] = {1.0, 1.0, 1.08, 1.4, 2.3, 3.5, 6.0};        // rows of 256, 128, ... 4 bytes
     const int ngroups = D / vec;
     const double cap = (double)sms * LS_CTAS_PER_SM * LS_WARPS;                 // resident warps
-    int best = 1;
-    double best_cost = 0.0;
+    LsPick best{1, 0.0};
     for (int ts = 1, lg = 0; ts <= 32; ts <<= 1, ++lg) {
-        if (ts > 1 && (ts / 2) * LS_SEG >= T) break;                            // the sequence has no more pieces to hand out
+        if (ts > 1 && (ts / 2) * k.seg >= T) break;                             // the sequence has no more pieces to hand out
         const int cq = 32 / ts;
-        const long long warps = (long long)B * ((ngroups + cq - 1) / cq), tiles = (T + ts * LS_SEG - 1) / (ts * LS_SEG);
+        const long long warps = (long long)B * ((ngroups + cq - 1) / cq), tiles = (T + ts * k.seg - 1) / (ts * k.seg);
         int w = 0;
         for (int row = 4 * vec * cq; row < 256; row <<= 1) ++w;
         double f = width[w < 6 ? w : 6];
         if (!k.adjoint && w <= 4) f = sqrt(f);
         if (ts == 32 && warps <= 8LL * sms && f > 1.4) f = 1.4;                 // few warps do not load the memory: a narrow row costs no more than another
         const double walk = (double)tiles * (k.tile_us + 0.1 * lg) * (warps > cap ? (double)warps / cap : 1.0);
-        const double move = (double)B * T * D * 1e-6 * (k.ps * f + (vec == 1 ? k.narrow_ps : 0.0));
+        const double move = (double)B * (k.adjoint ? T : tiles * ts * k.seg) * D * 1e-6 * (k.ps * f + (vec == 1 ? k.narrow_ps : 0.0));
         const double cost = walk * walk + move * move;
-        if (ts == 1 || cost < best_cost) { best = ts; best_cost = cost; }
+        if (ts == 1 || cost < best.cost) best = {ts, cost};
     }
     return best;
 }
-static LsCost ls_cost_fwd(bool bcast, bool keep) { return {1.2, 3.2 - (bcast ? 0.8 : 0.0) + (keep ? 0.8 : 0.0), 3.0, false}; }
+// brief: half the steps a tile, requested a tile ahead into registers, at four fifths of the slots' pace once the memory is loaded
+static LsCost ls_cost_fwd(bool bcast, bool keep, bool brief) {
+    const double ps = 3.2 - (bcast ? 0.8 : 0.0) + (keep ? 0.8 : 0.0);
+    return brief ? LsCost{bcast ? 0.45 : 0.6, 1.25 * ps, 3.0, false, 2} : LsCost{1.2, ps, 3.0, false, LS_SEG};
+}
 int lambda_scan_pick_ts(int B, int T, int D, int vec, int sms, int force_ts) {
-    return force_ts > 0 ? force_ts : ls_pick(B, T, D, vec, ls_cost_fwd(false, false), sms);
+    return force_ts > 0 ? force_ts : ls_pick(B, T, D, vec, ls_cost_fwd(false, false, false), sms).ts;
 }
 
 int lambda_scan_launch(const float *u, const float *lm, const float *an, long long sb, long long st, const float *h0r,
                        const float *h0i, float *y, float *hro, float *hio, float *hia, int B, int T, int D, int force_ts,
                        cudaStream_t stream) {
-    const int vec = ls_vec(D, sb, st, u, lm, an, y, hia, hro, hio, h0r, h0i);
-    const int ts = force_ts > 0 ? force_ts : ls_pick(B, T, D, vec, ls_cost_fwd(sb == 0 && st == 0, hia != nullptr), sm_count());
-    return launch_any(vec, ts, LsArgs{u, lm, an, sb, st, h0r, h0i, y, hro, hio, hia, B, T, D}, stream);
+    const int vec = ls_vec(D, sb, st, u, lm, an, y, hia, hro, hio, h0r, h0i), sms = sm_count();
+    const bool bcast = sb == 0 && st == 0, keep = hia != nullptr;
+    LsPick pick = force_ts > 0 ? LsPick{force_ts, 0.0} : ls_pick(B, T, D, vec, ls_cost_fwd(bcast, keep, false), sms);
+    bool brief = false;
+    if (force_ts <= 0 && vec == 4) {
+        const LsPick other = ls_pick(B, T, D, vec, ls_cost_fwd(bcast, keep, true), sms);
+        if (other.cost < pick.cost) { pick = other; brief = true; }
+    }
+    return launch_any(vec, pick.ts, LsArgs{u, lm, an, sb, st, h0r, h0i, y, hro, hio, hia, B, T, D, brief}, stream);
 }
 
 int lambda_scan_bwd_launch(const float *g, const float *u, const float *lm, const float *an, long long sb, long long st,
                            const float *hr_all, const float *hi_all, const float *gli, float *du, float *dlm, float *dan,
                            float *dh0r, float *dh0i, int B, int T, int D, cudaStream_t stream) {
     const int vec = ls_vec(D, sb, st, g, u, lm, an, hr_all, hi_all, gli, du, dlm, dan, dh0r, dh0i);
-    const int ts = ls_pick(B, T, D, vec, LsCost{1.75, sb == 0 && st == 0 ? 5.1 : 6.1, 4.5, true}, sm_count());
+    const int ts = ls_pick(B, T, D, vec, LsCost{1.75, sb == 0 && st == 0 ? 5.1 : 6.1, 4.5, true, LS_SEG}, sm_count()).ts;
     return launch_any(vec, ts, LsBwdArgs{g, u, lm, an, sb, st, hr_all, hi_all, gli, du, dlm, dan, dh0r, dh0i, B, T, D}, stream);
 }
 
