@@ -589,13 +589,17 @@ int decode_flow_error_flag(int *out) {
     return PGB_OK;
 }
 
+// dynamic shared memory at most, beside 7 KB of the kernel's own; also the function's limit at every call, whatever the call's model needs (other
+// threads may be launching the same function for other models)
+constexpr size_t FL_SMEM_MOST = 220 * 1024;
+
 static size_t decode_flow_smem(int NB, int L, int d, int dff) {
     return (size_t)DT_DEPTH * FL_STAGE_U4 * sizeof(uint4) + (size_t)NB * (2 * (size_t)d + (dff > d ? dff : d)) * sizeof(__nv_bfloat16) + (size_t)(L + 1) * sizeof(DtLayer);
 }
-// bytes of marked words; 0: the shapes need more shared memory than a CTA has (beside 7 KB of the kernel's own), or have rows of which not
+// bytes of marked words; 0: the shapes need more shared memory than a CTA has, or have rows of which not
 // even one a warp (the MLP's second layer: one) fits a stage
 size_t decode_flow_work_bytes(int L, int B, int d, int NP, int dff) {
-    if (d / 8 > FL_STAGE_U4 / DT_WARPS || dff / 8 > FL_STAGE_U4 || decode_flow_smem(B <= 2 ? B : 4, L, d, dff) > 220 * 1024) return 0;
+    if (d / 8 > FL_STAGE_U4 / DT_WARPS || dff / 8 > FL_STAGE_U4 || decode_flow_smem(B <= 2 ? B : 4, L, d, dff) > FL_SMEM_MOST) return 0;
     return (size_t)L * B * ((size_t)NP + 3 * d + dff) * sizeof(unsigned);
 }
 
@@ -606,7 +610,7 @@ static int decode_flow_go(const FlArgs &a, cudaStream_t stream) {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t smem = decode_flow_smem(NB, a.L, a.d, a.dff);
     auto kern = decode_flow_kernel<D, DELTA, NB>;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL_SMEM_MOST);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, DT_THREADS, smem);
     if (e != cudaSuccess || sms <= 0 || per_sm <= 0) {
         set_cuda_error(e == cudaSuccess ? cudaErrorLaunchOutOfResources : e, "decode_flow set-up");

@@ -458,7 +458,9 @@ static int decode_token_go(const DtArgs &a, cudaStream_t stream) {
     const size_t smem = (size_t)DT_WARPS * DT_STAGE_U4 * sizeof(uint4) + (size_t)NB * (size_t)(a.dff > a.d ? a.dff : a.d) * sizeof(__nv_bfloat16) +
                         (size_t)a.L * sizeof(DtLayer);
     auto kern = decode_token_kernel<D, DELTA, NB>;
-    if (e == cudaSuccess && smem > 32 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // rows and layer table are 72 KB at most (checked at the C entry); the limit is the function's, so the same whatever the call's model needs
+    constexpr size_t MOST = (size_t)DT_WARPS * DT_STAGE_U4 * sizeof(uint4) + 72 * 1024;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, DT_THREADS, smem);
     if (e != cudaSuccess || sms <= 0 || per_sm <= 0) {
         set_cuda_error(e == cudaSuccess ? cudaErrorLaunchOutOfResources : e, "decode_token set-up");

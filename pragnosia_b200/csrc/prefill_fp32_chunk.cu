@@ -244,9 +244,12 @@ static int prefill_fp32_chunk_go(const PrefillArgs &a, int o_dtype, float *scrat
     const PcParams p{(const float *)a.q, (const float *)a.k, (const float *)a.v, a.la, scratch, Ltot, a.o, o_dtype == PGB_BF16, a.T, NC};
     // Output CTAs that come while the first kernel's are still there go wherever there is room, three to an SM beside SMs with none: where they
     // all fit one or two to an SM, as many bytes of shared memory as leave room for no more keep them there (192 CTAs on 148 SMs: 30.7 us the call without, 20.7 with).
+    // The size is the launch's; the limit belongs to the function, which threads with calls of other sizes share, so it is the same at every call.
+    constexpr size_t ONE_PER_SM = 116 * 1024, TWO_PER_SM = 78 * 1024;
+    static_assert(PcOut<D>::bytes <= ONE_PER_SM, "the function's limit is the largest size of all calls");
     const long long ctas = (long long)BH * NC * (D / 64), sms = sm_count();
-    const size_t least = ctas <= sms ? 116 * 1024 : ctas <= 2 * sms ? 78 * 1024 : 0, out_bytes = PcOut<D>::bytes > least ? PcOut<D>::bytes : least;
-    const cudaError_t e = cudaFuncSetAttribute(fp32_out_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_bytes);
+    const size_t least = ctas <= sms ? ONE_PER_SM : ctas <= 2 * sms ? TWO_PER_SM : 0, out_bytes = PcOut<D>::bytes > least ? PcOut<D>::bytes : least;
+    const cudaError_t e = cudaFuncSetAttribute(fp32_out_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ONE_PER_SM);
     if (e != cudaSuccess) { set_cuda_error(e, "fp32_out smem attribute"); return PGB_ERR_CUDA; }
     fp32_outer_kernel<D><<<dim3((unsigned)NC, (unsigned)BH, (D / 64) * (D / 64)), PC_NT, 0, st>>>(p);
     int rc = check_launch("fp32_outer_kernel");

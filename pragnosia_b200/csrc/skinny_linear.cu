@@ -227,8 +227,8 @@ __global__ void __launch_bounds__(SK_WARPS * 32) skinny_linear_kernel(SkinnyArgs
 
 template <int B>
 static cudaError_t skinny_go(const SkinnyArgs &a, int ctas, size_t smem, cudaStream_t stream) {
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(skinny_linear_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) {                                               // the limit is the function's, so the same whatever the call's K: eight rows of 6144
+        cudaError_t e = cudaFuncSetAttribute(skinny_linear_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
         if (e != cudaSuccess) return e;
     }
     return pdl_launch(skinny_linear_kernel<B>, dim3((unsigned)ctas), dim3(SK_WARPS * 32), smem, stream, a);
