@@ -8,7 +8,9 @@ namespace pgb {
 
 static thread_local char g_err[256] = "";
 
+// The runtime keeps a refused launch's error for the thread's next look: taken off here, so that no later call reports it as its own.
 void set_cuda_error(cudaError_t e, const char *where) {
+    cudaGetLastError();
     snprintf(g_err, sizeof(g_err), "%s: %s (%s)", where, cudaGetErrorName(e), cudaGetErrorString(e));
 }
 

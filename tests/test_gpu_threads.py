@@ -1,10 +1,11 @@
-"""The tensor-core paths as the first CUDA work of a thread: its results are the main thread's."""
+"""Threads: first CUDA work in one, calls of several sizes at once, what a refused call leaves behind."""
+import ctypes
 import threading
 
 import pytest
 import torch
 
-from pragnosia_b200 import ops, synth
+from pragnosia_b200 import _lib, ops, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -63,3 +64,24 @@ def test_fp32_calls_of_two_sizes_at_once(D):
     torch.cuda.synchronize()
     assert not errors, errors[0]
     assert [int(o) for o in off] == [0, 0]
+
+
+def test_a_refused_launch_leaves_no_error_behind():
+    """A launch that the runtime refuses on the host (into a capture that is no longer valid) is that call's error alone: the thread's
+    next call succeeds."""
+    rt = ctypes.CDLL("libcudart.so.12")                              # the one torch has loaded
+    x, w, z = (torch.ones(4, 64, device="cuda") for _ in range(3))
+    torch.cuda.synchronize()
+    bad, graph = ctypes.c_void_p(), ctypes.c_void_p()
+    assert rt.cudaStreamCreate(ctypes.byref(bad)) == 0
+    call = lambda stream: _lib.lib().pgb_add_norm(*(ctypes.c_void_p(p) for p in (x.data_ptr(), 0, w.data_ptr(), 0)), ctypes.c_float(1e-6), 0,
+                                                  None, ctypes.c_void_p(z.data_ptr()), ctypes.c_longlong(4), 64, 0, stream)
+    assert call(None) == 0
+    assert rt.cudaStreamBeginCapture(bad, 0) == 0
+    assert rt.cudaDeviceSynchronize() != 0                           # not allowed meanwhile: the capture is lost
+    assert call(bad) != 0
+    assert rt.cudaStreamEndCapture(bad, ctypes.byref(graph)) != 0
+    rt.cudaGetLastError()
+    assert call(None) == 0
+    torch.cuda.synchronize()
+    assert rt.cudaStreamDestroy(bad) == 0
