@@ -348,3 +348,33 @@ def test_replaced_mlp_layers_are_called(name):
     dec.prefill(ids(6, 70, 1))
     want = dec.step(ids(6, 1, 2)[:, 0]).float()
     assert float((got - want).norm() / want.norm()) < 2e-2 < float((plain - want).norm() / want.norm())
+
+
+def test_the_benchmarks_decode_leg_times_no_capture(monkeypatch):
+    """Both timed calls of a leg, the sampled loop and the prompt pass subtracted from it, replay what is captured by then."""
+    import types
+    import bench
+    from pragnosia_b200 import kernel_bench
+    model = LM(vocab=bench.CFG["vocab"], d=128, layers=2, mlp_mult=4, ctx=512, mixer="aspin", norm="rms").cuda().bfloat16().eval()
+    captures, calls, capture, generate, prefill = [0], [], LM.capture, Decoder.generate, Decoder.prefill
+
+    def counted(*a, **k):
+        captures[0] += 1
+        return capture(*a, **k)
+
+    def logged(name, f):
+        def call(*a, **k):
+            before, out = captures[0], f(*a, **k)
+            calls.append((name, captures[0] - before))
+            return out
+        return call
+
+    monkeypatch.setattr(LM, "capture", counted)
+    monkeypatch.setattr(Decoder, "generate", logged("generate", generate))
+    monkeypatch.setattr(Decoder, "prefill", logged("prefill", prefill))
+    monkeypatch.setattr(kernel_bench, "time_case", lambda name: (1.0, 1.0))
+    bench.decode_numbers(model, torch.device("cuda"), dict(hbm_gbs=1.0), types.SimpleNamespace(decode_steps=8))
+    timed = [i for i, (name, _) in enumerate(calls) if name == "generate"][1::2]      # per batch: the warm-up, then the timed call
+    assert len(timed) == 2 and sum(n for _, n in calls) >= 4                          # per batch, the prompt and the token
+    for i in timed:
+        assert calls[i] == ("generate", 0) and calls[i + 1] == ("prefill", 0), calls
