@@ -449,8 +449,9 @@ int pgb_decode_embed_ex(const long long *tok, const long long *pos, const void *
  *   sync: two 64-bit words, zero before the first launch and then left to the kernel (the grid barrier's counters); one
  *         pair per stream of launches, never shared by two launches in flight.
  *   B <= 4, D in {64, 128}, d = H * D, NP >= 3d + 2H, NP and dff multiples of 8; delta: 0 plain rule, 1 delta rule.
- * Every barrier wait is bounded; a wait that runs out makes the whole grid return and pgb_tc_error_flag reads 81 (zero the
- * sync words before the next launch).
+ * Every barrier wait is bounded; a wait that runs out makes the whole grid return and pgb_tc_error_flag reads 81. Zero the
+ * sync words before the next launch with them, and take the prompts in again: the step is lost (logits undefined), the states of
+ * the layers already stepped are advanced, position and shift are not. Launches with other sync words are not affected.
  * ------------------------------------------------------------------------------------------------------- */
 long long pgb_decode_token_work_bytes(int B, int d, int NP, int dff);
 /* Self-test of that kernel's failure path: one CTA arrives at a grid barrier nobody else will reach; after `limit_polls`
@@ -472,8 +473,15 @@ int pgb_decode_token_step_fwd(const void *layer_table, int L, const void *E, con
  *   work: pgb_decode_flow_work_bytes(L, B, d, NP, dff) bytes, 16-byte aligned, zero before the first launch and then left to the kernel
  *         (0: the shapes want more shared memory than there is; take the step above).
  *   sync: as above, and the pair belongs to its work: both are zeroed or replaced together, and another device's launches have their own.
- * A wait that runs out makes the whole grid return and pgb_tc_error_flag reads 82; nothing needs resetting after it. */
+ * A wait that runs out makes the whole grid return and pgb_tc_error_flag reads 82. The words and sync need no resetting: the launches
+ * behind it and those of other models don't see it. But the step is lost: its logits are undefined, the states of the layers already stepped
+ * are advanced, and position and shift (window > 0) as a rule are not, so take the prompts in again before the next step. */
 long long pgb_decode_flow_work_bytes(int L, int B, int d, int NP, int dff);
+/* Self-test of its waits: a kernel of one CTA looks for 128 words of its own `limit_looks` times (1 .. 2^20, rounded up to a
+ * multiple of 64), as the first launch of the pair; they are written `late_cycles` of the SM clock after its start (at most 2^31; negative: never). A wait that runs out leaves 1 in
+ * sync[1] and 82 in pgb_tc_error_flag, one that is served leaves sync[1] alone; the kernel returns normally either way. words: 128 zero words,
+ * sync: two zero 64-bit words, both 16-byte aligned. No counterpart in the reference. */
+int pgb_decode_flow_wait_selftest(unsigned *words, unsigned long long *sync, long long limit_looks, long long late_cycles, void *stream);
 int pgb_decode_flow_step_fwd(const void *layer_table, int L, const void *E, const void *P, const void *final_norm_weight,
                              const void *final_norm_bias, int final_norm_kind, float final_norm_eps, const long long *tok,
                              long long *pos, float *shift, int window, void *work, long long work_bytes, float *logits,

@@ -70,6 +70,7 @@ SIGNATURES = {
                              _i, _vp],
     "pgb_decode_token_step_fwd": [_vp, _i, _vp, _vp, _vp, _vp, _i, _f, _vp, _vp, _vp, _i, _vp, _ll, _vp, _vp, _i, _i, _i, _i, _i, _i, _i,
                                   _i, _i, _vp],
+    "pgb_decode_flow_wait_selftest": [_vp, _vp, _ll, _ll, _vp],
     "pgb_decode_flow_work_bytes": [_i, _i, _i, _i, _i],
     "pgb_decode_flow_step_fwd": [_vp, _i, _vp, _vp, _vp, _vp, _i, _f, _vp, _vp, _vp, _i, _vp, _ll, _vp, _vp, _i, _i, _i, _i, _i, _i, _i,
                                  _i, _i, _vp],

@@ -92,6 +92,7 @@ int decode_flow_launch(const void *, int, const void *, const void *, const void
                        void *, float *, unsigned long long *, int, int, int, int, int, int, int, int, int, int, cudaStream_t);
 size_t decode_flow_work_bytes(int L, int B, int d, int NP, int dff);
 int decode_flow_error_flag(int *);
+int decode_flow_wait_selftest_launch(unsigned *, unsigned long long *, unsigned, long long, cudaStream_t);
 int batch_linear_launch(const void *, const void *, const void *, void *, int, int, int, int, const float *, int, const float *, const float *,
                         int, float, const void *, float *, int, cudaStream_t);
 int batch_linear_parts(int N);
@@ -622,6 +623,13 @@ int pgb_decode_token_wait_selftest(unsigned long long *sync, long long limit_pol
     if (limit_polls < 1 || limit_polls > (1ll << 20)) return PGB_ERR_BAD_SHAPE;          // at most about a second
     if (!aligned(sync, 16)) return PGB_ERR_MISALIGNED;
     return decode_token_wait_selftest_launch(sync, (unsigned)limit_polls, (cudaStream_t)stream);
+}
+
+int pgb_decode_flow_wait_selftest(unsigned *words, unsigned long long *sync, long long limit_looks, long long late_cycles, void *stream) {
+    if (!words || !sync) return PGB_ERR_NULL_POINTER;
+    if (limit_looks < 1 || limit_looks > (1ll << 20) || late_cycles > (1ll << 31)) return PGB_ERR_BAD_SHAPE;   // at most about a second each
+    if (!aligned(words, 16) || !aligned(sync, 16)) return PGB_ERR_MISALIGNED;
+    return decode_flow_wait_selftest_launch(words, sync, (unsigned)limit_looks, late_cycles, (cudaStream_t)stream);
 }
 
 long long pgb_decode_token_work_bytes(int B, int d, int NP, int dff) {

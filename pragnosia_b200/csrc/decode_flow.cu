@@ -19,8 +19,9 @@
 // d 768, 12 layers, vocabulary 8192, microseconds a token with barriers and without: batch 1 231 -> 172, batch 2 251 -> 190, batch 4 307 -> 216
 // (28 us is what the weights' bytes take).
 //
-// Waits are bounded: a thread that gives up raises a flag that every other one looks at, the CTA's threads agree on it at their next
-// barrier, and the kernel winds down. All CTAs are resident (a cooperative launch), and a phase only waits for earlier ones.
+// Waits are bounded: a thread that gives up raises a word beside the launch counter that every other one looks at, the CTA's threads agree on
+// it at their next barrier, and the kernel winds down; the last CTA takes the word back, so launches behind it, and those of other models,
+// never see it. All CTAs are resident (a cooperative launch), and a phase only waits for earlier ones.
 #include "decode_token.cuh"
 #include "tc_common.cuh"
 
@@ -38,7 +39,8 @@ struct FlArgs {
     float *shift;
     unsigned *words;                                                  // [L] x ([B][NP] y, [B][d] o, [B][d] d1, [B][d] d2, [B][dff] hmid)
     float *logits;
-    unsigned long long *sync;                                         // [0] CTAs that have come to the head so far, over all launches
+    unsigned long long *sync;                                         // [0] CTAs that have come to the head so far, over all launches; [1] not zero
+                                                                      // while a launch winds down
     int L, B, d, H, NP, dff, V, ctx, fn_kind, window;
     float fn_eps;
 };
@@ -57,20 +59,30 @@ __device__ __forceinline__ unsigned fl_ld1(const unsigned *at) {
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(at) : "memory");
     return v;
 }
-// false: the wait ran out, here or at another thread
-__device__ __forceinline__ bool fl_again(unsigned &spins) {
-    if (++spins > DT_SPIN_LIMIT || ((spins & 63u) == 0u && *reinterpret_cast<volatile int *>(&g_fl_error) != 0)) {
-        atomicExch(&g_fl_error, 82);
-        return false;
-    }
+// what a wait is for, and what ends it
+struct FlWait {
+    unsigned mark;
+    unsigned *given_up;                                               // sync[1]
+    unsigned limit = DT_SPIN_LIMIT;
+};
+// the 64th look, 128th, ... at something: true: the wait ran out, here or at another thread of the launch (out of line: rarely called, and the
+// kernel's code is fetched once a token)
+__device__ __noinline__ bool fl_gone(unsigned spins, unsigned limit, unsigned *given_up) {
+    if (spins < limit && *reinterpret_cast<volatile unsigned *>(given_up) == 0u) return false;
+    atomicExch(given_up, 1u);
+    atomicExch(&g_fl_error, 82);
     return true;
+}
+__device__ __forceinline__ bool fl_again(unsigned &spins, const FlWait &wt) {
+    return (++spins & 63u) != 0u || !fl_gone(spins, wt.limit, wt.given_up);
 }
 // N vectors of four words each, those of `want` (a bit each): read until all of them carry the mark. A whole warp calls it. While
 // something is missing one lane looks for the first of it: a line that the whole chip reads again and again takes microseconds to be
 // written. Batch 1: all lanes on their own words 212 us a token where one lane a warp took 181; every CTA another word first 176 where
 // all on the same took 172; eight words a load 187; a line of its own to wait on, written behind the values, 190: a round trip more.
 template <int N>
-__device__ __forceinline__ bool fl_take4(const unsigned *(&at)[N], unsigned want, unsigned mark, uint4 (&v)[N]) {
+__device__ __forceinline__ bool fl_take4(const unsigned *(&at)[N], unsigned want, const FlWait &wt, uint4 (&v)[N]) {
+    const unsigned mark = wt.mark;
     constexpr unsigned FULL = 0xffffffffu;
     while (true) {
 #pragma unroll
@@ -88,22 +100,22 @@ __device__ __forceinline__ bool fl_take4(const unsigned *(&at)[N], unsigned want
             for (int i = N - 1; i > 0; --i) if (want >> i & 1u) p = at[i];
             if (want & 1u) p = at[0];
             unsigned spins = 0;
-            while (found != 0 && (fl_ld1(p) ^ mark) >= 0x10000u) found = fl_again(spins);
+            while (found != 0 && (fl_ld1(p) ^ mark) >= 0x10000u) found = fl_again(spins, wt);
         }
         if (__shfl_sync(FULL, found, leader) == 0) return false;
     }
 }
 template <int N>
-__device__ __forceinline__ bool fl_take1(const unsigned *(&at)[N], unsigned mark, float (&x)[N]) {
+__device__ __forceinline__ bool fl_take1(const unsigned *(&at)[N], const FlWait &wt, float (&x)[N]) {
     unsigned spins = 0, v[N];
     while (true) {
         unsigned off = 0;
 #pragma unroll
         for (int i = 0; i < N; ++i) v[i] = fl_ld1(at[i]);
 #pragma unroll
-        for (int i = 0; i < N; ++i) { off |= v[i] ^ mark; x[i] = __uint_as_float(v[i] << 16); }
+        for (int i = 0; i < N; ++i) { off |= v[i] ^ wt.mark; x[i] = __uint_as_float(v[i] << 16); }
         if (off < 0x10000u) return true;
-        if (!fl_again(spins)) return false;
+        if (!fl_again(spins, wt)) return false;
     }
 }
 // the values of four words as two pairs of bf16
@@ -115,27 +127,27 @@ struct FlRows {
     const unsigned *y;                                                // the sequence's row
     unsigned *o;                                                      // the head's words
     int d, H, h;
-    unsigned mark;
+    const FlWait &wt;
     bool &lost, &alive;
     __device__ __forceinline__ bool between() const { return true; }
     __device__ __forceinline__ void vec(int which, int lane, float (&x)[D / 32]) const {
         const unsigned *at[D / 32];
 #pragma unroll
         for (int i = 0; i < D / 32; ++i) at[i] = y + which * d + h * D + lane + 32 * i;
-        if (!fl_take1(at, mark, x)) lost = true;
+        if (!fl_take1(at, wt, x)) lost = true;
     }
     __device__ __forceinline__ void scalars(float &dec, float &g) const {
         const unsigned *at[2] = {y + 3 * d + h, y + 3 * d + H + h};
         float x[2];
-        if (!fl_take1(at, mark, x)) lost = true;
+        if (!fl_take1(at, wt, x)) lost = true;
         dec = x[0]; g = x[1];
     }
     __device__ __forceinline__ bool sync() const { alive = __syncthreads_or(lost) == 0; return alive; }
-    __device__ __forceinline__ void put(int j, float v) const { fl_put(o + j, v, mark); }
+    __device__ __forceinline__ void put(int j, float v) const { fl_put(o + j, v, wt.mark); }
 };
 
 // rows of z in shared memory as they were exchanged; false: the wait ran out (the same for the whole CTA)
-__device__ __forceinline__ bool fl_rows(const unsigned *src, int n, unsigned mark, uint4 *zs, bool lost) {
+__device__ __forceinline__ bool fl_rows(const unsigned *src, int n, const FlWait &wt, uint4 *zs, bool lost) {
     for (int base = 0; base < n / 4 && !lost; base += 4 * DT_THREADS) {
         const unsigned *at[4];
         unsigned want = 0;
@@ -145,7 +157,7 @@ __device__ __forceinline__ bool fl_rows(const unsigned *src, int n, unsigned mar
             at[i] = src + 4 * (base + i * DT_THREADS + threadIdx.x);
             if (base + i * DT_THREADS + threadIdx.x < n / 4) want |= 1u << i;
         }
-        lost = !fl_take4(at, want, mark, v);
+        lost = !fl_take4(at, want, wt, v);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (want >> i & 1u) reinterpret_cast<uint2 *>(zs)[base + i * DT_THREADS + threadIdx.x] = fl_pairs(v[i]);
@@ -157,7 +169,7 @@ struct FlNorm { int kind; float eps; const __nv_bfloat16 *w, *b; };
 
 // The residual stream xs += what src holds (first: xs = E[tok] + P[pos]), rounded, and z = norm(xs); warps are dealt to the rows as in
 // decode_token.cu and every sum is formed in its order. A thread only meets its own pieces of xs.
-__device__ __forceinline__ bool fl_norm_rows(const FlArgs &a, const unsigned *src, const FlNorm &nm, unsigned mark, uint4 *xs, uint4 *zs,
+__device__ __forceinline__ bool fl_norm_rows(const FlArgs &a, const unsigned *src, const FlNorm &nm, const FlWait &wt, uint4 *xs, uint4 *zs,
                                              float (*part)[DT_WARPS], bool lost) {
     const int K = a.d, K8 = K >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wpr = a.B == 1 ? DT_WARPS : (a.B == 2 ? DT_WARPS / 2 : DT_WARPS / 4);
@@ -199,7 +211,7 @@ __device__ __forceinline__ bool fl_norm_rows(const FlArgs &a, const unsigned *sr
                 const unsigned *r0 = src + (size_t)b * K + 8 * k0, *r1 = r0 + 8 * stride;
                 const unsigned *at[4] = {r0, r0 + 4, r1, r1 + 4};
                 uint4 v[4];
-                lost = !fl_take4(at, (k0 < K8 ? 3u : 0u) | (k1 < K8 ? 12u : 0u), mark, v);
+                lost = !fl_take4(at, (k0 < K8 ? 3u : 0u) | (k1 < K8 ? 12u : 0u), wt, v);
                 if (k0 < K8) {
                     const uint2 lo = fl_pairs(v[0]), hi = fl_pairs(v[1]);
                     add(k0, xs[b * K8 + k0], make_uint4(lo.x, lo.y, hi.x, hi.y));
@@ -458,6 +470,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) decode_flow_kernel(FlArgs a) {
     }
     __syncthreads();
     const unsigned mark = s_mark;
+    const FlWait wt{mark, reinterpret_cast<unsigned *>(a.sync + 1)};
     FlQueue q{0, (int)blockIdx.x * kinds[0].run, 0, 0, 0, 0, 0, 0u, smem_u32(fl_smem), smem_u32(bars)};
     if (tid == 0)
 #pragma unroll 1
@@ -492,7 +505,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) decode_flow_kernel(FlArgs a) {
             out = y;
             // the state of this CTA's (sequence, head) is on its way while the projection is formed (at head dim 128 it is 64 registers a thread: not held)
             if (D == 64 && blockIdx.x < a.B * a.H) held.request(da, blockIdx.x / a.H, blockIdx.x % a.H);
-            alive = fl_norm_rows(a, p == 0 ? nullptr : d2 - per, FlNorm{ly.ln_kind, ly.ln_eps, ly.ln_w, ly.ln_b}, mark, xs, zs, part[0], lost);
+            alive = fl_norm_rows(a, p == 0 ? nullptr : d2 - per, FlNorm{ly.ln_kind, ly.ln_eps, ly.ln_w, ly.ln_b}, wt, xs, zs, part[0], lost);
         } else if (kd == 1) {
             // the recurrent state step, one (sequence, head) per CTA
             out = d1;
@@ -501,16 +514,16 @@ __global__ void __launch_bounds__(DT_THREADS, 1) decode_flow_kernel(FlArgs a) {
                 const int b = bh / a.H, h = bh % a.H;
                 if (D != 64 || bh != blockIdx.x) held.request(da, b, h);
                 held.constants();
-                decode_step_body<D, DELTA>(da, b, h, held, FlRows<D>{y + (size_t)b * a.NP, o + (size_t)b * a.d + h * D, a.d, a.H, h, mark, lost, alive});
+                decode_step_body<D, DELTA>(da, b, h, held, FlRows<D>{y + (size_t)b * a.NP, o + (size_t)b * a.d + h * D, a.d, a.H, h, wt, lost, alive});
                 __syncthreads();
             }
-            if (alive && works) alive = fl_rows(o, a.B * a.d, mark, zs, lost);
+            if (alive && works) alive = fl_rows(o, a.B * a.d, wt, zs, lost);
         } else if (kd == 2) {
             out = hm;
-            alive = fl_norm_rows(a, d1, FlNorm{ly.n_kind, ly.n_eps, ly.n_w, ly.n_b}, mark, xs, zs, part[1], lost);
+            alive = fl_norm_rows(a, d1, FlNorm{ly.n_kind, ly.n_eps, ly.n_w, ly.n_b}, wt, xs, zs, part[1], lost);
         } else {
             out = d2;
-            if (works) alive = fl_rows(hm, a.B * a.dff, mark, zs, lost);
+            if (works) alive = fl_rows(hm, a.B * a.dff, wt, zs, lost);
         }
         if (alive) {
             if (works) { q.freed += q.used; q.used = 0; }             // the rows' barriers are behind every warp's last run
@@ -541,14 +554,23 @@ __global__ void __launch_bounds__(DT_THREADS, 1) decode_flow_kernel(FlArgs a) {
     // ---- final norm and the tied head
     if (alive) {
         const unsigned *d2 = a.words + (size_t)(a.L - 1) * per + a.B * (a.NP + 2 * a.d);
-        alive = fl_norm_rows(a, d2, FlNorm{a.fn_kind, a.fn_eps, a.fn_w, a.fn_b}, mark, xs, zeven, part[0], lost);
+        alive = fl_norm_rows(a, d2, FlNorm{a.fn_kind, a.fn_eps, a.fn_w, a.fn_b}, wt, xs, zeven, part[0], lost);
     }
     if (tid == 0) {
-        // this CTA has read the position and the shift for the last time; the last one to say so leaves them as the next token needs them
+        // this CTA has read the position and the shift for the last time, and waits for no more words; the last one to say so leaves them as
+        // the next token needs them
+        if (!alive) {                                                 // a wait for weights may have run out unseen by the other CTAs
+            atomicExch(wt.given_up, 1u);
+            __threadfence();
+        }
         const unsigned long long c = atomicAdd(a.sync, 1ull) + 1ull;
-        if (alive && a.window > 0 && c % gridDim.x == 0ull) {
-            a.pos[0] = (a.pos[0] + 1) % a.window;
-            a.shift[0] = 1.f;
+        if (c % gridDim.x == 0ull) {
+            if (alive && a.window > 0) {
+                a.pos[0] = (a.pos[0] + 1) % a.window;
+                a.shift[0] = 1.f;
+            }
+            __threadfence();
+            atomicExch(wt.given_up, 0u);
         }
     }
     if (alive) {
@@ -579,6 +601,29 @@ __global__ void __launch_bounds__(DT_THREADS, 1) decode_flow_kernel(FlArgs a) {
             q.parity ^= 1u << q.buf;
             q.buf = q.buf + 1 == DT_DEPTH ? 0 : q.buf + 1;
         }
+}
+
+// The waits' failure path on its own: one CTA as the first launch of a pair. Its first warp looks for 128 words, `limit` times or up to 63 more;
+// its second writes them `late` cycles from the start (late < 0: never), and the kernel returns normally either way.
+__global__ void __launch_bounds__(64) decode_flow_wait_selftest_kernel(unsigned *words, unsigned long long *sync, unsigned limit, long long late) {
+    const int lane = threadIdx.x & 31;
+    const FlWait wt{1u << 16, reinterpret_cast<unsigned *>(sync + 1), limit};
+    if (threadIdx.x < 32) {
+        const unsigned *at[1] = {words + 4 * lane};
+        uint4 v[1];
+        fl_take4(at, 1u, wt, v);
+    } else if (late >= 0) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < late) {}
+        for (int i = 0; i < 4; ++i) fl_put(words + 4 * lane + i, (float)i, wt.mark);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(sync, 1ull);
+}
+
+int decode_flow_wait_selftest_launch(unsigned *words, unsigned long long *sync, unsigned limit, long long late, cudaStream_t stream) {
+    decode_flow_wait_selftest_kernel<<<1, 64, 0, stream>>>(words, sync, limit, late);
+    return check_launch("decode_flow_wait_selftest_kernel");
 }
 
 int decode_flow_error_flag(int *out) {

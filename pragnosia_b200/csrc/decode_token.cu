@@ -39,7 +39,7 @@ struct DtArgs {
     const float *shift;
     __nv_bfloat16 *xa, *xb, *y, *o, *hmid, *dl;
     float *logits;
-    unsigned long long *sync;                                         // [0] arrivals, [1] reserved
+    unsigned long long *sync;                                         // [0] arrivals, [1] not zero once a wait has been given up
     int L, B, d, H, NP, dff, V, ctx, fn_kind;
     int window;                                                       // > 0: leave pos and shift as the next token needs them
     float fn_eps;
@@ -48,7 +48,7 @@ struct DtArgs {
 // Grid-wide barrier number gen + 1 (every CTA passes the same barriers in the same order), in two halves so that work which
 // does not depend on the other CTAs can sit between them. Arrive: one fire-and-forget add to the arrival counter once the
 // whole CTA has written its results. Wait: polls of the counter itself; false when the wait ran out (or another CTA's
-// did): the flag is up and the kernel winds down.
+// did): the kernel winds down, and the flag is up for the host.
 __device__ __forceinline__ void dt_arrive(unsigned long long *sync) {
     __syncthreads();
     // release: this CTA's writes (ordered before this by the CTA barrier above) are visible to whoever sees the count
@@ -65,7 +65,8 @@ __device__ __forceinline__ bool dt_wait(unsigned long long *sync, unsigned long 
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(sync) : "memory");
             if (c >= target) break;
             ++spins;
-            if (spins > limit || ((spins & 63u) == 0u && *reinterpret_cast<volatile int *>(&g_dt_error) != 0)) {
+            if (spins > limit || ((spins & 63u) == 0u && *reinterpret_cast<volatile unsigned long long *>(sync + 1) != 0)) {
+                atomicExch(sync + 1, 1ull);                           // seen by this pair of words' launches only
                 atomicExch(&g_dt_error, 81);
                 alive = 0;
                 break;

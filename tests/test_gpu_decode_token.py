@@ -118,7 +118,40 @@ def test_a_barrier_wait_that_runs_out_raises_the_flag_and_returns():
     rc = _lib.lib().pgb_decode_token_wait_selftest(ctypes.c_void_p(sync.data_ptr()), 2000, None)
     assert rc == 0
     torch.cuda.synchronize()
-    assert sync[0].item() == 1                                        # it did arrive
+    assert sync.tolist() == [1, 1]                                    # it did arrive, and gave up
     assert healthy() == 81 and healthy() == 0                         # reported once, then clear
     x = torch.ones(8, device=DEV)                                     # the context is still usable
     assert (x + 1).sum().item() == 16
+
+
+def test_a_wait_for_words_that_runs_out_ends_its_own_launch_only():
+    """The step without barriers: a wait that nothing serves raises the flag and returns; while the flag is up, a wait of another pair
+    that takes some hundred looks is served all the same, and a model's step is what it was."""
+    import ctypes
+    assert healthy() == 0
+    m, _, _ = small_lm("aspin", "rms", torch.bfloat16)
+    ids = synth.token_ids(1, 40, 256, seed=5).to(DEV)
+
+    def steps():
+        dec = Decoder(m, batch=1)
+        dec.prefill(ids[:, :36])
+        out = torch.stack([dec.step(ids[:, t]).clone() for t in range(36, 40)])
+        assert dec._plan["flow"]
+        return out
+
+    def wait(limit, late):
+        words, sync = torch.zeros(128, dtype=torch.int32, device=DEV), torch.zeros(2, dtype=torch.int64, device=DEV)
+        rc = _lib.lib().pgb_decode_flow_wait_selftest(ctypes.c_void_p(words.data_ptr()), ctypes.c_void_p(sync.data_ptr()), limit, late, None)
+        assert rc == 0
+        torch.cuda.synchronize()
+        return words, sync.tolist()
+
+    want = steps()
+    words, sync = wait(2000, -1)
+    assert sync == [1, 1] and not words.any()
+    words, sync = wait(1 << 20, 1_000_000)                            # half a millisecond: far more than 64 looks
+    assert sync == [1, 0] and bool((words >> 16 == 1).all())
+    assert torch.equal(steps(), want)
+    assert healthy() == 82 and healthy() == 0                         # reported once, then clear
+    L, one = _lib.lib(), ctypes.c_void_p(16)
+    assert L.pgb_decode_flow_wait_selftest(one, one, 0, 0, None) == 2 and L.pgb_decode_flow_wait_selftest(None, one, 1, 0, None) == 1
