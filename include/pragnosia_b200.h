@@ -61,9 +61,12 @@ int pgb_lambda_scan_fwd_ex(const float *u, const float *logmag, const float *ang
                            long long ang_stride_t, const float *h0r, const float *h0i, float *y, float *hr_out,
                            float *hi_out, int B, int T, int D, int time_segments, void *stream);
 
-/* The number of time segments a warp scans in parallel that pgb_lambda_scan_fwd picks for this shape on a GPU with
- * sm_count multiprocessors (host arithmetic only; 0 for a bad shape): more segments when channels are too few to fill the
- * GPU, never more than the sequence has pieces to hand out. No counterpart in the reference. */
+/* The time_segments that pgb_lambda_scan_fwd_ex is estimated to run this shape fastest with on a GPU with sm_count multiprocessors, for an angle
+ * per token and pointers aligned as D allows (host arithmetic only; 0 for a bad shape): more when channels are too few to fill
+ * the GPU, never more than the sequence has pieces of four steps to hand out, rounded up to a power of two. pgb_lambda_scan_fwd takes
+ * this number too, with two exceptions: where D is a multiple of four a walk of a few tiles may take segments of two steps,
+ * up to twice as many, and an angle per channel is weighed by its own traffic. Either way the choice depends on the sizes, the alignment and the angle's form
+ * alone, so pgb_lambda_scan_fwd and pgb_lambda_scan_fwd_train give the same bits. No counterpart in the reference. */
 int pgb_lambda_scan_time_segments(int B, int T, int D, int sm_count);
 
 /* The same forward pass for a caller that will differentiate through it: additionally stores Im h_t for every token

@@ -39,7 +39,7 @@ int prefix_scan_bwd_launch(const void *, const void *, int, const float *, const
                            float *, float *, float *, float *, int, int, int, cudaStream_t);
 int key_topk_launch(void *, int, long long, long long, long long, int, int, int, int, int, cudaStream_t);
 int short_conv_launch(const void *, int, long long, long long, const void *, const void *, void *, void *, int, int, int, int, cudaStream_t);
-int lambda_scan_pick_ts(int B, int T, int D, int vec, int sms, int force_ts);
+int lambda_scan_pick_ts(int B, int T, int D, int sms);
 int prep_launch(const void *, const void *, const void *, int, long long, long long, long long, const void *, long long,
                 long long, const float *, const long long *, void *, void *, void *, int, int, int, int, int, cudaStream_t);
 int prefill_fp32_launch(const PrefillArgs &, int, int, int, cudaStream_t);
@@ -189,7 +189,7 @@ int pgb_lambda_scan_bwd(const float *g, const float *u, const float *logmag, con
 
 int pgb_lambda_scan_time_segments(int B, int T, int D, int sm_count) {
     if (B <= 0 || T <= 0 || D <= 0 || sm_count <= 0) return 0;
-    return lambda_scan_pick_ts(B, T, D, (D % 4 == 0) ? 4 : 1, sm_count, 0);
+    return lambda_scan_pick_ts(B, T, D, sm_count);
 }
 
 int pgb_aspin_prep_bwd_tiles(int T) { return T > 0 ? prep_bwd_tiles(T) : 0; }

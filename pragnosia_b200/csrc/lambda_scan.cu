@@ -532,26 +532,29 @@ static LsPick ls_pick(int B, int T, int D, int vec, const LsCost &k, int sms) {
     return best;
 }
 // brief: half the steps a tile, requested a tile ahead into registers, at four fifths of the slots' pace once the memory is loaded
-static LsCost ls_cost_fwd(bool bcast, bool keep, bool brief) {
-    const double ps = 3.2 - (bcast ? 0.8 : 0.0) + (keep ? 0.8 : 0.0);
+static LsCost ls_cost_fwd(bool bcast, bool brief) {
+    const double ps = bcast ? 2.4 : 3.2;
     return brief ? LsCost{bcast ? 0.45 : 0.6, 1.25 * ps, 3.0, false, 2} : LsCost{1.2, ps, 3.0, false, LS_SEG};
 }
-int lambda_scan_pick_ts(int B, int T, int D, int vec, int sms, int force_ts) {
-    return force_ts > 0 ? force_ts : ls_pick(B, T, D, vec, ls_cost_fwd(false, false, false), sms).ts;
+// Segments and form of a forward call: from its sizes and the angle's form only. A pass that also writes Im h for a backward moves a quarter
+// more bytes, for which another choice would now and then be the estimate's best (7 % of shapes, 0.3 % of the time on average, 11 to 19 at most),
+// but it takes the same one, so that a sequence gives the same bits in training and in inference.
+struct LsForward { int ts; bool brief; };
+static LsForward ls_choose_fwd(int B, int T, int D, int vec, bool bcast, int sms) {
+    const LsPick slots = ls_pick(B, T, D, vec, ls_cost_fwd(bcast, false), sms);
+    if (vec != 4) return {slots.ts, false};
+    const LsPick brief = ls_pick(B, T, D, vec, ls_cost_fwd(bcast, true), sms);
+    return brief.cost < slots.cost ? LsForward{brief.ts, true} : LsForward{slots.ts, false};
 }
+// the number to ask for by force_ts, whose segments have LS_SEG steps: an angle per token, rows aligned as D allows
+int lambda_scan_pick_ts(int B, int T, int D, int sms) { return ls_pick(B, T, D, ls_vec(D, 0, 0), ls_cost_fwd(false, false), sms).ts; }
 
 int lambda_scan_launch(const float *u, const float *lm, const float *an, long long sb, long long st, const float *h0r,
                        const float *h0i, float *y, float *hro, float *hio, float *hia, int B, int T, int D, int force_ts,
                        cudaStream_t stream) {
-    const int vec = ls_vec(D, sb, st, u, lm, an, y, hia, hro, hio, h0r, h0i), sms = sm_count();
-    const bool bcast = sb == 0 && st == 0, keep = hia != nullptr;
-    LsPick pick = force_ts > 0 ? LsPick{force_ts, 0.0} : ls_pick(B, T, D, vec, ls_cost_fwd(bcast, keep, false), sms);
-    bool brief = false;
-    if (force_ts <= 0 && vec == 4) {
-        const LsPick other = ls_pick(B, T, D, vec, ls_cost_fwd(bcast, keep, true), sms);
-        if (other.cost < pick.cost) { pick = other; brief = true; }
-    }
-    return launch_any(vec, pick.ts, LsArgs{u, lm, an, sb, st, h0r, h0i, y, hro, hio, hia, B, T, D, brief}, stream);
+    const int vec = ls_vec(D, sb, st, u, lm, an, y, hia, hro, hio, h0r, h0i);
+    const LsForward f = force_ts > 0 ? LsForward{force_ts, false} : ls_choose_fwd(B, T, D, vec, sb == 0 && st == 0, sm_count());
+    return launch_any(vec, f.ts, LsArgs{u, lm, an, sb, st, h0r, h0i, y, hro, hio, hia, B, T, D, f.brief}, stream);
 }
 
 int lambda_scan_bwd_launch(const float *g, const float *u, const float *lm, const float *an, long long sb, long long st,

@@ -1,11 +1,11 @@
 """The forms the lambda scan, the prep backward and the fp32 chunked prefill choose between, at the edges of their ranges, against
-the fp64 definitions: lanes of 4, 2 or 1 channels, the form with many warps and the one that loads ahead, angles past the range
+the fp64 definitions: lanes of 4, 2 or 1 channels, tiles through slots in shared memory and through registers, angles past the range
 of the fast sin/cos; rows read 16 bytes at a time or not."""
 import pytest
 import torch
 
 import oracle.carrier_oracle as oracle
-from pragnosia_b200 import ops, synth
+from pragnosia_b200 import _lib, ops, synth
 from pragnosia_b200._lib import PREFILL_FP32
 
 pytestmark = pytest.mark.gpu
@@ -36,6 +36,31 @@ def test_lambda_scan_and_adjoint_forms(B, T, D, per_channel):
         ref = oracle.lambda_scan_grads(u, lm, an, h0, w, torch.zeros(B, D, device=DEV), torch.zeros(B, D, device=DEV))
         for a, b in zip(d, ref):
             assert rel(a, b) < 2e-5
+
+
+# shapes for which a pass that also writes Im h would by its own bytes be given other segments, or the other form
+@pytest.mark.parametrize("B,T,D,per_channel", [
+    (18, 65, 91, False), (4, 74, 305, False), (16, 88, 326, False), (21, 56, 180, False), (16, 115, 384, False),
+    (22, 34, 159, True), (6, 72, 231, True), (16, 83, 158, True), (18, 53, 292, True), (11, 407, 144, True)])
+def test_training_and_inference_give_the_same_bits(B, T, D, per_channel):
+    g = torch.Generator(device=DEV).manual_seed(D)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    u, lm, h0 = r(B, T, D), -r(B, T, D).abs(), (r(B, D), r(B, D))
+    an = r(1, 1, D).expand(B, T, D) if per_channel else r(B, T, D)
+    y, (hr, hi), _ = ops.lambda_scan(u, lm, an, h0, keep_imag=True)
+    y0, (hr0, hi0) = ops.lambda_scan(u, lm, an, h0)
+    assert torch.equal(y, y0) and torch.equal(hr, hr0) and torch.equal(hi, hi0)
+
+
+@pytest.mark.parametrize("B,T,D", [(2, 100, 766), (2, 1000, 766), (64, 256, 256), (3, 200, 65)])    # lanes of two channels, of four, of one
+def test_the_segments_the_library_names_are_those_it_takes(B, T, D):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    u, lm, an = r(B, T, D), -r(B, T, D).abs(), r(B, T, D)
+    ts = _lib.lib().pgb_lambda_scan_time_segments(B, T, D, torch.cuda.get_device_properties(0).multi_processor_count)
+    y, (hr, hi) = ops.lambda_scan(u, lm, an)
+    y0, (hr0, hi0) = ops.lambda_scan(u, lm, an, time_segments=ts)
+    assert torch.equal(y, y0) and torch.equal(hr, hr0) and torch.equal(hi, hi0)
 
 
 @pytest.mark.parametrize("ts", [1, 4, 32])
