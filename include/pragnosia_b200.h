@@ -191,7 +191,9 @@ int pgb_aspin_prefill_fwd(const void *q, const void *k, const void *v, int io_dt
 
 /* The plain rule on bf16 operands at D = 64 with scratch (pgb_aspin_prefill_segments_scratch_bytes bytes; 0: the sequences are too
  * short, or the chains fill the GPU evenly, and pgb_aspin_prefill_fwd is the call): the same arithmetic with chains cut into segments
- * that run side by side -- all of them where they leave the GPU half empty, those of the last round where that leaves it so. S_out must not be S0. */
+ * that run side by side -- all of them where they leave the GPU half empty, those of the last round where that leaves it so. S_out must not be S0.
+ * A cut chain combines its state in another order (fp32) and rounds it at other places. Where only the last round is cut, that is the last rows of
+ * the batch: a sequence's result then differs in rounding with its row, as it does with the size of the batch. */
 long long pgb_aspin_prefill_segments_scratch_bytes(int B, int H, int T, int D);
 int pgb_aspin_prefill_segments_fwd(const void *q, const void *k, const void *v, const float *la, const float *S0, const float *theta,
                                    const float *shift_dev, float shift_host, void *o, int o_dtype, float *S_out, void *sent, void *scratch,

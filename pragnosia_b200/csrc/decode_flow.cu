@@ -2,7 +2,9 @@
 // barriers between its phases: every value that one CTA hands to another carries the mark of the launch it belongs to.
 //
 // The phases are those of decode_token.cu -- per layer projection, state step, output projection, MLP up, MLP down; the tied head
-// at the end -- and so are the roundings and the order of every sum. There, a phase ends with a grid-wide barrier: the results are
+// at the end -- and so are the roundings, and the order of every sum but one kind's: rows of the output projection or the MLP's second layer
+// that are few and long (the latter at K 3072, N 768) are shared across a CTA's eight warps, whose fp32 sums are added in warp order. A
+// bf16 rounding may then fall the other way. There, a phase ends with a grid-wide barrier: the results are
 // made visible (a release), counted (148 additions to one word), the count is seen (a round trip), and only then are the
 // results fetched (another): 3.7 us a phase, 61 phases a token. Here an exchanged value is a 32-bit word, the bf16
 // value in the low half and the launch's mark in the high half, written and read with relaxed accesses of that size or vectors of them. A consumer

@@ -154,7 +154,9 @@ def prefill(q, k, v, la, beta=None, S0=None, theta=None, shift=0.0, want_sent: b
             precision: int = _lib.PREFILL_AUTO, out_dtype=None, S_out=None):
     """Chunked prefill. q,k,v (B,H,T,D) fp32 or bf16 (same dtype); la (B,H,T); beta (B,H,T) or None (plain rule);
     S0 (B,H,D,D) or None.  theta/shift: rebase S0's key axis by -shift*theta first (shift: number or 0-d CUDA tensor).
-    Returns (o in out_dtype (default q's dtype), S fp32, sent bf16 (B,H,NC,D,D) or None)."""
+    Returns (o in out_dtype (default q's dtype), S fp32, sent bf16 (B,H,NC,D,D) or None).
+    Plain rule, bf16, D = 64: long chains that would leave SMs idle are cut into segments, which round their states at other places; where
+    B*H is past the SM count, those are the last rows' only, so equal sequences in one batch may differ in rounding."""
     theta, shift_dev, shift_host = _shift_args(theta, S0, shift)
     if not _compiling():
         return host().prefill(q, k, v, la, beta, S0, theta, shift_dev, shift_host, want_sent, precision,

@@ -1,6 +1,7 @@
-"""The decode step as ONE launch per token (decode_token.cu) against the same step chained from this library's separate
-kernels (five launches a layer), whose parity with the oracle the model tests pin: same roundings, same accumulation
-order, so logits and states are compared at a few bf16 ulps, ids exactly."""
+"""The decode step as ONE launch per token (decode_flow.cu; decode_token.cu, with barriers, where it is asked for) against the same step
+chained from this library's separate kernels (five launches a layer), whose parity with the oracle the model tests pin: same roundings,
+sums of the same fp32 products in an order that the row length decides, so logits and states are compared at a few bf16 ulps. Ids are
+exact between graph and eager launches of one step."""
 import pytest
 import torch
 
@@ -39,7 +40,7 @@ def test_one_launch_step_matches_the_chained_kernels(mixer, norm, B):
         close(lg, ref_lg, 2e-2, f"logits one-launch={key[0]} graph={key[1]}")
         for a, b in zip(S, ref_S):
             close(a, b, 5e-3, f"state one-launch={key[0]} graph={key[1]}")
-    # the one-launch step repeats the chained kernels' arithmetic: most logits agree to the bit
+    # rows this short are summed in the chained kernels' order: most logits agree to the bit
     same = (outs[(True, True)][0] == ref_lg).float().mean().item()
     assert same > 0.9, same
     assert healthy() == 0
