@@ -1,11 +1,12 @@
 // Per-token complex recurrence h_t = lambda_t h_{t-1} + u_t as a chunked parallel scan, and its adjoint.
 //
 // Layout in HBM: u, logmag, y are [B][T][D] fp32 with D contiguous: 12 B read (8 B when the angle is one value per
-// channel) and 4 B written per (b,t,d) element. What bounds it is memory: the bytes move at 4.9 TB/s (0.75 of a copy; the adjoint, nine
-// streams, 5.2) with a tile's loads in flight under the arithmetic of the one before. e^x, sin, cos and
-// the recurrence run on pairs of channels (scan_math.cuh, 68 instructions an element, 50 with one angle per channel). B64 T4096 D768:
-// 760 us with loads ahead of their use but inside the tile, 660 with the slots below (one angle per channel 587 -> 447); B16 T4096 D768
-// 253 -> 200 (199 -> 141).
+// channel) and 4 B written per (b,t,d) element. What bounds it is the SM's arithmetic: a tile's loads fly under the arithmetic of the one
+// before, and pairs of channels (e^x, sin, cos and the recurrence, scan_math.cuh: 68 instructions an element, 50 with one angle per channel) keep
+// the FMA pipe two cycles each, so the time goes with the SM clock. B64 T4096 D768: 660 us at 1965 MHz (4.9 TB/s, 0.74 of a copy; the adjoint, nine
+// streams, 5.2), 735 to 760 once the chip's power limit has taken the clock to 1610 - 1690 MHz, which some 50 ms of such calls do (one angle per
+// channel 440 and 500). At the full clock, with loads ahead of their use but inside the tile 760, with the slots below 660 (one angle per
+// channel 587 -> 447); B16 T4096 D768 253 -> 200 (199 -> 141).
 //
 // Work split. A lane owns VEC adjacent channels (4 where D, pointers and strides allow: one 128-bit access; else 2 or 1). A warp is TS time-segments x CQ
 // channel groups (TS * CQ = 32): lanes of one segment read 16*CQ contiguous bytes of one time row, so every 128-byte
