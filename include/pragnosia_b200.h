@@ -431,6 +431,25 @@ int pgb_batch_linear_ex(const void *x, const void *W, const void *bias, void *y,
                         int parts_in, const float *c1, const float *c2, int norm_kind, float eps, const void *resid, float *row_sums_out,
                         int flags, void *stream);
 int pgb_batch_linear_parts(int N);
+/* The linear layers of a batch's decode step as links of a chain of programmatic dependents, RMS norms and residual adds inside them
+ * (bf16, B <= 64 rows, N and K multiples of 8, W [N][K]):
+ *   x [B][K]. With squares_in [B][parts_in] (the parts of each row's sum of squares) x is the residual stream times the weight of the norm
+ *   ahead, and the layer is  v = r (x W^T) + bias,  r = 1 / sqrt(sum / K + eps); without, v = x W^T + bias. v is rounded to bf16; then
+ *   y [B][N] = v, or its erf-GELU (act 1); or logits [B][N] fp32 = v (y NULL);
+ *   or with resid [B][N]: y = resid + v, the new residual stream; yw = y next_w (next_w [N]: the weight of the norm behind); and
+ *   squares_out [B][pgb_decode_linear_parts(N, K)].
+ *   window > 0: the launch also leaves pos = (pos + 1) mod window and shift = 1, for the last layer of a token.
+ * Whether a layer is taken depends on K alone (256 at least): pgb_decode_linear_takes(kind 0 plain or activation, 1 residual, 2 logits; N, K).
+ * pgb_decode_embed_norm is such a token's first kernel: x = E[tok] + P[pos], xw = x next_w and squares [B] (one part).
+ * Every kernel of the chain requests W, bias and next_w before it waits for the one ahead: they are complete before the token's first kernel is
+ * launched. A wait that runs out: pgb_tc_error_flag reads 78 or 79. */
+int pgb_decode_embed_norm(const long long *tok, const long long *pos, const void *E, const void *P, const void *next_w, void *x, void *xw,
+                          float *squares, int B, int d, int vocab, int ctx, void *stream);
+int pgb_decode_linear_takes(int kind, int N, int K);
+int pgb_decode_linear_parts(int N, int K);
+int pgb_decode_linear(const void *x, const void *W, const void *bias, const float *squares_in, int parts_in, float eps, int act, const void *resid,
+                      const void *next_w, void *y, void *yw, float *squares_out, float *logits, long long *pos, float *shift, int window, int B,
+                      int N, int K, void *stream);
 int pgb_decode_embed_ex(const long long *tok, const long long *pos, const void *E, const void *P, void *x, float *row_sums, int B, int d,
                         int vocab, int ctx, void *stream);
 
@@ -558,6 +577,16 @@ int pgb_aspin_decode_step(const void *qp, const void *kp, const void *vp, int in
                           const float *shift_dev, float shift_host, const float *S_in, float *S_out,
                           const float *rms_weight, float rms_eps, void *o, int out_dtype, long long out_stride_b,
                           int B, int H, int D, void *stream);
+/* The same with flags. PGB_DECODE_STATE_EARLY: S_in, theta, decay_A, rms_weight and the word at shift_dev are complete before the kernel ahead on the
+ * stream is launched, and no kernel that may still run writes them (as between the layers of a token whose first kernel is pgb_decode_embed_norm):
+ * they are read ahead of the wait on that kernel. */
+enum { PGB_DECODE_STATE_EARLY = 1 };
+int pgb_aspin_decode_step_ex(const void *qp, const void *kp, const void *vp, int in_dtype, long long in_stride_b,
+                             int normalize, const void *gate, long long gate_stride_b, int gate_is_logit, int delta,
+                             const void *decay, long long decay_stride_b, const float *decay_A, const float *theta,
+                             const float *shift_dev, float shift_host, const float *S_in, float *S_out,
+                             const float *rms_weight, float rms_eps, void *o, int out_dtype, long long out_stride_b,
+                             int B, int H, int D, int flags, void *stream);
 
 /* Which kernel pgb_aspin_decode_step uses at head dim 64: 0 (default) = from 512 (sequence, head) pairs up one warp per
  * pair, a lane owning two value columns of all key rows (no block barrier, no partial sums through shared memory), below

@@ -63,6 +63,10 @@ SIGNATURES = {
     "pgb_batch_linear_ex": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _i, _vp, _vp, _i, _f, _vp, _vp, _i, _vp],
     "pgb_batch_linear_parts": [_i],
     "pgb_decode_embed_ex": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
+    "pgb_decode_embed_norm": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
+    "pgb_decode_linear_takes": [_i, _i, _i],
+    "pgb_decode_linear_parts": [_i, _i],
+    "pgb_decode_linear": [_vp, _vp, _vp, _vp, _i, _f, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "pgb_decode_advance": [_vp, _vp, _i, _vp],
     "pgb_decode_token_work_bytes": [_i, _i, _i, _i],
     "pgb_decode_token_wait_selftest": [_vp, _ll, _vp],
@@ -102,6 +106,8 @@ SIGNATURES = {
     "pgb_short_conv_fwd": [_vp, _i, _ll, _ll, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "pgb_aspin_decode_step": [_vp, _vp, _vp, _i, _ll, _i, _vp, _ll, _i, _i, _vp, _ll, _vp, _vp, _vp, _f, _vp, _vp, _vp,
                               _f, _vp, _i, _ll, _i, _i, _i, _vp],
+    "pgb_aspin_decode_step_ex": [_vp, _vp, _vp, _i, _ll, _i, _vp, _ll, _i, _i, _vp, _ll, _vp, _vp, _vp, _f, _vp, _vp, _vp,
+                              _f, _vp, _i, _ll, _i, _i, _i, _i, _vp],
 }
 
 _lib = None

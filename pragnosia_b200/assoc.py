@@ -254,7 +254,7 @@ class AssocCarrier(nn.Module):
             bt = bt.clamp(min=0.75)                                   # beta = 1 makes the chunk inverse singular
         return bt
 
-    def _step(self, qp, kp, vp, a_logit, g_logit, c, S0, shift, inplace):
+    def _step(self, qp, kp, vp, a_logit, g_logit, c, S0, shift, inplace, early=False):
         """One token per sequence: the fused recurrent step. With an option that changes the gates, the log-decay / write
         strength are formed here and handed over as values instead of logits."""
         B, H, dk, d = qp.shape[0], self.h, self.dk, self.d
@@ -272,20 +272,20 @@ class AssocCarrier(nn.Module):
         o = torch.empty(B, d, device=qp.device, dtype=qp.dtype)
         _, S = ops.decode_step(q3, k3, v3, decay, S0, c["theta"], gate=gate, delta=self.delta, gate_is_logit=is_logit,
                                decay_A=decay_A, normalize=True, shift=shift, rms_weight=c["onw"], rms_eps=self._rms_eps(),
-                               out=o.view(B, H, dk), S_out=S0 if inplace else None)
+                               out=o.view(B, H, dk), S_out=S0 if inplace else None, early=early)
         return o, S
 
-    def step_from_projection(self, y2, S0, shift, inplace: bool | None = None):
+    def step_from_projection(self, y2, S0, shift, inplace: bool | None = None, early: bool = False):
         """The recurrent step of one token per sequence from the fused projection's output y2 (B, 3d+2h[+pad]) =
         [q | k | v | decay logits | gate logits]: one kernel (normalise, gates, rotate the state, write, read, per-head RMS
         norm). Returns (o (B,d), S); with inplace_state the state is updated where it lies. For a layer without options
-        (plain_step)."""
+        (plain_step). early: ops.decode_step's."""
         c = self._consts()
         H, dk, d = self.h, self.dk, self.d
         y3 = y2.unsqueeze(1)
         qp, kp, vp = (y3[..., i * d:(i + 1) * d].unflatten(-1, (H, dk)) for i in range(3))
         return self._step(qp, kp, vp, y3[..., 3 * d:3 * d + H], y3[..., 3 * d + H:3 * d + 2 * H], c, S0, shift,
-                          self.inplace_state if inplace is None else inplace)
+                          self.inplace_state if inplace is None else inplace, early)
 
     def _rot_table(self, T, c):
         """(cos, sin) of position * theta for this layer's window positions (wrapped by pos_wrap when set); rebuilt when

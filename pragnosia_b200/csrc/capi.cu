@@ -69,7 +69,13 @@ size_t prefill_fp32_chunk_scratch_bytes(int B, int H, int T, int D);
 int prefill_fp32_chunk_launch(const PrefillArgs &, int, int, void *, cudaStream_t);
 int rot_table_launch(const float *, float *, int, int, int, cudaStream_t);
 int decode_advance_launch(long long *, float *, int, cudaStream_t);
-int decode_embed_launch(const long long *, const long long *, const void *, const void *, void *, int, int, int, int, float *, cudaStream_t);
+int decode_embed_launch(const long long *, const long long *, const void *, const void *, void *, int, int, int, int, float *, const void *, void *, float *,
+                        cudaStream_t);
+int decode_linear_parts(int N, int K);
+bool decode_linear_takes(int kind, int N, int K);
+int decode_linear_launch(const void *, const void *, const void *, const float *, int, float, int, const void *, const void *, void *, void *, float *,
+                         float *, long long *, float *, int, int, int, int, cudaStream_t);
+int decode_linear_error_flag(int *);
 int decode_sample_launch(const void *, int, float, float, unsigned long long, long long *, long long *, int, long long *, long long *, float *,
                          unsigned int *, int, int, int, cudaStream_t);
 int linear_gelu_launch(const void *, const void *, const void *, void *, long long, int, int, int, cudaStream_t);
@@ -610,7 +616,39 @@ int pgb_decode_embed_ex(const long long *tok, const long long *pos, const void *
     if (B < 1 || d < 8 || (d % 8) != 0 || vocab < 1 || ctx < 1) return PGB_ERR_BAD_SHAPE;
     if (!aligned(E, 16) || !aligned(P, 16) || !aligned(x, 16) || !aligned(tok, 8) || !aligned(pos, 8) || (row_sums && !aligned(row_sums, 8)))
         return PGB_ERR_MISALIGNED;
-    return decode_embed_launch(tok, pos, E, P, x, B, d, vocab, ctx, row_sums, (cudaStream_t)stream);
+    return decode_embed_launch(tok, pos, E, P, x, B, d, vocab, ctx, row_sums, nullptr, nullptr, nullptr, (cudaStream_t)stream);
+}
+
+int pgb_decode_embed_norm(const long long *tok, const long long *pos, const void *E, const void *P, const void *next_w, void *x, void *xw,
+                          float *squares, int B, int d, int vocab, int ctx, void *stream) {
+    if (!tok || !pos || !E || !P || !x || !next_w || !xw || !squares) return PGB_ERR_NULL_POINTER;
+    if (B < 1 || d < 8 || (d % 8) != 0 || vocab < 1 || ctx < 1) return PGB_ERR_BAD_SHAPE;
+    if (!aligned(E, 16) || !aligned(P, 16) || !aligned(x, 16) || !aligned(next_w, 16) || !aligned(xw, 16) || !aligned(squares, 4) || !aligned(tok, 8) ||
+        !aligned(pos, 8))
+        return PGB_ERR_MISALIGNED;
+    return decode_embed_launch(tok, pos, E, P, x, B, d, vocab, ctx, nullptr, next_w, xw, squares, (cudaStream_t)stream);
+}
+
+int pgb_decode_linear_takes(int kind, int N, int K) {
+    return kind >= 0 && kind <= 2 && N >= 8 && N % 8 == 0 && K >= 8 && K % 8 == 0 && decode_linear_takes(kind, N, K) ? 1 : 0;
+}
+int pgb_decode_linear_parts(int N, int K) { return N < 8 || K < 8 ? 0 : decode_linear_parts(N, K); }
+
+int pgb_decode_linear(const void *x, const void *W, const void *bias, const float *squares_in, int parts_in, float eps, int act, const void *resid,
+                      const void *next_w, void *y, void *yw, float *squares_out, float *logits, long long *pos, float *shift, int window, int B,
+                      int N, int K, void *stream) {
+    if (!x || !W || (!y && !logits) || (y && logits)) return PGB_ERR_NULL_POINTER;
+    if ((resid != nullptr) != (next_w != nullptr) || (resid != nullptr) != (yw != nullptr) || (resid != nullptr) != (squares_out != nullptr)) return PGB_ERR_NULL_POINTER;
+    if (resid && logits) return PGB_ERR_BAD_SHAPE;
+    if (window < 0 || (window > 0 && (!pos || !shift))) return window < 0 ? PGB_ERR_BAD_SHAPE : PGB_ERR_NULL_POINTER;
+    if (B < 1 || N < 8 || K < 8 || (N % 8) != 0 || (K % 8) != 0 || act < 0 || act > 1 || (act && (resid || logits)) || (squares_in && parts_in < 1))
+        return PGB_ERR_BAD_SHAPE;
+    if (B > 64 || !decode_linear_takes(resid ? 1 : (logits ? 2 : 0), N, K)) return PGB_ERR_TOO_LARGE;
+    if (!aligned(x, 16) || !aligned(W, 16) || !aligned(bias, 8) || !aligned(squares_in, 4) || !aligned(resid, 8) || !aligned(next_w, 8) || !aligned(y, 8) ||
+        !aligned(yw, 8) || !aligned(squares_out, 4) || !aligned(logits, 16) || !aligned(pos, 8) || !aligned(shift, 4))
+        return PGB_ERR_MISALIGNED;
+    return decode_linear_launch(x, W, bias, squares_in, parts_in, eps, act, resid, next_w, y, yw, squares_out, logits, pos, shift, window, B, N, K,
+                                (cudaStream_t)stream);
 }
 
 int pgb_decode_embed(const long long *tok, const long long *pos, const void *E, const void *P, void *x, int B, int d, int vocab,
@@ -821,6 +859,8 @@ int pgb_tc_error_flag(int *out_host) {
     f = f > g ? f : g;
     if (rc == PGB_OK) rc = decode_flow_error_flag(&g);
     f = f > g ? f : g;
+    if (rc == PGB_OK) rc = decode_linear_error_flag(&g);
+    f = f > g ? f : g;
     e = e > f ? e : f;
     b = b > c ? b : c;
     b = b > d ? b : d;
@@ -903,6 +943,17 @@ int pgb_aspin_decode_step(const void *qp, const void *kp, const void *vp, int in
                           const float *shift_dev, float shift_host, const float *S_in, float *S_out,
                           const float *rms_weight, float rms_eps, void *o, int out_dtype, long long out_stride_b, int B,
                           int H, int D, void *stream) {
+    return pgb_aspin_decode_step_ex(qp, kp, vp, in_dtype, in_stride_b, normalize, gate, gate_stride_b, gate_is_logit, delta, decay, decay_stride_b,
+                                    decay_A, theta, shift_dev, shift_host, S_in, S_out, rms_weight, rms_eps, o, out_dtype, out_stride_b, B, H, D, 0, stream);
+}
+
+int pgb_aspin_decode_step_ex(const void *qp, const void *kp, const void *vp, int in_dtype, long long in_stride_b,
+                          int normalize, const void *gate, long long gate_stride_b, int gate_is_logit, int delta,
+                          const void *decay, long long decay_stride_b, const float *decay_A, const float *theta,
+                          const float *shift_dev, float shift_host, const float *S_in, float *S_out,
+                          const float *rms_weight, float rms_eps, void *o, int out_dtype, long long out_stride_b, int B,
+                          int H, int D, int flags, void *stream) {
+    if (flags & ~PGB_DECODE_STATE_EARLY) return PGB_ERR_BAD_SHAPE;
     if (!qp || !kp || !vp || !decay || !theta || !S_in || !S_out || !o) return PGB_ERR_NULL_POINTER;
     if (delta && !gate) return PGB_ERR_NULL_POINTER;                  // the delta rule needs its beta
     if (!dtype_ok(in_dtype) || !dtype_ok(out_dtype)) return PGB_ERR_BAD_DTYPE;
@@ -913,7 +964,7 @@ int pgb_aspin_decode_step(const void *qp, const void *kp, const void *vp, int in
     if (!aligned(S_in, 16) || !aligned(S_out, 16) || !aligned(qp, esize(in_dtype)) || !aligned(o, esize(out_dtype)))
         return PGB_ERR_MISALIGNED;
     DecodeArgs a{qp, kp, vp, in_stride_b, normalize, gate, gate_stride_b, gate_is_logit, decay, decay_stride_b, decay_A,
-                 theta, shift_dev, shift_host, S_in, S_out, rms_weight, rms_eps, o, out_stride_b, B, H};
+                 theta, shift_dev, shift_host, S_in, S_out, rms_weight, rms_eps, o, out_stride_b, B, H, flags & PGB_DECODE_STATE_EARLY};
     return decode_launch(a, in_dtype, out_dtype, D, delta, (cudaStream_t)stream);
 }
 

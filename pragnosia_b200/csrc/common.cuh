@@ -106,6 +106,7 @@ struct DecodeArgs {
     const float *theta; const float *shift_dev; float shift_host;
     const float *S_in; float *S_out; const float *rms_w; float rms_eps;
     void *o; long long out_sb; int B, H;
+    int early = 0;                                                    // the state, shift and constants are complete before the kernel ahead is launched
 };
 
 }  // namespace pgb

@@ -15,11 +15,11 @@ namespace pgb {
 
 template <typename TIN, typename TOUT, int D, bool DELTA>
 __global__ void __launch_bounds__(DEC_THREADS) decode_step_kernel(DecodeArgs a) {
-    // Launched as a programmatic dependent: nothing is read before the kernel ahead (the projection) has completed, and the
-    // kernel behind (the output projection) may start requesting its weights now.
-    pdl_wait();
+    // Launched as a programmatic dependent: nothing of the kernel ahead (the projection) is read before it has completed -- the state neither, unless
+    // the caller says that no kernel still running writes it -- and the kernel behind (the output projection) may start requesting its weights now.
+    if (!a.early) pdl_wait();
     pdl_launch_dependents();
-    auto ready = [] { return true; };
+    auto ready = [&] { if (a.early) pdl_wait(); return true; };
     const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
     decode_step_body<D, DELTA>(a, b, h, DecodeRows<TIN, TOUT, D, decltype(ready)>{a, b, h, ready});
 }
@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(DEC_THREADS) decode_step_kernel(DecodeArgs a) 
 // shared memory. With enough pairs to fill the SMs with warps (configuration 2's 64 sequences: 768) the step is one round
 // of loads, a few hundred instructions and one round of stores and is a seventh shorter than the block-per-head kernel
 // above with its three barriers; at large batches both run at the HBM rate; with few pairs the block kernel is quicker.
-constexpr int DW_WARPS = 4;                                           // (sequence, head) units per CTA
+constexpr int DW_WARPS = 2;                                           // (sequence, head) units per CTA: small, so that 768 of them spread evenly (four: 3 % a token more)
 
 template <typename TIN, typename TOUT, bool DELTA>
 __global__ void __launch_bounds__(DW_WARPS * 32) decode_step_warp_kernel(DecodeArgs a) {
@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(DW_WARPS * 32) decode_step_warp_kernel(DecodeA
     __shared__ __align__(16) float2 srot[DW_WARPS][D / 2];            // alpha * (cos, sin) of the rebase rotation, per row pair
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int unit = blockIdx.x * DW_WARPS + w;
-    pdl_wait();                                                       // nothing is read before the kernel ahead has completed
+    if (!a.early) pdl_wait();                                         // nothing is read before the kernel ahead has completed
     pdl_launch_dependents();
     if (unit >= a.B * a.H) return;                                    // whole warps leave; the warps of a CTA never meet
     const int b = unit / a.H, h = unit - b * a.H;
@@ -53,6 +53,14 @@ __global__ void __launch_bounds__(DW_WARPS * 32) decode_step_warp_kernel(DecodeA
 #pragma unroll
     for (int i = 0; i < D; ++i) s[i] = __ldcs(Sin + i * (D / 2));
 
+    float sn = 0.f, cs = 1.f;
+    {
+        const float shift = a.shift_dev != nullptr ? *a.shift_dev : a.shift_host;
+        if (shift != 0.f) sincosf(-shift * a.theta[(size_t)h * (D / 2) + lane], &sn, &cs);   // lane = row pair
+    }
+    const float expA = a.decay_A != nullptr ? expf(a.decay_A[h]) : 0.f;
+    if (a.early) pdl_wait();
+
     // ---- vectors and scalars
     const TIN *qp = (const TIN *)a.qp + (size_t)b * a.in_sb + (size_t)h * D;
     const TIN *kp = (const TIN *)a.kp + (size_t)b * a.in_sb + (size_t)h * D;
@@ -61,7 +69,7 @@ __global__ void __launch_bounds__(DW_WARPS * 32) decode_step_warp_kernel(DecodeA
     float k0 = to_f32(kp[lane]), k1 = to_f32(kp[lane + 32]);
     float2 vv = make_float2(to_f32(vp[2 * lane]), to_f32(vp[2 * lane + 1]));   // this lane's two columns
     float dl = to_f32(((const TIN *)a.decay)[(size_t)b * a.decay_sb + h]);
-    if (a.decay_A != nullptr) dl = -softplusf_(dl) * expf(a.decay_A[h]);
+    if (a.decay_A != nullptr) dl = -softplusf_(dl) * expA;
     const float alpha = expf(dl);
     float g = 1.f;
     if (a.gate != nullptr) {
@@ -77,12 +85,7 @@ __global__ void __launch_bounds__(DW_WARPS * 32) decode_step_warp_kernel(DecodeA
     const float kscale = DELTA ? 1.f : g;                             // plain rule: the write gate scales k; delta rule: g is beta
     sq[w][lane] = q0; sq[w][lane + 32] = q1;
     sk[w][lane] = k0 * kscale; sk[w][lane + 32] = k1 * kscale;
-    {
-        const float shift = a.shift_dev != nullptr ? *a.shift_dev : a.shift_host;
-        float sn = 0.f, cs = 1.f;
-        if (shift != 0.f) sincosf(-shift * a.theta[(size_t)h * (D / 2) + lane], &sn, &cs);   // lane = row pair
-        srot[w][lane] = make_float2(alpha * cs, alpha * sn);
-    }
+    srot[w][lane] = make_float2(alpha * cs, alpha * sn);
     __syncwarp();
 
     float2 acc = make_float2(0.f, 0.f);                               // delta: sum_r k_r Sd[r][j];  plain: sum_r q_r S'[r][j]

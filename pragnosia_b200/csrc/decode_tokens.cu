@@ -22,7 +22,10 @@ namespace pgb {
 __global__ void __launch_bounds__(128) decode_embed_kernel(const long long *__restrict__ tok, const long long *__restrict__ pos,
                                                            const __nv_bfloat16 *__restrict__ E, const __nv_bfloat16 *__restrict__ P,
                                                            __nv_bfloat16 *__restrict__ x, int d, int vocab, int ctx,
-                                                           float *__restrict__ stats) {
+                                                           float *__restrict__ stats, const __nv_bfloat16 *__restrict__ w,
+                                                           __nv_bfloat16 *__restrict__ xw, float *__restrict__ sq) {
+    // Nothing behind this kernel starts before everything ahead of it is complete: the kernels of a token may then read what the last token left
+    // (the state) ahead of their own waits.
     pdl_wait();
     pdl_launch_dependents();
     __shared__ float red[2][4];
@@ -46,12 +49,20 @@ __global__ void __launch_bounds__(128) decode_embed_kernel(const long long *__re
             s1 += r.x + r.y; s2 = fmaf(r.x, r.x, fmaf(r.y, r.y, s2));
         }
         xr[i] = o;
+        if (w != nullptr) {                                           // times the weight of the norm behind it
+            const uint4 wr = reinterpret_cast<const uint4 *>(w)[i];
+            const __nv_bfloat162 *w2 = reinterpret_cast<const __nv_bfloat162 *>(&wr);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o2[j] = __hmul2_rn(o2[j], w2[j]);
+            reinterpret_cast<uint4 *>(xw + (size_t)b * d)[i] = o;
+        }
     }
-    if (stats != nullptr) {                                           // blockDim.x = 128: four warps
+    if (stats != nullptr || sq != nullptr) {                          // blockDim.x = 128: four warps
         s1 = warp_sum(s1); s2 = warp_sum(s2);
         if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = s1; red[1][threadIdx.x >> 5] = s2; }
         __syncthreads();
-        if (threadIdx.x == 0)
+        if (threadIdx.x == 0 && sq != nullptr) sq[b] = red[1][0] + red[1][1] + red[1][2] + red[1][3];
+        if (threadIdx.x == 0 && stats != nullptr)
             *reinterpret_cast<float2 *>(stats + 2 * b) = make_float2(red[0][0] + red[0][1] + red[0][2] + red[0][3],
                                                                      red[1][0] + red[1][1] + red[1][2] + red[1][3]);
     }
@@ -203,9 +214,9 @@ int decode_advance_launch(long long *pos, float *shift, int window, cudaStream_t
 }
 
 int decode_embed_launch(const long long *tok, const long long *pos, const void *E, const void *P, void *x, int B, int d, int vocab,
-                        int ctx, float *stats, cudaStream_t stream) {
+                        int ctx, float *stats, const void *w, void *xw, float *sq, cudaStream_t stream) {
     cudaError_t e = pdl_launch(decode_embed_kernel, dim3((unsigned)B), dim3(128), 0, stream, tok, pos, (const __nv_bfloat16 *)E,
-                               (const __nv_bfloat16 *)P, (__nv_bfloat16 *)x, d, vocab, ctx, stats);
+                               (const __nv_bfloat16 *)P, (__nv_bfloat16 *)x, d, vocab, ctx, stats, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)xw, sq);
     if (e != cudaSuccess) { set_cuda_error(e, "decode_embed launch"); return PGB_ERR_CUDA; }
     return check_launch("decode_embed_kernel");
 }

@@ -322,10 +322,12 @@ def rotate(x, theta, pos):
 @on_device_of
 def decode_step(qp, kp, vp, decay, S, theta, *, gate=None, delta: bool = False, gate_is_logit: bool = True,
                 decay_A=None, normalize: bool = True, shift=0.0, rms_weight=None, rms_eps: float = 0.0,
-                out: Optional[torch.Tensor] = None, S_out: Optional[torch.Tensor] = None, out_dtype=None):
+                out: Optional[torch.Tensor] = None, S_out: Optional[torch.Tensor] = None, out_dtype=None, early: bool = False):
     """One fused recurrent step. qp,kp,vp: (B,H,D) views with unit strides over (H,D) and a common batch stride;
     decay, gate: (B,H) views with unit stride over H.  S (B,H,D,D) fp32; S_out defaults to a new tensor (pass S itself
-    for an in-place update).  Returns (o (B,H,D), S_out)."""
+    for an in-place update).  Returns (o (B,H,D), S_out).
+    early: the state and the constants are complete before the kernel ahead is launched (a link of a token's chain, decode_linear): they
+    are read while it runs."""
     need_cuda(qp, kp, vp, decay, S, theta)
     B, H, D = qp.shape
     for t in (qp, kp, vp):
@@ -349,11 +351,11 @@ def decode_step(qp, kp, vp, decay, S, theta, *, gate=None, delta: bool = False, 
     if out is None:
         out = torch.empty(B, H, D, device=qp.device, dtype=out_dtype)
     sb = lambda t: t.stride(0) if B > 1 else max(t.stride(0), H * (t.shape[2] if t.dim() == 3 else 1))
-    check(lib().pgb_aspin_decode_step(
+    check(lib().pgb_aspin_decode_step_ex(
         ptr(qp), ptr(kp), ptr(vp), dtype_code(qp), sb(qp), int(normalize), ptr(gate), 0 if gate is None else gate.stride(0),
         int(gate_is_logit), int(delta), ptr(decay), decay.stride(0), ptr(decay_A), ptr(theta),
         ptr(shift_dev), shift_host, ptr(S), ptr(S_out), ptr(rms_weight), float(rms_eps), ptr(out), dtype_code(out),
-        sb(out), B, H, D, stream_of(qp)), "pgb_aspin_decode_step")
+        sb(out), B, H, D, 1 if early else 0, stream_of(qp)), "pgb_aspin_decode_step")
     return out, S_out
 
 
@@ -488,6 +490,55 @@ def decode_embed(tok, pos, E, P, want_sums: bool = False):
     check(lib().pgb_decode_embed_ex(ptr(tok.contiguous()), ptr(pos), ptr(E.contiguous()), ptr(P.contiguous()), ptr(x), ptr(sums), B, d,
                                     E.shape[0], P.shape[0], stream_of(E)), "pgb_decode_embed")
     return (x, sums) if want_sums else x
+
+
+def decode_linear_takes(kind: int, N: int, K: int) -> bool:
+    """Whether decode_linear takes a layer of these sizes (kind 0: plain or activation, 1: residual, 2: logits)."""
+    return bool(lib().pgb_decode_linear_takes(kind, N, K))
+
+
+@on_device_of
+def decode_embed_norm(tok, pos, E, P, next_w):
+    """The first kernel of a token whose linear layers are decode_linear's: x (B,d) = E[tok] + P[pos], x next_w, and the rows' sums of squares (B,1)."""
+    need_cuda(tok, pos, E, P, next_w)
+    if any(t.dtype != torch.bfloat16 for t in (E, P, next_w)) or tok.dtype != torch.long or pos.dtype != torch.long:
+        raise ValueError("decode_embed_norm: bf16 tables and weight, int64 ids")
+    B, d = tok.numel(), E.shape[1]
+    x, xw = (torch.empty(B, d, device=E.device, dtype=E.dtype) for _ in range(2))
+    sq = torch.empty(B, 1, device=E.device, dtype=torch.float32)
+    check(lib().pgb_decode_embed_norm(ptr(tok.contiguous()), ptr(pos), ptr(E), ptr(P), ptr(next_w), ptr(x), ptr(xw), ptr(sq), B, d, E.shape[0], P.shape[0],
+                                      stream_of(E)), "pgb_decode_embed_norm")
+    return x, xw, sq
+
+
+@on_device_of
+def decode_linear(x, W, bias=None, squares=None, eps: float = 0.0, act: Optional[str] = None, resid=None, next_w=None, logits=None, pos=None, shift=None,
+                  window: int = 0):
+    """One linear layer of the decode step of up to 64 sequences as a link of a chain of dependent launches; x (B,K), W (N,K), bias (N,) bf16, N and K
+    multiples of 8. squares (B,parts) fp32: x is the residual stream times the weight of the RMS norm ahead of the layer, and its rows' 1 / rms (eps)
+    is applied to the product. act None or "gelu". resid (B,N), next_w (N,): returns (resid + y, that times next_w, the parts of its rows' sums of
+    squares) for the next norm. logits (B,N) fp32: written instead of a bf16 result. window > 0: also pos = (pos + 1) mod window, shift = 1.
+    W, bias and next_w are read before the wait on the kernel ahead: they are complete before the chain's first kernel (decode_embed_norm)."""
+    need_cuda(x, W)
+    if any(t is not None and t.dtype != torch.bfloat16 for t in (x, W, bias, resid, next_w)) or x.dim() != 2 or not x.is_contiguous():
+        raise ValueError("decode_linear: bf16, x (B,K) contiguous")
+    if not all(t is None or t.is_contiguous() for t in (W, bias, squares, resid, next_w, logits)):
+        raise ValueError("decode_linear: contiguous tensors")
+    if any(t is not None and t.dtype != torch.float32 for t in (squares, logits, shift)) or (pos is not None and pos.dtype != torch.long):
+        raise ValueError("decode_linear: fp32 sums, logits and shift, int64 position")
+    (B, K), N = x.shape, W.shape[0]
+    if W.shape[1] != K or (squares is not None and squares.shape[0] != B) or any(t is not None and tuple(t.shape) != (B, N) for t in (resid, logits)):
+        raise ValueError("decode_linear: shapes")
+    y = yw = sq = None
+    if logits is None:
+        y = torch.empty(B, N, device=x.device, dtype=x.dtype)
+    if resid is not None:
+        yw = torch.empty_like(y)
+        sq = torch.empty(B, int(lib().pgb_decode_linear_parts(N, K)), device=x.device, dtype=torch.float32)
+    check(lib().pgb_decode_linear(ptr(x), ptr(W), ptr(bias), ptr(squares), 0 if squares is None else squares.shape[1], float(eps), 1 if act == "gelu" else 0,
+                                  ptr(resid), ptr(next_w), ptr(y), ptr(yw), ptr(sq), ptr(logits), ptr(pos), ptr(shift), int(window), B, N, K, stream_of(x)),
+          "pgb_decode_linear")
+    return logits if logits is not None else y if resid is None else (y, yw, sq)
 
 
 @on_device_of

@@ -147,6 +147,14 @@ def test_new_entry_points_reject_bad_calls(L):
     tok = lambda **kw: L.pgb_decode_token_fwd(one, 12, one, one, one, kw.get("nb", one), 2, 1e-5, one, one, one, one, kw.get("wb", 10 ** 6),
                                               one, one, kw.get("B", 1), 768, 12, kw.get("D", 64), 2328, 3072, 50257, 512, 0, None)
     assert tok(nb=None) == 1 and tok(wb=10) == 2 and tok(B=5) == 7 and tok(D=96) == 3
+    # the linear layers of a batch's step: which K they take, then the rejects (batch, a residual without its norm weight, both results, K too long)
+    assert L.pgb_decode_linear_takes(0, 2328, 768) == 1 and L.pgb_decode_linear_takes(1, 768, 768 * 16) == 0 and L.pgb_decode_linear_takes(0, 12, 768) == 0
+    assert L.pgb_decode_linear_parts(768, 768) == 24 and L.pgb_decode_linear_parts(768, 256) == 48 and L.pgb_decode_linear_parts(768, 192) == 0
+    lin = lambda **kw: L.pgb_decode_linear(one, one, one, None, 0, 0.0, 0, kw.get("resid"), kw.get("next_w"), kw.get("y", one), kw.get("yw"), kw.get("sq"),
+                                           kw.get("logits"), None, None, kw.get("window", 0), kw.get("B", 4), 768, kw.get("K", 768), None)
+    assert lin(B=65) == 7 and lin(K=768 * 16) == 7 and lin(K=12) == 2 and lin(resid=one) == 1 and lin(logits=one) == 1 and lin(y=None) == 1
+    assert lin(window=512) == 1 and lin(y=ctypes.c_void_p(0x1004)) == 4
+    assert L.pgb_decode_embed_norm(one, one, one, one, None, one, one, one, 4, 768, 100, 16, None) == 1
     # the same step without barriers: 32-bit words of every layer's exchanges; 0 where a row does not fit a stage or the rows shared memory
     assert L.pgb_decode_flow_work_bytes(12, 2, 768, 2328, 3072) == 4 * 12 * 2 * (2328 + 3 * 768 + 3072)
     assert L.pgb_decode_flow_work_bytes(12, 1, 3200, 9624, 12800) == 0 and L.pgb_decode_flow_work_bytes(12, 4, 2048, 6208, 8192) == 0

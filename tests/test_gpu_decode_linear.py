@@ -1,0 +1,81 @@
+"""The decode step of a batch as a chain of dependent launches (decode_linear.cu) against the same step through the separate kernels, whose
+parity with the oracle the model tests pin. Both round after every linear layer, norm, activation and add; the chain applies a norm's
+1 / rms to the fp32 sum instead of the row ahead of it and adds a product's K in parts, so a bf16 rounding may fall the other way
+(2^-8 of a value). So both are measured against the same model in fp32 (weights of the same values): the 2-norm of the chain's error is that
+of the separate kernels', as two draws of the same roundings (measured 0.95 to 1.07 of it)."""
+import copy
+
+import pytest
+import torch
+
+from pragnosia_b200 import synth
+from pragnosia_b200.generate import Decoder
+from pragnosia_b200.model import LM
+
+from test_gpu_decode_token import healthy
+from test_gpu_model import DEV
+
+pytestmark = pytest.mark.gpu
+
+
+def model(d, mixer, mult, vocab, layers=3, norm="rms"):
+    torch.manual_seed(d)
+    m = LM(vocab=vocab, d=d, layers=layers, mlp_mult=mult, ctx=16, mixer=mixer, norm=norm)
+    with torch.no_grad():
+        for n, p in m.named_parameters():
+            if p.dim() == 1:                                          # norms' weights, biases, gates: away from their initial ones and zeros
+                p.add_(0.2 * torch.randn_like(p))
+    return m.to(DEV).bfloat16().eval()
+
+
+def steps(m, B, vocab, n=10, **kw):
+    ids = synth.token_ids(B, 40, vocab, seed=B).to(DEV)
+    dec = Decoder(m, batch=B, **kw)
+    lg = [dec.prefill(ids[:, :20])]
+    for t in range(20, 20 + n):                                       # crosses the window's edge (ctx 16)
+        lg.append(dec.step(ids[:, t]).clone())
+    lg.append(dec.prefill(ids[:, :17]))                               # a new prompt on the same decoder
+    lg.append(dec.step(ids[:, 17]).clone())
+    return dec, torch.stack(lg, 1), [st[0].clone() for st in dec.states]
+
+
+@pytest.mark.parametrize("d,mixer,mult,vocab", [
+    (256, "hspin", 1, 40),                                            # the least K, clusters of two; a head of one tile; head dim 128
+    (704, "dspin", 3, 1000),                                          # eleven blocks over two and four CTAs, 33 over eight; ragged tiles of every width
+    (768, "aspin", 4, 8192),
+    (1536, "hdspin", 4, 5000),                                        # twelve blocks a CTA
+])
+@pytest.mark.parametrize("B", [5, 16, 17, 44, 64])
+def test_chained_step_of_a_batch(d, mixer, mult, vocab, B):
+    m = model(d, mixer, mult, vocab)
+    _, lg_x, S_x = steps(copy.deepcopy(m).float(), B, vocab)
+    ref, lg0, S0 = steps(m, B, vocab, fused=False)
+    assert not ref._chain_ok()
+    off = lambda lg, S: [float((a.double() - x.double()).norm() / x.double().norm()) for a, x in zip((lg, *S), (lg_x, *S_x))]
+    outs = []
+    for use_graph in (True, False):
+        dec, lg, S = steps(m, B, vocab, use_graph=use_graph)
+        assert dec._chain_ok() and dec.launches_per_token == 3 + 5 * m.layers
+        assert all(torch.isfinite(t).all() for t in (lg, *S))
+        ratios = [e / e0 for e, e0 in zip(off(lg, S), off(lg0, S0))]
+        assert max(ratios) < 1.2
+        outs.append((lg, S))
+    assert torch.equal(outs[0][0], outs[1][0]) and all(torch.equal(a, b) for a, b in zip(outs[0][1], outs[1][1]))   # every sum in a fixed order
+    assert healthy() == 0
+
+
+def test_models_that_keep_the_separate_kernels():
+    for m, B, kw in ((model(192, "aspin", 2, 256), 8, {}), (model(256, "aspin", 2, 256, norm="ln"), 8, {}), (model(256, "aspin", 2, 256), 65, {}), (model(256, "aspin", 2, 256), 8, dict(folded=True)),
+                     (model(256, "aspin", 2, 252), 8, {})):
+        dec, lg, _ = steps(m, B, 250, n=2, **kw)
+        assert not dec._chain_ok() and torch.isfinite(lg).all()
+
+
+def test_generate_through_the_chained_step():
+    m = model(256, "aspin", 4, 512)
+    prompt = synth.token_ids(9, 40, 512, seed=3).to(DEV)
+    for temp in (0.0, 1.0):
+        a = Decoder(m, batch=9).generate(prompt, 24, temp=temp, seed=5)
+        c = Decoder(m, batch=9, use_graph=False).generate(prompt, 24, temp=temp, seed=5)
+        assert torch.equal(a, c)                                      # graph replay and eager launches draw the same ids
+    assert healthy() == 0
