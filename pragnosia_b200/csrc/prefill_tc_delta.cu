@@ -72,6 +72,34 @@ __device__ __forceinline__ void inv_product(float (&acc)[2][4], const float *A, 
     }
 }
 
+// rows r0 + RS i and columns c0..c0+3 of P = A B, i < 4, over k0 <= k < K: eight loads of 16 bytes for 64 products, and rows RS apart so
+// that the rows a warp reads at once lie in different banks
+template <int K, int RS>
+__device__ __forceinline__ void inv_product4(float (&acc)[4][4], const float *A, int pa, const float *B, int pb, int r0, int c0, int k0) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
+#pragma unroll 2
+    for (int k = k0; k < K; k += 4) {
+        float f[4][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float4 a = *reinterpret_cast<const float4 *>(A + (r0 + RS * r) * pa + k);
+            f[r][0] = a.x; f[r][1] = a.y; f[r][2] = a.z; f[r][3] = a.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 b = *reinterpret_cast<const float4 *>(B + (k + i) * pb + c0);
+            const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(f[r][i], bv[c], acc[r][c]);
+        }
+    }
+}
+
 template <int D>
 __global__ void __launch_bounds__(128) delta_inv_kernel(const __grid_constant__ CUtensorMap mk, const float *__restrict__ la_all,
                                                         const float *__restrict__ beta_all, __nv_bfloat16 *__restrict__ X, int T,
@@ -139,76 +167,90 @@ __global__ void __launch_bounds__(128) delta_inv_kernel(const __grid_constant__ 
     tc_fence_before();
     __syncthreads();                                                  // K is consumed (the product is complete): X takes its place
     if (warp == 3) tmem_dealloc(tmem, 64);
-    // ---- diagonal blocks: lane j < 16 of warp b owns column j of block b;  x_t = [t == j] - sum_{s<t} N[t][s] x_s
-    if (lane < 16) {
-        const float *Nb = Nf + 16 * warp * (NP + 1);
-        float *Xb = Xf + 16 * warp * (NP + 1);
+    // ---- diagonal blocks: lane j of a half warp owns column j of a block;  x_t = [t == j] - sum_{s<t} N[t][s] x_s
+    if (warp < 2) {
+        const int j = lane & 15, blk = 2 * warp + (lane >> 4);
+        const float *Nb = Nf + 16 * blk * (NP + 1);
+        float *Xb = Xf + 16 * blk * (NP + 1);
         float x[16];
 #pragma unroll
         for (int t = 0; t < 16; ++t) {
-            float a0 = t == lane ? 1.f : 0.f, a1 = 0.f;
+            float a0 = t == j ? 1.f : 0.f, a1 = 0.f;
 #pragma unroll
             for (int s4 = 0; s4 < (t + 3) / 4; ++s4) {
-                const float4 n = *reinterpret_cast<const float4 *>(Nb + t * NP + 4 * s4);   // the same address for every lane: a broadcast
+                const float4 n = *reinterpret_cast<const float4 *>(Nb + t * NP + 4 * s4);   // the same address for every lane of a half: a broadcast
                 if (4 * s4 + 0 < t) a0 = fmaf(-n.x, x[4 * s4 + 0], a0);
                 if (4 * s4 + 1 < t) a1 = fmaf(-n.y, x[4 * s4 + 1], a1);
                 if (4 * s4 + 2 < t) a0 = fmaf(-n.z, x[4 * s4 + 2], a0);
                 if (4 * s4 + 3 < t) a1 = fmaf(-n.w, x[4 * s4 + 3], a1);
             }
             x[t] = a0 + a1;
-            Xb[t * NP + lane] = x[t];
+            Xb[t * NP + j] = x[t];
         }
+    } else {                                                          // the two blocks above the diagonal that the joins below read: zero
+        const int g = 32 * (warp & 1), r = 2 * (lane >> 2), cc = 4 * (lane & 3);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Xf + (g + r + i) * NP + g + 16 + cc) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
-    // ---- join 16 x 16 blocks, a pair of blocks per pair of warps: the first warp's lanes cover the new block as two rows by four
-    //      columns each
-    float acc[2][4];
-    {
-        const int g = 32 * (warp >> 1), r = 2 * (lane >> 2), cc = 4 * (lane & 3);   // the pair's first row; only its first warp works
-        const bool mine = (warp & 1) == 0;
-        float *Tb = Tf + (warp >> 1) * 16 * TP;
-        if (mine) {
-            inv_product<16>(acc, Nf + (g + 16) * NP + g, NP, Xf + g * NP + g, NP, r, cc);
+    // ---- join 16 x 16 blocks, a warp per pair of blocks, whose lanes cover the new block as two rows by four columns each
+    if (warp < 2) {
+        float acc[2][4];
+        const int g = 32 * warp, r = 2 * (lane >> 2), cc = 4 * (lane & 3);         // the pair's first row
+        float *Tb = Tf + warp * 16 * TP;
+        inv_product<16>(acc, Nf + (g + 16) * NP + g, NP, Xf + g * NP + g, NP, r, cc);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Tb + (r + i) * TP + cc) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-            __syncwarp();
-            inv_product<16>(acc, Xf + (g + 16) * NP + g + 16, NP, Tb, TP, r, cc);
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Tb + (r + i) * TP + cc) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        __syncwarp();
+        inv_product<16>(acc, Xf + (g + 16) * NP + g + 16, NP, Tb, TP, r, cc);
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-                *reinterpret_cast<float4 *>(Xf + (g + 16 + r + i) * NP + g + cc) = make_float4(-acc[i][0], -acc[i][1], -acc[i][2], -acc[i][3]);
-        } else {                                                      // its second warp zeroes the block above the diagonal
+        for (int i = 0; i < 2; ++i)
+            *reinterpret_cast<float4 *>(Xf + (g + 16 + r + i) * NP + g + cc) = make_float4(-acc[i][0], -acc[i][1], -acc[i][2], -acc[i][3]);
+    }
+    __syncthreads();
+    // ---- join the 32 x 32 blocks by two warps, which store the new block from their registers; the other two store the rest meanwhile.
+    //      Head then tail, 8 KB each, to the scratch buffer; or the head alone, densely packed (the stand-alone operator).
+    uint4 *dst = reinterpret_cast<uint4 *>(X + ((size_t)bh * NC + c) * ((with_tail ? 2 : 1) * TC_C * TC_C));
+    if (warp < 2) {
+        float acc[4][4];
+        {   // T = N21 X11, 16 columns a warp: X11 is lower triangular, so the right half's products begin at its row 16
+            const int r = lane >> 2, cc = 16 * warp + 4 * (lane & 3);
+            inv_product4<32, 8>(acc, Nf + 32 * NP, NP, Xf, NP, r, cc, 16 * warp);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Xf + (g + r + i) * NP + g + 16 + cc) = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int i = 0; i < 4; ++i) *reinterpret_cast<float4 *>(Tf + (r + 8 * i) * TP + cc) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
         }
-    }
-    __syncthreads();
-    // ---- join the 32 x 32 blocks: 128 threads, two rows by four columns each
-    {
-        const int r = 2 * (tid >> 3), cc = 4 * (tid & 7);
-        inv_product<32>(acc, Nf + 32 * NP, NP, Xf, NP, r, cc);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Tf + (r + i) * TP + cc) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        __syncthreads();
-        inv_product<32>(acc, Xf + 32 * NP + 32, NP, Tf, TP, r, cc);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Xf + (32 + r + i) * NP + cc) = make_float4(-acc[i][0], -acc[i][1], -acc[i][2], -acc[i][3]);
-    }
-    __syncthreads();
-    // ---- head then tail, 8 KB each, to the scratch buffer; or the head alone, densely packed (the stand-alone operator)
-    {
-        uint4 *dst = reinterpret_cast<uint4 *>(X + ((size_t)bh * NC + c) * ((with_tail ? 2 : 1) * TC_C * TC_C));
+        named_sync(1, 64);
+        // X21 = -X22 T, 16 rows a warp: the upper half's products end at column 16
+        const int r = 16 * warp + (lane >> 3), cc = 4 * (lane & 7);
+        if (warp == 0) inv_product4<16, 4>(acc, Xf + 32 * NP + 32, NP, Tf, TP, r, cc, 0);
+        else inv_product4<32, 4>(acc, Xf + 32 * NP + 32, NP, Tf, TP, r, cc, 0);
+        uint2 *d2 = reinterpret_cast<uint2 *>(dst);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int idx = tid + 128 * i, row = idx >> 3, col = 8 * (idx & 7);
-            uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
-            if (col < (row < 32 ? 32 : 64)) {                         // the block above the diagonal is never written: zero
-                const float4 a = *reinterpret_cast<const float4 *>(Xf + row * NP + col), b = *reinterpret_cast<const float4 *>(Xf + row * NP + col + 4);
-                const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                split8(x, hi, lo);
-            }
-            dst[idx] = hi;
-            if (with_tail) dst[512 + idx] = lo;
+            uint32_t h0, l0, h1, l1;
+            split2(-acc[i][0], -acc[i][1], h0, l0);
+            split2(-acc[i][2], -acc[i][3], h1, l1);
+            d2[(32 + r + 4 * i) * 16 + (lane & 7)] = make_uint2(h0, h1);
+            if (with_tail) d2[1024 + (32 + r + 4 * i) * 16 + (lane & 7)] = make_uint2(l0, l1);
         }
+    } else {
+        auto store = [&](int row, int piece) {                        // eight columns
+            const float4 a = *reinterpret_cast<const float4 *>(Xf + row * NP + 8 * piece), b = *reinterpret_cast<const float4 *>(Xf + row * NP + 8 * piece + 4);
+            const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            uint4 hi, lo;
+            split8(x, hi, lo);
+            dst[row * 8 + piece] = hi;
+            if (with_tail) dst[512 + row * 8 + piece] = lo;
+            if (row < 32) {                                           // the block above the diagonal: zero
+                dst[row * 8 + piece + 4] = make_uint4(0u, 0u, 0u, 0u);
+                if (with_tail) dst[512 + row * 8 + piece + 4] = make_uint4(0u, 0u, 0u, 0u);
+            }
+        };
+        const int t = tid - 64;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) store((t >> 2) + 16 * i, t & 3);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) store(32 + (t >> 2) + 16 * i, 4 + (t & 3));
     }
 }
 
