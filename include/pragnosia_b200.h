@@ -437,7 +437,7 @@ int pgb_batch_linear_parts(int N);
  *   ahead, and the layer is  v = r (x W^T) + bias,  r = 1 / sqrt(sum / K + eps); without, v = x W^T + bias. v is rounded to bf16; then
  *   y [B][N] = v, or its erf-GELU (act 1); or logits [B][N] fp32 = v (y NULL);
  *   or with resid [B][N]: y = resid + v, the new residual stream; yw = y next_w (next_w [N]: the weight of the norm behind); and
- *   squares_out [B][pgb_decode_linear_parts(N, K)].
+ *   squares_out [B][pgb_decode_linear_parts(N, K, B)].
  *   window > 0: the launch also leaves pos = (pos + 1) mod window and shift = 1, for the last layer of a token.
  * Whether a layer is taken depends on K alone (256 at least): pgb_decode_linear_takes(kind 0 plain or activation, 1 residual, 2 logits; N, K).
  * pgb_decode_embed_norm is such a token's first kernel: x = E[tok] + P[pos], xw = x next_w and squares [B] (one part).
@@ -446,7 +446,7 @@ int pgb_batch_linear_parts(int N);
 int pgb_decode_embed_norm(const long long *tok, const long long *pos, const void *E, const void *P, const void *next_w, void *x, void *xw,
                           float *squares, int B, int d, int vocab, int ctx, void *stream);
 int pgb_decode_linear_takes(int kind, int N, int K);
-int pgb_decode_linear_parts(int N, int K);
+int pgb_decode_linear_parts(int N, int K, int B);
 int pgb_decode_linear(const void *x, const void *W, const void *bias, const float *squares_in, int parts_in, float eps, int act, const void *resid,
                       const void *next_w, void *y, void *yw, float *squares_out, float *logits, long long *pos, float *shift, int window, int B,
                       int N, int K, void *stream);

@@ -12,11 +12,13 @@
 //     weight; rounded once, as the normalised row would be) and each row's sum of squares by tiles; here x w is multiplied, and the row's
 //     1 / rms applied to the fp32 sum.
 //
-// A token of 12 layers of 768 (graph replay): batch 64 421 -> 316 us, batch 16 383 -> 265, batch 5 372 -> 260, against the library's products with
-// separate norms. What bounds it now is the chain: about 4.2 us a link at batch 5 (grid completion to the next grid's first load, x, the products,
-// the exchange over the cluster, the way out), 5.2 at batch 64 (48 KB of x a CTA, 12.6 MB of states a layer).
+// A token of 12 layers of 768 (graph replay): batch 64 421 -> 316 us, batch 16 383 -> 240, batch 5 372 -> 223, against the library's products with
+// separate norms. What bounds it now is the chain: at batch 5 3.6 us a link, of which 1.6 are the launch alone (links that return behind their wait), 0.8 x (only the
+// batch's rows are fetched: all 64 took 0.4 more), 0.9 the sums of squares, products and waits, 0.3 the exchange, 0.5 the way out; 5.2 at batch 64
+// (48 KB of x a CTA; of the 12.6 MB of states a layer, their stores are 0.3). An L2 prefetch of the weights two links ahead gave nothing, one barrier for
+// all blocks of K instead of one each 0.4 more a link, two issuing warps 0.2 more.
 //
-// x [B][K] bf16 is the K-major A operand (64 rows, those past the batch zero-filled), W [N][K] the B operand. Replaces, for T = 1, F.linear with the
+// x [B][K] bf16 is the K-major A operand (64 rows; those past the batch are zero or whatever shared memory holds, each its own row's only), W [N][K] the B operand. Replaces, for T = 1, F.linear with the
 // norm, GELU and residual add around it (src/assoc.py:384-512, src/model.py:552-560). Every wait is bounded; one that runs out sets the error flag, and
 // the cluster winds down together.
 #include "tc_common.cuh"
@@ -33,7 +35,7 @@ struct DlArgs {
     const __nv_bfloat16 *resid, *next_w;                              // residual stream to add to [B][N]; weight of the norm behind it [N]
     __nv_bfloat16 *y, *yw; float *logits, *sums_out;                  // y [B][N], or logits in fp32; with resid: y next_w and [B][tiles] sums of squares
     long long *pos; float *shift; int window;                         // the last layer of a token: the next one's position and shift
-    int B, N, K, act;
+    int B, N, K, act, xrows;                                          // xrows: rows of x fetched, the batch rounded up
 };
 
 template <int BN> __host__ __device__ constexpr int dl_block() { return DL_ROWS * 128 + BN * 128; }      // bytes of a K block: 64 rows of x, BN of W
@@ -82,7 +84,7 @@ __global__ void __launch_bounds__(DL_NT) decode_linear_kernel(const __grid_const
         __syncwarp();
         if (lane == 0)
             for (int i = 0; i < nk; ++i) {
-                mbar_expect_tx(bar + 8 * i, dl_block<BN>());
+                mbar_expect_tx(bar + 8 * i, (a.xrows + BN) * 128);
                 tma_load_3d(ws + i * (BN * 128), &mw, bar + 8 * i, (kb0 + i) * 64, n0, 0);
             }
         if (lane == 1 && live) mbar_expect_tx(bar_p, S * RR * BN * 4);
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(DL_NT) decode_linear_kernel(const __grid_const
 template <int BN, int S>
 static int decode_linear_go(const void *x, const void *W, const DlArgs &a, cudaStream_t stream) {
     CUtensorMap mx, mw;
-    if (!tc_make_map(&mx, x, 1, a.B, a.K, a.K, (long long)a.B * a.K, DL_ROWS) || !tc_make_map(&mw, W, 1, a.N, a.K, a.K, (long long)a.N * a.K, BN)) {
+    if (!tc_make_map(&mx, x, 1, a.B, a.K, a.K, (long long)a.B * a.K, a.xrows) || !tc_make_map(&mw, W, 1, a.N, a.K, a.K, (long long)a.N * a.K, BN)) {
         set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled");
         return PGB_ERR_CUDA;
     }
@@ -257,33 +259,34 @@ struct DlForm { int bn, s; };
 // Two things pull: x is read once a tile (wide tiles, few clusters), and CTAs of neighbouring links must fit an SM together, at best one of each (about
 // 100 to 130 CTAs of 80 to 100 KB a link). Batch 64, d 768, dff 3072, us a token, all else equal: projection 48,2 335 (32,2 345, 64,4 341, 16,1 333
 // but 276 against 275 at batch 16); output projection 32,4 312 (16,4 344, 32,2 318, 16,1 326); MLP up 48,2 331 (32,2 344, 32,4 347, 64,2 349); MLP
-// down 32,8 344 (32,4 350, 16,8 379, 48,8 and 64,8 2 to 5 % slower at batch 64, as much faster at batch 5); head the same in every form.
+// down 32,8 344 (32,4 350, 16,8 379, 48,8 2 % slower; but at batch 5 223 against 239, at 16 240 against 245, at 32 271 against 276); head the same in
+// every form.
 // Every CTA keeps at least two blocks of K; shorter K is not taken.
-static DlForm decode_linear_form(int kind, int N, int K) {
+static DlForm decode_linear_form(int kind, int K, int B) {
     const int kb = (K + 63) / 64;
     DlForm f;
     if (kb < 4) return DlForm{0, 0};
-    if (kind == 1) f = kb >= 32 ? DlForm{32, 8} : (kb >= 8 ? DlForm{32, 4} : DlForm{16, 2});
+    if (kind == 1) f = kb >= 32 ? (B <= 32 ? DlForm{48, 8} : DlForm{32, 8}) : (kb >= 8 ? DlForm{32, 4} : DlForm{16, 2});
     else f = kind == 2 ? DlForm{64, 2} : DlForm{48, 2};
     while (f.s < 8 && ((kb + f.s - 1) / f.s > DL_KB || (kb + f.s - 1) / f.s * (DL_ROWS + f.bn) * 128 + DL_ROWS * (f.bn + 4) * 4 + 1024 > DL_SMEM_MOST)) f.s *= 2;
     if ((kb + f.s - 1) / f.s > DL_KB || (kb + f.s - 1) / f.s * (DL_ROWS + f.bn) * 128 + DL_ROWS * (f.bn + 4) * 4 + 1024 > DL_SMEM_MOST) return DlForm{0, 0};
     return f;
 }
 // tiles (= sums of squares a row) of a residual layer; 0: not taken
-int decode_linear_parts(int N, int K) {
-    const DlForm f = decode_linear_form(1, N, K);
+int decode_linear_parts(int N, int K, int B) {
+    const DlForm f = decode_linear_form(1, K, B);
     return f.bn == 0 ? 0 : (N + f.bn - 1) / f.bn;
 }
-bool decode_linear_takes(int kind, int N, int K) { return decode_linear_form(kind, N, K).bn != 0; }
+bool decode_linear_takes(int kind, int K, int B) { return decode_linear_form(kind, K, B).bn != 0; }
 
 int decode_linear_launch(const void *x, const void *W, const void *bias, const float *sums, int parts, float eps, int act, const void *resid,
                          const void *next_w, void *y, void *yw, float *sums_out, float *logits, long long *pos, float *shift, int window, int B, int N,
                          int K, cudaStream_t stream) {
     const DlArgs a{(const __nv_bfloat16 *)bias, sums, parts, eps, (const __nv_bfloat16 *)resid, (const __nv_bfloat16 *)next_w, (__nv_bfloat16 *)y,
-                   (__nv_bfloat16 *)yw, logits, sums_out, pos, shift, window, B, N, K, act};
-    const DlForm f = decode_linear_form(resid != nullptr ? 1 : (logits != nullptr ? 2 : 0), N, K);
+                   (__nv_bfloat16 *)yw, logits, sums_out, pos, shift, window, B, N, K, act, (B + 7) / 8 * 8};
+    const DlForm f = decode_linear_form(resid != nullptr ? 1 : (logits != nullptr ? 2 : 0), K, B);
 #define PGB_DL(BN_, S_) if (f.bn == BN_ && f.s == S_) return decode_linear_go<BN_, S_>(x, W, a, stream)
-    PGB_DL(16, 2); PGB_DL(32, 4); PGB_DL(32, 8);
+    PGB_DL(16, 2); PGB_DL(32, 4); PGB_DL(32, 8);                      // 48, 8 as a residual's, too
     PGB_DL(48, 2); PGB_DL(48, 4); PGB_DL(48, 8);
     PGB_DL(64, 2); PGB_DL(64, 4); PGB_DL(64, 8);
 #undef PGB_DL

@@ -534,7 +534,7 @@ def decode_linear(x, W, bias=None, squares=None, eps: float = 0.0, act: Optional
         y = torch.empty(B, N, device=x.device, dtype=x.dtype)
     if resid is not None:
         yw = torch.empty_like(y)
-        sq = torch.empty(B, int(lib().pgb_decode_linear_parts(N, K)), device=x.device, dtype=torch.float32)
+        sq = torch.empty(B, int(lib().pgb_decode_linear_parts(N, K, B)), device=x.device, dtype=torch.float32)
     check(lib().pgb_decode_linear(ptr(x), ptr(W), ptr(bias), ptr(squares), 0 if squares is None else squares.shape[1], float(eps), 1 if act == "gelu" else 0,
                                   ptr(resid), ptr(next_w), ptr(y), ptr(yw), ptr(sq), ptr(logits), ptr(pos), ptr(shift), int(window), B, N, K, stream_of(x)),
           "pgb_decode_linear")

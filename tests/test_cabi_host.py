@@ -149,7 +149,8 @@ def test_new_entry_points_reject_bad_calls(L):
     assert tok(nb=None) == 1 and tok(wb=10) == 2 and tok(B=5) == 7 and tok(D=96) == 3
     # the linear layers of a batch's step: which K they take, then the rejects (batch, a residual without its norm weight, both results, K too long)
     assert L.pgb_decode_linear_takes(0, 2328, 768) == 1 and L.pgb_decode_linear_takes(1, 768, 768 * 16) == 0 and L.pgb_decode_linear_takes(0, 12, 768) == 0
-    assert L.pgb_decode_linear_parts(768, 768) == 24 and L.pgb_decode_linear_parts(768, 256) == 48 and L.pgb_decode_linear_parts(768, 192) == 0
+    assert L.pgb_decode_linear_parts(768, 768, 64) == 24 and L.pgb_decode_linear_parts(768, 256, 8) == 48 and L.pgb_decode_linear_parts(768, 192, 8) == 0
+    assert L.pgb_decode_linear_parts(768, 3072, 32) == 16 and L.pgb_decode_linear_parts(768, 3072, 33) == 24
     lin = lambda **kw: L.pgb_decode_linear(one, one, one, None, 0, 0.0, 0, kw.get("resid"), kw.get("next_w"), kw.get("y", one), kw.get("yw"), kw.get("sq"),
                                            kw.get("logits"), None, None, kw.get("window", 0), kw.get("B", 4), 768, kw.get("K", 768), None)
     assert lin(B=65) == 7 and lin(K=768 * 16) == 7 and lin(K=12) == 2 and lin(resid=one) == 1 and lin(logits=one) == 1 and lin(y=None) == 1
