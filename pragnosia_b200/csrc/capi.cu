@@ -61,7 +61,9 @@ int tc_train_error_flag(int *);
 int prep_gates_launch(const void *, const void *, const void *, long long, long long, long long, const void *, const void *, long long, long long,
                       const float *, const float *, const long long *, void *, void *, void *, float *, float *, int, int, int, int, cudaStream_t);
 int head_norm_launch(const void *, const float *, float, void *, int, int, int, int, cudaStream_t);
-size_t segment_scratch_bytes(int B, int H, int T, int seg_len);
+size_t segment_scratch_bytes(int B, int H, int T, const SegCut &seg);
+SegCut windows_cut(int B, int H, int T, int window);
+static SegCut equal_pieces(int tokens) { SegCut s; s.win = tokens; return s; }
 int segment_states_launch(const PrefillArgs &, float *, cudaStream_t);
 SegPlan segment_plan(int B, int H, int T);
 int tc_segment_error_flag(int *);
@@ -351,7 +353,7 @@ int pgb_aspin_prefill_fwd(const void *q, const void *k, const void *v, int io_dt
 long long pgb_aspin_prefill_segments_scratch_bytes(int B, int H, int T, int D) {
     if (B <= 0 || H <= 0 || T <= 0 || D != 64 || g_tc_variant != 0) return 0;
     const SegPlan plan = segment_plan(B, H, T);
-    return plan.len == 0 ? 0 : (long long)segment_scratch_bytes(plan.rows, H, T, plan.len);
+    return plan.len == 0 ? 0 : (long long)segment_scratch_bytes(plan.rows, H, T, equal_pieces(plan.len));
 }
 
 // the plain rule on prepared operands at head dim 64: rows of the batch whose chains are walked whole, then those that are cut
@@ -372,7 +374,7 @@ static int plain_with_segments(const PrefillArgs &all, int o_dtype, const SegPla
         a.S_out += chains * DD;
         if (a.sent != nullptr) a.sent += chains * NC * DD;
     }
-    a.seg_len = plan.len;
+    a.seg = equal_pieces(plan.len);
     a.seg_states = (const float *)scratch;
     const int rc = segment_states_launch(a, (float *)scratch, stream);
     return rc != PGB_OK ? rc : prefill_tc_ws_launch(a, o_dtype, stream);
@@ -476,7 +478,7 @@ int pgb_aspin_layer_prefill_fwd(const void *qp, const void *kp, const void *vp, 
 
 long long pgb_aspin_layer_windows_scratch_bytes(int B, int H, int T, int window) {
     if (B <= 0 || H <= 0 || T <= 0 || window <= 0) return 0;
-    return T <= window ? 0 : (long long)segment_scratch_bytes(B, H, T, window);
+    return T <= window ? 0 : (long long)segment_scratch_bytes(B, H, T, window < 64 || window % 64 ? equal_pieces(window) : windows_cut(B, H, T, window));
 }
 
 int pgb_aspin_layer_prefill_windows_ex(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
@@ -492,7 +494,9 @@ int pgb_aspin_layer_prefill_windows_ex(const void *qp, const void *kp, const voi
     if (B <= 0 || H <= 0 || T <= 0 || (long long)B * H > 65535 || aux_stride_b < 0 || aux_stride_t < H || in_stride_t < (long long)H * D ||
         in_stride_b < 0 || rot_T < (longest + 63) / 64 * 64 || (long long)B * H * ((T + window - 1) / window) > 0x7fffffffLL)
         return PGB_ERR_BAD_SHAPE;
-    if (T > window && (!scratch || scratch_bytes < pgb_aspin_layer_windows_scratch_bytes(B, H, T, window))) return PGB_ERR_BAD_SHAPE;
+    SegCut cut = windows_cut(B, H, T, window);
+    if (T > window && scratch_bytes < (long long)segment_scratch_bytes(B, H, T, cut)) cut = equal_pieces(window);
+    if (T > window && (!scratch || scratch_bytes < (long long)segment_scratch_bytes(B, H, T, cut))) return PGB_ERR_BAD_SHAPE;
     if (!aligned(qp, 16) || !aligned(kp, 16) || !aligned(vp, 16) || in_stride_b % 8 || in_stride_t % 8 || !aligned(o, 16) || !aligned(S_out, 16) ||
         !aligned(rot_table, 16) || (scratch && !aligned(scratch, 16)) || (S0 && !aligned(S0, 16)))
         return PGB_ERR_MISALIGNED;
@@ -517,7 +521,7 @@ int pgb_aspin_layer_prefill_windows_ex(const void *qp, const void *kp, const voi
             }
         return PGB_OK;
     }
-    a.seg_len = window; a.seg_rotates = 1; a.seg_states = T > window ? (const float *)scratch : nullptr;
+    a.seg = cut; a.seg_rotates = 1; a.seg_states = T > window ? (const float *)scratch : nullptr;
     if (T > window) {
         const int rc = segment_states_launch(a, (float *)scratch, (cudaStream_t)stream);
         if (rc != PGB_OK) return rc;

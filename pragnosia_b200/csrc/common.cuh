@@ -72,6 +72,29 @@ __device__ __forceinline__ float fast_exp2(float x) {
 __device__ __forceinline__ float fast_sigmoid(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
 __device__ __forceinline__ float fast_softplus(float x) { return x > 20.0f ? x : __logf(1.0f + __expf(x)); }
 
+// How a chain is cut into segments: the first `whole` pieces of `win` tokens (windows, or a prepared chain's equal pieces) as they are, each of
+// the others into parts of `len` (all whole chunks of 64). win 0: not cut.
+struct SegCut {
+    int whole = 0x7fffffff, win = 0, len = 0;
+    __host__ __device__ int parts() const { return (win + len - 1) / len; }
+    __host__ __device__ int count(int T) const {
+        const int n = (T + win - 1) / win;
+        if (n <= whole) return n;
+        const int rest = T - whole * win;
+        return whole + rest / win * parts() + (rest % win + len - 1) / len;
+    }
+    // segment s: its first token, that token's place in its piece, and the segment's tokens (the chain may end before)
+    __host__ __device__ void at(int s, int &begin, int &in_piece, int &tokens) const {
+        in_piece = 0; tokens = win; begin = s * win;
+        if (s >= whole) {
+            const int j = s - whole, P = parts(), piece = j / P;
+            in_piece = (j - piece * P) * len;
+            begin = (whole + piece) * win + in_piece;
+            tokens = win - in_piece < len ? win - in_piece : len;
+        }
+    }
+};
+
 // launch arguments shared between the C ABI layer and the kernels' translation units
 struct PrefillArgs {
     const void *q, *k, *v; const float *la, *beta, *S0; void *o; float *S_out; __nv_bfloat16 *sent;
@@ -84,8 +107,8 @@ struct PrefillArgs {
     // normalise / gate / rotate itself (gate_raw: write-gate logits with la_raw's strides; rot: table [H][rot_T][D/2])
     void *W_out = nullptr;                                            // delta rule: the residuals written, bf16 [BH][T][D]
     int raw = 0; long long raw_sb = 0, raw_st = 0; const void *gate_raw = nullptr; const float *rot = nullptr; int rot_T = 0;
-    // > 0: chains cut into segments (head dim 64; see TcParams), entered with seg_states from the second on
-    int seg_len = 0; const float *seg_states = nullptr; int seg_rotates = 0;
+    // seg.win > 0: chains cut into segments (head dim 64; see TcParams), entered with seg_states from the second on
+    SegCut seg; const float *seg_states = nullptr; int seg_rotates = 0;
     // plain rule on prepared operands: the scaled keys K w enter the state update in three bf16 terms instead of two, which is fp32's
     // own error on the final state (training, whose operators formed it in fp32: 2.1e-6 with two terms, 3.9e-7 in fp32)
     int fine = 0;

@@ -84,10 +84,12 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
     auto bar_q = [&](int s) { return mb + SM::bar_q + 8 * s; };           // P, U issued: tiles of c final    c&3
 
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5);
-    // A chain may be cut into segments of seg_len tokens (whole chunks), each with its own entering state: one CTA a segment.
-    // T, positions and chunks below are the segment's own; tb is its first token.
+    // A chain may be cut into segments (whole chunks), each with its own entering state: one CTA a segment.
+    // T and chunks below are the segment's own; tb is its first token, t_in that token's position in its window.
     const int seg = blockIdx.x / p.BH, bh = blockIdx.x - seg * p.BH, h = bh % p.H, b = bh / p.H;
-    const int tb = seg * p.seg_len, T = min(p.T - tb, p.seg_len), NC = (T + TC_C - 1) / TC_C;
+    int tb, t_in, seg_tokens;
+    p.seg.at(seg, tb, t_in, seg_tokens);
+    const int T = min(p.T - tb, seg_tokens), NC = (T + TC_C - 1) / TC_C;
     const float *S0 = seg == 0 ? p.S0 : p.seg_states + (size_t)(seg - 1) * p.BH * WS_D * WS_D;
     const int tma_c0 = RAW ? h * D : 0, tma_c2 = RAW ? b : bh;
 
@@ -219,7 +221,7 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
 #pragma unroll
         for (int j = 0; j < 16; ++j) S[j] = 0.f;
         if (S0 != nullptr) {
-            const float shift = p.theta == nullptr || (seg > 0 && !p.seg_rotates) ? 0.f : (p.shift_dev != nullptr ? *p.shift_dev : p.shift_host);
+            const float shift = p.theta == nullptr || (seg > 0 && (!p.seg_rotates || t_in > 0)) ? 0.f : (p.shift_dev != nullptr ? *p.shift_dev : p.shift_host);
 #pragma unroll
             for (int hi8 = 0; hi8 < 2; ++hi8) {
                 const int row = hi8 ? row1 : row0;
@@ -466,7 +468,7 @@ __global__ void __launch_bounds__(WS_NT, 1) prefill_tc_ws_kernel(const __grid_co
         auto load_rot = [&](int c) {
             if (RAW && lane == 0) {
                 mbar_expect_tx(bar_rot(c & 1), ROT_BYTES);
-                bulk_load_1d(base + SM::off_rot + (c & 1) * ROT_BYTES, p.rot + ((size_t)h * p.rot_T + (size_t)c * TC_C) * (D / 2), ROT_BYTES,
+                bulk_load_1d(base + SM::off_rot + (c & 1) * ROT_BYTES, p.rot + ((size_t)h * p.rot_T + t_in + (size_t)c * TC_C) * (D / 2), ROT_BYTES,
                              bar_rot(c & 1));
             }
             __syncwarp();
@@ -549,10 +551,12 @@ int prefill_tc_ws_launch(const PrefillArgs &a, int o_dtype, cudaStream_t stream)
         made = tc_make_map(&mq, a.q, BH, a.T, D, D, (long long)a.T * D) && tc_make_map(&mk, a.k, BH, a.T, D, D, (long long)a.T * D) &&
                tc_make_map(&mv, a.v, BH, a.T, D, D, (long long)a.T * D);
     if (!made) { set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled"); return PGB_ERR_CUDA; }
-    const int seg_len = a.seg_len > 0 ? a.seg_len : (a.T + TC_C - 1) / TC_C * TC_C, nseg = (a.T + seg_len - 1) / seg_len;
+    SegCut seg = a.seg;
+    if (seg.win == 0) seg.win = (a.T + TC_C - 1) / TC_C * TC_C;
+    const int nseg = seg.count(a.T);
     TcParams p{a.la, a.S0, a.theta, a.shift_dev, a.shift_host, a.o, a.S_out, a.sent, a.H, a.T, o_dtype == PGB_F32,
                (const __nv_bfloat16 *)a.la_raw, a.la_sb, a.la_st, a.decay_A, a.rms_w, a.rms_eps, a.o_token_major,
-               (const __nv_bfloat16 *)a.gate_raw, (const float2 *)a.rot, a.rot_T, BH, seg_len, a.seg_states, a.seg_rotates};
+               (const __nv_bfloat16 *)a.gate_raw, (const float2 *)a.rot, a.rot_T, BH, seg, a.seg_states, a.seg_rotates};
     auto go = [&](auto kern) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WsSmem::bytes);
         return e != cudaSuccess ? e : pdl_launch(kern, dim3((unsigned)(BH * nseg)), dim3(WS_NT), (size_t)WsSmem::bytes, stream, mq, mk, mv, p);

@@ -339,9 +339,9 @@ struct TcParams {
     const float *rms_w; float rms_eps; int o_token_major;
     // RAW mode: write-gate logits (same strides as la_raw) and the rotation table [H][rot_T][D/2] of (cos, sin)
     const __nv_bfloat16 *gate_raw; const float2 *rot; int rot_T;
-    // warp-specialised kernel: chains, and tokens of a segment (>= T: one segment, entered with S0; else the states entering
-    // segments 1, 2, ... are seg_states [nseg - 1][BH][D][D], rebased like S0 where seg_rotates)
-    int BH, seg_len; const float *seg_states; int seg_rotates;
+    // warp-specialised kernel: chains, and their segments (the first is entered with S0, the states entering segments 1, 2, ... are
+    // seg_states [nseg - 1][BH][D][D], where seg_rotates rebased like S0 at a piece's beginning)
+    int BH; SegCut seg; const float *seg_states; int seg_rotates;
 };
 
 

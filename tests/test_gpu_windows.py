@@ -50,6 +50,12 @@ def test_all_windows_at_once_match_window_by_window(delta, head_dim, window, T, 
     assert rel(m.mix_windows(z, window, pos, tail)[0], got[:, T - tail:]) <= 5e-3
 
 
+@pytest.mark.parametrize("window,T", [(512, 13 * 512 + 200), (256, 14 * 256 + 1), (1024, 12 * 1024 + 900), (320, 20 * 320)])
+def test_windows_of_the_last_round_in_parts(window, T):
+    """Twelve chains of more windows than SMs: whole windows, then those of the last round cut into parts (a ragged one last)."""
+    test_all_windows_at_once_match_window_by_window(False, 64, window, T, 3)
+
+
 @pytest.mark.parametrize("mixer", ["aspin", "dspin"])
 def test_shape_graphs_and_what_the_caller_keeps(mixer):
     """First call eager, second captured, later ones replayed: the same logits and states every time, and a state kept from one
