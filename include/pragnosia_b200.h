@@ -227,6 +227,9 @@ int pgb_aspin_delta_prefill_fwd(const void *q, const void *k, const void *v, con
                                 int o_dtype, float *S_out, void *sent, void *x_scratch, long long x_scratch_bytes, int B,
                                 int H, int T, int D, void *stream);
 long long pgb_aspin_delta_scratch_bytes(int B, int H, int T);
+/* What pgb_aspin_delta_prefill_fwd can use of x_scratch: with this much, a call without `sent` whose chains are few (head dim 64) walks segments of them
+ * side by side; with less (but the size above) each chain as a whole. Never more than 256 MiB above it. */
+long long pgb_aspin_delta_prefill_scratch_bytes(int B, int H, int T, int D);
 
 /* ---------------------------------------------------------------------------------------------------------
  * pgb_aspin_delta_prefill_fwd without the x_scratch argument. It has no counterpart in the reference.
@@ -327,6 +330,7 @@ int pgb_aspin_layer_prefill_windows_ex(const void *qp, const void *kp, const voi
                                         const float *decay_A, const float *rot_table, int rot_T, const float *theta, const float *S0, const float *rms_weight,
                                         float rms_eps, void *o, float *S_out, void *scratch, long long scratch_bytes, int window, int B, int H,
                                         int T, int D, void *stream);
+long long pgb_aspin_delta_layer_scratch_least_bytes(int B, int H, int T, int D);   /* taken as well: the chains are then walked whole */
 long long pgb_aspin_delta_layer_scratch_bytes(int B, int H, int T, int D);
 int pgb_aspin_delta_layer_windows_fwd(const void *qp, const void *kp, const void *vp, long long in_stride_b, long long in_stride_t,
                                       const void *decay_logits, const void *beta_logits, long long aux_stride_b, long long aux_stride_t,

@@ -36,6 +36,7 @@ SIGNATURES = {
     "pgb_aspin_prefill_fp32_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _vp],
     "pgb_aspin_delta_prefill_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _vp],
     "pgb_aspin_delta_scratch_bytes": [_i, _i, _i],
+    "pgb_aspin_delta_prefill_scratch_bytes": [_i, _i, _i, _i],
     "pgb_aspin_delta_prefill_noscratch_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _vp, _i, _vp, _vp, _i, _i, _i, _i, _vp],
     "pgb_aspin_delta_prefill_train_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _vp],
     "pgb_aspin_train_scratch_bytes": [_i, _i, _i, _i, _i],
@@ -50,6 +51,7 @@ SIGNATURES = {
     "pgb_aspin_layer_prefill_windows_ex": [_vp, _vp, _vp, _ll, _ll, _vp, _vp, _ll, _ll, _vp, _vp, _i, _vp, _vp, _vp, _f, _vp, _vp, _vp, _ll,
                                            _i, _i, _i, _i, _i, _vp],
     "pgb_aspin_delta_layer_scratch_bytes": [_i, _i, _i, _i],
+    "pgb_aspin_delta_layer_scratch_least_bytes": [_i, _i, _i, _i],
     "pgb_aspin_delta_layer_windows_fwd": [_vp, _vp, _vp, _ll, _ll, _vp, _vp, _ll, _ll, _vp, _vp, _vp, _vp, _f, _vp, _vp, _vp, _ll,
                                           _i, _i, _i, _i, _i, _vp],
     "pgb_aspin_delta_layer_windows_ex": [_vp, _vp, _vp, _ll, _ll, _vp, _vp, _ll, _ll, _vp, _vp, _vp, _vp, _vp, _f, _vp, _vp, _vp, _ll,

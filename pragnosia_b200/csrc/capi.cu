@@ -60,6 +60,9 @@ int train_bwd_launch(const TrainBwdArgs &, int, cudaStream_t);
 int tc_train_error_flag(int *);
 int prep_gates_launch(const void *, const void *, const void *, long long, long long, long long, const void *, const void *, long long, long long,
                       const float *, const float *, const long long *, void *, void *, void *, float *, float *, int, int, int, int, cudaStream_t);
+size_t delta_segment_scratch_bytes(int B, int H, int T, int D);
+int delta_segments_launch(const PrefillArgs &, int, void *, void *, cudaStream_t);
+int delta_segments_error_flag(int *);
 int head_norm_launch(const void *, const float *, float, void *, int, int, int, int, cudaStream_t);
 size_t segment_scratch_bytes(int B, int H, int T, const SegCut &seg);
 SegCut windows_cut(int B, int H, int T, int window);
@@ -120,12 +123,15 @@ static int tc_dispatch(const PrefillArgs &a, int o_dtype, int D, cudaStream_t st
 
 // one buffer for what lies between the delta layer's two GEMMs: the scan's operands and output, gates, inverses
 struct DeltaLayerScratch {
-    size_t q, k, v, o, la, beta, x, bytes;
+    size_t q, k, v, o, la, beta, x, seg, bytes, plain_bytes;          // seg: for segments side by side, where few chains are planned so
     DeltaLayerScratch(long long B, long long H, long long T, int D) {
         auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
         const size_t rows = (size_t)(B * H * T), tile = up(rows * D * 2);
         q = 0; k = tile; v = 2 * tile; o = 3 * tile; la = 4 * tile; beta = la + up(rows * 4); x = beta + up(rows * 4);
-        bytes = x + prefill_tc_delta_scratch_bytes((int)B, (int)H, (int)T);
+        plain_bytes = x + prefill_tc_delta_scratch_bytes((int)B, (int)H, (int)T);
+        seg = up(plain_bytes);
+        const size_t n = delta_segment_scratch_bytes((int)B, (int)H, (int)T, D);
+        bytes = n > 0 ? seg + n : plain_bytes;
     }
 };
 
@@ -552,7 +558,7 @@ int pgb_aspin_delta_layer_windows_ex(const void *qp, const void *kp, const void 
         window % 64 != 0)
         return PGB_ERR_BAD_SHAPE;
     if ((long long)B * H > 65535 || (T + 63) / 64 > 65535) return PGB_ERR_TOO_LARGE;
-    if (scratch_bytes < pgb_aspin_delta_layer_scratch_bytes(B, H, T, D)) return PGB_ERR_BAD_SHAPE;
+    if (scratch_bytes < (long long)DeltaLayerScratch(B, H, T, D).plain_bytes) return PGB_ERR_BAD_SHAPE;
     if (!aligned(qp, 16) || !aligned(kp, 16) || !aligned(vp, 16) || in_stride_b % 8 || in_stride_t % 8 || !aligned(o, 16) || !aligned(S_out, 16) ||
         !aligned(scratch, 256) || !aligned(theta, 16) || !aligned(rms_weight, 16) || (S0 && !aligned(S0, 16)))
         return PGB_ERR_MISALIGNED;
@@ -565,6 +571,10 @@ int pgb_aspin_delta_layer_windows_ex(const void *qp, const void *kp, const void 
     if (rc != PGB_OK) return rc;
     PrefillArgs a{q, k, v, la, beta, S0, os, S_out, nullptr, theta, nullptr, (float)window, B, H, T};
     a.rebase_chunks = window / 64;
+    if (sc.bytes > sc.plain_bytes && scratch_bytes >= (long long)sc.bytes) {
+        a.o = o; a.rms_w = rms_weight; a.rms_eps = rms_eps; a.o_token_major = 1;
+        return delta_segments_launch(a, PGB_BF16, buf + sc.x, buf + sc.seg, (cudaStream_t)stream);
+    }
     rc = prefill_tc_delta_launch(a, PGB_BF16, D, buf + sc.x, (cudaStream_t)stream);
     return rc != PGB_OK ? rc : head_norm_launch(os, rms_weight, rms_eps, o, B, T, H, D, (cudaStream_t)stream);
 }
@@ -578,6 +588,9 @@ int pgb_aspin_delta_layer_windows_fwd(const void *qp, const void *kp, const void
                                             pos, nullptr, rms_weight, rms_eps, o, S_out, scratch, scratch_bytes, window, B, H, T, D, stream);
 }
 
+long long pgb_aspin_delta_layer_scratch_least_bytes(int B, int H, int T, int D) {
+    return B <= 0 || H <= 0 || T <= 0 || (D != 64 && D != 128) ? 0 : (long long)DeltaLayerScratch(B, H, T, D).plain_bytes;
+}
 long long pgb_aspin_delta_layer_scratch_bytes(int B, int H, int T, int D) {
     if (B <= 0 || H <= 0 || T <= 0 || (D != 64 && D != 128)) return 0;
     return (long long)DeltaLayerScratch(B, H, T, D).bytes;
@@ -865,6 +878,8 @@ int pgb_tc_error_flag(int *out_host) {
     f = f > g ? f : g;
     if (rc == PGB_OK) rc = decode_linear_error_flag(&g);
     f = f > g ? f : g;
+    if (rc == PGB_OK) rc = delta_segments_error_flag(&g);
+    f = f > g ? f : g;
     e = e > f ? e : f;
     b = b > c ? b : c;
     b = b > d ? b : d;
@@ -876,6 +891,12 @@ int pgb_tc_error_flag(int *out_host) {
 long long pgb_aspin_delta_scratch_bytes(int B, int H, int T) {
     if (B <= 0 || H <= 0 || T <= 0) return 0;
     return (long long)prefill_tc_delta_scratch_bytes(B, H, T);
+}
+
+long long pgb_aspin_delta_prefill_scratch_bytes(int B, int H, int T, int D) {
+    if (B <= 0 || H <= 0 || T <= 0) return 0;
+    const long long x = pgb_aspin_delta_scratch_bytes(B, H, T), seg = (long long)delta_segment_scratch_bytes(B, H, T, D);
+    return seg > 0 ? (x + 255) / 256 * 256 + seg : x;
 }
 
 int pgb_aspin_delta_prefill_fwd(const void *q, const void *k, const void *v, const float *la, const float *beta, const float *S0,
@@ -892,6 +913,9 @@ int pgb_aspin_delta_prefill_fwd(const void *q, const void *k, const void *v, con
         (S0 && !aligned(S0, 16)) || (sent && !aligned(sent, 16)) || !aligned(x_scratch, 16))
         return PGB_ERR_MISALIGNED;
     PrefillArgs a{q, k, v, la, beta, S0, o, S_out, (__nv_bfloat16 *)sent, theta, shift_dev, shift_host, B, H, T};
+    const long long x = (pgb_aspin_delta_scratch_bytes(B, H, T) + 255) / 256 * 256, seg = (long long)delta_segment_scratch_bytes(B, H, T, D);
+    if (seg > 0 && sent == nullptr && x_scratch_bytes >= x + seg)
+        return delta_segments_launch(a, o_dtype, x_scratch, (char *)x_scratch + x, (cudaStream_t)stream);
     return prefill_tc_delta_launch(a, o_dtype, D, x_scratch, (cudaStream_t)stream);
 }
 

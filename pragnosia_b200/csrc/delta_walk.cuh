@@ -44,6 +44,8 @@ struct DwParams {
     const float *dW0, *Dc;                                            // backward inputs
     int H, T, o_is_f32, want_sent, want_w, rebase_chunks;                               // rebase_chunks > 0: the state is rotated by -shift theta every so many chunks
     float rebase_shift;
+    int BH, seg_chunks;                                               // WITH_MAP: chains, chunks of a segment; S_out and S_map are [segment][BH][D][D]
+    float *S_map;
 };
 
 // tensor maps: tiles in, and what a warp stores 32 value columns at a time (a lane owns a column; its rows are staged in
@@ -99,10 +101,15 @@ struct DwStore {
     }
 };
 
-template <int D, bool BWD>
+// WITH_MAP (forward, head dim 64): a CTA walks one SEGMENT of a chain, entered with S0 by the first segment and with zero by the others, and in the 64 lanes that
+// the value columns leave idle (a product of 128 rows takes as long as one of 64) the segment's linear map of the state: the same walk with V = 0 and the
+// identity as the entering state. Its outputs q_t^T (map to t) go to m.w, the map to the segment's end to S_map; what S adds to the outputs and to
+// the state behind the segment is then a product each (delta_segments.cu), and the segments of a chain need not wait for one another.
+template <int D, bool BWD, bool WITH_MAP = false>
 __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_constant__ DwMaps m, DwParams p) {
     using SM = DwSmem<D, BWD>;
-    constexpr int SUB = D / 64, NMATH = 2 * (D / 32), KH = D / 2;     // math warps with live lanes; keys a math thread owns
+    static_assert(!WITH_MAP || (D == 64 && !BWD), "the map lies in the lanes that head dim 64 leaves idle");
+    constexpr int SUB = D / 64, NMATH = WITH_MAP ? DW_MATH : 2 * (D / 32), KH = D / 2;     // math warps with live lanes; keys a math thread owns
     constexpr uint32_t TM_S = 0, TM_SH = D, TM_SL = TM_SH + D / 2;    // S^T in fp32; its heads and tails
     constexpr uint32_t TM_WWH = TM_SH, TM_WWL = TM_SH + 32;           // (w W)^T reuses their columns: consumed by then
     constexpr uint32_t TM_KS = 2 * D, TM_QS = TM_KS + 64, TM_RH = TM_QS + 64, TM_RL = TM_RH + 32, TM_P = TM_RL + 32, TM_COLS = 512;
@@ -125,9 +132,9 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
     // warp index and tensor-memory base through a shuffle: values the compiler then knows to be uniform over the warp, so the
     // MMA's operands stay in uniform registers (an MMA issued every 34 cycles instead of every 110)
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5), sub = warp & 3;
-    const int bh = blockIdx.x, h = bh % p.H;
-    const int T = p.T, NC = (T + TC_C - 1) / TC_C;
-    auto chunk = [&](int i) { return BWD ? NC - 1 - i : i; };
+    const int seg = WITH_MAP ? blockIdx.x / p.BH : 0, bh = WITH_MAP ? blockIdx.x - seg * p.BH : blockIdx.x, h = bh % p.H;
+    const int T = p.T, NCT = (T + TC_C - 1) / TC_C, c_first = WITH_MAP ? seg * p.seg_chunks : 0, NC = WITH_MAP ? min(p.seg_chunks, NCT - c_first) : NCT;
+    auto chunk = [&](int i) { return BWD ? NC - 1 - i : c_first + i; };
 
     if (tid == 0) {
         for (int s = 0; s < 4; ++s) {
@@ -156,8 +163,9 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
 
     if (warp < DW_MATH) {
         // ====================================================================================================== math
-        if (sub * 32 < D) {
-            const int v = 32 * sub + lane, g = warp >> 2;             // value column; which half of the tokens / keys
+        if (WITH_MAP || sub * 32 < D) {
+            const bool map = WITH_MAP && sub >= 2;                    // this warp's lanes hold the map's columns
+            const int v = 32 * (WITH_MAP ? sub & 1 : sub) + lane, g = warp >> 2;      // value column; which half of the tokens / keys
             const int k0 = g * KH;
             const uint32_t lb = tmem + ((uint32_t)(32 * sub) << 16);
             const size_t sbase = (size_t)bh * D * D + (size_t)k0 * D + v;
@@ -168,12 +176,12 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
                 if (lane == 0) mbar_arrive(bar);
             };
             {
-                const float shift = (BWD || p.S0 == nullptr || p.theta == nullptr) ? 0.f : (p.shift_dev != nullptr ? *p.shift_dev : p.shift_host);
+                const float shift = (BWD || map || seg > 0 || p.S0 == nullptr || p.theta == nullptr) ? 0.f : (p.shift_dev != nullptr ? *p.shift_dev : p.shift_host);
 #pragma unroll 1
                 for (int b = 0; b < KH; b += 16) {
                     float x[16];
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) x[k] = p.S0 != nullptr ? p.S0[sbase + (size_t)(b + k) * D] : 0.f;
+                    for (int k = 0; k < 16; ++k) x[k] = map ? (k0 + b + k == v ? 1.f : 0.f) : p.S0 != nullptr && seg == 0 ? p.S0[sbase + (size_t)(b + k) * D] : 0.f;
                     if (shift != 0.f) {
 #pragma unroll
                         for (int k = 0; k < 16; k += 2) {
@@ -239,7 +247,7 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
                 } else {
                     if (!(ok = mbar_wait_warp(full(st), (i / SM::NST) & 1, 12))) break;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) d0[j] = __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t *>(vt + swz(32 * g + j, vj)) << 16);
+                    for (int j = 0; j < 32; ++j) d0[j] = map ? 0.f : __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t *>(vt + swz(32 * g + j, vj)) << 16);
 #pragma unroll
                     for (int j = 0; j < 32; j += 4) {
                         const float4 bb = *reinterpret_cast<const float4 *>(bes + 32 * g + j);
@@ -298,9 +306,9 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
                     }
                 }
                 if (BWD) {
-                    out.end(&m.g, 32 * sub, k0, (bh * NC + c) * 2);
-                    out2.end(&m.g, 32 * sub, k0, (bh * NC + c) * 2 + 1);
-                } else if (keep) out.end(&m.sent, 32 * sub, k0, bh * NC + c);
+                    out.end(&m.g, 32 * sub, k0, (bh * NCT + c) * 2);
+                    out2.end(&m.g, 32 * sub, k0, (bh * NCT + c) * 2 + 1);
+                } else if (keep) out.end(&m.sent, 32 * sub, k0, bh * NCT + c);
                 // ---- 3. W (or dR), scaled, as the operand of the state update; then W itself, which only O1 waits for
                 if (!(ok = mbar_wait_warp(mb + SM::b_w, i & 1, 14))) break;
                 tc_fence_after();
@@ -357,7 +365,7 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
                     tmem_ld16_nowait(lb + TM_S + k0 + b, x);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) p.S_out[sbase + (size_t)(b + k) * D] = x[k];
+                    for (int k = 0; k < 16; ++k) (map ? p.S_map : p.S_out)[(size_t)seg * (WITH_MAP ? p.BH : 0) * D * D + sbase + (size_t)(b + k) * D] = x[k];
                 }
             }
         }
@@ -365,7 +373,9 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
         // ====================================================================================================== output
         if constexpr (!BWD) {
             const uint32_t lb = tmem + ((uint32_t)(32 * sub) << 16);
-            const bool mine = 32 * sub < D;                           // this warp's lanes hold value columns
+            const bool mine = WITH_MAP ? sub < 2 || seg > 0 : 32 * sub < D;   // this warp's lanes hold value columns, or the map's where it is wanted
+            const CUtensorMap *to = WITH_MAP && sub >= 2 ? &m.w : &m.o;
+            const int col = 32 * (WITH_MAP ? sub & 1 : sub);
             const uint32_t slot = SM::off_out + DW_MATH * SM::MSLOT + sub * SM::TSLOT;
             const DwStore out{sm + slot, base + slot, lane};
             const DwStore half2{out.slot + 2048, out.addr + 2048, lane};
@@ -407,16 +417,16 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
                     if (p.o_is_f32) {
 #pragma unroll
                         for (int j = 0; j < 32; ++j) out.put(j, y[j]);
-                        out.end(&m.o, 32 * sub, i * TC_C, bh);
+                        out.end(to, col, chunk(i) * TC_C, bh);
                         out.begin();
 #pragma unroll
                         for (int j = 0; j < 32; ++j) out.put(j, y[32 + j]);
-                        out.end(&m.o, 32 * sub, i * TC_C + 32, bh);
+                        out.end(to, col, chunk(i) * TC_C + 32, bh);
                     } else {
 #pragma unroll
                         for (int j = 0; j < 64; ++j) out.put(j, __float2bfloat16_rn(y[j]));
-                        out.end(&m.o, 32 * sub, i * TC_C, bh);
-                        half2.end(&m.o, 32 * sub, i * TC_C + 32, bh);
+                        out.end(to, col, chunk(i) * TC_C, bh);
+                        half2.end(to, col, chunk(i) * TC_C + 32, bh);
                     }
                 }
             }
@@ -569,8 +579,8 @@ __global__ void __launch_bounds__(DW_NT, 1) delta_walk_kernel(const __grid_const
                 if constexpr (SM::FETCH_DC) bulk_load_1d(sb + SM::o_dc, p.Dc + ((size_t)bh * NC + c) * D * D, dcb, bar);
 #pragma unroll
                 for (int s = 0; s < SUB; ++s) tma_load_3d(sb + SM::o_k + s * 8192, &m.k, bar, 64 * s, t0, bh);
-                tma_load_3d(sb + SM::o_x, &m.x, bar, 0, 0, (bh * NC + c) * 2);
-                tma_load_3d(sb + SM::o_x + SM::SQ, &m.x, bar, 0, 0, (bh * NC + c) * 2 + 1);
+                tma_load_3d(sb + SM::o_x, &m.x, bar, 0, 0, (bh * NCT + c) * 2);
+                tma_load_3d(sb + SM::o_x + SM::SQ, &m.x, bar, 0, 0, (bh * NCT + c) * 2 + 1);
                 if constexpr (!BWD) {
 #pragma unroll
                     for (int s = 0; s < SUB; ++s) {

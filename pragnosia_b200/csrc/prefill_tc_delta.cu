@@ -249,6 +249,22 @@ __global__ void __launch_bounds__(128, 9) delta_inv_kernel(const __grid_constant
 
 // ------------------------------------------------------------------------------------------------ host side
 template <int D>
+static int delta_inverse_go(const PrefillArgs &a, void *x_scratch, cudaStream_t stream) {
+    const int BH = a.B * a.H, NC = (a.T + TC_C - 1) / TC_C;
+    CUtensorMap mk;
+    if (!tc_make_map(&mk, a.k, BH, a.T, D, D, (long long)a.T * D)) { set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled"); return PGB_ERR_CUDA; }
+    auto inv = delta_inv_kernel<D>;
+    const cudaError_t e = cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, InvSmem::bytes);
+    if (e != cudaSuccess) { set_cuda_error(e, "delta_inv smem attribute"); return PGB_ERR_CUDA; }
+    inv<<<dim3(NC, BH), 128, InvSmem::bytes, stream>>>(mk, a.la, a.beta, (__nv_bfloat16 *)x_scratch, a.T, 1);
+    return check_launch("delta_inv_kernel");
+}
+// the inverses of the chunks of `a` into x_scratch
+int delta_inverse_launch(const PrefillArgs &a, int D, void *x_scratch, cudaStream_t stream) {
+    return D == 64 ? delta_inverse_go<64>(a, x_scratch, stream) : delta_inverse_go<128>(a, x_scratch, stream);
+}
+
+template <int D>
 static int delta_go(const PrefillArgs &a, int o_dtype, void *x_scratch, cudaStream_t stream) {
     const int BH = a.B * a.H, NC = (a.T + TC_C - 1) / TC_C;
     const bool f32 = o_dtype == PGB_F32;
@@ -262,13 +278,10 @@ static int delta_go(const PrefillArgs &a, int o_dtype, void *x_scratch, cudaStre
         set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled");
         return PGB_ERR_CUDA;
     }
-    auto inv = delta_inv_kernel<D>;
     auto walk = delta_walk_kernel<D, false>;
-    cudaError_t e = cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, InvSmem::bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, DwSmem<D, false>::bytes);
+    cudaError_t e = cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, DwSmem<D, false>::bytes);
     if (e != cudaSuccess) { set_cuda_error(e, "delta_walk smem attribute"); return PGB_ERR_CUDA; }
-    inv<<<dim3(NC, BH), 128, InvSmem::bytes, stream>>>(m.k, a.la, a.beta, (__nv_bfloat16 *)x_scratch, a.T, 1);
-    int rc = check_launch("delta_inv_kernel");
+    const int rc = delta_inverse_go<D>(a, x_scratch, stream);
     if (rc != PGB_OK) return rc;
     DwParams p{};
     p.la = a.la; p.beta = a.beta; p.S0 = a.S0; p.theta = a.theta; p.shift_dev = a.shift_dev; p.shift_host = a.shift_host;

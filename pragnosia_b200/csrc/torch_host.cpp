@@ -291,8 +291,15 @@ ScanOut prefill(const Tensor &q_, const Tensor &k_, const Tensor &v_, const Tens
     const int oc = code(o);
     if (beta.defined() && dt == at::kBFloat16 && precision != PGB_PREFILL_FP32 && B * H <= 65535) {
         // delta rule on the tensor cores: the chunk inverses go through a scratch buffer
-        const long long n = pgb_aspin_delta_scratch_bytes(B, H, T);
-        const Tensor scratch = bytes(q, n);
+        long long n = want_sent ? pgb_aspin_delta_scratch_bytes(B, H, T) : pgb_aspin_delta_prefill_scratch_bytes(B, H, T, D);
+        Tensor scratch;
+        try {
+            scratch = bytes(q, n);
+        } catch (const c10::OutOfMemoryError &) {                     // without the segments' share, then
+            const long long least = pgb_aspin_delta_scratch_bytes(B, H, T);
+            if (n == least) throw;
+            scratch = bytes(q, n = least);
+        }
         check(pgb_aspin_delta_prefill_fwd(vp(q), vp(k), vp(v), fp(la), fp(beta), fp(S0), fp(theta), fp(shift), shift_host, vp(o), oc, fp(S), vp(sent),
                                           vp(scratch), n, B, H, T, D, dev.stream), "pgb_aspin_delta_prefill_fwd");
         return {o, S, some(sent)};

@@ -290,7 +290,13 @@ def delta_layer_windows(qp, kp, vp, decay_logits, beta_logits, decay_A, theta, p
     S = _state_out(S_out, B, H, D, qp.device)
     L = lib()
     nbytes = L.pgb_aspin_delta_layer_scratch_bytes(B, H, T, D)
-    scratch = torch.empty(nbytes, device=qp.device, dtype=torch.uint8)
+    try:
+        scratch = torch.empty(nbytes, device=qp.device, dtype=torch.uint8)
+    except torch.cuda.OutOfMemoryError:                      # without the share that lets segments of few chains run side by side
+        least = L.pgb_aspin_delta_layer_scratch_least_bytes(B, H, T, D)
+        if least == nbytes:
+            raise
+        nbytes, scratch = least, torch.empty(least, device=qp.device, dtype=torch.uint8)
     S0 = _f32c(S0)
     sbq = qp.stride(0) if B > 1 else T * qp.stride(1)
     sba = decay_logits.stride(0) if B > 1 else T * decay_logits.stride(1)

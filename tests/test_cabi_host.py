@@ -156,6 +156,11 @@ def test_new_entry_points_reject_bad_calls(L):
     assert lin(B=65) == 7 and lin(K=768 * 16) == 7 and lin(K=12) == 2 and lin(resid=one) == 1 and lin(logits=one) == 1 and lin(y=None) == 1
     assert lin(window=512) == 1 and lin(y=ctypes.c_void_p(0x1004)) == 4
     assert L.pgb_decode_embed_norm(one, one, one, one, None, one, one, one, 4, 768, 100, 16, None) == 1
+    # delta rule: scratch beyond the inverses where few chains at head dim 64 are walked in segments side by side, never more than 256 MiB of it
+    x, more = L.pgb_aspin_delta_scratch_bytes, L.pgb_aspin_delta_prefill_scratch_bytes
+    assert more(3, 12, 1333, 64) > x(3, 12, 1333) and more(1, 2, 2048, 64) > x(1, 2, 2048) and more(3, 12, 1333, 128) == x(3, 12, 1333)
+    assert more(8, 16, 8192, 64) == x(8, 16, 8192) and more(1, 2, 128, 64) == x(1, 2, 128) and more(1, 1, 1 << 22, 64) == x(1, 1, 1 << 22)
+    assert 0 <= L.pgb_aspin_delta_layer_scratch_bytes(3, 12, 1333, 64) - L.pgb_aspin_delta_layer_scratch_least_bytes(3, 12, 1333, 64) <= 256 << 20
     # the same step without barriers: 32-bit words of every layer's exchanges; 0 where a row does not fit a stage or the rows shared memory
     assert L.pgb_decode_flow_work_bytes(12, 2, 768, 2328, 3072) == 4 * 12 * 2 * (2328 + 3 * 768 + 3072)
     assert L.pgb_decode_flow_work_bytes(12, 1, 3200, 9624, 12800) == 0 and L.pgb_decode_flow_work_bytes(12, 4, 2048, 6208, 8192) == 0

@@ -1,0 +1,36 @@
+"""The delta rule with few chains, segments side by side (delta_segments.cu), against the same call given the inverses' scratch only, which walks every
+chain as a whole. Each is 5.2e-6 (o) and 3.6e-6 (S) from 64 bits in the 2-norm, so the two lie within the sums of those."""
+import ctypes
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+from pragnosia_b200 import _lib, ops
+
+pytestmark = pytest.mark.gpu
+torch.set_grad_enabled(False)
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("B,H,T", [(3, 12, 1333), (1, 2, 2048), (1, 12, 4000), (1, 5, 1025), (2, 3, 700), (1, 40, 2048), (1, 1, 8192)])
+@pytest.mark.parametrize("S0,shift", [(False, 0.0), (True, 0.0), (True, 37.0)])
+def test_segments_side_by_side_match_whole_chains(B, H, T, S0, shift):
+    D, L = 64, _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(T + H)
+    rn = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    q, k, v = rn(B, H, T, D).bfloat16(), F.normalize(rn(B, H, T, D), dim=-1).bfloat16(), rn(B, H, T, D).bfloat16()
+    la, beta, th = F.logsigmoid(2.0 + rn(B, H, T)), torch.sigmoid(rn(B, H, T)), rn(H, D // 2).abs()
+    S_in = rn(B, H, D, D) if S0 else None
+    n = L.pgb_aspin_delta_scratch_bytes(B, H, T)
+    assert L.pgb_aspin_delta_prefill_scratch_bytes(B, H, T, D) > n                       # these are cut
+    p = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    whole = [torch.empty(B, H, T, D, device=DEV), torch.empty(B, H, D, D, device=DEV)]
+    x = torch.empty(n, device=DEV, dtype=torch.uint8)
+    assert L.pgb_aspin_delta_prefill_fwd(p(q), p(k), p(v), p(la), p(beta), p(S_in), p(th), None, shift, p(whole[0]), 0, p(whole[1]), None, p(x), n, B, H, T, D,
+                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    o, S, _ = ops.prefill(q, k, v, la, beta, S_in, theta=th, shift=shift, out_dtype=torch.float32)
+    rel = lambda a, b: float((a.double() - b.double()).norm() / b.double().norm())
+    assert rel(o, whole[0]) <= 1.1e-5 and rel(S, whole[1]) <= 7.5e-6, (rel(o, whole[0]), rel(S, whole[1]))
+    ob, Sb, _ = ops.prefill(q, k, v, la, beta, S_in, theta=th, shift=shift)
+    assert torch.equal(ob, o.bfloat16()) and torch.equal(Sb, S)                          # the bf16 read is the fp32 one, rounded
