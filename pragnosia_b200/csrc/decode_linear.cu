@@ -12,7 +12,7 @@
 //     weight; rounded once, as the normalised row would be) and each row's sum of squares by tiles; here x w is multiplied, and the row's
 //     1 / rms applied to the fp32 sum.
 //
-// A token of 12 layers of 768 (graph replay): batch 64 421 -> 316 us, batch 16 383 -> 240, batch 5 372 -> 223, against the library's products with
+// A token of 12 layers of 768 (graph replay): batch 64 421 -> 315 us, batch 16 383 -> 240, batch 5 372 -> 223, against the library's products with
 // separate norms. What bounds it now is the chain: at batch 5 3.6 us a link, of which 1.6 are the launch alone (links that return behind their wait), 0.8 x (only the
 // batch's rows are fetched: all 64 took 0.4 more), 0.9 the sums of squares, products and waits, 0.3 the exchange, 0.5 the way out; 5.2 at batch 64
 // (48 KB of x a CTA; of the 12.6 MB of states a layer, their stores are 0.3). An L2 prefetch of the weights two links ahead gave nothing, one barrier for

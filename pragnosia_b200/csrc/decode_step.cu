@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(DEC_THREADS) decode_step_kernel(DecodeArgs a) 
 // shared memory. With enough pairs to fill the SMs with warps (configuration 2's 64 sequences: 768) the step is one round
 // of loads, a few hundred instructions and one round of stores and is a seventh shorter than the block-per-head kernel
 // above with its three barriers; at large batches both run at the HBM rate; with few pairs the block kernel is quicker.
-constexpr int DW_WARPS = 2;                                           // (sequence, head) units per CTA: small, so that 768 of them spread evenly (four: 3 % a token more)
+constexpr int DW_WARPS = 4;                                           // (sequence, head) units per CTA
 
 template <typename TIN, typename TOUT, bool DELTA>
 __global__ void __launch_bounds__(DW_WARPS * 32) decode_step_warp_kernel(DecodeArgs a) {
@@ -133,7 +133,9 @@ __global__ void __launch_bounds__(DW_WARPS * 32) decode_step_warp_kernel(DecodeA
 // kernel; 2: the warp-per-head kernel at any size (A/B timing, tests). Measured inside the configuration-2 decode step
 // (graph replay, ms per token, block / warp kernel): batch 64 (768 pairs) 0.507 / 0.494, the kernel itself 8.9 / 7.6 us
 // against 3.9 us of bytes; batch 16 (192 pairs) 0.467 / 0.477 and batch 8 0.476 / 0.491 -- with few pairs a pair is better
-// served by 256 threads than by one warp's few hundred instructions in a row; batch 1024: the same 70 us (the HBM rate).
+// served by 256 threads than by one warp's few hundred instructions in a row; batch 1024: the same 70 us (the HBM rate). In the chained step, whose state
+// is loaded ahead of the wait, the block kernel is the quicker or as quick at every batch (64: 315-317 against 318-327 us a token, 48: 294-299
+// against 302-312, two warps a pair, a column a lane, in between): there it is always taken.
 constexpr int DW_MIN_UNITS = 512;
 static int g_decode_variant = 0;
 int decode_variant() { return g_decode_variant; }
@@ -147,7 +149,7 @@ template <typename TIN, typename TOUT>
 static int decode_dispatch(const DecodeArgs &a, int D, int delta, cudaStream_t stream) {
     const unsigned grid = (unsigned)(a.B * a.H);
     cudaError_t e;
-    if (D == 64 && (g_decode_variant == 2 || (g_decode_variant == 0 && grid >= (unsigned)DW_MIN_UNITS))) {
+    if (D == 64 && (g_decode_variant == 2 || (g_decode_variant == 0 && !a.early && grid >= (unsigned)DW_MIN_UNITS))) {
         const unsigned gw = (grid + DW_WARPS - 1) / DW_WARPS;
         if (delta) e = pdl_launch(decode_step_warp_kernel<TIN, TOUT, true>, dim3(gw), dim3(DW_WARPS * 32), 0, stream, a);
         else e = pdl_launch(decode_step_warp_kernel<TIN, TOUT, false>, dim3(gw), dim3(DW_WARPS * 32), 0, stream, a);
