@@ -443,7 +443,8 @@ int pgb_batch_linear_parts(int N);
  *   or with resid [B][N]: y = resid + v, the new residual stream; yw = y next_w (next_w [N]: the weight of the norm behind); and
  *   squares_out [B][pgb_decode_linear_parts(N, K, B)].
  *   window > 0: the launch also leaves pos = (pos + 1) mod window and shift = 1, for the last layer of a token.
- * Whether a layer is taken depends on K alone (256 at least): pgb_decode_linear_takes(kind 0 plain or activation, 1 residual, 2 logits; N, K).
+ * Whether a layer is taken does not depend on the batch (K more than 192, and what of it fits a CTA): pgb_decode_linear_takes(kind 0 plain or
+ *   activation, 1 residual, 2 logits; N, K).
  * pgb_decode_embed_norm is such a token's first kernel: x = E[tok] + P[pos], xw = x next_w and squares [B] (one part).
  * Every kernel of the chain requests W, bias and next_w before it waits for the one ahead: they are complete before the token's first kernel is
  * launched. A wait that runs out: pgb_tc_error_flag reads 78 or 79. */

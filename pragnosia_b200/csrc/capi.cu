@@ -77,7 +77,7 @@ int decode_advance_launch(long long *, float *, int, cudaStream_t);
 int decode_embed_launch(const long long *, const long long *, const void *, const void *, void *, int, int, int, int, float *, const void *, void *, float *,
                         cudaStream_t);
 int decode_linear_parts(int N, int K, int B);
-bool decode_linear_takes(int kind, int K, int B);
+bool decode_linear_takes(int kind, int K);
 int decode_linear_launch(const void *, const void *, const void *, const float *, int, float, int, const void *, const void *, void *, void *, float *,
                          float *, long long *, float *, int, int, int, int, cudaStream_t);
 int decode_linear_error_flag(int *);
@@ -647,7 +647,7 @@ int pgb_decode_embed_norm(const long long *tok, const long long *pos, const void
 }
 
 int pgb_decode_linear_takes(int kind, int N, int K) {
-    return kind >= 0 && kind <= 2 && N >= 8 && N % 8 == 0 && K >= 8 && K % 8 == 0 && decode_linear_takes(kind, K, 64) ? 1 : 0;
+    return kind >= 0 && kind <= 2 && N >= 8 && N % 8 == 0 && K >= 8 && K % 8 == 0 && decode_linear_takes(kind, K) ? 1 : 0;
 }
 int pgb_decode_linear_parts(int N, int K, int B) { return N < 8 || K < 8 || B < 1 ? 0 : decode_linear_parts(N, K, B); }
 
@@ -660,7 +660,7 @@ int pgb_decode_linear(const void *x, const void *W, const void *bias, const floa
     if (window < 0 || (window > 0 && (!pos || !shift))) return window < 0 ? PGB_ERR_BAD_SHAPE : PGB_ERR_NULL_POINTER;
     if (B < 1 || N < 8 || K < 8 || (N % 8) != 0 || (K % 8) != 0 || act < 0 || act > 1 || (act && (resid || logits)) || (squares_in && parts_in < 1))
         return PGB_ERR_BAD_SHAPE;
-    if (B > 64 || !decode_linear_takes(resid ? 1 : (logits ? 2 : 0), K, B)) return PGB_ERR_TOO_LARGE;
+    if (B > 64 || !decode_linear_takes(resid ? 1 : (logits ? 2 : 0), K)) return PGB_ERR_TOO_LARGE;
     if (!aligned(x, 16) || !aligned(W, 16) || !aligned(bias, 8) || !aligned(squares_in, 4) || !aligned(resid, 8) || !aligned(next_w, 8) || !aligned(y, 8) ||
         !aligned(yw, 8) || !aligned(squares_out, 4) || !aligned(logits, 16) || !aligned(pos, 8) || !aligned(shift, 4))
         return PGB_ERR_MISALIGNED;

@@ -261,23 +261,27 @@ struct DlForm { int bn, s; };
 // but 276 against 275 at batch 16); output projection 32,4 312 (16,4 344, 32,2 318, 16,1 326); MLP up 48,2 331 (32,2 344, 32,4 347, 64,2 349); MLP
 // down 32,8 344 (32,4 350, 16,8 379, 48,8 2 % slower; but at batch 5 223 against 239, at 16 240 against 245, at 32 271 against 276); head the same in
 // every form.
-// Every CTA keeps at least two blocks of K; shorter K is not taken.
+// Every CTA keeps at least two blocks of K; shorter K is not taken. The wider tiles of few rows hold K up to 6656, the others up to 7680 in MLP down:
+// where the wider do not fit the others are taken, so that whether a layer is taken does not depend on the batch.
 static DlForm decode_linear_form(int kind, int K, int B) {
     const int kb = (K + 63) / 64;
+    auto fits = [kb](DlForm f) {
+        const int n = (kb + f.s - 1) / f.s;
+        return n <= DL_KB && n * (DL_ROWS + f.bn) * 128 + DL_ROWS * (f.bn + 4) * 4 + 1024 <= DL_SMEM_MOST;
+    };
     DlForm f;
     if (kb < 4) return DlForm{0, 0};
-    if (kind == 1) f = kb >= 32 ? (B <= 32 ? DlForm{48, 8} : DlForm{32, 8}) : (kb >= 8 ? DlForm{32, 4} : DlForm{16, 2});
+    if (kind == 1) f = kb >= 32 ? (B <= 32 && fits(DlForm{48, 8}) ? DlForm{48, 8} : DlForm{32, 8}) : (kb >= 8 ? DlForm{32, 4} : DlForm{16, 2});
     else f = kind == 2 ? DlForm{64, 2} : DlForm{48, 2};
-    while (f.s < 8 && ((kb + f.s - 1) / f.s > DL_KB || (kb + f.s - 1) / f.s * (DL_ROWS + f.bn) * 128 + DL_ROWS * (f.bn + 4) * 4 + 1024 > DL_SMEM_MOST)) f.s *= 2;
-    if ((kb + f.s - 1) / f.s > DL_KB || (kb + f.s - 1) / f.s * (DL_ROWS + f.bn) * 128 + DL_ROWS * (f.bn + 4) * 4 + 1024 > DL_SMEM_MOST) return DlForm{0, 0};
-    return f;
+    while (f.s < 8 && !fits(f)) f.s *= 2;
+    return fits(f) ? f : DlForm{0, 0};
 }
 // tiles (= sums of squares a row) of a residual layer; 0: not taken
 int decode_linear_parts(int N, int K, int B) {
     const DlForm f = decode_linear_form(1, K, B);
     return f.bn == 0 ? 0 : (N + f.bn - 1) / f.bn;
 }
-bool decode_linear_takes(int kind, int K, int B) { return decode_linear_form(kind, K, B).bn != 0; }
+bool decode_linear_takes(int kind, int K) { return decode_linear_form(kind, K, DL_ROWS).bn != 0; }   // at every batch
 
 int decode_linear_launch(const void *x, const void *W, const void *bias, const float *sums, int parts, float eps, int act, const void *resid,
                          const void *next_w, void *y, void *yw, float *sums_out, float *logits, long long *pos, float *shift, int window, int B, int N,

@@ -204,3 +204,21 @@ def test_bench_table_names_are_kernel_bench_cases():
     asked = [n for n in names if n in kb.CASES or n.startswith(("prefill", "decode", "lambda", "layer_"))]
     assert len(asked) >= 15 and all(n in kb.CASES for n in asked), [n for n in asked if n not in kb.CASES]
     assert all(n in kb.CASES for n in kb.FLOPS)
+
+
+def test_linear_layers_of_a_batchs_step_are_taken_at_every_batch_or_at_none(L):
+    """pgb_decode_linear_takes knows no batch: what it accepts, pgb_decode_linear and pgb_decode_linear_parts accept at every batch up to 64, and what it
+    refuses they refuse. x misaligned: a call whose sizes are accepted ends at that check (4), so none is launched; 7 is a refused size."""
+    one, odd = ctypes.c_void_p(0x1000), ctypes.c_void_p(0x1004)
+    taken = 0
+    for K in (*range(8, 1024, 8), *range(1024, 17408, 64)):
+        for kind in range(3):
+            takes = L.pgb_decode_linear_takes(kind, 768, K)
+            taken += takes
+            for B in range(1, 65):
+                r, lg = (one if kind == 1 else None), (one if kind == 2 else None)
+                rc = L.pgb_decode_linear(odd, one, None, None, 0, 0.0, 0, r, r, None if lg else one, r, r, lg, None, None, 0, B, 768, K, None)
+                assert rc == (4 if takes else 7), (kind, K, B)
+                if kind == 1:
+                    assert (L.pgb_decode_linear_parts(768, K, B) > 0) == bool(takes), (K, B)
+    assert taken > 0 and L.pgb_decode_linear_takes(1, 1792, 7168) == 1

@@ -8,7 +8,7 @@ import copy
 import pytest
 import torch
 
-from pragnosia_b200 import synth
+from pragnosia_b200 import ops, synth
 from pragnosia_b200.generate import Decoder
 from pragnosia_b200.model import LM
 
@@ -78,4 +78,21 @@ def test_generate_through_the_chained_step():
         a = Decoder(m, batch=9).generate(prompt, 24, temp=temp, seed=5)
         c = Decoder(m, batch=9, use_graph=False).generate(prompt, 24, temp=temp, seed=5)
         assert torch.equal(a, c)                                      # graph replay and eager launches draw the same ids
+    assert healthy() == 0
+
+
+@pytest.mark.parametrize("K", [6656, 6720, 7168, 7680])               # the longest rows of the wider tiles, the shortest and longest past them
+@pytest.mark.parametrize("B", [5, 32, 33, 64])
+def test_long_rows_of_a_residual_layer(K, B):
+    """Against 64 bits: v is rounded to bf16 and so is resid + v (2^-9 of each); the products' sums are fp32 (K 2^-24 of the sum of magnitudes at most)."""
+    g = torch.Generator(device=DEV).manual_seed(K + B)
+    N = 136                                                           # ragged tiles of 32 and of 48 columns
+    x, W, r, w = (torch.randn(*s, device=DEV, generator=g).bfloat16() for s in ((B, K), (N, K), (B, N), (N,)))
+    y, yw, sq = ops.decode_linear(x, W, resid=r, next_w=w)
+    v = x.double() @ W.double().T
+    slack = 2.0 ** -24 * K * (x.double().abs() @ W.double().abs().T)
+    want = v + r.double()
+    assert bool(((y.double() - want).abs() <= 2.0 ** -9 * 1.01 * (v.abs() + want.abs() + 2.0 ** -8 * v.abs()) + 2 * slack).all())
+    assert torch.equal(yw, (y.float() * w.float()).bfloat16())
+    torch.testing.assert_close(sq.double().sum(1), y.double().square().sum(1), rtol=2.0 ** -24 * 64, atol=0)     # sums of 136 squares in fp32
     assert healthy() == 0
