@@ -506,10 +506,12 @@ def decode_linear_takes(kind: int, N: int, K: int) -> bool:
 @on_device_of
 def decode_embed_norm(tok, pos, E, P, next_w):
     """The first kernel of a token whose linear layers are decode_linear's: x (B,d) = E[tok] + P[pos], x next_w, and the rows' sums of squares (B,1)."""
-    need_cuda(tok, pos, E, P, next_w)
     if any(t.dtype != torch.bfloat16 for t in (E, P, next_w)) or tok.dtype != torch.long or pos.dtype != torch.long:
         raise ValueError("decode_embed_norm: bf16 tables and weight, int64 ids")
-    B, d = tok.numel(), E.shape[1]
+    B, d = tok.numel(), E.shape[-1]
+    if E.dim() != 2 or P.dim() != 2 or P.shape[1] != d or tuple(next_w.shape) != (d,) or pos.numel() < 1 or not all(t.is_contiguous() for t in (E, P, next_w)):
+        raise ValueError("decode_embed_norm: contiguous tables (rows, d), weight (d,), a position")
+    need_cuda(tok, pos, E, P, next_w)
     x, xw = (torch.empty(B, d, device=E.device, dtype=E.dtype) for _ in range(2))
     sq = torch.empty(B, 1, device=E.device, dtype=torch.float32)
     check(lib().pgb_decode_embed_norm(ptr(tok.contiguous()), ptr(pos), ptr(E), ptr(P), ptr(next_w), ptr(x), ptr(xw), ptr(sq), B, d, E.shape[0], P.shape[0],
@@ -525,16 +527,19 @@ def decode_linear(x, W, bias=None, squares=None, eps: float = 0.0, act: Optional
     is applied to the product. act None or "gelu". resid (B,N), next_w (N,): returns (resid + y, that times next_w, the parts of its rows' sums of
     squares) for the next norm. logits (B,N) fp32: written instead of a bf16 result. window > 0: also pos = (pos + 1) mod window, shift = 1.
     W, bias and next_w are read before the wait on the kernel ahead: they are complete before the chain's first kernel (decode_embed_norm)."""
-    need_cuda(x, W)
-    if any(t is not None and t.dtype != torch.bfloat16 for t in (x, W, bias, resid, next_w)) or x.dim() != 2 or not x.is_contiguous():
-        raise ValueError("decode_linear: bf16, x (B,K) contiguous")
+    if any(t is not None and t.dtype != torch.bfloat16 for t in (x, W, bias, resid, next_w)) or x.dim() != 2 or W.dim() != 2 or not x.is_contiguous():
+        raise ValueError("decode_linear: bf16, x (B,K) contiguous, W (N,K)")
     if not all(t is None or t.is_contiguous() for t in (W, bias, squares, resid, next_w, logits)):
         raise ValueError("decode_linear: contiguous tensors")
     if any(t is not None and t.dtype != torch.float32 for t in (squares, logits, shift)) or (pos is not None and pos.dtype != torch.long):
         raise ValueError("decode_linear: fp32 sums, logits and shift, int64 position")
     (B, K), N = x.shape, W.shape[0]
-    if W.shape[1] != K or (squares is not None and squares.shape[0] != B) or any(t is not None and tuple(t.shape) != (B, N) for t in (resid, logits)):
+    if (W.shape[1] != K or any(t is not None and tuple(t.shape) != (N,) for t in (bias, next_w)) or (resid is None) != (next_w is None) or
+            (squares is not None and (squares.dim() != 2 or squares.shape[0] != B or squares.shape[1] < 1)) or
+            any(t is not None and tuple(t.shape) != (B, N) for t in (resid, logits)) or
+            (window > 0 and any(t is None or t.numel() < 1 for t in (pos, shift)))):
         raise ValueError("decode_linear: shapes")
+    need_cuda(x, W, bias, squares, resid, next_w, logits, pos, shift)
     y = yw = sq = None
     if logits is None:
         y = torch.empty(B, N, device=x.device, dtype=x.dtype)

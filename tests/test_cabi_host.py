@@ -222,3 +222,28 @@ def test_linear_layers_of_a_batchs_step_are_taken_at_every_batch_or_at_none(L):
                 if kind == 1:
                     assert (L.pgb_decode_linear_parts(768, K, B) > 0) == bool(takes), (K, B)
     assert taken > 0 and L.pgb_decode_linear_takes(1, 1792, 7168) == 1
+
+
+def test_wrappers_of_the_chained_step_see_lengths():
+    """The kernels read bias, norm weights and tables to the sizes of x and W, and the C entry points see addresses only: a tensor that is too short, of
+    another width or not laid out row by row is refused by the wrapper, ahead of the check for the device that right ones end at here."""
+    from pragnosia_b200 import ops
+    bf = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)
+    B, N, K = 5, 24, 256
+    lin = lambda **kw: ops.decode_linear(kw.pop("x", bf(B, K)), kw.pop("W", bf(N, K)), kw.pop("bias", bf(N)), **kw)
+    long, f32 = (lambda n: torch.zeros(n, dtype=torch.long)), torch.zeros
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        lin(squares=f32(B, 3), resid=bf(B, N), next_w=bf(N))
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        lin(logits=f32(B, N), pos=long(1), shift=f32(()), window=8)
+    for bad in (dict(bias=bf(N - 2)), dict(bias=bf(1, N)), dict(resid=bf(B, N), next_w=bf(N - 8)), dict(resid=bf(B, N - 8), next_w=bf(N)), dict(resid=bf(B, N)),
+                dict(W=bf(N * K)), dict(squares=f32(B)), dict(squares=f32(B, 0)), dict(squares=f32(B - 1, 3)), dict(logits=f32(B, N), window=8),
+                dict(logits=f32(B, N), pos=long(0), shift=f32(()), window=8), dict(logits=f32(B, N), pos=long(1), shift=f32(0), window=8)):
+        with pytest.raises(ValueError):
+            lin(**bad)
+    emb = lambda **kw: ops.decode_embed_norm(long(B), kw.pop("pos", long(1)), kw.pop("E", bf(64, K)), kw.pop("P", bf(16, K)), kw.pop("w", bf(K)))
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        emb()
+    for bad in (dict(pos=long(0)), dict(E=bf(K, 64).T), dict(P=bf(16, K - 8)), dict(P=bf(K, 16).T), dict(w=bf(K - 8)), dict(w=bf(2 * K)[::2])):
+        with pytest.raises(ValueError):
+            emb(**bad)
