@@ -244,15 +244,16 @@ class Decoder:
 
     def _chain_ok(self):
         """A batch past the few-row kernels, up to one 64-row tensor-core tile: every linear layer as one link of a chain of dependent launches
-        (ops.decode_linear) that carries the RMS norm ahead of it and the residual add behind it. bf16 weights, layers that are plain
-        nn.Linear and whose K the kernel takes; else the separate kernels."""
+        (ops.decode_linear) that carries the RMS norm ahead of it and the residual add behind it. bf16 weights whose K the kernel takes, layers of
+        exactly these types (a carrier's subclass may have a mix of its own; a parametrized weight would be formed between two links, the second of which
+        reads it ahead of its wait); else the separate kernels."""
         m = self.m
         if not (self.fused and not self.folded and 4 < self.B <= 64 and m.e.weight.is_cuda and m.e.weight.dtype == m.p.weight.dtype == torch.bfloat16 and
-                all(isinstance(mx, AssocCarrier) and mx.plain_step for mx in m.mix) and
+                type(m.e) is type(m.p) is torch.nn.Embedding and all(type(mx) is AssocCarrier and mx.plain_step for mx in m.mix) and
                 all(mp.fused_up and type(mp.a) is type(mp.b) is torch.nn.Linear for mp in m.mlp)):
             return False
         norms = [m.n, *(mx.ln for mx in m.mix), *(mp.n for mp in m.mlp)]
-        if not all(isinstance(n, torch.nn.RMSNorm) and n.weight is not None for n in norms):
+        if not all(type(n) is torch.nn.RMSNorm and n.weight is not None for n in norms):
             return False
         held = [m.e.weight, m.p.weight, *(n.weight for n in norms), *(t for mp in m.mlp for t in (mp.a.weight, mp.a.bias, mp.b.weight, mp.b.bias) if t is not None)]
         takes, d, V = ops.decode_linear_takes, m.d, m.e.weight.shape[0]

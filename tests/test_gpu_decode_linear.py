@@ -7,8 +7,10 @@ import copy
 
 import pytest
 import torch
+import torch.nn.utils.parametrize
 
-from pragnosia_b200 import ops, synth
+from pragnosia_b200 import _lib, ops, synth
+from pragnosia_b200.assoc import AssocCarrier
 from pragnosia_b200.generate import Decoder
 from pragnosia_b200.model import LM
 
@@ -96,3 +98,45 @@ def test_long_rows_of_a_residual_layer(K, B):
     assert torch.equal(yw, (y.float() * w.float()).bfloat16())
     torch.testing.assert_close(sq.double().sum(1), y.double().square().sum(1), rtol=2.0 ** -24 * 64, atol=0)     # sums of 136 squares in fp32
     assert healthy() == 0
+
+
+class HalfCarrier(AssocCarrier):
+    def mix(self, z, h0=None, inplace=None):
+        delta, st = super().mix(z, h0, inplace)
+        return 0.5 * delta, st
+
+
+class OwnNorm(torch.nn.RMSNorm):
+    pass
+
+
+def test_layers_of_other_types_keep_their_own_step():
+    """The chain calls kernels, not the layers: a carrier with a mix of its own, and norms and tables whose type may form their weight as it is
+    asked for (the chain's kernels read weights ahead of their waits), stay with the separate kernels."""
+    ids = synth.token_ids(8, 30, 256, seed=1).to(DEV)
+    for change in ("mix", "norm", "table"):
+        m = model(256, "aspin", 2, 256)
+        if change == "mix":
+            m.mix[1].__class__ = HalfCarrier
+        elif change == "norm":
+            m.mlp[0].n.__class__ = OwnNorm
+        else:
+            torch.nn.utils.parametrize.register_parametrization(m.e, "weight", torch.nn.Identity())
+        outs = []
+        for fused in (True, False):
+            dec = Decoder(m, batch=8, fused=fused, use_graph=False)
+            dec.prefill(ids[:, :20])
+            outs.append([dec.step(ids[:, t]).clone() for t in range(20, 24)])
+            assert not dec._chain_ok()
+        assert all(torch.equal(a, b) for a, b in zip(*outs)), change
+
+
+@pytest.mark.parametrize("d,mixer,B", [(704, "dspin", 17), (768, "aspin", 44)])          # an odd number of pairs: the last CTA has one
+def test_chained_step_with_a_warp_per_pair(d, mixer, B):
+    """The chain takes a CTA per pair of its own accord; where the other kernel is asked for, it reads its state ahead of the wait, too."""
+    L = _lib.lib()
+    _lib.check(L.pgb_decode_set_variant(2), "pgb_decode_set_variant")
+    try:
+        test_chained_step_of_a_batch(d, mixer, 3, 1000, B)
+    finally:
+        _lib.check(L.pgb_decode_set_variant(0), "pgb_decode_set_variant")
