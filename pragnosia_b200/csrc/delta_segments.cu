@@ -101,16 +101,7 @@ struct DjParams {
     int T, H, BH, seg_chunks, o_is_f32, token_major;
 };
 
-__device__ __forceinline__ void dj_split(float x, uint32_t &hi, uint32_t &lo) {
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(x - __uint_as_float(hi)));
-}
-__device__ __forceinline__ void dj_mma(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-// A CTA per chunk of 64 tokens; warp w has tokens 16 (w % 4) .. and columns 32 (w / 4) .. Factors as two tf32 parts, tail by tail left out: 2^-23 of a product.
+// A CTA per chunk of 64 tokens; warp w has tokens 16 (w % 4) .. and columns 32 (w / 4) .. Factors as two tf32 parts, tail by tail left out: 2^-21 of a product at most (the walk's own products keep 2^-16).
 // 756 chunks: 13 us, as fp32 register tiles 17.
 __global__ void __launch_bounds__(256) delta_join_kernel(const __grid_constant__ DjParams p) {
     __shared__ __align__(16) float as[64 * DS_P], es[64 * DS_PE], red[2][64];
@@ -151,15 +142,15 @@ __global__ void __launch_bounds__(256) delta_join_kernel(const __grid_constant__
         for (int k = 0; k < 64; k += 8) {
             uint32_t ah[4], al[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) dj_split(as[row[i & 1] * DS_P + k + t4 + 4 * (i >> 1)], ah[i], al[i]);
+            for (int i = 0; i < 4; ++i) tf32_split(as[row[i & 1] * DS_P + k + t4 + 4 * (i >> 1)], ah[i], al[i]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 uint32_t eh[2], el[2];
 #pragma unroll
-                for (int i = 0; i < 2; ++i) dj_split(es[(k + t4 + 4 * i) * DS_PE + n0 + 8 * j + g], eh[i], el[i]);
-                dj_mma(acc[j], al, eh);
-                dj_mma(acc[j], ah, el);
-                dj_mma(acc[j], ah, eh);
+                for (int i = 0; i < 2; ++i) tf32_split(es[(k + t4 + 4 * i) * DS_PE + n0 + 8 * j + g], eh[i], el[i]);
+                mma_tf32(acc[j], al, eh);
+                mma_tf32(acc[j], ah, el);
+                mma_tf32(acc[j], ah, eh);
             }
         }
     }

@@ -54,15 +54,7 @@ static_assert(InvSmem::off_misc >= TC_C * 128 * 2, "the K tile lies in the array
 
 // P = A B for 16 rows and NT tiles of eight columns over the K blocks k0 <= k < k1 of eight, by a warp. A element (m, k) lies at A[m ra + k ka], an
 // element (k, n) of B at B[n P + k]. Lane l of the accumulator has rows l / 4 and l / 4 + 8, columns 2 (l % 4) and the next of each tile. A factor is split into two parts of eleven bits, of whose products
-// all but tail by tail are added: 2^-23 of a product, fp32's own rounding.
-__device__ __forceinline__ void tf32_split(float x, uint32_t &hi, uint32_t &lo) {
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(x - __uint_as_float(hi)));
-}
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
+// all but tail by tail are added: 2^-21 of a product at most.
 template <int NT>
 __device__ __forceinline__ void inv_product(float (&acc)[NT][4], const float *A, int ra, int ka, const float *B, int k0, int k1, int lane) {
     const float *ap = A + (lane >> 2) * ra + (lane & 3) * ka, *bp = B + (lane >> 2) * InvSmem::P + (lane & 3);
