@@ -4,7 +4,7 @@ import pytest
 import torch
 import torch.nn.functional as F
 
-from pragnosia_b200 import ops, synth
+from pragnosia_b200 import _lib, ops, synth
 from pragnosia_b200.assoc import AssocCarrier
 from pragnosia_b200.model import LM
 
@@ -54,6 +54,19 @@ def test_all_windows_at_once_match_window_by_window(delta, head_dim, window, T, 
 def test_windows_of_the_last_round_in_parts(window, T):
     """Twelve chains of more windows than SMs: whole windows, then those of the last round cut into parts (a ragged one last)."""
     test_all_windows_at_once_match_window_by_window(False, 64, window, T, 3)
+
+
+@pytest.mark.parametrize("window,T", [
+    (512, 16 * 512), (512, 16 * 512 - 150), (512, 15 * 512 + 1),      # twelve whole windows a chain, then eight chunks as 3 + 3 + 2; the last one ragged
+    (320, 5 * 320 - 30), (320, 17 * 320 + 200), (320, 17 * 320 + 30), # five chunks as 3 + 2, with whole windows ahead of them and without
+    (448, 6 * 448), (1024, 3 * 1024 - 70),                            # seven as 4 + 3; sixteen as 4 x 4 with the end inside one
+])
+def test_windows_in_parts_that_do_not_divide_them(window, T):
+    """A part that is shorter than its neighbours ends its window: the first tokens, positions and rotations behind it follow from that."""
+    L, B, H = _lib.lib(), 3, 4
+    uncut = ((T + window - 1) // window - 1) * B * H * (64 * 64 + 1) * 4
+    assert L.pgb_aspin_layer_windows_scratch_bytes(B, H, T, window) > uncut              # more segments than windows: some are cut
+    test_all_windows_at_once_match_window_by_window(False, 64, window, T, B)
 
 
 @pytest.mark.parametrize("mixer", ["aspin", "dspin"])
