@@ -14,7 +14,7 @@
 // Everything fp32 that re-enters the tensor core (S, rhs, X, A, W) is split into bf16 head + tail and multiplied as
 // head*head + head*tail + tail*head. Every mbarrier wait is bounded.
 //
-// Measured, B8 H16 T8192 D128 (1.1 GB of operands): walk 396 us, inverse 138.
+// Measured, B8 H16 T8192 D128 (1.1 GB of operands): walk 396 us, inverse 166.
 #include "delta_walk.cuh"
 
 namespace pgb {
@@ -39,12 +39,13 @@ __device__ __forceinline__ void chunk_stats(const float *la, const float *beta, 
 // ------------------------------------------------------------------------------------------------ X = (I + N)^-1
 // One column of X per thread is a chain of 2016 dependent multiply-adds on half the threads. The blocked form keeps the chain to 16 steps: the four
 // 16 x 16 diagonal blocks are inverted side by side (half a warp each, a lane per column), then twice X21 = -X22 (N21 X11) joins neighbouring blocks, 16
-// and 32 wide, as warp-level products (m16n8k8, too small for the tensor-memory kind) of factors split into two tf32 parts.
+// and 32 wide, as warp-level products (m16n8k8, too small for the tensor-memory kind) of factors split into three tf32 parts, which are all of fp32.
 // One array holds all of it, in the K tile's place once that is consumed: N below the diagonal; X transposed above it, a diagonal block of X over N's own
 // once its columns are done; T = N21 X11, transposed, in the quarter that X21 would take (X21 itself goes from registers to memory). 20 KB a CTA where
-// N, X and T side by side were 43: nine CTAs an SM instead of five.
-// B8 H16 T8192 D128: 193.7 us with the joins as fp32 register tiles, whose 16-byte shared loads filled the load unit, 137.6 so; B4 H11 T2048 D64 20.6 and
-// 16.8. Errors of o and S against 64 bits are the same to three digits (5.1e-6 and 3.5e-6). What bounds it now: issue slots (55 %) and the CTA's own chain.
+// N, X and T side by side were 43: eight CTAs an SM (the tensor memory's limit, too) instead of five.
+// B8 H16 T8192 D128: 194 us with the joins as fp32 register tiles, whose 16-byte shared loads filled the load unit, 166 so; B64 H12 T512 D64 77 and 67. Two
+// parts a factor took 137 and 55, but X21's error against 64 bits rose by 10 to 15 % where keys resemble one another (2.9e-6 -> 3.2e-6 of it, 3.7e-6 -> 4.3e-6
+// for keys that all but repeat); with three it is the register tiles', 0.3 % below to 0.7 % above, X's as a whole 0.02 % below to 0.07 % above. What bounds it: issue slots.
 struct InvSmem {
     static constexpr int P = 68;                                      // row pitch, in floats (16-byte aligned, four banks on)
     static constexpr int off_misc = TC_C * P * 4;                     // not below a K tile of 64 x 128 bf16
@@ -53,32 +54,44 @@ struct InvSmem {
 static_assert(InvSmem::off_misc >= TC_C * 128 * 2, "the K tile lies in the array's place");
 
 // P = A B for 16 rows and NT tiles of eight columns over the K blocks k0 <= k < k1 of eight, by a warp. A element (m, k) lies at A[m ra + k ka], an
-// element (k, n) of B at B[n P + k]. Lane l of the accumulator has rows l / 4 and l / 4 + 8, columns 2 (l % 4) and the next of each tile. A factor is split into two parts of eleven bits, of whose products
-// all but tail by tail are added: 2^-21 of a product at most.
+// element (k, n) of B at B[n P + k]. Lane l of the accumulator has rows l / 4 and l / 4 + 8, columns 2 (l % 4) and the next of each tile. Of the products of
+// the factors' three parts all are added but those below 2^-33 of the whole. The heads' products of a block are added by an addition that rounds:
+// accumulated in the tensor core, which cuts off, X was off by 0.1 % more where nothing decays (162 us).
 template <int NT>
 __device__ __forceinline__ void inv_product(float (&acc)[NT][4], const float *A, int ra, int ka, const float *B, int k0, int k1, int lane) {
     const float *ap = A + (lane >> 2) * ra + (lane & 3) * ka, *bp = B + (lane >> 2) * InvSmem::P + (lane & 3);
+    float low[NT][4];
 #pragma unroll
     for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
+        for (int i = 0; i < 4; ++i) acc[n][i] = low[n][i] = 0.f;
 #pragma unroll 2
     for (int k = k0; k < k1; ++k) {
-        uint32_t ah[4], al[4];
-        tf32_split(ap[8 * k * ka], ah[0], al[0]);
-        tf32_split(ap[8 * ra + 8 * k * ka], ah[1], al[1]);
-        tf32_split(ap[(8 * k + 4) * ka], ah[2], al[2]);
-        tf32_split(ap[8 * ra + (8 * k + 4) * ka], ah[3], al[3]);
+        uint32_t ah[4], am[4], al[4];
+        tf32_split(ap[8 * k * ka], ah[0], am[0], al[0]);
+        tf32_split(ap[8 * ra + 8 * k * ka], ah[1], am[1], al[1]);
+        tf32_split(ap[(8 * k + 4) * ka], ah[2], am[2], al[2]);
+        tf32_split(ap[8 * ra + (8 * k + 4) * ka], ah[3], am[3], al[3]);
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
-            uint32_t bh[2], bl[2];
-            tf32_split(bp[8 * n * InvSmem::P + 8 * k], bh[0], bl[0]);
-            tf32_split(bp[8 * n * InvSmem::P + 8 * k + 4], bh[1], bl[1]);
-            mma_tf32(acc[n], al, bh);
-            mma_tf32(acc[n], ah, bl);
-            mma_tf32(acc[n], ah, bh);
+            uint32_t bh[2], bm[2], bl[2];
+            tf32_split(bp[8 * n * InvSmem::P + 8 * k], bh[0], bm[0], bl[0]);
+            tf32_split(bp[8 * n * InvSmem::P + 8 * k + 4], bh[1], bm[1], bl[1]);
+            mma_tf32(low[n], al, bh);
+            mma_tf32(low[n], ah, bl);
+            mma_tf32(low[n], am, bm);
+            mma_tf32(low[n], am, bh);
+            mma_tf32(low[n], ah, bm);
+            float hh[4] = {0.f, 0.f, 0.f, 0.f};
+            mma_tf32(hh, ah, bh);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[n][i] += hh[i];
         }
     }
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[n][i] += low[n][i];
 }
 // such an accumulator (or its negative) transposed: element (m, n) to at[n P + m]
 template <int NT, bool NEG>
@@ -91,7 +104,7 @@ __device__ __forceinline__ void inv_put(float *at, const float (&acc)[NT][4], in
 }
 
 template <int D>
-__global__ void __launch_bounds__(128, 9) delta_inv_kernel(const __grid_constant__ CUtensorMap mk, const float *__restrict__ la_all,
+__global__ void __launch_bounds__(128, 8) delta_inv_kernel(const __grid_constant__ CUtensorMap mk, const float *__restrict__ la_all,
                                                         const float *__restrict__ beta_all, __nv_bfloat16 *__restrict__ X, int T,
                                                         int with_tail) {
     using SM = InvSmem;

@@ -34,3 +34,32 @@ def test_segments_side_by_side_match_whole_chains(B, H, T, S0, shift):
     assert rel(o, whole[0]) <= 1.1e-5 and rel(S, whole[1]) <= 7.5e-6, (rel(o, whole[0]), rel(S, whole[1]))
     ob, Sb, _ = ops.prefill(q, k, v, la, beta, S_in, theta=th, shift=shift)
     assert torch.equal(ob, o.bfloat16()) and torch.equal(Sb, S)                          # the bf16 read is the fp32 one, rounded
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("half", [16, 32])                            # the join of 16-wide blocks, and that of 32-wide ones
+def test_joins_of_the_chunk_inverse_keep_fp32(D, half):
+    """Tokens s < t < u of one unit key, no decay: N[t][s] = b_t, N[u][s] = N[u][t] = b_u, all 24 bits of them, and X[u][s] = -b_u + b_u b_t, which for b_t just
+    below 1 cancels down to the factors' last bits. In fp32 the one rounding of b_u b_t is 2^-25 of b_u, and the pair of bf16 it is stored as misses 2^-17 of a
+    result below 2^-8: 2^-24 in all. Factors as two tf32 parts: up to 2^-22.5 (emulated)."""
+    n, L = half // 2, _lib.lib()                                      # triples a chunk: s = i in the upper block, t and u neighbours in the lower
+    B, H, NC = 1, 4, 64
+    T = 64 * NC
+    own = torch.arange(64)
+    for i in range(n):
+        own[half + 2 * i] = own[half + 2 * i + 1] = i
+    k = F.one_hot(own, D).bfloat16().to(DEV).repeat(B * H * NC, 1, 1).view(B, H, T, D)
+    g = torch.Generator(device=DEV).manual_seed(half)
+    beta = 0.5 + 0.5 * torch.rand(B, H, NC, 64, device=DEV, generator=g)
+    s, t = torch.arange(n, device=DEV), half + 2 * torch.arange(n, device=DEV)
+    beta[..., t] = 1 - (1 + torch.rand(B, H, NC, n, device=DEV, generator=g)) * 2.0 ** -9
+    q, v, la = torch.zeros_like(k), torch.zeros_like(k), torch.zeros(B, H, T, device=DEV)
+    p = lambda a: ctypes.c_void_p(a.data_ptr())
+    x = torch.empty(L.pgb_aspin_delta_scratch_bytes(B, H, T), device=DEV, dtype=torch.uint8)
+    o, S = torch.empty(B, H, T, D, device=DEV), torch.empty(B, H, D, D, device=DEV)
+    assert L.pgb_aspin_delta_prefill_fwd(p(q), p(k), p(v), p(la), p(beta), None, None, None, 0.0, p(o), 0, p(S), None, p(x), x.numel(), B, H, T, D,
+                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    X = x[:B * H * NC * 2 * 8192].view(torch.bfloat16).view(B, H, NC, 2, 64, 64).double().sum(3)        # head + tail
+    bt, bu = beta[..., t].double(), beta[..., t + 1].double()
+    off = (X[..., t + 1, s] - (bu * bt - bu)).abs() / bu
+    assert float(off.max()) <= 2.0 ** -24, float(off.max().log2())
