@@ -452,6 +452,8 @@ int pgb_decode_embed_norm(const long long *tok, const long long *pos, const void
                           float *squares, int B, int d, int vocab, int ctx, void *stream);
 int pgb_decode_linear_takes(int kind, int N, int K);
 int pgb_decode_linear_parts(int N, int K, int B);
+/* in how many rounds such a layer's thread blocks go over the chip (0: not taken): what a wide layer's time follows */
+int pgb_decode_linear_rounds(int kind, int N, int K, int B);
 int pgb_decode_linear(const void *x, const void *W, const void *bias, const float *squares_in, int parts_in, float eps, int act, const void *resid,
                       const void *next_w, void *y, void *yw, float *squares_out, float *logits, long long *pos, float *shift, int window, int B,
                       int N, int K, void *stream);

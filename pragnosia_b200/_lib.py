@@ -68,6 +68,7 @@ SIGNATURES = {
     "pgb_decode_embed_norm": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "pgb_decode_linear_takes": [_i, _i, _i],
     "pgb_decode_linear_parts": [_i, _i, _i],
+    "pgb_decode_linear_rounds": [_i, _i, _i, _i],
     "pgb_decode_linear": [_vp, _vp, _vp, _vp, _i, _f, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "pgb_decode_advance": [_vp, _vp, _i, _vp],
     "pgb_decode_token_work_bytes": [_i, _i, _i, _i],

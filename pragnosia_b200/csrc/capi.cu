@@ -77,6 +77,7 @@ int decode_advance_launch(long long *, float *, int, cudaStream_t);
 int decode_embed_launch(const long long *, const long long *, const void *, const void *, void *, int, int, int, int, float *, const void *, void *, float *,
                         cudaStream_t);
 int decode_linear_parts(int N, int K, int B);
+int decode_linear_rounds(int kind, int N, int K, int B);
 bool decode_linear_takes(int kind, int K);
 int decode_linear_launch(const void *, const void *, const void *, const float *, int, float, int, const void *, const void *, void *, void *, float *,
                          float *, long long *, float *, int, int, int, int, cudaStream_t);
@@ -648,6 +649,9 @@ int pgb_decode_embed_norm(const long long *tok, const long long *pos, const void
 
 int pgb_decode_linear_takes(int kind, int N, int K) {
     return kind >= 0 && kind <= 2 && N >= 8 && N % 8 == 0 && K >= 8 && K % 8 == 0 && decode_linear_takes(kind, K) ? 1 : 0;
+}
+int pgb_decode_linear_rounds(int kind, int N, int K, int B) {
+    return kind < 0 || kind > 2 || N < 8 || K < 8 || B < 1 ? 0 : decode_linear_rounds(kind, N, K, B);
 }
 int pgb_decode_linear_parts(int N, int K, int B) { return N < 8 || K < 8 || B < 1 ? 0 : decode_linear_parts(N, K, B); }
 

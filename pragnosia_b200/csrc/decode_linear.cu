@@ -27,7 +27,7 @@ namespace pgb {
 
 constexpr int DL_NT = 256, DL_ROWS = 64;
 constexpr int DL_KB = 16;                                             // K blocks (of 64) of a CTA at most
-constexpr int DL_SMEM_MOST = 200 * 1024;
+constexpr int DL_SMEM_MOST = 224 * 1024, DL_SMEM_FIRST = 200 * 1024;
 
 struct DlArgs {
     const __nv_bfloat16 *bias;
@@ -60,8 +60,8 @@ template <int BN, int S>
 __global__ void __launch_bounds__(DL_NT) decode_linear_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw,
                                                              const __grid_constant__ DlArgs a) {
     constexpr int RR = DL_ROWS / S, PROW = BN + 4, G4 = BN / 4;       // rows a CTA finishes; padded row of the sums; groups of four columns
-    constexpr int GL = G4 <= 4 ? 4 : (G4 <= 8 ? 8 : 16);              // lanes of a row behind the sums: one a group, rounded up to a power of two
-    constexpr int TCOLS = BN <= 32 ? 32 : 64;
+    constexpr int GL = G4 <= 4 ? 4 : (G4 <= 8 ? 8 : (G4 <= 16 ? 16 : 32));              // lanes of a row behind the sums: one a group, rounded up to a power of two
+    constexpr int TCOLS = BN <= 32 ? 32 : (BN <= 64 ? 64 : 128);
     extern __shared__ uint8_t dl_smem[];
     __shared__ __align__(8) unsigned long long bars[DL_KB + 2];
     __shared__ uint32_t tmem_slot;
@@ -255,7 +255,16 @@ static int decode_linear_go(const void *x, const void *W, const DlArgs &a, cudaS
 }
 
 struct DlForm { int bn, s; };
-// Columns of a tile and CTAs of a cluster. kind 0: plain or activation, 1: residual, 2: logits. {0, 0}: K too short or too long.
+static int dl_bytes(DlForm f, int kb) { return (kb + f.s - 1) / f.s * (DL_ROWS + f.bn) * 128 + DL_ROWS * (f.bn + 4) * 4 + 1024; }
+static bool dl_fits(DlForm f, int kb, int most) { return (kb + f.s - 1) / f.s <= DL_KB && dl_bytes(f, kb) <= most; }
+// in how many rounds a link's clusters go over the chip: what cudaOccupancyMaxActiveClusters says of 148 SMs at 1, 2, 3, 4 CTAs of this memory an SM
+static int dl_rounds(DlForm f, int N, int kb) {
+    constexpr int ACTIVE[3][4] = {{74, 148, 222, 296}, {33, 71, 104, 142}, {15, 33, 48, 71}};
+    const int per_sm = 233472 / (dl_bytes(f, kb) + 1024 + 512);        // the system's own, and the static share
+    const int fit = ACTIVE[f.s == 2 ? 0 : (f.s == 4 ? 1 : 2)][per_sm < 1 ? 0 : (per_sm > 4 ? 3 : per_sm - 1)];
+    return ((N + f.bn - 1) / f.bn + fit - 1) / fit;
+}
+// Columns of a tile and CTAs of a cluster. kind 0: plain or activation, 1: residual, 2: logits. {0, 0}: K too short or too long, at whatever batch and N.
 // Two things pull: x is read once a tile (wide tiles, few clusters), and CTAs of neighbouring links must fit an SM together, at best one of each (about
 // 100 to 130 CTAs of 80 to 100 KB a link). Batch 64, d 768, dff 3072, us a token, all else equal: projection 48,2 335 (32,2 345, 64,4 341, 16,1 333
 // but 276 against 275 at batch 16); output projection 32,4 312 (16,4 344, 32,2 318, 16,1 326); MLP up 48,2 331 (32,2 344, 32,4 347, 64,2 349); MLP
@@ -263,36 +272,55 @@ struct DlForm { int bn, s; };
 // every form.
 // Every CTA keeps at least two blocks of K; shorter K is not taken. The wider tiles of few rows hold K up to 6656, the others up to 7680 in MLP down:
 // where the wider do not fit the others are taken, so that whether a layer is taken does not depend on the batch.
-static DlForm decode_linear_form(int kind, int K, int B) {
-    const int kb = (K + 63) / 64;
-    auto fits = [kb](DlForm f) {
-        const int n = (kb + f.s - 1) / f.s;
-        return n <= DL_KB && n * (DL_ROWS + f.bn) * 128 + DL_ROWS * (f.bn + 4) * 4 + 1024 <= DL_SMEM_MOST;
-    };
+static DlForm decode_linear_first_form(int kind, int kb, int B) {
     DlForm f;
     if (kb < 4) return DlForm{0, 0};
-    if (kind == 1) f = kb >= 32 ? (B <= 32 && fits(DlForm{48, 8}) ? DlForm{48, 8} : DlForm{32, 8}) : (kb >= 8 ? DlForm{32, 4} : DlForm{16, 2});
+    if (kind == 1) f = kb >= 32 ? (B <= 32 && dl_fits(DlForm{48, 8}, kb, DL_SMEM_FIRST) ? DlForm{48, 8} : DlForm{32, 8}) : (kb >= 8 ? DlForm{32, 4} : DlForm{16, 2});
     else f = kind == 2 ? DlForm{64, 2} : DlForm{48, 2};
-    while (f.s < 8 && !fits(f)) f.s *= 2;
-    return fits(f) ? f : DlForm{0, 0};
+    while (f.s < 8 && !dl_fits(f, kb, DL_SMEM_FIRST)) f.s *= 2;
+    return dl_fits(f, kb, DL_SMEM_FIRST) ? f : DlForm{0, 0};
+}
+// That is for links of one round. In wider models it takes two to four, and a link's time follows their number (d 2048, batch 16, projection: 633 us a token in two,
+// 676 in three, 725 in four): where another form needs fewer, the one with the fewest is taken, of those the smallest cluster, then the least shared memory. The head
+// stays: its many rounds go at the memory's rate. Twelve layers, us a token, the first forms / these / the separate kernels:
+//   d 1024, dff 4096: batch 16 373 / 296 / 435, batch 64 456 / 406 / 485      d 1536, dff 6144: 569 / 475 / 684, 806 / 627 / 758
+//   d 1792, dff 7168: 711 / 653 / 775, 904 / 843 / 874                        d 2048, dff 4096: 722 / 577 / 716, 962 / 759 / 834
+static DlForm decode_linear_form(int kind, int N, int K, int B) {
+    const int kb = (K + 63) / 64;
+    DlForm f = decode_linear_first_form(kind, kb, B);
+    if (f.bn == 0 || kind == 2) return f;
+    int rounds = dl_rounds(f, N, kb);
+    bool first = true;
+    for (DlForm c : {DlForm{32, 4}, DlForm{32, 8}, DlForm{48, 2}, DlForm{48, 4}, DlForm{48, 8}, DlForm{64, 2}, DlForm{64, 4}, DlForm{64, 8}, DlForm{96, 4}, DlForm{96, 8}}) {
+        if (kb < 2 * c.s || !dl_fits(c, kb, DL_SMEM_MOST)) continue;
+        const int r = dl_rounds(c, N, kb);
+        if (r > rounds || (r == rounds && (first || c.s > f.s || (c.s == f.s && dl_bytes(c, kb) >= dl_bytes(f, kb))))) continue;
+        f = c; rounds = r; first = false;
+    }
+    return f;
 }
 // tiles (= sums of squares a row) of a residual layer; 0: not taken
 int decode_linear_parts(int N, int K, int B) {
-    const DlForm f = decode_linear_form(1, K, B);
+    const DlForm f = decode_linear_form(1, N, K, B);
     return f.bn == 0 ? 0 : (N + f.bn - 1) / f.bn;
 }
-bool decode_linear_takes(int kind, int K) { return decode_linear_form(kind, K, DL_ROWS).bn != 0; }   // at every batch
+int decode_linear_rounds(int kind, int N, int K, int B) {
+    const DlForm f = decode_linear_form(kind, N, K, B);
+    return f.bn == 0 ? 0 : dl_rounds(f, N, (K + 63) / 64);
+}
+bool decode_linear_takes(int kind, int K) { return decode_linear_first_form(kind, (K + 63) / 64, DL_ROWS).bn != 0; }   // at every batch and N
 
 int decode_linear_launch(const void *x, const void *W, const void *bias, const float *sums, int parts, float eps, int act, const void *resid,
                          const void *next_w, void *y, void *yw, float *sums_out, float *logits, long long *pos, float *shift, int window, int B, int N,
                          int K, cudaStream_t stream) {
     const DlArgs a{(const __nv_bfloat16 *)bias, sums, parts, eps, (const __nv_bfloat16 *)resid, (const __nv_bfloat16 *)next_w, (__nv_bfloat16 *)y,
                    (__nv_bfloat16 *)yw, logits, sums_out, pos, shift, window, B, N, K, act, (B + 7) / 8 * 8};
-    const DlForm f = decode_linear_form(resid != nullptr ? 1 : (logits != nullptr ? 2 : 0), K, B);
+    const DlForm f = decode_linear_form(resid != nullptr ? 1 : (logits != nullptr ? 2 : 0), N, K, B);
 #define PGB_DL(BN_, S_) if (f.bn == BN_ && f.s == S_) return decode_linear_go<BN_, S_>(x, W, a, stream)
-    PGB_DL(16, 2); PGB_DL(32, 4); PGB_DL(32, 8);                      // 48, 8 as a residual's, too
+    PGB_DL(16, 2); PGB_DL(32, 4); PGB_DL(32, 8);
     PGB_DL(48, 2); PGB_DL(48, 4); PGB_DL(48, 8);
     PGB_DL(64, 2); PGB_DL(64, 4); PGB_DL(64, 8);
+    PGB_DL(96, 4); PGB_DL(96, 8);
 #undef PGB_DL
     return PGB_ERR_TOO_LARGE;
 }

@@ -257,9 +257,14 @@ class Decoder:
             return False
         held = [m.e.weight, m.p.weight, *(n.weight for n in norms), *(t for mp in m.mlp for t in (mp.a.weight, mp.a.bias, mp.b.weight, mp.b.bias) if t is not None)]
         takes, d, V = ops.decode_linear_takes, m.d, m.e.weight.shape[0]
-        return (all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in held) and
-                all(mx.q.weight.dtype == torch.bfloat16 and takes(0, (3 * d + 2 * mx.h + 7) // 8 * 8, d) for mx in m.mix) and takes(1, d, d) and takes(2, V, d) and
-                all(takes(0, mp.a.weight.shape[0], d) and takes(1, d, mp.a.weight.shape[0]) for mp in m.mlp))
+        links = [((0, (3 * d + 2 * mx.h + 7) // 8 * 8, d), (1, d, d), (0, mp.a.weight.shape[0], d), (1, d, mp.a.weight.shape[0])) for mx, mp in zip(m.mix, m.mlp)]
+        if not (all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in held) and
+                all(mx.q.weight.dtype == torch.bfloat16 for mx in m.mix) and takes(2, V, d) and all(takes(*ln) for layer in set(links) for ln in layer)):
+            return False
+        # Links of many rounds over the chip hide nothing of one another. Time of the chain to that of the separate kernels, by the rounds of a layer: up to 7 (d 2048, MLP
+        # 4096) below 0.91 at every batch; 8 or 9 (d 1664 to 1920, MLP 4 d) 0.93 to 0.98 at batch 33, 0.97 to 1.03 at 64; 11 (2304, 6912) 0.82 at batch 5, 1.01 at 16; 14 1.10 to 1.33
+        most = 11 if self.B <= 8 else 9 if self.B <= 48 else 7
+        return all(sum(ops.decode_linear_rounds(*ln, self.B) for ln in layer) <= most for layer in set(links))
 
     def _step_chain(self, advance: bool = True, out: Optional[torch.Tensor] = None):
         """Embedding, five launches a layer and the head, each requesting its weights (the recurrent step: its states) while the one ahead still

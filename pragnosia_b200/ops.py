@@ -503,6 +503,11 @@ def decode_linear_takes(kind: int, N: int, K: int) -> bool:
     return bool(lib().pgb_decode_linear_takes(kind, N, K))
 
 
+def decode_linear_rounds(kind: int, N: int, K: int, B: int) -> int:
+    """In how many rounds the thread blocks of decode_linear go over the chip at these sizes (kinds as for decode_linear_takes)."""
+    return int(lib().pgb_decode_linear_rounds(kind, N, K, B))
+
+
 @on_device_of
 def decode_embed_norm(tok, pos, E, P, next_w):
     """The first kernel of a token whose linear layers are decode_linear's: x (B,d) = E[tok] + P[pos], x next_w, and the rows' sums of squares (B,1)."""

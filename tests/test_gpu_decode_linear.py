@@ -140,3 +140,46 @@ def test_chained_step_with_a_warp_per_pair(d, mixer, B):
         test_chained_step_of_a_batch(d, mixer, 3, 1000, B)
     finally:
         _lib.check(L.pgb_decode_set_variant(0), "pgb_decode_set_variant")
+
+
+def between(y, want, slack, then=lambda t: t):
+    """Rounding is monotone: y = then(bf16(fp32 sum)) lies between what the ends of the sum's interval give."""
+    return bool(((y >= then((want - slack).bfloat16())) & (y <= then((want + slack).bfloat16()))).all())
+
+
+@pytest.mark.parametrize("N,K,tile", [(1080, 3256, 48), (568, 4600, 48), (2104, 2104, 64), (760, 6136, 64), (2168, 2168, 96), (1080, 4344, 96)])
+def test_tiles_of_wide_residual_layers(N, K, tile):
+    """Links that take more than one round in the first form: tiles and clusters of the others, N and K ragged. The fp32 sum is within K 2^-24 of the sum of
+    magnitudes; v, then resid + v, are rounded to bf16."""
+    B = 64
+    assert _lib.lib().pgb_decode_linear_parts(N, K, B) == -(-N // tile)
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x, W, r, w = (torch.randn(*s, device=DEV, generator=g).bfloat16() for s in ((B, K), (N, K), (B, N), (N,)))
+    y, yw, sq = ops.decode_linear(x, W, resid=r, next_w=w)
+    v = x.double() @ W.double().T
+    assert between(y, v, 2.0 ** -24 * K * (x.double().abs() @ W.double().abs().T), lambda t: (t.float() + r.float()).bfloat16())
+    assert torch.equal(yw, (y.float() * w.float()).bfloat16())
+    torch.testing.assert_close(sq.double().sum(1), y.double().square().sum(1), rtol=2.0 ** -24 * 64, atol=0)
+    assert healthy() == 0
+
+
+@pytest.mark.parametrize("N,K", [(1976, 1976), (3832, 952), (2104, 2104), (4664, 4664), (6008, 1976), (3896, 3896)])     # 32 x 4, 64 x 2, 4 and 8, 96 x 4 and 8
+@pytest.mark.parametrize("B", [5, 64])
+def test_tiles_of_wide_layers_behind_a_norm(N, K, B):
+    """v = r (x W^T) + bias, rounded to bf16 once; r is off by its sum, division and root, each in fp32 (2^-20 covers them)."""
+    g = torch.Generator(device=DEV).manual_seed(N + B)
+    x, W, b = (torch.randn(*s, device=DEV, generator=g).bfloat16() for s in ((B, K), (N, K), (N,)))
+    sq = torch.rand(B, 24, device=DEV, generator=g) * K
+    y = ops.decode_linear(x, W, b, sq, 1e-5)
+    rs = (sq.double().sum(1, keepdim=True) / K + 1e-5).rsqrt()
+    v = rs * (x.double() @ W.double().T)
+    slack = rs * 2.0 ** -24 * K * (x.double().abs() @ W.double().abs().T) + 2.0 ** -20 * v.abs() + 2.0 ** -24 * b.double().abs()
+    assert between(y, v + b.double(), slack)
+    assert healthy() == 0
+
+
+@pytest.mark.parametrize("d,mult,B,taken", [(1664, 4, 48, True), (1664, 4, 49, False), (1536, 4, 64, True), (2304, 3, 8, True), (2304, 3, 9, False), (3072, 2, 5, False)])
+def test_wide_models_whose_links_take_many_rounds(d, mult, B, taken):
+    """The chain where it is the quicker, the separate kernels elsewhere: by the rounds of a layer's links and the batch."""
+    m = model(d, "aspin", mult, 256, layers=1)
+    assert Decoder(m, batch=B)._chain_ok() == taken
