@@ -223,53 +223,73 @@ __global__ void __launch_bounds__(SG_NT, FINE ? 1 : 2) segment_state_kernel(cons
     if (warp == 1) tmem_dealloc(tmem, 64);
 }
 
-// A thread owns one value column of a pair of key rows; sixteen segments' additions are requested ahead of the recurrence, whose factors the CTA
-// forms side by side. B1 H12 T8192, cold caches: 9.2 us for 15 segments when a thread owned two columns and asked for four segments at a time.
-constexpr int SC_NT = 128, SC_AHEAD = 16, SC_SEGS = 128;
-__global__ void __launch_bounds__(SC_NT) segment_combine_kernel(float *__restrict__ E, const float *__restrict__ Lend, const float *__restrict__ S0,
-                                                                const float *__restrict__ theta, const float *__restrict__ shift_dev, int n, int BH, int H,
-                                                                float shift_host, bool windows, SegCut seg) {
+// A thread owns COLS value columns of a pair of key rows; AHEAD segments' additions are requested ahead of the recurrence, the first ones also ahead of the factors,
+// which the CTA forms side by side. Up to four segments: two columns a thread, four CTAs of 256 a chain; more: one column, 16 CTAs of 128, sixteen segments ahead. The whole
+// call, us, the first form at any number / the second behind its factors / these: 44 chains of 2048 tokens (training) 34.5 / 35.9 / 33.9, 36 of 1333 22.7 / 23.1 / 22.3,
+// 12 of 8192 35.3 / 33.1 / 32.9, 2 of 4096 18.1 / 14.3 / 14.3, 1 of 8192 22.9 / 16.5 / 16.2.
+constexpr int SC_SEGS = 128, SC_FEW = 4;
+template <int COLS, int AHEAD, int NT>
+__global__ void __launch_bounds__(NT) segment_combine_kernel(float *__restrict__ E, const float *__restrict__ Lend, const float *__restrict__ S0,
+                                                             const float *__restrict__ theta, const float *__restrict__ shift_dev, int n, int BH, int H,
+                                                             float shift_host, bool windows, SegCut seg) {
     __shared__ float2 fac[SC_SEGS];                                   // e^{L}; not zero: the segment begins a window
+    auto get = [](float (&v)[COLS], const float *p) {
+        if constexpr (COLS == 2) { const float2 t = *reinterpret_cast<const float2 *>(p); v[0] = t.x; v[1] = t.y; }
+        else v[0] = *p;
+    };
+    auto put = [](float *p, const float (&v)[COLS]) {
+        if constexpr (COLS == 2) *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+        else *p = v[0];
+    };
     pdl_wait();
-    const int e = blockIdx.x * SC_NT + threadIdx.x, bh = blockIdx.y, i = e / SG_D, j = e % SG_D;
+    const int e = blockIdx.x * NT + threadIdx.x, bh = blockIdx.y, i = e / (SG_D / COLS), j = COLS * (e % (SG_D / COLS));
     const size_t step = (size_t)BH * SG_D * SG_D;
     float *at = E + ((size_t)bh * SG_D + 2 * i) * SG_D + j;
-    float a = 0.f, b = 0.f;                                           // rows 2i, 2i + 1
+    float a[COLS], b[COLS], ua[AHEAD][COLS], ub[AHEAD][COLS];         // rows 2i, 2i + 1
+    auto request = [&](const float *from, int m) {
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k)
+            if (k < m) { get(ua[k], from + k * step); get(ub[k], from + k * step + SG_D); }
+    };
+    request(at, n);
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) a[c] = b[c] = 0.f;
     if (S0 != nullptr) {
         const float *src = S0 + ((size_t)bh * SG_D + 2 * i) * SG_D + j;
-        a = src[0]; b = src[SG_D];
+        get(a, src); get(b, src + SG_D);
     }
     float sn = 0.f, cs = 1.f;
     const float shift = theta == nullptr ? 0.f : (shift_dev != nullptr ? *shift_dev : shift_host);
     if (shift != 0.f) sincosf(-shift * theta[(size_t)(bh % H) * (SG_D / 2) + i], &sn, &cs);
     auto rotate = [&]() {
-        const float ra = a * cs - b * sn;
-        b = a * sn + b * cs; a = ra;
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+            const float ra = a[c] * cs - b[c] * sn;
+            b[c] = a[c] * sn + b[c] * cs; a[c] = ra;
+        }
     };
     if (!windows) rotate();
     for (int s0 = 0; s0 < n; s0 += SC_SEGS) {
         if (s0 > 0) __syncthreads();
-        if (s0 + threadIdx.x < n) {
+        if (threadIdx.x < SC_SEGS && s0 + threadIdx.x < n) {
             int begin, in_piece, tokens;
             seg.at(s0 + threadIdx.x, begin, in_piece, tokens);
             fac[threadIdx.x] = make_float2(expf(Lend[(size_t)(s0 + threadIdx.x) * BH + bh]), in_piece == 0 ? 1.f : 0.f);
         }
         __syncthreads();
         const int m = min(n - s0, SC_SEGS);
-        for (int w0 = 0; w0 < m; w0 += SC_AHEAD) {
+        for (int w0 = 0; w0 < m; w0 += AHEAD) {
             float *here = at + (size_t)(s0 + w0) * step;
-            float ua[SC_AHEAD], ub[SC_AHEAD];
+            if (s0 + w0 > 0) request(here, m - w0);
 #pragma unroll
-            for (int k = 0; k < SC_AHEAD; ++k)
-                if (w0 + k < m) { ua[k] = here[k * step]; ub[k] = here[k * step + SG_D]; }
-#pragma unroll
-            for (int k = 0; k < SC_AHEAD; ++k)
+            for (int k = 0; k < AHEAD; ++k)
                 if (w0 + k < m) {
                     const float2 f = fac[w0 + k];
                     // the state enters a window rotated back by the previous one's length, the sequence's own (S0) too
                     if (windows && f.y != 0.f) rotate();
-                    a = fmaf(f.x, a, ua[k]); b = fmaf(f.x, b, ub[k]);
-                    here[k * step] = a; here[k * step + SG_D] = b;
+#pragma unroll
+                    for (int c = 0; c < COLS; ++c) { a[c] = fmaf(f.x, a[c], ua[k][c]); b[c] = fmaf(f.x, b[c], ub[k][c]); }
+                    put(here + k * step, a); put(here + k * step + SG_D, b);
                 }
         }
     }
@@ -351,9 +371,12 @@ int segment_states_launch(const PrefillArgs &a, float *scratch, cudaStream_t str
     cudaError_t e = a.raw    ? go(segment_state_kernel<true, false>, SgSmem<true, false>::bytes)
                     : a.fine ? go(segment_state_kernel<false, true>, SgSmem<false, true>::bytes)
                              : go(segment_state_kernel<false, false>, SgSmem<false, false>::bytes);
+    auto combine = [&](auto kern, int cols, int threads) {
+        return pdl_launch(kern, dim3((unsigned)(SG_D * SG_D / 2 / cols / threads), (unsigned)BH), dim3((unsigned)threads), (size_t)0, stream, scratch,
+                          (const float *)Lend, a.S0, a.theta, a.shift_dev, nseg - 1, BH, a.H, a.shift_host, (bool)a.seg_rotates, a.seg);
+    };
     if (e == cudaSuccess)
-        e = pdl_launch(segment_combine_kernel, dim3(SG_D * SG_D / 2 / SC_NT, (unsigned)BH), dim3(SC_NT), (size_t)0, stream, scratch, (const float *)Lend, a.S0,
-                       a.theta, a.shift_dev, nseg - 1, BH, a.H, a.shift_host, (bool)a.seg_rotates, a.seg);
+        e = nseg - 1 <= SC_FEW ? combine(segment_combine_kernel<2, 4, 256>, 2, 256) : combine(segment_combine_kernel<1, 16, 128>, 1, 128);
     if (e != cudaSuccess) { set_cuda_error(e, "segment_state launch"); return PGB_ERR_CUDA; }
     return check_launch("segment_state_kernel");
 }

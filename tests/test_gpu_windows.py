@@ -69,6 +69,12 @@ def test_windows_in_parts_that_do_not_divide_them(window, T):
     test_all_windows_at_once_match_window_by_window(False, 64, window, T, B)
 
 
+@pytest.mark.parametrize("n", [4, 5, 16, 17, 128, 129])
+def test_combination_of_few_and_many_segments(n):
+    """The states entering n later windows: at both sides of the two forms' line, of what is requested ahead and of the factors held at a time."""
+    test_all_windows_at_once_match_window_by_window(False, 64, 64, 64 * n + 30, 1)
+
+
 @pytest.mark.parametrize("mixer", ["aspin", "dspin"])
 def test_shape_graphs_and_what_the_caller_keeps(mixer):
     """First call eager, second captured, later ones replayed: the same logits and states every time, and a state kept from one
