@@ -6,7 +6,7 @@
 // (reference src/assoc.py:207-251). N does not depend on the state, so
 //
 //   delta_inv_kernel   (chunk-parallel, one CTA per (sequence-head, chunk)): K K^T on the tensor core, N in fp32, then
-//                      X = (I + N)^-1 by blocked forward substitution to fp32's precision, every intermediate bounded (the
+//                      X = (I + N)^-1 by blocked forward substitution in true fp32 FFMA, every intermediate bounded (the
 //                      reduced-precision Neumann doubling the reference warns about at src/assoc_kernel.py:577-582 is
 //                      never formed). X goes to a scratch buffer as bf16 head + tail.
 //   delta_walk_kernel  (delta_walk.cuh; one CTA per (sequence, head), walking the chunks): W = X rhs, the state update and o.
@@ -14,7 +14,7 @@
 // Everything fp32 that re-enters the tensor core (S, rhs, X, A, W) is split into bf16 head + tail and multiplied as
 // head*head + head*tail + tail*head. Every mbarrier wait is bounded.
 //
-// Measured, B8 H16 T8192 D128 (1.1 GB of operands): walk 396 us, inverse 166.
+// Measured, B8 H16 T8192 D128 (1.1 GB of operands): walk 396 us, inverse 170.
 #include "delta_walk.cuh"
 
 namespace pgb {
@@ -37,82 +37,82 @@ __device__ __forceinline__ void chunk_stats(const float *la, const float *beta, 
 }
 
 // ------------------------------------------------------------------------------------------------ X = (I + N)^-1
-// One column of X per thread is a chain of 2016 dependent multiply-adds on half the threads. The blocked form keeps the chain to 16 steps: the four
-// 16 x 16 diagonal blocks are inverted side by side (half a warp each, a lane per column), then twice X21 = -X22 (N21 X11) joins neighbouring blocks, 16
-// and 32 wide, as warp-level products (m16n8k8, too small for the tensor-memory kind) of factors split into three tf32 parts, which are all of fp32.
-// One array holds all of it, in the K tile's place once that is consumed: N below the diagonal; X transposed above it, a diagonal block of X over N's own
-// once its columns are done; T = N21 X11, transposed, in the quarter that X21 would take (X21 itself goes from registers to memory). 20 KB a CTA where
-// N, X and T side by side were 43: eight CTAs an SM (the tensor memory's limit, too) instead of five.
-// B8 H16 T8192 D128: 194 us with the joins as fp32 register tiles, whose 16-byte shared loads filled the load unit, 166 so; B64 H12 T512 D64 77 and 67. Two
-// parts a factor took 137 and 55, but X21's error against 64 bits rose by 10 to 15 % where keys resemble one another (2.9e-6 -> 3.2e-6 of it, 3.7e-6 -> 4.3e-6
-// for keys that all but repeat); with three it is the register tiles', 0.3 % below to 0.7 % above, X's as a whole 0.02 % below to 0.07 % above. What bounds it: issue slots.
+// One column of X per thread is a chain of 2016 dependent multiply-adds on half the threads. The blocked form keeps the chain to 16 steps: the four 16 x 16
+// diagonal blocks are inverted side by side (half a warp each, a lane per column), then twice X21 = -X22 (N21 X11) joins neighbouring blocks, 16 and 32 wide, as fp32
+// products in register tiles of two by four and four by four, read 16 bytes at a time. Bound by the passes of the shared-memory loads; five CTAs share an SM.
+// B8 H16 T8192 D128: 193 us with tiles of two by four throughout, 170 so; B64 H12 T512 D64 76 and 68.
+// Products on the tensor cores instead (m16n8k8, one array of 20 KB a CTA): factors in two tf32 parts 135 us, but X21's error against 64 bits rises by 10 to 15 % where keys resemble
+// one another (2.9e-6 -> 3.2e-6 of it, 3.7e-6 -> 4.3e-6 for keys that all but repeat) and X's as a whole by 1 %; in three parts, which are all of fp32, 158 to 166.
+template <int D>
 struct InvSmem {
-    static constexpr int P = 68;                                      // row pitch, in floats (16-byte aligned, four banks on)
-    static constexpr int off_misc = TC_C * P * 4;                     // not below a K tile of 64 x 128 bf16
+    static constexpr int NP = 68, TP = 36;                            // row pitches of N / X and of the product T, in floats (16-byte aligned)
+    static constexpr int XB = TC_C * NP * 4;
+    static constexpr int off_k = 0;                                   // K tile, TC_C x D bf16; then X fp32 [64][NP] in its place
+    static constexpr int off_n = XB > TC_C * D * 2 ? (XB + 1023) / 1024 * 1024 : TC_C * D * 2;
+    static constexpr int off_t = off_n + XB;                          // T fp32 [32][TP]
+    static constexpr int off_misc = off_t + 32 * TP * 4;
     static constexpr int bytes = off_misc + 1024 + 1024;
 };
-static_assert(InvSmem::off_misc >= TC_C * 128 * 2, "the K tile lies in the array's place");
 
-// P = A B for 16 rows and NT tiles of eight columns over the K blocks k0 <= k < k1 of eight, by a warp. A element (m, k) lies at A[m ra + k ka], an
-// element (k, n) of B at B[n P + k]. Lane l of the accumulator has rows l / 4 and l / 4 + 8, columns 2 (l % 4) and the next of each tile. Of the products of
-// the factors' three parts all are added but those below 2^-33 of the whole. The heads' products of a block are added by an addition that rounds:
-// accumulated in the tensor core, which cuts off, X was off by 0.1 % more where nothing decays (162 us).
-template <int NT>
-__device__ __forceinline__ void inv_product(float (&acc)[NT][4], const float *A, int ra, int ka, const float *B, int k0, int k1, int lane) {
-    const float *ap = A + (lane >> 2) * ra + (lane & 3) * ka, *bp = B + (lane >> 2) * InvSmem::P + (lane & 3);
-    float low[NT][4];
+// rows r0, r0 + 1 and columns c0..c0+3 of P = A B for K-long rows of A (pitch pa) and rows of B (pitch pb); K a multiple of 4
+template <int K>
+__device__ __forceinline__ void inv_product(float (&acc)[2][4], const float *A, int pa, const float *B, int pb, int r0, int c0) {
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[n][i] = low[n][i] = 0.f;
-#pragma unroll 2
-    for (int k = k0; k < k1; ++k) {
-        uint32_t ah[4], am[4], al[4];
-        tf32_split(ap[8 * k * ka], ah[0], am[0], al[0]);
-        tf32_split(ap[8 * ra + 8 * k * ka], ah[1], am[1], al[1]);
-        tf32_split(ap[(8 * k + 4) * ka], ah[2], am[2], al[2]);
-        tf32_split(ap[8 * ra + (8 * k + 4) * ka], ah[3], am[3], al[3]);
+        for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
 #pragma unroll
-        for (int n = 0; n < NT; ++n) {
-            uint32_t bh[2], bm[2], bl[2];
-            tf32_split(bp[8 * n * InvSmem::P + 8 * k], bh[0], bm[0], bl[0]);
-            tf32_split(bp[8 * n * InvSmem::P + 8 * k + 4], bh[1], bm[1], bl[1]);
-            mma_tf32(low[n], al, bh);
-            mma_tf32(low[n], ah, bl);
-            mma_tf32(low[n], am, bm);
-            mma_tf32(low[n], am, bh);
-            mma_tf32(low[n], ah, bm);
-            float hh[4] = {0.f, 0.f, 0.f, 0.f};
-            mma_tf32(hh, ah, bh);
+    for (int k = 0; k < K; k += 4) {
+        const float4 a0 = *reinterpret_cast<const float4 *>(A + r0 * pa + k), a1 = *reinterpret_cast<const float4 *>(A + (r0 + 1) * pa + k);
+        const float f0[4] = {a0.x, a0.y, a0.z, a0.w}, f1[4] = {a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) acc[n][i] += hh[i];
+        for (int i = 0; i < 4; ++i) {
+            const float4 b = *reinterpret_cast<const float4 *>(B + (k + i) * pb + c0);
+            const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) { acc[0][c] = fmaf(f0[i], bv[c], acc[0][c]); acc[1][c] = fmaf(f1[i], bv[c], acc[1][c]); }
         }
     }
-#pragma unroll
-    for (int n = 0; n < NT; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[n][i] += low[n][i];
 }
-// such an accumulator (or its negative) transposed: element (m, n) to at[n P + m]
-template <int NT, bool NEG>
-__device__ __forceinline__ void inv_put(float *at, const float (&acc)[NT][4], int lane) {
-    float *p = at + 2 * (lane & 3) * InvSmem::P + (lane >> 2);
+
+// rows r0 + RS i and columns c0..c0+3 of P = A B, i < 4, over k0 <= k < K: eight loads of 16 bytes for 64 products, and rows RS apart so
+// that the rows a warp reads at once lie in different banks
+template <int K, int RS>
+__device__ __forceinline__ void inv_product4(float (&acc)[4][4], const float *A, int pa, const float *B, int pb, int r0, int c0, int k0) {
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) p[(8 * n + (i & 1)) * InvSmem::P + 8 * (i >> 1)] = NEG ? -acc[n][i] : acc[n][i];
+        for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
+#pragma unroll 2
+    for (int k = k0; k < K; k += 4) {
+        float f[4][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float4 a = *reinterpret_cast<const float4 *>(A + (r0 + RS * r) * pa + k);
+            f[r][0] = a.x; f[r][1] = a.y; f[r][2] = a.z; f[r][3] = a.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 b = *reinterpret_cast<const float4 *>(B + (k + i) * pb + c0);
+            const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(f[r][i], bv[c], acc[r][c]);
+        }
+    }
 }
 
 template <int D>
-__global__ void __launch_bounds__(128, 8) delta_inv_kernel(const __grid_constant__ CUtensorMap mk, const float *__restrict__ la_all,
+__global__ void __launch_bounds__(128) delta_inv_kernel(const __grid_constant__ CUtensorMap mk, const float *__restrict__ la_all,
                                                         const float *__restrict__ beta_all, __nv_bfloat16 *__restrict__ X, int T,
                                                         int with_tail) {
-    using SM = InvSmem;
-    constexpr int P = SM::P;
+    using SM = InvSmem<D>;
+    constexpr int NP = SM::NP, TP = SM::TP;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *sm = smem_raw + (base - smem_u32(smem_raw));
-    float *M = reinterpret_cast<float *>(sm);                         // the array: N[t][s] at M[t P + s], s < t; X[t][s] at M[s P + t]
+    float *Nf = reinterpret_cast<float *>(sm + SM::off_n), *Xf = reinterpret_cast<float *>(sm + SM::off_k), *Tf = reinterpret_cast<float *>(sm + SM::off_t);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + SM::off_misc + 32);
     float *Ls = reinterpret_cast<float *>(sm + SM::off_misc + 64), *bes = Ls + 64;
     const uint32_t bar_k = base + SM::off_misc, bar_m = bar_k + 8;
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(128, 8) delta_inv_kernel(const __grid_constant
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         mbar_expect_tx(bar_k, TC_C * D * 2);
 #pragma unroll
-        for (int s = 0; s < D / 64; ++s) tma_load_3d(base + s * 8192, &mk, bar_k, 64 * s, t0, bh);
+        for (int s = 0; s < D / 64; ++s) tma_load_3d(base + SM::off_k + s * 8192, &mk, bar_k, 64 * s, t0, bh);
     }
     if (warp == 3) tmem_alloc(smem_u32(tmem_slot), 64);
     if (warp < 2) chunk_stats(la_all + (size_t)bh * T, beta_all + (size_t)bh * T, t0, T, tid, lane, warp, Ls, bes);
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(128, 8) delta_inv_kernel(const __grid_constant
     bool ok = mbar_wait_warp(bar_k, 0, 11);
     if (warp == 2 && ok) {
         constexpr uint32_t I_KK = idesc_bf16(64, 64, 0, 0);
-        const uint64_t dk = smem_desc(base, 16, 1024);
+        const uint64_t dk = smem_desc(base + SM::off_k, 16, 1024);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
             const uint32_t ko = ((uint32_t)(k >> 2) * 8192u + (uint32_t)(k & 3) * 32u) >> 4;
@@ -146,8 +146,7 @@ __global__ void __launch_bounds__(128, 8) delta_inv_kernel(const __grid_constant
     }
     if (ok) ok = mbar_wait_warp(bar_m, 0, 12);
     tc_fence_after();
-    // ---- over K, which the finished product has consumed: N = beta_t (k_t . k_s) exp(min(L_t - L_s, 0)) for s < t.   Each warp: its 16 rows, the columns up to its
-    //      diagonal block's end (beyond lies X's place).
+    // ---- N = beta_t (k_t . k_s) exp(min(L_t - L_s, 0)) for s < t, else 0.   Each warp: its 16 rows, all 64 columns.
     {
         const int fr = lane >> 2, fq = lane & 3, r0 = 16 * warp + fr, r1 = r0 + 8;
         float kk[32];
@@ -156,7 +155,6 @@ __global__ void __launch_bounds__(128, 8) delta_inv_kernel(const __grid_constant
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            if (j > 2 * warp + 1) break;
             const int s = 8 * j + 2 * fq;
             const float2 Lp = *reinterpret_cast<const float2 *>(Ls + s);
             const float La = Lp.x * TD_LOG2E, Lb = Lp.y * TD_LOG2E;
@@ -165,90 +163,97 @@ __global__ void __launch_bounds__(128, 8) delta_inv_kernel(const __grid_constant
             n0.y = (s + 1 < r0) ? b0 * kk[4 * j + 1] * fast_exp2(fminf(L0 - Lb, 0.f)) : 0.f;
             n1.x = (s < r1) ? b1 * kk[4 * j + 2] * fast_exp2(fminf(L1 - La, 0.f)) : 0.f;
             n1.y = (s + 1 < r1) ? b1 * kk[4 * j + 3] * fast_exp2(fminf(L1 - Lb, 0.f)) : 0.f;
-            *reinterpret_cast<float2 *>(M + r0 * P + s) = n0;
-            *reinterpret_cast<float2 *>(M + r1 * P + s) = n1;
+            *reinterpret_cast<float2 *>(Nf + r0 * NP + s) = n0;
+            *reinterpret_cast<float2 *>(Nf + r1 * NP + s) = n1;
         }
     }
     tc_fence_before();
-    __syncthreads();
+    __syncthreads();                                                  // K is consumed (the product is complete): X takes its place
     if (warp == 3) tmem_dealloc(tmem, 64);
     // ---- diagonal blocks: lane j of a half warp owns column j of a block;  x_t = [t == j] - sum_{s<t} N[t][s] x_s
     if (warp < 2) {
         const int j = lane & 15, blk = 2 * warp + (lane >> 4);
-        float *Mb = M + 16 * blk * (P + 1);
+        const float *Nb = Nf + 16 * blk * (NP + 1);
+        float *Xb = Xf + 16 * blk * (NP + 1);
         float x[16];
 #pragma unroll
         for (int t = 0; t < 16; ++t) {
             float a0 = t == j ? 1.f : 0.f, a1 = 0.f;
 #pragma unroll
             for (int s4 = 0; s4 < (t + 3) / 4; ++s4) {
-                const float4 n = *reinterpret_cast<const float4 *>(Mb + t * P + 4 * s4);   // the same address for every lane of a half: a broadcast
+                const float4 n = *reinterpret_cast<const float4 *>(Nb + t * NP + 4 * s4);   // the same address for every lane of a half: a broadcast
                 if (4 * s4 + 0 < t) a0 = fmaf(-n.x, x[4 * s4 + 0], a0);
                 if (4 * s4 + 1 < t) a1 = fmaf(-n.y, x[4 * s4 + 1], a1);
                 if (4 * s4 + 2 < t) a0 = fmaf(-n.z, x[4 * s4 + 2], a0);
                 if (4 * s4 + 3 < t) a1 = fmaf(-n.w, x[4 * s4 + 3], a1);
             }
             x[t] = a0 + a1;
+            Xb[t * NP + j] = x[t];
         }
-        __syncwarp();                                                 // nobody needs N's block any more: X's takes its place, zeros and all
+    } else {                                                          // the two blocks above the diagonal that the joins below read: zero
+        const int g = 32 * (warp & 1), r = 2 * (lane >> 2), cc = 4 * (lane & 3);
 #pragma unroll
-        for (int t = 0; t < 16; t += 4) *reinterpret_cast<float4 *>(Mb + j * P + t) = make_float4(x[t], x[t + 1], x[t + 2], x[t + 3]);
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Xf + (g + r + i) * NP + g + 16 + cc) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
-    // ---- join 16 x 16 blocks, two warps a pair of blocks, eight columns each
-    {
-        const int pair = warp >> 1, g = 32 * pair, c0 = 8 * (warp & 1);            // the pair's first row
-        float *Tt = M + 16 * pair * P + 32 + c0 * P, acc[1][4];
-        inv_product<1>(acc, M + (g + 16) * P + g, P, 1, M + (g + c0) * P + g, 0, 2, lane);
-        inv_put<1, false>(Tt, acc, lane);
-        __syncwarp();                                                 // a warp reads its own columns only
-        inv_product<1>(acc, M + (g + 16) * P + g + 16, 1, P, Tt, 0, 2, lane);
-        inv_put<1, true>(M + (g + c0) * P + g + 16, acc, lane);
+    // ---- join 16 x 16 blocks, a warp per pair of blocks, whose lanes cover the new block as two rows by four columns each
+    if (warp < 2) {
+        float acc[2][4];
+        const int g = 32 * warp, r = 2 * (lane >> 2), cc = 4 * (lane & 3);         // the pair's first row
+        float *Tb = Tf + warp * 16 * TP;
+        inv_product<16>(acc, Nf + (g + 16) * NP + g, NP, Xf + g * NP + g, NP, r, cc);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<float4 *>(Tb + (r + i) * TP + cc) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        __syncwarp();
+        inv_product<16>(acc, Xf + (g + 16) * NP + g + 16, NP, Tb, TP, r, cc);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            *reinterpret_cast<float4 *>(Xf + (g + 16 + r + i) * NP + g + cc) = make_float4(-acc[i][0], -acc[i][1], -acc[i][2], -acc[i][3]);
     }
     __syncthreads();
-    // ---- join the 32 x 32 blocks: T = N21 X11, X21 = -X22 T. A warp has 16 rows by 16 columns of each; blocks of zeros are left out (X11 and X22 are
-    //      lower triangular; N lies in their place).
-    const int m16 = 16 * (warp & 1), n16 = 16 * (warp >> 1);
-    float acc[2][4];
-    inv_product<2>(acc, M + (32 + m16) * P, P, 1, M + n16 * P, n16 / 8, 4, lane);
-    inv_put<2, false>(M + n16 * P + 32 + m16, acc, lane);
-    __syncthreads();
-    inv_product<2>(acc, M + 32 * P + 32 + m16, 1, P, M + n16 * P + 32, 0, m16 / 8 + 2, lane);
-    // ---- head then tail, 8 KB each, to the scratch buffer; or the head alone, densely packed (the stand-alone operator). The last block from the
-    //      registers, neighbouring lanes trading column pairs so that a row's quad stores a whole 32-byte sector.
+    // ---- join the 32 x 32 blocks by two warps, which store the new block from their registers; the other two store the rest meanwhile.
+    //      Head then tail, 8 KB each, to the scratch buffer; or the head alone, densely packed (the stand-alone operator).
     uint4 *dst = reinterpret_cast<uint4 *>(X + ((size_t)bh * NC + c) * ((with_tail ? 2 : 1) * TC_C * TC_C));
-    {
-        const int fr = lane >> 2, fq = lane & 3;
+    if (warp < 2) {
+        float acc[4][4];
+        {   // T = N21 X11, 16 columns a warp: X11 is lower triangular, so the right half's products begin at its row 16
+            const int r = lane >> 2, cc = 16 * warp + 4 * (lane & 3);
+            inv_product4<32, 8>(acc, Nf + 32 * NP, NP, Xf, NP, r, cc, 16 * warp);
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            uint32_t h[2], l[2];
-#pragma unroll
-            for (int n = 0; n < 2; ++n) split2(-acc[n][2 * r], -acc[n][2 * r + 1], h[n], l[n]);
-            const uint32_t gh = __shfl_xor_sync(0xffffffffu, (fq & 1) ? h[0] : h[1], 1), gl = __shfl_xor_sync(0xffffffffu, (fq & 1) ? l[0] : l[1], 1);
-            const int at = (32 + m16 + fr + 8 * r) * 16 + (n16 + 8 * (fq & 1)) / 4 + (fq >> 1);       // in pieces of four columns
-            uint2 *d2 = reinterpret_cast<uint2 *>(dst);
-            d2[at] = (fq & 1) ? make_uint2(gh, h[1]) : make_uint2(h[0], gh);
-            if (with_tail) d2[1024 + at] = (fq & 1) ? make_uint2(gl, l[1]) : make_uint2(l[0], gl);
+            for (int i = 0; i < 4; ++i) *reinterpret_cast<float4 *>(Tf + (r + 8 * i) * TP + cc) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
         }
-    }
-    // the two blocks on the diagonal, eight columns a thread and time, of which the upper block's upper quarter is zero (N lies there)
+        named_sync(1, 64);
+        // X21 = -X22 T, 16 rows a warp: the upper half's products end at column 16
+        const int r = 16 * warp + (lane >> 3), cc = 4 * (lane & 7);
+        if (warp == 0) inv_product4<16, 4>(acc, Xf + 32 * NP + 32, NP, Tf, TP, r, cc, 0);
+        else inv_product4<32, 4>(acc, Xf + 32 * NP + 32, NP, Tf, TP, r, cc, 0);
+        uint2 *d2 = reinterpret_cast<uint2 *>(dst);
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int row = (tid >> 2) + 32 * i, piece = (tid & 3) + 4 * i, rr = row & 31;
-        float x[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = M[(8 * piece + e) * P + row];
-        if (rr < 16 && (tid & 2))
-#pragma unroll
-            for (int e = 0; e < 8; ++e) x[e] = 0.f;
-        uint4 hi, lo;
-        split8(x, hi, lo);
-        dst[row * 8 + piece] = hi;
-        if (with_tail) dst[512 + row * 8 + piece] = lo;
-        if (i == 0) {                                                 // the block above the diagonal: zero
-            dst[row * 8 + piece + 4] = make_uint4(0u, 0u, 0u, 0u);
-            if (with_tail) dst[512 + row * 8 + piece + 4] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = 0; i < 4; ++i) {
+            uint32_t h0, l0, h1, l1;
+            split2(-acc[i][0], -acc[i][1], h0, l0);
+            split2(-acc[i][2], -acc[i][3], h1, l1);
+            d2[(32 + r + 4 * i) * 16 + (lane & 7)] = make_uint2(h0, h1);
+            if (with_tail) d2[1024 + (32 + r + 4 * i) * 16 + (lane & 7)] = make_uint2(l0, l1);
         }
+    } else {
+        auto store = [&](int row, int piece) {                        // eight columns
+            const float4 a = *reinterpret_cast<const float4 *>(Xf + row * NP + 8 * piece), b = *reinterpret_cast<const float4 *>(Xf + row * NP + 8 * piece + 4);
+            const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            uint4 hi, lo;
+            split8(x, hi, lo);
+            dst[row * 8 + piece] = hi;
+            if (with_tail) dst[512 + row * 8 + piece] = lo;
+            if (row < 32) {                                           // the block above the diagonal: zero
+                dst[row * 8 + piece + 4] = make_uint4(0u, 0u, 0u, 0u);
+                if (with_tail) dst[512 + row * 8 + piece + 4] = make_uint4(0u, 0u, 0u, 0u);
+            }
+        };
+        const int t = tid - 64;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) store((t >> 2) + 16 * i, t & 3);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) store(32 + (t >> 2) + 16 * i, 4 + (t & 3));
     }
 }
 
@@ -259,9 +264,9 @@ static int delta_inverse_go(const PrefillArgs &a, void *x_scratch, cudaStream_t 
     CUtensorMap mk;
     if (!tc_make_map(&mk, a.k, BH, a.T, D, D, (long long)a.T * D)) { set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled"); return PGB_ERR_CUDA; }
     auto inv = delta_inv_kernel<D>;
-    const cudaError_t e = cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, InvSmem::bytes);
+    const cudaError_t e = cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, InvSmem<D>::bytes);
     if (e != cudaSuccess) { set_cuda_error(e, "delta_inv smem attribute"); return PGB_ERR_CUDA; }
-    inv<<<dim3(NC, BH), 128, InvSmem::bytes, stream>>>(mk, a.la, a.beta, (__nv_bfloat16 *)x_scratch, a.T, 1);
+    inv<<<dim3(NC, BH), 128, InvSmem<D>::bytes, stream>>>(mk, a.la, a.beta, (__nv_bfloat16 *)x_scratch, a.T, 1);
     return check_launch("delta_inv_kernel");
 }
 // the inverses of the chunks of `a` into x_scratch
@@ -315,9 +320,9 @@ static int delta_inv_go(const void *k, const float *la, const float *beta, void 
     CUtensorMap mk;
     if (!tc_make_map(&mk, k, BH, T, D, D, (long long)T * D)) { set_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled"); return PGB_ERR_CUDA; }
     auto inv = delta_inv_kernel<D>;
-    cudaError_t e = cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, InvSmem::bytes);
+    cudaError_t e = cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, InvSmem<D>::bytes);
     if (e != cudaSuccess) { set_cuda_error(e, "delta_inv smem attribute"); return PGB_ERR_CUDA; }
-    inv<<<dim3(NC, BH), 128, InvSmem::bytes, stream>>>(mk, la, beta, (__nv_bfloat16 *)X, T, 0);
+    inv<<<dim3(NC, BH), 128, InvSmem<D>::bytes, stream>>>(mk, la, beta, (__nv_bfloat16 *)X, T, 0);
     return check_launch("delta_inv_kernel");
 }
 int delta_inv_launch(const void *k, const float *la, const float *beta, void *X, int BH, int T, int D, cudaStream_t stream) {

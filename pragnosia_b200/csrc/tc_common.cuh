@@ -332,11 +332,6 @@ __device__ __forceinline__ void tf32_split(float x, uint32_t &hi, uint32_t &lo) 
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(x - __uint_as_float(hi)));
 }
-// the same with what both leave over as a third, a bit at most: all of x
-__device__ __forceinline__ void tf32_split(float x, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
-    tf32_split(x, hi, mid);
-    lo = __float_as_uint(x - __uint_as_float(hi) - __uint_as_float(mid));
-}
 __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
     asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
