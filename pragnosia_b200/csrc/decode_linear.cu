@@ -4,7 +4,7 @@
 // Such a layer reads its weight once (a few MB) and multiplies next to nothing, so it costs its latency: the kernel ahead, x from the L2, the
 // sums, the way out. This kernel keeps all else off that path:
 //   * The weights, which no kernel ahead writes, are requested before the wait on the kernel ahead. A CTA is small (its share of x and W at
-//     once, 50 to 110 KB, and 64 columns of tensor memory), so that it is resident, set up and holding its weights while the kernel ahead still runs.
+//     once, 50 to 110 KB up to d 960, and 64 columns of tensor memory), so that it is resident, set up and holding its weights while the kernel ahead still runs.
 //   * K is cut over a cluster of S CTAs, so that x (64 rows, all of K) is read once a cluster and not once a CTA: of 64 rows by K 768 a CTA's whole
 //     share would be 98 KB, 3 us from the L2. The sums meet by rows: CTA r of the cluster gets its 64 / S rows from all S (st.async into its shared
 //     memory, counted by its barrier), adds them in rank order and finishes them.
@@ -12,11 +12,12 @@
 //     weight; rounded once, as the normalised row would be) and each row's sum of squares by tiles; here x w is multiplied, and the row's
 //     1 / rms applied to the fp32 sum.
 //
-// A token of 12 layers of 768 (graph replay): batch 64 421 -> 315 us, batch 16 383 -> 240, batch 5 372 -> 223, against the library's products with
-// separate norms. What bounds it now is the chain: at batch 5 3.6 us a link, of which 1.6 are the launch alone (links that return behind their wait), 0.8 x (only the
-// batch's rows are fetched: all 64 took 0.4 more), 0.9 the sums of squares, products and waits, 0.3 the exchange, 0.5 the way out; 5.2 at batch 64
-// (48 KB of x a CTA; of the 12.6 MB of states a layer, their stores are 0.3). An L2 prefetch of the weights two links ahead gave nothing, one barrier for
-// all blocks of K instead of one each 0.4 more a link, two issuing warps 0.2 more.
+// A token of 12 layers of 768 (graph replay): batch 64 421 -> 317 us, batch 16 383 -> 240, batch 5 372 -> 224, against the library's products with
+// separate norms. What bounds it now is the chain, 62 links a token. Linear links that leave early, each variant doing what the one ahead of it does and one thing more, us a
+// token at batch 5 / 64: behind the wait on the kernel ahead 143 / 220 (the state steps in full), x landed 147 / 216, products and row sums done 150 / 228, sums exchanged
+// 186 / 278, all 227 / 318. So of the 3.6 us a link at batch 5 the launch and the wait are 2.3; the exchange is 0.7 of a linear link and the way out 0.9. Only the batch's rows of x
+// are fetched: all 64 took 0.4 a link more. An L2 prefetch of the weights two links ahead gave nothing, one barrier for all blocks of K instead of
+// one each 0.4 more a link, two issuing warps 0.2 more.
 //
 // x [B][K] bf16 is the K-major A operand (64 rows; those past the batch are zero or whatever shared memory holds, each its own row's only), W [N][K] the B operand. Replaces, for T = 1, F.linear with the
 // norm, GELU and residual add around it (src/assoc.py:384-512, src/model.py:552-560). Every wait is bounded; one that runs out sets the error flag, and

@@ -156,7 +156,9 @@ def prefill(q, k, v, la, beta=None, S0=None, theta=None, shift=0.0, want_sent: b
     S0 (B,H,D,D) or None.  theta/shift: rebase S0's key axis by -shift*theta first (shift: number or 0-d CUDA tensor).
     Returns (o in out_dtype (default q's dtype), S fp32, sent bf16 (B,H,NC,D,D) or None).
     Plain rule, bf16, D = 64: long chains that would leave SMs idle are cut into segments, which round their states at other places; where
-    B*H is past the SM count, those are the last rows' only, so equal sequences in one batch may differ in rounding."""
+    B*H is past the SM count, those are the last rows' only, so equal sequences in one batch may differ in rounding.
+    Delta rule, bf16, D = 64, no sent: few chains are cut likewise, as many segments as B*H leaves SMs for. Where the memory for that cannot be had (at
+    most 256 MiB) the chains are walked whole, so a call's last bits depend on B*H and on the memory that is free."""
     theta, shift_dev, shift_host = _shift_args(theta, S0, shift)
     if not _compiling():
         return host().prefill(q, k, v, la, beta, S0, theta, shift_dev, shift_host, want_sent, precision,

@@ -41,7 +41,7 @@ def test_segments_side_by_side_match_whole_chains(B, H, T, S0, shift):
 def test_joins_of_the_chunk_inverse_keep_fp32(D, half):
     """Tokens s < t < u of one unit key, no decay: N[t][s] = b_t, N[u][s] = N[u][t] = b_u, all 24 bits of them, and X[u][s] = -b_u + b_u b_t, which for b_t just
     below 1 cancels down to the factors' last bits. In fp32 the one rounding of b_u b_t is 2^-25 of b_u, and the pair of bf16 it is stored as misses 2^-17 of a
-    result below 2^-8: 2^-24 in all. Factors as two tf32 parts: up to 2^-22.5 (emulated)."""
+    result below 2^-8: 2^-24 in all. Factors as two tf32 parts: up to 2^-22.5 (emulated; they were taken back)."""
     n, L = half // 2, _lib.lib()                                      # triples a chunk: s = i in the upper block, t and u neighbours in the lower
     B, H, NC = 1, 4, 64
     T = 64 * NC
@@ -63,3 +63,36 @@ def test_joins_of_the_chunk_inverse_keep_fp32(D, half):
     bt, bu = beta[..., t].double(), beta[..., t + 1].double()
     off = (X[..., t + 1, s] - (bu * bt - bu)).abs() / bu
     assert float(off.max()) <= 2.0 ** -24, float(off.max().log2())
+
+
+@pytest.mark.parametrize("entry", ["prefill", "layer"])
+def test_segments_whose_memory_cannot_be_had(entry):
+    """Room for the inverses but not for the segments' share: the chains are walked whole, as a call with the least scratch walks them."""
+    B, H, T, D, L = 1, 12, 16000, 64, _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(3)
+    rn = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    if entry == "prefill":
+        q, k, v = rn(B, H, T, D).bfloat16(), F.normalize(rn(B, H, T, D), dim=-1).bfloat16(), rn(B, H, T, D).bfloat16()
+        la, beta = F.logsigmoid(2.0 + rn(B, H, T)), torch.sigmoid(rn(B, H, T))
+        full, least = L.pgb_aspin_delta_prefill_scratch_bytes(B, H, T, D), L.pgb_aspin_delta_scratch_bytes(B, H, T)
+        call = lambda: ops.prefill(q, k, v, la, beta)[:2]
+    else:
+        y, A, onw = rn(B, T, 3 * H * D + 2 * H).bfloat16(), torch.linspace(-2, -8, H, device=DEV), torch.ones(D, device=DEV)
+        qp, kp, vp = (y[..., i * H * D:(i + 1) * H * D].unflatten(-1, (H, D)) for i in range(3))
+        a, b, th, pos = y[..., 3 * H * D:3 * H * D + H], y[..., 3 * H * D + H:], rn(H, D // 2).abs(), torch.arange(T, device=DEV) % 512
+        full, least = L.pgb_aspin_delta_layer_scratch_bytes(B, H, T, D), L.pgb_aspin_delta_layer_scratch_least_bytes(B, H, T, D)
+        call = lambda: ops.delta_layer_windows(qp, kp, vp, a, b, A, th, pos, 512, onw, 1e-6)
+    assert full > least + (64 << 20)
+    want = call()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    ooms = torch.cuda.memory_stats()["num_ooms"]
+    room = least + B * H * T * D * 2 + (32 << 20)
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + room) / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        got = call()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.cuda.memory_stats()["num_ooms"] == ooms + 1
+    rel = lambda x, y: float((x.double() - y.double()).norm() / y.double().norm())
+    assert rel(got[0], want[0]) <= 2.0 ** -8 and rel(got[1], want[1]) <= 7.5e-6         # o is rounded to bf16 either way
