@@ -7,8 +7,8 @@
 //   delta_join_kernel    o = oB + E^T a to fp32's precision, a CTA per chunk; then what the walk's caller does with the read (the per-head RMS norm and the token-major
 //                        layout of the layer, or neither).
 // The chain of a sequence is a segment long instead of a sequence: 36 chains of 21 chunks: 55 us -> 24 for
-// the walk of four segments of six, 6 and 13 (a language model's pass of three sequences of 1333 tokens, six layers, 954 -> 834 us); 12 chains of 63 chunks
-// 174 -> 61 with their inverses (12 of it), 2 of 32 89 -> 36. Error against 64 bits, segments to whole chains, over decays and keys of seven kinds and four shapes: S (5e-6 where
+// the walk of four segments of six, 6 and 13 (a language model's pass of three sequences of 1333 tokens, six layers, 958 -> 847 us); 12 chains of 63 chunks
+// 175 -> 62 with their inverses (12 of it), 2 of 32 88 -> 36. Error against 64 bits, segments to whole chains, over decays and keys of seven kinds and four shapes: S (5e-6 where
 // keys are drawn alike) 0.97 to 1.06 times, 1.00 on the mean; o (5.1e-6, read in fp32) 1.00 to 1.02 times, 1.004 on the mean: oB and E^T a round apart. The read in bf16, the
 // default, rounds to 300 times that.
 #include "delta_walk.cuh"

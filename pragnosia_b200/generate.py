@@ -269,7 +269,7 @@ class Decoder:
     def _step_chain(self, advance: bool = True, out: Optional[torch.Tensor] = None):
         """Embedding, five launches a layer and the head, each requesting its weights (the recurrent step: its states) while the one ahead still
         runs. Roundings are those of the separate kernels, but for a norm's 1 / rms, which is applied to the fp32 product behind the
-        rounding of the row instead of ahead of it. B 64, 12 layers of 768: 421 -> 316 us a token; B 5: 372 -> 223."""
+        rounding of the row instead of ahead of it. B 64, 12 layers of 768: 421 -> 317 us a token; B 5: 372 -> 224."""
         m = self.m
         per = [mx._consts() for mx in m.mix]                          # whatever they launch comes ahead of the chain
         after = [*(mx.ln for mx in m.mix[1:]), m.n]
